@@ -25,9 +25,8 @@
 //           (r*P+s)*128 bytes into the halo tile: the 128-byte swizzle is a function of the
 //           absolute shared-memory address, so a view shifted by whole rows reads consistently.
 //           MT accumulators of 128 x BN fp32 live in TMEM, double-buffered when they fit.
-//   warps 2-9  epilogue (two warps per TMEM lane quadrant, 32 columns each): tcgen05.ld, scale/shift (+ residual) (+ ReLU), zero the pad slots,
-//           convert, write a swizzled 128 x 64 slab in shared memory, TMA store.  Each thread
-//           fetches the residual of its own row one slab ahead, straight into registers.
+//   warps 2-9  epilogue (epilogue.cuh; two warps per TMEM lane quadrant, slabs in turn): tcgen05.ld, scale/shift
+//           (+ residual, brought into the staging buffer by TMA) (+ ReLU), zero the pad slots, convert, TMA store.
 // Every wait is bounded and abortable; a timed-out wait sets the device status word.
 #include <cuda.h>
 #include <cudaTypedefs.h>
@@ -37,6 +36,7 @@
 
 #include <mutex>
 
+#include "epilogue.cuh"
 #include "kernels.h"
 #include "ptx.cuh"
 
@@ -44,24 +44,21 @@ namespace nncv_b200 {
 
 namespace {
 
-constexpr int kEpiWarps = 8;               // two warps per TMEM lane quadrant, 32 columns each
-constexpr int kEpiThreads = kEpiWarps * 32;
-constexpr int kThreads = 64 + kEpiThreads;  // warp 0 TMA, warp 1 MMA, warps 2.. epilogue
-constexpr int kSlabBytes = 128 * 128;  // 128 rows x 64 fp16
-constexpr int kResPrefetch = 5;  // slabs between the L2 prefetch of a residual row and its use
+constexpr int kThreads = 64 + epi::kThreads;  // warp 0 TMA, warp 1 MMA, warps 2.. epilogue
 constexpr int kMaxInStages = 4;
 constexpr int kMaxWStages = 8;
+constexpr size_t kBarBytes = 8 * (2 * kMaxInStages + 2 * kMaxWStages + 4 + epi::kWarps * epi::kMaxBufs) + 16;
 
 struct C3Params {
   const uint8_t* wpack;
   const float* scale;
   const float* shift;
-  const uint16_t* residual;  // shared-pad [T, Kout] or null
   int Kout;
   int* error_flag;
   int T;          // total slots
   int P;          // row pitch in slots (W + 1)
   int Himg;       // rows per image (H + 1)
+  epi::FastDiv div_p, div_h, div_nt;   // by P, Himg, n_tiles
   int CB;         // channel blocks of 64
   int n_tiles;    // Kout / BN
   int m_items;    // ceil(T / (MT * 128))
@@ -69,13 +66,15 @@ struct C3Params {
   int in_boxes;   // boxes per input stage
   int in_stages;  // input ring depth
   int w_stages;   // weight ring depth (streamed mode)
-  int relu, has_res, bf16;
+  int relu, bf16;
+  int has_res;    // tm_res holds a shared-pad [T, Kout] tensor that is added before the activation
+  int epi_bufs;   // staging buffers per epilogue warp (1 .. epi::kMaxBufs)
 };
 
 template <int BN, int MT, bool RESIDENT>
 __global__ void __launch_bounds__(kThreads, 1)
 conv3x3_kernel(const __grid_constant__ CUtensorMap tm_in, const __grid_constant__ CUtensorMap tm_out,
-               const C3Params p) {
+               const __grid_constant__ CUtensorMap tm_res, const C3Params p) {
   constexpr int AB = (2 * MT * BN <= 512) ? 2 : 1;  // accumulator buffers in TMEM
   constexpr int ACC_COLS = AB * MT * BN;
   constexpr int WTILE = BN * 128;
@@ -84,6 +83,7 @@ conv3x3_kernel(const __grid_constant__ CUtensorMap tm_in, const __grid_constant_
 
   extern __shared__ uint8_t smem_raw[];
   __shared__ int s_abort;
+  __shared__ __align__(16) float4 s_cols[epi::kWarps][32];   // scale / shift of the slab each epilogue warp works on
   const uint32_t raw = ptx::smem_u32(smem_raw);
   const uint32_t base = (raw + 1023u) & ~1023u;
   const int in_stage_bytes = p.in_boxes * p.box_rows * 128;  // multiple of 1024
@@ -91,11 +91,12 @@ conv3x3_kernel(const __grid_constant__ CUtensorMap tm_in, const __grid_constant_
   const uint32_t sIn = base;
   const uint32_t sW = sIn + (uint32_t)p.in_stages * in_stage_bytes;
   const uint32_t sStage = sW + (uint32_t)(RESIDENT ? kb_total : p.w_stages) * WTILE;
-  const uint32_t bars = sStage + 2 * kSlabBytes;
+  const uint32_t bars = sStage + (uint32_t)(epi::kWarps * p.epi_bufs) * epi::kBufBytes;
   const uint32_t in_full = bars, in_empty = bars + 8 * kMaxInStages;
   const uint32_t w_full = in_empty + 8 * kMaxInStages, w_empty = w_full + 8 * kMaxWStages;
   const uint32_t acc_full = w_empty + 8 * kMaxWStages, acc_empty = acc_full + 16;
-  const uint32_t tmem_slot = acc_empty + 16;
+  const uint32_t res_full = acc_empty + 16;
+  const uint32_t tmem_slot = res_full + 8 * epi::kWarps * epi::kMaxBufs;
   {
     // the carve-up above must fit the dynamic shared memory of this launch: refuse to run otherwise
     uint32_t dyn_bytes;
@@ -121,11 +122,13 @@ conv3x3_kernel(const __grid_constant__ CUtensorMap tm_in, const __grid_constant_
     }
     for (int i = 0; i < 2; ++i) {
       ptx::mbar_init(acc_full + 8 * i, 1);
-      ptx::mbar_init(acc_empty + 8 * i, kEpiThreads);
+      ptx::mbar_init(acc_empty + 8 * i, epi::kWarps);
     }
+    for (int i = 0; i < epi::kWarps * epi::kMaxBufs; ++i) ptx::mbar_init(res_full + 8 * i, 1);
     ptx::mbar_fence_init();
     ptx::prefetch_tensormap(&tm_in);
     ptx::prefetch_tensormap(&tm_out);
+    if (p.has_res) ptx::prefetch_tensormap(&tm_res);
   }
   if (warp == 1) {
     ptx::tmem_alloc(tmem_slot, ACC_COLS);
@@ -151,7 +154,7 @@ conv3x3_kernel(const __grid_constant__ CUtensorMap tm_in, const __grid_constant_
       m_item = w;
       n_tile = (int)blockIdx.y;
     } else {
-      m_item = w / p.n_tiles;
+      m_item = (int)epi::div_by((uint32_t)w, p.div_nt);
       n_tile = w - m_item * p.n_tiles;
     }
     return w < total_items;
@@ -257,163 +260,116 @@ conv3x3_kernel(const __grid_constant__ CUtensorMap tm_in, const __grid_constant_
     }
   } else {
     // ------------------------------------------------------------------ epilogue --------
-    const int quad = warp & 3;            // TMEM lane quadrant this warp may read
-    const int half = (warp - 2) >> 2;     // which 32 of the slab's 64 columns this warp handles
-    const int row = quad * 32 + lane;     // row of the 128-row sub-tile
-    const bool elected = threadIdx.x == 64;
-    const uint32_t sw = (uint32_t)(row & 7);
-    // slab j of this CTA -> (item, sub-tile, 64-column slab)
-    auto slab_of = [&](int j, int& q_tile, int& ncol) {
+    // Eight independent warps (epilogue.cuh); slabs of an item: sub-tile major, then 64 columns.
+    const int ew = warp - 2, quad = warp & 3, half = ew >> 2;
+    const uint32_t sw = (uint32_t)(lane & 7);
+    const int nb = p.epi_bufs;
+    const uint32_t my_stage = sStage + (uint32_t)(ew * nb) * epi::kBufBytes;
+    const uint32_t my_res = res_full + (uint32_t)(ew * epi::kMaxBufs) * 8u;
+    const uint32_t tab = ptx::smem_u32(&s_cols[ew][0]);
+    const int mode = epi::mode_of(p.bf16 != 0, p.has_res != 0, p.relu != 0, 0);
+    // slab j -> first slot of this warp's rows, first column
+    auto slab_of = [&](int j, int& q0, int& ncol) {
       const int i = j / SPI, rem = j - i * SPI;
       int m_item, n_tile;
       if (!item_of(i, m_item, n_tile)) return false;
       const int t = rem / SLABS, sl = rem - t * SLABS;
-      q_tile = m_item * (MT * 128) + t * 128;
+      q0 = m_item * (MT * 128) + t * 128 + quad * 32;
       ncol = n_tile * BN + sl * 64;
       return true;
     };
-    // residual of the first slab (later slabs are fetched one slab ahead inside the loop).  Two
-    // register sets alternate between "in use" and "in flight": copying one into the other at the
-    // end of a slab would make every slab wait for the loads it has just issued.
-    uint32_t res_a[2][8], res_b[2][8];
-    bool have_a = false, have_b = false;
-    if (p.has_res) {
-      int q_tile, ncol;
-      if (slab_of(0, q_tile, ncol) && q_tile + row < p.T) {
-        have_a = true;
-        const uint16_t* rp = p.residual + ((size_t)(q_tile + row) * p.Kout + ncol + half * 32);
-        ptx::ldg_256(rp, res_a[0]);
-        ptx::ldg_256(rp + 16, res_a[1]);
-      }
-    }
-    if (p.has_res) {
-      for (int j = 1; j < kResPrefetch; ++j) {
-        int qf, nf;
-        if (slab_of(j, qf, nf) && qf + row < p.T)
-          asm volatile("prefetch.global.L2 [%0];" ::"l"(p.residual + ((size_t)(qf + row) * p.Kout + nf + half * 32)));
-      }
-    }
-    uint32_t acc_cnt = 0;
-    bool okw = true;
-    // one slab; returns false when the loop is over (no more slabs, or a wait gave up: okw false)
-    auto do_slab = [&](int j, uint32_t (&res_cur)[2][8], bool& have_cur, uint32_t (&res_next)[2][8], bool& have_next) -> bool {
-      int q_tile, ncol;
-      if (!slab_of(j, q_tile, ncol)) return false;
-      const int rem = j % SPI;
-      const int t = rem / SLABS, sl = rem - t * SLABS;
-      const uint32_t sb = (uint32_t)j & 1u;
-      const uint32_t ab = acc_cnt % AB;
-      // Everything that does not depend on the accumulator is issued before the waits: pad test,
-      // per-channel scale/shift, and (below) the residual of the NEXT slab.
-      const int q = q_tile + row;
-      bool valid = q < p.T;
-      if (valid) {
-        const int yrow = q / p.P;
-        valid = (q - yrow * p.P != 0) && (yrow % p.Himg != 0);
-      }
-      const int n0 = ncol + half * 32;
-      float4 sc[8], sh[8];
-#pragma unroll
-      for (int i = 0; i < 8; ++i) {
-        sc[i] = p.scale ? __ldg(reinterpret_cast<const float4*>(p.scale + n0) + i) : make_float4(1.f, 1.f, 1.f, 1.f);
-        sh[i] = p.shift ? __ldg(reinterpret_cast<const float4*>(p.shift + n0) + i) : make_float4(0.f, 0.f, 0.f, 0.f);
-      }
-      bool got = true;
-      if (rem == 0) got = ptx::mbar_wait_abortable(acc_full + 8 * ab, (acc_cnt / AB) & 1u, abort_flag);
-      // all epilogue threads take the same exit: nobody is left alone at a named barrier
-      if (!ptx::named_bar_and(3, kEpiThreads, got)) { okw = false; return false; }
-      ptx::tc_fence_after();
-      const uint32_t srow = sStage + sb * kSlabBytes + (uint32_t)row * 128u;
-      const uint32_t t_addr = tmem_base + ((uint32_t)(quad * 32) << 16) + ab * (MT * BN) + t * BN + sl * 64;
-      uint32_t acc[32];
-      __syncwarp();
-      ptx::tmem_ld_32x32(t_addr + half * 32, acc);
-      // residual of the next slab: in flight while this slab is converted and stored
-      have_next = false;
-      if (p.has_res) {
-        int qn, nn;
-        if (slab_of(j + 1, qn, nn)) {
-          const int qr = qn + row;
-          if (qr < p.T) {
-            have_next = true;
-            const uint16_t* rp = p.residual + ((size_t)qr * p.Kout + nn + half * 32);
-            ptx::ldg_256(rp, res_next[0]);
-            ptx::ldg_256(rp + 16, res_next[1]);
-          }
+    uint32_t phase = 0, inflight = 0;   // per staging buffer: parity of its next residual, one on its way
+    int ahead_j = half, ahead_b = 0;
+    auto fetch_res = [&]() {   // residual rows of the next slab in line -> its staging buffer
+      int q0, ncol;
+      if (slab_of(ahead_j, q0, ncol) && q0 < p.T) {
+        inflight |= 1u << ahead_b;
+        if (lane == 0) {
+          ptx::mbar_arrive_expect_tx(my_res + 8 * ahead_b, epi::kBufBytes);
+          ptx::tma_load_2d(my_stage + (uint32_t)ahead_b * epi::kBufBytes, &tm_res, ncol, q0, my_res + 8 * ahead_b);
         }
       }
-      __syncwarp();
-      if (p.has_res) {  // and pull the residual rows of a later slab from HBM into L2
-        int qf, nf;
-        if (slab_of(j + kResPrefetch, qf, nf) && qf + row < p.T)
-          asm volatile("prefetch.global.L2 [%0];" ::"l"(p.residual + ((size_t)(qf + row) * p.Kout + nf + half * 32)));
-      }
-      ptx::tmem_ld_wait();
-      if (rem == SPI - 1) {  // the accumulator is in registers: hand the TMEM buffer back
-        ptx::tc_fence_before();
-        ptx::mbar_arrive(acc_empty + 8 * ab);
-        ++acc_cnt;
-      }
-      float v[32];
-#pragma unroll
-      for (int i = 0; i < 8; ++i) {
-        v[4 * i] = fmaf(__uint_as_float(acc[4 * i]), sc[i].x, sh[i].x);
-        v[4 * i + 1] = fmaf(__uint_as_float(acc[4 * i + 1]), sc[i].y, sh[i].y);
-        v[4 * i + 2] = fmaf(__uint_as_float(acc[4 * i + 2]), sc[i].z, sh[i].z);
-        v[4 * i + 3] = fmaf(__uint_as_float(acc[4 * i + 3]), sc[i].w, sh[i].w);
-      }
-#pragma unroll
-      for (int c4 = 0; c4 < 4; ++c4) {
-        const uint32_t chunk = (uint32_t)(half * 4 + c4);
-        const uint32_t addr = srow + ((chunk ^ sw) << 4);
-        if (p.has_res && have_cur) {
-          const uint32_t w4[4] = {res_cur[c4 >> 1][(c4 & 1) * 4], res_cur[c4 >> 1][(c4 & 1) * 4 + 1],
-                                  res_cur[c4 >> 1][(c4 & 1) * 4 + 2], res_cur[c4 >> 1][(c4 & 1) * 4 + 3]};
-#pragma unroll
-          for (int h = 0; h < 4; ++h) {
-            float2 f;
-            if (p.bf16) f = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&w4[h]));
-            else f = __half22float2(*reinterpret_cast<const __half2*>(&w4[h]));
-            v[c4 * 8 + h * 2] += f.x;
-            v[c4 * 8 + h * 2 + 1] += f.y;
-          }
-        }
-        uint32_t o[4];
-#pragma unroll
-        for (int h = 0; h < 4; ++h) {
-          const float a = v[c4 * 8 + h * 2], b = v[c4 * 8 + h * 2 + 1];
-          uint32_t packed;
-          // conversion and ReLU in one instruction (cvt.rn.relu: negative -> +0, a NaN stays NaN, like cmpf ugt + select)
-          if (p.bf16) {
-            if (p.relu) {
-              packed = ptx::pack_bf162_relu(a, b);
-            } else {
-              const __nv_bfloat162 x = __floats2bfloat162_rn(a, b);
-              packed = *reinterpret_cast<const uint32_t*>(&x);
-            }
-          } else {
-            packed = p.relu ? ptx::pack_half2_sat_relu(a, b) : ptx::pack_half2_sat(a, b);
-          }
-          o[h] = valid ? packed : 0u;
-        }
-        asm volatile("st.shared.v4.u32 [%0], {%1,%2,%3,%4};" ::"r"(addr), "r"(o[0]), "r"(o[1]), "r"(o[2]), "r"(o[3]) : "memory");
-      }
-      ptx::fence_proxy_async_smem();
-      ptx::named_bar_sync(1, kEpiThreads);
-      if (elected) {
-        ptx::tma_store_2d(&tm_out, ncol, q_tile, sStage + sb * kSlabBytes);
-        ptx::bulk_commit();
-        ptx::bulk_wait_read<1>();  // the store that last read the other buffer has finished
-      }
-      ptx::named_bar_sync(2, kEpiThreads);  // the other staging buffer is free for everyone
-      return true;
+      ahead_j += 2;
+      if (++ahead_b == nb) ahead_b = 0;
     };
-    for (int j = 0;; j += 2) {
-      if (!do_slab(j, res_a, have_a, res_b, have_b)) break;
-      if (!do_slab(j + 1, res_b, have_b, res_a, have_a)) break;
+    int j = half, b = 0;
+    int q0 = 0, ncol = 0;
+    bool have = slab_of(j, q0, ncol);
+    epi::ColParams cols = epi::fetch_cols(p.scale, p.shift, have ? ncol : 0, p.Kout, lane);
+    if (p.has_res)
+      for (int k = 0; k + 1 < nb; ++k) fetch_res();
+    bool okw = true;
+    for (int i = 0; okw; ++i) {
+      int m_item, n_tile;
+      if (!item_of(i, m_item, n_tile)) break;
+      const uint32_t ab = (uint32_t)i % AB;
+      okw = ptx::mbar_wait_abortable(acc_full + 8 * ab, ((uint32_t)i / AB) & 1u, abort_flag);
+      okw = __all_sync(0xffffffffu, okw);
+      if (!okw) break;
+      ptx::tc_fence_after();
+      auto hand_back = [&]() {   // this warp has read its part of the accumulator
+        ptx::tc_fence_before();
+        __syncwarp();
+        if (lane == 0) ptx::mbar_arrive(acc_empty + 8 * ab);
+      };
+      const int end_j = (i + 1) * SPI;
+      if (j >= end_j) hand_back();   // no slab of this item is this warp's
+      for (; j < end_j; j += 2) {
+        const int rem = j - i * SPI;
+        const int t = rem / SLABS, sl = rem - t * SLABS;
+        const bool live = q0 < p.T;
+        const uint32_t taddr = tmem_base + ((uint32_t)(quad * 32) << 16) + ab * (MT * BN) + (uint32_t)(t * BN + sl * 64);
+        uint32_t acc[64];
+        ptx::tmem_ld_32x64(taddr, acc);
+        epi::put_cols(tab, cols, lane);
+        if (p.has_res) {
+          if (lane == 0) ptx::bulk_wait_read<0>();   // the buffer the next residual goes to was stored from one slab ago
+          __syncwarp();
+          fetch_res();
+        } else if (lane == 0) {
+          if (nb == 1) ptx::bulk_wait_read<0>();
+          else ptx::bulk_wait_read<1>();
+        }
+        // pad slots (column 0 of a row, row 0 of an image) leave as zeros
+        const int q = q0 + lane;
+        const uint32_t yrow = epi::div_by((uint32_t)q, p.div_p), img = epi::div_by(yrow, p.div_h);
+        const bool keep = (uint32_t)q != yrow * (uint32_t)p.P && yrow != img * (uint32_t)p.Himg;
+        ptx::tmem_ld_wait();
+        __syncwarp();
+        if (j + 2 >= end_j) hand_back();
+        int q0n = 0, ncoln = 0;
+        have = slab_of(j + 2, q0n, ncoln);
+        cols = epi::fetch_cols(p.scale, p.shift, have ? ncoln : 0, p.Kout, lane);
+        if (live) {
+          const uint32_t srow = my_stage + (uint32_t)b * epi::kBufBytes + (uint32_t)lane * 128u;
+          if (p.has_res) {
+            okw = ptx::mbar_wait_abortable(my_res + 8 * b, (phase >> b) & 1u, abort_flag);
+            okw = __all_sync(0xffffffffu, okw);
+            if (!okw) break;
+            phase ^= 1u << b;
+            inflight &= ~(1u << b);
+          }
+          epi::row64_by_mode<1>(mode, acc, tab, srow, sw);
+          if (!keep) epi::zero_row(srow);
+          ptx::fence_proxy_async_smem();
+          __syncwarp();
+          if (lane == 0) {
+            ptx::tma_store_2d(&tm_out, ncol, q0, my_stage + (uint32_t)b * epi::kBufBytes);
+            ptx::bulk_commit();
+          }
+        }
+        __syncwarp();
+        q0 = q0n;
+        ncol = ncoln;
+        if (++b == nb) b = 0;
+      }
     }
-    if (elected) ptx::bulk_wait<0>();
-    if (!okw && p.error_flag) atomicCAS(p.error_flag, 0, (int)kErrWaitEpilogue);
+    if (!okw) {
+      if (lane == 0 && p.error_flag) atomicCAS(p.error_flag, 0, (int)kErrWaitEpilogue);
+      for (int k = 0; k < nb; ++k)   // residual rows still on their way land before the block ends
+        if ((inflight >> k) & 1u) ptx::mbar_wait_limit(my_res + 8 * k, (phase >> k) & 1u, 1LL << 24);
+    }
+    if (lane == 0) ptx::bulk_wait<0>();
   }
 
   ptx::tc_fence_before();
@@ -453,40 +409,45 @@ bool make_map(CUtensorMap* m, const void* ptr, long long rows, int cols, int box
              CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-constexpr size_t kSmemLimit = 227 * 1024;
+constexpr size_t kSmemLimit = 222 * 1024;   // dynamic part; the kernel also holds 4 KB of static shared memory
 
 template <int BN, int MT, bool RESIDENT>
 cudaError_t launch_cfg(const Conv3x3Args& a, cudaStream_t stream) {
   C3Params p;
   p.wpack = static_cast<const uint8_t*>(a.wpack);
   p.scale = a.scale; p.shift = a.shift; p.error_flag = a.error_flag;
-  p.residual = static_cast<const uint16_t*>(a.residual); p.Kout = a.Kout;
+  p.Kout = a.Kout; p.has_res = a.residual != nullptr;
   p.P = a.W + 1; p.Himg = a.H + 1;
+  p.div_p = epi::fast_div((uint32_t)p.P); p.div_h = epi::fast_div((uint32_t)p.Himg);
   const long long T = (long long)a.N * p.Himg * p.P;
   if (T <= 0 || T > 0x7fffff00LL) return cudaErrorInvalidValue;
   p.T = (int)T;
   p.CB = a.C / 64;
   p.n_tiles = a.Kout / BN;
+  p.div_nt = epi::fast_div((uint32_t)p.n_tiles);
   p.m_items = (int)((T + MT * 128 - 1) / (MT * 128));
   const int rows_in = MT * 128 + 2 * p.P + 2;
   p.in_boxes = (rows_in + 255) / 256;
   p.box_rows = ((rows_in + p.in_boxes - 1) / p.in_boxes + 7) & ~7;
   if (p.box_rows > 256) return cudaErrorInvalidValue;
   const size_t in_stage = (size_t)p.in_boxes * p.box_rows * 128;
-  const size_t fixed = 1024 + 2 * kSlabBytes + 512;
   const size_t wtile = (size_t)BN * 128;
+  const size_t wres = (size_t)9 * p.CB * wtile;
+  p.epi_bufs = epi::pick_bufs(p.has_res != 0, kSmemLimit - 1024 - kBarBytes, (RESIDENT ? wres : 4 * wtile) + 2 * in_stage,
+                              (RESIDENT ? wres : 2 * wtile) + 2 * in_stage);
+  const size_t fixed = 1024 + (size_t)(epi::kWarps * p.epi_bufs) * epi::kBufBytes + kBarBytes;
   size_t wbytes;
   if (RESIDENT) {
     wbytes = (size_t)9 * p.CB * wtile;
-    if (fixed + wbytes + 2 * in_stage > kSmemLimit) return cudaErrorInvalidConfiguration;
+    if (fixed + wbytes + in_stage > kSmemLimit) return cudaErrorInvalidConfiguration;
     p.w_stages = 0;
     size_t room = kSmemLimit - fixed - wbytes;
     p.in_stages = (int)(room / in_stage);
     if (p.in_stages > kMaxInStages) p.in_stages = kMaxInStages;
   } else {
-    p.in_stages = 2;
-    if (fixed + 2 * in_stage + 2 * wtile > kSmemLimit) return cudaErrorInvalidConfiguration;
-    size_t room = kSmemLimit - fixed - 2 * in_stage;
+    p.in_stages = fixed + 2 * in_stage + 2 * wtile <= kSmemLimit ? 2 : 1;   // very wide maps: one halo tile at a time
+    if (fixed + p.in_stages * in_stage + 2 * wtile > kSmemLimit) return cudaErrorInvalidConfiguration;
+    size_t room = kSmemLimit - fixed - p.in_stages * in_stage;
     p.w_stages = (int)(room / wtile);
     if (p.w_stages > kMaxWStages) p.w_stages = kMaxWStages;
     // spare room beyond a deep weight ring goes to a third input stage
@@ -499,11 +460,11 @@ cudaError_t launch_cfg(const Conv3x3Args& a, cudaStream_t stream) {
     wbytes = (size_t)p.w_stages * wtile;
   }
   const size_t smem = fixed + wbytes + (size_t)p.in_stages * in_stage;
-  p.relu = a.relu; p.has_res = a.residual != nullptr; p.bf16 = a.ab == kBF16;
+  p.relu = a.relu; p.bf16 = a.ab == kBF16;
 
-  CUtensorMap tm_in, tm_out;
-  if (!make_map(&tm_in, a.in, T, a.C, p.box_rows, p.bf16) ||
-      !make_map(&tm_out, a.out, T, a.Kout, 128, p.bf16))
+  CUtensorMap tm_in, tm_out, tm_res;
+  if (!make_map(&tm_in, a.in, T, a.C, p.box_rows, p.bf16) || !make_map(&tm_out, a.out, T, a.Kout, 32, p.bf16) ||
+      !make_map(&tm_res, p.has_res ? a.residual : a.out, T, a.Kout, 32, p.bf16))
     return cudaErrorInvalidValue;
 
   auto kern = conv3x3_kernel<BN, MT, RESIDENT>;
@@ -520,7 +481,7 @@ cudaError_t launch_cfg(const Conv3x3Args& a, cudaStream_t stream) {
     const int items = p.m_items * p.n_tiles;
     grid = dim3(items < sms ? items : sms, 1);
   }
-  return launch_pdl(kern, grid, dim3(kThreads), smem, stream, tm_in, tm_out, p);
+  return launch_pdl(kern, grid, dim3(kThreads), smem, stream, tm_in, tm_out, tm_res, p);
 }
 
 }  // namespace

@@ -13,7 +13,7 @@
 //                       two arrivals), so the issuing lane tests one barrier per stage.
 //   in_empty / w_empty  the leader commits its MMAs to the local AND (mapped address) the peer's
 //                       barrier, so both producers reuse the stage.
-//   acc_full            committed to both CTAs; acc_empty (leader) collects one arrive per CTA.
+//   acc_full            committed to both CTAs; acc_empty (leader) collects one arrive per epilogue warp of both.
 // No cluster-multicast copies are used anywhere.  Every wait is bounded and abortable.
 #include <cuda.h>
 #include <cudaTypedefs.h>
@@ -23,6 +23,7 @@
 
 #include <mutex>
 
+#include "epilogue.cuh"
 #include "kernels.h"
 #include "ptx.cuh"
 
@@ -30,20 +31,18 @@ namespace nncv_b200 {
 
 namespace {
 
-constexpr int kEpiWarps = 8;
-constexpr int kEpiThreads = kEpiWarps * 32;
-constexpr int kThreads = 64 + kEpiThreads;
-constexpr int kSlabBytes = 128 * 128;
+constexpr int kThreads = 64 + epi::kThreads;
 constexpr int kWGroup = 3;            // taps (one filter row) per weight stage: fewer barrier round trips per MMA
 constexpr int kMaxIn = 4, kMaxW = 12;
+constexpr size_t kBarBytes = 8 * (2 * kMaxIn + 2 * kMaxW + 4 + epi::kWarps * epi::kMaxBufs) + 16;
 
 struct PairParams {
   const uint8_t* wpack;      // packed for N tile max(64, BNP / 2); each CTA of the pair takes BNP / 2 rows
   const float* scale;
   const float* shift;
-  const uint16_t* residual;
   int* error_flag;
   int T, P, Himg, CB, Kout, n_tiles, m_items;   // m_items of mt * 256 slots
+  epi::FastDiv div_p, div_h, div_nt;   // by P, Himg, n_tiles
   int mt;                    // sub-tiles of 256 slots per item: every weight stage feeds mt times the MMAs
   int box_rows, n_boxes;     // a CTA's halo tile (mt * 128 + 2P + 2 rows) arrives as n_boxes TMA boxes
   int in_stages, w_stages;
@@ -53,13 +52,15 @@ struct PairParams {
   // column slices (BNP / tail_parts columns each) that run on different pairs at the same time.
   // Items [0, tail_start) are whole; tail_start is a multiple of the number of pairs.
   int tail_start, tail_parts;
-  int relu, has_res, bf16;
+  int relu, bf16;
+  int has_res;    // tm_res holds a tensor of the output's layout that is added before the activation
+  int epi_bufs;   // staging buffers per epilogue warp (1 .. epi::kMaxBufs)
 };
 
 template <int BNP, int MT>   // columns of the pair's tile (64, 128 or 256), sub-tiles of 256 slots per item
 __global__ void __launch_bounds__(kThreads, 1)
 conv3x3_pair_kernel(const __grid_constant__ CUtensorMap tm_in, const __grid_constant__ CUtensorMap tm_out,
-                    const PairParams p) {
+                    const __grid_constant__ CUtensorMap tm_res, const PairParams p) {
   constexpr int kBNPair = BNP;
   constexpr int kMT = MT;
   constexpr int kWTile = (BNP / 2) * 128;          // this CTA's half of a weight tile
@@ -71,6 +72,7 @@ conv3x3_pair_kernel(const __grid_constant__ CUtensorMap tm_in, const __grid_cons
   constexpr uint32_t kAccCols = kAB * BNP * MT;
   extern __shared__ uint8_t smem_raw[];
   __shared__ int s_abort;
+  __shared__ __align__(16) float4 s_cols[epi::kWarps][32];   // scale / shift of the slab each epilogue warp works on
   const uint32_t raw = ptx::smem_u32(smem_raw);
   const uint32_t base = (raw + 1023u) & ~1023u;
   const int in_stage_bytes = p.box_rows * p.n_boxes * 128;
@@ -78,11 +80,12 @@ conv3x3_pair_kernel(const __grid_constant__ CUtensorMap tm_in, const __grid_cons
   const uint32_t sIn = base;
   const uint32_t sW = sIn + (uint32_t)p.in_stages * in_stage_bytes;
   const uint32_t sStage = sW + (uint32_t)p.w_stages * kWStage;
-  const uint32_t bars = sStage + 2 * kSlabBytes;
+  const uint32_t bars = sStage + (uint32_t)(epi::kWarps * p.epi_bufs) * epi::kBufBytes;
   const uint32_t in_full = bars, in_empty = in_full + 8 * kMaxIn;
   const uint32_t w_full = in_empty + 8 * kMaxIn, w_empty = w_full + 8 * kMaxW;
   const uint32_t acc_full = w_empty + 8 * kMaxW, acc_empty = acc_full + 16;
-  const uint32_t tmem_slot = acc_empty + 16;
+  const uint32_t res_full = acc_empty + 16;
+  const uint32_t tmem_slot = res_full + 8 * epi::kWarps * epi::kMaxBufs;
   {
     // the carve-up above must fit the dynamic shared memory of this launch: refuse to run otherwise
     uint32_t dyn_bytes;
@@ -107,11 +110,13 @@ conv3x3_pair_kernel(const __grid_constant__ CUtensorMap tm_in, const __grid_cons
     }
     for (int i = 0; i < 2; ++i) {
       ptx::mbar_init(acc_full + 8 * i, 1);
-      ptx::mbar_init(acc_empty + 8 * i, 2);   // one arrive per CTA of the pair
+      ptx::mbar_init(acc_empty + 8 * i, 2 * epi::kWarps);   // every epilogue warp of both CTAs
     }
+    for (int i = 0; i < epi::kWarps * epi::kMaxBufs; ++i) ptx::mbar_init(res_full + 8 * i, 1);
     ptx::mbar_fence_init();
     ptx::prefetch_tensormap(&tm_in);
     ptx::prefetch_tensormap(&tm_out);
+    if (p.has_res) ptx::prefetch_tensormap(&tm_res);
   }
   if (warp == 1) {
     ptx::tmem_alloc_pair(tmem_slot, kAccCols);
@@ -141,7 +146,7 @@ conv3x3_pair_kernel(const __grid_constant__ CUtensorMap tm_in, const __grid_cons
       sub = pair & (parts - 1);
     }
     if (p.n_tiles == 1) { m_item = w; n_tile = 0; }
-    else { m_item = w / p.n_tiles; n_tile = w - m_item * p.n_tiles; }
+    else { m_item = (int)epi::div_by((uint32_t)w, p.div_nt); n_tile = w - m_item * p.n_tiles; }
     return w < total_items;
   };
 

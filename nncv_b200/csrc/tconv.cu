@@ -17,8 +17,8 @@
 // Weights are the packed [Kout tile][k-block] images of launch_pack_weights(): resident in shared
 // memory for the whole kernel when they fit, otherwise streamed with the A stage.
 // Roles: warp 0 TMA producer, warp 1 MMA issuer (accumulator double-buffered in TMEM), warps 2-9
-// epilogue (scale/shift, residual, ReLU, 128-byte-row slab in shared memory, 4-D TMA store, which
-// clips ragged tiles and keeps the pads of shared-pad tensors untouched).
+// epilogue (epilogue.cuh: residual rows in by TMA, scale/shift, ReLU, 128-byte rows in a staging buffer of
+// the warp, 4-D TMA store, which clips ragged tiles and keeps the pads of shared-pad tensors untouched).
 // Every wait is bounded and abortable; a timed-out wait sets the device status word.
 #include <cuda.h>
 #include <cudaTypedefs.h>
@@ -28,6 +28,7 @@
 
 #include <mutex>
 
+#include "epilogue.cuh"
 #include "kernels.h"
 #include "ptx.cuh"
 
@@ -35,19 +36,15 @@ namespace nncv_b200 {
 
 namespace {
 
-constexpr int kEpiWarps = 8;
-constexpr int kEpiThreads = kEpiWarps * 32;
-constexpr int kThreads = 64 + kEpiThreads;
+constexpr int kThreads = 64 + epi::kThreads;
 constexpr int kABytes = 128 * 128;
-constexpr int kSlabBytes = 128 * 128;
-constexpr int kOutBufs = 2;     // staging buffers of the epilogue: kOutBufs - 1 stores may be reading shared memory at once
 constexpr int kMaxStages = 8;
+constexpr size_t kBarBytes = 8 * (2 * kMaxStages + 2 + 2 + 1 + epi::kWarps * epi::kMaxBufs) + 16;
 
 struct TcParams {
   const uint8_t* wpack;
   const float* scale;
   const float* shift;
-  const uint8_t* residual;   // same layout / type as out, or null
   const uint8_t* wpack2;     // DUAL: packed 1x1 weights of the fused downsample branch
   const float* scale2;
   const float* shift2;
@@ -59,8 +56,11 @@ struct TcParams {
   int out_pitch, out_rows;   // output layout: slots per row, rows per image
   int tw, th, tn;            // M tile shape
   int tiles_x, tiles_y, tiles_n, n_tiles, m_items;
+  epi::FastDiv div_tx, div_ty, div_nt;   // by tiles_x, tiles_y, n_tiles
   int stages;                // A (+ streamed weight) ring depth
   int relu, bf16, out_f32;
+  int residual;   // tm_res holds a tensor of the output's layout and type, added before the activation
+  int epi_bufs;   // staging buffers per epilogue warp (1 .. epi::kMaxBufs)
   int act;   // 0, or kActHardSwish / kActSilu applied after the residual add (16-bit outputs)
 };
 
@@ -83,7 +83,8 @@ struct TcParams {
 template <int BN, bool RESIDENT, bool DUAL, bool PAIR, bool BROW>
 __global__ void __launch_bounds__(kThreads, 1)
 tconv_kernel(const __grid_constant__ CUtensorMap tm_in, const __grid_constant__ CUtensorMap tm_out,
-             const __grid_constant__ CUtensorMap tm_out2, const __grid_constant__ CUtensorMap tm_b, const TcParams p) {
+             const __grid_constant__ CUtensorMap tm_out2, const __grid_constant__ CUtensorMap tm_b,
+             const __grid_constant__ CUtensorMap tm_res, const TcParams p) {
   static_assert(!PAIR || !RESIDENT, "the pair kernel streams its weights");
   static_assert(!BROW || (!RESIDENT && !DUAL && !PAIR), "a row-major B is streamed by one CTA");
   constexpr int WTILE = (PAIR ? BN / 2 : BN) * 128;   // this CTA's part of a weight tile
@@ -93,7 +94,7 @@ tconv_kernel(const __grid_constant__ CUtensorMap tm_in, const __grid_constant__ 
 
   extern __shared__ uint8_t smem_raw[];
   __shared__ int s_abort;
-  __shared__ __align__(16) float s_scale[256], s_shift[256];   // per-channel scale / shift of the N tile in work (single-output kernels)
+  __shared__ __align__(16) float4 s_cols[epi::kWarps][32];   // scale / shift of the slab each epilogue warp works on
   const uint32_t raw = ptx::smem_u32(smem_raw);
   const uint32_t base = (raw + 1023u) & ~1023u;
   const int KB = p.taps * p.CB;
@@ -101,11 +102,12 @@ tconv_kernel(const __grid_constant__ CUtensorMap tm_in, const __grid_constant__ 
   const uint32_t sRing = base;
   const uint32_t sW = sRing + (uint32_t)p.stages * stage_bytes;       // resident weights
   const uint32_t sStage = sW + (RESIDENT ? (uint32_t)(KB + (DUAL ? p.CB : 0)) * WTILE : 0u);   // resident: main tiles, then the branch's
-  const uint32_t bars = sStage + kOutBufs * kSlabBytes;
+  const uint32_t bars = sStage + (uint32_t)(epi::kWarps * p.epi_bufs) * epi::kBufBytes;
   const uint32_t full = bars, empty = bars + 8 * kMaxStages;
   const uint32_t acc_full = empty + 8 * kMaxStages, acc_empty = acc_full + 16;
   const uint32_t w_full = acc_empty + 16;
-  const uint32_t tmem_slot = w_full + 8;
+  const uint32_t res_full = w_full + 8;
+  const uint32_t tmem_slot = res_full + 8 * epi::kWarps * epi::kMaxBufs;
   {
     // the carve-up above must fit the dynamic shared memory of this launch: refuse to run otherwise
     uint32_t dyn_bytes;
@@ -126,14 +128,16 @@ tconv_kernel(const __grid_constant__ CUtensorMap tm_in, const __grid_constant__ 
     }
     for (int i = 0; i < 2; ++i) {
       ptx::mbar_init(acc_full + 8 * i, 1);
-      ptx::mbar_init(acc_empty + 8 * i, PAIR ? 2 : kEpiThreads);   // pair: one arrival per CTA
+      ptx::mbar_init(acc_empty + 8 * i, PAIR ? 2 * epi::kWarps : epi::kWarps);   // one arrival per epilogue warp (of both CTAs)
     }
     ptx::mbar_init(w_full, 1);
+    for (int i = 0; i < epi::kWarps * epi::kMaxBufs; ++i) ptx::mbar_init(res_full + 8 * i, 1);
     ptx::mbar_fence_init();
     ptx::prefetch_tensormap(&tm_in);
     ptx::prefetch_tensormap(&tm_out);
     if (DUAL) ptx::prefetch_tensormap(&tm_out2);
     if (BROW) ptx::prefetch_tensormap(&tm_b);
+    if (p.residual) ptx::prefetch_tensormap(&tm_res);
   }
   if (warp == 1) {
     if (PAIR) {
@@ -170,14 +174,15 @@ tconv_kernel(const __grid_constant__ CUtensorMap tm_in, const __grid_constant__ 
       m_item = w;
       n_tile = (int)blockIdx.y;
     } else {
-      m_item = w / p.n_tiles;
+      m_item = (int)epi::div_by((uint32_t)w, p.div_nt);
       n_tile = w - m_item * p.n_tiles;
     }
     if (PAIR) m_item = 2 * m_item + (int)rank;
-    const int tx = m_item % p.tiles_x;
-    const int t2 = m_item / p.tiles_x;
-    const int ty = t2 % p.tiles_y;
-    n0 = (t2 / p.tiles_y) * p.tn;
+    const int t2 = (int)epi::div_by((uint32_t)m_item, p.div_tx);
+    const int tx = m_item - t2 * p.tiles_x;
+    const int t3 = (int)epi::div_by((uint32_t)t2, p.div_ty);
+    const int ty = t2 - t3 * p.tiles_y;
+    n0 = t3 * p.tn;
     oy0 = ty * p.th;
     ox0 = tx * p.tw;
     return true;
@@ -315,230 +320,143 @@ tconv_kernel(const __grid_constant__ CUtensorMap tm_in, const __grid_constant__ 
     }
   } else {
     // ------------------------------------------------------------------ epilogue --------
-    const int quad = warp & 3;
-    const int half = (warp - 2) >> 2;
-    const int row = quad * 32 + lane;
-    const bool elected = threadIdx.x == 64;
-    const uint32_t sw = (uint32_t)(row & 7);
+    // Eight independent warps (epilogue.cuh).  Slabs of an item are numbered output-major, then by column; warp group
+    // `half` takes every second slab of the running count, so both groups drain one accumulator together when it has
+    // several slabs and alternate between the accumulators when it has one.
+    const int ew = warp - 2, quad = warp & 3, half = ew >> 2;
+    const uint32_t sw = (uint32_t)(lane & 7);
+    const int nb = p.epi_bufs;
+    const uint32_t my_stage = sStage + (uint32_t)(ew * nb) * epi::kBufBytes;
+    const uint32_t my_res = res_full + (uint32_t)(ew * epi::kMaxBufs) * 8u;
+    const uint32_t tab = ptx::smem_u32(&s_cols[ew][0]);
     const int slab_cols = p.out_f32 ? 32 : 64;      // 128-byte rows either way
-    const int slabs = BN / slab_cols;
-    const int esz = p.out_f32 ? 4 : 2;
-    // row of the tile -> pixel inside the tile
-    const int tj = row % p.tw, ti = (row / p.tw) % p.th, tnn = row / (p.tw * p.th);
-    uint32_t acc_cnt = 0;
-    int jglob = 0;   // slab counter for the two staging buffers
-    int cur_ntile = -1;
+    // slabs of an output and of an item, as powers of two
+    const int slabs_log = (BN == 64 ? 0 : (BN == 128 ? 1 : 2)) + (p.out_f32 ? 1 : 0);
+    const int spi_log = slabs_log + (DUAL ? 1 : 0);
+    const int spi = 1 << spi_log, slabs = 1 << slabs_log;
+    const int mode = epi::mode_of(p.bf16 != 0, p.residual != 0, p.relu != 0, p.act), mode2 = epi::mode_of(p.bf16 != 0, false, false, 0);
+    // the 32 pixels of this warp's rows form a box inside the tile
+    const int qx = (quad * 32) % p.tw, qy = (quad * 32 / p.tw) % p.th, qn = quad * 32 / (p.tw * p.th);
+    const bool has_res = p.residual != 0;
+    // where a slab lies; the item is looked up only when it changes
+    struct Pos { int i, n0, oy0, ox0, n_tile; bool ok; };
+    auto seek = [&](Pos& q, int i) {
+      if (q.i != i) {
+        q.i = i;
+        q.ok = item_of(i, q.n0, q.oy0, q.ox0, q.n_tile);
+      }
+      return q.ok;
+    };
+    auto live_at = [&](const Pos& q, int ncol) {
+      return ncol < p.Kout && q.ox0 + qx < p.OW && q.oy0 + qy < p.OH && q.n0 + qn < p.NB;
+    };
+    Pos cur{-1, 0, 0, 0, 0, false}, ahead{-1, 0, 0, 0, 0, false};
+    uint32_t phase = 0, inflight = 0;   // per staging buffer: parity of its next residual, one on its way
+    int ahead_j = half, ahead_b = 0;
+    // residual rows of the next slab in line -> its staging buffer
+    auto fetch_res = [&]() {
+      const int i = ahead_j >> spi_log, sl = ahead_j & (spi - 1);
+      if (seek(ahead, i)) {
+        const int ncol = ahead.n_tile * BN + sl * slab_cols;
+        if (live_at(ahead, ncol)) {
+          inflight |= 1u << ahead_b;
+          if (lane == 0) {
+            ptx::mbar_arrive_expect_tx(my_res + 8 * ahead_b, epi::kBufBytes);
+            ptx::tma_load_4d(my_stage + (uint32_t)ahead_b * epi::kBufBytes, &tm_res, ncol, ahead.ox0 + qx + p.out_off,
+                             ahead.oy0 + qy + p.out_off, ahead.n0 + qn, my_res + 8 * ahead_b);
+          }
+        }
+      }
+      ahead_j += 2;
+      if (++ahead_b == nb) ahead_b = 0;
+    };
+    auto cols_of = [&](int i, int rem, Pos& q) {
+      if (!seek(q, i)) return epi::ColParams{1.0f, 1.0f, 0.0f, 0.0f};
+      const int oi = DUAL ? rem >> slabs_log : 0, sl = DUAL ? rem & (slabs - 1) : rem;
+      return epi::fetch_cols(oi ? p.scale2 : p.scale, oi ? p.shift2 : p.shift, q.n_tile * BN + sl * slab_cols, p.Kout, lane);
+    };
+    Pos colpos{-1, 0, 0, 0, 0, false};
+    int j = half, b = 0;   // running slab count of this warp (+= 2), staging buffer
+    epi::ColParams cols = cols_of(j >> spi_log, j & (spi - 1), colpos);
+    if (has_res)
+      for (int k = 0; k + 1 < nb; ++k) fetch_res();
     bool okw = true;
     for (int i = 0; okw; ++i) {
-      int n0, oy0, ox0, n_tile;
-      if (!item_of(i, n0, oy0, ox0, n_tile)) break;
-      const uint32_t ab = acc_cnt & 1u;
-      const int nimg = n0 + tnn, oy = oy0 + ti, ox = ox0 + tj;
-      const bool valid = nimg < p.NB && oy < p.OH && ox < p.OW;
-      const size_t pix = ((size_t)nimg * p.out_rows + oy + p.out_off) * p.out_pitch + ox + p.out_off;
-      if (p.residual != nullptr) {
-        // pull the residual rows of the NEXT item from HBM into L2 while this item's accumulator is awaited
-        // and drained, so that the epilogue's per-row loads of the next item do not start from DRAM
-        int n0n, oy0n, ox0n, n_tile_n;
-        if (item_of(i + 1, n0n, oy0n, ox0n, n_tile_n)) {
-          const int nin = n0n + tnn, oyn = oy0n + ti, oxn = ox0n + tj;
-          if (nin < p.NB && oyn < p.OH && oxn < p.OW) {
-            const size_t pixn = ((size_t)nin * p.out_rows + oyn + p.out_off) * p.out_pitch + oxn + p.out_off;
-            const int cfirst = n_tile_n * BN + (p.out_f32 ? 0 : half * 32);
-            for (int sl = 0; sl < slabs; ++sl) {
-              const int col = cfirst + sl * slab_cols;
-              if (col < p.Kout)
-                asm volatile("prefetch.global.L2 [%0];" ::"l"(p.residual + (pixn * (size_t)p.Kout + col) * 2));
-            }
-          }
-        }
-      }
-      if (!DUAL && n_tile != cur_ntile) {
-        // scale / shift of this N tile into shared memory: the slabs read them as broadcast vectors instead of sixteen
-        // global loads per thread and slab.  Every thread has passed the last slab's barrier of the previous item, so
-        // nobody still reads the old values; the barrier below publishes the new ones.
-        for (int c = (int)threadIdx.x - 64; c < BN; c += kEpiThreads) {
-          const int col = n_tile * BN + c;
-          s_scale[c] = (p.scale && col < p.Kout) ? __ldg(p.scale + col) : 1.0f;
-          s_shift[c] = (p.shift && col < p.Kout) ? __ldg(p.shift + col) : 0.0f;
-        }
-        cur_ntile = n_tile;
-      }
-      const bool got = PAIR ? ptx::mbar_wait_cluster_abortable(acc_full + 8 * ab, (acc_cnt >> 1) & 1u, abort_flag)
-                            : ptx::mbar_wait_abortable(acc_full + 8 * ab, (acc_cnt >> 1) & 1u, abort_flag);
-      if (!ptx::named_bar_and(3, kEpiThreads, got)) { okw = false; break; }
+      if (!seek(cur, i)) break;
+      const uint32_t ab = (uint32_t)i & 1u;
+      okw = PAIR ? ptx::mbar_wait_cluster_abortable(acc_full + 8 * ab, ((uint32_t)i >> 1) & 1u, abort_flag)
+                 : ptx::mbar_wait_abortable(acc_full + 8 * ab, ((uint32_t)i >> 1) & 1u, abort_flag);
+      okw = __all_sync(0xffffffffu, okw);
+      if (!okw) break;
       ptx::tc_fence_after();
-      uint32_t res_next[2][8];   // residual of the next slab of this item, in flight one slab ahead
-      bool have_next = false;
-      for (int oi = 0; oi < (DUAL ? 2 : 1); ++oi)
-      for (int sl = 0; sl < slabs; ++sl, ++jglob) {
-        const float* scale_o = oi ? p.scale2 : p.scale;
-        const float* shift_o = oi ? p.shift2 : p.shift;
-        const uint8_t* residual_o = oi ? nullptr : p.residual;
-        const bool relu_o = oi ? false : p.relu != 0;
-        const uint32_t sb = (uint32_t)jglob % (uint32_t)kOutBufs;
-        const int ncol = n_tile * BN + sl * slab_cols;     // first column of the slab
-        // this warp's 32 accumulator columns inside the slab: 16-bit output -> columns
-        // [half*32, +32) of a 64-column slab; fp32 output -> both halves share a 32-column
-        // slab, so each warp takes 16 columns twice... keep it simple: for fp32 only half 0 works
-        // on columns [0,32) and half 1 idles through the barriers.
-        const bool active = p.out_f32 ? (half == 0) : true;
-        const int c0 = p.out_f32 ? 0 : half * 32;
-        const int n_first = ncol + c0;
-        uint32_t acc[32];
+      auto hand_back = [&]() {   // this warp has read its part of the accumulator
+        ptx::tc_fence_before();
         __syncwarp();
-        ptx::tmem_ld_32x32(tmem_base + ((uint32_t)(quad * 32) << 16) + ab * ACC_W + (uint32_t)(oi * BN + sl * slab_cols + c0), acc);
-        uint32_t res[2][8];
-        // 32-byte loads need a pixel pitch that is a multiple of 32 bytes and a full group of 32 columns; other
-        // widths (Kout a multiple of 8: column pairs never straddle the end) take guarded 4-byte loads
-        const bool use_res = residual_o != nullptr && valid && active && n_first < p.Kout;
-        if (use_res) {
-          const uint8_t* rp = residual_o + (pix * (size_t)p.Kout + n_first) * 2;
-          if (have_next) {   // fetched while the previous slab was converted and stored
-#pragma unroll
-            for (int e = 0; e < 8; ++e) { res[0][e] = res_next[0][e]; res[1][e] = res_next[1][e]; }
-          } else if (n_first + 32 <= p.Kout && (p.Kout & 15) == 0) {
-            ptx::ldg_256(rp, res[0]);
-            ptx::ldg_256(rp + 32, res[1]);
-          } else {
-#pragma unroll
-            for (int e = 0; e < 16; ++e)
-              res[e >> 3][e & 7] = (n_first + 2 * e < p.Kout) ? __ldg(reinterpret_cast<const uint32_t*>(rp + 4 * e)) : 0u;
-          }
-          // the next slab's residual of this row goes into flight now (the same item: the row stays, the columns move on)
-          have_next = false;
-          const int n_next = n_first + slab_cols;
-          if (sl + 1 < slabs && n_next + 32 <= p.Kout && (p.Kout & 15) == 0) {
-            ptx::ldg_256(rp + slab_cols * 2, res_next[0]);
-            ptx::ldg_256(rp + slab_cols * 2 + 32, res_next[1]);
-            have_next = true;
+        if (lane == 0) {
+          if (!PAIR || rank == 0) ptx::mbar_arrive(acc_empty + 8 * ab);
+          else ptx::mbar_arrive_remote(ptx::map_to_cta(acc_empty, 0) + 8 * ab);
+        }
+      };
+      const int end_j = (i + 1) << spi_log;
+      if (j >= end_j) hand_back();   // no slab of this item is this warp's
+      for (; j < end_j; j += 2) {
+        const int rem = j & (spi - 1);
+        const int oi = DUAL ? rem >> slabs_log : 0, sl = DUAL ? rem & (slabs - 1) : rem;
+        const int ncol = cur.n_tile * BN + sl * slab_cols;
+        const bool live = live_at(cur, ncol);
+        const uint32_t taddr = tmem_base + ((uint32_t)(quad * 32) << 16) + ab * ACC_W + (uint32_t)(oi * BN + sl * slab_cols);
+        uint32_t acc[64];
+        if (p.out_f32) ptx::tmem_ld_32x32(taddr, reinterpret_cast<uint32_t (&)[32]>(acc));
+        else ptx::tmem_ld_32x64(taddr, acc);
+        epi::put_cols(tab, cols, lane);
+        if (has_res) {
+          // the buffer the next residual goes to was stored from one slab ago
+          if (lane == 0) ptx::bulk_wait_read<0>();
+          __syncwarp();
+          fetch_res();
+        } else {
+          if (lane == 0) {
+            if (nb == 1) ptx::bulk_wait_read<0>();
+            else ptx::bulk_wait_read<1>();
           }
         }
-        __syncwarp();
         ptx::tmem_ld_wait();
-        const bool last_slab = sl == slabs - 1 && oi == (DUAL ? 1 : 0);
-        if (last_slab) {
-          ptx::tc_fence_before();
-          if (!PAIR) ptx::mbar_arrive(acc_empty + 8 * ab);   // pair: one arrival per CTA, after the barrier below
-        }
-        if (active) {
-          float v[32];
-          if constexpr (!DUAL) {
-#pragma unroll
-            for (int e = 0; e < 32; e += 4) {
-              const float4 sc = *reinterpret_cast<const float4*>(&s_scale[sl * slab_cols + c0 + e]);
-              const float4 sh = *reinterpret_cast<const float4*>(&s_shift[sl * slab_cols + c0 + e]);
-              v[e] = fmaf(__uint_as_float(acc[e]), sc.x, sh.x);
-              v[e + 1] = fmaf(__uint_as_float(acc[e + 1]), sc.y, sh.y);
-              v[e + 2] = fmaf(__uint_as_float(acc[e + 2]), sc.z, sh.z);
-              v[e + 3] = fmaf(__uint_as_float(acc[e + 3]), sc.w, sh.w);
-            }
-          } else if (n_first + 32 <= p.Kout) {
-#pragma unroll
-            for (int e = 0; e < 32; e += 4) {
-              float4 sc = make_float4(1.f, 1.f, 1.f, 1.f), sh = make_float4(0.f, 0.f, 0.f, 0.f);
-              if (scale_o) sc = __ldg(reinterpret_cast<const float4*>(scale_o + n_first + e));
-              if (shift_o) sh = __ldg(reinterpret_cast<const float4*>(shift_o + n_first + e));
-              v[e] = fmaf(__uint_as_float(acc[e]), sc.x, sh.x);
-              v[e + 1] = fmaf(__uint_as_float(acc[e + 1]), sc.y, sh.y);
-              v[e + 2] = fmaf(__uint_as_float(acc[e + 2]), sc.z, sh.z);
-              v[e + 3] = fmaf(__uint_as_float(acc[e + 3]), sc.w, sh.w);
-            }
-          } else {
-#pragma unroll
-            for (int e = 0; e < 32; ++e) {
-              const int n = n_first + e;
-              float x = __uint_as_float(acc[e]);
-              if (n < p.Kout) {
-                if (scale_o) x *= __ldg(scale_o + n);
-                if (shift_o) x += __ldg(shift_o + n);
-              }
-              v[e] = x;
-            }
+        __syncwarp();
+        if (j + 2 >= end_j) hand_back();
+        cols = cols_of((j + 2) >> spi_log, (j + 2) & (spi - 1), colpos);
+        if (live) {
+          const uint32_t srow = my_stage + (uint32_t)b * epi::kBufBytes + (uint32_t)lane * 128u;
+          if (has_res) {
+            okw = ptx::mbar_wait_abortable(my_res + 8 * b, (phase >> b) & 1u, abort_flag);
+            okw = __all_sync(0xffffffffu, okw);
+            if (!okw) break;
+            phase ^= 1u << b;
+            inflight &= ~(1u << b);
           }
-          if (use_res) {
-#pragma unroll
-            for (int e = 0; e < 16; ++e) {
-              const uint32_t w = res[e >> 3][e & 7];
-              float2 f;
-              if (p.bf16) f = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&w));
-              else f = __half22float2(*reinterpret_cast<const __half2*>(&w));
-              v[2 * e] += f.x;
-              v[2 * e + 1] += f.y;
-            }
-          }
-          if (p.act != 0 && oi == 0) {
-            // hard-swish x * min(max(x + 3, 0), 6) / 6 or SiLU x / (1 + exp(-x)); a NaN stays NaN through the product with x
-            if (p.act == kActHardSwish) {
-#pragma unroll
-              for (int e = 0; e < 32; ++e) v[e] *= fminf(fmaxf(fmaf(v[e], 0.16666667f, 0.5f), 0.0f), 1.0f);
-            } else {
-#pragma unroll
-              for (int e = 0; e < 32; ++e) v[e] *= __fdividef(1.0f, __expf(-v[e]) + 1.0f);
-            }
-          }
-          const uint32_t srow = sStage + sb * kSlabBytes + (uint32_t)row * 128u;
           if (p.out_f32) {
-#pragma unroll
-            for (int c4 = 0; c4 < 8; ++c4) {
-              float o[4];
-#pragma unroll
-              for (int h = 0; h < 4; ++h) {
-                const float a = v[c4 * 4 + h];
-                o[h] = relu_o ? (!(a <= 0.0f) ? a : 0.0f) : a;
-              }
-              asm volatile("st.shared.v4.f32 [%0], {%1,%2,%3,%4};" ::"r"(srow + (((uint32_t)c4 ^ sw) << 4)), "f"(o[0]),
-                           "f"(o[1]), "f"(o[2]), "f"(o[3])
-                           : "memory");
-            }
+            if (p.relu) epi::row32_f32<true>(reinterpret_cast<const uint32_t (&)[32]>(acc), tab, srow, sw);
+            else epi::row32_f32<false>(reinterpret_cast<const uint32_t (&)[32]>(acc), tab, srow, sw);
           } else {
-#pragma unroll
-            for (int c4 = 0; c4 < 4; ++c4) {
-              uint32_t o[4];
-#pragma unroll
-              for (int h = 0; h < 4; ++h) {
-                const float a = v[c4 * 8 + h * 2], b = v[c4 * 8 + h * 2 + 1];
-                // conversion and ReLU in one instruction (cvt.rn.relu: negative -> +0, NaN stays NaN)
-                if (p.bf16) {
-                  if (relu_o) {
-                    o[h] = ptx::pack_bf162_relu(a, b);
-                  } else {
-                    const __nv_bfloat162 x = __floats2bfloat162_rn(a, b);
-                    o[h] = *reinterpret_cast<const uint32_t*>(&x);
-                  }
-                } else {
-                  o[h] = relu_o ? ptx::pack_half2_sat_relu(a, b) : ptx::pack_half2_sat(a, b);
-                }
-              }
-              const uint32_t chunk = (uint32_t)(half * 4 + c4);
-              asm volatile("st.shared.v4.u32 [%0], {%1,%2,%3,%4};" ::"r"(srow + ((chunk ^ sw) << 4)), "r"(o[0]), "r"(o[1]),
-                           "r"(o[2]), "r"(o[3])
-                           : "memory");
-            }
+            epi::row64_by_mode<DUAL ? 1 : 3>(oi ? mode2 : mode, acc, tab, srow, sw);
+          }
+          ptx::fence_proxy_async_smem();
+          __syncwarp();
+          if (lane == 0) {
+            ptx::tma_store_4d((DUAL && oi) ? &tm_out2 : &tm_out, ncol, cur.ox0 + qx + p.out_off, cur.oy0 + qy + p.out_off, cur.n0 + qn,
+                              my_stage + (uint32_t)b * epi::kBufBytes);
+            ptx::bulk_commit();
           }
         }
-        ptx::fence_proxy_async_smem();
-        // One barrier per slab.  Before it the storing thread makes sure the previous slab's store has finished
-        // reading its staging buffer: past the barrier every thread may fill that buffer for the next slab while
-        // this slab's store (issued right after the barrier) reads the other one.  Nobody can run two slabs ahead,
-        // because the next barrier needs the storing thread too.
-        if (elected) ptx::bulk_wait_read<kOutBufs - 2>();
-        ptx::named_bar_sync(1, kEpiThreads);
-        if (elected) {
-          if (PAIR && last_slab) {   // every thread of this CTA has read the accumulator: tell the leader
-            if (rank == 0) ptx::mbar_arrive(acc_empty + 8 * ab);
-            else ptx::mbar_arrive_remote(ptx::map_to_cta(acc_empty, 0) + 8 * ab);
-          }
-          if (ncol < p.Kout)
-            ptx::tma_store_4d((DUAL && oi) ? &tm_out2 : &tm_out, ncol, ox0 + p.out_off, oy0 + p.out_off, n0, sStage + sb * kSlabBytes);
-          ptx::bulk_commit();
-        }
+        __syncwarp();
+        if (++b == nb) b = 0;
       }
-      ++acc_cnt;
-      (void)esz;
     }
-    if (elected) ptx::bulk_wait<0>();
-    if (!okw && p.error_flag) atomicCAS(p.error_flag, 0, (int)kErrWaitEpilogue);
+    if (!okw) {
+      if (lane == 0 && p.error_flag) atomicCAS(p.error_flag, 0, (int)kErrWaitEpilogue);
+      for (int k = 0; k < nb; ++k)   // residual rows still on their way land before the block ends
+        if ((inflight >> k) & 1u) ptx::mbar_wait_limit(my_res + 8 * k, (phase >> k) & 1u, 1LL << 24);
+    }
+    if (lane == 0) ptx::bulk_wait<0>();
   }
 
   ptx::tc_fence_before();
@@ -579,7 +497,7 @@ bool make_map4(CUtensorMap* m, const void* ptr, CUtensorMapDataType dt, int esz,
          CUDA_SUCCESS;
 }
 
-constexpr size_t kSmemLimit = 225 * 1024;   // dynamic part: the kernel also holds 2 KB of static shared memory (scale / shift of an N tile)
+constexpr size_t kSmemLimit = 222 * 1024;   // dynamic part: the kernel also holds 4 KB of static shared memory (scale / shift of the slabs in work)
 
 // 2-D map over a row-major [K, N] 16-bit matrix, box 64 columns x 64 rows, 128-byte swizzle, zero fill.
 bool make_map_b(CUtensorMap* m, const void* ptr, CUtensorMapDataType dt, long long K, long long N) {
@@ -597,9 +515,10 @@ template <int BN, bool RESIDENT, bool DUAL = false, bool PAIR = false, bool BROW
 cudaError_t launch_cfg(const TconvArgs& a, TcParams p, cudaStream_t stream) {
   const size_t wtile = (size_t)(PAIR ? BN / 2 : BN) * 128;
   const int KB = p.taps * p.CB;
-  const size_t fixed = 1024 + kOutBufs * kSlabBytes + 512;
   const size_t stage = RESIDENT ? kABytes : kABytes + wtile;
   const size_t wres = RESIDENT ? (size_t)(KB + (DUAL ? p.CB : 0)) * wtile : 0;
+  p.epi_bufs = epi::pick_bufs(p.residual != 0, kSmemLimit - 1024 - kBarBytes, wres + 3 * stage, wres + 2 * stage);
+  const size_t fixed = 1024 + (size_t)(epi::kWarps * p.epi_bufs) * epi::kBufBytes + kBarBytes;
   if (fixed + wres + 2 * stage > kSmemLimit) return cudaErrorInvalidConfiguration;
   size_t st = (kSmemLimit - fixed - wres) / stage;
   if (st > kMaxStages) st = kMaxStages;
@@ -613,11 +532,16 @@ cudaError_t launch_cfg(const TconvArgs& a, TcParams p, cudaStream_t stream) {
                  p.stride, p.stride))
     return cudaErrorInvalidValue;
   const bool f32 = p.out_f32 != 0;
+  // an epilogue warp stores its own 32 pixels: a box of the tile (all three extents are powers of two)
+  const int qw = p.tw < 32 ? p.tw : 32, qh = p.th < 32 / qw ? p.th : 32 / qw, qn = 32 / (qw * qh);
   if (!make_map4(&tm_out, a.out, f32 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : dt, f32 ? 4 : 2, a.Kout, ol.pitch, ol.img_rows,
-                 a.N, f32 ? 32 : 64, p.tw, p.th, p.tn, 1, 1))
+                 a.N, f32 ? 32 : 64, qw, qh, qn, 1, 1))
     return cudaErrorInvalidValue;
   CUtensorMap tm_out2 = tm_out;
-  if (DUAL && !make_map4(&tm_out2, a.out2, dt, 2, a.Kout, ol.pitch, ol.img_rows, a.N, 64, p.tw, p.th, p.tn, 1, 1))
+  if (DUAL && !make_map4(&tm_out2, a.out2, dt, 2, a.Kout, ol.pitch, ol.img_rows, a.N, 64, qw, qh, qn, 1, 1))
+    return cudaErrorInvalidValue;
+  CUtensorMap tm_res = tm_out;
+  if (p.residual && !make_map4(&tm_res, a.residual, dt, 2, a.Kout, ol.pitch, ol.img_rows, a.N, 64, qw, qh, qn, 1, 1))
     return cudaErrorInvalidValue;
   CUtensorMap tm_b = tm_out;
   if (BROW && !make_map_b(&tm_b, a.b_rowmajor, dt, a.b_rows, a.Kout)) return cudaErrorInvalidValue;
@@ -649,12 +573,12 @@ cudaError_t launch_cfg(const TconvArgs& a, TcParams p, cudaStream_t stream) {
     attr[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 2;
-    return cudaLaunchKernelEx(&cfg, kern, tm_in, tm_out, tm_out2, tm_b, p);
+    return cudaLaunchKernelEx(&cfg, kern, tm_in, tm_out, tm_out2, tm_b, tm_res, p);
   } else {
     const long long items = (long long)p.m_items * p.n_tiles;
     grid = dim3((unsigned)(items < sms ? items : sms), 1);
   }
-  return launch_pdl(kern, grid, dim3(kThreads), smem, stream, tm_in, tm_out, tm_out2, tm_b, p);
+  return launch_pdl(kern, grid, dim3(kThreads), smem, stream, tm_in, tm_out, tm_out2, tm_b, tm_res, p);
 }
 
 }  // namespace
@@ -706,7 +630,8 @@ cudaError_t launch_tconv(const TconvArgs& a, cudaStream_t stream) {
     return cudaErrorMisalignedAddress;
   TcParams p;
   p.wpack = static_cast<const uint8_t*>(a.wpack);
-  p.scale = a.scale; p.shift = a.shift; p.residual = static_cast<const uint8_t*>(a.residual);
+  p.scale = a.scale; p.shift = a.shift; p.residual = a.residual != nullptr;
+  p.epi_bufs = 1;
   p.wpack2 = static_cast<const uint8_t*>(a.wpack2); p.scale2 = a.scale2; p.shift2 = a.shift2;
   p.error_flag = a.error_flag;
   p.Kout = a.Kout; p.CB = (a.C + 63) / 64; p.taps = a.R * a.S; p.S = a.S; p.stride = a.stride; p.pad = a.pad;
@@ -722,6 +647,8 @@ cudaError_t launch_tconv(const TconvArgs& a, cudaStream_t stream) {
   const long long mi = (long long)p.tiles_x * p.tiles_y * p.tiles_n;
   if (mi <= 0 || mi * p.n_tiles > 0x7fffffffLL) return cudaErrorInvalidValue;
   p.m_items = (int)mi;
+  p.div_tx = epi::fast_div((uint32_t)p.tiles_x); p.div_ty = epi::fast_div((uint32_t)p.tiles_y);
+  p.div_nt = epi::fast_div((uint32_t)p.n_tiles);
   p.relu = a.relu; p.bf16 = a.ab == kBF16; p.out_f32 = a.out_dtype == kF32;
   p.act = a.act;
   p.stages = 0;
@@ -762,7 +689,7 @@ cudaError_t launch_tconv(const TconvArgs& a, cudaStream_t stream) {
 // N tile and residency: keep all weights of one Kout tile in shared memory when they fit beside
 // four A stages; otherwise stream them with the widest tile the grid can still fill.
 void tconv_pick(long long m_items, int C, int Kout, int taps, int* bn, int* resident) {
-  const size_t budget = kSmemLimit - (1024 + kOutBufs * kSlabBytes + 512) - 4 * (size_t)kABytes;
+  const size_t budget = kSmemLimit - (1024 + (size_t)epi::kWarps * epi::kBufBytes + kBarBytes) - 4 * (size_t)kABytes;
   const size_t kb = (size_t)taps * ((C + 63) / 64);
   for (int b : {128, 64}) {
     if (Kout >= b && kb * b * 128 <= budget) {
