@@ -107,7 +107,7 @@ conv3x3_kernel(const __grid_constant__ CUtensorMap tm_in, const __grid_constant_
     }
   }
 
-  const int warp = threadIdx.x >> 5;
+  const int warp = ptx::warp_uniform((int)threadIdx.x >> 5);
   const int lane = threadIdx.x & 31;
 
   if (threadIdx.x == 0) {
@@ -137,11 +137,7 @@ conv3x3_kernel(const __grid_constant__ CUtensorMap tm_in, const __grid_constant_
   ptx::tc_fence_before();
   __syncthreads();
   ptx::tc_fence_after();
-  const uint32_t tmem_base = *reinterpret_cast<volatile uint32_t*>(smem_raw + (tmem_slot - raw));
-  // The prologue above touched nothing the previous kernel of the stream writes; everything
-  // below may, so wait for that kernel here and let the next one start its own prologue.
-  ptx::grid_dependency_wait();
-  ptx::grid_launch_dependents();
+  const uint32_t tmem_base = (uint32_t)ptx::warp_uniform(*reinterpret_cast<volatile int*>(smem_raw + (tmem_slot - raw)));
   volatile int* abort_flag = &s_abort;
 
   // Work items of this CTA.  Resident weights pin the CTA to one Kout tile (blockIdx.y) and it
@@ -160,15 +156,34 @@ conv3x3_kernel(const __grid_constant__ CUtensorMap tm_in, const __grid_constant_
     return w < total_items;
   };
 
+  // Packed weights never change, so their copies start before the previous kernel of the stream has finished.
+  auto weight_tile = [&](int n_tile, int cb, int tap) { return p.wpack + ((size_t)n_tile * kb_total + (size_t)tap * p.CB + cb) * WTILE; };
+  uint32_t early = 0;   // stages of the weight ring already on their way
+  if (warp == 0 && lane == 0) {
+    if (RESIDENT) {
+      const uint8_t* src = p.wpack + (size_t)blockIdx.y * kb_total * WTILE;
+      ptx::mbar_arrive_expect_tx(w_full, (uint32_t)kb_total * WTILE);
+      for (int i = 0; i < kb_total; ++i)
+        ptx::bulk_g2s(sW + (uint32_t)i * WTILE, src + (size_t)i * WTILE, WTILE, w_full);
+    } else {
+      for (int i = 0; early < (uint32_t)p.w_stages; ++i) {
+        int m_item, n_tile;
+        if (!item_of(i, m_item, n_tile)) break;
+        for (int cb = 0; cb < p.CB && early < (uint32_t)p.w_stages; ++cb)
+          for (int tap = 0; tap < 9 && early < (uint32_t)p.w_stages; ++tap, ++early) {
+            ptx::mbar_arrive_expect_tx(w_full + 8 * early, WTILE);
+            ptx::bulk_g2s(sW + early * WTILE, weight_tile(n_tile, cb, tap), WTILE, w_full + 8 * early);
+          }
+      }
+    }
+  }
+  // The rest reads what the previous kernel wrote, or writes what it may still be reading.
+  ptx::grid_dependency_wait();
+  ptx::grid_launch_dependents();
+
   if (warp == 0) {
     // ------------------------------------------------------------------ TMA producer ----
     if (lane == 0) {
-      if (RESIDENT) {
-        const uint8_t* src = p.wpack + (size_t)blockIdx.y * kb_total * WTILE;
-        ptx::mbar_arrive_expect_tx(w_full, (uint32_t)kb_total * WTILE);
-        for (int i = 0; i < kb_total; ++i)
-          ptx::bulk_g2s(sW + (uint32_t)i * WTILE, src + (size_t)i * WTILE, WTILE, w_full);
-      }
       uint32_t in_cnt = 0, w_cnt = 0;
       bool okw = true;
       for (int i = 0; okw; ++i) {
@@ -185,15 +200,13 @@ conv3x3_kernel(const __grid_constant__ CUtensorMap tm_in, const __grid_constant_
                              row0 + b * p.box_rows, in_full + 8 * st);
           ++in_cnt;
           if (!RESIDENT) {
-            for (int tap = 0; tap < 9; ++tap) {
+            for (int tap = 0; tap < 9; ++tap, ++w_cnt) {
+              if (w_cnt < early) continue;
               const uint32_t ws = w_cnt % (uint32_t)p.w_stages;
               const uint32_t wpar = ((w_cnt / (uint32_t)p.w_stages) & 1u) ^ 1u;
               if (!ptx::mbar_wait_abortable(w_empty + 8 * ws, wpar, abort_flag)) { okw = false; break; }
               ptx::mbar_arrive_expect_tx(w_full + 8 * ws, WTILE);
-              ptx::bulk_g2s(sW + ws * WTILE,
-                            p.wpack + ((size_t)n_tile * kb_total + (size_t)tap * p.CB + cb) * WTILE, WTILE,
-                            w_full + 8 * ws);
-              ++w_cnt;
+              ptx::bulk_g2s(sW + ws * WTILE, weight_tile(n_tile, cb, tap), WTILE, w_full + 8 * ws);
             }
           }
         }
@@ -202,21 +215,22 @@ conv3x3_kernel(const __grid_constant__ CUtensorMap tm_in, const __grid_constant_
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------------ MMA issuer ------
-    if (lane == 0) {
+    {
+      const uint32_t issue = ptx::elect_one();
       const uint32_t idesc = ptx::umma_idesc(128, BN, p.bf16 ? 1 : 0);
       bool okw = true;
-      if (RESIDENT) okw = ptx::mbar_wait_abortable(w_full, 0, abort_flag);
+      if (RESIDENT) okw = ptx::warp_wait(w_full, 0, abort_flag);
       uint32_t in_cnt = 0, w_cnt = 0, acc_cnt = 0;
       for (int i = 0; okw; ++i) {
         int m_item, n_tile;
         if (!item_of(i, m_item, n_tile)) break;
         const uint32_t ab = acc_cnt % AB;
-        if (!ptx::mbar_wait_abortable(acc_empty + 8 * ab, ((acc_cnt / AB) & 1u) ^ 1u, abort_flag)) { okw = false; break; }
+        if (!ptx::warp_wait(acc_empty + 8 * ab, ((acc_cnt / AB) & 1u) ^ 1u, abort_flag)) { okw = false; break; }
         ptx::tc_fence_after();
         const uint32_t d_base = tmem_base + ab * (MT * BN);
         for (int cb = 0; cb < p.CB && okw; ++cb) {
           const uint32_t st = in_cnt % (uint32_t)p.in_stages;
-          if (!ptx::mbar_wait_abortable(in_full + 8 * st, (in_cnt / (uint32_t)p.in_stages) & 1u, abort_flag)) { okw = false; break; }
+          if (!ptx::warp_wait(in_full + 8 * st, (in_cnt / (uint32_t)p.in_stages) & 1u, abort_flag)) { okw = false; break; }
           ptx::tc_fence_after();
           const uint32_t a_stage = sIn + st * in_stage_bytes;
           for (int tap = 0; tap < 9; ++tap) {
@@ -226,7 +240,7 @@ conv3x3_kernel(const __grid_constant__ CUtensorMap tm_in, const __grid_constant_
               w_addr = sW + (uint32_t)(tap * p.CB + cb) * WTILE;
             } else {
               ws = w_cnt % (uint32_t)p.w_stages;
-              if (!ptx::mbar_wait_abortable(w_full + 8 * ws, (w_cnt / (uint32_t)p.w_stages) & 1u, abort_flag)) { okw = false; break; }
+              if (!ptx::warp_wait(w_full + 8 * ws, (w_cnt / (uint32_t)p.w_stages) & 1u, abort_flag)) { okw = false; break; }
               ptx::tc_fence_after();
               w_addr = sW + ws * WTILE;
             }
@@ -242,21 +256,21 @@ conv3x3_kernel(const __grid_constant__ CUtensorMap tm_in, const __grid_constant_
                 ptx::umma_f16(d_base + t * BN,
                               ptx::desc_from_halves(a_lo + (uint32_t)(t * (128 * 128) + k4 * 32) / 16u, ptx::kSmemDescK128Hi),
                               ptx::desc_from_halves(b_lo + (uint32_t)(k4 * 32) / 16u, ptx::kSmemDescK128Hi), idesc,
-                              k4 == 0 ? first : 1u);
+                              k4 == 0 ? first : 1u, issue);
               }
             }
             if (!RESIDENT) {
-              ptx::tc_commit(w_empty + 8 * ws);
+              ptx::tc_commit(w_empty + 8 * ws, issue);
               ++w_cnt;
             }
           }
-          ptx::tc_commit(in_empty + 8 * st);
+          ptx::tc_commit(in_empty + 8 * st, issue);
           ++in_cnt;
         }
-        ptx::tc_commit(acc_full + 8 * ab);
+        ptx::tc_commit(acc_full + 8 * ab, issue);
         ++acc_cnt;
       }
-      if (!okw && p.error_flag) atomicCAS(p.error_flag, 0, (int)kErrWaitMma);
+      if (!okw && lane == 0 && p.error_flag) atomicCAS(p.error_flag, 0, (int)kErrWaitMma);
     }
   } else {
     // ------------------------------------------------------------------ epilogue --------

@@ -11,8 +11,8 @@
 //   in_full / w_full    local TMA completion in each CTA; the peer CTA's idle MMA warp relays each
 //                       completion to the LEADER's in_full / w_full with a remote arrive (those expect
 //                       two arrivals), so the issuing lane tests one barrier per stage.
-//   in_empty / w_empty  the leader commits its MMAs to the local AND (mapped address) the peer's
-//                       barrier, so both producers reuse the stage.
+//   in_empty / w_empty  the leader's commit arrives on the barrier of BOTH CTAs (one multicast commit),
+//                       so both producers reuse the stage.
 //   acc_full            committed to both CTAs; acc_empty (leader) collects one arrive per epilogue warp of both.
 // No cluster-multicast copies are used anywhere.  Every wait is bounded and abortable.
 #include <cuda.h>
@@ -96,7 +96,7 @@ conv3x3_pair_kernel(const __grid_constant__ CUtensorMap tm_in, const __grid_cons
     }
   }
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = ptx::warp_uniform((int)threadIdx.x >> 5), lane = threadIdx.x & 31;
   const uint32_t rank = ptx::cluster_ctarank();   // 0 = leader
   if (threadIdx.x == 0) {
     s_abort = 0;
@@ -126,10 +126,8 @@ conv3x3_pair_kernel(const __grid_constant__ CUtensorMap tm_in, const __grid_cons
   __syncthreads();
   ptx::cluster_sync_all();   // both CTAs' barriers exist before anyone arrives remotely
   ptx::tc_fence_after();
-  const uint32_t tmem_base = *reinterpret_cast<volatile uint32_t*>(smem_raw + (tmem_slot - raw));
+  const uint32_t tmem_base = (uint32_t)ptx::warp_uniform(*reinterpret_cast<volatile int*>(smem_raw + (tmem_slot - raw)));
   volatile int* abort_flag = &s_abort;
-  ptx::grid_dependency_wait();
-  ptx::grid_launch_dependents();
 
   const int pairs = (int)gridDim.x >> 1, pair = (int)blockIdx.x >> 1;
   const int total_items = p.m_items * p.n_tiles;
@@ -150,6 +148,42 @@ conv3x3_pair_kernel(const __grid_constant__ CUtensorMap tm_in, const __grid_cons
     return w < total_items;
   };
 
+  // This CTA's half of an item's columns for filter row fr of channel block cb -> weight stage ws (three taps).  False: the
+  // copy would leave the packed weights or the ring (reported; the waits then run out).
+  auto load_weights = [&](int n_tile, int sub, int parts, int cb, int fr, uint32_t ws) {
+    const int ncols = BNP / parts;
+    const int wrow = n_tile * BNP + sub * ncols + (int)rank * (ncols / 2);   // as rows of the packed N tiles
+    const uint32_t wbytes = (uint32_t)(ncols / 2) * 128u;                    // per tap
+    const uint8_t* wsrc = p.wpack + (size_t)(wrow / kPackBN) * kb_total * kPackTile + (size_t)(wrow % kPackBN) * 128;
+    ptx::mbar_arrive_expect_tx(w_full + 8 * ws, kWGroup * wbytes);
+#pragma unroll
+    for (int s3 = 0; s3 < kWGroup; ++s3) {
+      const uint8_t* src = wsrc + ((size_t)(fr * 3 + s3) * p.CB + cb) * kPackTile;
+      if ((size_t)(src - p.wpack) + wbytes > p.wpack_bytes || sW + ws * kWStage + (s3 + 1) * kWTile > sStage) {
+        if (p.error_flag) atomicCAS(p.error_flag, 0, (int)kErrBounds);
+        *abort_flag = 1;
+        return false;
+      }
+      ptx::bulk_g2s(sW + ws * kWStage + s3 * kWTile, src, wbytes, w_full + 8 * ws);
+    }
+    return true;
+  };
+  // Packed weights never change, so their copies start before the previous kernel of the stream has finished.
+  uint32_t early = 0;   // stages of the weight ring already on their way
+  if (warp == 0 && lane == 0) {
+    bool ok = true;
+    for (int i = 0; ok && early < (uint32_t)p.w_stages && !(p.w_resident && i > 0); ++i) {
+      int m_item, n_tile, sub, parts;
+      if (!item_of(i, m_item, n_tile, sub, parts)) break;
+      for (int cb = 0; ok && cb < p.CB && early < (uint32_t)p.w_stages; ++cb)
+        for (int fr = 0; ok && fr < 3 && early < (uint32_t)p.w_stages; ++fr, ++early)
+          ok = load_weights(n_tile, sub, parts, cb, fr, early);
+    }
+  }
+  // The rest reads what the previous kernel wrote, or writes what it may still be reading.
+  ptx::grid_dependency_wait();
+  ptx::grid_launch_dependents();
+
   if (warp == 0) {
     // ------------------------------------------------------------------ TMA producer ----
     if (lane == 0) {
@@ -161,11 +195,6 @@ conv3x3_pair_kernel(const __grid_constant__ CUtensorMap tm_in, const __grid_cons
         // the leader owns the first mt * 128 slots of the item, the peer the rest: sub-tile t is rows
         // [t * 128, +128) of both CTAs' tiles
         const int row0 = (m_item * 2 + (int)rank) * 128 * MT - p.P - 1;
-        // this CTA's half of the item's columns, as rows of the packed N tiles
-        const int ncols = BNP / parts;
-        const int wrow = n_tile * BNP + sub * ncols + (int)rank * (ncols / 2);
-        const uint32_t wbytes = (uint32_t)(ncols / 2) * 128u;   // per tap
-        const uint8_t* wsrc = p.wpack + (size_t)(wrow / kPackBN) * kb_total * kPackTile + (size_t)(wrow % kPackBN) * 128;
         for (int cb = 0; cb < p.CB && okw; ++cb) {
           const uint32_t st = in_cnt % (uint32_t)p.in_stages;
           if (!ptx::mbar_wait_cluster_abortable(in_empty + 8 * st, ((in_cnt / (uint32_t)p.in_stages) & 1u) ^ 1u, abort_flag)) { okw = false; break; }
@@ -176,33 +205,20 @@ conv3x3_pair_kernel(const __grid_constant__ CUtensorMap tm_in, const __grid_cons
           ++in_cnt;
           if (p.w_resident && i > 0) continue;       // resident weights were loaded with the first item
           for (int fr = 0; fr < 3; ++fr, ++w_cnt) {   // one filter row (three taps) per weight stage
+            if (w_cnt < early) continue;
             const uint32_t ws = w_cnt % (uint32_t)p.w_stages;
             if (!ptx::mbar_wait_cluster_abortable(w_empty + 8 * ws, ((w_cnt / (uint32_t)p.w_stages) & 1u) ^ 1u, abort_flag)) { okw = false; break; }
-            ptx::mbar_arrive_expect_tx(w_full + 8 * ws, kWGroup * wbytes);
-#pragma unroll
-            for (int s3 = 0; s3 < kWGroup; ++s3) {
-              const uint8_t* src = wsrc + ((size_t)(fr * 3 + s3) * p.CB + cb) * kPackTile;
-              // never start a copy that would leave the packed weights: report and let the waits run out
-              if ((size_t)(src - p.wpack) + wbytes > p.wpack_bytes || sW + ws * kWStage + (s3 + 1) * kWTile > sStage) {
-                if (p.error_flag) atomicCAS(p.error_flag, 0, (int)kErrBounds);
-                *abort_flag = 1;
-                okw = false;
-                break;
-              }
-              ptx::bulk_g2s(sW + ws * kWStage + s3 * kWTile, src, wbytes, w_full + 8 * ws);
-            }
-            if (!okw) break;
+            if (!load_weights(n_tile, sub, parts, cb, fr, ws)) { okw = false; break; }
           }
         }
       }
       if (!okw && p.error_flag) atomicCAS(p.error_flag, 0, (int)kErrWaitProducer);
     }
   } else if (warp == 1) {
-    if (lane == 0 && rank == 0) {
+    if (rank == 0) {
       // ---------------------------------------------------------------- MMA issuer (leader) --
+      const uint32_t issue = ptx::elect_one();
       const uint32_t idesc_full = ptx::umma_idesc(256, kBNPair, p.bf16 ? 1 : 0);
-      const uint32_t peer_in_empty = ptx::map_to_cta(in_empty, 1), peer_w_empty = ptx::map_to_cta(w_empty, 1);
-      const uint32_t peer_acc_full = ptx::map_to_cta(acc_full, 1);
       uint32_t in_cnt = 0, w_cnt = 0, acc_cnt = 0;
       bool okw = true;
       for (int i = 0; okw; ++i) {
@@ -210,13 +226,13 @@ conv3x3_pair_kernel(const __grid_constant__ CUtensorMap tm_in, const __grid_cons
         if (!item_of(i, m_item, n_tile, sub, parts)) break;
         const uint32_t idesc = parts == 1 ? idesc_full : ptx::umma_idesc(256, kBNPair / parts, p.bf16 ? 1 : 0);
         const uint32_t ab = acc_cnt % kAB;
-        if (!ptx::mbar_wait_cluster_abortable(acc_empty + 8 * ab, ((acc_cnt / kAB) & 1u) ^ 1u, abort_flag)) { okw = false; break; }
+        if (!ptx::warp_wait_cluster(acc_empty + 8 * ab, ((acc_cnt / kAB) & 1u) ^ 1u, abort_flag)) { okw = false; break; }
         ptx::tc_fence_after();
         const uint32_t d = tmem_base + ab * (uint32_t)(kBNPair * MT);
         for (int cb = 0; cb < p.CB && okw; ++cb) {
           const uint32_t st = in_cnt % (uint32_t)p.in_stages;
           const uint32_t ipar = (in_cnt / (uint32_t)p.in_stages) & 1u;
-          if (!ptx::mbar_wait_cluster_abortable(in_full + 8 * st, ipar, abort_flag)) { okw = false; break; }
+          if (!ptx::warp_wait_cluster(in_full + 8 * st, ipar, abort_flag)) { okw = false; break; }
           ptx::tc_fence_after();
           const uint32_t a_stage = sIn + st * in_stage_bytes;
           for (int fr = 0; fr < 3; ++fr, ++w_cnt) {
@@ -224,7 +240,7 @@ conv3x3_pair_kernel(const __grid_constant__ CUtensorMap tm_in, const __grid_cons
             const uint32_t ws = p.w_resident ? (uint32_t)(cb * 3 + fr) : w_cnt % (uint32_t)p.w_stages;
             const uint32_t wpar = p.w_resident ? 0u : (w_cnt / (uint32_t)p.w_stages) & 1u;
             if (!p.w_resident || i == 0) {
-              if (!ptx::mbar_wait_cluster_abortable(w_full + 8 * ws, wpar, abort_flag)) { okw = false; break; }
+              if (!ptx::warp_wait_cluster(w_full + 8 * ws, wpar, abort_flag)) { okw = false; break; }
               ptx::tc_fence_after();
             }
 #pragma unroll
@@ -237,25 +253,22 @@ conv3x3_pair_kernel(const __grid_constant__ CUtensorMap tm_in, const __grid_cons
                 for (int k4 = 0; k4 < 4; ++k4)
                   ptx::umma_f16_pair(d + (uint32_t)(t * kBNPair), ptx::desc_from_halves(a_lo + k4 * 2, ptx::kSmemDescK128Hi),
                                      ptx::desc_from_halves(b_lo + k4 * 2, ptx::kSmemDescK128Hi), idesc,
-                                     (cb | fr | s3 | k4) != 0 ? 1u : 0u);
+                                     (cb | fr | s3 | k4) != 0 ? 1u : 0u, issue);
               }
             }
             if (!p.w_resident) {
-              ptx::tc_commit_pair(w_empty + 8 * ws);
-              ptx::tc_commit_pair(peer_w_empty + 8 * ws);
+              ptx::tc_commit_pair(w_empty + 8 * ws, issue);
             }
           }
           if (!okw) break;
-          ptx::tc_commit_pair(in_empty + 8 * st);
-          ptx::tc_commit_pair(peer_in_empty + 8 * st);
+          ptx::tc_commit_pair(in_empty + 8 * st, issue);
           ++in_cnt;
         }
         if (!okw) break;
-        ptx::tc_commit_pair(acc_full + 8 * ab);
-        ptx::tc_commit_pair(peer_acc_full + 8 * ab);
+        ptx::tc_commit_pair(acc_full + 8 * ab, issue);
         ++acc_cnt;
       }
-      if (!okw && p.error_flag) atomicCAS(p.error_flag, 0, (int)kErrWaitMma);
+      if (!okw && lane == 0 && p.error_flag) atomicCAS(p.error_flag, 0, (int)kErrWaitMma);
     } else if (lane == 0) {
       // ---------------------------------------------------------------- relay (peer CTA) ----
       // Tells the leader when this CTA's stages are full.

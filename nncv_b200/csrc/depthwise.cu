@@ -128,6 +128,8 @@ __device__ __forceinline__ float act1(float x, int act) {
 
 template <typename T, int KS, int STRIDE>
 __global__ void __launch_bounds__(kThreads, KS == 3 ? 3 : 2) depthwise_tma_kernel(const __grid_constant__ CUtensorMap tm_in, const DwParams p) {
+  ptx::grid_dependency_wait();
+  ptx::grid_launch_dependents();
   constexpr int V = 16 / sizeof(T);
   constexpr int NR = (kP - 1) * STRIDE + KS;            // input rows under one strip of kP outputs
   extern __shared__ __align__(128) unsigned char smem[];
@@ -296,7 +298,7 @@ cudaError_t launch_one(const CUtensorMap& tm, const DwParams& p, dim3 grid, size
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
   }
-  kern<<<grid, kThreads, smem, st>>>(tm, p);
+  launch_pdl(kern, grid, dim3(kThreads), smem, st, tm, p);
   return cudaGetLastError();
 }
 

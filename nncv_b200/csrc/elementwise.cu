@@ -76,6 +76,8 @@ template <typename T, typename WT>
 __global__ void depthwise_kernel(const T* __restrict__ x, const WT* __restrict__ w, const float* __restrict__ scale,
                                  const float* __restrict__ shift, T* __restrict__ y, int N, int H, int W, int C, int OH,
                                  int OW, int R, int S, int stride, int pad, int act, Layout il, Layout ol) {
+  ptx::grid_dependency_wait();
+  ptx::grid_launch_dependents();
   constexpr int V = 16 / sizeof(T);
   const int cv = C / V;
   const long long total = (long long)N * OH * OW * cv;
@@ -116,6 +118,8 @@ __global__ void depthwise_kernel(const T* __restrict__ x, const WT* __restrict__
 // ---------------------------------------------------------------- elementwise ------------
 template <typename T>
 __global__ void activation_kernel(const T* __restrict__ x, T* __restrict__ y, size_t n_vec, int act) {
+  ptx::grid_dependency_wait();
+  ptx::grid_launch_dependents();
   constexpr int V = 16 / sizeof(T);
   for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n_vec; i += (size_t)gridDim.x * blockDim.x) {
     const uint4 raw = __ldg(reinterpret_cast<const uint4*>(x) + i);
@@ -131,6 +135,8 @@ __global__ void activation_kernel(const T* __restrict__ x, T* __restrict__ y, si
 template <typename T>
 __global__ void scale_channels_kernel(const T* __restrict__ x, const T* __restrict__ gate, T* __restrict__ y, int N,
                                       long long HW, int C) {
+  ptx::grid_dependency_wait();
+  ptx::grid_launch_dependents();
   constexpr int V = 16 / sizeof(T);
   const int cv = C / V;
   const long long total = (long long)N * HW * cv;
@@ -161,6 +167,8 @@ template <typename T>
 __global__ void __cluster_dims__(kSeCluster, 1, 1) __launch_bounds__(256)
 se_gate_kernel(const T* __restrict__ pooled, const float* __restrict__ w1, const float* __restrict__ b1,
                const float* __restrict__ w2, const float* __restrict__ b2, T* __restrict__ gate, int N, int C, int Cr) {
+  ptx::grid_dependency_wait();
+  ptx::grid_launch_dependents();
   extern __shared__ float sm[];
   float* p = sm;                          // [kSeImages][C]
   float* hid = sm + kSeImages * C;        // [kSeImages][Cr]: this CTA's units, read by the whole cluster
@@ -232,6 +240,8 @@ struct ConcatParams {
   int n_in, cv_out;
 };
 __global__ void concat_kernel(const ConcatParams p, uint4* __restrict__ out, long long pixels) {
+  ptx::grid_dependency_wait();
+  ptx::grid_launch_dependents();
   const long long total = pixels * p.cv_out;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
     const int v = (int)(i % p.cv_out);
@@ -247,6 +257,8 @@ __global__ void concat_kernel(const ConcatParams p, uint4* __restrict__ out, lon
 // Nearest-neighbour 2x upsampling: out[n, y, x, :] = in[n, y / 2, x / 2, :].
 // One thread per input vector: one load, four stores (the two copies along x are adjacent in memory).
 __global__ void upsample2x_kernel(const uint4* __restrict__ in, uint4* __restrict__ out, int N, int H, int W, int cv) {
+  ptx::grid_dependency_wait();
+  ptx::grid_launch_dependents();
   const long long total = (long long)N * H * W * cv;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
     const int c = (int)(i % cv);
@@ -294,7 +306,7 @@ cudaError_t launch_depthwise(const void* x, const void* w, DType w_dt, const flo
   const long long work = (long long)N * OH * OW * (C / V);
   const int g = grid_for(work, 256);
 #define NNCV_DW(T, WT)                                                                                                        \
-  depthwise_kernel<T, WT><<<g, 256, 0, st>>>((const T*)x, (const WT*)w, scale, shift, (T*)y, N, H, W, C, OH, OW, R, S, stride, \
+  launch_pdl(depthwise_kernel<T, WT>, dim3(g), dim3(256), 0, st, (const T*)x, (const WT*)w, scale, shift, (T*)y, N, H, W, C, OH, OW, R, S, stride, \
                                              pad, act, in_l, out_l)
   if (dt == kF32) { if (w_dt != kF32) return cudaErrorInvalidValue; NNCV_DW(float, float); }
   else if (dt == kF16) { if (w_dt == kF32) NNCV_DW(__half, float); else NNCV_DW(__half, __half); }
@@ -307,9 +319,9 @@ cudaError_t launch_activation(const void* x, void* y, DType dt, size_t n, int ac
   const size_t V = 16 / dtype_size(dt);
   if (n % V != 0) return cudaErrorInvalidValue;
   const int g = grid_for((long long)(n / V), 256);
-  if (dt == kF32) activation_kernel<float><<<g, 256, 0, st>>>((const float*)x, (float*)y, n / V, act);
-  else if (dt == kF16) activation_kernel<__half><<<g, 256, 0, st>>>((const __half*)x, (__half*)y, n / V, act);
-  else activation_kernel<__nv_bfloat16><<<g, 256, 0, st>>>((const __nv_bfloat16*)x, (__nv_bfloat16*)y, n / V, act);
+  if (dt == kF32) launch_pdl(activation_kernel<float>, dim3(g), dim3(256), 0, st, (const float*)x, (float*)y, n / V, act);
+  else if (dt == kF16) launch_pdl(activation_kernel<__half>, dim3(g), dim3(256), 0, st, (const __half*)x, (__half*)y, n / V, act);
+  else launch_pdl(activation_kernel<__nv_bfloat16>, dim3(g), dim3(256), 0, st, (const __nv_bfloat16*)x, (__nv_bfloat16*)y, n / V, act);
   return cudaGetLastError();
 }
 
@@ -317,9 +329,9 @@ cudaError_t launch_scale_channels(const void* x, const void* gate, void* y, DTyp
   const int V = 16 / (int)dtype_size(dt);
   if (C % V != 0) return cudaErrorInvalidValue;
   const int g = grid_for((long long)N * HW * (C / V), 256);
-  if (dt == kF32) scale_channels_kernel<float><<<g, 256, 0, st>>>((const float*)x, (const float*)gate, (float*)y, N, HW, C);
-  else if (dt == kF16) scale_channels_kernel<__half><<<g, 256, 0, st>>>((const __half*)x, (const __half*)gate, (__half*)y, N, HW, C);
-  else scale_channels_kernel<__nv_bfloat16><<<g, 256, 0, st>>>((const __nv_bfloat16*)x, (const __nv_bfloat16*)gate, (__nv_bfloat16*)y, N, HW, C);
+  if (dt == kF32) launch_pdl(scale_channels_kernel<float>, dim3(g), dim3(256), 0, st, (const float*)x, (const float*)gate, (float*)y, N, HW, C);
+  else if (dt == kF16) launch_pdl(scale_channels_kernel<__half>, dim3(g), dim3(256), 0, st, (const __half*)x, (const __half*)gate, (__half*)y, N, HW, C);
+  else launch_pdl(scale_channels_kernel<__nv_bfloat16>, dim3(g), dim3(256), 0, st, (const __nv_bfloat16*)x, (const __nv_bfloat16*)gate, (__nv_bfloat16*)y, N, HW, C);
   return cudaGetLastError();
 }
 
@@ -333,7 +345,7 @@ cudaError_t launch_se_gate(const void* pooled, const float* w1, const float* b1,
   do {                                                                                                               \
     auto kern = se_gate_kernel<T>;                                                                                   \
     if (smem > 48 * 1024) e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);    \
-    if (e == cudaSuccess) kern<<<g, 256, smem, st>>>((const T*)pooled, w1, b1, w2, b2, (T*)gate, N, C, Cr);          \
+    if (e == cudaSuccess) launch_pdl(kern, dim3(g), dim3(256), smem, st, (const T*)pooled, w1, b1, w2, b2, (T*)gate, N, C, Cr);          \
   } while (0)
   if (dt == kF32) NNCV_SE(float);
   else if (dt == kF16) NNCV_SE(__half);
@@ -353,14 +365,14 @@ cudaError_t launch_concat(const void* const* in, const int* channels, int n_in, 
     off += channels[i] / V;
   }
   p.n_in = n_in; p.cv_out = off;
-  concat_kernel<<<grid_for(pixels * off, 256), 256, 0, st>>>(p, (uint4*)out, pixels);
+  launch_pdl(concat_kernel, dim3(grid_for(pixels * off, 256)), dim3(256), 0, st, p, (uint4*)out, pixels);
   return cudaGetLastError();
 }
 
 cudaError_t launch_upsample2x(const void* in, void* out, DType dt, int N, int H, int W, int C, cudaStream_t st) {
   const int V = 16 / (int)dtype_size(dt);
   if (C % V != 0) return cudaErrorInvalidValue;
-  upsample2x_kernel<<<grid_for((long long)N * H * W * (C / V), 256), 256, 0, st>>>((const uint4*)in, (uint4*)out, N, H, W, C / V);
+  launch_pdl(upsample2x_kernel, dim3(grid_for((long long)N * H * W * (C / V), 256)), dim3(256), 0, st, (const uint4*)in, (uint4*)out, N, H, W, C / V);
   return cudaGetLastError();
 }
 

@@ -78,7 +78,7 @@ gemm_tf32x3_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_consta
       return;
     }
   }
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = ptx::warp_uniform((int)threadIdx.x >> 5), lane = threadIdx.x & 31;
   if (threadIdx.x == 0) {
     s_abort = 0;
     for (int i = 0; i < kStages; ++i) {
@@ -101,7 +101,7 @@ gemm_tf32x3_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_consta
   ptx::tc_fence_before();
   __syncthreads();
   ptx::tc_fence_after();
-  const uint32_t tmem_base = *reinterpret_cast<volatile uint32_t*>(smem_raw + (tmem_slot - raw));
+  const uint32_t tmem_base = (uint32_t)ptx::warp_uniform(*reinterpret_cast<volatile int*>(smem_raw + (tmem_slot - raw)));
   ptx::grid_dependency_wait();
   ptx::grid_launch_dependents();
   volatile int* abort_flag = &s_abort;
@@ -135,7 +135,8 @@ gemm_tf32x3_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_consta
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------------ MMA issuer ------
-    if (lane == 0) {
+    {
+      const uint32_t issue = ptx::elect_one();
       const uint32_t idesc = ptx::umma_idesc(128, kBN, 2);   // kind::tf32, fp32 accumulate, both operands K-major
       uint32_t cnt = 0, acc_cnt = 0;
       bool okw = true;
@@ -143,7 +144,7 @@ gemm_tf32x3_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_consta
         int m0, n0;
         if (!item_of(i, m0, n0)) break;
         const uint32_t ab = acc_cnt & 1u;
-        if (!ptx::mbar_wait_abortable(acc_empty + 8 * ab, ((acc_cnt >> 1) & 1u) ^ 1u, abort_flag)) { okw = false; break; }
+        if (!ptx::warp_wait(acc_empty + 8 * ab, ((acc_cnt >> 1) & 1u) ^ 1u, abort_flag)) { okw = false; break; }
         ptx::tc_fence_after();
         // two accumulators per buffer: the hi*hi products, and the two small cross terms.  The tensor core
         // cuts (does not round) every accumulation into TMEM, an error of one sign per step: keeping the
@@ -151,7 +152,7 @@ gemm_tf32x3_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_consta
         const uint32_t d = tmem_base + ab * (2 * kBN), dl = d + kBN;
         for (int kb = 0; kb < p.k_blocks; ++kb, ++cnt) {
           const uint32_t st = cnt % kStages;
-          if (!ptx::mbar_wait_abortable(conv + 8 * st, (cnt / kStages) & 1u, abort_flag)) { okw = false; break; }
+          if (!ptx::warp_wait(conv + 8 * st, (cnt / kStages) & 1u, abort_flag)) { okw = false; break; }
           ptx::tc_fence_after();
           const uint32_t s0 = sRing + st * kStageBytes;
           const uint32_t a_hi = ptx::smem_desc_k128_lo(s0), a_lo = ptx::smem_desc_k128_lo(s0 + kTile);
@@ -162,17 +163,17 @@ gemm_tf32x3_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_consta
             const uint64_t al = ptx::desc_from_halves(a_lo + k4 * 2, ptx::kSmemDescK128Hi);
             const uint64_t bh = ptx::desc_from_halves(b_hi + k4 * 2, ptx::kSmemDescK128Hi);
             const uint64_t bl = ptx::desc_from_halves(b_lo + k4 * 2, ptx::kSmemDescK128Hi);
-            ptx::umma_tf32(dl, al, bh, idesc, (kb | (int)k4) != 0 ? 1u : 0u);
-            ptx::umma_tf32(dl, ah, bl, idesc, 1u);
-            ptx::umma_tf32(d, ah, bh, idesc, (kb | (int)k4) != 0 ? 1u : 0u);
+            ptx::umma_tf32(dl, al, bh, idesc, (kb | (int)k4) != 0 ? 1u : 0u, issue);
+            ptx::umma_tf32(dl, ah, bl, idesc, 1u, issue);
+            ptx::umma_tf32(d, ah, bh, idesc, (kb | (int)k4) != 0 ? 1u : 0u, issue);
           }
-          ptx::tc_commit(empty + 8 * st);
+          ptx::tc_commit(empty + 8 * st, issue);
         }
         if (!okw) break;
-        ptx::tc_commit(acc_full + 8 * ab);
+        ptx::tc_commit(acc_full + 8 * ab, issue);
         ++acc_cnt;
       }
-      if (!okw && p.error_flag) atomicCAS(p.error_flag, 0, (int)kErrWaitMma);
+      if (!okw && lane == 0 && p.error_flag) atomicCAS(p.error_flag, 0, (int)kErrWaitMma);
     }
   } else if (warp < 2 + kConvGroups * kConvWarps) {
     // ------------------------------------------------------------------ transpose B, hi / lo split ----

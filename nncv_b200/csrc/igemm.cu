@@ -58,6 +58,8 @@ __device__ __forceinline__ void report(int* flag, int code) {
 
 template <int BN>
 __global__ void __launch_bounds__(kThreads) conv_igemm_kernel(const IgemmParams p) {
+  ptx::grid_dependency_wait();
+  ptx::grid_launch_dependents();
   constexpr int kBBytes = BN * 128;
   extern __shared__ uint8_t smem_raw[];
   const uint32_t raw = ptx::smem_u32(smem_raw);
@@ -277,11 +279,11 @@ __global__ void __launch_bounds__(kThreads) conv_igemm_kernel(const IgemmParams 
 #pragma unroll
         for (int k4 = 0; k4 < kBK / 16; ++k4) {
           ptx::umma_f16(tmem_base, ptx::smem_desc_k128(a_addr + k4 * 32),
-                        ptx::smem_desc_k128(b_addr + k4 * 32), idesc, (kb | k4) != 0 ? 1u : 0u);
+                        ptx::smem_desc_k128(b_addr + k4 * 32), idesc, (kb | k4) != 0 ? 1u : 0u, 1u);
         }
-        ptx::tc_commit(empty + 8 * stage);
+        ptx::tc_commit(empty + 8 * stage, 1u);
       }
-      ptx::tc_commit(accum);
+      ptx::tc_commit(accum, 1u);
     }
   } else {
     // ------------------------------------------------------------- weight loader ------
@@ -373,7 +375,7 @@ cudaError_t launch_bn(const IgemmParams& p, int m_tiles, int n_tiles, cudaStream
   cudaError_t e = cudaFuncSetAttribute(conv_igemm_kernel<BN>,
                                        cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;
-  conv_igemm_kernel<BN><<<dim3(m_tiles, n_tiles), kThreads, smem, stream>>>(p);
+  launch_pdl(conv_igemm_kernel<BN>, dim3(m_tiles, n_tiles), dim3(kThreads), smem, stream, p);
   return cudaGetLastError();
 }
 

@@ -72,7 +72,7 @@ struct Conv3x3Config {
 };
 struct Conv3x3Args {
   const void* in = nullptr;
-  const void* wpack = nullptr;     // packed by launch_pack_weights for N tile `bn`
+  const void* wpack = nullptr;     // packed by launch_pack_weights for N tile `bn`; complete before this launch
   const float* scale = nullptr;
   const float* shift = nullptr;
   const void* residual = nullptr;
@@ -96,6 +96,7 @@ cudaError_t launch_conv3x3_pair(const Conv3x3Args& a, cudaStream_t stream);
 struct TconvArgs {
   const void* in = nullptr;        // activation in layout in_l, or A[M,K] as {1, M, 0}
   const void* wpack = nullptr;     // packed by launch_pack_weights for N tile `bn`
+  int weights_ready = 0;           // wpack (and wpack2) were complete before this launch: they may be read before earlier work of the stream ends
   const float* scale = nullptr;
   const float* shift = nullptr;
   const void* residual = nullptr;  // layout out_l, 16-bit

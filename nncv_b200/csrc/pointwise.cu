@@ -54,6 +54,8 @@ struct PwParams {
 
 template <bool BF16>
 __global__ void __launch_bounds__(256) pointwise_kernel(const PwParams p) {
+  ptx::grid_dependency_wait();
+  ptx::grid_launch_dependents();
   extern __shared__ __align__(16) float sw[];     // [C][Kp] weights, [Kp] scale, [Kp] shift
   float* ssc = sw + (size_t)p.C * p.Kp;
   float* ssh = ssc + p.Kp;
@@ -172,10 +174,10 @@ cudaError_t launch_pointwise(const PointwiseArgs& a, cudaStream_t st) {
   cudaError_t e = cudaSuccess;
   if (a.ab == kBF16) {
     if (smem > 48 * 1024) e = cudaFuncSetAttribute(pointwise_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e == cudaSuccess) pointwise_kernel<true><<<(unsigned)blocks, 256, smem, st>>>(p);
+    if (e == cudaSuccess) launch_pdl(pointwise_kernel<true>, dim3((unsigned)blocks), dim3(256), smem, st, p);
   } else {
     if (smem > 48 * 1024) e = cudaFuncSetAttribute(pointwise_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e == cudaSuccess) pointwise_kernel<false><<<(unsigned)blocks, 256, smem, st>>>(p);
+    if (e == cudaSuccess) launch_pdl(pointwise_kernel<false>, dim3((unsigned)blocks), dim3(256), smem, st, p);
   }
   return e != cudaSuccess ? e : cudaGetLastError();
 }

@@ -393,6 +393,8 @@ int conv_prepare(nncv_b200_conv* c, int bn, cudaStream_t st, const void** wpack,
     if (rc) return rc;
     LAUNCH(launch_pack_weights(c->raw, c->raw_dt, c->sn, c->sc, c->stap, c->Kout, c->C, cpad,
                                c->R * c->S, bn, c->dtype, buf->p, st));
+    // the convolution kernels read packed weights without waiting for earlier work of their stream
+    CU(cudaStreamSynchronize(st));
     it = c->packed.emplace(key, std::move(buf)).first;
   }
   *wpack = it->second->p;
@@ -528,6 +530,7 @@ int conv_run(nncv_b200_conv* c, const void* in, Layout in_l, void* out, Layout o
       TconvArgs a;
       a.in = in; a.wpack = wpack; a.scale = scale; a.shift = shift; a.residual = residual; a.out = out;
       a.pair = ch.kernel == 8;
+      a.weights_ready = 1;
       if (fb) {
         rc = conv_prepare(fb->conv, a.pair ? 64 : 128, st, &a.wpack2, true);
         if (rc) return rc;

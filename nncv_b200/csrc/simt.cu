@@ -161,6 +161,8 @@ __global__ void repack_weights_f32_kernel(const SrcT* __restrict__ src, long lon
 template <typename SrcT, typename DstT>
 __global__ void nchw_to_nhwc_kernel(const SrcT* __restrict__ src, DstT* __restrict__ dst, int N,
                                     int C, long long HW, int Cpad) {
+  ptx::grid_dependency_wait();
+  ptx::grid_launch_dependents();
   const long long total = (long long)N * HW;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total;
        i += (long long)gridDim.x * blockDim.x) {
@@ -199,6 +201,8 @@ template <typename T>
 __global__ void maxpool_nhwc_kernel(const T* __restrict__ src, T* __restrict__ dst, int N, int H,
                                     int W, int C, int OH, int OW, int k, int stride, int pad,
                                     Layout il, Layout ol) {
+  ptx::grid_dependency_wait();
+  ptx::grid_launch_dependents();
   constexpr int V = 16 / sizeof(T);
   const int cv = C / V;
   // the launcher keeps the count of (output pixel, vector) items below 2^31: the index arithmetic is
@@ -269,6 +273,8 @@ __global__ void maxpool_nhwc_kernel(const T* __restrict__ src, T* __restrict__ d
 template <typename T>
 __global__ void avgpool_nhwc_kernel(const T* __restrict__ src, T* __restrict__ dst, int N, int H,
                                     int W, int C, Layout il) {
+  ptx::grid_dependency_wait();
+  ptx::grid_launch_dependents();
   const int HW = H * W;
   constexpr int V = 16 / sizeof(T);
   constexpr int kSlices = 8;
@@ -316,6 +322,8 @@ constexpr int kPoolCluster = 8;
 template <typename T>
 __global__ void __cluster_dims__(kPoolCluster, 1, 1) __launch_bounds__(256)
 avgpool_cluster_kernel(const T* __restrict__ src, T* __restrict__ dst, int N, int H, int W, int C, Layout il) {
+  ptx::grid_dependency_wait();
+  ptx::grid_launch_dependents();
   constexpr int V = 16 / sizeof(T);
   __shared__ __align__(16) float part[256 * V];     // [slice][vector][V]
   __shared__ __align__(16) float tot[256 * V];      // [vector][V]: this CTA's sum
@@ -379,6 +387,8 @@ avgpool_cluster_kernel(const T* __restrict__ src, T* __restrict__ dst, int N, in
 // Layout change, one thread per 16-byte vector of a destination slot; pads are written as zero.
 __global__ void relayout_kernel(const uint4* __restrict__ src, Layout sl, uint4* __restrict__ dst,
                                 Layout dl, int N, int H, int W, int cv) {
+  ptx::grid_dependency_wait();
+  ptx::grid_launch_dependents();
   const long long total = (long long)N * dl.img_rows * dl.pitch * cv;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total;
        i += (long long)gridDim.x * blockDim.x) {
@@ -410,6 +420,8 @@ __global__ void bn_fold_kernel(const T* gamma, const T* beta, const T* mean, con
 
 template <typename S, typename D>
 __global__ void convert_kernel(const S* __restrict__ src, D* __restrict__ dst, size_t n) {
+  ptx::grid_dependency_wait();
+  ptx::grid_launch_dependents();
   for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x)
     dst[i] = from_f<D>(to_f<S>(src[i]));
 }
@@ -488,9 +500,8 @@ cudaError_t launch_nchw_to_nhwc(const void* src, DType src_dt, void* dst, DType 
     using S = decltype(stag);
     return by_dtype(dst_dt, [&](auto dtag) {
       using D = decltype(dtag);
-      nchw_to_nhwc_kernel<S, D><<<grid_for((long long)N * HW, 256), 256, 0, stream>>>(
+      return launch_pdl(nchw_to_nhwc_kernel<S, D>, dim3(grid_for((long long)N * HW, 256)), dim3(256), 0, stream,
           static_cast<const S*>(src), static_cast<D*>(dst), N, C, HW, Cpad);
-      return cudaGetLastError();
     });
   });
 }
@@ -507,10 +518,9 @@ cudaError_t launch_maxpool_nhwc(const void* src, void* dst, DType dt, int N, int
     if (C % V != 0) return cudaErrorInvalidValue;
     const long long total = (long long)N * OH * OW * (C / V);
     if (total >= (1LL << 31) - (1LL << 21)) return cudaErrorInvalidValue;   // 16 GiB of fp16 output: beyond any plan here
-    maxpool_nhwc_kernel<T><<<grid_for(total, 256), 256, 0, stream>>>(
+    return launch_pdl(maxpool_nhwc_kernel<T>, dim3(grid_for(total, 256)), dim3(256), 0, stream,
         static_cast<const T*>(src), static_cast<T*>(dst), N, H, W, C, OH, OW, k, stride, pad, in_l,
         out_l);
-    return cudaGetLastError();
   });
 }
 
@@ -523,14 +533,12 @@ cudaError_t launch_avgpool_nhwc(const void* src, void* dst, DType dt, int N, int
     if (C % V != 0) return cudaErrorInvalidValue;
     if ((long long)H * W >= 512 && N <= 65535) {
       const int cv = C / V;
-      avgpool_cluster_kernel<T><<<dim3(kPoolCluster, N, (cv + 255) / 256), 256, 0, stream>>>(
+      return launch_pdl(avgpool_cluster_kernel<T>, dim3(kPoolCluster, N, (cv + 255) / 256), dim3(256), 0, stream,
           static_cast<const T*>(src), static_cast<T*>(dst), N, H, W, C, in_l);
-      return cudaGetLastError();
     }
     const long long total = (long long)N * (C / V) * 8;
-    avgpool_nhwc_kernel<T><<<grid_for(total, 256), 256, 0, stream>>>(
+    return launch_pdl(avgpool_nhwc_kernel<T>, dim3(grid_for(total, 256)), dim3(256), 0, stream,
         static_cast<const T*>(src), static_cast<T*>(dst), N, H, W, C, in_l);
-    return cudaGetLastError();
   });
 }
 
@@ -541,9 +549,8 @@ cudaError_t launch_relayout(const void* src, Layout src_l, void* dst, Layout dst
   if (src_l.pitch == 0) src_l = dense_layout(H, W);
   if (dst_l.pitch == 0) dst_l = dense_layout(H, W);
   const long long total = layout_slots(dst_l, N) * cv;
-  relayout_kernel<<<grid_for(total, 256), 256, 0, stream>>>(
+  return launch_pdl(relayout_kernel, dim3(grid_for(total, 256)), dim3(256), 0, stream,
       static_cast<const uint4*>(src), src_l, static_cast<uint4*>(dst), dst_l, N, H, W, cv);
-  return cudaGetLastError();
 }
 
 cudaError_t launch_bn_fold(const void* gamma, const void* beta, const void* mean,
@@ -564,9 +571,8 @@ cudaError_t launch_convert(const void* src, DType src_dt, void* dst, DType dst_d
     using S = decltype(stag);
     return by_dtype(dst_dt, [&](auto dtag) {
       using D = decltype(dtag);
-      convert_kernel<S, D><<<grid_for((long long)n, 256), 256, 0, stream>>>(
+      return launch_pdl(convert_kernel<S, D>, dim3(grid_for((long long)n, 256)), dim3(256), 0, stream,
           static_cast<const S*>(src), static_cast<D*>(dst), n);
-      return cudaGetLastError();
     });
   });
 }

@@ -114,7 +114,7 @@ __global__ void __launch_bounds__(kThreads, 1) stem_pool_kernel(const __grid_con
   const uint32_t go = w_full + 8;                 // pair kernel: "everything pair seq needs is there", 4 in flight
   const uint32_t tmem_slot = go + 8 * 4;
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = ptx::warp_uniform((int)threadIdx.x >> 5), lane = threadIdx.x & 31;
   if (threadIdx.x == 0) {
     s_abort = 0;
     s_consumed = -1;
@@ -138,7 +138,7 @@ __global__ void __launch_bounds__(kThreads, 1) stem_pool_kernel(const __grid_con
   ptx::tc_fence_before();
   __syncthreads();
   ptx::tc_fence_after();
-  const uint32_t tmem_base = *reinterpret_cast<volatile uint32_t*>(smem_raw + (tmem_slot - raw));
+  const uint32_t tmem_base = (uint32_t)ptx::warp_uniform(*reinterpret_cast<volatile int*>(smem_raw + (tmem_slot - raw)));
   // The prologue above touched nothing the previous kernel of the stream writes; everything
   // below may, so wait for that kernel here and let the next one start its own prologue.
   ptx::grid_dependency_wait();
@@ -196,15 +196,15 @@ __global__ void __launch_bounds__(kThreads, 1) stem_pool_kernel(const __grid_con
     // consecutive slots (two pieces where they wrap).  The pair's newest row has no partial
     // sum yet, so it takes MMAs of its own with the accumulate flag off at the first K step.
     // Compared with one N = 64 MMA per (row, filter-row pair) the A tile is read from shared
-    // memory twice instead of four times and the issuing thread -- a single lane, ~10 clocks
-    // per instruction, ~300 per tcgen05.commit -- has 8 MMAs and ONE commit per conv row: the
+    // memory twice instead of four times and there are 8 MMAs and ONE commit per conv row: the
     // commit frees the pair's tile for the producer and tells the epilogue that every row
     // whose last pair this was is complete.
-    if (lane == 0) {
+    {
+      const uint32_t issue = ptx::elect_one();
       // instruction descriptor for N = 64 * k: the N field (N >> 3 at bit 17) grows by 8 per block
       const uint32_t idesc64 = ptx::umma_idesc(128, 64, p.bf16 ? 1 : 0);
       const uint32_t ring_lo = ptx::smem_desc_k128_lo(sRing), w_lo = ptx::smem_desc_k128_lo(sW);
-      bool okw = ptx::mbar_wait_abortable(w_full, 0, abort_flag);
+      bool okw = ptx::warp_wait(w_full, 0, abort_flag);
       uint32_t seq = 0, rc_base = 0;
       for (int i = 0; okw; ++i) {
         int n, p0, p1, y0, y1, ir0, ir1;
@@ -213,7 +213,7 @@ __global__ void __launch_bounds__(kThreads, 1) stem_pool_kernel(const __grid_con
           const uint32_t slot = seq % kRingSlots;
           // the scout warp has seen the pair's tile arrive, the epilogue move past pair seq - 8 and
           // the accumulator slots of the rows this pair starts come free
-          if (!ptx::mbar_wait_abortable(go + 8 * (seq & 3u), (seq >> 2) & 1u, abort_flag)) { okw = false; break; }
+          if (!ptx::warp_wait(go + 8 * (seq & 3u), (seq >> 2) & 1u, abort_flag)) { okw = false; break; }
           ptx::tc_fence_after();
           const uint32_t a_lo = ring_lo + slot * (uint32_t)(kSwSlot >> 4);
           if (pk > ir0 && pk < ir1 && pk - 1 >= y0 && pk + 2 <= y1) {
@@ -226,23 +226,23 @@ __global__ void __launch_bounds__(kThreads, 1) stem_pool_kernel(const __grid_con
 #pragma unroll
               for (uint32_t k4 = 0; k4 < 4; ++k4)
                 ptx::umma_f16(tmem_base + s0 * 64, ptx::desc_from_halves(a_lo + k4 * 2, ptx::kSmemDescK128Hi),
-                              ptx::desc_from_halves(w_lo + k4 * 2, ptx::kSmemDescK128Hi), idesc64 + (2u << 20), 1u);
+                              ptx::desc_from_halves(w_lo + k4 * 2, ptx::kSmemDescK128Hi), idesc64 + (2u << 20), 1u, issue);
             } else {
               const uint32_t n1 = kAcc - s0;   // 1 or 2 rows before the wrap
 #pragma unroll
               for (uint32_t k4 = 0; k4 < 4; ++k4)
                 ptx::umma_f16(tmem_base + s0 * 64, ptx::desc_from_halves(a_lo + k4 * 2, ptx::kSmemDescK128Hi),
-                              ptx::desc_from_halves(w_lo + k4 * 2, ptx::kSmemDescK128Hi), idesc64 + ((n1 - 1) << 20), 1u);
+                              ptx::desc_from_halves(w_lo + k4 * 2, ptx::kSmemDescK128Hi), idesc64 + ((n1 - 1) << 20), 1u, issue);
 #pragma unroll
               for (uint32_t k4 = 0; k4 < 4; ++k4)
                 ptx::umma_f16(tmem_base, ptx::desc_from_halves(a_lo + k4 * 2, ptx::kSmemDescK128Hi),
-                              ptx::desc_from_halves(w_lo + n1 * 512u + k4 * 2, ptx::kSmemDescK128Hi), idesc64 + ((2 - n1) << 20), 1u);
+                              ptx::desc_from_halves(w_lo + n1 * 512u + k4 * 2, ptx::kSmemDescK128Hi), idesc64 + ((2 - n1) << 20), 1u, issue);
             }
 #pragma unroll
             for (uint32_t k4 = 0; k4 < 4; ++k4)
               ptx::umma_f16(tmem_base + (cf % kAcc) * 64, ptx::desc_from_halves(a_lo + k4 * 2, ptx::kSmemDescK128Hi),
-                            ptx::desc_from_halves(w_lo + 3u * 512u + k4 * 2, ptx::kSmemDescK128Hi), idesc64, k4 > 0 ? 1u : 0u);
-            ptx::tc_commit(empty + 8 * slot);
+                            ptx::desc_from_halves(w_lo + 3u * 512u + k4 * 2, ptx::kSmemDescK128Hi), idesc64, k4 > 0 ? 1u : 0u, issue);
+            ptx::tc_commit(empty + 8 * slot, issue);
             continue;
           }
           const int lo = max(y0, pk - 1), hi = min(y1, pk + 2);
@@ -272,7 +272,7 @@ __global__ void __launch_bounds__(kThreads, 1) stem_pool_kernel(const __grid_con
 #pragma unroll
               for (uint32_t k4 = 0; k4 < 4; ++k4)
                 ptx::umma_f16(dA[pc], ptx::desc_from_halves(a_lo + k4 * 2, ptx::kSmemDescK128Hi),
-                              ptx::desc_from_halves(bA[pc] + k4 * 2, ptx::kSmemDescK128Hi), iA[pc], 1u);
+                              ptx::desc_from_halves(bA[pc] + k4 * 2, ptx::kSmemDescK128Hi), iA[pc], 1u, issue);
             }
           }
 #pragma unroll
@@ -281,14 +281,14 @@ __global__ void __launch_bounds__(kThreads, 1) stem_pool_kernel(const __grid_con
 #pragma unroll
               for (uint32_t k4 = 0; k4 < 4; ++k4)
                 ptx::umma_f16(dF[pc], ptx::desc_from_halves(a_lo + k4 * 2, ptx::kSmemDescK128Hi),
-                              ptx::desc_from_halves(bF[pc] + k4 * 2, ptx::kSmemDescK128Hi), iF[pc], k4 > 0 ? 1u : 0u);
+                              ptx::desc_from_halves(bF[pc] + k4 * 2, ptx::kSmemDescK128Hi), iF[pc], k4 > 0 ? 1u : 0u, issue);
             }
           }
-          ptx::tc_commit(empty + 8 * slot);
+          ptx::tc_commit(empty + 8 * slot, issue);
         }
         rc_base += (uint32_t)(y1 - y0 + 1);
       }
-      if (!okw && p.error_flag) atomicCAS(p.error_flag, 0, (int)kErrWaitMma);
+      if (!okw && lane == 0 && p.error_flag) atomicCAS(p.error_flag, 0, (int)kErrWaitMma);
     }
   } else if (SW && warp == kIssuerBWarp) {
     // ---------------------------------------------------------------- scout (pairs) -------
@@ -336,10 +336,11 @@ __global__ void __launch_bounds__(kThreads, 1) stem_pool_kernel(const __grid_con
     // Two issuing threads take alternate accumulators (conv rows): while one waits on its
     // barriers and commits, the other keeps the tensor pipe fed.  Input row pairs are handed
     // back by the epilogue (it sees every row finish, in order), not by the issuers.
-    if (lane == 0) {
+    {
+      const uint32_t issue = ptx::elect_one();
       const uint32_t issuer = warp == 1 ? 0u : 1u;
       const uint32_t idesc = ptx::umma_idesc(128, 64, p.bf16 ? 1 : 0);
-      bool okw = ptx::mbar_wait_abortable(w_full, 0, abort_flag);
+      bool okw = ptx::warp_wait(w_full, 0, abort_flag);
       uint32_t seq_base = 0, acc_cnt = 0;
       for (int i = 0; okw; ++i) {
         int n, p0, p1, y0, y1, ir0, ir1;
@@ -353,7 +354,7 @@ __global__ void __launch_bounds__(kThreads, 1) stem_pool_kernel(const __grid_con
           const int need = min(ir1, y + 1);            // conv row y reads pairs y-2 .. y+1
           for (; waited_upto <= need; ++waited_upto) {
             const uint32_t s = seq_base + (uint32_t)(waited_upto - ir0);
-            if (!ptx::mbar_wait_abortable(full + 8 * (s % kRingSlots), (s / kRingSlots) & 1u, abort_flag)) { okw = false; break; }
+            if (!ptx::warp_wait(full + 8 * (s % kRingSlots), (s / kRingSlots) & 1u, abort_flag)) { okw = false; break; }
           }
           if (!okw) break;
           ptx::tc_fence_after();
@@ -371,7 +372,7 @@ __global__ void __launch_bounds__(kThreads, 1) stem_pool_kernel(const __grid_con
           for (int xt = 0; xt < p.x_tiles && okw; ++xt, ++acc_cnt) {
             if ((acc_cnt & 1u) != issuer) continue;
             const uint32_t ab = acc_cnt % kAcc;
-            if (!ptx::mbar_wait_abortable(acc_empty + 8 * ab, ((acc_cnt / kAcc) & 1u) ^ 1u, abort_flag)) { okw = false; break; }
+            if (!ptx::warp_wait(acc_empty + 8 * ab, ((acc_cnt / kAcc) & 1u) ^ 1u, abort_flag)) { okw = false; break; }
             ptx::tc_fence_after();
             uint32_t accumulate = 0;
             {
@@ -383,17 +384,17 @@ __global__ void __launch_bounds__(kThreads, 1) stem_pool_kernel(const __grid_con
 #pragma unroll
               for (int k2 = 0; k2 < 2; ++k2) {
                 ptx::umma_f16(tmem_base + ab * 64, desc_noswz(a_addr + k2 * 32, 16, 128),
-                              desc_noswz(b_addr + k2 * 2048, 1024, 128), idesc, accumulate);
+                              desc_noswz(b_addr + k2 * 2048, 1024, 128), idesc, accumulate, issue);
                 accumulate = 1;
               }
             }
             }
-            ptx::tc_commit(acc_full + 8 * ab);
+            ptx::tc_commit(acc_full + 8 * ab, issue);
           }
         }
         seq_base += (uint32_t)(ir1 - ir0 + 1);
       }
-      if (!okw && p.error_flag) atomicCAS(p.error_flag, 0, (int)kErrWaitMma);
+      if (!okw && lane == 0 && p.error_flag) atomicCAS(p.error_flag, 0, (int)kErrWaitMma);
     }
   } else if (warp >= 2 && warp < 2 + kEpiWarps) {
     // ---------------------------------------------------------------- epilogue ---------
@@ -569,6 +570,8 @@ __global__ void __launch_bounds__(kThreads, 1) stem_pool_kernel(const __grid_con
 template <typename SrcT, typename DstT>
 __global__ void nchw_to_stem_rows_kernel(const SrcT* __restrict__ src, DstT* __restrict__ dst, int N,
                                          int H, int W, int RW, bool paired) {
+  ptx::grid_dependency_wait();
+  ptx::grid_launch_dependents();
   const long long total = (long long)N * H * RW;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total;
        i += (long long)gridDim.x * blockDim.x) {
@@ -600,6 +603,8 @@ __global__ void nchw_to_stem_rows_kernel(const SrcT* __restrict__ src, DstT* __r
 template <typename SrcT, typename DstT>
 __global__ void nchw_to_stem_rows8_kernel(const SrcT* __restrict__ src, DstT* __restrict__ dst, int N,
                                           int H, int W, int RW) {
+  ptx::grid_dependency_wait();
+  ptx::grid_launch_dependents();
   const int gw = W / 8;
   const long long total = (long long)N * H * gw;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total;
@@ -638,6 +643,8 @@ __global__ void nchw_to_stem_rows8_kernel(const SrcT* __restrict__ src, DstT* __
 template <typename SrcT, typename DstT>
 __global__ void nchw_to_stem_pairs2_kernel(const SrcT* __restrict__ src, DstT* __restrict__ dst, int N,
                                            int H, int W, int RW) {
+  ptx::grid_dependency_wait();
+  ptx::grid_launch_dependents();
   const int cw = RW;                       // chunks per row pair: RW / 2 per row, two rows
   const long long total = (long long)N * (H / 2) * cw;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total;
@@ -682,6 +689,8 @@ __global__ void nchw_to_stem_pairs2_kernel(const SrcT* __restrict__ src, DstT* _
 template <typename SrcT, typename DstT>
 __global__ void nchw_to_stem_pairs4_kernel(const SrcT* __restrict__ src, DstT* __restrict__ dst, int N,
                                            int H, int W, int RW) {
+  ptx::grid_dependency_wait();
+  ptx::grid_launch_dependents();
   const int gw = RW / 2;                   // threads per row pair: RW / 4 per row, two rows
   const long long total = (long long)N * (H / 2) * gw;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total;
@@ -810,30 +819,30 @@ cudaError_t launch_nchw_to_stem_rows(const void* src, DType src_dt, void* dst, D
       long long b4 = ((long long)N * (H / 2) * (RW / 2) + 255) / 256;
       if (b4 > 148LL * 32) b4 = 148LL * 32;
       if (dst_dt == kBF16)
-        nchw_to_stem_pairs4_kernel<S, __nv_bfloat16><<<(int)b4, 256, 0, stream>>>(
+        launch_pdl(nchw_to_stem_pairs4_kernel<S, __nv_bfloat16>, dim3((int)b4), dim3(256), 0, stream,
             static_cast<const S*>(src), static_cast<__nv_bfloat16*>(dst), N, H, W, RW);
       else
-        nchw_to_stem_pairs4_kernel<S, __half><<<(int)b4, 256, 0, stream>>>(
+        launch_pdl(nchw_to_stem_pairs4_kernel<S, __half>, dim3((int)b4), dim3(256), 0, stream,
             static_cast<const S*>(src), static_cast<__half*>(dst), N, H, W, RW);
     } else if (fast && paired) {
       if (dst_dt == kBF16)
-        nchw_to_stem_pairs2_kernel<S, __nv_bfloat16><<<(int)blocks, 256, 0, stream>>>(
+        launch_pdl(nchw_to_stem_pairs2_kernel<S, __nv_bfloat16>, dim3((int)blocks), dim3(256), 0, stream,
             static_cast<const S*>(src), static_cast<__nv_bfloat16*>(dst), N, H, W, RW);
       else
-        nchw_to_stem_pairs2_kernel<S, __half><<<(int)blocks, 256, 0, stream>>>(
+        launch_pdl(nchw_to_stem_pairs2_kernel<S, __half>, dim3((int)blocks), dim3(256), 0, stream,
             static_cast<const S*>(src), static_cast<__half*>(dst), N, H, W, RW);
     } else if (fast) {
       if (dst_dt == kBF16)
-        nchw_to_stem_rows8_kernel<S, __nv_bfloat16><<<(int)blocks, 256, 0, stream>>>(
+        launch_pdl(nchw_to_stem_rows8_kernel<S, __nv_bfloat16>, dim3((int)blocks), dim3(256), 0, stream,
             static_cast<const S*>(src), static_cast<__nv_bfloat16*>(dst), N, H, W, RW);
       else
-        nchw_to_stem_rows8_kernel<S, __half><<<(int)blocks, 256, 0, stream>>>(
+        launch_pdl(nchw_to_stem_rows8_kernel<S, __half>, dim3((int)blocks), dim3(256), 0, stream,
             static_cast<const S*>(src), static_cast<__half*>(dst), N, H, W, RW);
     } else if (dst_dt == kBF16) {
-      nchw_to_stem_rows_kernel<S, __nv_bfloat16><<<(int)blocks, 256, 0, stream>>>(
+      launch_pdl(nchw_to_stem_rows_kernel<S, __nv_bfloat16>, dim3((int)blocks), dim3(256), 0, stream,
           static_cast<const S*>(src), static_cast<__nv_bfloat16*>(dst), N, H, W, RW, paired);
     } else {
-      nchw_to_stem_rows_kernel<S, __half><<<(int)blocks, 256, 0, stream>>>(
+      launch_pdl(nchw_to_stem_rows_kernel<S, __half>, dim3((int)blocks), dim3(256), 0, stream,
           static_cast<const S*>(src), static_cast<__half*>(dst), N, H, W, RW, paired);
     }
     return cudaGetLastError();

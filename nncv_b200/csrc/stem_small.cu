@@ -57,6 +57,8 @@ __global__ void __launch_bounds__(256) stem3x3_kernel(const TI* __restrict__ src
                                                       const float* __restrict__ scale, const float* __restrict__ shift,
                                                       void* __restrict__ dst, Layout ol, int N, int H, int W, int OH, int OW, int Cout,
                                                       int stride, int pad, int act) {
+  ptx::grid_dependency_wait();
+  ptx::grid_launch_dependents();
   extern __shared__ __align__(16) float sw[];     // [27][Cout] filter, [Cout] scale, [Cout] shift
   float* ssc = sw + 27 * Cout;
   float* ssh = ssc + Cout;
@@ -155,7 +157,7 @@ cudaError_t launch_stem3x3(const void* src, DType src_dt, const float* w, const 
   if (blocks > 148 * 16) blocks = 148 * 16;
   const size_t smem = (size_t)29 * Cout * sizeof(float);
 #define NNCV_ST(TI, BF) \
-  stem3x3_kernel<TI, BF><<<(unsigned)blocks, 256, smem, st>>>((const TI*)src, w, scale, shift, dst, out_l, N, H, W, OH, OW, Cout, stride, pad, act)
+  launch_pdl(stem3x3_kernel<TI, BF>, dim3((unsigned)blocks), dim3(256), smem, st, (const TI*)src, w, scale, shift, dst, out_l, N, H, W, OH, OW, Cout, stride, pad, act)
   if (src_dt == kF32) { if (dt == kBF16) NNCV_ST(float, true); else NNCV_ST(float, false); }
   else { if (dt == kBF16) NNCV_ST(__half, true); else NNCV_ST(__half, false); }
 #undef NNCV_ST

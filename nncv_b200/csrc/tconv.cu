@@ -59,6 +59,7 @@ struct TcParams {
   epi::FastDiv div_tx, div_ty, div_nt;   // by tiles_x, tiles_y, n_tiles
   int stages;                // A (+ streamed weight) ring depth
   int relu, bf16, out_f32;
+  int w_ready;    // the packed weights were complete before this launch (not written by earlier work of its stream)
   int residual;   // tm_res holds a tensor of the output's layout and type, added before the activation
   int epi_bufs;   // staging buffers per epilogue warp (1 .. epi::kMaxBufs)
   int act;   // 0, or kActHardSwish / kActSilu applied after the residual add (16-bit outputs)
@@ -118,7 +119,7 @@ tconv_kernel(const __grid_constant__ CUtensorMap tm_in, const __grid_constant__ 
     }
   }
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = ptx::warp_uniform((int)threadIdx.x >> 5), lane = threadIdx.x & 31;
   const uint32_t rank = PAIR ? ptx::cluster_ctarank() : 0u;   // 0 = leader
   if (threadIdx.x == 0) {
     s_abort = 0;
@@ -152,11 +153,7 @@ tconv_kernel(const __grid_constant__ CUtensorMap tm_in, const __grid_constant__ 
   __syncthreads();
   if (PAIR) ptx::cluster_sync_all();   // both CTAs' barriers exist before anyone arrives remotely
   ptx::tc_fence_after();
-  const uint32_t tmem_base = *reinterpret_cast<volatile uint32_t*>(smem_raw + (tmem_slot - raw));
-  // The prologue above touched nothing the previous kernel of the stream writes; everything
-  // below may, so wait for that kernel here and let the next one start its own prologue.
-  ptx::grid_dependency_wait();
-  ptx::grid_launch_dependents();
+  const uint32_t tmem_base = (uint32_t)ptx::warp_uniform(*reinterpret_cast<volatile int*>(smem_raw + (tmem_slot - raw)));
   volatile int* abort_flag = &s_abort;
 
   // Resident weights pin a CTA to one Kout tile (blockIdx.y); otherwise the CTA strides over
@@ -188,19 +185,48 @@ tconv_kernel(const __grid_constant__ CUtensorMap tm_in, const __grid_constant__ 
     return true;
   };
 
+  // Packed weights are the plan's own and nobody writes them once they are made, so their copies start before the previous
+  // kernel of the stream has finished: everything the ring holds.  At small batches, where a kernel leaves most SMs idle,
+  // that hides the whole weight fetch behind the previous layer.
+  auto weight_tile = [&](int n_tile, int cb, int tap) {
+    // pair: the weights are packed for N tile BN/2; this CTA takes tile 2 * n_tile + rank
+    const int wt = PAIR ? 2 * n_tile + (int)rank : n_tile;
+    return (DUAL && tap == p.taps) ? p.wpack2 + ((size_t)wt * p.CB + cb) * WTILE
+                                   : p.wpack + ((size_t)wt * KB + (size_t)tap * p.CB + cb) * WTILE;
+  };
+  uint32_t early = 0;   // ring stages whose weights are on their way
+  auto load_resident = [&]() {
+    const uint8_t* src = p.wpack + (size_t)blockIdx.y * KB * WTILE;
+    ptx::mbar_arrive_expect_tx(w_full, (uint32_t)(KB + (DUAL ? p.CB : 0)) * WTILE);
+    for (int i = 0; i < KB; ++i) ptx::bulk_g2s(sW + (uint32_t)i * WTILE, src + (size_t)i * WTILE, WTILE, w_full);
+    if (DUAL) {
+      const uint8_t* src2 = p.wpack2 + (size_t)blockIdx.y * p.CB * WTILE;
+      for (int i = 0; i < p.CB; ++i) ptx::bulk_g2s(sW + (uint32_t)(KB + i) * WTILE, src2 + (size_t)i * WTILE, WTILE, w_full);
+    }
+  };
+  if (warp == 0 && lane == 0 && !BROW && p.w_ready) {
+    if (RESIDENT) {
+      load_resident();
+    } else {
+      for (int i = 0; early < (uint32_t)p.stages; ++i) {
+        int n0, oy0, ox0, n_tile;
+        if (!item_of(i, n0, oy0, ox0, n_tile)) break;
+        for (int cb = 0; cb < p.CB && early < (uint32_t)p.stages; ++cb)
+          for (int tap = 0; tap < taps_x && early < (uint32_t)p.stages; ++tap, ++early) {
+            ptx::mbar_arrive_expect_tx(full + 8 * early, (uint32_t)stage_bytes);
+            ptx::bulk_g2s(sRing + early * stage_bytes + kABytes, weight_tile(n_tile, cb, tap), WTILE, full + 8 * early);
+          }
+      }
+    }
+  }
+  // The rest reads what the previous kernel wrote, or writes what it may still be reading.
+  ptx::grid_dependency_wait();
+  ptx::grid_launch_dependents();
+
   if (warp == 0) {
     // ------------------------------------------------------------------ TMA producer ----
     if (lane == 0) {
-      if (RESIDENT) {
-        const uint8_t* src = p.wpack + (size_t)blockIdx.y * KB * WTILE;
-        ptx::mbar_arrive_expect_tx(w_full, (uint32_t)(KB + (DUAL ? p.CB : 0)) * WTILE);
-        for (int i = 0; i < KB; ++i) ptx::bulk_g2s(sW + (uint32_t)i * WTILE, src + (size_t)i * WTILE, WTILE, w_full);
-        if (DUAL) {
-          const uint8_t* src2 = p.wpack2 + (size_t)blockIdx.y * p.CB * WTILE;
-          for (int i = 0; i < p.CB; ++i)
-            ptx::bulk_g2s(sW + (uint32_t)(KB + i) * WTILE, src2 + (size_t)i * WTILE, WTILE, w_full);
-        }
-      }
+      if (RESIDENT && !p.w_ready) load_resident();
       uint32_t cnt = 0;
       bool okw = true;
       for (int i = 0; okw; ++i) {
@@ -214,22 +240,21 @@ tconv_kernel(const __grid_constant__ CUtensorMap tm_in, const __grid_constant__ 
             const int gtap = tap < p.taps ? tap : p.taps / 2;   // the extra tap re-reads the centre tap's pixels
             const int r = gtap / p.S, s = gtap - r * p.S;
             const uint32_t st = cnt % (uint32_t)p.stages;
-            const bool freed = PAIR ? ptx::mbar_wait_cluster_abortable(empty + 8 * st, ((cnt / (uint32_t)p.stages) & 1u) ^ 1u, abort_flag)
-                                    : ptx::mbar_wait_abortable(empty + 8 * st, ((cnt / (uint32_t)p.stages) & 1u) ^ 1u, abort_flag);
-            if (!freed) { okw = false; break; }
-            ptx::mbar_arrive_expect_tx(full + 8 * st, (uint32_t)stage_bytes);
+            const bool begun = cnt < early;   // this stage's first use: weights already issued
+            if (!begun) {
+              const bool freed = PAIR ? ptx::mbar_wait_cluster_abortable(empty + 8 * st, ((cnt / (uint32_t)p.stages) & 1u) ^ 1u, abort_flag)
+                                      : ptx::mbar_wait_abortable(empty + 8 * st, ((cnt / (uint32_t)p.stages) & 1u) ^ 1u, abort_flag);
+              if (!freed) { okw = false; break; }
+              ptx::mbar_arrive_expect_tx(full + 8 * st, (uint32_t)stage_bytes);
+            }
             const uint32_t dst = sRing + st * stage_bytes;
             ptx::tma_load_4d(dst, &tm_in, cb * 64, xb + s, yb + r, n0, full + 8 * st);
             if (BROW) {
 #pragma unroll
               for (int j = 0; j < BN / 64; ++j)
                 ptx::tma_load_2d(dst + kABytes + (uint32_t)j * 8192u, &tm_b, n_tile * BN + j * 64, cb * 64, full + 8 * st);
-            } else if (!RESIDENT) {
-              // pair: the weights are packed for N tile BN/2; this CTA takes tile 2 * n_tile + rank
-              const int wt = PAIR ? 2 * n_tile + (int)rank : n_tile;
-              const uint8_t* wsrc = (DUAL && tap == p.taps) ? p.wpack2 + ((size_t)wt * p.CB + cb) * WTILE
-                                                             : p.wpack + ((size_t)wt * KB + (size_t)tap * p.CB + cb) * WTILE;
-              ptx::bulk_g2s(dst + kABytes, wsrc, WTILE, full + 8 * st);
+            } else if (!RESIDENT && !begun) {
+              ptx::bulk_g2s(dst + kABytes, weight_tile(n_tile, cb, tap), WTILE, full + 8 * st);
             }
           }
         }
@@ -258,65 +283,52 @@ tconv_kernel(const __grid_constant__ CUtensorMap tm_in, const __grid_constant__ 
       }
     } else
     // ------------------------------------------------------------------ MMA issuer ------
-    if (lane == 0) {
+    {
+      const uint32_t issue = ptx::elect_one();
       const uint32_t idesc = ptx::umma_idesc(PAIR ? 256 : 128, BN, p.bf16 ? 1 : 0) | (BROW ? (1u << 16) : 0u);   // bit 16: B is MN-major
-      const uint32_t peer_empty = PAIR ? ptx::map_to_cta(empty, 1) : 0u, peer_acc_full = PAIR ? ptx::map_to_cta(acc_full, 1) : 0u;
+      auto wait = [&](uint32_t bar, uint32_t parity) {
+        return PAIR ? ptx::warp_wait_cluster(bar, parity, abort_flag) : ptx::warp_wait(bar, parity, abort_flag);
+      };
       bool okw = true;
-      if (RESIDENT) okw = ptx::mbar_wait_abortable(w_full, 0, abort_flag);
-      uint32_t cnt = 0, acc_cnt = 0;
+      if (RESIDENT) okw = ptx::warp_wait(w_full, 0, abort_flag);
+      uint32_t st = 0, ring = 0, acc_cnt = 0;   // stage, parity of the ring's round
       for (int i = 0; okw; ++i) {
         int n0, oy0, ox0, n_tile;
         if (!item_of(i, n0, oy0, ox0, n_tile)) break;
         const uint32_t ab = acc_cnt & 1u;
-        const bool drained = PAIR ? ptx::mbar_wait_cluster_abortable(acc_empty + 8 * ab, ((acc_cnt >> 1) & 1u) ^ 1u, abort_flag)
-                                  : ptx::mbar_wait_abortable(acc_empty + 8 * ab, ((acc_cnt >> 1) & 1u) ^ 1u, abort_flag);
-        if (!drained) { okw = false; break; }
+        if (!wait(acc_empty + 8 * ab, ((acc_cnt >> 1) & 1u) ^ 1u)) { okw = false; break; }
         ptx::tc_fence_after();
         const uint32_t d = tmem_base + ab * ACC_W;
-        const int KBX = taps_x * p.CB;
-        for (int kb = 0; kb < KBX; ++kb, ++cnt) {
-          const int cb = kb / taps_x, tap = kb - cb * taps_x;   // producer order: cb outer, tap inner
-          const bool second = DUAL && tap == p.taps;
-          const uint32_t st = cnt % (uint32_t)p.stages;
-          const bool landed = PAIR ? ptx::mbar_wait_cluster_abortable(full + 8 * st, (cnt / (uint32_t)p.stages) & 1u, abort_flag)
-                                   : ptx::mbar_wait_abortable(full + 8 * st, (cnt / (uint32_t)p.stages) & 1u, abort_flag);
-          if (!landed) { okw = false; break; }
-          ptx::tc_fence_after();
-          const uint32_t a_addr = sRing + st * stage_bytes;
-          const uint32_t a_lo = ptx::smem_desc_k128_lo(a_addr);
-          // MN-major B: leading-dimension offset 8192 bytes (next 64 columns), one k step of 16 = two 8-row groups
-          const uint32_t b_lo = BROW ? ((((a_addr + kABytes) & 0x3FFFFu) >> 4) | ((8192u >> 4) << 16))
-                                     : ptx::smem_desc_k128_lo(
-              RESIDENT ? sW + (uint32_t)(second ? KB + cb : tap * p.CB + cb) * WTILE : a_addr + kABytes);
-          constexpr uint32_t kBStep = BROW ? (2048u >> 4) : 2u;
+        for (int cb = 0; cb < p.CB && okw; ++cb)
+          for (int tap = 0; tap < taps_x; ++tap) {   // producer order: cb outer, tap inner
+            const bool second = DUAL && tap == p.taps;
+            if (!wait(full + 8 * st, ring)) { okw = false; break; }
+            ptx::tc_fence_after();
+            const uint32_t a_addr = sRing + st * stage_bytes;
+            const uint32_t a_lo = ptx::smem_desc_k128_lo(a_addr);
+            // MN-major B: leading-dimension offset 8192 bytes (next 64 columns), one k step of 16 = two 8-row groups
+            const uint32_t b_lo = BROW ? ((((a_addr + kABytes) & 0x3FFFFu) >> 4) | ((8192u >> 4) << 16))
+                                       : ptx::smem_desc_k128_lo(
+                RESIDENT ? sW + (uint32_t)(second ? KB + cb : tap * p.CB + cb) * WTILE : a_addr + kABytes);
+            constexpr uint32_t kBStep = BROW ? (2048u >> 4) : 2u;
+            const uint32_t first = second ? (uint32_t)cb : (uint32_t)(cb | tap);
 #pragma unroll
-          for (int k4 = 0; k4 < 4; ++k4) {
-            if (PAIR)
-              ptx::umma_f16_pair(second ? d + BN : d, ptx::desc_from_halves(a_lo + k4 * 2, ptx::kSmemDescK128Hi),
-                                 ptx::desc_from_halves(b_lo + k4 * 2, ptx::kSmemDescK128Hi), idesc,
-                                 (second ? (cb | k4) : (cb | tap | k4)) != 0 ? 1u : 0u);
-            else
-              ptx::umma_f16(second ? d + BN : d, ptx::desc_from_halves(a_lo + k4 * 2, ptx::kSmemDescK128Hi),
-                            ptx::desc_from_halves(b_lo + k4 * kBStep, ptx::kSmemDescK128Hi), idesc,
-                            (second ? (cb | k4) : (cb | tap | k4)) != 0 ? 1u : 0u);
+            for (uint32_t k4 = 0; k4 < 4; ++k4) {
+              const uint64_t da = ptx::desc_from_halves(a_lo + k4 * 2, ptx::kSmemDescK128Hi);
+              const uint64_t db = ptx::desc_from_halves(b_lo + k4 * kBStep, ptx::kSmemDescK128Hi);
+              if (PAIR) ptx::umma_f16_pair(second ? d + BN : d, da, db, idesc, first | k4, issue);
+              else ptx::umma_f16(second ? d + BN : d, da, db, idesc, first | k4, issue);
+            }
+            if (PAIR) ptx::tc_commit_pair(empty + 8 * st, issue);
+            else ptx::tc_commit(empty + 8 * st, issue);
+            if (++st == (uint32_t)p.stages) { st = 0; ring ^= 1u; }
           }
-          if (PAIR) {
-            ptx::tc_commit_pair(empty + 8 * st);
-            ptx::tc_commit_pair(peer_empty + 8 * st);
-          } else {
-            ptx::tc_commit(empty + 8 * st);
-          }
-        }
         if (!okw) break;
-        if (PAIR) {
-          ptx::tc_commit_pair(acc_full + 8 * ab);
-          ptx::tc_commit_pair(peer_acc_full + 8 * ab);
-        } else {
-          ptx::tc_commit(acc_full + 8 * ab);
-        }
+        if (PAIR) ptx::tc_commit_pair(acc_full + 8 * ab, issue);
+        else ptx::tc_commit(acc_full + 8 * ab, issue);
         ++acc_cnt;
       }
-      if (!okw && p.error_flag) atomicCAS(p.error_flag, 0, (int)kErrWaitMma);
+      if (!okw && lane == 0 && p.error_flag) atomicCAS(p.error_flag, 0, (int)kErrWaitMma);
     }
   } else {
     // ------------------------------------------------------------------ epilogue --------
@@ -651,6 +663,7 @@ cudaError_t launch_tconv(const TconvArgs& a, cudaStream_t stream) {
   p.div_nt = epi::fast_div((uint32_t)p.n_tiles);
   p.relu = a.relu; p.bf16 = a.ab == kBF16; p.out_f32 = a.out_dtype == kF32;
   p.act = a.act;
+  p.w_ready = a.weights_ready;
   p.stages = 0;
   if (p.residual && p.out_f32) return cudaErrorInvalidValue;
   if (brow) {
