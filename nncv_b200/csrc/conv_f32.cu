@@ -1,0 +1,761 @@
+// fp32 convolutions on the tensor cores: implicit GEMM over THREE bf16 PLANES per operand.
+//
+// Every fp32 value x is kept as x = x1 + x2 + x3, three bf16 numbers, each the nearest to what the ones before leave; with
+// 8 significand bits each and signed remainders the sum is exact.  A product is then six bf16 products with fp32
+// accumulation,
+//     a*b ~= a1*b1 + (a1*b2 + a2*b1) + a2*b2 + (a1*b3 + a3*b1),
+// and what is dropped (a2*b3, a3*b2, a3*b3) is below 2^-26 of the product: less than the rounding of ONE fp32 multiply.
+// (Two tf32 parts, the other way to do this, keep 22 of the 24 bits, take as much tensor time -- three products at half
+// the rate -- and 8 bytes an element instead of 6.)
+// tcgen05.mma cuts every accumulation to fp32 instead of rounding it, an error of one sign per step.  So the products stay in
+// TMEM for ONE block of 64 channels (four steps of the large products a1*b1, twenty of the small ones, which have an
+// accumulator of their own) before the epilogue warps add them, rounded, to a sum in registers: logits of ResNet-18 are
+// within 4.9e-7 of the fp64-accumulated oracle (the CUDA-core kernel's: 2.3e-7; with four blocks a promotion: 1.1e-6).
+//
+// Activations between the layers of an fp32 network are stored as planes, [3][N][H][W][C] bf16: the epilogue splits each
+// result once, and the tile loads are plain TMA copies of all three planes (nncv's fp32 graph: tests/Nets/Res18.mlir:118-629).
+// The 7x7 stride-2 stem reads row pairs through a tensor map with overlapping strides, as stem.cu does: it becomes a
+// convolution with four taps of 64 "channels".
+//
+// One CTA computes 128 pixels x 64 or 128 output channels.  What bounds it: 72 or 96 KB of planes from L2 per block of 64
+// channels (1960 or 2700 clocks at what all SMs together get), then the 24 MMAs (1150 or 1540 clocks).  With few pixels (batch 1) a
+// cluster of up to eight CTAs splits the reduction of a tile; each leaves its partial sums in shared memory and finishes
+// its share of the rows from all of them, in rank order, so that the result does not depend on timing.  (The CUDA-core
+// kernel needed a second pass over partial sums in global memory for that, and ran at a fifth of the fp32 rate.)
+//
+// ResNet-18 fp32 from host memory: 1x256 571 -> 337 us, 8x224 1945 -> 791 us.
+// Roles: warp 0 TMA producer, one plane of both operands per ring slot; warp 1 MMA issuer; warps 2-9 epilogue.
+// Every wait is bounded and abortable; a timed-out wait sets the device status word.
+#include <cuda.h>
+#include <cudaTypedefs.h>
+#include <cuda_bf16.h>
+#include <cuda_runtime.h>
+
+#include <cfloat>
+#include <mutex>
+
+#include "epilogue.cuh"
+#include "kernels.h"
+#include "ptx.cuh"
+
+namespace nncv_b200 {
+
+namespace {
+
+constexpr int kEpiThreads = epi::kThreads;
+constexpr int kThreads = 64 + kEpiThreads;
+constexpr int kABytes = 128 * 128;
+constexpr int kBBytes = 64 * 128;           // packed weights: tiles of 64 output channels x 64 input channels
+constexpr int kTileBytes = 128 * 64 * 4;    // partial sums of 64 of the tile's columns, fp32
+template <int BN>
+struct Ring {   // a slot holds one plane of a block: 128 pixels and BN output channels x 64 channels
+  static constexpr int kSlots = BN == 64 ? 7 : 5;
+  static constexpr int kSlot = kABytes + BN / 64 * kBBytes;
+  static constexpr size_t kSmem = 1024 + (size_t)kSlots * kSlot + kTileBytes + 256;
+};
+
+struct F32Params {
+  const uint8_t* wpack;       // [Kout tile][plane][k block] 64 x 64 bf16 tiles, swizzled
+  const float* scale;
+  const float* shift;
+  const void* residual;       // planes (res_f32: fp32) of the output's shape, or null
+  void* out;                  // planes, or fp32 with row pitch ldo
+  long long res_plane, out_plane;  // elements from one plane to the next
+  long long ldo;
+  int* error_flag;
+  int out_f32, res_f32, relu;
+  int Kout, CB, taps, S, stride, pad_x, pad_y;
+  int OH, OW, NB;
+  int tw, th;
+  int tn, tiles_x, tiles_y, n_tiles, items;
+  epi::FastDiv div_tx, div_ty, div_nt, div_tw, div_th;
+  int splits;                 // CTAs of a cluster that share a tile's reduction (a power of two up to 8)
+};
+
+__device__ __forceinline__ void split3(float x, __nv_bfloat16& a, __nv_bfloat16& b, __nv_bfloat16& c) {
+  a = __float2bfloat16_rn(x);
+  const float h = __bfloat162float(a);
+  const float r = fabsf(h) <= FLT_MAX ? x - h : 0.0f;   // infinities and NaN stay in the first plane
+  b = __float2bfloat16_rn(r);
+  c = __float2bfloat16_rn(r - __bfloat162float(b));
+}
+// four values -> 8 bytes of each plane
+__device__ __forceinline__ void split4(const float4& v, uint2 (&o)[3]) {
+  const float x[4] = {v.x, v.y, v.z, v.w};
+  __nv_bfloat16 s[3][4];
+#pragma unroll
+  for (int e = 0; e < 4; ++e) split3(x[e], s[0][e], s[1][e], s[2][e]);
+#pragma unroll
+  for (int q = 0; q < 3; ++q) o[q] = *reinterpret_cast<const uint2*>(s[q]);
+}
+__device__ __forceinline__ float4 join4(const uint2 (&w)[3]) {
+  float4 v;
+  float* f = reinterpret_cast<float*>(&v);
+#pragma unroll
+  for (int e = 0; e < 4; ++e) {
+    float p[3];
+#pragma unroll
+    for (int q = 0; q < 3; ++q) {
+      const uint32_t u = (e & 2) ? w[q].y : w[q].x;
+      p[q] = __uint_as_float((e & 1) ? (u & 0xffff0000u) : (u << 16));
+    }
+    f[e] = p[0] + (p[1] + p[2]);
+  }
+  return v;
+}
+
+template <int kBN>   // output channels of a tile: 64 or 128
+__global__ void __launch_bounds__(kThreads, 1)
+conv_f32_kernel(const __grid_constant__ CUtensorMap tm_in, const F32Params p) {
+  constexpr int kSlots = Ring<kBN>::kSlots, kSlot = Ring<kBN>::kSlot, kNT = kBN / 64;
+  constexpr uint32_t kTmemCols = 4 * kBN;   // two buffers of two accumulators (large and small products)
+  constexpr int kCols = kBN / 2;            // columns of a thread's row
+  extern __shared__ uint8_t smem_raw[];
+  __shared__ int s_abort;
+  __shared__ __align__(8) unsigned long long s_bars[2 * kSlots + 2 + 2 + 2];
+  const uint32_t raw = ptx::smem_u32(smem_raw);
+  const uint32_t sRing = (raw + 1023u) & ~1023u;
+  const uint32_t sTile = sRing + kSlots * kSlot;
+  const uint32_t full = ptx::smem_u32(s_bars), empty = full + 8 * kSlots;
+  const uint32_t d_full = empty + 8 * kSlots, d_empty = d_full + 16;
+  const uint32_t part_ready = d_empty + 16, part_done = part_ready + 8;
+  __shared__ uint32_t s_tmem;
+  const int warp = ptx::warp_uniform((int)threadIdx.x >> 5), lane = threadIdx.x & 31;
+  const int S = p.splits;
+  const uint32_t rank = S > 1 ? ptx::cluster_ctarank() : 0u;
+
+  if (threadIdx.x == 0) {
+    s_abort = 0;
+    for (int i = 0; i < kSlots; ++i) {
+      ptx::mbar_init(full + 8 * i, 1);
+      ptx::mbar_init(empty + 8 * i, 1);
+    }
+    for (int i = 0; i < 2; ++i) {
+      ptx::mbar_init(d_full + 8 * i, 1);
+      ptx::mbar_init(d_empty + 8 * i, epi::kWarps);
+    }
+    ptx::mbar_init(part_ready, S);
+    ptx::mbar_init(part_done, S);
+    ptx::mbar_fence_init();
+    ptx::prefetch_tensormap(&tm_in);
+  }
+  if (warp == 1) {
+    ptx::tmem_alloc(ptx::smem_u32(&s_tmem), kTmemCols);
+    ptx::tmem_relinquish();
+  }
+  ptx::tc_fence_before();
+  __syncthreads();
+  if (S > 1) ptx::cluster_sync_all();   // every CTA's barriers exist before anyone arrives remotely
+  ptx::tc_fence_after();
+  const uint32_t tmem_base = (uint32_t)ptx::warp_uniform((int)*reinterpret_cast<volatile uint32_t*>(&s_tmem));
+  volatile int* abort_flag = &s_abort;
+
+  const int cluster_id = (int)blockIdx.x / S, clusters = (int)gridDim.x / S;
+  const int kb_all = p.taps * p.CB;
+  const int kb0 = kb_all * (int)rank / S, kb1 = kb_all * ((int)rank + 1) / S;   // this CTA's part of the reduction
+  auto item_of = [&](int i, int& n0, int& oy0, int& ox0, int& n_tile) {
+    const int w = cluster_id + i * clusters;
+    if (w >= p.items) return false;
+    const int m = (int)epi::div_by((uint32_t)w, p.div_nt);
+    n_tile = w - m * p.n_tiles;
+    const int t2 = (int)epi::div_by((uint32_t)m, p.div_tx);
+    ox0 = (m - t2 * p.tiles_x) * p.tw;
+    const int t3 = (int)epi::div_by((uint32_t)t2, p.div_ty);
+    oy0 = (t2 - t3 * p.tiles_y) * p.th;
+    n0 = t3 * p.tn;
+    return true;
+  };
+  // block kb of the reduction: channel block outermost, then the taps
+  const int packed_tiles = (p.Kout + 63) / 64;
+  auto load_weights = [&](int n_tile, int plane, int kb, uint32_t slot) {
+    const int cb = kb / p.taps, tap = kb - cb * p.taps;
+#pragma unroll
+    for (int q = 0; q < kNT; ++q) {
+      // the second half of the last, ragged tile has no weights: its columns are never stored, any tile will do
+      const int t = min(n_tile * kNT + q, packed_tiles - 1);
+      ptx::bulk_g2s(sRing + slot * kSlot + kABytes + q * kBBytes,
+                    p.wpack + (((size_t)t * 3 + plane) * kb_all + (size_t)tap * p.CB + cb) * kBBytes, kBBytes, full + 8 * slot);
+    }
+  };
+  // the packed weights never change: their first copies do not wait for the previous kernel
+  uint32_t early = 0;
+  if (warp == 0 && lane == 0) {
+    int n0, oy0, ox0, n_tile;
+    if (item_of(0, n0, oy0, ox0, n_tile))
+      for (int kb = kb0; kb < kb1 && early < (uint32_t)kSlots; ++kb)
+        for (int pl = 0; pl < 3 && early < (uint32_t)kSlots; ++pl, ++early) {
+          ptx::mbar_arrive_expect_tx(full + 8 * early, kSlot);
+          load_weights(n_tile, pl, kb, early);
+        }
+  }
+  ptx::grid_dependency_wait();
+  ptx::grid_launch_dependents();
+
+  if (warp == 0) {
+    // ------------------------------------------------------------------ TMA producer ----
+    if (lane == 0) {
+      uint32_t slot = 0, ring = 0, cnt = 0;
+      bool okw = true;
+      for (int i = 0; okw; ++i) {
+        int n0, oy0, ox0, n_tile;
+        if (!item_of(i, n0, oy0, ox0, n_tile)) break;
+        const int xb = p.stride * ox0 - p.pad_x, yb = p.stride * oy0 - p.pad_y;
+        int cb = kb0 / p.taps, tap = kb0 - cb * p.taps;
+        for (int kb = kb0; kb < kb1 && okw; ++kb) {
+          const int r = tap / p.S, s = tap - r * p.S;
+          for (int pl = 0; pl < 3; ++pl, ++cnt) {
+            const bool begun = cnt < early;
+            if (!begun) {
+              if (!ptx::mbar_wait_abortable(empty + 8 * slot, ring ^ 1u, abort_flag)) { okw = false; break; }
+              ptx::mbar_arrive_expect_tx(full + 8 * slot, kSlot);
+            }
+            const uint32_t dst = sRing + slot * kSlot;
+            ptx::tma_load_5d(dst, &tm_in, cb * 64, xb + s, yb + r, n0, pl, full + 8 * slot);
+            if (!begun) load_weights(n_tile, pl, kb, slot);
+            if (++slot == kSlots) { slot = 0; ring ^= 1u; }
+          }
+          if (++tap == p.taps) { tap = 0; ++cb; }
+        }
+      }
+      if (!okw && p.error_flag) atomicCAS(p.error_flag, 0, (int)kErrWaitProducer);
+    }
+  } else if (warp == 1) {
+    // ------------------------------------------------------------------ MMA issuer ------
+    const uint32_t issue = ptx::elect_one();
+    const uint32_t idesc = ptx::umma_idesc(128, kBN, 1);
+    uint32_t slot = 0, ring = 0, blk = 0;   // blk: running count of blocks; accumulator buffer blk % 2
+    bool okw = true;
+    auto step = [&]() { if (++slot == kSlots) { slot = 0; ring ^= 1u; } };
+    // one product of the block's planes: four k steps of 16
+    auto product = [&](uint32_t d, uint32_t a, uint32_t b, uint32_t fresh) {
+      const uint32_t a_lo = ptx::smem_desc_k128_lo(a), b_lo = ptx::smem_desc_k128_lo(b);
+#pragma unroll
+      for (uint32_t k4 = 0; k4 < 4; ++k4)
+        ptx::umma_f16(d, ptx::desc_from_halves(a_lo + k4 * 2, ptx::kSmemDescK128Hi), ptx::desc_from_halves(b_lo + k4 * 2, ptx::kSmemDescK128Hi),
+                      idesc, k4 == 0 ? (fresh ^ 1u) : 1u, issue);
+    };
+    for (int i = 0; okw; ++i) {
+      int n0, oy0, ox0, n_tile;
+      if (!item_of(i, n0, oy0, ox0, n_tile)) break;
+      for (int kb = kb0; kb < kb1; ++kb, ++blk) {
+        const uint32_t d0 = tmem_base + (blk & 1u) * (2 * kBN), d1 = d0 + kBN;
+        if (!ptx::warp_wait(d_empty + 8 * (blk & 1u), ((blk >> 1) & 1u) ^ 1u, abort_flag)) { okw = false; break; }
+        uint32_t at[3], sl[3];
+#pragma unroll
+        for (int pl = 0; pl < 3; ++pl) {
+          if (okw && !ptx::warp_wait(full + 8 * slot, ring, abort_flag)) okw = false;
+          if (!okw) break;
+          ptx::tc_fence_after();
+          sl[pl] = slot;
+          at[pl] = sRing + slot * kSlot;
+          step();
+          if (pl == 0) {
+            product(d0, at[0], at[0] + kABytes, 1u);
+          } else if (pl == 1) {
+            product(d1, at[0], at[1] + kABytes, 1u);
+            product(d1, at[1], at[0] + kABytes, 0u);
+            product(d1, at[1], at[1] + kABytes, 0u);
+          } else {
+            product(d1, at[0], at[2] + kABytes, 0u);
+            product(d1, at[2], at[0] + kABytes, 0u);
+          }
+        }
+        if (!okw) break;
+#pragma unroll
+        for (int pl = 0; pl < 3; ++pl) ptx::tc_commit(empty + 8 * sl[pl], issue);
+        ptx::tc_commit(d_full + 8 * (blk & 1u), issue);
+      }
+    }
+    if (!okw && lane == 0 && p.error_flag) atomicCAS(p.error_flag, 0, (int)kErrWaitMma);
+  } else {
+    // ------------------------------------------------------------------ epilogue --------
+    const int ew = warp - 2, quad = warp & 3, half = ew >> 2;
+    const int row = quad * 32 + lane;
+    const int et = (int)threadIdx.x - 64;
+    const int rows_each = 128 / S, row_lo = (int)rank * rows_each;
+    const int g = et & 15;             // four columns of the tile
+    uint32_t blk = 0;
+    bool okw = true;
+    for (int i = 0; okw; ++i) {
+      int n0, oy0, ox0, n_tile;
+      if (!item_of(i, n0, oy0, ox0, n_tile)) break;
+      const uint32_t lane_base = tmem_base + ((uint32_t)(quad * 32) << 16) + (uint32_t)(half * kCols);
+      // the pixels this thread finishes: row r of the tile -> its index in the output, -1 outside
+      int pix[8];
+#pragma unroll
+      for (int k = 0; k < 8; ++k) {
+        const int rr = (et >> 4) + k * (kEpiThreads / 16), r = row_lo + rr;
+        const int t1 = (int)epi::div_by((uint32_t)r, p.div_tw), tj = r - t1 * p.tw;
+        const int t2 = (int)epi::div_by((uint32_t)t1, p.div_th), ti = t1 - t2 * p.th;
+        const int img = n0 + t2, oy = oy0 + ti, ox = ox0 + tj;
+        pix[k] = rr < rows_each && img < p.NB && oy < p.OH && ox < p.OW ? (img * p.OH + oy) * p.OW + ox : -1;
+      }
+      auto load_res = [&](int k, int n, uint2 (&w)[3]) {
+#pragma unroll
+        for (int q = 0; q < 3; ++q)
+          w[q] = __ldg(reinterpret_cast<const uint2*>(static_cast<const __nv_bfloat16*>(p.residual) + q * p.res_plane + (long long)pix[k] * p.Kout + n));
+      };
+      const int n_first = n_tile * kBN + (g >> 3) * kCols + 4 * (g & 7);
+      // residual planes, requested before the sums are there (the wide tile needs its registers for the sums)
+      constexpr bool kEarlyRes = kNT == 1;
+      uint2 res[kEarlyRes ? 8 : 1][3];
+      if (kEarlyRes && p.residual && !p.res_f32 && n_first < p.Kout) {
+#pragma unroll
+        for (int k = 0; k < 8; ++k)
+          if (pix[k] >= 0) load_res(k, n_first, res[kEarlyRes ? k : 0]);
+      }
+      float sum[kCols];
+#pragma unroll
+      for (int e = 0; e < kCols; ++e) sum[e] = 0.0f;
+      for (int kb = kb0; kb < kb1; ++kb, ++blk) {
+        okw = ptx::warp_wait(d_full + 8 * (blk & 1u), (blk >> 1) & 1u, abort_flag);
+        if (!okw) break;
+        ptx::tc_fence_after();
+#pragma unroll
+        for (int h = 0; h < kCols / 32; ++h) {
+          uint32_t big[32], small[32];
+          ptx::tmem_ld_32x32(lane_base + (blk & 1u) * (2 * kBN) + h * 32, big);
+          ptx::tmem_ld_32x32(lane_base + (blk & 1u) * (2 * kBN) + kBN + h * 32, small);
+          ptx::tmem_ld_wait();
+          if (h == kCols / 32 - 1) {
+            ptx::tc_fence_before();
+            __syncwarp();
+            if (lane == 0) ptx::mbar_arrive(d_empty + 8 * (blk & 1u));
+          }
+#pragma unroll
+          for (int e = 0; e < 32; ++e) sum[h * 32 + e] += __uint_as_float(big[e]) + __uint_as_float(small[e]);
+        }
+      }
+      // 64 columns at a time: 32 of either half of the tile
+#pragma unroll
+      for (int pass = 0; pass < kNT; ++pass) {
+      const uint32_t turn = (uint32_t)(i * kNT + pass);   // uses of the shared tile
+      const int n = n_first + pass * 32;
+      // the previous item's partial sums have been read by everybody
+      if (okw && turn > 0 && S > 1) okw = ptx::warp_wait_cluster(part_done, (turn - 1) & 1u, abort_flag);
+      if (!ptx::named_bar_and(1, kEpiThreads, okw)) { okw = false; break; }
+#pragma unroll
+      for (int c = 0; c < 8; ++c)
+        epi::sts128(sTile + (uint32_t)row * 256u + (((uint32_t)(half * 8 + c) ^ (uint32_t)(row & 7)) << 4), __float_as_uint(sum[pass * 32 + 4 * c]),
+                    __float_as_uint(sum[pass * 32 + 4 * c + 1]), __float_as_uint(sum[pass * 32 + 4 * c + 2]), __float_as_uint(sum[pass * 32 + 4 * c + 3]));
+      ptx::named_bar_sync(2, kEpiThreads);
+      if (S > 1) {
+        if (et < S) ptx::mbar_arrive_remote(ptx::map_to_cta(part_ready, (uint32_t)et));
+        okw = ptx::warp_wait_cluster(part_ready, turn & 1u, abort_flag);
+        if (!ptx::named_bar_and(1, kEpiThreads, okw)) { okw = false; break; }
+      }
+      if (n < p.Kout) {
+        float4 sc = make_float4(1.f, 1.f, 1.f, 1.f), sh = make_float4(0.f, 0.f, 0.f, 0.f);
+        float* scp = reinterpret_cast<float*>(&sc);
+        float* shp = reinterpret_cast<float*>(&sh);
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          if (p.scale) scp[e] = __ldg(p.scale + n + e);
+          if (p.shift) shp[e] = __ldg(p.shift + n + e);
+        }
+#pragma unroll
+        for (int k = 0; k < 8; ++k) {
+          if (pix[k] < 0) continue;
+          const int r = row_lo + (et >> 4) + k * (kEpiThreads / 16);
+          const uint32_t at = sTile + (uint32_t)r * 256u + (((uint32_t)g ^ (uint32_t)(r & 7)) << 4);
+          float4 v;
+          if (S == 1) {
+            const uint4 w = epi::lds128(at);
+            v = make_float4(__uint_as_float(w.x), __uint_as_float(w.y), __uint_as_float(w.z), __uint_as_float(w.w));
+          } else {
+            v = ptx::ld_cluster_f4(ptx::map_to_cta(at, 0));
+            for (int q = 1; q < S; ++q) {
+              const float4 w = ptx::ld_cluster_f4(ptx::map_to_cta(at, (uint32_t)q));
+              v.x += w.x; v.y += w.y; v.z += w.z; v.w += w.w;
+            }
+          }
+          v.x = fmaf(v.x, sc.x, sh.x); v.y = fmaf(v.y, sc.y, sh.y); v.z = fmaf(v.z, sc.z, sh.z); v.w = fmaf(v.w, sc.w, sh.w);
+          if (p.residual) {
+            float4 f;
+            if (p.res_f32) {
+              f = __ldg(reinterpret_cast<const float4*>(static_cast<const float*>(p.residual) + (long long)pix[k] * p.ldo + n));
+            } else {
+              if (!kEarlyRes) load_res(k, n, res[0]);
+              f = join4(res[kEarlyRes ? k : 0]);
+            }
+            v.x += f.x; v.y += f.y; v.z += f.z; v.w += f.w;
+          }
+          if (p.relu) {
+            v.x = !(v.x <= 0.0f) ? v.x : 0.0f; v.y = !(v.y <= 0.0f) ? v.y : 0.0f;
+            v.z = !(v.z <= 0.0f) ? v.z : 0.0f; v.w = !(v.w <= 0.0f) ? v.w : 0.0f;
+          }
+          if (p.out_f32) {
+            *reinterpret_cast<float4*>(reinterpret_cast<float*>(p.out) + (long long)pix[k] * p.ldo + n) = v;
+          } else {
+            uint2 o[3];
+            split4(v, o);
+#pragma unroll
+            for (int q = 0; q < 3; ++q)
+              *reinterpret_cast<uint2*>(reinterpret_cast<__nv_bfloat16*>(p.out) + q * p.out_plane + (long long)pix[k] * p.Kout + n) = o[q];
+          }
+        }
+      }
+      if (S > 1) {
+        ptx::named_bar_sync(2, kEpiThreads);
+        if (et < S) ptx::mbar_arrive_remote(ptx::map_to_cta(part_done, (uint32_t)et));
+      }
+      }
+    }
+    if (!okw && et == 0 && p.error_flag) atomicCAS(p.error_flag, 0, (int)kErrWaitEpilogue);
+  }
+
+  ptx::tc_fence_before();
+  __syncthreads();
+  if (S > 1) ptx::cluster_sync_all();   // the peers' reads of this CTA's partial sums are over
+  if (warp == 1) {
+    __syncwarp();
+    ptx::tmem_dealloc(tmem_base, kTmemCols);
+  }
+}
+
+// ------------------------------------------------------------------ weights and layouts ----
+// Filter value w(n, t, c), t = tap, c = channel of a block, as three planes of swizzled 64 x 64 tiles.  STEM: the four
+// "taps" are pairs of input rows, the 64 "channels" the 2 rows x 8 pixels x 4 channels of a window (see nchw_to_planes).
+template <typename SrcT, bool STEM>
+__global__ void pack_planes_kernel(const SrcT* __restrict__ src, long long sn, long long sc, long long stap, int Kout, int C, int CB, int taps,
+                                   int n_tiles, uint8_t* __restrict__ dst) {
+  const int kb_all = taps * CB;
+  const long long total = (long long)n_tiles * kb_all * 64 * 64;
+  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
+    const int k = (int)(i & 63), row = (int)(i >> 6) & 63;
+    const long long tile = i >> 12;
+    const int kb = (int)(tile % kb_all), nt = (int)(tile / kb_all);
+    const int n = nt * 64 + row, tap = kb / CB, c = (kb - tap * CB) * 64 + k;
+    float v = 0.0f;
+    if (STEM) {
+      // element k of a window: 16-byte chunks alternate between the rows of the pair, two pixels of four channels each
+      const int chunk = k >> 3, px = 2 * (chunk >> 1) + ((k & 7) >> 2), ch = k & 3;
+      const int r = 2 * tap + (chunk & 1) - 1, s = px - 1;
+      if (n < Kout && ch < 3 && r >= 0 && r < 7 && s >= 0) v = (float)src[n * sn + ch * sc + (long long)(r * 7 + s) * stap];
+    } else if (n < Kout && c < C) {
+      v = (float)src[n * sn + c * sc + tap * stap];
+    }
+    __nv_bfloat16 q[3];
+    split3(v, q[0], q[1], q[2]);
+    const uint32_t off = (uint32_t)row * 128u + ((((uint32_t)k >> 3) ^ ((uint32_t)row & 7u)) << 4) + ((uint32_t)k & 7u) * 2u;
+#pragma unroll
+    for (int pl = 0; pl < 3; ++pl)
+      *reinterpret_cast<__nv_bfloat16*>(dst + ((size_t)(nt * 3 + pl) * kb_all + kb) * kBBytes + off) = q[pl];
+  }
+}
+
+// fp32 tensor -> planes, four elements a thread.
+__global__ void split_planes_kernel(const float* __restrict__ src, __nv_bfloat16* __restrict__ dst, long long n4, long long plane) {
+  ptx::grid_dependency_wait();
+  ptx::grid_launch_dependents();
+  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n4; i += (long long)gridDim.x * blockDim.x) {
+    uint2 o[3];
+    split4(__ldg(reinterpret_cast<const float4*>(src) + i), o);
+#pragma unroll
+    for (int q = 0; q < 3; ++q) *reinterpret_cast<uint2*>(dst + q * plane + 4 * i) = o[q];
+  }
+}
+
+// Stem input: NCHW images of three channels -> planes [3][N][row pair][pixel pair][row of the pair][2 pixels x 4 channels],
+// four zero pixels in front of a row and at least four behind (the buffer is zeroed once; only pixels are written).  A
+// stride-2 window of 8 pixels of both rows is then 128 contiguous bytes, 32 bytes from one output pixel's to the next.
+template <typename SrcT>
+__global__ void nchw_to_planes_kernel(const SrcT* __restrict__ src, __nv_bfloat16* __restrict__ dst, int N, int H, int W, int pair_elems,
+                                      long long plane) {
+  ptx::grid_dependency_wait();
+  ptx::grid_launch_dependents();
+  const long long total = (long long)N * H * W;
+  const int H2 = (H + 1) / 2;
+  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
+    const int x = (int)(i % W);
+    const long long t = i / W;
+    const int y = (int)(t % H);
+    const long long n = t / H;
+    const SrcT* s = src + (size_t)n * 3 * H * W + (size_t)y * W + x;
+    float4 v = make_float4((float)s[0], (float)s[(size_t)H * W], (float)s[2 * (size_t)H * W], 0.0f);
+    uint2 o[3];
+    split4(v, o);
+    const int px = x + 4;
+    const long long at = ((long long)n * H2 + (y >> 1)) * pair_elems + (px >> 1) * 16 + (y & 1) * 8 + (px & 1) * 4;
+#pragma unroll
+    for (int q = 0; q < 3; ++q) *reinterpret_cast<uint2*>(dst + q * plane + at) = o[q];
+  }
+}
+
+// Max-pool over a -inf padded map, planes in and out (the maximum of fp32 values; NaN propagates).
+__global__ void maxpool_planes_kernel(const __nv_bfloat16* __restrict__ src, __nv_bfloat16* __restrict__ dst, int N, int H, int W, int C, int OH,
+                                      int OW, int k, int stride, int pad, long long in_plane, long long out_plane) {
+  ptx::grid_dependency_wait();
+  ptx::grid_launch_dependents();
+  const int cv = C / 4;
+  const unsigned total = (unsigned)N * OH * OW * cv;
+  for (unsigned i = blockIdx.x * blockDim.x + threadIdx.x; i < total; i += gridDim.x * blockDim.x) {
+    unsigned t = i / (unsigned)cv;
+    const int c = (int)(i - t * cv) * 4;
+    const unsigned t2 = t / (unsigned)OW;
+    const int ox = (int)(t - t2 * OW);
+    const int n = (int)(t2 / (unsigned)OH), oy = (int)(t2 - (unsigned)n * OH);
+    float4 m = make_float4(-INFINITY, -INFINITY, -INFINITY, -INFINITY);
+    auto up = [](float a, float b) { return (a < b || b != b) ? b : a; };
+    for (int r = 0; r < k; ++r) {
+      const int iy = oy * stride - pad + r;
+      if ((unsigned)iy >= (unsigned)H) continue;
+      for (int s = 0; s < k; ++s) {
+        const int ix = ox * stride - pad + s;
+        if ((unsigned)ix >= (unsigned)W) continue;
+        const long long at = (((long long)n * H + iy) * W + ix) * C + c;
+        uint2 w[3];
+#pragma unroll
+        for (int q = 0; q < 3; ++q) w[q] = __ldg(reinterpret_cast<const uint2*>(src + q * in_plane + at));
+        const float4 v = join4(w);
+        m = make_float4(up(m.x, v.x), up(m.y, v.y), up(m.z, v.z), up(m.w, v.w));
+      }
+    }
+    uint2 o[3];
+    split4(m, o);
+    const long long at = (((long long)n * OH + oy) * OW + ox) * C + c;
+#pragma unroll
+    for (int q = 0; q < 3; ++q) *reinterpret_cast<uint2*>(dst + q * out_plane + at) = o[q];
+  }
+}
+
+// Global average pool, planes in and out: eight adjacent lanes share one (image, four channels) and add their sums by shuffles.
+__global__ void avgpool_planes_kernel(const __nv_bfloat16* __restrict__ src, __nv_bfloat16* __restrict__ dst, int N, int HW, int C,
+                                      long long in_plane, long long out_plane) {
+  ptx::grid_dependency_wait();
+  ptx::grid_launch_dependents();
+  const int cv = C / 4;
+  const long long total = (long long)N * cv * 8;
+  for (long long i0 = blockIdx.x * (long long)blockDim.x; i0 < total; i0 += (long long)gridDim.x * blockDim.x) {
+    const long long i = i0 + threadIdx.x;
+    const bool live = i < total;
+    const int slice = (int)(i & 7);
+    const long long g = live ? i >> 3 : 0;
+    const int c = (int)(g % cv) * 4;
+    const long long n = g / cv;
+    float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (live)
+      for (int px = slice; px < HW; px += 8) {
+        uint2 w[3];
+#pragma unroll
+        for (int q = 0; q < 3; ++q) w[q] = __ldg(reinterpret_cast<const uint2*>(src + q * in_plane + (n * HW + px) * C + c));
+        const float4 v = join4(w);
+        s.x += v.x; s.y += v.y; s.z += v.z; s.w += v.w;
+      }
+#pragma unroll
+    for (int d = 1; d < 8; d <<= 1) {
+      s.x += __shfl_xor_sync(0xffffffffu, s.x, d);
+      s.y += __shfl_xor_sync(0xffffffffu, s.y, d);
+      s.z += __shfl_xor_sync(0xffffffffu, s.z, d);
+      s.w += __shfl_xor_sync(0xffffffffu, s.w, d);
+    }
+    if (live && slice == 0) {
+      const float inv = (float)HW;
+      uint2 o[3];
+      split4(make_float4(s.x / inv, s.y / inv, s.z / inv, s.w / inv), o);
+#pragma unroll
+      for (int q = 0; q < 3; ++q) *reinterpret_cast<uint2*>(dst + q * out_plane + n * C + c) = o[q];
+    }
+  }
+}
+
+PFN_cuTensorMapEncodeTiled_v12000 f32_get_encode() {
+  static PFN_cuTensorMapEncodeTiled_v12000 fn = nullptr;
+  static std::once_flag once;
+  std::call_once(once, [] {
+    void* ptr = nullptr;
+    cudaDriverEntryPointQueryResult q;
+    if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &ptr, cudaEnableDefault, &q) == cudaSuccess &&
+        q == cudaDriverEntryPointSuccess)
+      fn = reinterpret_cast<PFN_cuTensorMapEncodeTiled_v12000>(ptr);
+  });
+  return fn;
+}
+
+int grid_of(long long total, int threads) {
+  const long long b = (total + threads - 1) / threads, cap = 148LL * 16;
+  return (int)(b < 1 ? 1 : (b > cap ? cap : b));
+}
+
+}  // namespace
+
+size_t packed_planes_bytes(int Kout, int C, int taps) { return (size_t)((Kout + 63) / 64) * 3 * taps * ((C + 63) / 64) * kBBytes; }
+
+cudaError_t launch_pack_planes(const void* src, DType src_dt, long long sn, long long sc, long long stap, int Kout, int C, int taps, bool stem,
+                               void* dst, cudaStream_t stream) {
+  const int CB = stem ? 1 : (C + 63) / 64, nt = (Kout + 63) / 64, tp = stem ? 4 : taps;
+  const int grid = grid_of((long long)nt * tp * CB * 4096, 256);
+  uint8_t* d = static_cast<uint8_t*>(dst);
+#define NNCV_PK(T_) \
+  if (stem) pack_planes_kernel<T_, true><<<grid, 256, 0, stream>>>(static_cast<const T_*>(src), sn, sc, stap, Kout, C, CB, tp, nt, d); \
+  else pack_planes_kernel<T_, false><<<grid, 256, 0, stream>>>(static_cast<const T_*>(src), sn, sc, stap, Kout, C, CB, tp, nt, d)
+  if (src_dt == kF32) { NNCV_PK(float); }
+  else if (src_dt == kF16) { NNCV_PK(__half); }
+  else { NNCV_PK(__nv_bfloat16); }
+#undef NNCV_PK
+  return cudaGetLastError();
+}
+
+cudaError_t launch_split_planes(const float* src, void* dst, long long n, cudaStream_t stream) {
+  if (n % 4 != 0) return cudaErrorInvalidValue;
+  return launch_pdl(split_planes_kernel, dim3(grid_of(n / 4, 256)), dim3(256), 0, stream, src, static_cast<__nv_bfloat16*>(dst), n / 4, n);
+}
+
+int stem_planes_pair_elems(int W) { return ((W + 8 + 1) & ~1) * 8; }   // pixels of a padded row, even, x 2 rows x 4 channels
+long long stem_planes_elems(int N, int H, int W) { return (long long)N * ((H + 1) / 2) * stem_planes_pair_elems(W); }
+
+cudaError_t launch_nchw_to_planes(const void* src, DType src_dt, void* dst, int N, int H, int W, cudaStream_t stream) {
+  const dim3 grid(grid_of((long long)N * H * W, 256));
+  const int pe = stem_planes_pair_elems(W);
+  const long long plane = stem_planes_elems(N, H, W);
+  __nv_bfloat16* d = static_cast<__nv_bfloat16*>(dst);
+  if (src_dt == kF32) return launch_pdl(nchw_to_planes_kernel<float>, grid, dim3(256), 0, stream, static_cast<const float*>(src), d, N, H, W, pe, plane);
+  if (src_dt == kF16) return launch_pdl(nchw_to_planes_kernel<__half>, grid, dim3(256), 0, stream, static_cast<const __half*>(src), d, N, H, W, pe, plane);
+  return launch_pdl(nchw_to_planes_kernel<__nv_bfloat16>, grid, dim3(256), 0, stream, static_cast<const __nv_bfloat16*>(src), d, N, H, W, pe, plane);
+}
+
+cudaError_t launch_maxpool_planes(const void* src, void* dst, int N, int H, int W, int C, int k, int stride, int pad, cudaStream_t stream) {
+  const int OH = (H + 2 * pad - k) / stride + 1, OW = (W + 2 * pad - k) / stride + 1;
+  const long long total = (long long)N * OH * OW * (C / 4);
+  if (C % 4 != 0 || total >= (1LL << 31) - (1LL << 21)) return cudaErrorInvalidValue;
+  return launch_pdl(maxpool_planes_kernel, dim3(grid_of(total, 256)), dim3(256), 0, stream, static_cast<const __nv_bfloat16*>(src),
+                    static_cast<__nv_bfloat16*>(dst), N, H, W, C, OH, OW, k, stride, pad, (long long)N * H * W * C, (long long)N * OH * OW * C);
+}
+
+cudaError_t launch_avgpool_planes(const void* src, void* dst, int N, int HW, int C, cudaStream_t stream) {
+  if (C % 4 != 0) return cudaErrorInvalidValue;
+  return launch_pdl(avgpool_planes_kernel, dim3(grid_of((long long)N * (C / 4) * 8, 256)), dim3(256), 0, stream,
+                    static_cast<const __nv_bfloat16*>(src), static_cast<__nv_bfloat16*>(dst), N, HW, C, (long long)N * HW * C, (long long)N * C);
+}
+
+bool conv_f32_supported(int C, int Kout, int tw_stride) { return C % 8 == 0 && Kout % 4 == 0 && tw_stride <= 256; }
+
+// Tile width and the CTAs of a cluster that share a tile's reduction: the pair with the least rounds x time.  A block of 64
+// channels takes about 1960 clocks with 64 columns and 2700 with 128 when every SM works (both bound by L2 -> shared
+// memory, 34 to 37 bytes a clock and SM: 72 and 96 KB); everything else about 8000 and 14000 a tile (the wide tile is
+// finished in two passes), a split 1500 more.  Clusters of sixteen were slower at batch 1 than clusters of eight (21 us
+// against 15 for a layer of 256 channels on 16 x 16 pixels).  Fewer clusters fit the GPU than its SMs would hold (they do not
+// cross GPC borders), so the runtime is asked.
+template <int BN>
+static int clusters_that_fit(int s, int sms) {
+  static int known[4] = {0, 0, 0, 0};   // per log2(s): the same on every device this library runs on
+  const int k = s == 1 ? 0 : (s == 2 ? 1 : (s == 4 ? 2 : 3));
+  if (s == 1) return sms;
+  if (known[k] == 0) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)(sms / s * s));
+    cfg.blockDim = dim3(kThreads);
+    cfg.dynamicSmemBytes = Ring<BN>::kSmem;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = (unsigned)s;
+    attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    int n = 0;
+    cudaFuncSetAttribute(conv_f32_kernel<BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Ring<BN>::kSmem);
+    if (cudaOccupancyMaxActiveClusters(&n, conv_f32_kernel<BN>, &cfg) != cudaSuccess || n < 1) {
+      cudaGetLastError();
+      n = sms / s * 3 / 4 > 0 ? sms / s * 3 / 4 : 1;
+    }
+    known[k] = n;
+  }
+  return known[k];
+}
+
+static void pick_tile(long long m_tiles, int Kout, int kb_all, int sms, int* bn, int* splits) {
+  double best = 1e30;
+  for (int b = 64; b <= (Kout > 64 ? 128 : 64); b *= 2)
+    for (int s = 1; s <= 8 && s <= kb_all; s *= 2) {
+      const int slots = b == 64 ? clusters_that_fit<64>(s, sms) : clusters_that_fit<128>(s, sms);
+      const long long tiles = m_tiles * ((Kout + b - 1) / b);
+      const double rounds = (double)((tiles + slots - 1) / slots);
+      const double t = rounds * (((kb_all + s - 1) / s) * (b == 64 ? 1960.0 : 2700.0) + (b == 64 ? 3000.0 : 9000.0)) + 5000.0 + (s > 1 ? 1500.0 : 0.0);
+      if (t < best) { best = t; *bn = b; *splits = s; }
+    }
+}
+
+template <int BN>
+static cudaError_t launch_f32_cfg(const CUtensorMap& tm, const F32Params& p, int sms, cudaStream_t stream) {
+  cudaError_t e = cudaFuncSetAttribute(conv_f32_kernel<BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Ring<BN>::kSmem);
+  if (e != cudaSuccess) return e;
+  const int slots = clusters_that_fit<BN>(p.splits, sms);
+  const int clusters = p.items < slots ? p.items : slots;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)(clusters * p.splits));
+  cfg.blockDim = dim3(kThreads);
+  cfg.dynamicSmemBytes = Ring<BN>::kSmem;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  attr[1].id = cudaLaunchAttributeClusterDimension;
+  attr[1].val.clusterDim.x = (unsigned)p.splits;
+  attr[1].val.clusterDim.y = 1;
+  attr[1].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = p.splits > 1 ? 2 : 1;
+  return cudaLaunchKernelEx(&cfg, conv_f32_kernel<BN>, tm, p);
+}
+
+cudaError_t launch_conv_f32(const ConvF32Args& a, cudaStream_t stream) {
+  const bool stem = a.stem != 0;
+  F32Params p{};
+  p.wpack = static_cast<const uint8_t*>(a.wpack);
+  p.scale = a.scale; p.shift = a.shift;
+  p.residual = a.residual; p.res_f32 = a.res_f32;
+  p.out = a.out; p.out_f32 = a.out_f32; p.relu = a.relu; p.error_flag = a.error_flag;
+  p.Kout = a.Kout; p.OH = a.OH; p.OW = a.OW; p.NB = a.N;
+  p.CB = stem ? 1 : (a.C + 63) / 64;
+  p.taps = stem ? 4 : a.R * a.S;
+  p.S = stem ? 1 : a.S;
+  p.stride = stem ? 1 : a.stride;
+  p.pad_x = stem ? 0 : a.pad;
+  p.pad_y = stem ? 2 : a.pad;
+  p.ldo = a.ldo;
+  const long long pixels = (long long)a.N * a.OH * a.OW;
+  if (pixels > 0x7fffffffLL) return cudaErrorInvalidValue;
+  p.res_plane = p.out_plane = pixels * a.Kout;
+  int tw, th, tn;
+  tconv_tile(a.N, a.OH, a.OW, &tw, &th, &tn);
+  if (!conv_f32_supported(stem ? 64 : a.C, a.Kout, (tw > th ? tw : th) * p.stride)) return cudaErrorInvalidValue;
+  if ((reinterpret_cast<uintptr_t>(a.in) & 15) || (reinterpret_cast<uintptr_t>(a.out) & 15) || (reinterpret_cast<uintptr_t>(a.residual) & (a.res_f32 ? 15 : 7)) ||
+      ((a.out_f32 || a.res_f32) && a.ldo % 4 != 0))
+    return cudaErrorMisalignedAddress;
+  p.tw = tw; p.th = th; p.tn = tn;
+  p.tiles_x = (a.OW + tw - 1) / tw; p.tiles_y = (a.OH + th - 1) / th;
+  const long long tiles_n = (a.N + tn - 1) / tn;
+  const int sms = a.sm_count > 0 ? a.sm_count : 148;
+  const long long m_tiles = (long long)p.tiles_x * p.tiles_y * tiles_n;
+  int bn = 64;
+  pick_tile(m_tiles, a.Kout, p.taps * p.CB, sms, &bn, &p.splits);
+  p.n_tiles = (a.Kout + bn - 1) / bn;
+  const long long items = m_tiles * p.n_tiles;
+  if (items <= 0 || items > 0x7fffffffLL) return cudaErrorInvalidValue;
+  p.items = (int)items;
+  p.div_tx = epi::fast_div((uint32_t)p.tiles_x); p.div_ty = epi::fast_div((uint32_t)p.tiles_y); p.div_nt = epi::fast_div((uint32_t)p.n_tiles);
+  p.div_tw = epi::fast_div((uint32_t)tw); p.div_th = epi::fast_div((uint32_t)th);
+
+  auto enc = f32_get_encode();
+  if (!enc) return cudaErrorNotSupported;
+  // [3][N][H][W][C] planes; the stem's [3][N][row pairs][windows][64] has windows that overlap
+  cuuint64_t gdim[5], gstr[4];
+  if (stem) {
+    const cuuint64_t H2 = (cuuint64_t)(a.H + 1) / 2, pair = (cuuint64_t)stem_planes_pair_elems(a.W) * 2;
+    gdim[0] = 64; gdim[1] = (cuuint64_t)a.OW; gdim[2] = H2; gdim[3] = (cuuint64_t)a.N; gdim[4] = 3;
+    gstr[0] = 32; gstr[1] = pair; gstr[2] = H2 * pair; gstr[3] = (cuuint64_t)a.N * H2 * pair;
+  } else {
+    const cuuint64_t px = (cuuint64_t)a.C * 2;
+    gdim[0] = (cuuint64_t)a.C; gdim[1] = (cuuint64_t)a.W; gdim[2] = (cuuint64_t)a.H; gdim[3] = (cuuint64_t)a.N; gdim[4] = 3;
+    gstr[0] = px; gstr[1] = px * a.W; gstr[2] = px * a.W * a.H; gstr[3] = px * a.W * a.H * a.N;
+  }
+  cuuint32_t box[5] = {64, (cuuint32_t)(tw * p.stride), (cuuint32_t)(th * p.stride), (cuuint32_t)tn, 1};
+  cuuint32_t estr[5] = {1, (cuuint32_t)p.stride, (cuuint32_t)p.stride, 1, 1};
+  CUtensorMap tm;
+  if (enc(&tm, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 5, const_cast<void*>(a.in), gdim, gstr, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+          CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
+    return cudaErrorInvalidValue;
+  return bn == 64 ? launch_f32_cfg<64>(tm, p, sms, stream) : launch_f32_cfg<128>(tm, p, sms, stream);
+}
+
+}  // namespace nncv_b200

@@ -182,6 +182,33 @@ cudaError_t launch_repack_weights_f32(const void* src, DType src_dt, long long s
                                       long long stap, int Kout, int C, int Cpad, int taps,
                                       float* dst, cudaStream_t stream);
 
+// ---- fp32 convolutions on the tensor cores: activations as three bf16 planes [3][N][H][W][C] -------------
+struct ConvF32Args {
+  const void* in = nullptr;         // planes; stem: what launch_nchw_to_planes writes
+  const void* wpack = nullptr;      // packed by launch_pack_planes; complete before this launch
+  const float* scale = nullptr;
+  const float* shift = nullptr;
+  const void* residual = nullptr;   // of the output's shape: planes, or fp32 with row pitch ldo
+  void* out = nullptr;              // planes, or fp32 with row pitch ldo (a multiple of 4)
+  int out_f32 = 0, res_f32 = 0;
+  long long ldo = 0;
+  int stem = 0;                     // 7x7 stride-2 pad-3 convolution of the 3-channel input (H, W: the image)
+  int N = 0, H = 0, W = 0, C = 0, OH = 0, OW = 0, Kout = 0, R = 1, S = 1, stride = 1, pad = 0;
+  int relu = 0;
+  int sm_count = 0;
+  int* error_flag = nullptr;
+};
+bool conv_f32_supported(int C, int Kout, int tw_stride);
+cudaError_t launch_conv_f32(const ConvF32Args& a, cudaStream_t stream);
+size_t packed_planes_bytes(int Kout, int C, int taps);   // stem: C = 64, taps = 4
+cudaError_t launch_pack_planes(const void* src, DType src_dt, long long sn, long long sc, long long stap, int Kout, int C, int taps, bool stem,
+                               void* dst, cudaStream_t stream);
+cudaError_t launch_split_planes(const float* src, void* dst, long long n, cudaStream_t stream);
+long long stem_planes_elems(int N, int H, int W);        // elements of one plane
+cudaError_t launch_nchw_to_planes(const void* src, DType src_dt, void* dst, int N, int H, int W, cudaStream_t stream);
+cudaError_t launch_maxpool_planes(const void* src, void* dst, int N, int H, int W, int C, int k, int stride, int pad, cudaStream_t stream);
+cudaError_t launch_avgpool_planes(const void* src, void* dst, int N, int HW, int C, cudaStream_t stream);
+
 // ---- memory-bound helpers (NHWC, 128-bit accesses) ---------------------------------------
 cudaError_t launch_nchw_to_nhwc(const void* src, DType src_dt, void* dst, DType dst_dt, int N,
                                 int C, int H, int W, int Cpad, cudaStream_t stream);

@@ -366,6 +366,9 @@ struct nncv_b200_conv {
   int want_act = 0;       // set by the plan executor: activation beyond ReLU it would like fused (hard-swish, SiLU)
   bool act_done = false;  // set by conv_run when the kernel it launched applied want_act
   std::map<int, std::unique_ptr<DevBuf>> packed;   // tcgen05 path: per N-tile width
+  DevBuf w_planes;                                 // fp32 on the tensor cores: filter as three bf16 planes
+  DevBuf in_planes;                                // the same, called on a dense fp32 map: its planes
+  bool w_planes_ready = false;
   DevBuf w_f32;                                    // fp32 path: [Kout][R*S][Cpad]
   bool w_f32_ready = false;
   DevBuf sp_in, sp_out, sp_res;                    // standalone algo 2: shared-pad copies
@@ -416,6 +419,43 @@ bool fused_branch_ok(const nncv_b200_conv& c, const nncv_b200_conv& b) {
          b.stride == c.stride && b.Cpad == c.Cpad && b.Kout == c.Kout && c.Kout % 128 == 0 && c.Cpad % 64 == 0;
 }
 
+// fp32 convolution on the tensor cores: activations as three bf16 planes (conv_f32.cu).  `stem`: the input is what
+// launch_nchw_to_planes wrote.  out_f32 / res_f32: that tensor is dense fp32 with row pitch ldo instead of planes.
+int conv_run_planes(nncv_b200_conv* c, const void* in, bool stem, int N, int H, int W, const float* scale, const float* shift,
+                    const void* residual, int res_f32, int relu, void* out, int out_f32, long long ldo, cudaStream_t st) {
+  if (!c->w_planes_ready) {
+    int rc = c->w_planes.reserve(stem ? packed_planes_bytes(c->Kout, 64, 4) : packed_planes_bytes(c->Kout, c->C, c->R * c->S));
+    if (rc) return rc;
+    LAUNCH(launch_pack_planes(c->raw, c->raw_dt, c->sn, c->sc, c->stap, c->Kout, c->C, c->R * c->S, stem, c->w_planes.p, st));
+    CU(cudaStreamSynchronize(st));   // the kernel reads packed weights without waiting for earlier work of its stream
+    c->w_planes_ready = true;
+  }
+  ConvF32Args a;
+  a.in = in; a.wpack = c->w_planes.p; a.scale = scale; a.shift = shift; a.residual = residual; a.res_f32 = res_f32;
+  a.out = out; a.out_f32 = out_f32; a.ldo = ldo; a.stem = stem;
+  a.N = N; a.H = H; a.W = W; a.C = c->C; a.Kout = c->Kout; a.R = c->R; a.S = c->S; a.stride = c->stride; a.pad = c->pad;
+  a.OH = (H + 2 * c->pad - c->R) / c->stride + 1;
+  a.OW = (W + 2 * c->pad - c->S) / c->stride + 1;
+  a.relu = relu; a.sm_count = g_dev.sm_count; a.error_flag = g_dev.error_flag;
+  const double Ms = (double)N * a.OH * a.OW;
+  prof_begin(1, 2.0 * Ms * c->Kout * c->C * c->R * c->S,
+             6.0 * ((double)N * H * W * c->C + (double)c->Kout * c->C * c->R * c->S + Ms * c->Kout * (residual ? 2 : 1)), (int)Ms, c->Kout,
+             c->C * c->R * c->S, 64, st);
+  LAUNCH(launch_conv_f32(a, st));
+  prof_end(st);
+  return NNCV_B200_OK;
+}
+
+// Does a convolution on a dense fp32 map go to the tensor cores?  It then takes a pass that splits the input into planes
+// (about 3 us), so short reductions onto few channels stay on the CUDA cores: 16 x 14 x 14 pixels, 64 -> 64 channels 1x1
+// took 8.2 us there against 8.6, but 72 -> 24 on 28 x 28 pixels 12.3 against 10.0, 40 -> 240 20.5 against 15.0, and a 3x3 filter
+// of 32 channels 30.7 against 16.3.
+bool f32_on_tensor_cores(const nncv_b200_conv& c, const void* in, const void* out, const void* residual, long long ldo) {
+  const uintptr_t al = reinterpret_cast<uintptr_t>(in) | reinterpret_cast<uintptr_t>(out) | reinterpret_cast<uintptr_t>(residual);
+  const long long k = (long long)c.C * c.R * c.S;
+  return c.C % 8 == 0 && c.Kout % 4 == 0 && ldo % 4 == 0 && c.stride <= 2 && !(al & 15) && (k >= 72 || k * c.Kout >= 8192);
+}
+
 int conv_run(nncv_b200_conv* c, const void* in, Layout in_l, void* out, Layout out_l, int N, int H,
              int W, const float* scale, const float* shift, const void* residual, int relu,
              DType out_dt, long long ldo, cudaStream_t st, const FusedBranch* fb = nullptr) {
@@ -426,6 +466,13 @@ int conv_run(nncv_b200_conv* c, const void* in, Layout in_l, void* out, Layout o
   if (out_l.pitch == 0) out_l = dense_layout(OH, OW);
   if (c->dtype == kF32) {
     if (in_l.off != 0 || out_l.off != 0) return fail(NNCV_B200_EINVAL, "fp32 conv takes dense NHWC only");
+    if (f32_on_tensor_cores(*c, in, out, residual, ldo)) {
+      const long long elems = (long long)N * H * W * c->C;
+      int rc = c->in_planes.reserve((size_t)elems * 6);
+      if (rc) return rc;
+      LAUNCH(launch_split_planes((const float*)in, c->in_planes.p, elems, st));
+      return conv_run_planes(c, c->in_planes.p, false, N, H, W, scale, shift, residual, 1, relu, out, 1, ldo, st);
+    }
     if (!c->w_f32_ready) {
       int rc = c->w_f32.reserve((size_t)c->Kout * c->R * c->S * c->Cpad * sizeof(float));
       if (rc) return rc;
@@ -1020,6 +1067,7 @@ struct Model {
   DevBuf in_stage, in_nhwc, stem, pooled, logits32, logits_io;
   DevBuf stem_rows, stem_w;  // fused stem (16-bit path): reformatted input rows, packed weights
   bool fused_stem = false;
+  bool planes = false;       // fp32 network whose activations live as three bf16 planes (conv_f32.cu)
   int stem_rows_paired = -1;  // layout the zeroed pad pixels of stem_rows belong to (-1: none yet)
   // Activation tensors of one forward live in one arena.  The first forward of a shape walks the
   // network once without launching anything (planning = true) to record every tensor's size, layout
@@ -1056,6 +1104,24 @@ void model_reset() {
 
 DType dt_from_width(size_t w) { return w == 4 ? kF32 : kF16; }
 
+// fp32 networks of convolutions, pools and FC layers run on the tensor cores over bf16 planes, if every layer's channel
+// counts suit the copies (8 channels = 16 bytes) and the input meets a 7x7 stride-2 stem.
+bool planes_ok(const Plan& plan) {
+  for (size_t i = 0; i < plan.nodes.size(); ++i) {
+    const PlanNode& n = plan.nodes[i];
+    if (n.act > kActRelu) return false;
+    if (n.kind == PlanNode::kConv) {
+      if (n.cout % 8 != 0 || n.stride > 2) return false;
+      if (n.in == 0 ? !(n.cin == 3 && n.k == 7 && n.stride == 2 && n.pad == 3 && n.res < 0) : n.cin % 8 != 0) return false;
+    } else if (n.kind == PlanNode::kFc) {
+      if (n.cin % 8 != 0 || n.cout % (i + 1 == plan.nodes.size() ? 4 : 8) != 0) return false;
+    } else if (n.kind != PlanNode::kMaxPool && n.kind != PlanNode::kAvgPool) {
+      return false;
+    }
+  }
+  return true;
+}
+
 int model_build(Plan plan, const void* host_blob, size_t n_elements, size_t ele_width,
                 const nncv_b200_opts* opts) {
   int rc = device_init();
@@ -1072,6 +1138,7 @@ int model_build(Plan plan, const void* host_blob, size_t n_elements, size_t ele_
     return fail(NNCV_B200_EINVAL, "bad compute_dtype %d", cd);
   m->act_dt = (DType)cd;
   if ((rc = finalize_plan(plan, m->act_dt != kF32))) return rc;
+  m->planes = m->act_dt == kF32 && planes_ok(plan);
   m->plan = std::move(plan);
   cudaStream_t st = g_dev.stream;
   rc = m->blob.reserve(n_elements * ele_width);
@@ -1200,7 +1267,11 @@ int ensure_workspace(Model& m, int N, int H, int W) {
   int rc = 0;
   const int of = m.plan.out_features;
   if ((rc = m.in_stage.reserve((size_t)N * 3 * H * W * m.ele_width))) return rc;
-  if (m.fused_stem && W <= 512 && H >= 7 && W >= 7) {
+  if (m.planes) {
+    const size_t bytes = (size_t)stem_planes_elems(N, H, W) * 6;
+    if ((rc = m.stem_rows.reserve(bytes))) return rc;
+    CU(cudaMemset(m.stem_rows.p, 0, bytes));   // the pad pixels of every row stay zero
+  } else if (m.fused_stem && W <= 512 && H >= 7 && W >= 7) {
     if ((rc = m.stem_rows.reserve(stem_rows_bytes(N, H, W)))) return rc;
     CU(cudaMemset(m.stem_rows.p, 0, stem_rows_bytes(N, H, W)));   // the pad pixels of every row stay zero
     m.stem_rows_paired = (int)stem_paired_ok(H, W);
@@ -1217,7 +1288,7 @@ int ensure_workspace(Model& m, int N, int H, int W) {
 // Next activation tensor of the current forward ([N,h,w,c] in layout l).  Planning pass: records it
 // and hands out a stand-in pointer; afterwards: its place in the arena.
 int next_act(Model& m, int N, int h, int w, int c, Layout l, cudaStream_t st, void** out) {
-  const size_t bytes = (size_t)layout_slots(l, N) * c * dtype_size(m.act_dt);
+  const size_t bytes = (size_t)layout_slots(l, N) * c * (m.planes ? 6 : dtype_size(m.act_dt));
   (void)h; (void)w; (void)st;
   if (m.planning) {
     m.act_plan.push_back(Model::ActRec{bytes, {l.img_rows, l.pitch, c}, m.op_idx + 1, m.op_idx + 1, 0});
@@ -1355,7 +1426,15 @@ int model_forward_device(Model& m, const void* src_dev, int N, int H, int W, cud
       continue;
     }
     Ten in;
-    if (n.in == 0) {
+    if (n.in == 0 && m.planes) {
+      if (!input_converted && begin_op({})) {
+        prof_begin(3, 0, (double)N * H * W * (3.0 * m.ele_width + 24.0), N * H * W, 3, 0, 3, st);
+        LAUNCH(launch_nchw_to_planes(src_dev, m.io_dt, m.stem_rows.p, N, H, W, st));
+        prof_end(st);
+      }
+      input_converted = true;
+      in.p = m.stem_rows.p; in.h = H; in.w = W; in.c = 3;
+    } else if (n.in == 0) {
       // NCHW -> NHWC (channels padded), io type -> activation type; once per forward
       if (!input_converted) {
         if (!m.in_nhwc.p || m.in_nhwc.bytes < (size_t)N * H * W * cpad0 * dtype_size(adt)) {
@@ -1396,6 +1475,13 @@ int model_forward_device(Model& m, const void* src_dev, int N, int H, int W, cud
         if (it == tens.end() || it->second.h != oh || it->second.w != ow)
           return fail(NNCV_B200_EINVAL, "plan: the residual of tensor %d does not have its shape", n.id);
         res = it->second.p;
+      }
+      if (m.planes) {
+        if (begin_op({in.p, res}) &&
+            (rc = conv_run_planes(&c, in.p, n.in == 0, N, in.h, in.w, m.scale[n.conv_idx], m.shift[n.conv_idx], res, 0, n.relu, o.p, 0, 0, st)))
+          return rc;
+        tens[n.id] = o;
+        continue;
       }
       bool done = false;
       if (n.branch >= 0 && sp && fused_branch_ok(c, conv_of(m.plan.nodes[n.branch]))) {
@@ -1530,7 +1616,8 @@ int model_forward_device(Model& m, const void* src_dev, int N, int H, int W, cud
       if ((rc = next_act(m, N, oh, ow, in.c, o.l, st, &o.p))) return rc;
       if (begin_op({in.p})) {
         prof_begin(3, 0, aes * in.c * N * ((double)in.h * in.w + (double)oh * ow), N * in.h * in.w, in.c, 0, 1, st);
-        LAUNCH(launch_maxpool_nhwc(in.p, o.p, adt, N, in.h, in.w, in.c, n.k, n.stride, n.pad, in.l, o.l, st));
+        if (m.planes) LAUNCH(launch_maxpool_planes(in.p, o.p, N, in.h, in.w, in.c, n.k, n.stride, n.pad, st));
+        else LAUNCH(launch_maxpool_nhwc(in.p, o.p, adt, N, in.h, in.w, in.c, n.k, n.stride, n.pad, in.l, o.l, st));
         prof_end(st);
       }
       tens[n.id] = o;
@@ -1541,7 +1628,8 @@ int model_forward_device(Model& m, const void* src_dev, int N, int H, int W, cud
       if ((rc = next_act(m, N, 1, 1, in.c, o.l, st, &o.p))) return rc;
       if (begin_op({in.p})) {
         prof_begin(3, 0, aes * in.c * N * (in.h * in.w + 1.0), N * in.h * in.w, in.c, 0, 2, st);
-        LAUNCH(launch_avgpool_nhwc(in.p, o.p, adt, N, in.h, in.w, in.c, in.l, st));
+        if (m.planes) LAUNCH(launch_avgpool_planes(in.p, o.p, N, in.h * in.w, in.c, st));
+        else LAUNCH(launch_avgpool_nhwc(in.p, o.p, adt, N, in.h, in.w, in.c, in.l, st));
         prof_end(st);
       }
       tens[n.id] = o;
@@ -1554,6 +1642,11 @@ int model_forward_device(Model& m, const void* src_dev, int N, int H, int W, cud
         Ten o;
         o.l = dense_layout(1, 1); o.h = o.w = 1; o.c = n.cout;
         if ((rc = next_act(m, N, 1, 1, n.cout, o.l, st, &o.p))) return rc;
+        if (m.planes) {
+          if (begin_op({in.p}) && (rc = conv_run_planes(fc, in.p, false, N, 1, 1, nullptr, bias, nullptr, 0, n.act == kActRelu, o.p, 0, 0, st))) return rc;
+          tens[n.id] = o;
+          continue;
+        }
         if (begin_op({in.p}) &&
             (rc = conv_run(fc, in.p, dense_layout(1, 1), o.p, dense_layout(1, 1), N, 1, 1, nullptr, bias, nullptr, n.act == kActRelu, adt,
                            n.cout, st)))
@@ -1570,7 +1663,8 @@ int model_forward_device(Model& m, const void* src_dev, int N, int H, int W, cud
         return conv_run(fc, in.p, dense_layout(1, 1), m.logits_io.p, dense_layout(1, 1), N, 1, 1, nullptr, bias, nullptr, 0, adt, of,
                         st);
       }
-      rc = conv_run(fc, in.p, dense_layout(1, 1), m.logits32.p, dense_layout(1, 1), N, 1, 1, nullptr, bias, nullptr, 0, kF32, of, st);
+      rc = m.planes ? conv_run_planes(fc, in.p, false, N, 1, 1, nullptr, bias, nullptr, 0, 0, m.logits32.p, 1, of, st)
+                    : conv_run(fc, in.p, dense_layout(1, 1), m.logits32.p, dense_layout(1, 1), N, 1, 1, nullptr, bias, nullptr, 0, kF32, of, st);
       if (rc) return rc;
       if (m.io_dt != kF32)
         LAUNCH(launch_convert(m.logits32.p, kF32, m.logits_io.p, m.io_dt, (size_t)N * of, st));
