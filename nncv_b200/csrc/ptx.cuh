@@ -144,6 +144,13 @@ __device__ __forceinline__ void ldg_256(const void* p, uint32_t (&r)[8]) {
                : "l"(p));
 }
 
+// 32-byte global store (address 32-byte aligned): a whole sector in one access.
+__device__ __forceinline__ void stg_256(void* p, const uint32_t (&r)[8]) {
+  asm volatile("st.global.v8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"l"(p), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]),
+               "r"(r[5]), "r"(r[6]), "r"(r[7])
+               : "memory");
+}
+
 // Untiled bulk copy global->shared; both addresses 16-byte aligned, size a multiple of 16.
 __device__ __forceinline__ void bulk_g2s(uint32_t dst, const void* src, uint32_t bytes,
                                          uint32_t bar) {

@@ -138,6 +138,156 @@ __global__ void __launch_bounds__(256) stem3x3_kernel(const TI* __restrict__ src
   }
 }
 
+// The same for stride 1 and 2, FOUR adjacent output pixels a thread.  With one pixel a thread the layer was bound by
+// instructions: a broadcast load of the filter for every four packed multiply-adds, 27 guarded loads of the input and their
+// addresses (146 us for MobileNetV3's first layer at batch 256, 180 MB: 28 us of HBM; the whole network 1234 us, with this
+// kernel 1177).  Here a filter value serves four pixels, the input comes as one row of 3 * STRIDE + 3 values per (channel,
+// filter row), and where rows are 16-byte aligned (VEC: stride 2, pad 1, W a multiple of 8) as 16-byte loads whose left
+// neighbour arrives by shuffle.
+constexpr int kPX = 4;
+
+template <typename TI, bool VEC, int STRIDE>
+__device__ __forceinline__ void input_row(const TI* rowp, bool yin, int ix0, int W, int gx, int lane, float (&v)[(kPX - 1) * STRIDE + 3]) {
+  constexpr int NC = (kPX - 1) * STRIDE + 3;
+  if constexpr (VEC) {
+    // columns 8 gx - 1 .. 8 gx + 7; the first one is the last value of the lane before, a pad at the row's start
+    if constexpr (sizeof(TI) == 2) {
+      uint4 q = make_uint4(0, 0, 0, 0);
+      if (yin) q = __ldg(reinterpret_cast<const uint4*>(rowp + 8 * gx));
+      const __half2* h = reinterpret_cast<const __half2*>(&q);
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const float2 f = __half22float2(h[e]);
+        v[1 + 2 * e] = f.x;
+        v[2 + 2 * e] = f.y;
+      }
+    } else {
+#pragma unroll
+      for (int e = 0; e < 2; ++e) {
+        float4 q = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (yin) q = __ldg(reinterpret_cast<const float4*>(rowp + 8 * gx) + e);
+        v[1 + 4 * e] = q.x; v[2 + 4 * e] = q.y; v[3 + 4 * e] = q.z; v[4 + 4 * e] = q.w;
+      }
+    }
+    float left = __shfl_up_sync(0xffffffffu, v[8], 1);
+    if (lane == 0) left = yin && gx > 0 ? ld<TI>(rowp + 8 * gx - 1) : 0.0f;
+    v[0] = gx > 0 ? left : 0.0f;
+  } else {
+#pragma unroll
+    for (int c = 0; c < NC; ++c) {
+      const bool in = yin && (unsigned)(ix0 + c) < (unsigned)W;
+      v[c] = in ? ld<TI>(rowp + ix0 + c) : 0.0f;
+    }
+  }
+}
+
+template <typename TI, bool BF16, bool VEC, int STRIDE>
+__global__ void __launch_bounds__(256) stem3x3_row_kernel(const TI* __restrict__ src, const float* __restrict__ w, const float* __restrict__ scale,
+                                                          const float* __restrict__ shift, void* __restrict__ dst, Layout ol, int N, int H, int W,
+                                                          int OH, int OW, int Cout, int pad, int act, int xgroups, long long total) {
+  constexpr int NC = (kPX - 1) * STRIDE + 3;
+  extern __shared__ __align__(16) float sw[];     // [27][Cout] filter, [Cout] scale, [Cout] shift
+  float* ssc = sw + 27 * Cout;
+  float* ssh = ssc + Cout;
+  ptx::grid_dependency_wait();
+  ptx::grid_launch_dependents();
+  for (int i = threadIdx.x; i < 27 * Cout; i += blockDim.x) {
+    const int k = i / 27, t = i - k * 27;           // source [Cout][3][3][3]: t = (ci*3 + ky)*3 + kx
+    sw[t * Cout + k] = w[i];
+  }
+  for (int c = threadIdx.x; c < Cout; c += blockDim.x) {
+    ssc[c] = scale ? scale[c] : 1.0f;
+    ssh[c] = shift ? shift[c] : 0.0f;
+  }
+  __syncthreads();
+  const int lane = threadIdx.x & 31;
+  const unsigned per = (unsigned)(total / (Cout / kCG));   // pixel groups of one channel group
+  // whole warps stay in the loop: the shuffle needs every lane
+  for (long long i0 = (long long)blockIdx.x * blockDim.x; i0 < total; i0 += (long long)gridDim.x * blockDim.x) {
+    const bool live = i0 + threadIdx.x < total;
+    const unsigned i = (unsigned)(live ? i0 + threadIdx.x : total - 1);
+    const int g = (int)(i / per);
+    const unsigned t = i - (unsigned)g * per;
+    const unsigned t2 = t / (unsigned)xgroups;
+    const int gx = (int)(t - t2 * xgroups);
+    const int n = (int)(t2 / (unsigned)OH), oy = (int)(t2 - (unsigned)n * OH);
+    float2 acc[kPX][kCG / 2];
+#pragma unroll
+    for (int x = 0; x < kPX; ++x)
+#pragma unroll
+      for (int e = 0; e < kCG / 2; ++e) acc[x][e] = make_float2(0.0f, 0.0f);
+    const int ix0 = gx * kPX * STRIDE - pad;
+    const TI* img = src + (size_t)n * 3 * H * W;
+#pragma unroll 1
+    for (int ky = 0; ky < 3; ++ky) {
+      const int iy = oy * STRIDE - pad + ky;
+      const bool yin = (unsigned)iy < (unsigned)H;
+      float v[3][NC];
+#pragma unroll
+      for (int ci = 0; ci < 3; ++ci) input_row<TI, VEC, STRIDE>(img + ((size_t)ci * H + (yin ? iy : 0)) * W, yin, ix0, W, gx, lane, v[ci]);
+#pragma unroll
+      for (int ci = 0; ci < 3; ++ci)
+#pragma unroll
+        for (int kx = 0; kx < 3; ++kx) {
+          const float* wp = sw + ((ci * 3 + ky) * 3 + kx) * Cout + g * kCG;
+#pragma unroll
+          for (int e = 0; e < kCG / 2; e += 2) {
+            const float4 w4 = *reinterpret_cast<const float4*>(wp + 2 * e);
+#pragma unroll
+            for (int x = 0; x < kPX; ++x) {
+              const float2 v2 = make_float2(v[ci][x * STRIDE + kx], v[ci][x * STRIDE + kx]);
+              acc[x][e] = fma2(v2, make_float2(w4.x, w4.y), acc[x][e]);
+              acc[x][e + 1] = fma2(v2, make_float2(w4.z, w4.w), acc[x][e + 1]);
+            }
+          }
+        }
+    }
+    if (!live) continue;
+#pragma unroll
+    for (int x = 0; x < kPX; ++x) {
+      const int ox = gx * kPX + x;
+      if (ox >= OW) break;
+      uint32_t o[kCG / 2];
+#pragma unroll
+      for (int e = 0; e < kCG / 2; ++e) {
+        const float2 sc = *reinterpret_cast<const float2*>(ssc + g * kCG + 2 * e);
+        const float2 sh = *reinterpret_cast<const float2*>(ssh + g * kCG + 2 * e);
+        float2 a = fma2(acc[x][e], sc, sh);
+        if (act == kActHardSwish) {   // a NaN stays NaN through the product
+          a.x *= __saturatef(fmaf(a.x, 0.16666667f, 0.5f));
+          a.y *= __saturatef(fmaf(a.y, 0.16666667f, 0.5f));
+        } else {
+          a.x = act16(a.x, act);
+          a.y = act16(a.y, act);
+        }
+        if (BF16) {
+          const __nv_bfloat162 b = __floats2bfloat162_rn(a.x, a.y);
+          o[e] = *reinterpret_cast<const uint32_t*>(&b);
+        } else {
+          o[e] = ptx::pack_half2_sat(a.x, a.y);
+        }
+      }
+      ptx::stg_256(reinterpret_cast<unsigned short*>(dst) + (((size_t)n * ol.img_rows + oy + ol.off) * ol.pitch + ox + ol.off) * Cout + g * kCG, o);
+    }
+  }
+}
+
+template <typename TI, bool BF16>
+cudaError_t launch_row(const TI* src, const float* w, const float* scale, const float* shift, void* dst, Layout ol, int N, int H, int W, int OH,
+                       int OW, int Cout, int stride, int pad, int act, cudaStream_t st) {
+  const int xg = (OW + kPX - 1) / kPX;
+  const long long total = (long long)N * OH * xg * (Cout / kCG);
+  const bool vec = stride == 2 && pad == 1 && W % 8 == 0 && !(reinterpret_cast<uintptr_t>(src) & 15);   // then OW == W / 2
+  long long blocks = (total + 255) / 256;
+  if (blocks > 148 * 2) blocks = 148 * 2;   // two blocks a SM (registers): the filter is loaded once
+  const size_t smem = (size_t)29 * Cout * sizeof(float);
+  auto go = [&](auto kern) {
+    return launch_pdl(kern, dim3((unsigned)blocks), dim3(256), smem, st, src, w, scale, shift, dst, ol, N, H, W, OH, OW, Cout, pad, act, xg, total);
+  };
+  if (vec) return go(stem3x3_row_kernel<TI, BF16, true, 2>);
+  return stride == 2 ? go(stem3x3_row_kernel<TI, BF16, false, 2>) : go(stem3x3_row_kernel<TI, BF16, false, 1>);
+}
+
 }  // namespace
 
 bool stem3x3_supported(int Cin, int Cout, int R, int S, DType act_dt, int act) {
@@ -153,6 +303,13 @@ cudaError_t launch_stem3x3(const void* src, DType src_dt, const float* w, const 
   if (out_l.pitch == 0) out_l = dense_layout(OH, OW);
   const long long total = (long long)N * OH * OW * (Cout / kCG);
   if (total >= (1LL << 31) - (1LL << 21)) return cudaErrorInvalidValue;
+  if (stride <= 2) {   // wider strides share no input between neighbours
+    if (src_dt == kF32)
+      return dt == kBF16 ? launch_row<float, true>((const float*)src, w, scale, shift, dst, out_l, N, H, W, OH, OW, Cout, stride, pad, act, st)
+                         : launch_row<float, false>((const float*)src, w, scale, shift, dst, out_l, N, H, W, OH, OW, Cout, stride, pad, act, st);
+    return dt == kBF16 ? launch_row<__half, true>((const __half*)src, w, scale, shift, dst, out_l, N, H, W, OH, OW, Cout, stride, pad, act, st)
+                       : launch_row<__half, false>((const __half*)src, w, scale, shift, dst, out_l, N, H, W, OH, OW, Cout, stride, pad, act, st);
+  }
   long long blocks = (total + 255) / 256;
   if (blocks > 148 * 16) blocks = 148 * 16;
   const size_t smem = (size_t)29 * Cout * sizeof(float);
