@@ -8,10 +8,13 @@
 // tiles of 8 output rows x TW output columns x CB channels and one thread issues, two tiles ahead,
 // ONE tensor copy per tile: the input patch with its halo, out-of-range pixels filled with zeros by
 // the copy engine (no bounds checks on the input side at all).  The 256 threads then read the
-// patch from shared memory with 16-byte loads: thread = (channel vector, output column, half of
-// the tile's rows) and computes a column strip of four output rows, so that each input value is
-// loaded from shared memory once per filter column and reused down the strip, in fp32 pairs
-// (fma.rn.f32x2).  The filter, scale and shift of the CTA's channel chunk sit in shared memory.
+// patch from shared memory: thread = (four channels, output column), computing a column strip of eight output rows in fp32
+// pairs (fma.rn.f32x2), so that each input value is loaded once per filter column and reused down the strip, and each
+// filter value serves eight outputs.  With eight channels a thread and strips of four rows the 5x5 layers were bound by
+// shared memory: a filter vector of eight fp32 is two loads at a stride of 32 bytes, two-way bank conflicts, and those loads
+// were two thirds of the traffic (14x14x240 at batch 256: 9.8 M wavefronts, 48 us); now a lane's four filter values are 16
+// contiguous bytes and are read half as often.  The filter times the scale, and the shift the sums start at, sit in shared
+// memory.
 // Every wait on a copy is bounded; a wait that gives up sets the status word and the CTA leaves.
 #include <cuda.h>
 #include <cuda_bf16.h>
@@ -21,6 +24,7 @@
 
 #include <mutex>
 
+#include "epilogue.cuh"
 #include "kernels.h"
 #include "ptx.cuh"
 
@@ -29,8 +33,10 @@ namespace nncv_b200 {
 namespace {
 
 constexpr int kThreads = 256;
-constexpr int kP = 4;            // output rows per thread
-constexpr int kTH = 2 * kP;      // output rows per tile
+constexpr int kTH = 8;           // output rows per tile
+// output rows per thread: the tile's eight, or four in fp32, whose rows are twice as long (with strips of eight a tile
+// needs 38 KB a stage and only two CTAs fit an SM)
+template <typename T> constexpr int kRows = sizeof(T) == 4 ? 4 : 8;
 constexpr int kMaxStages = 3;
 
 struct DwParams {
@@ -41,66 +47,45 @@ struct DwParams {
   void* y;             // [N,OH,OW,C]
   int N, H, W, C, OH, OW, pad, act;
   Layout in_l, out_l;  // input coordinates and output pixels are shifted by the layouts' pad offsets
-  int tw, cbv;         // output columns per tile, 16-byte channel vectors per chunk (tw * cbv == 128)
+  int tw, cbv;         // output columns per tile, 16-byte channel vectors per chunk (tw * cbv <= 128)
   int tiles_x, tiles_y, n_tiles;   // spatial tiles (n_tiles = N * tiles_y * tiles_x)
+  epi::FastDiv div_tx, div_ty;
   int stages;
   uint32_t stage_bytes, stage_stride;
   int* error_flag;
 };
 
-__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
-  unsigned long long ra, rb, rc, rd;
-  asm("mov.b64 %0, {%1, %2};" : "=l"(ra) : "f"(a.x), "f"(a.y));
-  asm("mov.b64 %0, {%1, %2};" : "=l"(rb) : "f"(b.x), "f"(b.y));
-  asm("mov.b64 %0, {%1, %2};" : "=l"(rc) : "f"(c.x), "f"(c.y));
-  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(rd) : "l"(ra), "l"(rb), "l"(rc));
-  float2 d;
-  asm("mov.b64 {%0, %1}, %2;" : "=f"(d.x), "=f"(d.y) : "l"(rd));
+typedef unsigned long long u64;   // two fp32 in a register pair
+__device__ __forceinline__ u64 mul2(u64 a, u64 b) {
+  u64 d;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
   return d;
 }
 
-__device__ __forceinline__ float2 mul2(float2 a, float2 b) {
-  unsigned long long ra, rb, rd;
-  asm("mov.b64 %0, {%1, %2};" : "=l"(ra) : "f"(a.x), "f"(a.y));
-  asm("mov.b64 %0, {%1, %2};" : "=l"(rb) : "f"(b.x), "f"(b.y));
-  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(rd) : "l"(ra), "l"(rb));
-  float2 d;
-  asm("mov.b64 {%0, %1}, %2;" : "=f"(d.x), "=f"(d.y) : "l"(rd));
-  return d;
+// A thread's vector: four channels, 8 bytes of a 16-bit type or 16 of fp32.
+template <typename T> struct Vec { using type = uint2; };
+template <> struct Vec<float> { using type = uint4; };
+__device__ __forceinline__ void unpack(const uint4& raw, u64 (&f)[2], float) {
+  f[0] = epi::pk(__uint_as_float(raw.x), __uint_as_float(raw.y));
+  f[1] = epi::pk(__uint_as_float(raw.z), __uint_as_float(raw.w));
 }
-
-template <typename T> __device__ __forceinline__ void unpack(const uint4& raw, float2* f);
-template <> __device__ __forceinline__ void unpack<float>(const uint4& raw, float2* f) {
-  f[0] = make_float2(__uint_as_float(raw.x), __uint_as_float(raw.y));
-  f[1] = make_float2(__uint_as_float(raw.z), __uint_as_float(raw.w));
+__device__ __forceinline__ void unpack(const uint2& raw, u64 (&f)[2], __half) {
+  const float2 a = __half22float2(*reinterpret_cast<const __half2*>(&raw.x)), b = __half22float2(*reinterpret_cast<const __half2*>(&raw.y));
+  f[0] = epi::pk(a.x, a.y);
+  f[1] = epi::pk(b.x, b.y);
 }
-template <> __device__ __forceinline__ void unpack<__half>(const uint4& raw, float2* f) {
-  const __half2* h = reinterpret_cast<const __half2*>(&raw);
-#pragma unroll
-  for (int e = 0; e < 4; ++e) f[e] = __half22float2(h[e]);
+__device__ __forceinline__ void unpack(const uint2& raw, u64 (&f)[2], __nv_bfloat16) {   // a bf16 is the upper half of an fp32
+  f[0] = epi::pk(__uint_as_float(raw.x << 16), __uint_as_float(raw.x & 0xffff0000u));
+  f[1] = epi::pk(__uint_as_float(raw.y << 16), __uint_as_float(raw.y & 0xffff0000u));
 }
-template <> __device__ __forceinline__ void unpack<__nv_bfloat16>(const uint4& raw, float2* f) {
-  const uint32_t* u = reinterpret_cast<const uint32_t*>(&raw);   // a bf16 is the upper half of an fp32
-#pragma unroll
-  for (int e = 0; e < 4; ++e) f[e] = make_float2(__uint_as_float(u[e] << 16), __uint_as_float(u[e] & 0xffff0000u));
+__device__ __forceinline__ uint4 pack(const float (&v)[4], float) {
+  return make_uint4(__float_as_uint(v[0]), __float_as_uint(v[1]), __float_as_uint(v[2]), __float_as_uint(v[3]));
 }
-template <typename T> __device__ __forceinline__ uint4 pack(const float2* r);
-template <> __device__ __forceinline__ uint4 pack<float>(const float2* r) {
-  return make_uint4(__float_as_uint(r[0].x), __float_as_uint(r[0].y), __float_as_uint(r[1].x), __float_as_uint(r[1].y));
+__device__ __forceinline__ uint2 pack(const float (&v)[4], __half) {   // saturating, NaN stays NaN
+  return make_uint2(epi::pack16(v[0], v[1], false, false), epi::pack16(v[2], v[3], false, false));
 }
-template <> __device__ __forceinline__ uint4 pack<__half>(const float2* r) {   // saturating, NaN stays NaN
-  return make_uint4(ptx::pack_half2_sat(r[0].x, r[0].y), ptx::pack_half2_sat(r[1].x, r[1].y),
-                    ptx::pack_half2_sat(r[2].x, r[2].y), ptx::pack_half2_sat(r[3].x, r[3].y));
-}
-template <> __device__ __forceinline__ uint4 pack<__nv_bfloat16>(const float2* r) {
-  uint4 o;
-  uint32_t* u = reinterpret_cast<uint32_t*>(&o);
-#pragma unroll
-  for (int e = 0; e < 4; ++e) {
-    const __nv_bfloat162 b = __floats2bfloat162_rn(r[e].x, r[e].y);
-    u[e] = *reinterpret_cast<const uint32_t*>(&b);
-  }
-  return o;
+__device__ __forceinline__ uint2 pack(const float (&v)[4], __nv_bfloat16) {
+  return make_uint2(epi::pack16(v[0], v[1], true, false), epi::pack16(v[2], v[3], true, false));
 }
 
 // The activations of MobileNetV3.mlir:345-383 and Yolov5s.mlir:158-169.  EXACT (fp32 tensors) keeps
@@ -130,7 +115,10 @@ template <typename T, int KS, int STRIDE>
 __global__ void __launch_bounds__(kThreads, KS == 3 ? 3 : 2) depthwise_tma_kernel(const __grid_constant__ CUtensorMap tm_in, const DwParams p) {
   ptx::grid_dependency_wait();
   ptx::grid_launch_dependents();
-  constexpr int V = 16 / sizeof(T);
+  constexpr int V = 4;                                  // channels of a thread
+  constexpr int kP = kRows<T>;                          // output rows of a thread
+  constexpr int kPer = 16 / (V * sizeof(T));            // threads of a 16-byte vector
+  using Raw = typename Vec<T>::type;
   constexpr int NR = (kP - 1) * STRIDE + KS;            // input rows under one strip of kP outputs
   extern __shared__ __align__(128) unsigned char smem[];
   __shared__ __align__(8) unsigned long long full_bar[kMaxStages];
@@ -139,12 +127,11 @@ __global__ void __launch_bounds__(kThreads, KS == 3 ? 3 : 2) depthwise_tma_kerne
 
   const int tid = threadIdx.x;
   const int cbv = p.cbv, tw = p.tw;
-  const int CB = cbv * V;                                // channels per chunk
+  const int CB = cbv * kPer * V;                         // channels per chunk
   const int IW = (tw - 1) * STRIDE + KS;
   const int c0 = blockIdx.y * CB;
-  float* sw = reinterpret_cast<float*>(smem + (size_t)p.stages * p.stage_stride);   // [KS*KS][CB], scale[CB], shift[CB]
-  float* ssc = sw + KS * KS * CB;
-  float* ssh = ssc + CB;
+  float* sw = reinterpret_cast<float*>(smem + (size_t)p.stages * p.stage_stride);   // [KS*KS][CB] filter times scale, shift[CB]
+  float* ssh = sw + KS * KS * CB;
 
   if (tid == 0) {
     abort_flag = 0;
@@ -158,22 +145,18 @@ __global__ void __launch_bounds__(kThreads, KS == 3 ? 3 : 2) depthwise_tma_kerne
     if (c0 + c < p.C) {
       const size_t idx = (size_t)(c0 + c) * (KS * KS) + tap;
       v = p.w_half ? __half2float(reinterpret_cast<const __half*>(p.w)[idx]) : reinterpret_cast<const float*>(p.w)[idx];
+      if (p.scale) v *= p.scale[c0 + c];
     }
     sw[i] = v;
   }
-  for (int c = tid; c < CB; c += kThreads) {
-    const bool in = c0 + c < p.C;
-    ssc[c] = (in && p.scale) ? p.scale[c0 + c] : 1.0f;
-    ssh[c] = (in && p.shift) ? p.shift[c0 + c] : 0.0f;
-  }
+  for (int c = tid; c < CB; c += kThreads) ssh[c] = (c0 + c < p.C && p.shift) ? p.shift[c0 + c] : 0.0f;
   __syncthreads();
 
   const int my_tiles = ((int)blockIdx.x < p.n_tiles) ? (p.n_tiles - 1 - (int)blockIdx.x) / (int)gridDim.x + 1 : 0;
   auto issue = [&](int k) {      // thread 0: the copy of this CTA's k-th tile into stage k % stages
     const int sp = blockIdx.x + k * gridDim.x;
-    const int n = sp / (p.tiles_y * p.tiles_x);
-    const int r = sp - n * (p.tiles_y * p.tiles_x);
-    const int ty = r / p.tiles_x, tx = r - ty * p.tiles_x;
+    const int t2 = (int)epi::div_by((uint32_t)sp, p.div_tx), tx = sp - t2 * p.tiles_x;
+    const int n = (int)epi::div_by((uint32_t)t2, p.div_ty), ty = t2 - n * p.tiles_y;
     const int s = k % p.stages;
     const uint32_t bar = ptx::smem_u32(&full_bar[s]);
     tile_info[s] = make_int4(n, ty * kTH, tx * tw, 0);   // read by the others after they have seen the barrier complete
@@ -185,9 +168,8 @@ __global__ void __launch_bounds__(kThreads, KS == 3 ? 3 : 2) depthwise_tma_kerne
   if (tid == 0)
     for (; issued < p.stages - 1 && issued < my_tiles; ++issued) issue(issued);
 
-  const int cvec = tid % cbv;
-  const int x = (tid / cbv) % tw;
-  const int ys = tid / (cbv * tw);                       // 0 or 1
+  const int xs = tid / (kPer * cbv), cvec = tid - xs * (kPer * cbv);
+  const int ys = kP == kTH ? 0 : xs / tw, x = xs - ys * tw;   // strip of rows, column
   int k = 0;
   for (; k < my_tiles; ++k) {
     const int s = k % p.stages;
@@ -196,76 +178,66 @@ __global__ void __launch_bounds__(kThreads, KS == 3 ? 3 : 2) depthwise_tma_kerne
     if (__syncthreads_or(!ok)) break;
     if (tid == 0 && issued < my_tiles) { issue(issued); ++issued; }
 
+    if (kP == kTH ? x >= tw : ys >= kTH / kP) continue;  // no strip of the tile is this thread's
     const unsigned char* st = smem + (size_t)s * p.stage_stride;
-    float2 acc[kP][V / 2];
+    // the sums start at the shift; the filter carries the scale
+    u64 acc[kP][2];
+    {
+      const ulonglong2 sh = *reinterpret_cast<const ulonglong2*>(ssh + cvec * V);
 #pragma unroll
-    for (int o = 0; o < kP; ++o)
-#pragma unroll
-      for (int e = 0; e < V / 2; ++e) acc[o][e] = make_float2(0.0f, 0.0f);
-    const int row0 = ys * kP * STRIDE;
+      for (int o = 0; o < kP; ++o) { acc[o][0] = sh.x; acc[o][1] = sh.y; }
+    }
 #pragma unroll
     for (int kx = 0; kx < KS; ++kx) {
-      float2 wr[KS][V / 2];
+      ulonglong2 wr[KS];
 #pragma unroll
-      for (int q = 0; q < KS; ++q)
-#pragma unroll
-        for (int e = 0; e < V / 2; e += 2) {
-          const float4 t4 = *reinterpret_cast<const float4*>(sw + (q * KS + kx) * CB + cvec * V + 2 * e);
-          wr[q][e] = make_float2(t4.x, t4.y);
-          wr[q][e + 1] = make_float2(t4.z, t4.w);
-        }
-      const unsigned char* col = st + ((size_t)(row0 * IW + x * STRIDE + kx) * cbv + cvec) * 16;
+      for (int q = 0; q < KS; ++q) wr[q] = *reinterpret_cast<const ulonglong2*>(sw + (q * KS + kx) * CB + cvec * V);
+      const unsigned char* col = st + (size_t)(ys * kP * STRIDE * IW + x * STRIDE + kx) * cbv * 16 + cvec * sizeof(Raw);
 #pragma unroll
       for (int ry = 0; ry < NR; ++ry) {
-        const uint4 raw = *reinterpret_cast<const uint4*>(col + (size_t)ry * IW * cbv * 16);
-        float2 f[V / 2];
-        unpack<T>(raw, f);
+        u64 f[2];
+        unpack(*reinterpret_cast<const Raw*>(col + (size_t)ry * IW * cbv * 16), f, T{});
 #pragma unroll
         for (int o = 0; o < kP; ++o) {
           const int q = ry - o * STRIDE;               // compile-time after unrolling
           if (q >= 0 && q < KS) {
-#pragma unroll
-            for (int e = 0; e < V / 2; ++e) acc[o][e] = fma2(f[e], wr[q][e], acc[o][e]);
+            acc[o][0] = epi::fma2(f[0], wr[q].x, acc[o][0]);
+            acc[o][1] = epi::fma2(f[1], wr[q].y, acc[o][1]);
           }
         }
       }
     }
-    // epilogue: scale, shift, activation, store
+    // epilogue: activation, store
     const int4 ti = tile_info[s];
-    const int n = ti.x;
-    const int ox = ti.z + x;
-    const int c = c0 + cvec * V;
+    const int ox = ti.z + x, c = c0 + cvec * V;
     if (ox < p.OW && c < p.C) {
-      float2 sc[V / 2], sh[V / 2];
+      T* yp = reinterpret_cast<T*>(p.y) + (((size_t)ti.x * p.out_l.img_rows + ti.y + ys * kP + p.out_l.off) * p.out_l.pitch + ox + p.out_l.off) * p.C + c;
+      const size_t row_step = (size_t)p.out_l.pitch * p.C;
+      const int rows = min(kP, p.OH - ti.y - ys * kP);
+      auto finish = [&](auto f4) {
 #pragma unroll
-      for (int e = 0; e < V / 2; e += 2) {
-        const float4 a4 = *reinterpret_cast<const float4*>(ssc + cvec * V + 2 * e);
-        const float4 b4 = *reinterpret_cast<const float4*>(ssh + cvec * V + 2 * e);
-        sc[e] = make_float2(a4.x, a4.y); sc[e + 1] = make_float2(a4.z, a4.w);
-        sh[e] = make_float2(b4.x, b4.y); sh[e + 1] = make_float2(b4.z, b4.w);
-      }
-#pragma unroll
-      for (int o = 0; o < kP; ++o) {
-        const int oy = ti.y + ys * kP + o;
-        if (oy >= p.OH) break;
-        float2 r2[V / 2];
-#pragma unroll
-        for (int e = 0; e < V / 2; ++e) {
-          // scale and shift default to 1 and 0 in shared memory, so one fused multiply-add serves every case
-          const float2 a = fma2(acc[o][e], sc[e], sh[e]);
-          if (sizeof(T) == 2 && p.act == kActHardSwish) {
-            // min/max clamp: a NaN still comes out as NaN because the clamped factor multiplies x itself
-            float2 t = fma2(a, make_float2(0.16666667f, 0.16666667f), make_float2(0.5f, 0.5f));
-            t.x = fminf(fmaxf(t.x, 0.0f), 1.0f);
-            t.y = fminf(fmaxf(t.y, 0.0f), 1.0f);
-            r2[e] = mul2(a, t);
-          } else {
-            r2[e] = make_float2(act1<sizeof(T) == 4>(a.x, p.act), act1<sizeof(T) == 4>(a.y, p.act));
-          }
+        for (int o = 0; o < kP; ++o) {
+          if (o >= rows) break;
+          float v[4];
+          f4(acc[o][0], v[0], v[1]);
+          f4(acc[o][1], v[2], v[3]);
+          *reinterpret_cast<Raw*>(yp + o * row_step) = pack(v, T{});
         }
-        *reinterpret_cast<uint4*>(reinterpret_cast<T*>(p.y) +
-                                  (((size_t)n * p.out_l.img_rows + oy + p.out_l.off) * p.out_l.pitch + ox + p.out_l.off) * p.C + c) =
-            pack<T>(r2);
+      };
+      if (p.act == kActNone) {
+        finish([](u64 a, float& r, float& t) { epi::unpk(a, r, t); });
+      } else if (sizeof(T) == 2 && p.act == kActHardSwish) {
+        // clamp of (x + 3) / 6 to [0, 1]: a NaN still comes out as NaN because the clamped factor multiplies x itself
+        finish([](u64 a, float& r, float& t) {
+          epi::unpk(a, r, t);
+          epi::unpk(mul2(a, epi::pk(__saturatef(fmaf(r, 0.16666667f, 0.5f)), __saturatef(fmaf(t, 0.16666667f, 0.5f)))), r, t);
+        });
+      } else {
+        finish([&](u64 a, float& r, float& t) {
+          epi::unpk(a, r, t);
+          r = act1<sizeof(T) == 4>(r, p.act);
+          t = act1<sizeof(T) == 4>(t, p.act);
+        });
       }
     }
   }
@@ -330,16 +302,23 @@ cudaError_t launch_depthwise_tma(const void* x, const void* w, DType w_dt, const
   const int es = (int)dtype_size(dt), V = 16 / es, cv = C / V;
   const int OH = (H + 2 * pad - R) / stride + 1, OW = (W + 2 * pad - S) / stride + 1;
   DwParams p{};
-  // 128 (column, vector) pairs per tile: wide tiles for wide maps, more channels per chunk for narrow ones;
-  // a chunk never holds more vectors than the tensor has
+  // 256 threads: (column, four-channel vector) pairs of a tile in any split of whole 16-byte vectors: the one that leaves the
+  // fewest threads idle or outside the map and the channels.  Halo columns, rows of a patch shorter than 128 bytes and
+  // stages so large that fewer than three CTAs fit an SM count against it.
+  const int slots = kThreads / 2;                      // 16-byte vectors of a tile
   int cbv = 0, tw = 0;
-  double best = 1e30;
-  for (int cand = 16; cand >= 2; cand /= 2) {          // ties go to the wider chunk (longer contiguous runs in memory)
+  double best = 0.0;
+  for (int cand = 32; cand >= 2; --cand) {             // ties go to the wider chunk (longer contiguous runs in memory)
     if (cand > cv) continue;
-    const int t = 128 / cand;
-    if (t > 8 && t >= 2 * OW) continue;                // a tile more than twice as wide as the map
-    const double waste = (double)((cv + cand - 1) / cand * cand) / cv * ((OW + t - 1) / t * t) / OW;
-    if (waste < best - 1e-9) { best = waste; cbv = cand; tw = t; }
+    const int tiles = (OW + slots / cand - 1) / (slots / cand), t = (OW + tiles - 1) / tiles;
+    const int chunks = (cv + cand - 1) / cand, iw = (t - 1) * stride + R, ih = (kTH - 1) * stride + R;
+    const size_t need = 2 * (((size_t)iw * ih * cand * 16 + 127) & ~(size_t)127) + (size_t)(R * S + 1) * cand * V * sizeof(float);
+    if (need > 200 * 1024 || iw > 256) continue;
+    double use = (double)cv / (chunks * cand) * OW / (tiles * t) * (t * cand) / slots;
+    use *= 0.5 + 0.5 * (t * stride) / iw;
+    if (cand < 8) use *= 0.5 + 0.5 * cand / 8.0;
+    if (need > 72 * 1024) use *= need > 110 * 1024 ? 0.6 : 0.9;
+    if (use > best + 1e-9) { best = use; cbv = cand; tw = t; }
   }
   if (cbv == 0) return cudaErrorInvalidValue;
   p.tw = tw; p.cbv = cbv;
@@ -347,7 +326,7 @@ cudaError_t launch_depthwise_tma(const void* x, const void* w, DType w_dt, const
   if (IW > 256 || IH > 256) return cudaErrorInvalidValue;
   p.stage_bytes = (uint32_t)IW * IH * cbv * 16;
   p.stage_stride = (p.stage_bytes + 127u) & ~127u;
-  const size_t wbytes = (size_t)(R * S + 2) * cbv * V * sizeof(float);
+  const size_t wbytes = (size_t)(R * S + 1) * cbv * V * sizeof(float);
   int stages = kMaxStages;
   while (stages > 2 && (size_t)stages * p.stage_stride + wbytes > 72 * 1024) --stages;   // three CTAs per SM when it fits
   const size_t smem = (size_t)stages * p.stage_stride + wbytes;
@@ -363,6 +342,7 @@ cudaError_t launch_depthwise_tma(const void* x, const void* w, DType w_dt, const
   p.in_l = in_l; p.out_l = out_l;
   p.tiles_x = (OW + tw - 1) / tw; p.tiles_y = (OH + kTH - 1) / kTH;
   p.n_tiles = N * p.tiles_y * p.tiles_x;
+  p.div_tx = epi::fast_div((uint32_t)p.tiles_x); p.div_ty = epi::fast_div((uint32_t)p.tiles_y);
   p.error_flag = error_flag;
 
   auto enc = dw_get_encode();

@@ -269,6 +269,10 @@ cudaError_t launch_activation(const void* x, void* y, DType dt, size_t n, int ac
 cudaError_t launch_scale_channels(const void* x, const void* gate, void* y, DType dt, int N, long long HW, int C, cudaStream_t st);
 cudaError_t launch_se_gate(const void* pooled, const float* w1, const float* b1, const float* w2, const float* b2, void* gate,
                            DType dt, int N, int C, int Cr, cudaStream_t st);
+// pool, gate and scaling of squeeze-and-excitation in place, in one kernel
+bool se_supported(DType dt, int C, int Cr);
+cudaError_t launch_se(void* x, Layout l, const float* w1, const float* b1, const float* w2, const float* b2, DType dt, int N, int H, int W, int C,
+                      int Cr, int sm_count, int* error_flag, cudaStream_t st);
 cudaError_t launch_concat(const void* const* in, const int* channels, int n_in, void* out, DType dt, long long pixels, cudaStream_t st);
 cudaError_t launch_upsample2x(const void* in, void* out, DType dt, int N, int H, int W, int C, cudaStream_t st);
 

@@ -1585,6 +1585,15 @@ int model_forward_device(Model& m, const void* src_dev, int N, int H, int W, cud
       // squeeze-and-excitation (MobileNetV3.mlir:319-389): pooled = mean(x); gate = hard-sigmoid(W2 relu(W1 pooled + b1) + b2);
       // x *= gate, in place (the plan checker has made sure nothing else reads the unscaled tensor)
       const Model::SeW& w = m.ses[n.aux_idx];
+      if (se_supported(adt, in.c, n.cr)) {
+        if (begin_op({in.p})) {
+          prof_begin(3, 4.0 * N * in.c * n.cr, 3.0 * aes * in.c * N * in.h * in.w, N * in.h * in.w, in.c, n.cr, 7, st);
+          LAUNCH(launch_se(in.p, in.l, w.w1, w.b1, w.w2, w.b2, adt, N, in.h, in.w, in.c, n.cr, g_dev.sm_count, g_dev.error_flag, st));
+          prof_end(st);
+        }
+        tens[n.id] = in;
+        continue;
+      }
       Ten pooled, gate;
       pooled.l = gate.l = dense_layout(1, 1);
       pooled.h = pooled.w = gate.h = gate.w = 1;
