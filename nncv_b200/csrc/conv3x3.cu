@@ -220,7 +220,9 @@ conv3x3_kernel(const __grid_constant__ CUtensorMap tm_in, const __grid_constant_
       const uint32_t idesc = ptx::umma_idesc(128, BN, p.bf16 ? 1 : 0);
       bool okw = true;
       if (RESIDENT) okw = ptx::warp_wait(w_full, 0, abort_flag);
-      uint32_t in_cnt = 0, w_cnt = 0, acc_cnt = 0;
+      uint32_t in_st = 0, in_ring = 0, acc_cnt = 0;
+      uint32_t ws = 0, w_ring = 0;   // weight stage, parity of the ring's round
+      uint32_t w_seen = RESIDENT || !okw ? 0u : ptx::mbar_peek(w_full, 0);
       for (int i = 0; okw; ++i) {
         int m_item, n_tile;
         if (!item_of(i, m_item, n_tile)) break;
@@ -229,20 +231,22 @@ conv3x3_kernel(const __grid_constant__ CUtensorMap tm_in, const __grid_constant_
         ptx::tc_fence_after();
         const uint32_t d_base = tmem_base + ab * (MT * BN);
         for (int cb = 0; cb < p.CB && okw; ++cb) {
-          const uint32_t st = in_cnt % (uint32_t)p.in_stages;
-          if (!ptx::warp_wait(in_full + 8 * st, (in_cnt / (uint32_t)p.in_stages) & 1u, abort_flag)) { okw = false; break; }
+          const uint32_t st = in_st;
+          if (!ptx::warp_wait(in_full + 8 * st, in_ring, abort_flag)) { okw = false; break; }
+          if (++in_st == (uint32_t)p.in_stages) { in_st = 0; in_ring ^= 1u; }
           ptx::tc_fence_after();
           const uint32_t a_stage = sIn + st * in_stage_bytes;
           for (int tap = 0; tap < 9; ++tap) {
             uint32_t w_addr;
-            uint32_t ws = 0;
+            const uint32_t w_now = ws;
             if (RESIDENT) {
               w_addr = sW + (uint32_t)(tap * p.CB + cb) * WTILE;
             } else {
-              ws = w_cnt % (uint32_t)p.w_stages;
-              if (!ptx::warp_wait(w_full + 8 * ws, (w_cnt / (uint32_t)p.w_stages) & 1u, abort_flag)) { okw = false; break; }
+              if (!ptx::warp_all(w_seen) && !ptx::warp_wait(w_full + 8 * ws, w_ring, abort_flag)) { okw = false; break; }
               ptx::tc_fence_after();
               w_addr = sW + ws * WTILE;
+              if (++ws == (uint32_t)p.w_stages) { ws = 0; w_ring ^= 1u; }
+              w_seen = ptx::mbar_peek(w_full + 8 * ws, w_ring);
             }
             const int r = tap / 3, s = tap - 3 * r;
             // descriptors differ only in the address bits of the low word: one add per MMA
@@ -259,13 +263,9 @@ conv3x3_kernel(const __grid_constant__ CUtensorMap tm_in, const __grid_constant_
                               k4 == 0 ? first : 1u, issue);
               }
             }
-            if (!RESIDENT) {
-              ptx::tc_commit(w_empty + 8 * ws, issue);
-              ++w_cnt;
-            }
+            if (!RESIDENT) ptx::tc_commit(w_empty + 8 * w_now, issue);
           }
           ptx::tc_commit(in_empty + 8 * st, issue);
-          ++in_cnt;
         }
         ptx::tc_commit(acc_full + 8 * ab, issue);
         ++acc_cnt;

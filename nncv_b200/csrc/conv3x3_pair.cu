@@ -8,9 +8,8 @@
 // 512-channel 3x3 convolutions, :442-582).
 //
 // Synchronisation (all barriers live at the same shared-memory offsets in both CTAs):
-//   in_full / w_full    local TMA completion in each CTA; the peer CTA's idle MMA warp relays each
-//                       completion to the LEADER's in_full / w_full with a remote arrive (those expect
-//                       two arrivals), so the issuing lane tests one barrier per stage.
+//   in_full / w_full    live in the LEADER: its barriers count the bytes that the copies of both CTAs bring, so the issuing
+//                       warp tests one barrier per stage and nobody has to relay the peer's.
 //   in_empty / w_empty  the leader's commit arrives on the barrier of BOTH CTAs (one multicast commit),
 //                       so both producers reuse the stage.
 //   acc_full            committed to both CTAs; acc_empty (leader) collects one arrive per epilogue warp of both.
@@ -37,7 +36,6 @@ constexpr int kMaxIn = 4, kMaxW = 12;
 constexpr size_t kBarBytes = 8 * (2 * kMaxIn + 2 * kMaxW + 4 + epi::kWarps * epi::kMaxBufs) + 16;
 
 struct PairParams {
-  const uint8_t* wpack;      // packed for N tile max(64, BNP / 2); each CTA of the pair takes BNP / 2 rows
   const float* scale;
   const float* shift;
   int* error_flag;
@@ -47,7 +45,7 @@ struct PairParams {
   int box_rows, n_boxes;     // a CTA's halo tile (mt * 128 + 2P + 2 rows) arrives as n_boxes TMA boxes
   int in_stages, w_stages;
   int w_resident;            // all 3 * CB weight stages stay in shared memory (one Kout tile only)
-  unsigned long long wpack_bytes;   // size of the packed weights (copies are range-checked against it)
+  int w_box;                 // rows of a weight copy: a CTA's half of a tile, or of a column slice of the tail
   // Tail of the item list: the items of the last, partly filled round are split into tail_parts
   // column slices (BNP / tail_parts columns each) that run on different pairs at the same time.
   // Items [0, tail_start) are whole; tail_start is a multiple of the number of pairs.
@@ -60,7 +58,7 @@ struct PairParams {
 template <int BNP, int MT>   // columns of the pair's tile (64, 128 or 256), sub-tiles of 256 slots per item
 __global__ void __launch_bounds__(kThreads, 1)
 conv3x3_pair_kernel(const __grid_constant__ CUtensorMap tm_in, const __grid_constant__ CUtensorMap tm_out,
-                    const __grid_constant__ CUtensorMap tm_res, const PairParams p) {
+                    const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CUtensorMap tm_res, const PairParams p) {
   constexpr int kBNPair = BNP;
   constexpr int kMT = MT;
   constexpr int kWTile = (BNP / 2) * 128;          // this CTA's half of a weight tile
@@ -101,11 +99,11 @@ conv3x3_pair_kernel(const __grid_constant__ CUtensorMap tm_in, const __grid_cons
   if (threadIdx.x == 0) {
     s_abort = 0;
     for (int i = 0; i < kMaxIn; ++i) {
-      ptx::mbar_init(in_full + 8 * i, rank == 0 ? 2 : 1);   // leader: own copy + the peer's relay
+      ptx::mbar_init(in_full + 8 * i, 1);
       ptx::mbar_init(in_empty + 8 * i, 1);
     }
     for (int i = 0; i < kMaxW; ++i) {
-      ptx::mbar_init(w_full + 8 * i, rank == 0 ? 2 : 1);
+      ptx::mbar_init(w_full + 8 * i, 1);
       ptx::mbar_init(w_empty + 8 * i, 1);
     }
     for (int i = 0; i < 2; ++i) {
@@ -116,6 +114,7 @@ conv3x3_pair_kernel(const __grid_constant__ CUtensorMap tm_in, const __grid_cons
     ptx::mbar_fence_init();
     ptx::prefetch_tensormap(&tm_in);
     ptx::prefetch_tensormap(&tm_out);
+    ptx::prefetch_tensormap(&tm_w);
     if (p.has_res) ptx::prefetch_tensormap(&tm_res);
   }
   if (warp == 1) {
@@ -148,36 +147,27 @@ conv3x3_pair_kernel(const __grid_constant__ CUtensorMap tm_in, const __grid_cons
     return w < total_items;
   };
 
-  // This CTA's half of an item's columns for filter row fr of channel block cb -> weight stage ws (three taps).  False: the
-  // copy would leave the packed weights or the ring (reported; the waits then run out).
+  const uint32_t lead_in_full = ptx::map_to_cta(in_full, 0), lead_w_full = ptx::map_to_cta(w_full, 0);
+  // This CTA's half of an item's columns for filter row fr of channel block cb -> weight stage ws (three taps).
   auto load_weights = [&](int n_tile, int sub, int parts, int cb, int fr, uint32_t ws) {
-    const int ncols = BNP / parts;
-    const int wrow = n_tile * BNP + sub * ncols + (int)rank * (ncols / 2);   // as rows of the packed N tiles
-    const uint32_t wbytes = (uint32_t)(ncols / 2) * 128u;                    // per tap
-    const uint8_t* wsrc = p.wpack + (size_t)(wrow / kPackBN) * kb_total * kPackTile + (size_t)(wrow % kPackBN) * 128;
-    ptx::mbar_arrive_expect_tx(w_full + 8 * ws, kWGroup * wbytes);
+    const int rows = BNP / parts / 2;                                           // per tap
+    const int wrow = n_tile * BNP + sub * (BNP / parts) + (int)rank * rows;     // as rows of the packed N tiles
+    if (rank == 0) ptx::mbar_arrive_expect_tx(w_full + 8 * ws, 2u * kWGroup * (uint32_t)rows * 128u);
 #pragma unroll
     for (int s3 = 0; s3 < kWGroup; ++s3) {
-      const uint8_t* src = wsrc + ((size_t)(fr * 3 + s3) * p.CB + cb) * kPackTile;
-      if ((size_t)(src - p.wpack) + wbytes > p.wpack_bytes || sW + ws * kWStage + (s3 + 1) * kWTile > sStage) {
-        if (p.error_flag) atomicCAS(p.error_flag, 0, (int)kErrBounds);
-        *abort_flag = 1;
-        return false;
-      }
-      ptx::bulk_g2s(sW + ws * kWStage + s3 * kWTile, src, wbytes, w_full + 8 * ws);
+      const int first = ((wrow / kPackBN) * kb_total + (fr * 3 + s3) * p.CB + cb) * kPackBN + wrow % kPackBN;
+      for (int r = 0; r < rows; r += p.w_box)
+        ptx::tma_load_2d_pair(sW + ws * kWStage + s3 * kWTile + (uint32_t)r * 128u, &tm_w, 0, first + r, lead_w_full + 8 * ws);
     }
-    return true;
   };
   // Packed weights never change, so their copies start before the previous kernel of the stream has finished.
   uint32_t early = 0;   // stages of the weight ring already on their way
   if (warp == 0 && lane == 0) {
-    bool ok = true;
-    for (int i = 0; ok && early < (uint32_t)p.w_stages && !(p.w_resident && i > 0); ++i) {
+    for (int i = 0; early < (uint32_t)p.w_stages && !(p.w_resident && i > 0); ++i) {
       int m_item, n_tile, sub, parts;
       if (!item_of(i, m_item, n_tile, sub, parts)) break;
-      for (int cb = 0; ok && cb < p.CB && early < (uint32_t)p.w_stages; ++cb)
-        for (int fr = 0; ok && fr < 3 && early < (uint32_t)p.w_stages; ++fr, ++early)
-          ok = load_weights(n_tile, sub, parts, cb, fr, early);
+      for (int cb = 0; cb < p.CB && early < (uint32_t)p.w_stages; ++cb)
+        for (int fr = 0; fr < 3 && early < (uint32_t)p.w_stages; ++fr, ++early) load_weights(n_tile, sub, parts, cb, fr, early);
     }
   }
   // The rest reads what the previous kernel wrote, or writes what it may still be reading.
@@ -198,17 +188,17 @@ conv3x3_pair_kernel(const __grid_constant__ CUtensorMap tm_in, const __grid_cons
         for (int cb = 0; cb < p.CB && okw; ++cb) {
           const uint32_t st = in_cnt % (uint32_t)p.in_stages;
           if (!ptx::mbar_wait_cluster_abortable(in_empty + 8 * st, ((in_cnt / (uint32_t)p.in_stages) & 1u) ^ 1u, abort_flag)) { okw = false; break; }
-          ptx::mbar_arrive_expect_tx(in_full + 8 * st, (uint32_t)in_stage_bytes);
+          if (rank == 0) ptx::mbar_arrive_expect_tx(in_full + 8 * st, 2u * (uint32_t)in_stage_bytes);
           for (int bx = 0; bx < p.n_boxes; ++bx)
-            ptx::tma_load_2d(sIn + st * in_stage_bytes + (uint32_t)(bx * p.box_rows) * 128u, &tm_in, cb * 64,
-                             row0 + bx * p.box_rows, in_full + 8 * st);
+            ptx::tma_load_2d_pair(sIn + st * in_stage_bytes + (uint32_t)(bx * p.box_rows) * 128u, &tm_in, cb * 64,
+                                  row0 + bx * p.box_rows, lead_in_full + 8 * st);
           ++in_cnt;
           if (p.w_resident && i > 0) continue;       // resident weights were loaded with the first item
           for (int fr = 0; fr < 3; ++fr, ++w_cnt) {   // one filter row (three taps) per weight stage
             if (w_cnt < early) continue;
             const uint32_t ws = w_cnt % (uint32_t)p.w_stages;
             if (!ptx::mbar_wait_cluster_abortable(w_empty + 8 * ws, ((w_cnt / (uint32_t)p.w_stages) & 1u) ^ 1u, abort_flag)) { okw = false; break; }
-            if (!load_weights(n_tile, sub, parts, cb, fr, ws)) { okw = false; break; }
+            load_weights(n_tile, sub, parts, cb, fr, ws);
           }
         }
       }
@@ -219,8 +209,10 @@ conv3x3_pair_kernel(const __grid_constant__ CUtensorMap tm_in, const __grid_cons
       // ---------------------------------------------------------------- MMA issuer (leader) --
       const uint32_t issue = ptx::elect_one();
       const uint32_t idesc_full = ptx::umma_idesc(256, kBNPair, p.bf16 ? 1 : 0);
-      uint32_t in_cnt = 0, w_cnt = 0, acc_cnt = 0;
+      uint32_t in_st = 0, in_ring = 0, acc_cnt = 0;
+      uint32_t w_st = 0, w_ring = 0;   // weight stage, parity of the ring's round (resident: each stage's first filling)
       bool okw = true;
+      uint32_t in_seen = ptx::mbar_peek_cluster(in_full, 0), w_seen = ptx::mbar_peek_cluster(w_full, 0);
       for (int i = 0; okw; ++i) {
         int m_item, n_tile, sub, parts;
         if (!item_of(i, m_item, n_tile, sub, parts)) break;
@@ -230,19 +222,20 @@ conv3x3_pair_kernel(const __grid_constant__ CUtensorMap tm_in, const __grid_cons
         ptx::tc_fence_after();
         const uint32_t d = tmem_base + ab * (uint32_t)(kBNPair * MT);
         for (int cb = 0; cb < p.CB && okw; ++cb) {
-          const uint32_t st = in_cnt % (uint32_t)p.in_stages;
-          const uint32_t ipar = (in_cnt / (uint32_t)p.in_stages) & 1u;
-          if (!ptx::warp_wait_cluster(in_full + 8 * st, ipar, abort_flag)) { okw = false; break; }
+          const uint32_t st = in_st;
+          if (!ptx::warp_all(in_seen) && !ptx::warp_wait_cluster(in_full + 8 * st, in_ring, abort_flag)) { okw = false; break; }
+          if (++in_st == (uint32_t)p.in_stages) { in_st = 0; in_ring ^= 1u; }
           ptx::tc_fence_after();
           const uint32_t a_stage = sIn + st * in_stage_bytes;
-          for (int fr = 0; fr < 3; ++fr, ++w_cnt) {
-            // resident: stage cb * 3 + fr, filled once (phase 0)
-            const uint32_t ws = p.w_resident ? (uint32_t)(cb * 3 + fr) : w_cnt % (uint32_t)p.w_stages;
-            const uint32_t wpar = p.w_resident ? 0u : (w_cnt / (uint32_t)p.w_stages) & 1u;
+          for (int fr = 0; fr < 3; ++fr) {
+            const uint32_t ws = w_st;   // resident: stage cb * 3 + fr, filled once
             if (!p.w_resident || i == 0) {
-              if (!ptx::warp_wait_cluster(w_full + 8 * ws, wpar, abort_flag)) { okw = false; break; }
+              if (!ptx::warp_all(w_seen) && !ptx::warp_wait_cluster(w_full + 8 * ws, w_ring, abort_flag)) { okw = false; break; }
               ptx::tc_fence_after();
             }
+            if (++w_st == (uint32_t)p.w_stages) { w_st = 0; w_ring ^= 1u; }
+            if (!p.w_resident || i == 0) w_seen = ptx::mbar_peek_cluster(w_full + 8 * w_st, w_ring);
+            if (fr == 2) in_seen = ptx::mbar_peek_cluster(in_full + 8 * in_st, in_ring);
 #pragma unroll
             for (int t = 0; t < MT; ++t) {   // the stage's three weight tiles serve every sub-tile
 #pragma unroll
@@ -262,36 +255,12 @@ conv3x3_pair_kernel(const __grid_constant__ CUtensorMap tm_in, const __grid_cons
           }
           if (!okw) break;
           ptx::tc_commit_pair(in_empty + 8 * st, issue);
-          ++in_cnt;
         }
         if (!okw) break;
         ptx::tc_commit_pair(acc_full + 8 * ab, issue);
         ++acc_cnt;
       }
       if (!okw && lane == 0 && p.error_flag) atomicCAS(p.error_flag, 0, (int)kErrWaitMma);
-    } else if (lane == 0) {
-      // ---------------------------------------------------------------- relay (peer CTA) ----
-      // Tells the leader when this CTA's stages are full.
-      const uint32_t lead_in_full = ptx::map_to_cta(in_full, 0), lead_w_full = ptx::map_to_cta(w_full, 0);
-      uint32_t in_cnt = 0, w_cnt = 0;
-      bool okw = true;
-      for (int i = 0; okw; ++i) {
-        int m_item, n_tile, sub, parts;
-        if (!item_of(i, m_item, n_tile, sub, parts)) break;
-        for (int cb = 0; cb < p.CB && okw; ++cb) {
-          const uint32_t st = in_cnt % (uint32_t)p.in_stages;
-          if (!ptx::mbar_wait_abortable(in_full + 8 * st, (in_cnt / (uint32_t)p.in_stages) & 1u, abort_flag)) { okw = false; break; }
-          ptx::mbar_arrive_remote(lead_in_full + 8 * st);
-          ++in_cnt;
-          if (p.w_resident && i > 0) continue;
-          for (int fr = 0; fr < 3; ++fr, ++w_cnt) {
-            const uint32_t ws = w_cnt % (uint32_t)p.w_stages;
-            if (!ptx::mbar_wait_abortable(w_full + 8 * ws, (w_cnt / (uint32_t)p.w_stages) & 1u, abort_flag)) { okw = false; break; }
-            ptx::mbar_arrive_remote(lead_w_full + 8 * ws);
-          }
-        }
-      }
-      if (!okw && p.error_flag) atomicCAS(p.error_flag, 0, (int)kErrWaitMma);
     }
   } else {
 #include "conv3x3_pair_epilogue.inc"

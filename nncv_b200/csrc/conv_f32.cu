@@ -641,25 +641,7 @@ static int clusters_that_fit(int s, int sms) {
   static int known[4] = {0, 0, 0, 0};   // per log2(s): the same on every device this library runs on
   const int k = s == 1 ? 0 : (s == 2 ? 1 : (s == 4 ? 2 : 3));
   if (s == 1) return sms;
-  if (known[k] == 0) {
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)(sms / s * s));
-    cfg.blockDim = dim3(kThreads);
-    cfg.dynamicSmemBytes = Ring<BN>::kSmem;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = (unsigned)s;
-    attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    int n = 0;
-    cudaFuncSetAttribute(conv_f32_kernel<BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Ring<BN>::kSmem);
-    if (cudaOccupancyMaxActiveClusters(&n, conv_f32_kernel<BN>, &cfg) != cudaSuccess || n < 1) {
-      cudaGetLastError();
-      n = sms / s * 3 / 4 > 0 ? sms / s * 3 / 4 : 1;
-    }
-    known[k] = n;
-  }
+  if (known[k] == 0) known[k] = max_clusters(conv_f32_kernel<BN>, s, kThreads, Ring<BN>::kSmem, sms);
   return known[k];
 }
 

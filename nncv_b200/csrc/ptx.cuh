@@ -290,6 +290,21 @@ __device__ __forceinline__ uint32_t elect_one() {
 }
 __device__ __forceinline__ bool warp_all(bool x) { return __all_sync(0xffffffffu, x) != 0; }
 __device__ __forceinline__ int warp_uniform(int x) { return __shfl_sync(0xffffffffu, x, 0); }
+// Is the phase over?  Asked one stage ahead, before the MMAs of the current one are issued: the answer is there when they
+// are, and the issuing warp does not stand still for the latency of a barrier test (ResNet-18 fp16 1x224: 205 -> 189 us).
+__device__ __forceinline__ uint32_t mbar_peek(uint32_t bar, uint32_t parity) {
+  uint32_t ok;
+  asm volatile(
+      "{\n"
+      ".reg .pred p;\n"
+      "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n"
+      "selp.u32 %0, 1, 0, p;\n"
+      "}\n"
+      : "=r"(ok)
+      : "r"(bar), "r"(parity)
+      : "memory");
+  return ok;
+}
 // Bounded waits of a whole warp: the same answer in every lane.
 __device__ __forceinline__ bool warp_wait(uint32_t bar, uint32_t parity, volatile int* abort_flag) {
   return warp_all(mbar_wait_abortable(bar, parity, abort_flag));
@@ -444,6 +459,22 @@ __device__ __forceinline__ bool mbar_wait_cluster_abortable(uint32_t bar, uint32
   }
   return true;
 }
+// Tiled copies into this CTA's shared memory whose completion is counted on a barrier of either CTA of the pair (`bar`: an
+// address from map_to_cta).  With the leader's barrier counting both CTAs' bytes, the issuing warp needs no word from the
+// peer: a relay thread there (wait for the local barrier, arrive on the leader's with release semantics) held a stage of
+// four MMAs to 1600 clocks.
+__device__ __forceinline__ void tma_load_2d_pair(uint32_t dst, const void* tmap, int c0, int c1, uint32_t bar) {
+  asm volatile(
+      "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::"r"(dst),
+      "l"(tmap), "r"(c0), "r"(c1), "r"(bar)
+      : "memory");
+}
+__device__ __forceinline__ void tma_load_4d_pair(uint32_t dst, const void* tmap, int c0, int c1, int c2, int c3, uint32_t bar) {
+  asm volatile(
+      "cp.async.bulk.tensor.4d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4, %5}], [%6];" ::"r"(dst),
+      "l"(tmap), "r"(c0), "r"(c1), "r"(c2), "r"(c3), "r"(bar)
+      : "memory");
+}
 __device__ __forceinline__ void tmem_alloc_pair(uint32_t slot_smem, uint32_t ncols) {
   asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(slot_smem), "r"(ncols) : "memory");
 }
@@ -452,6 +483,19 @@ __device__ __forceinline__ void tmem_relinquish_pair() {
 }
 __device__ __forceinline__ void tmem_dealloc_pair(uint32_t taddr, uint32_t ncols) {
   asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(ncols) : "memory");
+}
+__device__ __forceinline__ uint32_t mbar_peek_cluster(uint32_t bar, uint32_t parity) {
+  uint32_t ok;
+  asm volatile(
+      "{\n"
+      ".reg .pred p;\n"
+      "mbarrier.test_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n"
+      "selp.u32 %0, 1, 0, p;\n"
+      "}\n"
+      : "=r"(ok)
+      : "r"(bar), "r"(parity)
+      : "memory");
+  return ok;
 }
 __device__ __forceinline__ bool warp_wait_cluster(uint32_t bar, uint32_t parity, volatile int* abort_flag) {
   return warp_all(mbar_wait_cluster_abortable(bar, parity, abort_flag));
@@ -526,6 +570,30 @@ __host__ __device__ constexpr uint32_t umma_idesc(int m, int n, int ab_format) {
 }
 
 }  // namespace ptx
+
+// Host side: how many clusters of `size` CTAs (one CTA an SM) run at once.  Clusters do not cross the borders of the GPU's
+// SM groups, so fewer than SMs / size may fit; a persistent kernel that launched more would take a second wave.  The caller
+// keeps the answer.
+template <typename Kern>
+inline int max_clusters(Kern kern, int size, int threads, size_t smem, int sms) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)(sms / size * size));
+  cfg.blockDim = dim3((unsigned)threads);
+  cfg.dynamicSmemBytes = smem;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = (unsigned)size;
+  attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  int n = 0;
+  if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess ||
+      cudaOccupancyMaxActiveClusters(&n, kern, &cfg) != cudaSuccess || n < 1) {
+    cudaGetLastError();
+    n = sms / size * 3 / 4 > 0 ? sms / size * 3 / 4 : 1;
+  }
+  return n < sms / size ? n : sms / size;
+}
 
 // Host side: launch with programmatic stream serialization allowed (see grid_dependency_wait).
 template <typename... KArgs, typename... Args>

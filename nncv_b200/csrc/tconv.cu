@@ -80,14 +80,15 @@ struct TcParams {
 // BROW: the B operand is a plain row-major [K, N] matrix (linalg.matmul's right-hand side as it lies in
 // memory): 64 x 64 boxes of it land by TMA as MN-major 128-byte-swizzled tiles -- k rows of 128 bytes,
 // 8-row groups 1024 bytes apart, one box per 64 columns 8192 bytes apart -- and the instruction
-// descriptor marks B as MN-major, so nothing is repacked; rows and columns past the matrix read as zero.
+// descriptor marks B as MN-major, so nothing is repacked; rows and columns past the matrix read as zero.  On CTA pairs each
+// CTA brings half of the columns: 32 KB instead of 48 per 128 x 256 x 64 products.
 template <int BN, bool RESIDENT, bool DUAL, bool PAIR, bool BROW>
 __global__ void __launch_bounds__(kThreads, 1)
 tconv_kernel(const __grid_constant__ CUtensorMap tm_in, const __grid_constant__ CUtensorMap tm_out,
              const __grid_constant__ CUtensorMap tm_out2, const __grid_constant__ CUtensorMap tm_b,
-             const __grid_constant__ CUtensorMap tm_res, const TcParams p) {
+             const __grid_constant__ CUtensorMap tm_b2, const __grid_constant__ CUtensorMap tm_res, const TcParams p) {
   static_assert(!PAIR || !RESIDENT, "the pair kernel streams its weights");
-  static_assert(!BROW || (!RESIDENT && !DUAL && !PAIR), "a row-major B is streamed by one CTA");
+  static_assert(!BROW || (!RESIDENT && !DUAL), "a row-major B is streamed");
   constexpr int WTILE = (PAIR ? BN / 2 : BN) * 128;   // this CTA's part of a weight tile
   constexpr int ACC_W = DUAL ? 2 * BN : BN;   // columns of one accumulator buffer
   constexpr int ACC_COLS = 2 * ACC_W;         // two accumulator buffers
@@ -124,7 +125,7 @@ tconv_kernel(const __grid_constant__ CUtensorMap tm_in, const __grid_constant__ 
   if (threadIdx.x == 0) {
     s_abort = 0;
     for (int i = 0; i < kMaxStages; ++i) {
-      ptx::mbar_init(full + 8 * i, (PAIR && rank == 0) ? 2 : 1);   // leader: own copies + the peer's relay
+      ptx::mbar_init(full + 8 * i, 1);   // pair: only the leader's are used, for both CTAs' bytes
       ptx::mbar_init(empty + 8 * i, 1);
     }
     for (int i = 0; i < 2; ++i) {
@@ -137,7 +138,8 @@ tconv_kernel(const __grid_constant__ CUtensorMap tm_in, const __grid_constant__ 
     ptx::prefetch_tensormap(&tm_in);
     ptx::prefetch_tensormap(&tm_out);
     if (DUAL) ptx::prefetch_tensormap(&tm_out2);
-    if (BROW) ptx::prefetch_tensormap(&tm_b);
+    if (BROW || PAIR) ptx::prefetch_tensormap(&tm_b);
+    if (PAIR && DUAL) ptx::prefetch_tensormap(&tm_b2);
     if (p.residual) ptx::prefetch_tensormap(&tm_res);
   }
   if (warp == 1) {
@@ -188,11 +190,23 @@ tconv_kernel(const __grid_constant__ CUtensorMap tm_in, const __grid_constant__ 
   // Packed weights are the plan's own and nobody writes them once they are made, so their copies start before the previous
   // kernel of the stream has finished: everything the ring holds.  At small batches, where a kernel leaves most SMs idle,
   // that hides the whole weight fetch behind the previous layer.
-  auto weight_tile = [&](int n_tile, int cb, int tap) {
-    // pair: the weights are packed for N tile BN/2; this CTA takes tile 2 * n_tile + rank
-    const int wt = PAIR ? 2 * n_tile + (int)rank : n_tile;
-    return (DUAL && tap == p.taps) ? p.wpack2 + ((size_t)wt * p.CB + cb) * WTILE
-                                   : p.wpack + ((size_t)wt * KB + (size_t)tap * p.CB + cb) * WTILE;
+  const uint32_t full_lead = PAIR ? ptx::map_to_cta(full, 0) : full;
+  // the bytes of a stage, of both CTAs, are counted on the leader's barrier
+  auto expect_stage = [&](uint32_t st) {
+    if (!PAIR) ptx::mbar_arrive_expect_tx(full + 8 * st, (uint32_t)stage_bytes);
+    else if (rank == 0) ptx::mbar_arrive_expect_tx(full + 8 * st, 2u * (uint32_t)stage_bytes);
+  };
+  auto load_weights = [&](int n_tile, int cb, int tap, uint32_t st) {
+    const uint32_t dst = sRing + st * stage_bytes + kABytes;
+    const bool second = DUAL && tap == p.taps;
+    if (PAIR) {   // the weights are packed for N tile BN/2; this CTA takes tile 2 * n_tile + rank
+      const int wt = 2 * n_tile + (int)rank;
+      if (second) ptx::tma_load_2d_pair(dst, &tm_b2, 0, (wt * p.CB + cb) * (BN / 2), full_lead + 8 * st);
+      else ptx::tma_load_2d_pair(dst, &tm_b, 0, (wt * KB + tap * p.CB + cb) * (BN / 2), full_lead + 8 * st);
+    } else {
+      ptx::bulk_g2s(dst, second ? p.wpack2 + ((size_t)n_tile * p.CB + cb) * WTILE : p.wpack + ((size_t)n_tile * KB + (size_t)tap * p.CB + cb) * WTILE,
+                    WTILE, full + 8 * st);
+    }
   };
   uint32_t early = 0;   // ring stages whose weights are on their way
   auto load_resident = [&]() {
@@ -213,8 +227,8 @@ tconv_kernel(const __grid_constant__ CUtensorMap tm_in, const __grid_constant__ 
         if (!item_of(i, n0, oy0, ox0, n_tile)) break;
         for (int cb = 0; cb < p.CB && early < (uint32_t)p.stages; ++cb)
           for (int tap = 0; tap < taps_x && early < (uint32_t)p.stages; ++tap, ++early) {
-            ptx::mbar_arrive_expect_tx(full + 8 * early, (uint32_t)stage_bytes);
-            ptx::bulk_g2s(sRing + early * stage_bytes + kABytes, weight_tile(n_tile, cb, tap), WTILE, full + 8 * early);
+            expect_stage(early);
+            load_weights(n_tile, cb, tap, early);
           }
       }
     }
@@ -245,16 +259,19 @@ tconv_kernel(const __grid_constant__ CUtensorMap tm_in, const __grid_constant__ 
               const bool freed = PAIR ? ptx::mbar_wait_cluster_abortable(empty + 8 * st, ((cnt / (uint32_t)p.stages) & 1u) ^ 1u, abort_flag)
                                       : ptx::mbar_wait_abortable(empty + 8 * st, ((cnt / (uint32_t)p.stages) & 1u) ^ 1u, abort_flag);
               if (!freed) { okw = false; break; }
-              ptx::mbar_arrive_expect_tx(full + 8 * st, (uint32_t)stage_bytes);
+              expect_stage(st);
             }
             const uint32_t dst = sRing + st * stage_bytes;
-            ptx::tma_load_4d(dst, &tm_in, cb * 64, xb + s, yb + r, n0, full + 8 * st);
+            if (PAIR) ptx::tma_load_4d_pair(dst, &tm_in, cb * 64, xb + s, yb + r, n0, full_lead + 8 * st);
+            else ptx::tma_load_4d(dst, &tm_in, cb * 64, xb + s, yb + r, n0, full + 8 * st);
             if (BROW) {
 #pragma unroll
-              for (int j = 0; j < BN / 64; ++j)
-                ptx::tma_load_2d(dst + kABytes + (uint32_t)j * 8192u, &tm_b, n_tile * BN + j * 64, cb * 64, full + 8 * st);
+              for (int j = 0; j < WTILE / 8192; ++j) {
+                if (PAIR) ptx::tma_load_2d_pair(dst + kABytes + (uint32_t)j * 8192u, &tm_b, n_tile * BN + (int)rank * (BN / 2) + j * 64, cb * 64, full_lead + 8 * st);
+                else ptx::tma_load_2d(dst + kABytes + (uint32_t)j * 8192u, &tm_b, n_tile * BN + j * 64, cb * 64, full + 8 * st);
+              }
             } else if (!RESIDENT && !begun) {
-              ptx::bulk_g2s(dst + kABytes, weight_tile(n_tile, cb, tap), WTILE, full + 8 * st);
+              load_weights(n_tile, cb, tap, st);
             }
           }
         }
@@ -262,26 +279,7 @@ tconv_kernel(const __grid_constant__ CUtensorMap tm_in, const __grid_constant__ 
       if (!okw && p.error_flag) atomicCAS(p.error_flag, 0, (int)kErrWaitProducer);
     }
   } else if (warp == 1) {
-    if (PAIR && rank != 0) {
-      // ---------------------------------------------------------------- relay (peer CTA) ----
-      // tells the leader when this CTA's stage is full
-      if (lane == 0) {
-        const uint32_t lead_full = ptx::map_to_cta(full, 0);
-        uint32_t cnt = 0;
-        bool okw = true;
-        for (int i = 0; okw; ++i) {
-          int n0, oy0, ox0, n_tile;
-          if (!item_of(i, n0, oy0, ox0, n_tile)) break;
-          const int KBX = taps_x * p.CB;
-          for (int kb = 0; kb < KBX; ++kb, ++cnt) {
-            const uint32_t st = cnt % (uint32_t)p.stages;
-            if (!ptx::mbar_wait_abortable(full + 8 * st, (cnt / (uint32_t)p.stages) & 1u, abort_flag)) { okw = false; break; }
-            ptx::mbar_arrive_remote(lead_full + 8 * st);
-          }
-        }
-        if (!okw && p.error_flag) atomicCAS(p.error_flag, 0, (int)kErrWaitMma);
-      }
-    } else
+    if (!PAIR || rank == 0)
     // ------------------------------------------------------------------ MMA issuer ------
     {
       const uint32_t issue = ptx::elect_one();
@@ -291,7 +289,9 @@ tconv_kernel(const __grid_constant__ CUtensorMap tm_in, const __grid_constant__ 
       };
       bool okw = true;
       if (RESIDENT) okw = ptx::warp_wait(w_full, 0, abort_flag);
+      auto peek = [&](uint32_t bar, uint32_t parity) { return PAIR ? ptx::mbar_peek_cluster(bar, parity) : ptx::mbar_peek(bar, parity); };
       uint32_t st = 0, ring = 0, acc_cnt = 0;   // stage, parity of the ring's round
+      uint32_t seen = okw ? peek(full, 0) : 0u;
       for (int i = 0; okw; ++i) {
         int n0, oy0, ox0, n_tile;
         if (!item_of(i, n0, oy0, ox0, n_tile)) break;
@@ -302,8 +302,11 @@ tconv_kernel(const __grid_constant__ CUtensorMap tm_in, const __grid_constant__ 
         for (int cb = 0; cb < p.CB && okw; ++cb)
           for (int tap = 0; tap < taps_x; ++tap) {   // producer order: cb outer, tap inner
             const bool second = DUAL && tap == p.taps;
-            if (!wait(full + 8 * st, ring)) { okw = false; break; }
+            if (!ptx::warp_all(seen) && !wait(full + 8 * st, ring)) { okw = false; break; }
             ptx::tc_fence_after();
+            const bool wrap = st + 1 == (uint32_t)p.stages;
+            const uint32_t st_next = wrap ? 0u : st + 1, ring_next = ring ^ (wrap ? 1u : 0u);
+            seen = peek(full + 8 * st_next, ring_next);
             const uint32_t a_addr = sRing + st * stage_bytes;
             const uint32_t a_lo = ptx::smem_desc_k128_lo(a_addr);
             // MN-major B: leading-dimension offset 8192 bytes (next 64 columns), one k step of 16 = two 8-row groups
@@ -321,7 +324,8 @@ tconv_kernel(const __grid_constant__ CUtensorMap tm_in, const __grid_constant__ 
             }
             if (PAIR) ptx::tc_commit_pair(empty + 8 * st, issue);
             else ptx::tc_commit(empty + 8 * st, issue);
-            if (++st == (uint32_t)p.stages) { st = 0; ring ^= 1u; }
+            st = st_next;
+            ring = ring_next;
           }
         if (!okw) break;
         if (PAIR) ptx::tc_commit_pair(acc_full + 8 * ab, issue);
@@ -523,13 +527,26 @@ bool make_map_b(CUtensorMap* m, const void* ptr, CUtensorMapDataType dt, long lo
              CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
+// 2-D map over packed weights: `tiles` tiles of `rows` x 64 values that already lie in the order shared memory wants.
+bool make_map_w(CUtensorMap* m, const void* ptr, CUtensorMapDataType dt, int rows, long long tiles) {
+  auto enc = get_encode();
+  if (!enc) return false;
+  cuuint64_t gdim[2] = {64, (cuuint64_t)(tiles * rows)};
+  cuuint64_t gstr[1] = {128};
+  cuuint32_t box[2] = {64, (cuuint32_t)rows};
+  cuuint32_t estr[2] = {1, 1};
+  return enc(m, dt, 2, const_cast<void*>(ptr), gdim, gstr, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
+             CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
 template <int BN, bool RESIDENT, bool DUAL = false, bool PAIR = false, bool BROW = false>
 cudaError_t launch_cfg(const TconvArgs& a, TcParams p, cudaStream_t stream) {
   const size_t wtile = (size_t)(PAIR ? BN / 2 : BN) * 128;
   const int KB = p.taps * p.CB;
   const size_t stage = RESIDENT ? kABytes : kABytes + wtile;
   const size_t wres = RESIDENT ? (size_t)(KB + (DUAL ? p.CB : 0)) * wtile : 0;
-  p.epi_bufs = epi::pick_bufs(p.residual != 0, kSmemLimit - 1024 - kBarBytes, wres + 3 * stage, wres + 2 * stage);
+  // a long reduction (1024 and more) is better served by five stages than by a second staging buffer: one epilogue for many blocks
+  p.epi_bufs = epi::pick_bufs(p.residual != 0, kSmemLimit - 1024 - kBarBytes, wres + (PAIR && BROW && KB >= 16 ? 5 : 3) * stage, wres + 2 * stage);
   const size_t fixed = 1024 + (size_t)(epi::kWarps * p.epi_bufs) * epi::kBufBytes + kBarBytes;
   if (fixed + wres + 2 * stage > kSmemLimit) return cudaErrorInvalidConfiguration;
   size_t st = (kSmemLimit - fixed - wres) / stage;
@@ -555,7 +572,10 @@ cudaError_t launch_cfg(const TconvArgs& a, TcParams p, cudaStream_t stream) {
   CUtensorMap tm_res = tm_out;
   if (p.residual && !make_map4(&tm_res, a.residual, dt, 2, a.Kout, ol.pitch, ol.img_rows, a.N, 64, qw, qh, qn, 1, 1))
     return cudaErrorInvalidValue;
-  CUtensorMap tm_b = tm_out;
+  CUtensorMap tm_b = tm_out, tm_b2 = tm_out;
+  if (PAIR && !BROW && (!make_map_w(&tm_b, p.wpack, dt, BN / 2, (long long)p.n_tiles * 2 * KB) ||
+                        (DUAL && !make_map_w(&tm_b2, p.wpack2, dt, BN / 2, (long long)p.n_tiles * 2 * p.CB))))
+    return cudaErrorInvalidValue;
   if (BROW && !make_map_b(&tm_b, a.b_rowmajor, dt, a.b_rows, a.Kout)) return cudaErrorInvalidValue;
   auto kern = tconv_kernel<BN, RESIDENT, DUAL, PAIR, BROW>;
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
@@ -569,7 +589,8 @@ cudaError_t launch_cfg(const TconvArgs& a, TcParams p, cudaStream_t stream) {
     grid = dim3(gx, p.n_tiles);
   } else if (PAIR) {
     const long long items = (long long)((p.m_items + 1) / 2) * p.n_tiles;
-    const long long pairs = sms / 2;
+    static const int fit = max_clusters(kern, 2, kThreads, kSmemLimit, sms);   // the same on every device this library runs on
+    const long long pairs = fit;
     grid = dim3(2 * (unsigned)(items < pairs ? items : pairs), 1);
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = grid;
@@ -585,12 +606,12 @@ cudaError_t launch_cfg(const TconvArgs& a, TcParams p, cudaStream_t stream) {
     attr[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 2;
-    return cudaLaunchKernelEx(&cfg, kern, tm_in, tm_out, tm_out2, tm_b, tm_res, p);
+    return cudaLaunchKernelEx(&cfg, kern, tm_in, tm_out, tm_out2, tm_b, tm_b2, tm_res, p);
   } else {
     const long long items = (long long)p.m_items * p.n_tiles;
     grid = dim3((unsigned)(items < sms ? items : sms), 1);
   }
-  return launch_pdl(kern, grid, dim3(kThreads), smem, stream, tm_in, tm_out, tm_out2, tm_b, tm_res, p);
+  return launch_pdl(kern, grid, dim3(kThreads), smem, stream, tm_in, tm_out, tm_out2, tm_b, tm_b2, tm_res, p);
 }
 
 }  // namespace
@@ -632,7 +653,7 @@ cudaError_t launch_tconv(const TconvArgs& a, cudaStream_t stream) {
   const bool brow = a.b_rowmajor != nullptr;
   if (brow) {   // plain GEMM with a row-major B: K and N multiples of 8 (16-byte row pitches), nothing else
     if (a.ab == kF32 || a.C % 8 != 0 || a.Kout % 8 != 0 || a.R != 1 || a.S != 1 || a.stride != 1 || a.pad != 0 || a.wpack2 ||
-        a.pair || a.resident || a.b_rows != a.C || (reinterpret_cast<uintptr_t>(a.b_rowmajor) & 15))
+        a.resident || a.b_rows != a.C || (reinterpret_cast<uintptr_t>(a.b_rowmajor) & 15))
       return cudaErrorInvalidValue;
   } else if (a.ab == kF32 || !tconv_supported(a.C, a.Kout, a.out_dtype, a.Kout)) {
     return cudaErrorInvalidValue;
@@ -667,6 +688,10 @@ cudaError_t launch_tconv(const TconvArgs& a, cudaStream_t stream) {
   p.stages = 0;
   if (p.residual && p.out_f32) return cudaErrorInvalidValue;
   if (brow) {
+    if (a.pair) {   // CTA pairs: 256 x 256 (or 128) tiles
+      if (a.bn == 128) return launch_cfg<128, false, false, true, true>(a, p, stream);
+      return a.bn == 256 ? launch_cfg<256, false, false, true, true>(a, p, stream) : cudaErrorInvalidConfiguration;
+    }
     if (a.bn == 64) return launch_cfg<64, false, false, false, true>(a, p, stream);
     if (a.bn == 128) return launch_cfg<128, false, false, false, true>(a, p, stream);
     if (a.bn == 256) return launch_cfg<256, false, false, false, true>(a, p, stream);
