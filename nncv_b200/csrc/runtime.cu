@@ -12,6 +12,7 @@
 #include <condition_variable>
 #include <functional>
 #include <thread>
+#include <chrono>
 #include <cmath>
 #include <cstdarg>
 #include <cstdio>
@@ -27,6 +28,7 @@
 #include <nvtx3/nvToolsExt.h>
 
 #include "../../include/nncv_b200.h"
+#include "host_copy.h"
 #include "kernels.h"
 
 using namespace nncv_b200;
@@ -94,13 +96,14 @@ namespace {
 // current and kept until the process exits.  Every entry point works on the context of the
 // calling thread's current device, so kernels always run on the GPU that owns their buffers.
 struct Model;
+constexpr int kMaxParts = 8;   // of a batch in host memory
 struct Device {
   bool ready = false;
   int id = -1;
   cudaStream_t stream = nullptr;
   int* error_flag = nullptr;   // device
   cudaStream_t copy_stream = nullptr;  // host->device copies of a split batch
-  cudaEvent_t copy_done[5] = {nullptr, nullptr, nullptr, nullptr, nullptr};   // one per part + one ordering the copies after earlier work
+  cudaEvent_t copy_done[kMaxParts + 1] = {};   // one per part + one ordering the copies after earlier work
   cudaStream_t user_stream = nullptr;  // stream _mlir_ciface_forward runs on when set
   bool user_stream_set = false;
   int sm_count = 148;
@@ -271,6 +274,32 @@ bool is_device_ptr(const void* p) {
   }
   return attr.type == cudaMemoryTypeDevice || attr.type == cudaMemoryTypeManaged;
 }
+
+// Page-locked host memory the copy engine reads directly?
+bool is_pinned_ptr(const void* p) {
+  cudaPointerAttributes attr;
+  if (cudaPointerGetAttributes(&attr, p) != cudaSuccess) {
+    cudaGetLastError();
+    return false;
+  }
+  return attr.type == cudaMemoryTypeHost;
+}
+
+struct PinnedBuf {   // page-locked host memory
+  void* p = nullptr;
+  size_t bytes = 0;
+  ~PinnedBuf() { if (p) cudaFreeHost(p); }
+  PinnedBuf() = default;
+  PinnedBuf(const PinnedBuf&) = delete;
+  PinnedBuf& operator=(const PinnedBuf&) = delete;
+  int reserve(size_t n) {
+    if (n <= bytes) return NNCV_B200_OK;
+    if (p) { cudaFreeHost(p); p = nullptr; bytes = 0; }
+    if (cudaHostAlloc(&p, n, cudaHostAllocDefault) != cudaSuccess) return fail(NNCV_B200_ENOMEM, "cudaHostAlloc(%zu) failed", n);
+    bytes = n;
+    return NNCV_B200_OK;
+  }
+};
 
 struct DevBuf {
   void* p = nullptr;
@@ -1087,6 +1116,16 @@ struct Model {
   DevBuf arena;
   size_t act_bytes_unshared = 0;   // what one buffer per tensor would take
   size_t act_next = 0;
+  HostCopier copier;          // images from pageable memory
+  PinnedBuf result;           // status word, then logits on their way to pageable memory
+  size_t logits_off = 0;      // bytes: where the current part's logits go in logits_io / logits32
+  // How a batch in host memory is cut into parts: each way is run a few times, then the fastest is kept.
+  struct PartChoice {
+    std::vector<std::vector<int>> ways;   // sizes of the parts
+    std::vector<double> best;             // fastest call so far, seconds
+    int calls = 0, chosen = -1;
+  };
+  std::map<std::array<int, 4>, PartChoice> part_choice;   // by N, H, W, pinned
   static constexpr uintptr_t kFakeBase = (uintptr_t)0x7A00000000000000ull;   // planning pass: stand-in pointers
   void note_use(const void* p) {
     const uintptr_t v = (uintptr_t)p;
@@ -1256,8 +1295,14 @@ int model_build(Plan plan, const void* host_blob, size_t n_elements, size_t ele_
   return ok();
 }
 
+int reserve_logits(Model& m, size_t bytes) {
+  int rc = m.logits32.reserve(bytes);
+  return rc ? rc : m.logits_io.reserve(bytes);
+}
+
 int ensure_workspace(Model& m, int N, int H, int W) {
-  if (m.wsN == N && m.wsH == H && m.wsW == W) return NNCV_B200_OK;
+  // a workspace for more images of the same size serves fewer: every tensor starts at the same place, pads included
+  if (m.wsN >= N && m.wsH == H && m.wsW == W) return NNCV_B200_OK;
   const size_t es = dtype_size(m.act_dt);
   if (H < 1 || W < 1) return fail(NNCV_B200_EINVAL, "input %dx%d too small", H, W);
   cudaDeviceSynchronize();
@@ -1279,8 +1324,7 @@ int ensure_workspace(Model& m, int N, int H, int W) {
     const int cpad0 = m.act_dt == kF32 ? 4 : 8;
     if ((rc = m.in_nhwc.reserve((size_t)N * H * W * cpad0 * es))) return rc;
   }
-  if ((rc = m.logits32.reserve((size_t)N * of * sizeof(float)))) return rc;
-  if ((rc = m.logits_io.reserve((size_t)N * of * m.ele_width))) return rc;
+  if ((rc = reserve_logits(m, (size_t)N * of * sizeof(float)))) return rc;
   m.wsN = N; m.wsH = H; m.wsW = W;
   return NNCV_B200_OK;
 }
@@ -1295,7 +1339,7 @@ int next_act(Model& m, int N, int h, int w, int c, Layout l, cudaStream_t st, vo
     *out = (void*)(Model::kFakeBase + ((uintptr_t)(m.act_plan.size() - 1) << 8));
     return NNCV_B200_OK;
   }
-  if (m.act_next >= m.act_plan.size() || m.act_plan[m.act_next].bytes != bytes)
+  if (m.act_next >= m.act_plan.size() || m.act_plan[m.act_next].bytes < bytes || m.act_plan[m.act_next].geom != std::array<int, 3>{l.img_rows, l.pitch, c})
     return fail(NNCV_B200_ECUDA, "activation plan changed under a fixed shape");
   *out = (char*)m.arena.p + m.act_plan[m.act_next++].offset;
   return NNCV_B200_OK;
@@ -1339,7 +1383,7 @@ int model_forward_device(Model& m, const void* src_dev, int N, int H, int W, cud
     m.planning = true;
     m.act_plan.clear();
     m.op_idx = 0;
-    rc = model_forward_device(m, src_dev, N, H, W, st);
+    rc = model_forward_device(m, src_dev, m.wsN, H, W, st);
     m.planning = false;
     if (rc) return rc;
     if ((rc = finish_act_plan(m))) return rc;
@@ -1669,14 +1713,14 @@ int model_forward_device(Model& m, const void* src_dev, int N, int H, int W, cud
       if (m.io_dt == adt && adt != kF32) {
         // 16-bit logits wanted and computed in the same type: the FC epilogue rounds once, exactly as
         // the fp32 -> io conversion kernel would, and that kernel is not launched
-        return conv_run(fc, in.p, dense_layout(1, 1), m.logits_io.p, dense_layout(1, 1), N, 1, 1, nullptr, bias, nullptr, 0, adt, of,
+        return conv_run(fc, in.p, dense_layout(1, 1), (char*)m.logits_io.p + m.logits_off, dense_layout(1, 1), N, 1, 1, nullptr, bias, nullptr, 0, adt, of,
                         st);
       }
-      rc = m.planes ? conv_run_planes(fc, in.p, false, N, 1, 1, nullptr, bias, nullptr, 0, 0, m.logits32.p, 1, of, st)
-                    : conv_run(fc, in.p, dense_layout(1, 1), m.logits32.p, dense_layout(1, 1), N, 1, 1, nullptr, bias, nullptr, 0, kF32, of, st);
+      rc = m.planes ? conv_run_planes(fc, in.p, false, N, 1, 1, nullptr, bias, nullptr, 0, 0, (char*)m.logits32.p + m.logits_off, 1, of, st)
+                    : conv_run(fc, in.p, dense_layout(1, 1), (char*)m.logits32.p + m.logits_off, dense_layout(1, 1), N, 1, 1, nullptr, bias, nullptr, 0, kF32, of, st);
       if (rc) return rc;
       if (m.io_dt != kF32)
-        LAUNCH(launch_convert(m.logits32.p, kF32, m.logits_io.p, m.io_dt, (size_t)N * of, st));
+        LAUNCH(launch_convert((char*)m.logits32.p + m.logits_off, kF32, (char*)m.logits_io.p + m.logits_off, m.io_dt, (size_t)N * of, st));
       return NNCV_B200_OK;
     }
   }
@@ -1719,50 +1763,147 @@ int check_dst(nncv_memref2* dst, int N, int of, size_t ele_width, bool* allocate
   return NNCV_B200_OK;
 }
 
+// Slice [lo, hi) of n items owned by part `rank` of `world`: the first n % world parts get one more.
+void shard_range(int n, int rank, int world, int* lo, int* hi) {
+  const int base = n / world, extra = n % world;
+  *lo = rank * base + (rank < extra ? rank : extra);
+  *hi = *lo + base + (rank < extra ? 1 : 0);
+}
+
 // One device's share of a forward: images [sp, sp + N images) -> logits rows at dp (row pitch
 // dst_stride elements).  Runs on the calling thread's current device (g_dev), on stream st;
 // synchronises and reads the device status word unless device_only.
 int forward_slice(Model& m, const char* sp, bool src_dev, char* dp, bool dst_dev, size_t dst_stride, int N, int H, int W,
                   cudaStream_t st, bool device_only) {
   int rc;
-  const size_t ew = m.ele_width;
-  const int of = m.plan.out_features;
+  const size_t ew = m.ele_width, row = (size_t)m.plan.out_features * ew;
+  if (src_dev) {
+    if ((rc = ensure_workspace(m, N, H, W))) return rc;
+    m.logits_off = 0;
+    if ((rc = model_forward_device(m, sp, N, H, W, st))) return rc;
+    const void* logits = m.io_dt == kF32 ? m.logits32.p : m.logits_io.p;
+    if (device_only && dst_stride * ew == row) CU(cudaMemcpyAsync(dp, logits, row * N, cudaMemcpyDeviceToDevice, st));
+    else CU(cudaMemcpy2DAsync(dp, dst_stride * ew, logits, row, row, (size_t)N, dst_dev ? cudaMemcpyDeviceToDevice : cudaMemcpyDeviceToHost, st));
+    if (device_only) return ok();
+    CU(cudaStreamSynchronize(st));
+    if ((rc = check_kernel_status())) return rc;
+    return ok();
+  }
+  // Images in host memory: a batch may run in parts, so that the copies of later parts overlap the forward of earlier ones
+  // (copies on their own stream, ordered by events).  More parts leave less of the last one exposed but make smaller, less
+  // efficient forwards -- which way wins depends on the network and the link, so the first calls of a shape try each (a call
+  // to let the layers tune themselves, two that count).  ResNet-18 fp16 256x224 from pinned memory (1.41 ms of copying):
+  // 2.20 ms in halves with blocking reads of logits and status, 2.03 ms now (quarters lose more to smaller forwards than
+  // they hide).  fp32 convolutions split their sums by the batch, so there a batch keeps one way.
   const size_t img_bytes = (size_t)3 * H * W * ew;
-  // Host input, large batch: run the batch as two halves so that the host->device copy of the
-  // second half overlaps the forward of the first (copies on their own stream, ordered by events).
-  // Four parts were slower at batch 256 (2.48 ms against 2.27 ms): four forwards of 64 images take
-  // longer than two of 128, and the kernels, not the copy, are then the longer leg.
-  const int chunks = (!src_dev && !device_only && N >= 128 && N % 2 == 0) ? 2 : 1;
-  const int Nc = N / chunks;
-  if ((rc = ensure_workspace(m, Nc, H, W))) return rc;
-  if (!src_dev && (rc = m.in_stage.reserve((size_t)N * img_bytes))) return rc;
-  if (chunks > 1) {
+  const bool pinned = is_pinned_ptr(sp);
+  const bool halves = N >= 128 && N % 2 == 0;
+  std::vector<int> parts = halves ? std::vector<int>{N / 2, N / 2} : std::vector<int>{N};
+  Model::PartChoice* choice = nullptr;
+  int way = -1;
+  if (m.act_dt != kF32 && N >= 16 && g_autotune) {
+    choice = &m.part_choice[{N, H, W, (int)pinned}];
+    if (choice->ways.empty()) {
+      choice->ways.push_back(parts);
+      for (int n : {1, 2, 4, 8}) {
+        std::vector<int> w;
+        for (int r = 0; r < n; ++r) {
+          int lo, hi;
+          shard_range(N, r, n, &lo, &hi);
+          w.push_back(hi - lo);
+        }
+        if (w.back() < 8 || w == parts) continue;
+        choice->ways.push_back(w);
+        if (n == 4 && w.back() >= 16) {   // the last quarter in halves
+          const int h = w.back() / 2;
+          w.back() -= h;
+          w.push_back(h);
+          choice->ways.push_back(w);
+        }
+      }
+      choice->best.assign(choice->ways.size(), 1e30);
+    }
+    way = choice->chosen >= 0 ? choice->chosen : choice->calls / 3;
+    parts = choice->ways[(size_t)way];
+  }
+  const auto t0 = std::chrono::steady_clock::now();
+  const int most = *std::max_element(parts.begin(), parts.end());
+  if ((rc = ensure_workspace(m, most, H, W))) return rc;
+  if (m.in_stage.bytes < (size_t)N * img_bytes) {
+    cudaDeviceSynchronize();
+    if ((rc = m.in_stage.reserve((size_t)N * img_bytes))) return rc;
+  }
+  // logits of the parts one after another, each on a 256-byte boundary
+  auto part_bytes = [&](int n) { return ((size_t)n * m.plan.out_features * sizeof(float) + 255) & ~(size_t)255; };
+  size_t logits_bytes = 0;
+  for (int n : parts) logits_bytes += part_bytes(n);
+  if (m.logits_io.bytes < logits_bytes || m.logits32.bytes < logits_bytes) {
+    cudaDeviceSynchronize();
+    if ((rc = reserve_logits(m, logits_bytes))) return rc;
+  }
+  const bool stage_out = !dst_dev && !is_pinned_ptr(dp) && row * N <= (4u << 20);   // small results leave through pinned memory
+  if ((rc = m.result.reserve(256 + (stage_out ? row * N : 0)))) return rc;
+  cudaStream_t cst = st;
+  if (parts.size() > 1) {
     if (!g_dev.copy_stream) {
       CU(cudaStreamCreateWithFlags(&g_dev.copy_stream, cudaStreamNonBlocking));
       for (auto& e : g_dev.copy_done) CU(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
     }
+    cst = g_dev.copy_stream;
     // the copy stream must not overwrite the staging buffer before earlier work on `st` has read it
-    CU(cudaEventRecord(g_dev.copy_done[4], st));
-    CU(cudaStreamWaitEvent(g_dev.copy_stream, g_dev.copy_done[4], 0));
-    for (int c = 0; c < chunks; ++c) {
-      CU(cudaMemcpyAsync((char*)m.in_stage.p + (size_t)c * Nc * img_bytes, sp + (size_t)c * Nc * img_bytes,
-                         (size_t)Nc * img_bytes, cudaMemcpyHostToDevice, g_dev.copy_stream));
-      CU(cudaEventRecord(g_dev.copy_done[c], g_dev.copy_stream));
-    }
-  } else if (!src_dev) {
-    CU(cudaMemcpyAsync(m.in_stage.p, sp, (size_t)N * img_bytes, cudaMemcpyHostToDevice, st));
+    CU(cudaEventRecord(g_dev.copy_done[kMaxParts], st));
+    CU(cudaStreamWaitEvent(cst, g_dev.copy_done[kMaxParts], 0));
   }
-  for (int c = 0; c < chunks; ++c) {
-    const void* src_d = src_dev ? (const void*)sp : (const void*)((char*)m.in_stage.p + (size_t)c * Nc * img_bytes);
-    if (chunks > 1) CU(cudaStreamWaitEvent(st, g_dev.copy_done[c], 0));
-    if ((rc = model_forward_device(m, src_d, Nc, H, W, st))) return rc;
-    const void* logits = m.io_dt == kF32 ? m.logits32.p : m.logits_io.p;
-    CU(cudaMemcpy2DAsync(dp + (size_t)c * Nc * dst_stride * ew, dst_stride * ew, logits, (size_t)of * ew,
-                         (size_t)of * ew, (size_t)Nc, dst_dev ? cudaMemcpyDeviceToDevice : cudaMemcpyDeviceToHost, st));
+  auto copy_in = [&](size_t part, int first, int n) -> int {
+    char* to = (char*)m.in_stage.p + (size_t)first * img_bytes;
+    const char* from = sp + (size_t)first * img_bytes;
+    if (pinned || (size_t)n * img_bytes < HostCopier::kWorthIt) CU(cudaMemcpyAsync(to, from, (size_t)n * img_bytes, cudaMemcpyHostToDevice, cst));
+    else CU(m.copier.copy(to, from, (size_t)n * img_bytes, cst));
+    if (parts.size() > 1) CU(cudaEventRecord(g_dev.copy_done[part], cst));
+    return NNCV_B200_OK;
+  };
+  if (pinned) {   // nothing to wait for: all copies first
+    int first = 0;
+    for (size_t c = 0; c < parts.size(); first += parts[c++])
+      if ((rc = copy_in(c, first, parts[c]))) return rc;
   }
-  if (device_only) return ok();
+  const char* logits = (const char*)(m.io_dt == kF32 ? m.logits32.p : m.logits_io.p);
+  int first = 0;
+  m.logits_off = 0;
+  rc = NNCV_B200_OK;
+  for (size_t c = 0; c < parts.size() && !rc; first += parts[c++]) {
+    const int n = parts[c];
+    if (!pinned && (rc = copy_in(c, first, n))) break;
+    if (parts.size() > 1) CU(cudaStreamWaitEvent(st, g_dev.copy_done[c], 0));
+    if ((rc = model_forward_device(m, (char*)m.in_stage.p + (size_t)first * img_bytes, n, H, W, st))) break;
+    if (stage_out) CU(cudaMemcpyAsync((char*)m.result.p + 256 + row * first, logits + m.logits_off, row * n, cudaMemcpyDeviceToHost, st));
+    else CU(cudaMemcpy2DAsync(dp + (size_t)first * dst_stride * ew, dst_stride * ew, logits + m.logits_off, row, row, (size_t)n,
+                              dst_dev ? cudaMemcpyDeviceToDevice : cudaMemcpyDeviceToHost, st));
+    m.logits_off += part_bytes(n);
+  }
+  m.logits_off = 0;
+  if (rc) {
+    cudaStreamSynchronize(cst);   // the copies may still be reading the caller's memory
+    return rc;
+  }
+  int* status = (int*)m.result.p;
+  CU(cudaMemcpyAsync(status, g_dev.error_flag, sizeof(int), cudaMemcpyDeviceToHost, st));
   CU(cudaStreamSynchronize(st));
-  if ((rc = check_kernel_status())) return rc;
+  if (*status != 0) {
+    cudaMemset(g_dev.error_flag, 0, sizeof(int));
+    return report_kernel_error(*status, "forward");
+  }
+  if (stage_out)
+    for (int r = 0; r < N; ++r) memcpy(dp + (size_t)r * dst_stride * ew, (char*)m.result.p + 256 + row * r, row);
+  if (choice && choice->chosen < 0) {
+    const double s = std::chrono::duration<double>(std::chrono::steady_clock::now() - t0).count();
+    if (choice->calls % 3 != 0 && s < choice->best[(size_t)way]) choice->best[(size_t)way] = s;
+    if (++choice->calls == 3 * (int)choice->ways.size()) {
+      choice->chosen = (int)(std::min_element(choice->best.begin(), choice->best.end()) - choice->best.begin());
+      log_line(1, "host batch %d of %dx%d (%s): %zu parts, %.0f us", N, H, W, pinned ? "pinned" : "pageable",
+               choice->ways[(size_t)choice->chosen].size(), 1e6 * choice->best[(size_t)choice->chosen]);
+    }
+  }
   return ok();
 }
 
@@ -1821,13 +1962,6 @@ int forward_impl(nncv_memref2* dst, nncv_memref4* src, void* params, cudaStream_
 // sequence would otherwise queue behind the other devices' on one thread); the calling thread serves
 // the first device of the group.  nncv itself is single-device (include/nncv/compiler/Utils/
 // PlatformCtx.hpp:140-144 warns when the GPU count is not 1).
-
-// Slice [lo, hi) of n items owned by part `rank` of `world`: the first n % world parts get one more.
-void shard_range(int n, int rank, int world, int* lo, int* hi) {
-  const int base = n / world, extra = n % world;
-  *lo = rank * base + (rank < extra ? rank : extra);
-  *hi = *lo + base + (rank < extra ? 1 : 0);
-}
 
 struct Worker {
   std::thread th;
