@@ -52,10 +52,12 @@ __device__ __forceinline__ float tf32_round(float x) {
 struct GtParams {
   const float* bias;
   const float* B;
+  float* C;
   int* error_flag;
   int M, N, K;
   int m_tiles, n_tiles, k_blocks;
   int relu;
+  int splits;   // CTAs of a cluster that share a tile's k blocks (then every cluster has one tile); 1: no clusters
 };
 
 __global__ void __launch_bounds__(kThreads, 1)
@@ -107,8 +109,11 @@ gemm_tf32x3_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_consta
   volatile int* abort_flag = &s_abort;
 
   const int total = p.m_tiles * p.n_tiles;
+  const int S = p.splits;
+  const int rank = S > 1 ? (int)ptx::cluster_ctarank() : 0;
+  const int kb_lo = (int)((long long)p.k_blocks * rank / S), kb_hi = (int)((long long)p.k_blocks * (rank + 1) / S);
   auto item_of = [&](int i, int& m0, int& n0) {
-    const int w = (int)blockIdx.x + i * (int)gridDim.x;
+    const int w = (int)blockIdx.x / S + i * ((int)gridDim.x / S);
     if (w >= total) return false;
     const int mt = w / p.n_tiles;
     m0 = mt * 128;
@@ -124,7 +129,7 @@ gemm_tf32x3_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_consta
       for (int i = 0; okw; ++i) {
         int m0, n0;
         if (!item_of(i, m0, n0)) break;
-        for (int kb = 0; kb < p.k_blocks; ++kb, ++cnt) {
+        for (int kb = kb_lo; kb < kb_hi; ++kb, ++cnt) {
           const uint32_t st = cnt % kStages;
           if (!ptx::mbar_wait_abortable(empty + 8 * st, ((cnt / kStages) & 1u) ^ 1u, abort_flag)) { okw = false; break; }
           ptx::mbar_arrive_expect_tx(full + 8 * st, kTile);
@@ -150,7 +155,7 @@ gemm_tf32x3_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_consta
         // cuts (does not round) every accumulation into TMEM, an error of one sign per step: keeping the
         // large sum to one step per k block of 8 instead of three makes it three times smaller
         const uint32_t d = tmem_base + ab * (2 * kBN), dl = d + kBN;
-        for (int kb = 0; kb < p.k_blocks; ++kb, ++cnt) {
+        for (int kb = kb_lo; kb < kb_hi; ++kb, ++cnt) {
           const uint32_t st = cnt % kStages;
           if (!ptx::warp_wait(conv + 8 * st, (cnt / kStages) & 1u, abort_flag)) { okw = false; break; }
           ptx::tc_fence_after();
@@ -163,9 +168,9 @@ gemm_tf32x3_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_consta
             const uint64_t al = ptx::desc_from_halves(a_lo + k4 * 2, ptx::kSmemDescK128Hi);
             const uint64_t bh = ptx::desc_from_halves(b_hi + k4 * 2, ptx::kSmemDescK128Hi);
             const uint64_t bl = ptx::desc_from_halves(b_lo + k4 * 2, ptx::kSmemDescK128Hi);
-            ptx::umma_tf32(dl, al, bh, idesc, (kb | (int)k4) != 0 ? 1u : 0u, issue);
+            ptx::umma_tf32(dl, al, bh, idesc, kb != kb_lo || k4 != 0 ? 1u : 0u, issue);
             ptx::umma_tf32(dl, ah, bl, idesc, 1u, issue);
-            ptx::umma_tf32(d, ah, bh, idesc, (kb | (int)k4) != 0 ? 1u : 0u, issue);
+            ptx::umma_tf32(d, ah, bh, idesc, kb != kb_lo || k4 != 0 ? 1u : 0u, issue);
           }
           ptx::tc_commit(empty + 8 * st, issue);
         }
@@ -180,21 +185,26 @@ gemm_tf32x3_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_consta
     const int grp = (warp - 2) / kConvWarps;           // this group takes the stages with cnt % 2 == grp
     const int t = (threadIdx.x - 64) % kConvThreads;   // 0..127: column of the B tile / share of the A tile
     const uint32_t swz = (uint32_t)(t & 7);
-    uint32_t cnt = 0;
     bool okw = true;
-    for (int i = 0; okw; ++i) {
+    const uint32_t len = (uint32_t)(kb_hi - kb_lo);
+    float bv[32];
+    // this thread's column of the block with this number; false past the last one
+    auto load_b = [&](uint32_t cnt) {
+      const uint32_t i = cnt / len;
       int m0, n0;
-      if (!item_of(i, m0, n0)) break;
-      const int n = n0 + t;
-      for (int kb = 0; kb < p.k_blocks; ++kb, ++cnt) {
-        if ((cnt & 1u) != (uint32_t)grp) continue;
+      if (!item_of((int)i, m0, n0)) return false;
+      const int n = n0 + t, k0 = (kb_lo + (int)(cnt - i * len)) * 32;
+      const float* bp = p.B + (size_t)k0 * p.N + n;
+#pragma unroll
+      for (int k = 0; k < 32; ++k) bv[k] = (n < p.N && k0 + k < p.K) ? __ldg(bp + (size_t)k * p.N) : 0.0f;
+      return true;
+    };
+    {
+      bool more = load_b((uint32_t)grp);
+      for (uint32_t cnt = (uint32_t)grp; more; cnt += 2) {
         const uint32_t st = cnt % kStages;
         // the MMAs that read this stage last have finished: its B and lo tiles may be rewritten
         bool got = ptx::mbar_wait_abortable(empty + 8 * st, ((cnt / kStages) & 1u) ^ 1u, abort_flag);
-        float bv[32];
-        const float* bp = p.B + (size_t)(kb * 32) * p.N + n;
-#pragma unroll
-        for (int k = 0; k < 32; ++k) bv[k] = (n < p.N && kb * 32 + k < p.K) ? __ldg(bp + (size_t)k * p.N) : 0.0f;
         got = got && ptx::mbar_wait_abortable(full + 8 * st, (cnt / kStages) & 1u, abort_flag);
         if (!ptx::named_bar_and(4 + grp, kConvThreads, got)) { okw = false; break; }
         const uint32_t s0 = sRing + st * kStageBytes;
@@ -230,6 +240,7 @@ gemm_tf32x3_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_consta
         }
         ptx::fence_proxy_async_smem();
         ptx::mbar_arrive(conv + 8 * st);
+        more = load_b(cnt + 2);   // on its way while the group waits for the stage
       }
     }
     if (!okw && p.error_flag && t == 0) atomicCAS(p.error_flag, 0, (int)kErrWaitLoader);
@@ -249,6 +260,25 @@ gemm_tf32x3_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_consta
       const bool got = ptx::mbar_wait_abortable(acc_full + 8 * ab, (acc_cnt >> 1) & 1u, abort_flag);
       if (!ptx::named_bar_and(3, kEpiThreads, got)) { okw = false; break; }
       ptx::tc_fence_after();
+      if (S > 1) {   // partial sums into the ring, which nothing reads or fills any more: the tile's MMAs are complete
+        for (int sl = 0; sl < kBN / 32; ++sl) {
+          uint32_t acc[32], accl[32];
+          __syncwarp();
+          ptx::tmem_ld_32x32(tmem_base + ((uint32_t)(quad * 32) << 16) + ab * (2 * kBN) + (uint32_t)(sl * 32), acc);
+          ptx::tmem_ld_32x32(tmem_base + ((uint32_t)(quad * 32) << 16) + ab * (2 * kBN) + kBN + (uint32_t)(sl * 32), accl);
+          ptx::tmem_ld_wait();
+#pragma unroll
+          for (int c4 = 0; c4 < 8; ++c4) {
+            float o[4];
+#pragma unroll
+            for (int h = 0; h < 4; ++h) o[h] = __uint_as_float(acc[c4 * 4 + h]) + __uint_as_float(accl[c4 * 4 + h]);
+            asm volatile("st.shared.v4.f32 [%0], {%1,%2,%3,%4};" ::"r"(sRing + (uint32_t)row * (kBN * 4) + (((uint32_t)(sl * 8 + c4) ^ sw) << 4)),
+                         "f"(o[0]), "f"(o[1]), "f"(o[2]), "f"(o[3])
+                         : "memory");
+          }
+        }
+        break;
+      }
       for (int sl = 0; sl < kBN / 32; ++sl, ++jglob) {
         const uint32_t sb = (uint32_t)jglob & 1u;
         const int ncol = n0 + sl * 32;
@@ -293,6 +323,35 @@ gemm_tf32x3_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_consta
 
   ptx::tc_fence_before();
   __syncthreads();
+  if (S > 1) {
+    // every CTA finishes its share of the rows from all partial sums, in rank order: the result does not depend on timing
+    ptx::cluster_sync_all();
+    int m0, n0;
+    item_of(0, m0, n0);
+    const int n = n0 + lane * 4, rows = 128 / S;
+    float4 bias = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (p.bias && n < p.N) bias = make_float4(__ldg(p.bias + n), __ldg(p.bias + n + 1), __ldg(p.bias + n + 2), __ldg(p.bias + n + 3));
+    for (int r = rank * rows + warp; r < (rank + 1) * rows; r += kThreads / 32) {
+      if (n >= p.N || m0 + r >= p.M || s_abort) continue;
+      const uint32_t at = sRing + (uint32_t)r * (kBN * 4) + (((uint32_t)lane ^ (uint32_t)(r & 7)) << 4);
+      float4 part[8];
+#pragma unroll
+      for (int q = 0; q < 8; ++q)
+        if (q < S) part[q] = ptx::ld_cluster_f4(ptx::map_to_cta(at, (uint32_t)q));
+      float4 v = part[0];
+#pragma unroll
+      for (int q = 1; q < 8; ++q)
+        if (q < S) { v.x += part[q].x; v.y += part[q].y; v.z += part[q].z; v.w += part[q].w; }
+      v.x += bias.x; v.y += bias.y; v.z += bias.z; v.w += bias.w;
+      if (p.relu) {
+        v.x = !(v.x <= 0.0f) ? v.x : 0.0f; v.y = !(v.y <= 0.0f) ? v.y : 0.0f;
+        v.z = !(v.z <= 0.0f) ? v.z : 0.0f; v.w = !(v.w <= 0.0f) ? v.w : 0.0f;
+      }
+      *reinterpret_cast<float4*>(p.C + (size_t)(m0 + r) * p.N + n) = v;
+    }
+    __syncwarp();
+    ptx::cluster_sync_all();   // the peers' reads of this CTA's partial sums are over
+  }
   if (warp == 1) {
     __syncwarp();
     ptx::tmem_dealloc(tmem_base, 4 * kBN);
@@ -334,7 +393,7 @@ cudaError_t launch_gemm_tf32x3(const float* A, const float* B, float* C, int M, 
   if ((reinterpret_cast<uintptr_t>(A) & 15) || (reinterpret_cast<uintptr_t>(B) & 3) || (reinterpret_cast<uintptr_t>(C) & 15))
     return cudaErrorMisalignedAddress;
   GtParams p;
-  p.bias = bias; p.B = B; p.error_flag = error_flag; p.M = M; p.N = N; p.K = K; p.relu = relu;
+  p.bias = bias; p.B = B; p.C = C; p.error_flag = error_flag; p.M = M; p.N = N; p.K = K; p.relu = relu;
   p.m_tiles = (M + 127) / 128; p.n_tiles = (N + kBN - 1) / kBN; p.k_blocks = (K + 31) / 32;
   if ((long long)p.m_tiles * p.n_tiles > 0x7fffffffLL) return cudaErrorInvalidValue;
   CUtensorMap tm_a, tm_c;
@@ -344,7 +403,30 @@ cudaError_t launch_gemm_tf32x3(const float* A, const float* B, float* C, int M, 
   if (e != cudaSuccess) return e;
   const int sms = sm_count > 0 ? sm_count : 148;
   const int items = p.m_tiles * p.n_tiles;
-  return launch_pdl(gemm_tf32x3_kernel, dim3(items < sms ? items : sms), dim3(kThreads), smem, stream, tm_a, tm_c, p);
+  // Fewer tiles than SMs: clusters split the k blocks of a tile, as far as all of them run at once and each CTA keeps four
+  // blocks (a block takes about 0.9 us, the exchange of partial sums 2).
+  static int fit[9] = {};
+  p.splits = 1;
+  for (int s = 2; s <= 8; s *= 2) {
+    if (fit[s] == 0) fit[s] = max_clusters(gemm_tf32x3_kernel, s, kThreads, smem, sms);
+    if (items > fit[s] || p.k_blocks < 4 * s) break;
+    p.splits = s;
+  }
+  if (p.splits == 1) return launch_pdl(gemm_tf32x3_kernel, dim3(items < sms ? items : sms), dim3(kThreads), smem, stream, tm_a, tm_c, p);
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)(items * p.splits));
+  cfg.blockDim = dim3(kThreads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  attr[1].id = cudaLaunchAttributeClusterDimension;
+  attr[1].val.clusterDim.x = (unsigned)p.splits;
+  attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 2;
+  return cudaLaunchKernelEx(&cfg, gemm_tf32x3_kernel, tm_a, tm_c, p);
 }
 
 }  // namespace nncv_b200
