@@ -12,14 +12,21 @@
 // Alo*Blo term being about 2^-24 of the product.
 // Data path: kind::tf32 takes K-major operands only (an MN-major B, which the 16-bit kinds accept,
 // gives wrong products -- measured), so the row-major B[K,N] is transposed on the way in.  TMA lands
-// 128 x 32 fp32 tiles of A with the 128-byte swizzle; two groups of four converter warps take
-// alternate stages: a thread owns one column n of the 32 x 128 B tile, reads its 32 k values with
-// coalesced global loads (a warp reads 128 contiguous bytes of a row of B per load), and writes them
-// as row n of the K-major hi and lo tiles in the swizzled layout; the same group rewrites the A tile
-// in place as hi and writes A's lo twin at the same offsets.  One thread issues 3 x 4 MMAs per stage;
-// four epilogue warps drain the accumulator (double-buffered in TMEM) through a swizzled staging slab
-// and TMA stores.  Out-of-range rows/columns read as zero and are clipped on store, so N and K need
+// 128 x 32 fp32 tiles of A with the 128-byte swizzle; three groups of four converter warps take the
+// stages in turn.  A thread owns one column n of the 32 x 128 B tile: its 32 k values come with coalesced
+// global loads (a warp reads 128 contiguous bytes of a row of B per load) that are under way while the
+// group waits for its stage, and it writes them as row n of the K-major hi and lo tiles in the swizzled
+// layout.  It also owns one row of A, which it splits into TENSOR MEMORY: the MMAs then read only B from
+// shared memory, 4 KB instead of 8 in the 64 clocks that 128 bytes a clock allow for.  One warp issues
+// 3 x 4 MMAs per stage; four epilogue warps drain the accumulator through a swizzled staging slab and TMA
+// stores.  TMEM holds one pair of accumulators and the A parts of four stages: a second pair would hide
+// the 2 us of an epilogue, but leaves no room for A (2048 x 2048 x 256 takes as long either way).
+// With fewer tiles than SMs, clusters share a tile's k blocks (see the launch).  What bounds it now: the
+// converters' chain, 1700 clocks a block of 32 in three groups, and for small matrices 13 us of launch, cold
+// reads and epilogue.  Out-of-range rows/columns read as zero and are clipped on store, so N and K need
 // only be multiples of 4 (16-byte row pitches of A and C).
+// Cold L2, us, before the clusters and A in tensor memory and with them: 1024^3 41.0, 25.6; 2048^3 137, 122;
+// 100x1000x2048 69.6, 19.5; 1900x1500x520 44.0, 39.9.
 // Every wait is bounded and abortable; a timed-out wait sets the device status word.
 #include <cuda.h>
 #include <cudaTypedefs.h>
@@ -35,12 +42,14 @@ namespace nncv_b200 {
 namespace {
 
 constexpr int kBN = 128;                   // N tile
-constexpr int kConvWarps = 4, kConvGroups = 2, kEpiWarps = 4;
+constexpr int kConvWarps = 4, kConvGroups = 3, kEpiWarps = 4;
 constexpr int kConvThreads = kConvWarps * 32, kEpiThreads = kEpiWarps * 32;
 constexpr int kThreads = 64 + kConvGroups * kConvThreads + kEpiThreads;
 constexpr int kTile = 128 * 128;           // bytes of one operand tile: 128 rows (pixels of A / columns of B) x 32 fp32
-constexpr int kStageBytes = 4 * kTile;     // A, A_lo, B, B_lo
-constexpr int kStages = 3;
+constexpr int kStageBytes = 3 * kTile;     // A as it came, B hi, B lo
+constexpr int kStages = 4;
+// TMEM: the accumulators of the hi*hi products and of the cross terms, then A hi and A lo of every stage
+constexpr uint32_t kTmemA = 2 * kBN, kTmemStage = 64;
 constexpr int kSlabBytes = 128 * 128;      // 128 rows x 32 fp32
 
 // Nearest tf32 value (10 mantissa bits; ties away from zero): rounding, unlike cutting the low bits,
@@ -70,8 +79,8 @@ gemm_tf32x3_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_consta
   const uint32_t sStage = sRing + kStages * kStageBytes;
   const uint32_t bars = sStage + 2 * kSlabBytes;
   const uint32_t full = bars, conv = bars + 8 * kStages, empty = conv + 8 * kStages;
-  const uint32_t acc_full = empty + 8 * kStages, acc_empty = acc_full + 16;
-  const uint32_t tmem_slot = acc_empty + 16;
+  const uint32_t acc_full = empty + 8 * kStages, acc_empty = acc_full + 8;
+  const uint32_t tmem_slot = acc_empty + 8;
   {
     uint32_t dyn_bytes;
     asm volatile("mov.u32 %0, %%dynamic_smem_size;" : "=r"(dyn_bytes));
@@ -88,16 +97,14 @@ gemm_tf32x3_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_consta
       ptx::mbar_init(conv + 8 * i, kConvThreads);
       ptx::mbar_init(empty + 8 * i, 1);
     }
-    for (int i = 0; i < 2; ++i) {
-      ptx::mbar_init(acc_full + 8 * i, 1);
-      ptx::mbar_init(acc_empty + 8 * i, kEpiThreads);
-    }
+    ptx::mbar_init(acc_full, 1);
+    ptx::mbar_init(acc_empty, kEpiThreads);
     ptx::mbar_fence_init();
     ptx::prefetch_tensormap(&tm_a);
     ptx::prefetch_tensormap(&tm_c);
   }
   if (warp == 1) {
-    ptx::tmem_alloc(tmem_slot, 4 * kBN);
+    ptx::tmem_alloc(tmem_slot, kTmemA + kStages * kTmemStage);
     ptx::tmem_relinquish();
   }
   ptx::tc_fence_before();
@@ -148,43 +155,41 @@ gemm_tf32x3_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_consta
       for (int i = 0; okw; ++i) {
         int m0, n0;
         if (!item_of(i, m0, n0)) break;
-        const uint32_t ab = acc_cnt & 1u;
-        if (!ptx::warp_wait(acc_empty + 8 * ab, ((acc_cnt >> 1) & 1u) ^ 1u, abort_flag)) { okw = false; break; }
+        if (!ptx::warp_wait(acc_empty, (acc_cnt & 1u) ^ 1u, abort_flag)) { okw = false; break; }
         ptx::tc_fence_after();
-        // two accumulators per buffer: the hi*hi products, and the two small cross terms.  The tensor core
+        // two accumulators: the hi*hi products, and the two small cross terms.  The tensor core
         // cuts (does not round) every accumulation into TMEM, an error of one sign per step: keeping the
         // large sum to one step per k block of 8 instead of three makes it three times smaller
-        const uint32_t d = tmem_base + ab * (2 * kBN), dl = d + kBN;
+        const uint32_t d = tmem_base, dl = d + kBN;
         for (int kb = kb_lo; kb < kb_hi; ++kb, ++cnt) {
           const uint32_t st = cnt % kStages;
           if (!ptx::warp_wait(conv + 8 * st, (cnt / kStages) & 1u, abort_flag)) { okw = false; break; }
           ptx::tc_fence_after();
           const uint32_t s0 = sRing + st * kStageBytes;
-          const uint32_t a_hi = ptx::smem_desc_k128_lo(s0), a_lo = ptx::smem_desc_k128_lo(s0 + kTile);
-          const uint32_t b_hi = ptx::smem_desc_k128_lo(s0 + 2 * kTile), b_lo = ptx::smem_desc_k128_lo(s0 + 3 * kTile);
+          const uint32_t a_hi = tmem_base + kTmemA + st * kTmemStage, a_lo = a_hi + 32;
+          const uint32_t b_hi = ptx::smem_desc_k128_lo(s0 + kTile), b_lo = ptx::smem_desc_k128_lo(s0 + 2 * kTile);
 #pragma unroll
-          for (uint32_t k4 = 0; k4 < 4; ++k4) {   // k step of 8 fp32 = 32 bytes along the rows of both operands
-            const uint64_t ah = ptx::desc_from_halves(a_hi + k4 * 2, ptx::kSmemDescK128Hi);
-            const uint64_t al = ptx::desc_from_halves(a_lo + k4 * 2, ptx::kSmemDescK128Hi);
+          for (uint32_t k4 = 0; k4 < 4; ++k4) {   // k step of 8 fp32: 8 columns of A, 32 bytes along the rows of B
             const uint64_t bh = ptx::desc_from_halves(b_hi + k4 * 2, ptx::kSmemDescK128Hi);
             const uint64_t bl = ptx::desc_from_halves(b_lo + k4 * 2, ptx::kSmemDescK128Hi);
-            ptx::umma_tf32(dl, al, bh, idesc, kb != kb_lo || k4 != 0 ? 1u : 0u, issue);
-            ptx::umma_tf32(dl, ah, bl, idesc, 1u, issue);
-            ptx::umma_tf32(d, ah, bh, idesc, kb != kb_lo || k4 != 0 ? 1u : 0u, issue);
+            ptx::umma_tf32_ts(dl, a_lo + k4 * 8, bh, idesc, kb != kb_lo || k4 != 0 ? 1u : 0u, issue);
+            ptx::umma_tf32_ts(dl, a_hi + k4 * 8, bl, idesc, 1u, issue);
+            ptx::umma_tf32_ts(d, a_hi + k4 * 8, bh, idesc, kb != kb_lo || k4 != 0 ? 1u : 0u, issue);
           }
           ptx::tc_commit(empty + 8 * st, issue);
         }
         if (!okw) break;
-        ptx::tc_commit(acc_full + 8 * ab, issue);
+        ptx::tc_commit(acc_full, issue);
         ++acc_cnt;
       }
       if (!okw && lane == 0 && p.error_flag) atomicCAS(p.error_flag, 0, (int)kErrWaitMma);
     }
   } else if (warp < 2 + kConvGroups * kConvWarps) {
     // ------------------------------------------------------------------ transpose B, hi / lo split ----
-    const int grp = (warp - 2) / kConvWarps;           // this group takes the stages with cnt % 2 == grp
+    const int grp = (warp - 2) / kConvWarps;           // this group takes every kConvGroups-th block
     const int t = (threadIdx.x - 64) % kConvThreads;   // 0..127: column of the B tile / share of the A tile
     const uint32_t swz = (uint32_t)(t & 7);
+    const int quad = warp & 3;                         // tensor-memory lanes this warp may write
     bool okw = true;
     const uint32_t len = (uint32_t)(kb_hi - kb_lo);
     float bv[32];
@@ -201,31 +206,37 @@ gemm_tf32x3_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_consta
     };
     {
       bool more = load_b((uint32_t)grp);
-      for (uint32_t cnt = (uint32_t)grp; more; cnt += 2) {
+      for (uint32_t cnt = (uint32_t)grp; more; cnt += kConvGroups) {
         const uint32_t st = cnt % kStages;
         // the MMAs that read this stage last have finished: its B and lo tiles may be rewritten
         bool got = ptx::mbar_wait_abortable(empty + 8 * st, ((cnt / kStages) & 1u) ^ 1u, abort_flag);
         got = got && ptx::mbar_wait_abortable(full + 8 * st, (cnt / kStages) & 1u, abort_flag);
         if (!ptx::named_bar_and(4 + grp, kConvThreads, got)) { okw = false; break; }
         const uint32_t s0 = sRing + st * kStageBytes;
-        // A at s0 -> hi in place, lo at s0 + kTile at the same (swizzled) offsets
-#pragma unroll 4
-        for (int c = t; c < kTile / 16; c += kConvThreads) {
-          const uint32_t src = s0 + (uint32_t)c * 16u;
-          float4 v;
-          asm volatile("ld.shared.v4.f32 {%0,%1,%2,%3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(src));
-          float hi[4], lo[4];
-          const float in[4] = {v.x, v.y, v.z, v.w};
+        ptx::tc_fence_after();   // the MMAs that read the stage's columns of A are over
+        // row (quad, lane) of A: out of shared memory, in two parts into tensor memory
+        const uint32_t arow = s0 + (uint32_t)(quad * 32 + lane) * 128u;
+        const uint32_t acol = tmem_base + ((uint32_t)(quad * 32) << 16) + kTmemA + st * kTmemStage;
 #pragma unroll
-          for (int e = 0; e < 4; ++e) {
-            hi[e] = tf32_round(in[e]);
-            lo[e] = tf32_round(in[e] - hi[e]);
+        for (int h = 0; h < 2; ++h) {
+          float hi[16], lo[16];
+#pragma unroll
+          for (int c = 0; c < 4; ++c) {
+            float4 v;
+            asm volatile("ld.shared.v4.f32 {%0,%1,%2,%3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w)
+                         : "r"(arow + (((uint32_t)(h * 4 + c) ^ (uint32_t)(lane & 7)) << 4)));
+            const float in[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+              hi[c * 4 + e] = tf32_round(in[e]);
+              lo[c * 4 + e] = tf32_round(in[e] - hi[c * 4 + e]);
+            }
           }
-          asm volatile("st.shared.v4.f32 [%0], {%1,%2,%3,%4};" ::"r"(src), "f"(hi[0]), "f"(hi[1]), "f"(hi[2]), "f"(hi[3]) : "memory");
-          asm volatile("st.shared.v4.f32 [%0], {%1,%2,%3,%4};" ::"r"(src + kTile), "f"(lo[0]), "f"(lo[1]), "f"(lo[2]), "f"(lo[3]) : "memory");
+          ptx::tmem_st_32x16(acol + h * 16, hi);
+          ptx::tmem_st_32x16(acol + 32 + h * 16, lo);
         }
         // column n of B becomes row t of the K-major tiles: 8 chunks of 4 k values, chunk index XOR (row % 8)
-        const uint32_t brow = s0 + 2 * kTile + (uint32_t)t * 128u;
+        const uint32_t brow = s0 + kTile + (uint32_t)t * 128u;
 #pragma unroll
         for (int j = 0; j < 8; ++j) {
           float hi[4], lo[4];
@@ -239,8 +250,10 @@ gemm_tf32x3_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_consta
           asm volatile("st.shared.v4.f32 [%0], {%1,%2,%3,%4};" ::"r"(dst + kTile), "f"(lo[0]), "f"(lo[1]), "f"(lo[2]), "f"(lo[3]) : "memory");
         }
         ptx::fence_proxy_async_smem();
+        ptx::tmem_st_wait();
+        ptx::tc_fence_before();
         ptx::mbar_arrive(conv + 8 * st);
-        more = load_b(cnt + 2);   // on its way while the group waits for the stage
+        more = load_b(cnt + kConvGroups);   // on its way while the group waits for the stage
       }
     }
     if (!okw && p.error_flag && t == 0) atomicCAS(p.error_flag, 0, (int)kErrWaitLoader);
@@ -256,16 +269,15 @@ gemm_tf32x3_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_consta
     for (int i = 0; okw; ++i) {
       int m0, n0;
       if (!item_of(i, m0, n0)) break;
-      const uint32_t ab = acc_cnt & 1u;
-      const bool got = ptx::mbar_wait_abortable(acc_full + 8 * ab, (acc_cnt >> 1) & 1u, abort_flag);
+      const bool got = ptx::mbar_wait_abortable(acc_full, acc_cnt & 1u, abort_flag);
       if (!ptx::named_bar_and(3, kEpiThreads, got)) { okw = false; break; }
       ptx::tc_fence_after();
       if (S > 1) {   // partial sums into the ring, which nothing reads or fills any more: the tile's MMAs are complete
         for (int sl = 0; sl < kBN / 32; ++sl) {
           uint32_t acc[32], accl[32];
           __syncwarp();
-          ptx::tmem_ld_32x32(tmem_base + ((uint32_t)(quad * 32) << 16) + ab * (2 * kBN) + (uint32_t)(sl * 32), acc);
-          ptx::tmem_ld_32x32(tmem_base + ((uint32_t)(quad * 32) << 16) + ab * (2 * kBN) + kBN + (uint32_t)(sl * 32), accl);
+          ptx::tmem_ld_32x32(tmem_base + ((uint32_t)(quad * 32) << 16) + (uint32_t)(sl * 32), acc);
+          ptx::tmem_ld_32x32(tmem_base + ((uint32_t)(quad * 32) << 16) + kBN + (uint32_t)(sl * 32), accl);
           ptx::tmem_ld_wait();
 #pragma unroll
           for (int c4 = 0; c4 < 8; ++c4) {
@@ -284,12 +296,12 @@ gemm_tf32x3_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_consta
         const int ncol = n0 + sl * 32;
         uint32_t acc[32], accl[32];
         __syncwarp();
-        ptx::tmem_ld_32x32(tmem_base + ((uint32_t)(quad * 32) << 16) + ab * (2 * kBN) + (uint32_t)(sl * 32), acc);
-        ptx::tmem_ld_32x32(tmem_base + ((uint32_t)(quad * 32) << 16) + ab * (2 * kBN) + kBN + (uint32_t)(sl * 32), accl);
+        ptx::tmem_ld_32x32(tmem_base + ((uint32_t)(quad * 32) << 16) + (uint32_t)(sl * 32), acc);
+        ptx::tmem_ld_32x32(tmem_base + ((uint32_t)(quad * 32) << 16) + kBN + (uint32_t)(sl * 32), accl);
         ptx::tmem_ld_wait();
         if (sl == kBN / 32 - 1) {
           ptx::tc_fence_before();
-          ptx::mbar_arrive(acc_empty + 8 * ab);
+          ptx::mbar_arrive(acc_empty);
         }
         const uint32_t srow = sStage + sb * kSlabBytes + (uint32_t)row * 128u;
 #pragma unroll
@@ -354,7 +366,7 @@ gemm_tf32x3_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_consta
   }
   if (warp == 1) {
     __syncwarp();
-    ptx::tmem_dealloc(tmem_base, 4 * kBN);
+    ptx::tmem_dealloc(tmem_base, kTmemA + kStages * kTmemStage);
   }
 }
 
