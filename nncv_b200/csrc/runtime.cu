@@ -407,6 +407,7 @@ struct nncv_b200_conv {
   bool force_gather = false;                       // algo 3: the cp.async gather kernel even where TMA would do
   std::map<std::array<int, 5>, ConvChoice> tuned;  // measured best kernel/tile per (N, H, W, residual, out type)
   Conv3x3Config cfg3{0, 0, 0};                     // algo 2: forced tile configuration (bn 0 = auto)
+  std::map<std::array<int, 4>, bool> dense_ways;   // algo 2 on dense tensors, per (N, H, W, residual): without conversions?
   std::map<std::array<int, 3>, bool> fuse_tuned;   // per (N, H, W): is the launch fused with the 1x1 branch faster?
 };
 
@@ -570,9 +571,11 @@ int conv_run(nncv_b200_conv* c, const void* in, Layout in_l, void* out, Layout o
   // ---- tensor-core kernels fed by TMA: the shifted-view 3x3 kernel (needs shared-pad layouts) and
   // the per-tap kernel.  Which one, and with which tile, is timed once per (plan, shape).
   const bool sv_ok = c->algo == 2 && in_l.off == 1 && out_l.off == 1 && out_dt == c->dtype && ldo == c->Kout;
-  if (c->algo == 2 && !sv_ok) return fail(NNCV_B200_EINVAL, "conv3x3: needs shared-pad NHWC input and output");
   const bool tc_ok = !g_force_gather && !c->force_gather && tconv_supported(c->Cpad, c->Kout, out_dt, ldo) && c->Kout >= 8;
-  if (sv_ok || (c->algo == 0 && tc_ok)) {
+  if (c->algo == 2 && !sv_ok && !tc_ok) return fail(NNCV_B200_EINVAL, "conv3x3: needs shared-pad NHWC input and output");
+  if (sv_ok || tc_ok) {
+    // a shape is tuned once for each pair of operands (residual, fused branch) and, of a plan that has both, layout
+    const int variant = (residual ? 1 : 0) + (fb ? 2 : 0) + (c->algo == 2 && !sv_ok ? 4 : 0);
     auto launch_choice = [&](const ConvChoice& ch, bool profile) -> int {
       const void* wpack = nullptr;
       // the CTA-pair kernels (7: shifted-view, 8: per-tap) read weights packed for half their N tile
@@ -650,11 +653,11 @@ int conv_run(nncv_b200_conv* c, const void* in, Layout in_l, void* out, Layout o
         if (c->cfg3.resident >= 2 && !sv_ok) { ch.kernel = 8; ch.resident = 0; }                      // per-tap kernel on CTA pairs
       }
     } else if (g_autotune) {
-      const std::array<int, 5> key{N, H, W, (residual ? 1 : 0) + (fb ? 2 : 0), (int)out_dt};
+      const std::array<int, 5> key{N, H, W, variant, (int)out_dt};
       auto it = c->tuned.find(key);
       char ckey[192];
       snprintf(ckey, sizeof(ckey), "conv c%d k%d r%d s%d st%d p%d dt%d a%d n%d h%d w%d res%d o%d", c->Cpad, c->Kout, c->R, c->S,
-               c->stride, c->pad, (int)c->dtype, c->algo, N, H, W, (residual ? 1 : 0) + (fb ? 2 : 0), (int)out_dt);
+               c->stride, c->pad, (int)c->dtype, c->algo, N, H, W, variant, (int)out_dt);
       if (it == c->tuned.end()) {
         if (const std::string* v = g_tune_cache.find(ckey)) {
           ConvChoice m;
@@ -2643,24 +2646,76 @@ int nncv_b200_conv_run(nncv_b200_conv* c, const void* in, void* out, int N, int 
   if (c->device != g_dev.id)
     return fail(NNCV_B200_EINVAL, "conv_run: the plan lives on device %d, the current device is %d", c->device, g_dev.id);
   if (c->algo == 2) {
-    // The kernel works on shared-pad NHWC; this entry point takes dense NHWC, so convert on both
-    // sides (the network executor keeps its activations in shared-pad form and skips this).
-    const Layout dl = dense_layout(H, W), sl = sp_layout(H, W);
-    const size_t es = dtype_size(c->dtype);
-    const size_t slots = (size_t)layout_slots(sl, N);
-    if ((rc = c->sp_in.reserve(slots * c->Cpad * es))) return rc;
-    if ((rc = c->sp_out.reserve(slots * c->Kout * es))) return rc;
-    LAUNCH(launch_relayout(in, dl, c->sp_in.p, sl, c->dtype, N, H, W, c->Cpad, st));
-    const void* res = nullptr;
-    if (residual) {
-      if ((rc = c->sp_res.reserve(slots * c->Kout * es))) return rc;
-      LAUNCH(launch_relayout(residual, dl, c->sp_res.p, sl, c->dtype, N, H, W, c->Kout, st));
-      res = c->sp_res.p;
+    // The shifted-view kernel works on shared-pad NHWC; this entry point takes dense NHWC, so convert on both sides (the
+    // network executor keeps its activations in shared-pad form and skips this) ...
+    auto shifted = [&]() -> int {
+      const Layout dl = dense_layout(H, W), sl = sp_layout(H, W);
+      const size_t es = dtype_size(c->dtype);
+      const size_t slots = (size_t)layout_slots(sl, N);
+      int rc;
+      if ((rc = c->sp_in.reserve(slots * c->Cpad * es))) return rc;
+      if ((rc = c->sp_out.reserve(slots * c->Kout * es))) return rc;
+      if (residual && (rc = c->sp_res.reserve(slots * c->Kout * es))) return rc;
+      LAUNCH(launch_relayout(in, dl, c->sp_in.p, sl, c->dtype, N, H, W, c->Cpad, st));
+      const void* res = nullptr;
+      if (residual) {
+        LAUNCH(launch_relayout(residual, dl, c->sp_res.p, sl, c->dtype, N, H, W, c->Kout, st));
+        res = c->sp_res.p;
+      }
+      rc = conv_run(c, c->sp_in.p, sl, c->sp_out.p, sl, N, H, W, scale, shift, res, relu, c->dtype, c->Kout, st);
+      if (rc) return rc;
+      LAUNCH(launch_relayout(c->sp_out.p, sl, out, dl, c->dtype, N, H, W, c->Kout, st));
+      return NNCV_B200_OK;
+    };
+    // ... or, with the same sums in the same order, the kernel that copies every tap's tile straight from the dense tensor:
+    // nine times the tile traffic, but no passes over the tensors besides.  Which is faster is timed once per shape, as the
+    // tiles are: 50x64x64x64 with a residual 64 us converted, 49 direct; 16x14x14x512 34 and 43.
+    auto direct = [&]() -> int {
+      return conv_run(c, in, Layout{0, 0, 0}, out, Layout{0, 0, 0}, N, H, W, scale, shift, residual, relu, c->dtype, c->Kout, st);
+    };
+    // (a result that lies over an operand needs the conversions' copies, and must not be computed twice)
+    const char* ob = (const char*)out;
+    const size_t px = (size_t)N * H * W * dtype_size(c->dtype);
+    auto over = [&](const void* q, size_t ch) { return q && ob < (const char*)q + px * ch && (const char*)q < ob + px * c->Kout; };
+    bool dense = false;
+    if (g_autotune && !over(in, c->Cpad) && !over(residual, c->Kout) && !g_force_gather && c->cfg3.bn == 0 && tconv_supported(c->Cpad, c->Kout, c->dtype, c->Kout)) {
+      const std::array<int, 4> key{N, H, W, residual ? 1 : 0};
+      char ckey[160];
+      snprintf(ckey, sizeof(ckey), "conv3x3 way c%d k%d dt%d n%d h%d w%d res%d", c->Cpad, c->Kout, (int)c->dtype, N, H, W, residual ? 1 : 0);
+      auto it = c->dense_ways.find(key);
+      if (it == c->dense_ways.end()) {
+        const std::string* v = g_tune_cache.find(ckey);
+        if (v && (*v == "0" || *v == "1")) it = c->dense_ways.emplace(key, *v == "1").first;
+      }
+      if (it == c->dense_ways.end()) {
+        cudaEvent_t e0, e1;
+        CU(cudaEventCreate(&e0));
+        CU(cudaEventCreate(&e1));
+        float ms[2] = {1e30f, 1e30f};
+        rc = NNCV_B200_OK;
+        for (int way = 0; way < 2 && !rc; ++way) {
+          if ((rc = way ? direct() : shifted())) break;   // tunes the tiles
+          for (int grp = 0; grp < 3 && !rc; ++grp) {
+            cudaEventRecord(e0, st);
+            for (int rep = 0; rep < 4 && !rc; ++rep) rc = way ? direct() : shifted();
+            cudaEventRecord(e1, st);
+            float t = 0.f;
+            if (cudaEventSynchronize(e1) == cudaSuccess && cudaEventElapsedTime(&t, e0, e1) == cudaSuccess && t < ms[way]) ms[way] = t;
+          }
+        }
+        cudaEventDestroy(e0);
+        cudaEventDestroy(e1);
+        if (rc) return rc;
+        int flag = 0;   // a kernel that gave up leaves early: nothing measured then counts
+        if ((rc = read_kernel_status(&flag))) return rc;
+        if (flag != 0) return report_kernel_error(flag, "conv_run");
+        it = c->dense_ways.emplace(key, ms[1] < ms[0]).first;
+        g_tune_cache.put(ckey, it->second ? "1" : "0");
+      }
+      dense = it->second;
     }
-    rc = conv_run(c, c->sp_in.p, sl, c->sp_out.p, sl, N, H, W, scale, shift, res, relu, c->dtype, c->Kout, st);
-    if (rc) return rc;
-    LAUNCH(launch_relayout(c->sp_out.p, sl, out, dl, c->dtype, N, H, W, c->Kout, st));
-    return ok();
+    rc = dense ? direct() : shifted();
+    return rc ? rc : ok();
   }
   if (c->algo == 1) {
     // Winograd F(2x2,3x3): input transform -> 16 GEMMs [tiles x C] * [C x Kout] -> output transform

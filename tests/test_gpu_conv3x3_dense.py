@@ -1,0 +1,37 @@
+"""3x3 plans for the shifted-view kernel on dense tensors: the way that is chosen by timing (converted to shared-pad form, or
+straight from the dense tensor) changes no bit, and a result laid over an operand is still right."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+torch = pytest.importorskip("torch")
+from nncv_b200._lib import BF16, F16, check, lib  # noqa: E402
+import gpu_util as G  # noqa: E402
+
+
+@pytest.mark.parametrize("n,c,h,w,k", [(1, 64, 7, 7, 64), (3, 64, 56, 40, 64), (5, 128, 17, 23, 192), (2, 256, 14, 14, 256), (9, 64, 64, 64, 64)])
+@pytest.mark.parametrize("dtype", [F16, BF16])
+@pytest.mark.parametrize("res", [False, True])
+def test_ways_agree(n, c, h, w, k, dtype, res):
+    r = np.random.default_rng(n * c + h)
+    wt = (r.standard_normal((k, c, 3, 3)) / np.sqrt(9 * c)).astype(np.float32)
+    X, R = (G.dev(r.standard_normal((n, h, w, ch)).astype(np.float32), dtype) for ch in (c, k))
+    S, B = torch.rand(k, device="cuda") + 0.5, torch.randn(k, device="cuda")
+    chosen, forced = G.Conv(wt, 1, 1, dtype, algo=2), G.Conv(wt, 1, 1, dtype, algo=2)
+    check(lib().nncv_b200_conv_set_tile(forced.h, 64, 1, 0))   # a forced tile is the shifted-view kernel's
+
+    def run(conv, x, y, residual):
+        check(lib().nncv_b200_conv_run(conv.h, G.p(x), G.p(y), n, h, w, G.p(S), G.p(B), G.p(residual), 1, G.stream_ptr()))
+        G.sync_check()
+        return y
+
+    want = run(forced, X, torch.zeros_like(R), R if res else None)
+    for _ in range(2):
+        assert torch.equal(run(chosen, X, torch.zeros_like(R), R if res else None), want)
+    if res:
+        over = R.clone()
+        assert torch.equal(run(chosen, X, over, over), want)
+    if c == k:
+        over = X.clone()
+        assert torch.equal(run(chosen, over, over, R if res else None), want)
