@@ -182,7 +182,7 @@ __device__ __forceinline__ void input_row(const TI* rowp, bool yin, int ix0, int
 }
 
 template <typename TI, bool BF16, bool VEC, int STRIDE>
-__global__ void __launch_bounds__(256) stem3x3_row_kernel(const TI* __restrict__ src, const float* __restrict__ w, const float* __restrict__ scale,
+__global__ void __launch_bounds__(256, 2) stem3x3_row_kernel(const TI* __restrict__ src, const float* __restrict__ w, const float* __restrict__ scale,
                                                           const float* __restrict__ shift, void* __restrict__ dst, Layout ol, int N, int H, int W,
                                                           int OH, int OW, int Cout, int pad, int act, int xgroups, long long total) {
   constexpr int NC = (kPX - 1) * STRIDE + 3;
