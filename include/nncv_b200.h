@@ -74,7 +74,7 @@ enum {
 enum { NNCV_B200_F32 = 0, NNCV_B200_F16 = 1, NNCV_B200_BF16 = 2 };
 
 typedef struct {
-  int compute_dtype; /* NNCV_B200_F32 (CUDA-core fp32 path), _F16 or _BF16 (tcgen05 path);
+  int compute_dtype; /* NNCV_B200_F32 (fp32 accuracy: three bf16 planes per operand, tcgen05), _F16 or _BF16 (tcgen05 path);
                         -1 = follow the params file: eleWidth 4 -> F32, 2 -> F16 */
   unsigned device_mask; /* 0: the model lives on the current CUDA device only.  Otherwise bit d set =
                         a replica of the weights on device d (the current device must be among them):
@@ -212,8 +212,9 @@ int nncv_flat_array_write(const char* path, size_t n, const nncv_memref_indexer*
 /* ---- single kernels (device pointers; `stream` is a cudaStream_t; no synchronisation) ----
  * linalg.matmul C[M,N] = A[M,K] * B[K,N], row-major (tests/MatMulOptimization/MatMulNv.mlir:6-9),
  * optional bias[N] (fp32) and ReLU.  ab_dtype F16/BF16: tcgen05 with fp32 accumulate, K % 8 == 0;
- * ab_dtype F32: CUDA-core fp32.  c_dtype is F32 or ab_dtype.  B is repacked into a scratch
- * buffer owned by the library (grown with cudaMalloc on demand). */
+ * ab_dtype F32: three tf32 products on tcgen05 where N, K >= 32, CUDA-core fp32 otherwise.  c_dtype is F32 or
+ * ab_dtype.  Where the shape does not let B be read as it lies, it is repacked into a scratch buffer owned by the
+ * library (grown with cudaMalloc on demand). */
 int nncv_b200_matmul(const void* A, const void* B, void* C, int M, int N, int K, int ab_dtype,
                      int c_dtype, const float* bias, int relu, void* stream);
 
