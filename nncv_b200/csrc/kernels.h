@@ -123,6 +123,9 @@ struct TconvArgs {
 };
 bool tconv_supported(int C, int Kout, DType out_dt, long long ldo);
 void tconv_tile(int N, int OH, int OW, int* tw, int* th, int* tn);
+// matmul with B as it lies in memory (one kernel, no scratch); false where the shape or an address needs a repacked B.
+bool matmul_direct(const void* A, const void* B, void* C, int M, int N, int K, DType ab, DType c, const float* bias, int relu, int sms,
+                   int* error_flag, TconvArgs* out);
 void tconv_pick(long long m_items, int C, int Kout, int taps, int* bn, int* resident);
 cudaError_t launch_tconv(const TconvArgs& a, cudaStream_t stream);
 

@@ -5,7 +5,7 @@
 // handed every byte of device memory to its own pool (so a later cudaMalloc fails or evicts),
 // or a latency-bound loop in which cudaMalloc's implicit device-wide synchronisation would stall
 // the other streams of the process.  For them this file keeps the scratch in a fixed array in
-// device memory that comes with the library image: nothing is allocated or freed, ever, by this
+// device memory that comes with the library image (unused where B can be read as it lies): nothing is allocated or freed, ever, by this
 // entry point.  The price is a size limit and one array per GPU for the life of the process.
 //
 // This entry point has no counterpart in nncv (the reference never touches a device).
@@ -107,9 +107,13 @@ extern "C" int nncv_b200_matmul_noalloc(const void* A, const void* B, void* C, i
   // the packed image is rewritten in full (padding included) by the pack kernel.
   cudaError_t e = cudaMemsetAsync(status_word, 0, sizeof(int), st);
   if (e != cudaSuccess) return internal_fail(NNCV_B200_ECUDA, "matmul_noalloc: cudaMemsetAsync failed: %s", cudaGetErrorString(e));
-  e = launch_pack_weights(B, (DType)ab_dtype, 1, N, 0, N, K, K, 1, bn, (DType)ab_dtype, packed, st);
+  TconvArgs d;   // B as it lies in memory, if it can be read so: then the array holds the status word only
+  const bool direct = matmul_direct(A, B, C, M, N, K, (DType)ab_dtype, (DType)c_dtype, bias, relu, g_sm_count[dev], status_word, &d);
+  if (!direct) e = launch_pack_weights(B, (DType)ab_dtype, 1, N, 0, N, K, K, 1, bn, (DType)ab_dtype, packed, st);
   if (e != cudaSuccess) return internal_fail(NNCV_B200_ECUDA, "matmul_noalloc: packing B failed: %s", cudaGetErrorString(e));
-  if (tma) {
+  if (direct) {
+    e = launch_tconv(d, st);
+  } else if (tma) {
     TconvArgs a;
     a.in = A; a.wpack = packed; a.shift = bias; a.out = C;
     a.N = 1; a.H = 1; a.W = M; a.OH = 1; a.OW = M; a.C = K; a.Kout = N;

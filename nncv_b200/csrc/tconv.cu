@@ -58,6 +58,8 @@ struct TcParams {
   int tiles_x, tiles_y, tiles_n, n_tiles, m_items;
   epi::FastDiv div_tx, div_ty, div_nt;   // by tiles_x, tiles_y, n_tiles
   int tail_start;   // matmul on pairs: items from here on are cut into halves by columns, one half a pair; -1: none
+  int splits;       // matmul: CTAs of a cluster that share a tile's channel blocks (then every cluster has one tile); 1: no clusters
+  void* out;        // the result, where it does not leave through tm_out
   int stages;                // A (+ streamed weight) ring depth
   int relu, bf16, out_f32;
   int w_ready;    // the packed weights were complete before this launch (not written by earlier work of its stream)
@@ -165,7 +167,11 @@ tconv_kernel(const __grid_constant__ CUtensorMap tm_in, const __grid_constant__ 
   // the end reads zeros and stores nothing.
   const int m_units = PAIR ? (p.m_items + 1) / 2 : p.m_items;
   const int total_items = RESIDENT ? m_units : m_units * p.n_tiles;
-  const int worker = PAIR ? (int)blockIdx.x >> 1 : (int)blockIdx.x, workers = PAIR ? (int)gridDim.x >> 1 : (int)gridDim.x;
+  constexpr bool CAN_SPLIT = BROW && !PAIR;
+  const int S = CAN_SPLIT ? p.splits : 1, krank = CAN_SPLIT && S > 1 ? (int)ptx::cluster_ctarank() : 0;
+  const int cb_lo = CAN_SPLIT ? p.CB * krank / S : 0, cb_hi = CAN_SPLIT ? p.CB * (krank + 1) / S : p.CB;
+  const int per_worker = PAIR ? 2 : S;
+  const int worker = (int)blockIdx.x / per_worker, workers = (int)gridDim.x / per_worker;
   // The last round of a matmul on pairs, when at most half of the pairs would have an item: every item is cut in two by
   // columns and the halves run side by side (4096^3, 256 items on 74 pairs: 138 -> 128 us).
   const int full_rounds = PAIR && BROW && p.tail_start >= 0 ? p.tail_start / workers : 0x7fffffff;
@@ -259,7 +265,7 @@ tconv_kernel(const __grid_constant__ CUtensorMap tm_in, const __grid_constant__ 
         const int xb = p.stride * ox0 - p.pad + p.in_off, yb = p.stride * oy0 - p.pad + p.in_off;
         // channel block outermost, taps innermost: the same accumulation order as the shifted-view
         // 3x3 kernel, so both kernels give bit-identical sums
-        for (int cb = 0; cb < p.CB && okw; ++cb) {
+        for (int cb = cb_lo; cb < cb_hi && okw; ++cb) {
           for (int tap = 0; tap < taps_x; ++tap, ++cnt) {
             const int gtap = tap < p.taps ? tap : p.taps / 2;   // the extra tap re-reads the centre tap's pixels
             const int r = gtap / p.S, s = gtap - r * p.S;
@@ -315,7 +321,7 @@ tconv_kernel(const __grid_constant__ CUtensorMap tm_in, const __grid_constant__ 
         ptx::tc_fence_after();
         const uint32_t d = tmem_base + ab * ACC_W;
         const uint32_t id = halved(i) ? idesc - ((uint32_t)(BN / 2 / 8) << 17) : idesc;   // N field
-        for (int cb = 0; cb < p.CB && okw; ++cb)
+        for (int cb = cb_lo; cb < cb_hi && okw; ++cb)
           for (int tap = 0; tap < taps_x; ++tap) {   // producer order: cb outer, tap inner
             const bool second = DUAL && tap == p.taps;
             if (!ptx::warp_all(seen) && !wait(full + 8 * st, ring)) { okw = false; break; }
@@ -330,7 +336,7 @@ tconv_kernel(const __grid_constant__ CUtensorMap tm_in, const __grid_constant__ 
                                        : ptx::smem_desc_k128_lo(
                 RESIDENT ? sW + (uint32_t)(second ? KB + cb : tap * p.CB + cb) * WTILE : a_addr + kABytes);
             constexpr uint32_t kBStep = BROW ? (2048u >> 4) : 2u;
-            const uint32_t first = second ? (uint32_t)cb : (uint32_t)(cb | tap);
+            const uint32_t first = second ? (uint32_t)cb : (uint32_t)((cb - cb_lo) | tap);
 #pragma unroll
             for (uint32_t k4 = 0; k4 < 4; ++k4) {
               const uint64_t da = ptx::desc_from_halves(a_lo + k4 * 2, ptx::kSmemDescK128Hi);
@@ -421,6 +427,20 @@ tconv_kernel(const __grid_constant__ CUtensorMap tm_in, const __grid_constant__ 
       okw = __all_sync(0xffffffffu, okw);
       if (!okw) break;
       ptx::tc_fence_after();
+      if (CAN_SPLIT && S > 1) {   // partial sums into the ring, which nothing reads or fills any more: the tile's MMAs are complete
+        const int row = quad * 32 + lane;
+#pragma unroll
+        for (int c = 0; c < BN / 64; ++c) {
+          const int col = half * (BN / 2) + c * 32;
+          uint32_t acc[32];
+          ptx::tmem_ld_32x32(tmem_base + ((uint32_t)(quad * 32) << 16) + (uint32_t)col, acc);
+          ptx::tmem_ld_wait();
+#pragma unroll
+          for (int e = 0; e < 8; ++e)
+            epi::sts128(sRing + (uint32_t)row * (BN * 4) + (((uint32_t)(col / 4 + e) ^ sw) << 4), acc[4 * e], acc[4 * e + 1], acc[4 * e + 2], acc[4 * e + 3]);
+        }
+        break;
+      }
       auto hand_back = [&]() {   // this warp has read its part of the accumulator
         ptx::tc_fence_before();
         __syncwarp();
@@ -494,6 +514,40 @@ tconv_kernel(const __grid_constant__ CUtensorMap tm_in, const __grid_constant__ 
   ptx::tc_fence_before();
   __syncthreads();
   if (PAIR) ptx::cluster_sync_all();   // the peer's shared memory and barriers stay valid until both are done
+  if (CAN_SPLIT && S > 1) {
+    // every CTA finishes its share of the rows from all partial sums, in rank order: the result does not depend on timing
+    ptx::cluster_sync_all();
+    int n0, oy0, ox0, n_tile;
+    item_of(0, n0, oy0, ox0, n_tile);
+    const int rows = 128 / S;
+    for (int idx = threadIdx.x; idx < rows * (BN / 4); idx += kThreads) {
+      const int r = krank * rows + idx / (BN / 4), c4 = idx % (BN / 4), n = n_tile * BN + c4 * 4;
+      if (n >= p.Kout || ox0 + r >= p.OW || s_abort) continue;
+      const uint32_t at = sRing + (uint32_t)r * (BN * 4) + (((uint32_t)c4 ^ (uint32_t)(r & 7)) << 4);
+      float4 part[8];
+#pragma unroll
+      for (int q = 0; q < 8; ++q)
+        if (q < S) part[q] = ptx::ld_cluster_f4(ptx::map_to_cta(at, (uint32_t)q));
+      float v[4] = {part[0].x, part[0].y, part[0].z, part[0].w};
+#pragma unroll
+      for (int q = 1; q < 8; ++q)
+        if (q < S) { v[0] += part[q].x; v[1] += part[q].y; v[2] += part[q].z; v[3] += part[q].w; }
+#pragma unroll
+      for (int e = 0; e < 4; ++e) v[e] = fmaf(v[e], p.scale ? __ldg(p.scale + n + e) : 1.0f, p.shift ? __ldg(p.shift + n + e) : 0.0f);
+      const size_t o = (size_t)(ox0 + r) * p.Kout + n;
+      if (p.out_f32) {
+        if (p.relu)
+#pragma unroll
+          for (int e = 0; e < 4; ++e) v[e] = !(v[e] <= 0.0f) ? v[e] : 0.0f;
+        *reinterpret_cast<float4*>(static_cast<float*>(p.out) + o) = make_float4(v[0], v[1], v[2], v[3]);
+      } else {
+        *reinterpret_cast<uint2*>(static_cast<unsigned short*>(p.out) + o) =
+            make_uint2(epi::pack16(v[0], v[1], p.bf16 != 0, p.relu != 0), epi::pack16(v[2], v[3], p.bf16 != 0, p.relu != 0));
+      }
+    }
+    __syncwarp();
+    ptx::cluster_sync_all();   // the peers' reads of this CTA's partial sums are over
+  }
   if (warp == 1) {
     __syncwarp();
     if (PAIR) ptx::tmem_dealloc_pair(tmem_base, ACC_COLS);
@@ -529,6 +583,7 @@ bool make_map4(CUtensorMap* m, const void* ptr, CUtensorMapDataType dt, int esz,
          CUDA_SUCCESS;
 }
 
+constexpr int kSplitBlocks = 4;   // matmul: fewest blocks of 64 of a CTA that shares a tile's depth
 constexpr size_t kSmemLimit = 222 * 1024;   // dynamic part: the kernel also holds 4 KB of static shared memory (scale / shift of the slabs in work)
 
 // 2-D map over a row-major [K, N] 16-bit matrix, box 64 columns x 64 rows, 128-byte swizzle, zero fill.
@@ -629,6 +684,32 @@ cudaError_t launch_cfg(const TconvArgs& a, TcParams p, cudaStream_t stream) {
     return cudaLaunchKernelEx(&cfg, kern, tm_in, tm_out, tm_out2, tm_b, tm_b2, tm_res, p);
   } else {
     const long long items = (long long)p.m_items * p.n_tiles;
+    if (BROW) {
+      // Fewer tiles than SMs: clusters split the depth of a tile, as far as all of them run at once and each CTA keeps
+      // kSplitBlocks blocks of 64.
+      static int fit[9] = {};
+      for (int s = 2; s <= 8; s *= 2) {
+        if (fit[s] == 0) fit[s] = max_clusters(kern, s, kThreads, kSmemLimit, sms);   // the same on every device this library runs on
+        if (items > fit[s] || p.CB < kSplitBlocks * s || st * stage < (size_t)BN * 512) break;
+        p.splits = s;
+      }
+      if (p.splits > 1) {
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3((unsigned)(items * p.splits));
+        cfg.blockDim = dim3(kThreads);
+        cfg.dynamicSmemBytes = smem;
+        cfg.stream = stream;
+        cudaLaunchAttribute attr[2];
+        attr[0].id = cudaLaunchAttributeClusterDimension;
+        attr[0].val.clusterDim.x = (unsigned)p.splits;
+        attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+        attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr[1].val.programmaticStreamSerializationAllowed = 1;
+        cfg.attrs = attr;
+        cfg.numAttrs = 2;
+        return cudaLaunchKernelEx(&cfg, kern, tm_in, tm_out, tm_out2, tm_b, tm_b2, tm_res, p);
+      }
+    }
     grid = dim3((unsigned)(items < sms ? items : sms), 1);
   }
   return launch_pdl(kern, grid, dim3(kThreads), smem, stream, tm_in, tm_out, tm_out2, tm_b, tm_b2, tm_res, p);
@@ -669,7 +750,18 @@ void tconv_tile(int N, int OH, int OW, int* tw, int* th, int* tn) {
   (void)N;
 }
 
-cudaError_t launch_tconv(const TconvArgs& a, cudaStream_t stream) {
+cudaError_t launch_tconv(const TconvArgs& args, cudaStream_t stream) {
+  TconvArgs a = args;
+  // a pointwise convolution between dense tensors is a matrix of N * H * W rows (a fully connected layer's tile would hold
+  // sixteen of its one-pixel images)
+  if (a.R == 1 && a.S == 1 && a.stride == 1 && a.pad == 0 && !a.wpack2 && a.in_l.off == 0 && a.in_l.pitch == a.W && a.in_l.img_rows == a.H &&
+      a.out_l.off == 0 && a.out_l.pitch == a.W && a.out_l.img_rows == a.H && (long long)a.N * a.H * a.W < (1LL << 30)) {
+    const int rows = a.N * a.H * a.W;
+    a.N = 1;
+    a.H = a.OH = 1;
+    a.W = a.OW = rows;
+    a.in_l = a.out_l = Layout{1, rows, 0};
+  }
   const bool brow = a.b_rowmajor != nullptr;
   if (brow) {   // plain GEMM with a row-major B: K and N multiples of 8 (16-byte row pitches), nothing else
     if (a.ab == kF32 || a.C % 8 != 0 || a.Kout % 8 != 0 || a.R != 1 || a.S != 1 || a.stride != 1 || a.pad != 0 || a.wpack2 ||
@@ -692,6 +784,9 @@ cudaError_t launch_tconv(const TconvArgs& a, cudaStream_t stream) {
   p.OH = a.OH; p.OW = a.OW; p.NB = a.N;
   p.out_pitch = a.out_l.pitch; p.out_rows = a.out_l.img_rows;
   tconv_tile(a.N, a.OH, a.OW, &p.tw, &p.th, &p.tn);
+  // a single row (a matrix) takes whole tiles: in pieces of 32 or 64, which leave less of the last one empty, most of EVERY
+  // tile would lie outside (fp16 matmul 3000x2000x1504: 51.2 -> 34.8 us)
+  if (a.N == 1 && a.OH == 1 && a.stride == 1) { p.tw = 128; p.th = p.tn = 1; }
   if (p.tw * a.stride > 256 || p.th * a.stride > 256) return cudaErrorInvalidConfiguration;
   p.tiles_x = (a.OW + p.tw - 1) / p.tw;
   p.tiles_y = (a.OH + p.th - 1) / p.th;
@@ -706,6 +801,8 @@ cudaError_t launch_tconv(const TconvArgs& a, cudaStream_t stream) {
   p.act = a.act;
   p.w_ready = a.weights_ready;
   p.tail_start = -1;
+  p.splits = 1;
+  p.out = a.out;
   p.stages = 0;
   if (p.residual && p.out_f32) return cudaErrorInvalidValue;
   if (brow) {
@@ -743,6 +840,47 @@ cudaError_t launch_tconv(const TconvArgs& a, cudaStream_t stream) {
   NNCV_TC(256, false)
 #undef NNCV_TC
   return cudaErrorInvalidConfiguration;
+}
+
+// N tile of a matmul with a row-major B: the least rounds x (blocks x time + epilogue), in us as measured with every SM at
+// work: a block of 64 of a 128 x 64 tile 0.42, 128 x 128 0.47, 256 x 256 on a CTA pair 0.63; a pair's launch and an exchange
+// of partial sums 2 each.  (Before, the widest tile that still filled the SMs: 2048^3 took two rounds of 128 x 128, 38.7 us,
+// where one of 64 pairs takes 28.3; 2048x1024x1024 two of 128 x 64, 22.4, where one of 128 x 128 takes 16.4.)
+static int matmul_pick(int M, int N, int K, int sms) {
+  static const double block[3] = {0.42, 0.47, 0.63}, epilogue[3] = {0.5, 0.9, 1.8};
+  const long long mi = ((long long)M + 127) / 128;
+  const int CB = (K + 63) / 64;
+  int best_bn = 64;
+  double best = 1e30;
+  for (int i = 0; i < 3; ++i) {
+    const int bn = 64 << i;
+    if (bn > 64 && N <= bn / 2) break;
+    const bool pair = bn == 256;
+    const long long items = (pair ? (mi + 1) / 2 : mi) * ((N + bn - 1) / bn), slots = pair ? sms / 2 : sms;
+    int s = 1;
+    while (!pair && s < 8 && items * 2 * s <= slots * 15 / 16 && CB >= kSplitBlocks * 2 * s) s *= 2;
+    const double t = (double)((items + slots - 1) / slots) * ((CB + s - 1) / s * block[i] + epilogue[i]) + (pair || s > 1 ? 2.0 : 0.0);
+    if (t < best) { best = t; best_bn = bn; }
+  }
+  return best_bn;
+}
+
+bool matmul_direct(const void* A, const void* B, void* C, int M, int N, int K, DType ab, DType c, const float* bias, int relu, int sms,
+                   int* error_flag, TconvArgs* out) {
+  if (N % 8 != 0 || N < 64 || K < 64 || (reinterpret_cast<uintptr_t>(A) & 15) || (reinterpret_cast<uintptr_t>(B) & 15) ||
+      (reinterpret_cast<uintptr_t>(C) & 15))
+    return false;
+  // 64 x 64 boxes of the row-major [K, N] matrix are MN-major operand tiles
+  TconvArgs& a = *out;
+  a.in = A; a.b_rowmajor = B; a.b_rows = K; a.shift = bias; a.out = C;
+  a.N = 1; a.H = 1; a.W = M; a.OH = 1; a.OW = M; a.C = K; a.Kout = N;
+  a.in_l = Layout{1, M, 0}; a.out_l = Layout{1, M, 0};
+  a.bn = matmul_pick(M, N, K, sms); a.resident = 0; a.ab = ab; a.out_dtype = c; a.relu = relu;
+  // 256 x 256 tiles on CTA pairs read each column of B from L2 half as often: 4096^3 fp16 148 -> 138 us, 8192x4096x512
+  // 38.8 -> 38.1, and 2048^3, with less than a round of pairs, no slower than 128 x 256 on single CTAs
+  a.pair = a.bn == 256;
+  a.sm_count = sms; a.error_flag = error_flag;
+  return true;
 }
 
 // N tile and residency: keep all weights of one Kout tile in shared memory when they fit beside
