@@ -680,8 +680,16 @@ static cudaError_t launch_f32_cfg(const CUtensorMap& tm, const F32Params& p, int
   return cudaLaunchKernelEx(&cfg, conv_f32_kernel<BN>, tm, p);
 }
 
-cudaError_t launch_conv_f32(const ConvF32Args& a, cudaStream_t stream) {
+cudaError_t launch_conv_f32(const ConvF32Args& args, cudaStream_t stream) {
+  ConvF32Args a = args;
   const bool stem = a.stem != 0;
+  // a pointwise convolution is a matrix of N * H * W rows: no tile straddles an image's border (a 7 x 7 map fills 49 of the 64
+  // slots of its half tile)
+  const bool matrix = !stem && a.R == 1 && a.S == 1 && a.stride == 1 && a.pad == 0 && (long long)a.N * a.H * a.W < (1LL << 30);
+  if (matrix) {
+    a.W = a.OW = a.N * a.H * a.W;
+    a.N = a.H = a.OH = 1;
+  }
   F32Params p{};
   p.wpack = static_cast<const uint8_t*>(a.wpack);
   p.scale = a.scale; p.shift = a.shift;
@@ -700,6 +708,7 @@ cudaError_t launch_conv_f32(const ConvF32Args& a, cudaStream_t stream) {
   p.res_plane = p.out_plane = pixels * a.Kout;
   int tw, th, tn;
   tconv_tile(a.N, a.OH, a.OW, &tw, &th, &tn);
+  if (matrix) { tw = 128; th = tn = 1; }
   if (!conv_f32_supported(stem ? 64 : a.C, a.Kout, (tw > th ? tw : th) * p.stride)) return cudaErrorInvalidValue;
   if ((reinterpret_cast<uintptr_t>(a.in) & 15) || (reinterpret_cast<uintptr_t>(a.out) & 15) || (reinterpret_cast<uintptr_t>(a.residual) & (a.res_f32 ? 15 : 7)) ||
       ((a.out_f32 || a.res_f32) && a.ldo % 4 != 0))

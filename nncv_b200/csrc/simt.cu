@@ -266,6 +266,34 @@ __global__ void maxpool_nhwc_kernel(const T* __restrict__ src, T* __restrict__ d
   }
 }
 
+// s += the 16-byte vectors of the pixels first, first + step, ... below hi, in that order.  U loads are in flight together:
+// a pool is a chain of load latencies.  Maps from 256 pixels on take the cluster kernel (a rule by the map alone: an image's
+// sum must not depend on its batch).  fp16, cold L2, us: 3x18x18x16 30.3 -> 8.8, 2x66x112x200 22.8 -> 17.6, 256x14x14x512
+// 29.4 -> 22.5, 256x12x12x2048 61.6 -> 52.9, 200x20x20x64 35.1 -> 14.6.
+template <int U, typename T, typename F>
+__device__ __forceinline__ void sum_pixels(int first, int hi, int step, float (&s)[16 / sizeof(T)], F&& at) {
+  auto add = [&](const uint4& raw) {
+    const T* v = reinterpret_cast<const T*>(&raw);
+#pragma unroll
+    for (int e = 0; e < 16 / (int)sizeof(T); ++e) s[e] += to_f<T>(v[e]);
+  };
+  int px = first;
+  for (; px + (U - 1) * step < hi; px += U * step) {
+    uint4 raw[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) raw[u] = __ldg(reinterpret_cast<const uint4*>(at(px + u * step)));
+#pragma unroll
+    for (int u = 0; u < U; ++u) add(raw[u]);
+  }
+  uint4 raw[U - 1];
+#pragma unroll
+  for (int u = 0; u < U - 1; ++u)
+    if (px + u * step < hi) raw[u] = __ldg(reinterpret_cast<const uint4*>(at(px + u * step)));
+#pragma unroll
+  for (int u = 0; u < U - 1; ++u)
+    if (px + u * step < hi) add(raw[u]);
+}
+
 // Global average pool: sum in fp32 over HW then divide by HW.  Eight adjacent lanes share one
 // (image, 16-byte channel vector): each sums every eighth pixel, a shuffle tree adds the partial
 // sums, the first lane stores.  (One thread per vector would walk the map as a chain of dependent
@@ -291,14 +319,10 @@ __global__ void avgpool_nhwc_kernel(const T* __restrict__ src, T* __restrict__ d
 #pragma unroll
     for (int e = 0; e < V; ++e) s[e] = 0.0f;
     if (live) {
-      for (int px = slice; px < HW; px += kSlices) {
+      sum_pixels<4, T>(slice, HW, kSlices, s, [&](int px) {
         const int y = px / W, x = px - y * W;
-        const uint4 raw = __ldg(reinterpret_cast<const uint4*>(
-            src + (((size_t)n * il.img_rows + y + il.off) * il.pitch + x + il.off) * C + c));
-        const T* v = reinterpret_cast<const T*>(&raw);
-#pragma unroll
-        for (int e = 0; e < V; ++e) s[e] += to_f<T>(v[e]);
-      }
+        return src + (((size_t)n * il.img_rows + y + il.off) * il.pitch + x + il.off) * C + c;
+      });
     }
 #pragma unroll
     for (int d = 1; d < kSlices; d <<= 1)
@@ -319,7 +343,7 @@ __global__ void avgpool_nhwc_kernel(const T* __restrict__ src, T* __restrict__ d
 // slices are added through shared memory, the eight CTA totals through distributed shared memory
 // by the cluster's first CTA, in a fixed order.  No scratch memory, no atomics.
 constexpr int kPoolCluster = 8;
-template <typename T>
+template <typename T, int U>   // U loads of a thread in flight: four fill the memory system with many CTAs, eight shorten the chain of few
 __global__ void __cluster_dims__(kPoolCluster, 1, 1) __launch_bounds__(256)
 avgpool_cluster_kernel(const T* __restrict__ src, T* __restrict__ dst, int N, int H, int W, int C, Layout il) {
   ptx::grid_dependency_wait();
@@ -343,25 +367,13 @@ avgpool_cluster_kernel(const T* __restrict__ src, T* __restrict__ dst, int N, in
   if (slice < ps) {
     if (il.off == 0 && il.pitch == W && il.img_rows == H) {
       // dense map: pixels are C elements apart, no row arithmetic
-      const T* ptr = src + ((size_t)n * HW + lo + slice) * C + (size_t)(v0 + vc) * V;
-      const size_t step = (size_t)ps * C;
-#pragma unroll 4
-      for (int px = lo + slice; px < hi; px += ps, ptr += step) {
-        const uint4 raw = __ldg(reinterpret_cast<const uint4*>(ptr));
-        const T* v = reinterpret_cast<const T*>(&raw);
-#pragma unroll
-        for (int e = 0; e < V; ++e) s[e] += to_f<T>(v[e]);
-      }
+      const T* ptr = src + (size_t)n * HW * C + (size_t)(v0 + vc) * V;
+      sum_pixels<U, T>(lo + slice, hi, ps, s, [&](int px) { return ptr + (size_t)px * C; });
     } else {
-#pragma unroll 4
-      for (int px = lo + slice; px < hi; px += ps) {
+      sum_pixels<U, T>(lo + slice, hi, ps, s, [&](int px) {
         const int y = px / W, x = px - y * W;
-        const uint4 raw = __ldg(reinterpret_cast<const uint4*>(
-            src + (((size_t)n * il.img_rows + y + il.off) * il.pitch + x + il.off) * C + (size_t)(v0 + vc) * V));
-        const T* v = reinterpret_cast<const T*>(&raw);
-#pragma unroll
-        for (int e = 0; e < V; ++e) s[e] += to_f<T>(v[e]);
-      }
+        return src + (((size_t)n * il.img_rows + y + il.off) * il.pitch + x + il.off) * C + (size_t)(v0 + vc) * V;
+      });
     }
 #pragma unroll
     for (int e = 0; e < V; ++e) part[(slice * cvb + vc) * V + e] = s[e];
@@ -531,9 +543,11 @@ cudaError_t launch_avgpool_nhwc(const void* src, void* dst, DType dt, int N, int
     using T = decltype(tag);
     constexpr int V = 16 / sizeof(T);
     if (C % V != 0) return cudaErrorInvalidValue;
-    if ((long long)H * W >= 512 && N <= 65535) {
+    if ((long long)H * W >= 256 && N <= 65535) {
       const int cv = C / V;
-      return launch_pdl(avgpool_cluster_kernel<T>, dim3(kPoolCluster, N, (cv + 255) / 256), dim3(256), 0, stream,
+      const int z = (cv + 255) / 256;
+      return launch_pdl((long long)kPoolCluster * N * z <= 148 ? avgpool_cluster_kernel<T, 8> : avgpool_cluster_kernel<T, 4>,
+          dim3(kPoolCluster, N, z), dim3(256), 0, stream,
           static_cast<const T*>(src), static_cast<T*>(dst), N, H, W, C, in_l);
     }
     const long long total = (long long)N * (C / V) * 8;
