@@ -486,6 +486,30 @@ __device__ __forceinline__ void tma_load_4d_pair(uint32_t dst, const void* tmap,
       "l"(tmap), "r"(c0), "r"(c1), "r"(c2), "r"(c3), "r"(bar)
       : "memory");
 }
+// The same with the whole warp in the code and one elected lane issuing (`issue`: elect_one()).  The operands then are uniform
+// registers from the start; in a branch of one lane each is moved there first, and a producer's loop with four or five
+// copies a stage took 800 clocks, whatever the copies' size: it, and not the path from L2, set the pace of the kernels.
+__device__ __forceinline__ void mbar_arrive_expect_tx(uint32_t bar, uint32_t bytes, uint32_t issue) {
+  asm volatile("{\n.reg .pred q;\nsetp.ne.b32 q, %2, 0;\n@q mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n}\n" ::"r"(bar), "r"(bytes), "r"(issue) : "memory");
+}
+__device__ __forceinline__ void bulk_g2s(uint32_t dst, const void* src, uint32_t bytes, uint32_t bar, uint32_t issue) {
+  asm volatile("{\n.reg .pred q;\nsetp.ne.b32 q, %4, 0;\n@q cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];\n}\n" ::"r"(dst), "l"(src), "r"(bytes), "r"(bar), "r"(issue) : "memory");
+}
+__device__ __forceinline__ void tma_load_2d(uint32_t dst, const void* tmap, int c0, int c1, uint32_t bar, uint32_t issue) {
+  asm volatile("{\n.reg .pred q;\nsetp.ne.b32 q, %5, 0;\n@q cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];\n}\n" ::"r"(dst), "l"(tmap), "r"(c0), "r"(c1), "r"(bar), "r"(issue) : "memory");
+}
+__device__ __forceinline__ void tma_load_2d_pair(uint32_t dst, const void* tmap, int c0, int c1, uint32_t bar, uint32_t issue) {
+  asm volatile("{\n.reg .pred q;\nsetp.ne.b32 q, %5, 0;\n@q cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];\n}\n" ::"r"(dst), "l"(tmap), "r"(c0), "r"(c1), "r"(bar), "r"(issue) : "memory");
+}
+__device__ __forceinline__ void tma_load_4d(uint32_t dst, const void* tmap, int c0, int c1, int c2, int c3, uint32_t bar, uint32_t issue) {
+  asm volatile("{\n.reg .pred q;\nsetp.ne.b32 q, %7, 0;\n@q cp.async.bulk.tensor.4d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4, %5}], [%6];\n}\n" ::"r"(dst), "l"(tmap), "r"(c0), "r"(c1), "r"(c2), "r"(c3), "r"(bar), "r"(issue) : "memory");
+}
+__device__ __forceinline__ void tma_load_4d_pair(uint32_t dst, const void* tmap, int c0, int c1, int c2, int c3, uint32_t bar, uint32_t issue) {
+  asm volatile("{\n.reg .pred q;\nsetp.ne.b32 q, %7, 0;\n@q cp.async.bulk.tensor.4d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4, %5}], [%6];\n}\n" ::"r"(dst), "l"(tmap), "r"(c0), "r"(c1), "r"(c2), "r"(c3), "r"(bar), "r"(issue) : "memory");
+}
+__device__ __forceinline__ void tma_load_5d(uint32_t dst, const void* tmap, int c0, int c1, int c2, int c3, int c4, uint32_t bar, uint32_t issue) {
+  asm volatile("{\n.reg .pred q;\nsetp.ne.b32 q, %8, 0;\n@q cp.async.bulk.tensor.5d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4, %5, %6}], [%7];\n}\n" ::"r"(dst), "l"(tmap), "r"(c0), "r"(c1), "r"(c2), "r"(c3), "r"(c4), "r"(bar), "r"(issue) : "memory");
+}
 __device__ __forceinline__ void tmem_alloc_pair(uint32_t slot_smem, uint32_t ncols) {
   asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(slot_smem), "r"(ncols) : "memory");
 }

@@ -208,20 +208,20 @@ tconv_kernel(const __grid_constant__ CUtensorMap tm_in, const __grid_constant__ 
   // that hides the whole weight fetch behind the previous layer.
   const uint32_t full_lead = PAIR ? ptx::map_to_cta(full, 0) : full;
   // the bytes of a stage, of both CTAs, are counted on the leader's barrier
-  auto expect_stage = [&](uint32_t st, bool half = false) {
-    if (!PAIR) ptx::mbar_arrive_expect_tx(full + 8 * st, (uint32_t)stage_bytes);
-    else if (rank == 0) ptx::mbar_arrive_expect_tx(full + 8 * st, 2u * (uint32_t)(half ? kABytes + WTILE / 2 : stage_bytes));
+  auto expect_stage = [&](uint32_t st, uint32_t issue, bool half = false) {
+    if (!PAIR) ptx::mbar_arrive_expect_tx(full + 8 * st, (uint32_t)stage_bytes, issue);
+    else if (rank == 0) ptx::mbar_arrive_expect_tx(full + 8 * st, 2u * (uint32_t)(half ? kABytes + WTILE / 2 : stage_bytes), issue);
   };
-  auto load_weights = [&](int n_tile, int cb, int tap, uint32_t st) {
+  auto load_weights = [&](int n_tile, int cb, int tap, uint32_t st, uint32_t issue) {
     const uint32_t dst = sRing + st * stage_bytes + kABytes;
     const bool second = DUAL && tap == p.taps;
     if (PAIR) {   // the weights are packed for N tile BN/2; this CTA takes tile 2 * n_tile + rank
       const int wt = 2 * n_tile + (int)rank;
-      if (second) ptx::tma_load_2d_pair(dst, &tm_b2, 0, (wt * p.CB + cb) * (BN / 2), full_lead + 8 * st);
-      else ptx::tma_load_2d_pair(dst, &tm_b, 0, (wt * KB + tap * p.CB + cb) * (BN / 2), full_lead + 8 * st);
+      if (second) ptx::tma_load_2d_pair(dst, &tm_b2, 0, (wt * p.CB + cb) * (BN / 2), full_lead + 8 * st, issue);
+      else ptx::tma_load_2d_pair(dst, &tm_b, 0, (wt * KB + tap * p.CB + cb) * (BN / 2), full_lead + 8 * st, issue);
     } else {
       ptx::bulk_g2s(dst, second ? p.wpack2 + ((size_t)n_tile * p.CB + cb) * WTILE : p.wpack + ((size_t)n_tile * KB + (size_t)tap * p.CB + cb) * WTILE,
-                    WTILE, full + 8 * st);
+                    WTILE, full + 8 * st, issue);
     }
   };
   uint32_t early = 0;   // ring stages whose weights are on their way
@@ -234,17 +234,19 @@ tconv_kernel(const __grid_constant__ CUtensorMap tm_in, const __grid_constant__ 
       for (int i = 0; i < p.CB; ++i) ptx::bulk_g2s(sW + (uint32_t)(KB + i) * WTILE, src2 + (size_t)i * WTILE, WTILE, w_full);
     }
   };
-  if (warp == 0 && lane == 0 && !BROW && p.w_ready) {
+  if (warp == 0 && !BROW && p.w_ready) {
     if (RESIDENT) {
-      load_resident();
+      if (lane == 0) load_resident();
+      __syncwarp();
     } else {
+      const uint32_t issue = ptx::elect_one();
       for (int i = 0; early < (uint32_t)p.stages; ++i) {
         int n0, oy0, ox0, n_tile;
         if (!item_of(i, n0, oy0, ox0, n_tile)) break;
         for (int cb = 0; cb < p.CB && early < (uint32_t)p.stages; ++cb)
           for (int tap = 0; tap < taps_x && early < (uint32_t)p.stages; ++tap, ++early) {
-            expect_stage(early);
-            load_weights(n_tile, cb, tap, early);
+            expect_stage(early, issue);
+            load_weights(n_tile, cb, tap, early, issue);
           }
       }
     }
@@ -255,49 +257,58 @@ tconv_kernel(const __grid_constant__ CUtensorMap tm_in, const __grid_constant__ 
 
   if (warp == 0) {
     // ------------------------------------------------------------------ TMA producer ----
-    if (lane == 0) {
-      if (RESIDENT && !p.w_ready) load_resident();
-      uint32_t cnt = 0;
+    {
+      if (RESIDENT && !p.w_ready && lane == 0) load_resident();
+      __syncwarp();
+      const uint32_t issue = ptx::elect_one();
+      uint32_t cnt = 0, st = 0, ring = 1;   // stages begun; the next one and the parity of its round
+      auto peek = [&](uint32_t bar, uint32_t parity) { return PAIR ? ptx::mbar_peek_cluster(bar, parity) : ptx::mbar_peek(bar, parity); };
+      uint32_t seen = 1;                    // nothing has used the ring yet
       bool okw = true;
       for (int i = 0; okw; ++i) {
         int n0, oy0, ox0, n_tile;
         if (!item_of(i, n0, oy0, ox0, n_tile)) break;
         const int xb = p.stride * ox0 - p.pad + p.in_off, yb = p.stride * oy0 - p.pad + p.in_off;
+        const int centre_r = DUAL ? (p.taps / 2) / p.S : 0, centre_s = DUAL ? p.taps / 2 - centre_r * p.S : 0;
         // channel block outermost, taps innermost: the same accumulation order as the shifted-view
         // 3x3 kernel, so both kernels give bit-identical sums
         for (int cb = cb_lo; cb < cb_hi && okw; ++cb) {
+          int r = 0, s = 0;
           for (int tap = 0; tap < taps_x; ++tap, ++cnt) {
-            const int gtap = tap < p.taps ? tap : p.taps / 2;   // the extra tap re-reads the centre tap's pixels
-            const int r = gtap / p.S, s = gtap - r * p.S;
-            const uint32_t st = cnt % (uint32_t)p.stages;
+            if (DUAL && tap == p.taps) { r = centre_r; s = centre_s; }   // the extra tap re-reads the centre tap's pixels
             const bool begun = cnt < early;   // this stage's first use: weights already issued
-            if (!begun) {
-              const bool freed = PAIR ? ptx::mbar_wait_cluster_abortable(empty + 8 * st, ((cnt / (uint32_t)p.stages) & 1u) ^ 1u, abort_flag)
-                                      : ptx::mbar_wait_abortable(empty + 8 * st, ((cnt / (uint32_t)p.stages) & 1u) ^ 1u, abort_flag);
+            if (!ptx::warp_all(seen)) {
+              const bool freed = PAIR ? ptx::warp_wait_cluster(empty + 8 * st, ring, abort_flag) : ptx::warp_wait(empty + 8 * st, ring, abort_flag);
               if (!freed) { okw = false; break; }
-              expect_stage(st, halved(i));
             }
+            if (!begun) expect_stage(st, issue, halved(i));
             const uint32_t dst = sRing + st * stage_bytes;
-            if (PAIR) ptx::tma_load_4d_pair(dst, &tm_in, cb * 64, xb + s, yb + r, n0, full_lead + 8 * st);
-            else ptx::tma_load_4d(dst, &tm_in, cb * 64, xb + s, yb + r, n0, full + 8 * st);
+            if (PAIR) ptx::tma_load_4d_pair(dst, &tm_in, cb * 64, xb + s, yb + r, n0, full_lead + 8 * st, issue);
+            else ptx::tma_load_4d(dst, &tm_in, cb * 64, xb + s, yb + r, n0, full + 8 * st, issue);
             if (BROW) {
 #pragma unroll
               for (int j = 0; j < WTILE / 8192; ++j) {
                 if (PAIR) {
                   const int mine = halved(i) ? BN / 4 : BN / 2;   // columns of this CTA
                   if (j * 64 < mine)
-                    ptx::tma_load_2d_pair(dst + kABytes + (uint32_t)j * 8192u, &tm_b, first_col(i, n_tile) + (int)rank * mine + j * 64, cb * 64, full_lead + 8 * st);
+                    ptx::tma_load_2d_pair(dst + kABytes + (uint32_t)j * 8192u, &tm_b, first_col(i, n_tile) + (int)rank * mine + j * 64, cb * 64,
+                                          full_lead + 8 * st, issue);
                 } else {
-                  ptx::tma_load_2d(dst + kABytes + (uint32_t)j * 8192u, &tm_b, n_tile * BN + j * 64, cb * 64, full + 8 * st);
+                  ptx::tma_load_2d(dst + kABytes + (uint32_t)j * 8192u, &tm_b, n_tile * BN + j * 64, cb * 64, full + 8 * st, issue);
                 }
               }
             } else if (!RESIDENT && !begun) {
-              load_weights(n_tile, cb, tap, st);
+              load_weights(n_tile, cb, tap, st, issue);
             }
+            if (++s == p.S) { s = 0; ++r; }
+            const bool wrap = st + 1 == (uint32_t)p.stages;
+            st = wrap ? 0u : st + 1;
+            ring ^= wrap ? 1u : 0u;
+            seen = peek(empty + 8 * st, ring);
           }
         }
       }
-      if (!okw && p.error_flag) atomicCAS(p.error_flag, 0, (int)kErrWaitProducer);
+      if (!okw && lane == 0 && p.error_flag) atomicCAS(p.error_flag, 0, (int)kErrWaitProducer);
     }
   } else if (warp == 1) {
     if (!PAIR || rank == 0)
