@@ -159,20 +159,21 @@ conv3x3_kernel(const __grid_constant__ CUtensorMap tm_in, const __grid_constant_
   // Packed weights never change, so their copies start before the previous kernel of the stream has finished.
   auto weight_tile = [&](int n_tile, int cb, int tap) { return p.wpack + ((size_t)n_tile * kb_total + (size_t)tap * p.CB + cb) * WTILE; };
   uint32_t early = 0;   // stages of the weight ring already on their way
-  if (warp == 0 && lane == 0) {
+  if (warp == 0) {
+    const uint32_t issue = ptx::elect_one();
     if (RESIDENT) {
       const uint8_t* src = p.wpack + (size_t)blockIdx.y * kb_total * WTILE;
-      ptx::mbar_arrive_expect_tx(w_full, (uint32_t)kb_total * WTILE);
+      ptx::mbar_arrive_expect_tx(w_full, (uint32_t)kb_total * WTILE, issue);
       for (int i = 0; i < kb_total; ++i)
-        ptx::bulk_g2s(sW + (uint32_t)i * WTILE, src + (size_t)i * WTILE, WTILE, w_full);
+        ptx::bulk_g2s(sW + (uint32_t)i * WTILE, src + (size_t)i * WTILE, WTILE, w_full, issue);
     } else {
       for (int i = 0; early < (uint32_t)p.w_stages; ++i) {
         int m_item, n_tile;
         if (!item_of(i, m_item, n_tile)) break;
         for (int cb = 0; cb < p.CB && early < (uint32_t)p.w_stages; ++cb)
           for (int tap = 0; tap < 9 && early < (uint32_t)p.w_stages; ++tap, ++early) {
-            ptx::mbar_arrive_expect_tx(w_full + 8 * early, WTILE);
-            ptx::bulk_g2s(sW + early * WTILE, weight_tile(n_tile, cb, tap), WTILE, w_full + 8 * early);
+            ptx::mbar_arrive_expect_tx(w_full + 8 * early, WTILE, issue);
+            ptx::bulk_g2s(sW + early * WTILE, weight_tile(n_tile, cb, tap), WTILE, w_full + 8 * early, issue);
           }
       }
     }
@@ -183,35 +184,35 @@ conv3x3_kernel(const __grid_constant__ CUtensorMap tm_in, const __grid_constant_
 
   if (warp == 0) {
     // ------------------------------------------------------------------ TMA producer ----
-    if (lane == 0) {
-      uint32_t in_cnt = 0, w_cnt = 0;
+    {
+      const uint32_t issue = ptx::elect_one();
+      uint32_t w_cnt = 0, st = 0, par = 1, ws = 0, wpar = 1, w_seen = 1;   // stages, parities of their rings' rounds
       bool okw = true;
       for (int i = 0; okw; ++i) {
         int m_item, n_tile;
         if (!item_of(i, m_item, n_tile)) break;
         const int row0 = m_item * (MT * 128) - p.P - 1;
         for (int cb = 0; cb < p.CB && okw; ++cb) {
-          const uint32_t st = in_cnt % (uint32_t)p.in_stages;
-          const uint32_t par = ((in_cnt / (uint32_t)p.in_stages) & 1u) ^ 1u;
-          if (!ptx::mbar_wait_abortable(in_empty + 8 * st, par, abort_flag)) { okw = false; break; }
-          ptx::mbar_arrive_expect_tx(in_full + 8 * st, (uint32_t)in_stage_bytes);
+          if (!ptx::warp_wait(in_empty + 8 * st, par, abort_flag)) { okw = false; break; }
+          ptx::mbar_arrive_expect_tx(in_full + 8 * st, (uint32_t)in_stage_bytes, issue);
           for (int b = 0; b < p.in_boxes; ++b)
             ptx::tma_load_2d(sIn + st * in_stage_bytes + (uint32_t)b * p.box_rows * 128, &tm_in, cb * 64,
-                             row0 + b * p.box_rows, in_full + 8 * st);
-          ++in_cnt;
+                             row0 + b * p.box_rows, in_full + 8 * st, issue);
+          if (++st == (uint32_t)p.in_stages) { st = 0; par ^= 1u; }
           if (!RESIDENT) {
             for (int tap = 0; tap < 9; ++tap, ++w_cnt) {
-              if (w_cnt < early) continue;
-              const uint32_t ws = w_cnt % (uint32_t)p.w_stages;
-              const uint32_t wpar = ((w_cnt / (uint32_t)p.w_stages) & 1u) ^ 1u;
-              if (!ptx::mbar_wait_abortable(w_empty + 8 * ws, wpar, abort_flag)) { okw = false; break; }
-              ptx::mbar_arrive_expect_tx(w_full + 8 * ws, WTILE);
-              ptx::bulk_g2s(sW + ws * WTILE, weight_tile(n_tile, cb, tap), WTILE, w_full + 8 * ws);
+              if (w_cnt >= early) {
+                if (!ptx::warp_all(w_seen) && !ptx::warp_wait(w_empty + 8 * ws, wpar, abort_flag)) { okw = false; break; }
+                ptx::mbar_arrive_expect_tx(w_full + 8 * ws, WTILE, issue);
+                ptx::bulk_g2s(sW + ws * WTILE, weight_tile(n_tile, cb, tap), WTILE, w_full + 8 * ws, issue);
+              }
+              if (++ws == (uint32_t)p.w_stages) { ws = 0; wpar ^= 1u; }
+              w_seen = ptx::mbar_peek(w_empty + 8 * ws, wpar);
             }
           }
         }
       }
-      if (!okw && p.error_flag) atomicCAS(p.error_flag, 0, (int)kErrWaitProducer);
+      if (!okw && lane == 0 && p.error_flag) atomicCAS(p.error_flag, 0, (int)kErrWaitProducer);
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------------ MMA issuer ------

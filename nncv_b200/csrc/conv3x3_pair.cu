@@ -149,25 +149,26 @@ conv3x3_pair_kernel(const __grid_constant__ CUtensorMap tm_in, const __grid_cons
 
   const uint32_t lead_in_full = ptx::map_to_cta(in_full, 0), lead_w_full = ptx::map_to_cta(w_full, 0);
   // This CTA's half of an item's columns for filter row fr of channel block cb -> weight stage ws (three taps).
-  auto load_weights = [&](int n_tile, int sub, int parts, int cb, int fr, uint32_t ws) {
+  auto load_weights = [&](int n_tile, int sub, int parts, int cb, int fr, uint32_t ws, uint32_t issue) {
     const int rows = BNP / parts / 2;                                           // per tap
     const int wrow = n_tile * BNP + sub * (BNP / parts) + (int)rank * rows;     // as rows of the packed N tiles
-    if (rank == 0) ptx::mbar_arrive_expect_tx(w_full + 8 * ws, 2u * kWGroup * (uint32_t)rows * 128u);
+    if (rank == 0) ptx::mbar_arrive_expect_tx(w_full + 8 * ws, 2u * kWGroup * (uint32_t)rows * 128u, issue);
 #pragma unroll
     for (int s3 = 0; s3 < kWGroup; ++s3) {
       const int first = ((wrow / kPackBN) * kb_total + (fr * 3 + s3) * p.CB + cb) * kPackBN + wrow % kPackBN;
       for (int r = 0; r < rows; r += p.w_box)
-        ptx::tma_load_2d_pair(sW + ws * kWStage + s3 * kWTile + (uint32_t)r * 128u, &tm_w, 0, first + r, lead_w_full + 8 * ws);
+        ptx::tma_load_2d_pair(sW + ws * kWStage + s3 * kWTile + (uint32_t)r * 128u, &tm_w, 0, first + r, lead_w_full + 8 * ws, issue);
     }
   };
   // Packed weights never change, so their copies start before the previous kernel of the stream has finished.
   uint32_t early = 0;   // stages of the weight ring already on their way
-  if (warp == 0 && lane == 0) {
+  if (warp == 0) {
+    const uint32_t issue = ptx::elect_one();
     for (int i = 0; early < (uint32_t)p.w_stages && !(p.w_resident && i > 0); ++i) {
       int m_item, n_tile, sub, parts;
       if (!item_of(i, m_item, n_tile, sub, parts)) break;
       for (int cb = 0; cb < p.CB && early < (uint32_t)p.w_stages; ++cb)
-        for (int fr = 0; fr < 3 && early < (uint32_t)p.w_stages; ++fr, ++early) load_weights(n_tile, sub, parts, cb, fr, early);
+        for (int fr = 0; fr < 3 && early < (uint32_t)p.w_stages; ++fr, ++early) load_weights(n_tile, sub, parts, cb, fr, early, issue);
     }
   }
   // The rest reads what the previous kernel wrote, or writes what it may still be reading.
@@ -176,8 +177,9 @@ conv3x3_pair_kernel(const __grid_constant__ CUtensorMap tm_in, const __grid_cons
 
   if (warp == 0) {
     // ------------------------------------------------------------------ TMA producer ----
-    if (lane == 0) {
-      uint32_t in_cnt = 0, w_cnt = 0;
+    {
+      const uint32_t issue = ptx::elect_one();
+      uint32_t w_cnt = 0, st = 0, ring = 1, ws = 0, w_ring = 1, w_seen = 1;   // stages, parities of their rings' rounds
       bool okw = true;
       for (int i = 0; okw; ++i) {
         int m_item, n_tile, sub, parts;
@@ -186,23 +188,24 @@ conv3x3_pair_kernel(const __grid_constant__ CUtensorMap tm_in, const __grid_cons
         // [t * 128, +128) of both CTAs' tiles
         const int row0 = (m_item * 2 + (int)rank) * 128 * MT - p.P - 1;
         for (int cb = 0; cb < p.CB && okw; ++cb) {
-          const uint32_t st = in_cnt % (uint32_t)p.in_stages;
-          if (!ptx::mbar_wait_cluster_abortable(in_empty + 8 * st, ((in_cnt / (uint32_t)p.in_stages) & 1u) ^ 1u, abort_flag)) { okw = false; break; }
-          if (rank == 0) ptx::mbar_arrive_expect_tx(in_full + 8 * st, 2u * (uint32_t)in_stage_bytes);
+          if (!ptx::warp_wait_cluster(in_empty + 8 * st, ring, abort_flag)) { okw = false; break; }
+          if (rank == 0) ptx::mbar_arrive_expect_tx(in_full + 8 * st, 2u * (uint32_t)in_stage_bytes, issue);
           for (int bx = 0; bx < p.n_boxes; ++bx)
             ptx::tma_load_2d_pair(sIn + st * in_stage_bytes + (uint32_t)(bx * p.box_rows) * 128u, &tm_in, cb * 64,
-                                  row0 + bx * p.box_rows, lead_in_full + 8 * st);
-          ++in_cnt;
+                                  row0 + bx * p.box_rows, lead_in_full + 8 * st, issue);
+          if (++st == (uint32_t)p.in_stages) { st = 0; ring ^= 1u; }
           if (p.w_resident && i > 0) continue;       // resident weights were loaded with the first item
           for (int fr = 0; fr < 3; ++fr, ++w_cnt) {   // one filter row (three taps) per weight stage
-            if (w_cnt < early) continue;
-            const uint32_t ws = w_cnt % (uint32_t)p.w_stages;
-            if (!ptx::mbar_wait_cluster_abortable(w_empty + 8 * ws, ((w_cnt / (uint32_t)p.w_stages) & 1u) ^ 1u, abort_flag)) { okw = false; break; }
-            load_weights(n_tile, sub, parts, cb, fr, ws);
+            if (w_cnt >= early) {
+              if (!ptx::warp_all(w_seen) && !ptx::warp_wait_cluster(w_empty + 8 * ws, w_ring, abort_flag)) { okw = false; break; }
+              load_weights(n_tile, sub, parts, cb, fr, ws, issue);
+            }
+            if (++ws == (uint32_t)p.w_stages) { ws = 0; w_ring ^= 1u; }
+            w_seen = ptx::mbar_peek_cluster(w_empty + 8 * ws, w_ring);
           }
         }
       }
-      if (!okw && p.error_flag) atomicCAS(p.error_flag, 0, (int)kErrWaitProducer);
+      if (!okw && lane == 0 && p.error_flag) atomicCAS(p.error_flag, 0, (int)kErrWaitProducer);
     }
   } else if (warp == 1) {
     if (rank == 0) {

@@ -167,57 +167,62 @@ conv_f32_kernel(const __grid_constant__ CUtensorMap tm_in, const F32Params p) {
   };
   // block kb of the reduction: channel block outermost, then the taps
   const int packed_tiles = (p.Kout + 63) / 64;
-  auto load_weights = [&](int n_tile, int plane, int kb, uint32_t slot) {
-    const int cb = kb / p.taps, tap = kb - cb * p.taps;
+  auto load_weights = [&](int n_tile, int plane, int cb, int tap, uint32_t slot, uint32_t issue) {
 #pragma unroll
     for (int q = 0; q < kNT; ++q) {
       // the second half of the last, ragged tile has no weights: its columns are never stored, any tile will do
       const int t = min(n_tile * kNT + q, packed_tiles - 1);
       ptx::bulk_g2s(sRing + slot * kSlot + kABytes + q * kBBytes,
-                    p.wpack + (((size_t)t * 3 + plane) * kb_all + (size_t)tap * p.CB + cb) * kBBytes, kBBytes, full + 8 * slot);
+                    p.wpack + (((size_t)t * 3 + plane) * kb_all + (size_t)tap * p.CB + cb) * kBBytes, kBBytes, full + 8 * slot, issue);
     }
   };
   // the packed weights never change: their first copies do not wait for the previous kernel
   uint32_t early = 0;
-  if (warp == 0 && lane == 0) {
+  if (warp == 0) {
+    const uint32_t issue = ptx::elect_one();
     int n0, oy0, ox0, n_tile;
-    if (item_of(0, n0, oy0, ox0, n_tile))
-      for (int kb = kb0; kb < kb1 && early < (uint32_t)kSlots; ++kb)
+    if (item_of(0, n0, oy0, ox0, n_tile)) {
+      int cb = kb0 / p.taps, tap = kb0 - cb * p.taps;
+      for (int kb = kb0; kb < kb1 && early < (uint32_t)kSlots; ++kb) {
         for (int pl = 0; pl < 3 && early < (uint32_t)kSlots; ++pl, ++early) {
-          ptx::mbar_arrive_expect_tx(full + 8 * early, kSlot);
-          load_weights(n_tile, pl, kb, early);
+          ptx::mbar_arrive_expect_tx(full + 8 * early, kSlot, issue);
+          load_weights(n_tile, pl, cb, tap, early, issue);
         }
+        if (++tap == p.taps) { tap = 0; ++cb; }
+      }
+    }
   }
   ptx::grid_dependency_wait();
   ptx::grid_launch_dependents();
 
   if (warp == 0) {
     // ------------------------------------------------------------------ TMA producer ----
-    if (lane == 0) {
-      uint32_t slot = 0, ring = 0, cnt = 0;
+    {
+      const uint32_t issue = ptx::elect_one();
+      uint32_t slot = 0, ring = 0, cnt = 0, seen = 1;
       bool okw = true;
       for (int i = 0; okw; ++i) {
         int n0, oy0, ox0, n_tile;
         if (!item_of(i, n0, oy0, ox0, n_tile)) break;
         const int xb = p.stride * ox0 - p.pad_x, yb = p.stride * oy0 - p.pad_y;
         int cb = kb0 / p.taps, tap = kb0 - cb * p.taps;
+        int r = tap / p.S, s = tap - r * p.S;
         for (int kb = kb0; kb < kb1 && okw; ++kb) {
-          const int r = tap / p.S, s = tap - r * p.S;
           for (int pl = 0; pl < 3; ++pl, ++cnt) {
             const bool begun = cnt < early;
-            if (!begun) {
-              if (!ptx::mbar_wait_abortable(empty + 8 * slot, ring ^ 1u, abort_flag)) { okw = false; break; }
-              ptx::mbar_arrive_expect_tx(full + 8 * slot, kSlot);
-            }
+            if (!ptx::warp_all(seen) && !ptx::warp_wait(empty + 8 * slot, ring ^ 1u, abort_flag)) { okw = false; break; }
+            if (!begun) ptx::mbar_arrive_expect_tx(full + 8 * slot, kSlot, issue);
             const uint32_t dst = sRing + slot * kSlot;
-            ptx::tma_load_5d(dst, &tm_in, cb * 64, xb + s, yb + r, n0, pl, full + 8 * slot);
-            if (!begun) load_weights(n_tile, pl, kb, slot);
+            ptx::tma_load_5d(dst, &tm_in, cb * 64, xb + s, yb + r, n0, pl, full + 8 * slot, issue);
+            if (!begun) load_weights(n_tile, pl, cb, tap, slot, issue);
             if (++slot == kSlots) { slot = 0; ring ^= 1u; }
+            seen = ptx::mbar_peek(empty + 8 * slot, ring ^ 1u);
           }
-          if (++tap == p.taps) { tap = 0; ++cb; }
+          if (++s == p.S) { s = 0; ++r; }
+          if (++tap == p.taps) { tap = r = s = 0; ++cb; }
         }
       }
-      if (!okw && p.error_flag) atomicCAS(p.error_flag, 0, (int)kErrWaitProducer);
+      if (!okw && lane == 0 && p.error_flag) atomicCAS(p.error_flag, 0, (int)kErrWaitProducer);
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------------ MMA issuer ------
@@ -225,7 +230,11 @@ conv_f32_kernel(const __grid_constant__ CUtensorMap tm_in, const F32Params p) {
     const uint32_t idesc = ptx::umma_idesc(128, kBN, 1);
     uint32_t slot = 0, ring = 0, blk = 0;   // blk: running count of blocks; accumulator buffer blk % 2
     bool okw = true;
-    auto step = [&]() { if (++slot == kSlots) { slot = 0; ring ^= 1u; } };
+    uint32_t seen = ptx::mbar_peek(full, 0);
+    auto step = [&]() {
+      if (++slot == kSlots) { slot = 0; ring ^= 1u; }
+      seen = ptx::mbar_peek(full + 8 * slot, ring);
+    };
     // one product of the block's planes: four k steps of 16
     auto product = [&](uint32_t d, uint32_t a, uint32_t b, uint32_t fresh) {
       const uint32_t a_lo = ptx::smem_desc_k128_lo(a), b_lo = ptx::smem_desc_k128_lo(b);
@@ -243,7 +252,7 @@ conv_f32_kernel(const __grid_constant__ CUtensorMap tm_in, const F32Params p) {
         uint32_t at[3], sl[3];
 #pragma unroll
         for (int pl = 0; pl < 3; ++pl) {
-          if (okw && !ptx::warp_wait(full + 8 * slot, ring, abort_flag)) okw = false;
+          if (okw && !ptx::warp_all(seen) && !ptx::warp_wait(full + 8 * slot, ring, abort_flag)) okw = false;
           if (!okw) break;
           ptx::tc_fence_after();
           sl[pl] = slot;
