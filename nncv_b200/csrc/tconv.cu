@@ -854,11 +854,11 @@ cudaError_t launch_tconv(const TconvArgs& args, cudaStream_t stream) {
 }
 
 // N tile of a matmul with a row-major B: the least rounds x (blocks x time + epilogue), in us as measured with every SM at
-// work: a block of 64 of a 128 x 64 tile 0.42, 128 x 128 0.47, 256 x 256 on a CTA pair 0.63; a pair's launch and an exchange
-// of partial sums 2 each.  (Before, the widest tile that still filled the SMs: 2048^3 took two rounds of 128 x 128, 38.7 us,
+// work: a block of 64 of a 128 x 64 tile 0.28, 128 x 128 0.32, 256 x 256 on a CTA pair 0.42; a pair's launch 2, an exchange of
+// partial sums 3.  (Before, the widest tile that still filled the SMs: 2048^3 took two rounds of 128 x 128, 38.7 us,
 // where one of 64 pairs takes 28.3; 2048x1024x1024 two of 128 x 64, 22.4, where one of 128 x 128 takes 16.4.)
 static int matmul_pick(int M, int N, int K, int sms) {
-  static const double block[3] = {0.42, 0.47, 0.63}, epilogue[3] = {0.5, 0.9, 1.8};
+  static const double block[3] = {0.28, 0.32, 0.42}, epilogue[3] = {0.6, 0.9, 2.0};
   const long long mi = ((long long)M + 127) / 128;
   const int CB = (K + 63) / 64;
   int best_bn = 64;
@@ -870,7 +870,7 @@ static int matmul_pick(int M, int N, int K, int sms) {
     const long long items = (pair ? (mi + 1) / 2 : mi) * ((N + bn - 1) / bn), slots = pair ? sms / 2 : sms;
     int s = 1;
     while (!pair && s < 8 && items * 2 * s <= slots * 15 / 16 && CB >= kSplitBlocks * 2 * s) s *= 2;
-    const double t = (double)((items + slots - 1) / slots) * ((CB + s - 1) / s * block[i] + epilogue[i]) + (pair || s > 1 ? 2.0 : 0.0);
+    const double t = (double)((items + slots - 1) / slots) * ((CB + s - 1) / s * block[i] + epilogue[i]) + (pair ? 2.0 : s > 1 ? 3.0 : 0.0);
     if (t < best) { best = t; best_bn = bn; }
   }
   return best_bn;
