@@ -96,7 +96,7 @@ namespace {
 // current and kept until the process exits.  Every entry point works on the context of the
 // calling thread's current device, so kernels always run on the GPU that owns their buffers.
 struct Model;
-constexpr int kMaxParts = 8;   // of a batch in host memory
+constexpr int kMaxParts = 4;   // of a batch in host memory
 struct Device {
   bool ready = false;
   int id = -1;
@@ -1122,13 +1122,7 @@ struct Model {
   HostCopier copier;          // images from pageable memory
   PinnedBuf result;           // status word, then logits on their way to pageable memory
   size_t logits_off = 0;      // bytes: where the current part's logits go in logits_io / logits32
-  // How a batch in host memory is cut into parts: each way is run a few times, then the fastest is kept.
-  struct PartChoice {
-    std::vector<std::vector<int>> ways;   // sizes of the parts
-    std::vector<double> best;             // fastest call so far, seconds
-    int calls = 0, chosen = -1;
-  };
-  std::map<std::array<int, 4>, PartChoice> part_choice;   // by N, H, W, pinned
+  std::map<std::array<int, 4>, int> part_choice;   // parts a batch in host memory is cut into, by N, H, W, pinned
   static constexpr uintptr_t kFakeBase = (uintptr_t)0x7A00000000000000ull;   // planning pass: stand-in pointers
   void note_use(const void* p) {
     const uintptr_t v = (uintptr_t)p;
@@ -1773,63 +1767,17 @@ void shard_range(int n, int rank, int world, int* lo, int* hi) {
   *hi = *lo + base + (rank < extra ? 1 : 0);
 }
 
-// One device's share of a forward: images [sp, sp + N images) -> logits rows at dp (row pitch
-// dst_stride elements).  Runs on the calling thread's current device (g_dev), on stream st;
-// synchronises and reads the device status word unless device_only.
-int forward_slice(Model& m, const char* sp, bool src_dev, char* dp, bool dst_dev, size_t dst_stride, int N, int H, int W,
-                  cudaStream_t st, bool device_only) {
+// A batch of images in host memory, in n_parts parts: every copy, every forward, one wait.
+int forward_host(Model& m, const char* sp, bool pinned, char* dp, bool dst_dev, size_t dst_stride, int N, int H, int W, cudaStream_t st,
+                 int n_parts) {
   int rc;
-  const size_t ew = m.ele_width, row = (size_t)m.plan.out_features * ew;
-  if (src_dev) {
-    if ((rc = ensure_workspace(m, N, H, W))) return rc;
-    m.logits_off = 0;
-    if ((rc = model_forward_device(m, sp, N, H, W, st))) return rc;
-    const void* logits = m.io_dt == kF32 ? m.logits32.p : m.logits_io.p;
-    if (device_only && dst_stride * ew == row) CU(cudaMemcpyAsync(dp, logits, row * N, cudaMemcpyDeviceToDevice, st));
-    else CU(cudaMemcpy2DAsync(dp, dst_stride * ew, logits, row, row, (size_t)N, dst_dev ? cudaMemcpyDeviceToDevice : cudaMemcpyDeviceToHost, st));
-    if (device_only) return ok();
-    CU(cudaStreamSynchronize(st));
-    if ((rc = check_kernel_status())) return rc;
-    return ok();
+  const size_t ew = m.ele_width, row = (size_t)m.plan.out_features * ew, img_bytes = (size_t)3 * H * W * ew;
+  std::vector<int> parts;
+  for (int r = 0; r < n_parts; ++r) {
+    int lo, hi;
+    shard_range(N, r, n_parts, &lo, &hi);
+    parts.push_back(hi - lo);
   }
-  // Images in host memory: a batch may run in parts, so that the copies of later parts overlap the forward of earlier ones
-  // (copies on their own stream, ordered by events).  More parts leave less of the last one exposed but make smaller, less
-  // efficient forwards -- which way wins depends on the network and the link, so the first calls of a shape try each (a call
-  // to let the layers tune themselves, two that count).  ResNet-18 fp16 256x224 from pinned memory (1.41 ms of copying):
-  // 2.20 ms in halves with blocking reads of logits and status, 2.03 ms now (quarters lose more to smaller forwards than
-  // they hide).  fp32 convolutions split their sums by the batch, so there a batch keeps one way.
-  const size_t img_bytes = (size_t)3 * H * W * ew;
-  const bool pinned = is_pinned_ptr(sp);
-  const bool halves = N >= 128 && N % 2 == 0;
-  std::vector<int> parts = halves ? std::vector<int>{N / 2, N / 2} : std::vector<int>{N};
-  Model::PartChoice* choice = nullptr;
-  int way = -1;
-  if (m.act_dt != kF32 && N >= 16 && g_autotune) {
-    choice = &m.part_choice[{N, H, W, (int)pinned}];
-    if (choice->ways.empty()) {
-      choice->ways.push_back(parts);
-      for (int n : {1, 2, 4, 8}) {
-        std::vector<int> w;
-        for (int r = 0; r < n; ++r) {
-          int lo, hi;
-          shard_range(N, r, n, &lo, &hi);
-          w.push_back(hi - lo);
-        }
-        if (w.back() < 8 || w == parts) continue;
-        choice->ways.push_back(w);
-        if (n == 4 && w.back() >= 16) {   // the last quarter in halves
-          const int h = w.back() / 2;
-          w.back() -= h;
-          w.push_back(h);
-          choice->ways.push_back(w);
-        }
-      }
-      choice->best.assign(choice->ways.size(), 1e30);
-    }
-    way = choice->chosen >= 0 ? choice->chosen : choice->calls / 3;
-    parts = choice->ways[(size_t)way];
-  }
-  const auto t0 = std::chrono::steady_clock::now();
   const int most = *std::max_element(parts.begin(), parts.end());
   if ((rc = ensure_workspace(m, most, H, W))) return rc;
   if (m.in_stage.bytes < (size_t)N * img_bytes) {
@@ -1898,16 +1846,57 @@ int forward_slice(Model& m, const char* sp, bool src_dev, char* dp, bool dst_dev
   }
   if (stage_out)
     for (int r = 0; r < N; ++r) memcpy(dp + (size_t)r * dst_stride * ew, (char*)m.result.p + 256 + row * r, row);
-  if (choice && choice->chosen < 0) {
-    const double s = std::chrono::duration<double>(std::chrono::steady_clock::now() - t0).count();
-    if (choice->calls % 3 != 0 && s < choice->best[(size_t)way]) choice->best[(size_t)way] = s;
-    if (++choice->calls == 3 * (int)choice->ways.size()) {
-      choice->chosen = (int)(std::min_element(choice->best.begin(), choice->best.end()) - choice->best.begin());
-      log_line(1, "host batch %d of %dx%d (%s): %zu parts, %.0f us", N, H, W, pinned ? "pinned" : "pageable",
-               choice->ways[(size_t)choice->chosen].size(), 1e6 * choice->best[(size_t)choice->chosen]);
-    }
-  }
   return ok();
+}
+
+// One device's share of a forward: images [sp, sp + N images) -> logits rows at dp (row pitch
+// dst_stride elements).  Runs on the calling thread's current device (g_dev), on stream st;
+// synchronises and reads the device status word unless device_only.
+int forward_slice(Model& m, const char* sp, bool src_dev, char* dp, bool dst_dev, size_t dst_stride, int N, int H, int W,
+                  cudaStream_t st, bool device_only) {
+  int rc;
+  const size_t ew = m.ele_width, row = (size_t)m.plan.out_features * ew;
+  if (src_dev) {
+    if ((rc = ensure_workspace(m, N, H, W))) return rc;
+    m.logits_off = 0;
+    if ((rc = model_forward_device(m, sp, N, H, W, st))) return rc;
+    const void* logits = m.io_dt == kF32 ? m.logits32.p : m.logits_io.p;
+    if (device_only && dst_stride * ew == row) CU(cudaMemcpyAsync(dp, logits, row * N, cudaMemcpyDeviceToDevice, st));
+    else CU(cudaMemcpy2DAsync(dp, dst_stride * ew, logits, row, row, (size_t)N, dst_dev ? cudaMemcpyDeviceToDevice : cudaMemcpyDeviceToHost, st));
+    if (device_only) return ok();
+    CU(cudaStreamSynchronize(st));
+    if ((rc = check_kernel_status())) return rc;
+    return ok();
+  }
+  // Images in host memory: a batch may run in parts, so that the copies of later parts overlap the forward of earlier ones
+  // (copies on their own stream, ordered by events).  More parts leave less of the last one exposed but make smaller, less
+  // efficient forwards -- which way wins depends on the network and the link, so the first call of a shape tries whole, halves
+  // and quarters (a run to let the layers tune themselves, two that count).  ResNet-18 fp16 256x224 from pinned memory (1.41 ms
+  // of copying): 2.20 ms in halves with blocking reads of logits and status, 2.03 ms now.  fp32 convolutions split their sums
+  // by the batch, so there a batch keeps one way.
+  const bool pinned = is_pinned_ptr(sp);
+  int n_parts = N >= 128 && N % 2 == 0 ? 2 : 1;
+  if (m.act_dt != kF32 && N >= 16 && g_autotune) {
+    const std::array<int, 4> key{N, H, W, (int)pinned};
+    auto it = m.part_choice.find(key);
+    if (it == m.part_choice.end()) {
+      double best = 1e30;
+      for (int parts : {1, 2, 4}) {
+        if (N / parts < 8) break;
+        for (int rep = 0; rep < 3; ++rep) {
+          const auto t0 = std::chrono::steady_clock::now();
+          if ((rc = forward_host(m, sp, pinned, dp, dst_dev, dst_stride, N, H, W, st, parts))) return rc;
+          const double t = std::chrono::duration<double>(std::chrono::steady_clock::now() - t0).count();
+          if (rep > 0 && t < best) { best = t; n_parts = parts; }
+        }
+      }
+      m.part_choice.emplace(key, n_parts);
+      log_line(1, "host batch %d of %dx%d (%s): %d parts, %.0f us", N, H, W, pinned ? "pinned" : "pageable", n_parts, 1e6 * best);
+      return ok();   // the runs have left the logits, the same each time
+    }
+    n_parts = it->second;
+  }
+  return forward_host(m, sp, pinned, dp, dst_dev, dst_stride, N, H, W, st, n_parts);
 }
 
 int forward_fanout(const char* sp, char* dp, size_t dst_stride, int N, int H, int W);
