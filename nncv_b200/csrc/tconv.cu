@@ -870,7 +870,9 @@ static int matmul_pick(int M, int N, int K, int sms) {
     const long long items = (pair ? (mi + 1) / 2 : mi) * ((N + bn - 1) / bn), slots = pair ? sms / 2 : sms;
     int s = 1;
     while (!pair && s < 8 && items * 2 * s <= slots * 15 / 16 && CB >= kSplitBlocks * 2 * s) s *= 2;
-    const double t = (double)((items + slots - 1) / slots) * ((CB + s - 1) / s * block[i] + epilogue[i]) + (pair ? 2.0 : s > 1 ? 3.0 : 0.0);
+    double rounds = (double)((items + slots - 1) / slots);
+    if (pair && items > slots && items % slots != 0 && 2 * (items % slots) <= slots) rounds -= 0.3;   // a last round of halves
+    const double t = rounds * ((CB + s - 1) / s * block[i] + epilogue[i]) + (pair ? 2.0 : s > 1 ? 3.0 : 0.0);
     if (t < best) { best = t; best_bn = bn; }
   }
   return best_bn;
