@@ -7,10 +7,13 @@
 // and what is dropped (a2*b3, a3*b2, a3*b3) is below 2^-26 of the product: less than the rounding of ONE fp32 multiply.
 // (Two tf32 parts, the other way to do this, keep 22 of the 24 bits, take as much tensor time -- three products at half
 // the rate -- and 8 bytes an element instead of 6.)
-// tcgen05.mma cuts every accumulation to fp32 instead of rounding it, an error of one sign per step.  So the products stay in
-// TMEM for ONE block of 64 channels (four steps of the large products a1*b1, twenty of the small ones, which have an
-// accumulator of their own) before the epilogue warps add them, rounded, to a sum in registers: logits of ResNet-18 are
-// within 4.9e-7 of the fp64-accumulated oracle (the CUDA-core kernel's: 2.3e-7; with four blocks a promotion: 1.1e-6).
+// tcgen05.mma cuts its products and sums instead of rounding them, an error of one sign that the layers of a network add
+// up: with normal operands every step of 16 channels takes 0.2 * 2^-24 off the sum it leaves.  So the large products a1*b1
+// stay in TMEM for ONE step only: the epilogue warps add each step, rounded, to a sum in registers.  (With the four steps of a
+// block of 64 channels in one accumulator the logits of ResNet-18 and ResNet-50 were 5.6e-7 and 1.2e-6 off the result in 64 bits,
+// nearly all of it this bias; the CUDA-core kernel's are 2.2e-7 to 3.3e-7 and 3.5e-7 off, now these 1.4e-7 to 1.9e-7 and 1.9e-7.
+// Networks on the device 3 to 4 % slower for it: ResNet-18 8x224 429 -> 446 us, ResNet-50 4x224 725 -> 755.)  The small products,
+// 2^-8 of the large ones, share an accumulator for up to kSmallBlocks blocks.
 //
 // Activations between the layers of an fp32 network are stored as planes, [3][N][H][W][C] bf16: the epilogue splits each
 // result once, and the tile loads are plain TMA copies of all three planes (nncv's fp32 graph: tests/Nets/Res18.mlir:118-629).
@@ -18,12 +21,12 @@
 // convolution with four taps of 64 "channels".
 //
 // One CTA computes 128 pixels x 64 or 128 output channels.  What bounds it: 72 or 96 KB of planes from L2 per block of 64
-// channels (1960 or 2700 clocks at what all SMs together get), then the 24 MMAs (1150 or 1540 clocks).  With few pixels (batch 1) a
+// channels (1560 or 2000 clocks with every SM at work), then the 24 MMAs (1150 or 1540 clocks).  With few pixels (batch 1) a
 // cluster of up to eight CTAs splits the reduction of a tile; each leaves its partial sums in shared memory and finishes
 // its share of the rows from all of them, in rank order, so that the result does not depend on timing.  (The CUDA-core
 // kernel needed a second pass over partial sums in global memory for that, and ran at a fifth of the fp32 rate.)
 //
-// ResNet-18 fp32 from host memory: 1x256 571 -> 337 us, 8x224 1945 -> 791 us.
+// ResNet-18 fp32 against the CUDA-core kernel, from device memory: 1x256 470 -> 233 us, 8x224 1626 -> 446 us.
 // Roles: warp 0 TMA producer, one plane of both operands per ring slot; warp 1 MMA issuer; warps 2-9 epilogue.
 // Every wait is bounded and abortable; a timed-out wait sets the device status word.
 #include <cuda.h>
@@ -47,6 +50,8 @@ constexpr int kThreads = 64 + kEpiThreads;
 constexpr int kABytes = 128 * 128;
 constexpr int kBBytes = 64 * 128;           // packed weights: tiles of 64 output channels x 64 input channels
 constexpr int kTileBytes = 128 * 64 * 4;    // partial sums of 64 of the tile's columns, fp32
+constexpr int kSmallBlocks = 4;             // blocks of 64 channels whose small products share an accumulator
+constexpr float kCut = 3.0f / (1 << 28);    // what a step of the tensor core cuts off its sum, on average (0.19 * 2^-24)
 template <int BN>
 struct Ring {   // a slot holds one plane of a block: 128 pixels and BN output channels x 64 channels
   static constexpr int kSlots = BN == 64 ? 7 : 5;
@@ -108,17 +113,20 @@ template <int kBN>   // output channels of a tile: 64 or 128
 __global__ void __launch_bounds__(kThreads, 1)
 conv_f32_kernel(const __grid_constant__ CUtensorMap tm_in, const F32Params p) {
   constexpr int kSlots = Ring<kBN>::kSlots, kSlot = Ring<kBN>::kSlot, kNT = kBN / 64;
-  constexpr uint32_t kTmemCols = 4 * kBN;   // two buffers of two accumulators (large and small products)
+  // Accumulators: pairs for two steps of the large products, and two for the small ones.  A pair is handed over as one: the
+  // epilogue's time is the latency of a hand-over, about 400 clocks, and four a block of 64 channels took longer than the copies.
+  constexpr uint32_t kPairs = kBN == 64 ? 2 : 1, kAcc = kPairs + 2;
+  constexpr uint32_t kTmemCols = 512, kSmallCols = kPairs * 2 * kBN;
   constexpr int kCols = kBN / 2;            // columns of a thread's row
   extern __shared__ uint8_t smem_raw[];
   __shared__ int s_abort;
-  __shared__ __align__(8) unsigned long long s_bars[2 * kSlots + 2 + 2 + 2];
+  __shared__ __align__(8) unsigned long long s_bars[2 * kSlots + 2 * kAcc + 2];
   const uint32_t raw = ptx::smem_u32(smem_raw);
   const uint32_t sRing = (raw + 1023u) & ~1023u;
   const uint32_t sTile = sRing + kSlots * kSlot;
   const uint32_t full = ptx::smem_u32(s_bars), empty = full + 8 * kSlots;
-  const uint32_t d_full = empty + 8 * kSlots, d_empty = d_full + 16;
-  const uint32_t part_ready = d_empty + 16, part_done = part_ready + 8;
+  const uint32_t d_full = empty + 8 * kSlots, d_empty = d_full + 8 * kAcc;   // pairs first
+  const uint32_t part_ready = d_empty + 8 * kAcc, part_done = part_ready + 8;
   __shared__ uint32_t s_tmem;
   const int warp = ptx::warp_uniform((int)threadIdx.x >> 5), lane = threadIdx.x & 31;
   const int S = p.splits;
@@ -130,7 +138,7 @@ conv_f32_kernel(const __grid_constant__ CUtensorMap tm_in, const F32Params p) {
       ptx::mbar_init(full + 8 * i, 1);
       ptx::mbar_init(empty + 8 * i, 1);
     }
-    for (int i = 0; i < 2; ++i) {
+    for (uint32_t i = 0; i < kAcc; ++i) {
       ptx::mbar_init(d_full + 8 * i, 1);
       ptx::mbar_init(d_empty + 8 * i, epi::kWarps);
     }
@@ -228,51 +236,68 @@ conv_f32_kernel(const __grid_constant__ CUtensorMap tm_in, const F32Params p) {
     // ------------------------------------------------------------------ MMA issuer ------
     const uint32_t issue = ptx::elect_one();
     const uint32_t idesc = ptx::umma_idesc(128, kBN, 1);
-    uint32_t slot = 0, ring = 0, blk = 0;   // blk: running count of blocks; accumulator buffer blk % 2
+    uint32_t slot = 0, ring = 0;
+    uint32_t large = 0, small = 0;   // running counts of uses of pairs and of small accumulators
     bool okw = true;
     uint32_t seen = ptx::mbar_peek(full, 0);
     auto step = [&]() {
       if (++slot == kSlots) { slot = 0; ring ^= 1u; }
       seen = ptx::mbar_peek(full + 8 * slot, ring);
     };
-    // one product of the block's planes: four k steps of 16
-    auto product = [&](uint32_t d, uint32_t a, uint32_t b, uint32_t fresh) {
-      const uint32_t a_lo = ptx::smem_desc_k128_lo(a), b_lo = ptx::smem_desc_k128_lo(b);
-#pragma unroll
-      for (uint32_t k4 = 0; k4 < 4; ++k4)
-        ptx::umma_f16(d, ptx::desc_from_halves(a_lo + k4 * 2, ptx::kSmemDescK128Hi), ptx::desc_from_halves(b_lo + k4 * 2, ptx::kSmemDescK128Hi),
-                      idesc, k4 == 0 ? (fresh ^ 1u) : 1u, issue);
+    auto mma = [&](uint32_t d, uint32_t a, uint32_t b, uint32_t k4, uint32_t accumulate) {
+      ptx::umma_f16(d, ptx::desc_from_halves(ptx::smem_desc_k128_lo(a) + k4 * 2, ptx::kSmemDescK128Hi),
+                    ptx::desc_from_halves(ptx::smem_desc_k128_lo(b) + k4 * 2, ptx::kSmemDescK128Hi), idesc, accumulate, issue);
     };
+    // a product of two planes of the block: four steps of 16 channels
+    auto product = [&](uint32_t d, uint32_t a, uint32_t b, uint32_t fresh) {
+#pragma unroll
+      for (uint32_t k4 = 0; k4 < 4; ++k4) mma(d, a, b, k4, k4 == 0 ? (fresh ^ 1u) : 1u);
+    };
+    // waits until the epilogue has emptied accumulator acc, filled `turn` times before
+    auto wait_empty = [&](uint32_t acc, uint32_t turn) { return ptx::warp_wait(d_empty + 8 * acc, (turn & 1u) ^ 1u, abort_flag); };
     for (int i = 0; okw; ++i) {
       int n0, oy0, ox0, n_tile;
       if (!item_of(i, n0, oy0, ox0, n_tile)) break;
-      for (int kb = kb0; kb < kb1; ++kb, ++blk) {
-        const uint32_t d0 = tmem_base + (blk & 1u) * (2 * kBN), d1 = d0 + kBN;
-        if (!ptx::warp_wait(d_empty + 8 * (blk & 1u), ((blk >> 1) & 1u) ^ 1u, abort_flag)) { okw = false; break; }
+      for (int kb = kb0; kb < kb1; ++kb) {
+        const bool group_first = (kb - kb0) % kSmallBlocks == 0, group_last = (kb - kb0) % kSmallBlocks == kSmallBlocks - 1 || kb + 1 == kb1;
+        const uint32_t small_acc = kPairs + (small & 1u), ds = tmem_base + kSmallCols + (small & 1u) * kBN;
         uint32_t at[3], sl[3];
-#pragma unroll
-        for (int pl = 0; pl < 3; ++pl) {
-          if (okw && !ptx::warp_all(seen) && !ptx::warp_wait(full + 8 * slot, ring, abort_flag)) okw = false;
-          if (!okw) break;
+        // the next plane of the block
+        auto arrive = [&](int pl) {
+          if (!ptx::warp_all(seen) && !ptx::warp_wait(full + 8 * slot, ring, abort_flag)) return false;
           ptx::tc_fence_after();
           sl[pl] = slot;
           at[pl] = sRing + slot * kSlot;
           step();
-          if (pl == 0) {
-            product(d0, at[0], at[0] + kABytes, 1u);
-          } else if (pl == 1) {
-            product(d1, at[0], at[1] + kABytes, 1u);
-            product(d1, at[1], at[0] + kABytes, 0u);
-            product(d1, at[1], at[1] + kABytes, 0u);
-          } else {
-            product(d1, at[0], at[2] + kABytes, 0u);
-            product(d1, at[2], at[0] + kABytes, 0u);
-          }
-        }
-        if (!okw) break;
+          return true;
+        };
+        // two steps of the large products, each into an accumulator of its own
+        auto two_large = [&](uint32_t k4) {
+          const uint32_t pair = large % kPairs;
+          if (!wait_empty(pair, large / kPairs)) return false;
+          ptx::tc_fence_after();
+#pragma unroll
+          for (uint32_t j = 0; j < 2; ++j) mma(tmem_base + (2 * pair + j) * kBN, at[0], at[0] + kABytes, k4 + j, 0u);
+          ptx::tc_commit(d_full + 8 * pair, issue);
+          ++large;
+          return true;
+        };
+        if (!arrive(0) || !two_large(0)) { okw = false; break; }
+        if (!arrive(1) || (group_first && !wait_empty(small_acc, small >> 1))) { okw = false; break; }
+        ptx::tc_fence_after();
+        product(ds, at[0], at[1] + kABytes, group_first ? 1u : 0u);
+        product(ds, at[1], at[0] + kABytes, 0u);
+        product(ds, at[1], at[1] + kABytes, 0u);
+        // the other two steps, when the epilogue has had the time to empty the accumulators
+        if (!two_large(2) || !arrive(2)) { okw = false; break; }
+        product(ds, at[0], at[2] + kABytes, 0u);
+        product(ds, at[2], at[0] + kABytes, 0u);
 #pragma unroll
         for (int pl = 0; pl < 3; ++pl) ptx::tc_commit(empty + 8 * sl[pl], issue);
-        ptx::tc_commit(d_full + 8 * (blk & 1u), issue);
+        if (group_last) {
+          ptx::tc_commit(d_full + 8 * small_acc, issue);
+          ++small;
+        }
       }
     }
     if (!okw && lane == 0 && p.error_flag) atomicCAS(p.error_flag, 0, (int)kErrWaitMma);
@@ -283,7 +308,7 @@ conv_f32_kernel(const __grid_constant__ CUtensorMap tm_in, const F32Params p) {
     const int et = (int)threadIdx.x - 64;
     const int rows_each = 128 / S, row_lo = (int)rank * rows_each;
     const int g = et & 15;             // four columns of the tile
-    uint32_t blk = 0;
+    uint32_t large = 0, small = 0;     // running counts of uses of the accumulators
     bool okw = true;
     for (int i = 0; okw; ++i) {
       int n0, oy0, ox0, n_tile;
@@ -316,24 +341,47 @@ conv_f32_kernel(const __grid_constant__ CUtensorMap tm_in, const F32Params p) {
       float sum[kCols];
 #pragma unroll
       for (int e = 0; e < kCols; ++e) sum[e] = 0.0f;
-      for (int kb = kb0; kb < kb1; ++kb, ++blk) {
-        okw = ptx::warp_wait(d_full + 8 * (blk & 1u), (blk >> 1) & 1u, abort_flag);
-        if (!okw) break;
+      auto hand_back = [&](uint32_t acc) {
+        ptx::tc_fence_before();
+        __syncwarp();
+        if (lane == 0) ptx::mbar_arrive(d_empty + 8 * acc);
+      };
+      // adds a pair's columns (this thread's row) to the sums
+      auto take_pair = [&](uint32_t pair, uint32_t turn) {
+        if (!ptx::warp_wait(d_full + 8 * pair, turn & 1u, abort_flag)) return false;
         ptx::tc_fence_after();
 #pragma unroll
         for (int h = 0; h < kCols / 32; ++h) {
-          uint32_t big[32], small[32];
-          ptx::tmem_ld_32x32(lane_base + (blk & 1u) * (2 * kBN) + h * 32, big);
-          ptx::tmem_ld_32x32(lane_base + (blk & 1u) * (2 * kBN) + kBN + h * 32, small);
-          ptx::tmem_ld_wait();
-          if (h == kCols / 32 - 1) {
-            ptx::tc_fence_before();
-            __syncwarp();
-            if (lane == 0) ptx::mbar_arrive(d_empty + 8 * (blk & 1u));
-          }
+          uint32_t v[2][32];
 #pragma unroll
-          for (int e = 0; e < 32; ++e) sum[h * 32 + e] += __uint_as_float(big[e]) + __uint_as_float(small[e]);
+          for (uint32_t j = 0; j < 2; ++j) ptx::tmem_ld_32x32(lane_base + (2 * pair + j) * kBN + h * 32, v[j]);
+          ptx::tmem_ld_wait();
+          if (h == kCols / 32 - 1) hand_back(pair);
+#pragma unroll
+          for (int e = 0; e < 32; ++e) sum[h * 32 + e] += __uint_as_float(v[0][e]) + __uint_as_float(v[1][e]);
         }
+        return true;
+      };
+      // adds small products; `cut` of the sum is given back with the last of them, whose low bits decide how it rounds
+      auto take_small = [&](float cut) {
+        const uint32_t acc = kPairs + (small & 1u);
+        if (!ptx::warp_wait(d_full + 8 * acc, (small >> 1) & 1u, abort_flag)) return false;
+        ptx::tc_fence_after();
+#pragma unroll
+        for (int h = 0; h < kCols / 32; ++h) {
+          uint32_t v[32];
+          ptx::tmem_ld_32x32(lane_base + kSmallCols + (small & 1u) * kBN + h * 32, v);
+          ptx::tmem_ld_wait();
+          if (h == kCols / 32 - 1) hand_back(acc);
+#pragma unroll
+          for (int e = 0; e < 32; ++e) sum[h * 32 + e] += fmaf(sum[h * 32 + e], cut, __uint_as_float(v[e]));
+        }
+        ++small;
+        return true;
+      };
+      for (int kb = kb0; kb < kb1 && okw; ++kb) {
+        for (int k4 = 0; k4 < 4 && okw; k4 += 2, ++large) okw = take_pair(large % kPairs, large / kPairs);
+        if (okw && ((kb - kb0) % kSmallBlocks == kSmallBlocks - 1 || kb + 1 == kb1)) okw = take_small(kb + 1 == kb1 ? kCut : 0.0f);
       }
       // 64 columns at a time: 32 of either half of the tile
 #pragma unroll
@@ -640,9 +688,9 @@ cudaError_t launch_avgpool_planes(const void* src, void* dst, int N, int HW, int
 bool conv_f32_supported(int C, int Kout, int tw_stride) { return C % 8 == 0 && Kout % 4 == 0 && tw_stride <= 256; }
 
 // Tile width and the CTAs of a cluster that share a tile's reduction: the pair with the least rounds x time.  A block of 64
-// channels takes about 1960 clocks with 64 columns and 2700 with 128 when every SM works (both bound by L2 -> shared
-// memory, 34 to 37 bytes a clock and SM: 72 and 96 KB); everything else about 8000 and 14000 a tile (the wide tile is
-// finished in two passes), a split 1500 more.  Clusters of sixteen were slower at batch 1 than clusters of eight (21 us
+// channels takes about 1560 clocks with 64 columns and 2000 with 128 when every SM works (both bound by L2 -> shared
+// memory, 46 to 48 bytes a clock and SM: 72 and 96 KB; 3x3 filters of 256 and 512 channels at batch 64); everything else about
+// 4700 and 12000 a tile (the wide tile is finished in two passes), a split 1500 more.  Clusters of sixteen were slower at batch 1 than clusters of eight (21 us
 // against 15 for a layer of 256 channels on 16 x 16 pixels).  Fewer clusters fit the GPU than its SMs would hold (they do not
 // cross GPC borders), so the runtime is asked.
 template <int BN>
@@ -661,7 +709,7 @@ static void pick_tile(long long m_tiles, int Kout, int kb_all, int sms, int* bn,
       const int slots = b == 64 ? clusters_that_fit<64>(s, sms) : clusters_that_fit<128>(s, sms);
       const long long tiles = m_tiles * ((Kout + b - 1) / b);
       const double rounds = (double)((tiles + slots - 1) / slots);
-      const double t = rounds * (((kb_all + s - 1) / s) * (b == 64 ? 1960.0 : 2700.0) + (b == 64 ? 3000.0 : 9000.0)) + 5000.0 + (s > 1 ? 1500.0 : 0.0);
+      const double t = rounds * (((kb_all + s - 1) / s) * (b == 64 ? 1560.0 : 2000.0) + (b == 64 ? 4700.0 : 12000.0)) + 5000.0 + (s > 1 ? 1500.0 : 0.0);
       if (t < best) { best = t; *bn = b; *splits = s; }
     }
 }
