@@ -13,8 +13,10 @@
 // filter value serves eight outputs.  With eight channels a thread and strips of four rows the 5x5 layers were bound by
 // shared memory: a filter vector of eight fp32 is two loads at a stride of 32 bytes, two-way bank conflicts, and those loads
 // were two thirds of the traffic (14x14x240 at batch 256: 9.8 M wavefronts, 48 us); now a lane's four filter values are 16
-// contiguous bytes and are read half as often.  The filter times the scale, and the shift the sums start at, sit in shared
-// memory.
+// contiguous bytes and are read half as often.  Filter, scale and shift sit in shared memory: for the 16-bit types as the
+// filter times the scale and the shift the sums start at; for fp32, where the product's rounding would be one more error of
+// the size of the others (and the same for every pixel, so that it survives averaging: MobileNetV3's fp32 logits were
+// 4.3e-7 off the result in 64 bits instead of 3.3e-7), one by one.
 // Every wait on a copy is bounded; a wait that gives up sets the status word and the CTA leaves.
 #include <cuda.h>
 #include <cuda_bf16.h>
@@ -37,6 +39,7 @@ constexpr int kTH = 8;           // output rows per tile
 // output rows per thread: the tile's eight, or four in fp32, whose rows are twice as long (with strips of eight a tile
 // needs 38 KB a stage and only two CTAs fit an SM)
 template <typename T> constexpr int kRows = sizeof(T) == 4 ? 4 : 8;
+template <typename T> constexpr bool kFold = sizeof(T) == 2;   // the scale multiplied into the filter
 constexpr int kMaxStages = 3;
 
 struct DwParams {
@@ -130,8 +133,9 @@ __global__ void __launch_bounds__(kThreads, KS == 3 ? 3 : 2) depthwise_tma_kerne
   const int CB = cbv * kPer * V;                         // channels per chunk
   const int IW = (tw - 1) * STRIDE + KS;
   const int c0 = blockIdx.y * CB;
-  float* sw = reinterpret_cast<float*>(smem + (size_t)p.stages * p.stage_stride);   // [KS*KS][CB] filter times scale, shift[CB]
+  float* sw = reinterpret_cast<float*>(smem + (size_t)p.stages * p.stage_stride);   // [KS*KS][CB] filter, shift[CB], scale[CB] unless folded
   float* ssh = sw + KS * KS * CB;
+  float* ssc = ssh + CB;
 
   if (tid == 0) {
     abort_flag = 0;
@@ -145,11 +149,14 @@ __global__ void __launch_bounds__(kThreads, KS == 3 ? 3 : 2) depthwise_tma_kerne
     if (c0 + c < p.C) {
       const size_t idx = (size_t)(c0 + c) * (KS * KS) + tap;
       v = p.w_half ? __half2float(reinterpret_cast<const __half*>(p.w)[idx]) : reinterpret_cast<const float*>(p.w)[idx];
-      if (p.scale) v *= p.scale[c0 + c];
+      if (kFold<T> && p.scale) v *= p.scale[c0 + c];
     }
     sw[i] = v;
   }
-  for (int c = tid; c < CB; c += kThreads) ssh[c] = (c0 + c < p.C && p.shift) ? p.shift[c0 + c] : 0.0f;
+  for (int c = tid; c < CB; c += kThreads) {
+    ssh[c] = (c0 + c < p.C && p.shift) ? p.shift[c0 + c] : 0.0f;
+    if (!kFold<T>) ssc[c] = (c0 + c < p.C && p.scale) ? p.scale[c0 + c] : 1.0f;
+  }
   __syncthreads();
 
   const int my_tiles = ((int)blockIdx.x < p.n_tiles) ? (p.n_tiles - 1 - (int)blockIdx.x) / (int)gridDim.x + 1 : 0;
@@ -180,10 +187,10 @@ __global__ void __launch_bounds__(kThreads, KS == 3 ? 3 : 2) depthwise_tma_kerne
 
     if (kP == kTH ? x >= tw : ys >= kTH / kP) continue;  // no strip of the tile is this thread's
     const unsigned char* st = smem + (size_t)s * p.stage_stride;
-    // the sums start at the shift; the filter carries the scale
+    // folded: the sums start at the shift, the filter carries the scale
     u64 acc[kP][2];
     {
-      const ulonglong2 sh = *reinterpret_cast<const ulonglong2*>(ssh + cvec * V);
+      const ulonglong2 sh = kFold<T> ? *reinterpret_cast<const ulonglong2*>(ssh + cvec * V) : make_ulonglong2(0, 0);
 #pragma unroll
       for (int o = 0; o < kP; ++o) { acc[o][0] = sh.x; acc[o][1] = sh.y; }
     }
@@ -211,6 +218,14 @@ __global__ void __launch_bounds__(kThreads, KS == 3 ? 3 : 2) depthwise_tma_kerne
     const int4 ti = tile_info[s];
     const int ox = ti.z + x, c = c0 + cvec * V;
     if (ox < p.OW && c < p.C) {
+      if (!kFold<T>) {
+        const ulonglong2 sc = *reinterpret_cast<const ulonglong2*>(ssc + cvec * V), sh = *reinterpret_cast<const ulonglong2*>(ssh + cvec * V);
+#pragma unroll
+        for (int o = 0; o < kP; ++o) {
+          acc[o][0] = epi::fma2(acc[o][0], sc.x, sh.x);
+          acc[o][1] = epi::fma2(acc[o][1], sc.y, sh.y);
+        }
+      }
       T* yp = reinterpret_cast<T*>(p.y) + (((size_t)ti.x * p.out_l.img_rows + ti.y + ys * kP + p.out_l.off) * p.out_l.pitch + ox + p.out_l.off) * p.C + c;
       const size_t row_step = (size_t)p.out_l.pitch * p.C;
       const int rows = min(kP, p.OH - ti.y - ys * kP);
@@ -312,7 +327,7 @@ cudaError_t launch_depthwise_tma(const void* x, const void* w, DType w_dt, const
     if (cand > cv) continue;
     const int tiles = (OW + slots / cand - 1) / (slots / cand), t = (OW + tiles - 1) / tiles;
     const int chunks = (cv + cand - 1) / cand, iw = (t - 1) * stride + R, ih = (kTH - 1) * stride + R;
-    const size_t need = 2 * (((size_t)iw * ih * cand * 16 + 127) & ~(size_t)127) + (size_t)(R * S + 1) * cand * V * sizeof(float);
+    const size_t need = 2 * (((size_t)iw * ih * cand * 16 + 127) & ~(size_t)127) + (size_t)(R * S + (es == 2 ? 1 : 2)) * cand * V * sizeof(float);
     if (need > 200 * 1024 || iw > 256) continue;
     double use = (double)cv / (chunks * cand) * OW / (tiles * t) * (t * cand) / slots;
     use *= 0.5 + 0.5 * (t * stride) / iw;
@@ -326,7 +341,7 @@ cudaError_t launch_depthwise_tma(const void* x, const void* w, DType w_dt, const
   if (IW > 256 || IH > 256) return cudaErrorInvalidValue;
   p.stage_bytes = (uint32_t)IW * IH * cbv * 16;
   p.stage_stride = (p.stage_bytes + 127u) & ~127u;
-  const size_t wbytes = (size_t)(R * S + 1) * cbv * V * sizeof(float);
+  const size_t wbytes = (size_t)(R * S + (es == 2 ? 1 : 2)) * cbv * V * sizeof(float);
   int stages = kMaxStages;
   while (stages > 2 && (size_t)stages * p.stage_stride + wbytes > 72 * 1024) --stages;   // three CTAs per SM when it fits
   const size_t smem = (size_t)stages * p.stage_stride + wbytes;
