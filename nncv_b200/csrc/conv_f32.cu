@@ -1,7 +1,8 @@
 // fp32 convolutions on the tensor cores: implicit GEMM over THREE bf16 PLANES per operand.
 //
 // Every fp32 value x is kept as x = x1 + x2 + x3, three bf16 numbers, each the nearest to what the ones before leave; with
-// 8 significand bits each and signed remainders the sum is exact.  A product is then six bf16 products with fp32
+// 8 significand bits each and signed remainders the sum is exact (from 2^-110 on; below, the third falls short of bf16's smallest
+// number and x is kept to an absolute 2^-134).  A product is then six bf16 products with fp32
 // accumulation,
 //     a*b ~= a1*b1 + (a1*b2 + a2*b1) + a2*b2 + (a1*b3 + a3*b1),
 // and what is dropped (a2*b3, a3*b2, a3*b3) is below 2^-26 of the product: less than the rounding of ONE fp32 multiply.
@@ -12,7 +13,8 @@
 // stay in TMEM for ONE step only: the epilogue warps add each step, rounded, to a sum in registers.  (With the four steps of a
 // block of 64 channels in one accumulator the logits of ResNet-18 and ResNet-50 were 5.6e-7 and 1.2e-6 off the result in 64 bits,
 // nearly all of it this bias; the CUDA-core kernel's are 2.2e-7 to 3.3e-7 and 3.5e-7 off, now these 1.4e-7 to 1.9e-7 and 1.9e-7.
-// Networks on the device 3 to 4 % slower for it: ResNet-18 8x224 429 -> 446 us, ResNet-50 4x224 725 -> 755.)  The small products,
+// Networks on the device 3 to 4 % slower for it: ResNet-18 8x224 429 -> 446 us, ResNet-50 4x224 725 -> 755; with the care for
+// infinities 452 and 769.)  The small products,
 // 2^-8 of the large ones, share an accumulator for up to kSmallBlocks blocks.
 //
 // Activations between the layers of an fp32 network are stored as planes, [3][N][H][W][C] bf16: the epilogue splits each
@@ -26,7 +28,7 @@
 // its share of the rows from all of them, in rank order, so that the result does not depend on timing.  (The CUDA-core
 // kernel needed a second pass over partial sums in global memory for that, and ran at a fifth of the fp32 rate.)
 //
-// ResNet-18 fp32 against the CUDA-core kernel, from device memory: 1x256 470 -> 233 us, 8x224 1626 -> 446 us.
+// ResNet-18 fp32 against the CUDA-core kernel, from device memory: 1x256 470 -> 233 us, 8x224 1626 -> 452 us.
 // Roles: warp 0 TMA producer, one plane of both operands per ring slot; warp 1 MMA issuer; warps 2-9 epilogue.
 // Every wait is bounded and abortable; a timed-out wait sets the device status word.
 #include <cuda.h>
@@ -77,10 +79,12 @@ struct F32Params {
   int splits;                 // CTAs of a cluster that share a tile's reduction (a power of two up to 8)
 };
 
+// Infinities and NaN stay in the first plane; a finite value too large to be rounded to bf16 is cut to the largest one.
 __device__ __forceinline__ void split3(float x, __nv_bfloat16& a, __nv_bfloat16& b, __nv_bfloat16& c) {
-  a = __float2bfloat16_rn(x);
-  const float h = __bfloat162float(a);
-  const float r = fabsf(h) <= FLT_MAX ? x - h : 0.0f;   // infinities and NaN stay in the first plane
+  constexpr float kMaxBf16 = 3.38953139e38f;   // 2^128 - 2^120
+  const bool finite = fabsf(x) <= FLT_MAX;
+  a = __float2bfloat16_rn(finite ? fminf(fmaxf(x, -kMaxBf16), kMaxBf16) : x);
+  const float r = finite ? x - __bfloat162float(a) : 0.0f;
   b = __float2bfloat16_rn(r);
   c = __float2bfloat16_rn(r - __bfloat162float(b));
 }
@@ -362,7 +366,8 @@ conv_f32_kernel(const __grid_constant__ CUtensorMap tm_in, const F32Params p) {
         }
         return true;
       };
-      // adds small products; `cut` of the sum is given back with the last of them, whose low bits decide how it rounds
+      // adds small products; `cut` of the sum is given back with the last of them, whose low bits decide how it rounds.  An
+      // infinite or NaN operand has made the sum what it has to be; its small products (inf * 0, inf - inf) say nothing.
       auto take_small = [&](float cut) {
         const uint32_t acc = kPairs + (small & 1u);
         if (!ptx::warp_wait(d_full + 8 * acc, (small >> 1) & 1u, abort_flag)) return false;
@@ -374,7 +379,10 @@ conv_f32_kernel(const __grid_constant__ CUtensorMap tm_in, const F32Params p) {
           ptx::tmem_ld_wait();
           if (h == kCols / 32 - 1) hand_back(acc);
 #pragma unroll
-          for (int e = 0; e < 32; ++e) sum[h * 32 + e] += fmaf(sum[h * 32 + e], cut, __uint_as_float(v[e]));
+          for (int e = 0; e < 32; ++e) {
+            const float s = sum[h * 32 + e], t = s + fmaf(s, cut, __uint_as_float(v[e]));
+            sum[h * 32 + e] = fabsf(s) <= FLT_MAX ? t : s;
+          }
         }
         ++small;
         return true;

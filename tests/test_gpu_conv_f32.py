@@ -80,3 +80,49 @@ def test_conv_f32_sums_have_no_bias(kind, c):
     # a step of 16 channels takes 0.09 (half of the operands zero) to 0.28 (all of one sign) times 2^-24 off its sum, of which
     # 0.19 are given back; with four steps in one accumulator 0.46 to 1.3 were missing
     assert abs(float(off @ ref / (ref @ ref))) <= 0.25 * 2.0 ** -24
+
+
+@pytest.mark.parametrize("r,c,k", [(1, 128, 64), (1, 72, 128), (3, 64, 64), (3, 512, 8)])   # 3x3 over 512 channels: split over a cluster
+def test_conv_f32_infinities_nan_and_the_largest_values(r, c, k):
+    """Non-finite inputs and weights end where IEEE arithmetic puts them, and finite values above the largest bf16 stay finite."""
+    g = np.random.default_rng(r * c)
+    n, h, w = 1, 9, 12
+    x = g.standard_normal((n, c, h, w)).astype(np.float32)
+    wt = g.standard_normal((k, c, r, r)).astype(np.float32)
+    wt[::2] = np.round(wt[::2] * 4) / 4              # exact in bf16, zeros among them: the remainders are zero
+    x[0, 3, 1, 1], x[0, 5, 4, 9], x[0, 7, 7, 2], x[0, c - 1, 7, 9] = np.inf, -np.inf, np.nan, np.inf
+    x[0, 0, 7, 9] = -np.inf                          # meets the +inf of another channel
+    wt[3 % k, 1, 0, 0] = np.inf
+    big = np.float32(3.4e38)
+    x[0, :, 4, 5] = 0
+    x[0, 2, 4, 5] = big
+    wt[:, 2] = np.where(np.abs(wt[:, 2]) > 0.9, np.float32(1.0), np.float32(0.25))
+    conv = G.Conv(wt, 1, r // 2, F32)
+    try:
+        y, _ = conv.run(x, None, None, None, False)
+    finally:
+        conv.close()
+    with np.errstate(all="ignore"):
+        ref64 = torch.nn.functional.conv2d(torch.from_numpy(x).double(), torch.from_numpy(wt).double(), None, 1, r // 2).numpy()
+        ref = np.where(np.abs(ref64) > np.finfo(np.float32).max, np.sign(ref64) * np.inf, ref64)
+    sure = ~(np.abs(np.abs(ref64) / np.finfo(np.float32).max - 1) < 1e-5)   # the border to infinity itself
+    assert np.array_equal(np.isnan(y[sure]), np.isnan(ref[sure]))
+    inf = np.isinf(ref) & sure
+    assert inf.any() and np.isnan(ref).any() and (np.abs(ref[np.isfinite(ref)]) > 3e38).any()
+    assert np.array_equal(y[inf], ref[inf].astype(np.float32))
+    fin = np.isfinite(ref) & sure
+    size = torch.nn.functional.conv2d(torch.from_numpy(np.nan_to_num(np.abs(x), posinf=0)).double(),
+                                      torch.from_numpy(np.nan_to_num(np.abs(wt), posinf=0)).double(), None, 1, r // 2).numpy()
+    assert (np.abs(y[fin] - ref[fin]) <= 4e-6 * size[fin]).all()   # 2^-24 for each of at most 64 partial sums of the magnitudes
+
+
+def test_conv_f32_tiny_values():
+    """Below 2^-110 the third plane runs out of bf16's range: a value is kept to half of 2^-133."""
+    g = np.random.default_rng(8)
+    x = (g.standard_normal((1, 128, 6, 6)) * 2.0 ** -116).astype(np.float32)
+    conv = G.Conv(np.eye(128, dtype=np.float32)[:, :, None, None], 1, 0, F32)
+    try:
+        y, _ = conv.run(x, None, None, None, False)
+    finally:
+        conv.close()
+    assert np.abs(y.astype(np.float64) - x).max() <= 2.0 ** -134
