@@ -104,6 +104,8 @@ struct Device {
   int* error_flag = nullptr;   // device
   cudaStream_t copy_stream = nullptr;  // host->device copies of a split batch
   cudaEvent_t copy_done[kMaxParts + 1] = {};   // one per part + one ordering the copies after earlier work
+  cudaMemPool_t pool = nullptr;   // workspaces of convolution plans for the length of one call, in the order of its stream
+  int f32_plans = 0;              // plans that may take one; the pool's memory goes back when the last is destroyed
   cudaStream_t user_stream = nullptr;  // stream _mlir_ciface_forward runs on when set
   bool user_stream_set = false;
   int sm_count = 148;
@@ -317,6 +319,57 @@ struct DevBuf {
   }
 };
 
+// A workspace for the kernels of one call on `st`.  Calls on several streams, or several calls of one plan, each have their
+// own: it is taken and given back in the order of the stream.  While the stream is being captured it is ordinary memory of the
+// plan's, one piece for each captured call, since a graph may be replayed as long as the plan lives.  get() may find no memory.
+class StreamScratch {
+ public:
+  StreamScratch(std::vector<std::unique_ptr<DevBuf>>& kept, cudaStream_t st) : kept_(kept), st_(st) {}
+  StreamScratch(const StreamScratch&) = delete;
+  StreamScratch& operator=(const StreamScratch&) = delete;
+  ~StreamScratch() { if (p_) cudaFreeAsync(p_, st_); }
+  void* get(size_t bytes) {
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(st_, &cap) != cudaSuccess) cudaGetLastError();
+    if (cap != cudaStreamCaptureStatusNone) {
+      auto mode = cudaStreamCaptureModeRelaxed;   // a plain allocation does not concern the capture
+      cudaThreadExchangeStreamCaptureMode(&mode);
+      auto buf = std::make_unique<DevBuf>();
+      const cudaError_t e = cudaMalloc(&buf->p, bytes);
+      cudaThreadExchangeStreamCaptureMode(&mode);
+      if (e != cudaSuccess) {
+        buf->p = nullptr;
+        cudaGetLastError();
+        return nullptr;
+      }
+      buf->bytes = bytes;
+      kept_.push_back(std::move(buf));
+      return kept_.back()->p;
+    }
+    if (!g_dev.pool) {
+      cudaMemPoolProps props = {};
+      props.allocType = cudaMemAllocationTypePinned;
+      props.location.type = cudaMemLocationTypeDevice;
+      props.location.id = g_dev.id;
+      unsigned long long keep = ~0ull;   // from call to call; see f32_plans
+      if (cudaMemPoolCreate(&g_dev.pool, &props) != cudaSuccess || cudaMemPoolSetAttribute(g_dev.pool, cudaMemPoolAttrReleaseThreshold, &keep) != cudaSuccess) {
+        cudaGetLastError();
+        return nullptr;
+      }
+    }
+    if (cudaMallocFromPoolAsync(&p_, bytes, g_dev.pool, st_) != cudaSuccess) {
+      p_ = nullptr;
+      cudaGetLastError();
+    }
+    return p_;
+  }
+
+ private:
+  std::vector<std::unique_ptr<DevBuf>>& kept_;
+  cudaStream_t st_;
+  void* p_ = nullptr;
+};
+
 }  // namespace
 
 // =====================================================================================
@@ -396,7 +449,8 @@ struct nncv_b200_conv {
   bool act_done = false;  // set by conv_run when the kernel it launched applied want_act
   std::map<int, std::unique_ptr<DevBuf>> packed;   // tcgen05 path: per N-tile width
   DevBuf w_planes;                                 // fp32 on the tensor cores: filter as three bf16 planes
-  DevBuf in_planes;                                // the same, called on a dense fp32 map: its planes
+  std::vector<std::unique_ptr<DevBuf>> captured;   // planes of dense fp32 maps for the captured calls of the plan
+  bool counted = false;                            // in its device's f32_plans
   bool w_planes_ready = false;
   DevBuf w_f32;                                    // fp32 path: [Kout][R*S][Cpad]
   bool w_f32_ready = false;
@@ -486,9 +540,12 @@ bool f32_on_tensor_cores(const nncv_b200_conv& c, const void* in, const void* ou
   return c.C % 8 == 0 && c.Kout % 4 == 0 && ldo % 4 == 0 && c.stride <= 2 && !(al & 15) && (k >= 72 || k * c.Kout >= 8192);
 }
 
+// planes: workspace of the caller's for the planes of an fp32 input (bytes: planes_bytes); without one the call takes its own.
+size_t planes_bytes(const nncv_b200_conv& c, int N, int H, int W) { return (size_t)N * H * W * c.C * 6; }
+
 int conv_run(nncv_b200_conv* c, const void* in, Layout in_l, void* out, Layout out_l, int N, int H,
              int W, const float* scale, const float* shift, const void* residual, int relu,
-             DType out_dt, long long ldo, cudaStream_t st, const FusedBranch* fb = nullptr) {
+             DType out_dt, long long ldo, cudaStream_t st, const FusedBranch* fb = nullptr, const DevBuf* planes = nullptr) {
   const int OH = (H + 2 * c->pad - c->R) / c->stride + 1;
   const int OW = (W + 2 * c->pad - c->S) / c->stride + 1;
   if (N <= 0 || OH <= 0 || OW <= 0) return fail(NNCV_B200_EINVAL, "conv: empty output");
@@ -497,11 +554,13 @@ int conv_run(nncv_b200_conv* c, const void* in, Layout in_l, void* out, Layout o
   if (c->dtype == kF32) {
     if (in_l.off != 0 || out_l.off != 0) return fail(NNCV_B200_EINVAL, "fp32 conv takes dense NHWC only");
     if (f32_on_tensor_cores(*c, in, out, residual, ldo)) {
-      const long long elems = (long long)N * H * W * c->C;
-      int rc = c->in_planes.reserve((size_t)elems * 6);
-      if (rc) return rc;
-      LAUNCH(launch_split_planes((const float*)in, c->in_planes.p, elems, st));
-      return conv_run_planes(c, c->in_planes.p, false, N, H, W, scale, shift, residual, 1, relu, out, 1, ldo, st);
+      const size_t bytes = planes_bytes(*c, N, H, W);
+      StreamScratch own(c->captured, st);
+      void* q = planes ? (planes->bytes >= bytes ? planes->p : nullptr) : own.get(bytes);
+      if (q) {   // without the memory: the CUDA-core kernel
+        LAUNCH(launch_split_planes((const float*)in, q, (long long)(bytes / 6), st));
+        return conv_run_planes(c, q, false, N, H, W, scale, shift, residual, 1, relu, out, 1, ldo, st);
+      }
     }
     if (!c->w_f32_ready) {
       int rc = c->w_f32.reserve((size_t)c->Kout * c->R * c->S * c->Cpad * sizeof(float));
@@ -1117,6 +1176,8 @@ struct Model {
   bool planning = false, planned = false;
   int op_idx = 0;
   DevBuf arena;
+  DevBuf split_planes;             // fp32 network that is not `planes`: the planes of one convolution's input at a time
+  size_t split_bytes = 0;
   size_t act_bytes_unshared = 0;   // what one buffer per tensor would take
   size_t act_next = 0;
   HostCopier copier;          // images from pageable memory
@@ -1365,6 +1426,7 @@ int finish_act_plan(Model& m) {
   int rc = m.arena.reserve(base);
   if (rc) return rc;
   CU(cudaMemset(m.arena.p, 0, m.arena.bytes));
+  if (m.split_bytes && m.split_planes.reserve(m.split_bytes)) cudaGetLastError();   // the convolutions then stay on the CUDA cores
   log_line(1, "activation arena: %zu tensors in %zu bytes (%zu bytes as private buffers)", m.act_plan.size(), base, unshared);
   m.planned = true;
   return NNCV_B200_OK;
@@ -1379,6 +1441,7 @@ int model_forward_device(Model& m, const void* src_dev, int N, int H, int W, cud
     // first forward of this shape: one walk that launches nothing records the activation tensors
     m.planning = true;
     m.act_plan.clear();
+    m.split_bytes = 0;
     m.op_idx = 0;
     rc = model_forward_device(m, src_dev, m.wsN, H, W, st);
     m.planning = false;
@@ -1400,11 +1463,17 @@ int model_forward_device(Model& m, const void* src_dev, int N, int H, int W, cud
   struct Ten { void* p = nullptr; Layout l{0, 0, 0}; int h = 0, w = 0, c = 0; };
   std::map<int, Ten> tens;   // tensor id -> where it lives in this forward
   auto conv_of = [&](const PlanNode& n) -> nncv_b200_conv& { return *m.convs[n.conv_idx]; };
+  // the workspace conv_run may take for this convolution: noted in the planning pass
+  auto note_planes = [&](const nncv_b200_conv& c, const void* in, const void* out, const void* res, int h, int w) {
+    if (m.planning && adt == kF32 && !m.planes && f32_on_tensor_cores(c, in, out, res, c.Kout))
+      m.split_bytes = std::max(m.split_bytes, planes_bytes(c, N, h, w));
+  };
   auto run = [&](const PlanNode& n, const Ten& in, const Ten& out, const void* res) {
     nncv_b200_conv& c = conv_of(n);
+    note_planes(c, in.p, out.p, res, in.h, in.w);
     if (!begin_op({in.p, res})) return (int)NNCV_B200_OK;
     return conv_run(&c, in.p, in.l, out.p, out.l, N, in.h, in.w, m.scale[n.conv_idx], m.shift[n.conv_idx], res, n.relu, adt,
-                    c.Kout, st);
+                    c.Kout, st, nullptr, &m.split_planes);
   };
   const bool stem_fused_here = m.fused_stem && W <= 512 && H >= 7 && W >= 7;
   bool input_converted = false;
@@ -1697,15 +1766,17 @@ int model_forward_device(Model& m, const void* src_dev, int N, int H, int W, cud
           tens[n.id] = o;
           continue;
         }
+        note_planes(*fc, in.p, o.p, nullptr, 1, 1);
         if (begin_op({in.p}) &&
             (rc = conv_run(fc, in.p, dense_layout(1, 1), o.p, dense_layout(1, 1), N, 1, 1, nullptr, bias, nullptr, n.act == kActRelu, adt,
-                           n.cout, st)))
+                           n.cout, st, nullptr, &m.split_planes)))
           return rc;
         if (n.act > kActRelu && begin_op({o.p})) LAUNCH(launch_activation(o.p, o.p, adt, (size_t)N * n.cout, n.act, st));
         tens[n.id] = o;
         continue;
       }
       const int of = m.plan.out_features;
+      note_planes(*fc, in.p, m.logits32.p, nullptr, 1, 1);
       if (!begin_op({in.p})) return NNCV_B200_OK;   // the planning pass ends with the last reader of an activation tensor
       if (m.io_dt == adt && adt != kF32) {
         // 16-bit logits wanted and computed in the same type: the FC epilogue rounds once, exactly as
@@ -1714,7 +1785,7 @@ int model_forward_device(Model& m, const void* src_dev, int N, int H, int W, cud
                         st);
       }
       rc = m.planes ? conv_run_planes(fc, in.p, false, N, 1, 1, nullptr, bias, nullptr, 0, 0, (char*)m.logits32.p + m.logits_off, 1, of, st)
-                    : conv_run(fc, in.p, dense_layout(1, 1), (char*)m.logits32.p + m.logits_off, dense_layout(1, 1), N, 1, 1, nullptr, bias, nullptr, 0, kF32, of, st);
+                    : conv_run(fc, in.p, dense_layout(1, 1), (char*)m.logits32.p + m.logits_off, dense_layout(1, 1), N, 1, 1, nullptr, bias, nullptr, 0, kF32, of, st, nullptr, &m.split_planes);
       if (rc) return rc;
       if (m.io_dt != kF32)
         LAUNCH(launch_convert((char*)m.logits32.p + m.logits_off, kF32, (char*)m.logits_io.p + m.logits_off, m.io_dt, (size_t)N * of, st));
@@ -2601,6 +2672,10 @@ nncv_b200_conv* nncv_b200_conv_create(const void* weights, int w_dtype, int Kout
   }
   c->raw = c->raw_owned.p; c->raw_dt = (DType)w_dtype;
   c->sn = (long long)C * R * S; c->sc = (long long)R * S; c->stap = 1;
+  if (c->dtype == kF32) {
+    c->counted = true;
+    ++g_dev.f32_plans;
+  }
   ok();
   return c.release();
 }
@@ -2608,6 +2683,10 @@ nncv_b200_conv* nncv_b200_conv_create(const void* weights, int w_dtype, int Kout
 void nncv_b200_conv_destroy(nncv_b200_conv* c) {
   std::lock_guard<std::mutex> lk(g_mutex);
   if (c && current_device_or_null()) cudaDeviceSynchronize();
+  if (c && c->counted) {
+    Device& d = *g_devices[c->device];
+    if (--d.f32_plans == 0 && d.pool) cudaMemPoolTrimTo(d.pool, 0);
+  }
   delete c;
 }
 

@@ -126,3 +126,64 @@ def test_conv_f32_tiny_values():
     finally:
         conv.close()
     assert np.abs(y.astype(np.float64) - x).max() <= 2.0 ** -134
+
+
+def _plan_and_maps(sizes, c=128, k=128, r=3):
+    g = torch.Generator(device="cuda")
+    g.manual_seed(1)
+    w = torch.randn((k, c, r, r), device="cuda", generator=g) / (c * r * r) ** 0.5
+    conv = G.Conv(w.cpu().numpy(), 1, r // 2, F32)
+    xs = [torch.randn((n, 28, 28, c), device="cuda", generator=g) for n in sizes]
+
+    def run(x, y):
+        check(lib().nncv_b200_conv_run(conv.h, G.p(x), G.p(y), x.shape[0], 28, 28, None, None, None, 1, G.stream_ptr()))
+        return y
+
+    want = [run(x, torch.zeros((x.shape[0], 28, 28, k), device="cuda")) for x in xs]
+    G.sync_check()
+    return conv, xs, want, run
+
+
+def test_conv_f32_one_plan_on_two_streams():
+    """Calls of one plan on different streams share nothing that they write."""
+    conv, xs, want, run = _plan_and_maps([16, 16, 3])
+    try:
+        streams = [torch.cuda.Stream() for _ in xs]
+        got = [[torch.zeros_like(w) for w in want] for _ in range(20)]
+        G.sync_check()
+        for ys in got:
+            for s, x, y in zip(streams, xs, ys):
+                with torch.cuda.stream(s):
+                    run(x, y)
+        G.sync_check()
+        for ys in got:
+            assert all(torch.equal(y, w) for y, w in zip(ys, want))
+    finally:
+        conv.close()
+    assert lib().nncv_b200_device_status() == 0
+
+
+def test_conv_f32_captured_calls_keep_their_workspace():
+    """A graph of a plan's calls gives the same after larger calls of the plan, on another stream, and with two graphs in turn."""
+    conv, xs, want, run = _plan_and_maps([2, 5, 40])
+    try:
+        graphs, ys = [], [torch.zeros_like(w) for w in want[:2]]
+        for x, y in zip(xs, ys):
+            graphs.append(torch.cuda.CUDAGraph())
+            with torch.cuda.graph(graphs[-1]):
+                run(x, y)
+        assert torch.equal(run(xs[2], torch.zeros_like(want[2])), want[2])
+        for y in ys:
+            y.zero_()
+        G.sync_check()
+        streams = [torch.cuda.Stream() for _ in graphs]
+        for _ in range(10):
+            for s, gr in zip(streams, graphs):
+                with torch.cuda.stream(s):
+                    gr.replay()
+        G.sync_check()
+        assert all(torch.equal(y, w) for y, w in zip(ys, want))
+        del graphs
+    finally:
+        conv.close()
+    assert lib().nncv_b200_device_status() == 0
