@@ -2733,7 +2733,9 @@ int nncv_b200_conv_run(nncv_b200_conv* c, const void* in, void* out, int N, int 
     const size_t px = (size_t)N * H * W * dtype_size(c->dtype);
     auto over = [&](const void* q, size_t ch) { return q && ob < (const char*)q + px * ch && (const char*)q < ob + px * c->Kout; };
     bool dense = false;
-    if (g_autotune && !over(in, c->Cpad) && !over(residual, c->Kout) && !g_force_gather && c->cfg3.bn == 0 && tconv_supported(c->Cpad, c->Kout, c->dtype, c->Kout)) {
+    // (the copies of the conversions are aligned whatever the caller's tensors are)
+    const bool aligned = !((reinterpret_cast<uintptr_t>(in) | reinterpret_cast<uintptr_t>(out)) & 15) && !(reinterpret_cast<uintptr_t>(residual) & 31);
+    if (g_autotune && aligned && !over(in, c->Cpad) && !over(residual, c->Kout) && !g_force_gather && c->cfg3.bn == 0 && tconv_supported(c->Cpad, c->Kout, c->dtype, c->Kout)) {
       const std::array<int, 4> key{N, H, W, residual ? 1 : 0};
       char ckey[160];
       snprintf(ckey, sizeof(ckey), "conv3x3 way c%d k%d dt%d n%d h%d w%d res%d", c->Cpad, c->Kout, (int)c->dtype, N, H, W, residual ? 1 : 0);
@@ -2749,13 +2751,18 @@ int nncv_b200_conv_run(nncv_b200_conv* c, const void* in, void* out, int N, int 
         float ms[2] = {1e30f, 1e30f};
         rc = NNCV_B200_OK;
         for (int way = 0; way < 2 && !rc; ++way) {
-          if ((rc = way ? direct() : shifted())) break;   // tunes the tiles
+          rc = way ? direct() : shifted();   // tunes the tiles
           for (int grp = 0; grp < 3 && !rc; ++grp) {
             cudaEventRecord(e0, st);
             for (int rep = 0; rep < 4 && !rc; ++rep) rc = way ? direct() : shifted();
             cudaEventRecord(e1, st);
             float t = 0.f;
             if (cudaEventSynchronize(e1) == cudaSuccess && cudaEventElapsedTime(&t, e0, e1) == cudaSuccess && t < ms[way]) ms[way] = t;
+          }
+          if (way && rc) {   // refused, or without the memory it wants: not the better one
+            rc = NNCV_B200_OK;
+            ms[1] = 1e30f;
+            cudaGetLastError();
           }
         }
         cudaEventDestroy(e0);

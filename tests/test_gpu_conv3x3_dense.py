@@ -35,3 +35,26 @@ def test_ways_agree(n, c, h, w, k, dtype, res):
     if c == k:
         over = X.clone()
         assert torch.equal(run(chosen, over, over, R if res else None), want)
+
+
+@pytest.mark.parametrize("first", ["aligned", "offset"])
+def test_a_residual_at_sixteen_bytes(first):
+    """The conversions take a residual on any 16-byte boundary; the direct kernel wants 32 bytes and is then no candidate,
+    whichever came first."""
+    n, c, h, w = 4, 64, 56, 56
+    r = np.random.default_rng(2)
+    wt = (r.standard_normal((c, c, 3, 3)) / np.sqrt(9 * c)).astype(np.float32)
+    X = G.dev(r.standard_normal((n, h, w, c)).astype(np.float32), F16)
+    room = G.dev(r.standard_normal(X.numel() + 8).astype(np.float32), F16)
+    off = room[8:].view(n, h, w, c)
+    even = off.clone()
+    assert off.data_ptr() % 32 == 16 and even.data_ptr() % 32 == 0
+    conv = G.Conv(wt, 1, 1, F16, algo=2)
+    got = []
+    for res in (even, off, even) if first == "aligned" else (off, even, off):
+        y = torch.zeros_like(X)
+        check(lib().nncv_b200_conv_run(conv.h, G.p(X), G.p(y), n, h, w, None, None, G.p(res), 1, G.stream_ptr()))
+        got.append(y)
+    G.sync_check()
+    conv.close()
+    assert torch.equal(got[0], got[1]) and torch.equal(got[0], got[2])
