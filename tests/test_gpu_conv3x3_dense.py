@@ -58,3 +58,20 @@ def test_a_residual_at_sixteen_bytes(first):
     G.sync_check()
     conv.close()
     assert torch.equal(got[0], got[1]) and torch.equal(got[0], got[2])
+
+
+def test_the_trial_leaves_no_trace_in_the_profile():
+    """A profile around the first call of a shape, which times both ways, holds what a later call's holds."""
+    n, c, h, w = 2, 128, 30, 26
+    conv = G.Conv(np.random.default_rng(4).standard_normal((c, c, 3, 3)).astype(np.float32), 1, 1, F16, algo=2)
+    X = torch.randn((n, h, w, c), device="cuda", dtype=torch.float16)
+    Y = torch.zeros_like(X)
+    counts = []
+    for _ in range(2):
+        check(lib().nncv_b200_profile(1))
+        check(lib().nncv_b200_conv_run(conv.h, G.p(X), G.p(Y), n, h, w, None, None, None, 0, G.stream_ptr()))
+        G.sync_check()
+        counts.append(lib().nncv_b200_profile_count())
+        check(lib().nncv_b200_profile(0))
+    conv.close()
+    assert counts[0] == counts[1] == 1
