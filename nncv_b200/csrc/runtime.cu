@@ -2744,7 +2744,9 @@ int nncv_b200_conv_run(nncv_b200_conv* c, const void* in, void* out, int N, int 
         const std::string* v = g_tune_cache.find(ckey);
         if (v && (*v == "0" || *v == "1")) it = c->dense_ways.emplace(key, *v == "1").first;
       }
-      if (it == c->dense_ways.end()) {
+      cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+      if (it == c->dense_ways.end() && cudaStreamIsCapturing(st, &cap) != cudaSuccess) cudaGetLastError();
+      if (it == c->dense_ways.end() && cap == cudaStreamCaptureStatusNone) {   // nothing can be timed in a capture
         cudaEvent_t e0, e1;
         CU(cudaEventCreate(&e0));
         CU(cudaEventCreate(&e1));
@@ -2774,10 +2776,11 @@ int nncv_b200_conv_run(nncv_b200_conv* c, const void* in, void* out, int N, int 
         int flag = 0;   // a kernel that gave up leaves early: nothing measured then counts
         if ((rc = read_kernel_status(&flag))) return rc;
         if (flag != 0) return report_kernel_error(flag, "conv_run");
+        if (c->dense_ways.size() >= 1024) c->dense_ways.clear();   // what it forgets is in the tuning cache
         it = c->dense_ways.emplace(key, ms[1] < ms[0]).first;
         g_tune_cache.put(ckey, it->second ? "1" : "0");
       }
-      dense = it->second;
+      dense = it != c->dense_ways.end() && it->second;
     }
     rc = dense ? direct() : shifted();
     return rc ? rc : ok();

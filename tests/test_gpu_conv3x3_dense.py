@@ -1,5 +1,9 @@
 """3x3 plans for the shifted-view kernel on dense tensors: the way that is chosen by timing (converted to shared-pad form, or
 straight from the dense tensor) changes no bit, and a result laid over an operand is still right."""
+import os
+import subprocess
+import sys
+
 import numpy as np
 import pytest
 
@@ -75,3 +79,43 @@ def test_the_trial_leaves_no_trace_in_the_profile():
         check(lib().nncv_b200_profile(0))
     conv.close()
     assert counts[0] == counts[1] == 1
+
+
+ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+
+
+def in_a_process_of_its_own(cache, function):
+    """Runs a function of this module where the tuning cache is read from `cache`."""
+    code = f"import sys; sys.path[:0] = [{ROOT!r}, {os.path.join(ROOT, 'tests')!r}]; import test_gpu_conv3x3_dense as t; t.{function}()"
+    r = subprocess.run([sys.executable, "-c", code], env=dict(os.environ, NNCV_B200_TUNE_CACHE=str(cache)), capture_output=True, text=True, timeout=600)
+    assert r.returncode == 0, r.stdout[-2000:] + r.stderr[-2000:]
+
+
+def capture_one_image_after_a_call_of_two():
+    x = torch.randn((2, 16, 16, 64), device="cuda", dtype=torch.float16)
+    wt = np.random.default_rng(3).standard_normal((64, 64, 3, 3)).astype(np.float32) / 24
+    conv, forced = G.Conv(wt, 1, 1, F16, algo=2), G.Conv(wt, 1, 1, F16, algo=2)
+    check(lib().nncv_b200_conv_set_tile(forced.h, 64, 1, 0))
+
+    def run(c, n, y):
+        check(lib().nncv_b200_conv_run(c.h, G.p(x), G.p(y), n, 16, 16, None, None, None, 0, G.stream_ptr()))
+        return y
+
+    run(conv, 2, torch.zeros_like(x))
+    want = run(forced, 1, torch.zeros_like(x[:1]))
+    got = torch.zeros_like(want)
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        run(conv, 1, got)
+    graph.replay()
+    torch.cuda.synchronize()
+    assert torch.equal(got, want)
+
+
+def test_capture_with_a_cache_that_knows_the_tiles_only(tmp_path):
+    """A tuning cache from before there were two ways names a shape's tile and no way: its call can be captured all the same."""
+    cache = tmp_path / "tuned"
+    key = "conv c64 k64 r3 s3 st1 p1 dt1 a2 n%d h16 w16 res0 o1 = 2 64 1 0\n"
+    cache.write_text(key % 1 + key % 2 + "conv3x3 way c64 k64 dt1 n2 h16 w16 res0 = 0\n")
+    in_a_process_of_its_own(cache, "capture_one_image_after_a_call_of_two")
