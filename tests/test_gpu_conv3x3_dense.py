@@ -14,7 +14,10 @@ from nncv_b200._lib import BF16, F16, check, lib  # noqa: E402
 import gpu_util as G  # noqa: E402
 
 
-@pytest.mark.parametrize("n,c,h,w,k", [(1, 64, 7, 7, 64), (3, 64, 56, 40, 64), (5, 128, 17, 23, 192), (2, 256, 14, 14, 256), (9, 64, 64, 64, 64)])
+CASES = [(1, 64, 7, 7, 64), (3, 64, 56, 40, 64), (5, 128, 17, 23, 192), (2, 256, 14, 14, 256), (9, 64, 64, 64, 64)]
+
+
+@pytest.mark.parametrize("n,c,h,w,k", CASES)
 @pytest.mark.parametrize("dtype", [F16, BF16])
 @pytest.mark.parametrize("res", [False, True])
 def test_ways_agree(n, c, h, w, k, dtype, res):
@@ -119,3 +122,23 @@ def test_capture_with_a_cache_that_knows_the_tiles_only(tmp_path):
     key = "conv c64 k64 r3 s3 st1 p1 dt1 a2 n%d h16 w16 res0 o1 = 2 64 1 0\n"
     cache.write_text(key % 1 + key % 2 + "conv3x3 way c64 k64 dt1 n2 h16 w16 res0 = 0\n")
     in_a_process_of_its_own(cache, "capture_one_image_after_a_call_of_two")
+
+
+def compare_with_a_forced_tile():
+    for n, c, h, w, k in CASES:
+        for dtype in (F16, BF16):
+            for res in (False, True):
+                test_ways_agree(n, c, h, w, k, dtype, res)
+
+
+@pytest.mark.parametrize("way", ["0", "1"])
+def test_either_way_gives_the_same_bits(tmp_path, way):
+    """test_ways_agree compares the way that happens to be faster; here either is named by the tuning cache."""
+    cache = tmp_path / "tuned"
+    lines = [f"conv3x3 way c{c} k{k} dt{dt} n{n} h{h} w{w} res{res} = {way}\n" for n, c, h, w, k in CASES for dt in (F16, BF16) for res in (0, 1)]
+    cache.write_text("".join(lines))
+    in_a_process_of_its_own(cache, "compare_with_a_forced_tile")
+    text = cache.read_text()
+    assert text.startswith("".join(lines)) and "conv3x3 way" not in text[len("".join(lines)):]   # nothing was tried
+    direct = text.count(" res4 ") + text.count(" res5 ")   # tiles tuned for the direct kernel on dense tensors
+    assert (direct > 0) == (way == "1")
