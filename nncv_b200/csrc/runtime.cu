@@ -1838,6 +1838,21 @@ void shard_range(int n, int rank, int world, int* lo, int* hi) {
   *hi = *lo + base + (rank < extra ? 1 : 0);
 }
 
+// Copies from and to the caller's memory on two streams: unless they have been waited for, leaving the scope -- by any way --
+// waits for them.
+struct CopiesInFlight {
+  Model& m;
+  cudaStream_t a, b;
+  bool waited = false;
+  ~CopiesInFlight() {
+    m.logits_off = 0;
+    if (waited) return;
+    cudaStreamSynchronize(a);
+    if (b != a) cudaStreamSynchronize(b);
+    cudaGetLastError();   // reported; the launches of the next call ask for the last error too
+  }
+};
+
 // A batch of images in host memory, in n_parts parts: every copy, every forward, one wait.
 int forward_host(Model& m, const char* sp, bool pinned, char* dp, bool dst_dev, size_t dst_stride, int N, int H, int W, cudaStream_t st,
                  int n_parts) {
@@ -1876,6 +1891,7 @@ int forward_host(Model& m, const char* sp, bool pinned, char* dp, bool dst_dev, 
     CU(cudaEventRecord(g_dev.copy_done[kMaxParts], st));
     CU(cudaStreamWaitEvent(cst, g_dev.copy_done[kMaxParts], 0));
   }
+  CopiesInFlight flight{m, cst, st};
   auto copy_in = [&](size_t part, int first, int n) -> int {
     char* to = (char*)m.in_stage.p + (size_t)first * img_bytes;
     const char* from = sp + (size_t)first * img_bytes;
@@ -1892,25 +1908,20 @@ int forward_host(Model& m, const char* sp, bool pinned, char* dp, bool dst_dev, 
   const char* logits = (const char*)(m.io_dt == kF32 ? m.logits32.p : m.logits_io.p);
   int first = 0;
   m.logits_off = 0;
-  rc = NNCV_B200_OK;
-  for (size_t c = 0; c < parts.size() && !rc; first += parts[c++]) {
+  for (size_t c = 0; c < parts.size(); first += parts[c++]) {
     const int n = parts[c];
-    if (!pinned && (rc = copy_in(c, first, n))) break;
+    if (!pinned && (rc = copy_in(c, first, n))) return rc;
     if (parts.size() > 1) CU(cudaStreamWaitEvent(st, g_dev.copy_done[c], 0));
-    if ((rc = model_forward_device(m, (char*)m.in_stage.p + (size_t)first * img_bytes, n, H, W, st))) break;
+    if ((rc = model_forward_device(m, (char*)m.in_stage.p + (size_t)first * img_bytes, n, H, W, st))) return rc;
     if (stage_out) CU(cudaMemcpyAsync((char*)m.result.p + 256 + row * first, logits + m.logits_off, row * n, cudaMemcpyDeviceToHost, st));
     else CU(cudaMemcpy2DAsync(dp + (size_t)first * dst_stride * ew, dst_stride * ew, logits + m.logits_off, row, row, (size_t)n,
                               dst_dev ? cudaMemcpyDeviceToDevice : cudaMemcpyDeviceToHost, st));
     m.logits_off += part_bytes(n);
   }
-  m.logits_off = 0;
-  if (rc) {
-    cudaStreamSynchronize(cst);   // the copies may still be reading the caller's memory
-    return rc;
-  }
   int* status = (int*)m.result.p;
   CU(cudaMemcpyAsync(status, g_dev.error_flag, sizeof(int), cudaMemcpyDeviceToHost, st));
   CU(cudaStreamSynchronize(st));
+  flight.waited = true;   // the copies in come before the forwards that read them
   if (*status != 0) {
     cudaMemset(g_dev.error_flag, 0, sizeof(int));
     return report_kernel_error(*status, "forward");
