@@ -1183,7 +1183,12 @@ struct Model {
   HostCopier copier;          // images from pageable memory
   PinnedBuf result;           // status word, then logits on their way to pageable memory
   size_t logits_off = 0;      // bytes: where the current part's logits go in logits_io / logits32
-  std::map<std::array<int, 4>, int> part_choice;   // parts a batch in host memory is cut into, by N, H, W, pinned
+  struct HostParts {           // parts a batch in host memory is cut into
+    int chosen = 0, calls = 0;   // 0: halves and quarters still in turn
+    double us[2] = {1e30, 1e30};
+    std::string key;             // in the tuning cache
+  };
+  std::map<std::array<int, 4>, HostParts> host_parts;   // by N, H, W, pinned
   static constexpr uintptr_t kFakeBase = (uintptr_t)0x7A00000000000000ull;   // planning pass: stand-in pointers
   void note_use(const void* p) {
     const uintptr_t v = (uintptr_t)p;
@@ -1853,27 +1858,19 @@ struct CopiesInFlight {
   }
 };
 
-// A batch of images in host memory, in n_parts parts: every copy, every forward, one wait.
+// A batch of images in host memory, in n_parts equal parts: every copy, every forward, one wait.
 int forward_host(Model& m, const char* sp, bool pinned, char* dp, bool dst_dev, size_t dst_stride, int N, int H, int W, cudaStream_t st,
                  int n_parts) {
   int rc;
   const size_t ew = m.ele_width, row = (size_t)m.plan.out_features * ew, img_bytes = (size_t)3 * H * W * ew;
-  std::vector<int> parts;
-  for (int r = 0; r < n_parts; ++r) {
-    int lo, hi;
-    shard_range(N, r, n_parts, &lo, &hi);
-    parts.push_back(hi - lo);
-  }
-  const int most = *std::max_element(parts.begin(), parts.end());
-  if ((rc = ensure_workspace(m, most, H, W))) return rc;
+  const int n = N / n_parts;
+  if ((rc = ensure_workspace(m, n, H, W))) return rc;
   if (m.in_stage.bytes < (size_t)N * img_bytes) {
     cudaDeviceSynchronize();
     if ((rc = m.in_stage.reserve((size_t)N * img_bytes))) return rc;
   }
   // logits of the parts one after another, each on a 256-byte boundary
-  auto part_bytes = [&](int n) { return ((size_t)n * m.plan.out_features * sizeof(float) + 255) & ~(size_t)255; };
-  size_t logits_bytes = 0;
-  for (int n : parts) logits_bytes += part_bytes(n);
+  const size_t part_bytes = ((size_t)n * m.plan.out_features * sizeof(float) + 255) & ~(size_t)255, logits_bytes = part_bytes * n_parts;
   if (m.logits_io.bytes < logits_bytes || m.logits32.bytes < logits_bytes) {
     cudaDeviceSynchronize();
     if ((rc = reserve_logits(m, logits_bytes))) return rc;
@@ -1881,7 +1878,7 @@ int forward_host(Model& m, const char* sp, bool pinned, char* dp, bool dst_dev, 
   const bool stage_out = !dst_dev && !is_pinned_ptr(dp) && row * N <= (4u << 20);   // small results leave through pinned memory
   if ((rc = m.result.reserve(256 + (stage_out ? row * N : 0)))) return rc;
   cudaStream_t cst = st;
-  if (parts.size() > 1) {
+  if (n_parts > 1) {
     if (!g_dev.copy_stream) {
       CU(cudaStreamCreateWithFlags(&g_dev.copy_stream, cudaStreamNonBlocking));
       for (auto& e : g_dev.copy_done) CU(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
@@ -1892,31 +1889,28 @@ int forward_host(Model& m, const char* sp, bool pinned, char* dp, bool dst_dev, 
     CU(cudaStreamWaitEvent(cst, g_dev.copy_done[kMaxParts], 0));
   }
   CopiesInFlight flight{m, cst, st};
-  auto copy_in = [&](size_t part, int first, int n) -> int {
-    char* to = (char*)m.in_stage.p + (size_t)first * img_bytes;
-    const char* from = sp + (size_t)first * img_bytes;
-    if (pinned || (size_t)n * img_bytes < HostCopier::kWorthIt) CU(cudaMemcpyAsync(to, from, (size_t)n * img_bytes, cudaMemcpyHostToDevice, cst));
-    else CU(m.copier.copy(to, from, (size_t)n * img_bytes, cst));
-    if (parts.size() > 1) CU(cudaEventRecord(g_dev.copy_done[part], cst));
+  const size_t in_bytes = (size_t)n * img_bytes;
+  auto copy_in = [&](int c) -> int {
+    char* to = (char*)m.in_stage.p + c * in_bytes;
+    const char* from = sp + c * in_bytes;
+    if (pinned || in_bytes < HostCopier::kWorthIt) CU(cudaMemcpyAsync(to, from, in_bytes, cudaMemcpyHostToDevice, cst));
+    else CU(m.copier.copy(to, from, in_bytes, cst));
+    if (n_parts > 1) CU(cudaEventRecord(g_dev.copy_done[c], cst));
     return NNCV_B200_OK;
   };
-  if (pinned) {   // nothing to wait for: all copies first
-    int first = 0;
-    for (size_t c = 0; c < parts.size(); first += parts[c++])
-      if ((rc = copy_in(c, first, parts[c]))) return rc;
-  }
+  if (pinned)   // nothing to wait for: all copies first
+    for (int c = 0; c < n_parts; ++c)
+      if ((rc = copy_in(c))) return rc;
   const char* logits = (const char*)(m.io_dt == kF32 ? m.logits32.p : m.logits_io.p);
-  int first = 0;
-  m.logits_off = 0;
-  for (size_t c = 0; c < parts.size(); first += parts[c++]) {
-    const int n = parts[c];
-    if (!pinned && (rc = copy_in(c, first, n))) return rc;
-    if (parts.size() > 1) CU(cudaStreamWaitEvent(st, g_dev.copy_done[c], 0));
-    if ((rc = model_forward_device(m, (char*)m.in_stage.p + (size_t)first * img_bytes, n, H, W, st))) return rc;
+  for (int c = 0; c < n_parts; ++c) {
+    const size_t first = (size_t)c * n;
+    if (!pinned && (rc = copy_in(c))) return rc;
+    if (n_parts > 1) CU(cudaStreamWaitEvent(st, g_dev.copy_done[c], 0));
+    m.logits_off = c * part_bytes;
+    if ((rc = model_forward_device(m, (char*)m.in_stage.p + c * in_bytes, n, H, W, st))) return rc;
     if (stage_out) CU(cudaMemcpyAsync((char*)m.result.p + 256 + row * first, logits + m.logits_off, row * n, cudaMemcpyDeviceToHost, st));
-    else CU(cudaMemcpy2DAsync(dp + (size_t)first * dst_stride * ew, dst_stride * ew, logits + m.logits_off, row, row, (size_t)n,
+    else CU(cudaMemcpy2DAsync(dp + first * dst_stride * ew, dst_stride * ew, logits + m.logits_off, row, row, (size_t)n,
                               dst_dev ? cudaMemcpyDeviceToDevice : cudaMemcpyDeviceToHost, st));
-    m.logits_off += part_bytes(n);
   }
   int* status = (int*)m.result.p;
   CU(cudaMemcpyAsync(status, g_dev.error_flag, sizeof(int), cudaMemcpyDeviceToHost, st));
@@ -1929,6 +1923,38 @@ int forward_host(Model& m, const char* sp, bool pinned, char* dp, bool dst_dev, 
   if (stage_out)
     for (int r = 0; r < N; ++r) memcpy(dp + (size_t)r * dst_stride * ew, (char*)m.result.p + 256 + row * r, row);
   return ok();
+}
+
+// How many parts a batch in host memory runs in, so that the copies of later parts overlap the forward of earlier ones (copies on
+// their own stream, ordered by events).  More parts leave less of the last one exposed but make smaller, less efficient
+// forwards.  fp32 convolutions split their sums by the batch, so there a batch keeps one way: halves from 128 images on.  In 16
+// bits a part's logits are the whole's, and the bytes that are copied decide.  From kHalves on halves are the better way (fp16, 224 x 224,
+// pinned, whole and halves in us: ResNet-18 64 images, 19 MB, 749 707, 128 1320 1121; ResNet-50 64 1495 1598, 128 2603 2593;
+// MobileNetV3 64 862 974, 128 1413 1357), and the activations take half the room.  From kQuarters on quarters may be better still: 256
+// images, 77 MB, in halves and quarters: ResNet-18 2017 1910, ResNet-50 4473 4809, MobileNetV3 2092 2362; fp32 images 3424 3207 and,
+// MobileNetV3, 3495 3320.  There the first eight calls of a shape go either way in turn, and the faster one stays (it is kept in the
+// tuning cache).  A call never runs its batch twice.
+constexpr size_t kHalves = 24u << 20, kQuarters = 64u << 20;
+Model::HostParts& host_parts(Model& m, int N, int H, int W, bool pinned) {
+  const std::array<int, 4> key{N, H, W, (int)pinned};
+  auto it = m.host_parts.find(key);
+  if (it != m.host_parts.end()) return it->second;
+  if (m.host_parts.size() >= 1024) m.host_parts.clear();   // what was measured is in the tuning cache
+  Model::HostParts h;
+  const size_t bytes = (size_t)N * 3 * H * W * m.ele_width;
+  if (m.act_dt == kF32) {
+    h.chosen = N >= 128 && N % 2 == 0 ? 2 : 1;
+  } else {
+    char text[192];
+    snprintf(text, sizeof(text), "host parts %.40s %zu dt%d e%zu n%d h%d w%d pinned%d", m.plan.name.c_str(), m.plan.total, (int)m.act_dt, m.ele_width, N, H, W, (int)pinned);
+    h.key = text;
+    const std::string* v = g_tune_cache.find(h.key);
+    const int said = v ? atoi(v->c_str()) : 0;
+    if ((said == 1 || said == 2 || said == 4) && N % said == 0) h.chosen = said;
+    else if (N % 2 || bytes < kHalves) h.chosen = 1;
+    else if (N % 4 || bytes < kQuarters || !g_autotune) h.chosen = 2;
+  }
+  return m.host_parts.emplace(key, std::move(h)).first->second;
 }
 
 // One device's share of a forward: images [sp, sp + N images) -> logits rows at dp (row pitch
@@ -1950,35 +1976,20 @@ int forward_slice(Model& m, const char* sp, bool src_dev, char* dp, bool dst_dev
     if ((rc = check_kernel_status())) return rc;
     return ok();
   }
-  // Images in host memory: a batch may run in parts, so that the copies of later parts overlap the forward of earlier ones
-  // (copies on their own stream, ordered by events).  More parts leave less of the last one exposed but make smaller, less
-  // efficient forwards -- which way wins depends on the network and the link, so the first call of a shape tries whole, halves
-  // and quarters (a run to let the layers tune themselves, two that count).  ResNet-18 fp16 256x224 from pinned memory (1.41 ms
-  // of copying): 2.20 ms in halves with blocking reads of logits and status, 2.03 ms now.  fp32 convolutions split their sums
-  // by the batch, so there a batch keeps one way.
   const bool pinned = is_pinned_ptr(sp);
-  int n_parts = N >= 128 && N % 2 == 0 ? 2 : 1;
-  if (m.act_dt != kF32 && N >= 16 && g_autotune) {
-    const std::array<int, 4> key{N, H, W, (int)pinned};
-    auto it = m.part_choice.find(key);
-    if (it == m.part_choice.end()) {
-      double best = 1e30;
-      for (int parts : {1, 2, 4}) {
-        if (N / parts < 8) break;
-        for (int rep = 0; rep < 3; ++rep) {
-          const auto t0 = std::chrono::steady_clock::now();
-          if ((rc = forward_host(m, sp, pinned, dp, dst_dev, dst_stride, N, H, W, st, parts))) return rc;
-          const double t = std::chrono::duration<double>(std::chrono::steady_clock::now() - t0).count();
-          if (rep > 0 && t < best) { best = t; n_parts = parts; }
-        }
-      }
-      m.part_choice.emplace(key, n_parts);
-      log_line(1, "host batch %d of %dx%d (%s): %d parts, %.0f us", N, H, W, pinned ? "pinned" : "pageable", n_parts, 1e6 * best);
-      return ok();   // the runs have left the logits, the same each time
-    }
-    n_parts = it->second;
+  Model::HostParts& h = host_parts(m, N, H, W, pinned);
+  // a call in the way that is settled, or in the next of the two that are still compared
+  const int way = h.calls & 1, n_parts = h.chosen ? h.chosen : 2 << way;
+  const auto t0 = std::chrono::steady_clock::now();
+  if ((rc = forward_host(m, sp, pinned, dp, dst_dev, dst_stride, N, H, W, st, n_parts)) || h.chosen) return rc;
+  if (h.calls++ >= 2)   // the first call of either way tuned its layers
+    h.us[way] = std::min(h.us[way], std::chrono::duration<double, std::micro>(std::chrono::steady_clock::now() - t0).count());
+  if (h.calls == 8) {
+    h.chosen = h.us[1] < 0.98 * h.us[0] ? 4 : 2;
+    g_tune_cache.put(h.key, h.chosen == 4 ? "4" : "2");
+    log_line(1, "%s: %d (%.0f us in halves, %.0f in quarters)", h.key.c_str(), h.chosen, h.us[0], h.us[1]);
   }
-  return forward_host(m, sp, pinned, dp, dst_dev, dst_stride, N, H, W, st, n_parts);
+  return rc;
 }
 
 int forward_fanout(const char* sp, char* dp, size_t dst_stride, int N, int H, int W);

@@ -1,7 +1,10 @@
-"""Batches in host memory: the way a batch is cut into parts, which the first calls of a shape vary, changes no logit; pinned
-and pageable images (small enough for one staged copy, and large enough for the pinned ring, with a ragged last piece); a
-smaller batch in the workspace of a larger one."""
+"""Batches in host memory: the number of parts a batch runs in -- one, two or four, by its bytes, the way of the largest settled
+by their first eight calls -- changes no logit; pinned and pageable images (small enough for one staged copy, and large enough
+for the pinned ring, with a ragged last piece); a smaller batch in the workspace of a larger one; a call that fails."""
 import ctypes
+import os
+import subprocess
+import sys
 
 import numpy as np
 import pytest
@@ -24,7 +27,7 @@ def test_parts_change_nothing(n, h, w, pinned):
     try:
         want = torch.zeros((n, 1000), device="cuda")
         rt.forward(want, x.cuda())
-        for call in range(20):   # more than the calls that try the ways
+        for call in range(20):
             got = torch.full((n, 1000), float("nan"), pin_memory=pinned)
             rt.forward(got, x)
             assert torch.equal(got, want.cpu()), call
@@ -32,6 +35,46 @@ def test_parts_change_nothing(n, h, w, pinned):
         assert torch.equal(got[:3], want[:3].cpu())
     finally:
         rt.unload()
+
+
+@pytest.mark.parametrize("n,pinned", [(96, True), (256, True), (256, False)])   # 29 MB: halves; 77 MB: halves and quarters in turn
+def test_the_calls_that_settle_the_way(n, pinned):
+    x = torch.from_numpy(random_input(n, 224, 224, 3, "normal").astype(np.float16))
+    x = x.pin_memory() if pinned else x
+    rt.load_blob("resnet18", to_flat_array(18, random_state_dict(18, 0), np.float16).blob(), F16)
+    try:
+        want = torch.zeros((n, 1000), device="cuda", dtype=torch.float16)
+        rt.forward(want, x.cuda())
+        for call in range(11):
+            got = torch.full((n, 1000), float("nan"), dtype=torch.float16, pin_memory=pinned)
+            rt.forward(got, x)
+            assert torch.equal(got, want.cpu()), call
+    finally:
+        rt.unload()
+
+
+ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+FORCED = [(16, 64, 64), (20, 64, 40), (68, 32, 64), (100, 224, 220)]   # the last: 59 MB of fp32 images, quarters of 15 MB
+
+
+def each_in_the_forced_way():
+    for n, h, w in FORCED:
+        for pinned in (False, True):
+            test_parts_change_nothing(n, h, w, pinned)
+
+
+@pytest.mark.parametrize("parts", [1, 2, 4])
+def test_every_way_gives_the_same_logits(tmp_path, parts):
+    """The way named by the tuning cache, in a process of its own."""
+    total = to_flat_array(18, random_state_dict(18, 0)).blob().size
+    cache = tmp_path / "tuned"
+    lines = "".join(f"host parts resnet18 {total} dt1 e4 n{n} h{h} w{w} pinned{p} = {parts}\n" for n, h, w in FORCED for p in (0, 1))
+    cache.write_text(lines)
+    code = f"import sys; sys.path[:0] = [{ROOT!r}, {os.path.join(ROOT, 'tests')!r}]; import test_gpu_host_batches as t; t.each_in_the_forced_way()"
+    r = subprocess.run([sys.executable, "-c", code], env=dict(os.environ, NNCV_B200_TUNE_CACHE=str(cache)), capture_output=True, text=True, timeout=600)
+    assert r.returncode == 0, r.stdout[-2000:] + r.stderr[-2000:]
+    text = cache.read_text()
+    assert all(f" n{n // parts} h{h // 4} " in text for n, h, w in FORCED[:1])   # layers tuned for the parts' batch
 
 
 def test_a_call_that_fails_has_no_copy_in_flight():
