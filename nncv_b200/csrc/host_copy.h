@@ -12,6 +12,7 @@
 #include <condition_variable>
 #include <cstring>
 #include <mutex>
+#include <system_error>
 #include <thread>
 
 namespace nncv_b200 {
@@ -118,7 +119,10 @@ class HostCopier {
         return e;
       }
     ring_ = r;
-    for (auto& t : helpers_) t = std::thread([this] { help(); });
+    try {
+      for (auto& t : helpers_) t = std::thread([this] { help(); });
+    } catch (const std::system_error&) {   // no more threads to be had: those there are, at least the caller's, do the copying
+    }
     return cudaSuccess;
   }
   void help() {
