@@ -703,11 +703,8 @@ bool conv_f32_supported(int C, int Kout, int tw_stride) { return C % 8 == 0 && K
 // cross GPC borders), so the runtime is asked.
 template <int BN>
 static int clusters_that_fit(int s, int sms) {
-  static int known[4] = {0, 0, 0, 0};   // per log2(s): the same on every device this library runs on
-  const int k = s == 1 ? 0 : (s == 2 ? 1 : (s == 4 ? 2 : 3));
-  if (s == 1) return sms;
-  if (known[k] == 0) known[k] = max_clusters(conv_f32_kernel<BN>, s, kThreads, Ring<BN>::kSmem, sms);
-  return known[k];
+  static const ClusterFit fit = cluster_fit(conv_f32_kernel<BN>, kThreads, Ring<BN>::kSmem, sms);
+  return fit.of[s];
 }
 
 static void pick_tile(long long m_tiles, int Kout, int kb_all, int sms, int* bn, int* splits) {

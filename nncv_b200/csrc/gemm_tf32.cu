@@ -417,11 +417,10 @@ cudaError_t launch_gemm_tf32x3(const float* A, const float* B, float* C, int M, 
   const int items = p.m_tiles * p.n_tiles;
   // Fewer tiles than SMs: clusters split the k blocks of a tile, as far as all of them run at once and each CTA keeps four
   // blocks (a block takes about 0.9 us, the exchange of partial sums 2).
-  static int fit[9] = {};
+  static const ClusterFit fit = cluster_fit(gemm_tf32x3_kernel, kThreads, smem, sms);
   p.splits = 1;
   for (int s = 2; s <= 8; s *= 2) {
-    if (fit[s] == 0) fit[s] = max_clusters(gemm_tf32x3_kernel, s, kThreads, smem, sms);
-    if (items > fit[s] || p.k_blocks < 4 * s) break;
+    if (items > fit.of[s] || p.k_blocks < 4 * s) break;
     p.splits = s;
   }
   if (p.splits == 1) return launch_pdl(gemm_tf32x3_kernel, dim3(items < sms ? items : sms), dim3(kThreads), smem, stream, tm_a, tm_c, p);

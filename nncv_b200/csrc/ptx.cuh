@@ -630,6 +630,17 @@ inline int max_clusters(Kern kern, int size, int threads, size_t smem, int sms) 
   return n < sms / size ? n : sms / size;
 }
 
+// The same for clusters of 1, 2, 4 and 8, by size.  A caller keeps it in a static const: the threads that serve several devices
+// may ask at the same time, and the answer is the same on every device this library runs on.
+struct ClusterFit { int of[9]; };
+template <typename Kern>
+inline ClusterFit cluster_fit(Kern kern, int threads, size_t smem, int sms) {
+  ClusterFit f = {};
+  f.of[1] = sms;
+  for (int s = 2; s <= 8; s *= 2) f.of[s] = max_clusters(kern, s, threads, smem, sms);
+  return f;
+}
+
 // Host side: launch with programmatic stream serialization allowed (see grid_dependency_wait).
 template <typename... KArgs, typename... Args>
 inline cudaError_t launch_pdl(void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream,

@@ -698,10 +698,9 @@ cudaError_t launch_cfg(const TconvArgs& a, TcParams p, cudaStream_t stream) {
     if (BROW) {
       // Fewer tiles than SMs: clusters split the depth of a tile, as far as all of them run at once and each CTA keeps
       // kSplitBlocks blocks of 64.
-      static int fit[9] = {};
+      static const ClusterFit fit = cluster_fit(kern, kThreads, kSmemLimit, sms);
       for (int s = 2; s <= 8; s *= 2) {
-        if (fit[s] == 0) fit[s] = max_clusters(kern, s, kThreads, kSmemLimit, sms);   // the same on every device this library runs on
-        if (items > fit[s] || p.CB < kSplitBlocks * s || st * stage < (size_t)BN * 512) break;
+        if (items > fit.of[s] || p.CB < kSplitBlocks * s || st * stage < (size_t)BN * 512) break;
         p.splits = s;
       }
       if (p.splits > 1) {

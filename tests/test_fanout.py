@@ -3,6 +3,8 @@ rule, the worker threads, the join, and the hand-over of a failing part's status
 made on the host: a stand-in job that returns an error).  The GPU part runs where two devices are
 visible."""
 import ctypes
+import os
+import re
 
 import numpy as np
 import pytest
@@ -15,6 +17,18 @@ def c_shard(n, r, w):
     lo, hi = ctypes.c_int(), ctypes.c_int()
     assert lib().nncv_b200_shard_range(n, r, w, ctypes.byref(lo), ctypes.byref(hi)) == 0
     return lo.value, hi.value
+
+
+def test_launch_code_keeps_nothing_that_threads_would_race_for():
+    """The workers of a fan-out launch kernels at the same time: what a launch function keeps between calls is const (set once,
+    by whichever thread comes first) or set under a once_flag."""
+    csrc = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "nncv_b200", "csrc")
+    for name in sorted(os.listdir(csrc)):
+        if not name.endswith((".cu", ".cuh", ".inc")) or name == "runtime.cu":   # there the entry points hold a lock
+            continue
+        text = open(os.path.join(csrc, name)).read()
+        kept = re.findall(r"^[ \t]+static (?!const |constexpr |std::once_flag )\w[\w:<>* ]* \w+(?:\[\d*\])? *(?:=|;|\{)[^\n]*", text, re.M)
+        assert all("call_once" in text and "get_encode" in text and "PFN_" in k for k in kept), (name, kept)
 
 
 @pytest.mark.parametrize("n,world", [(256, 8), (256, 3), (5, 8), (0, 2), (7, 7), (1000, 6)])
