@@ -46,6 +46,7 @@ struct PairParams {
   int in_stages, w_stages;
   int w_resident;            // all 3 * CB weight stages stay in shared memory (one Kout tile only)
   int w_box;                 // rows of a weight copy: a CTA's half of a tile, or of a column slice of the tail
+  int w_rows;                // rows of 128 bytes of the packed weights
   // Tail of the item list: the items of the last, partly filled round are split into tail_parts
   // column slices (BNP / tail_parts columns each) that run on different pairs at the same time.
   // Items [0, tail_start) are whole; tail_start is a multiple of the number of pairs.
@@ -156,6 +157,8 @@ conv3x3_pair_kernel(const __grid_constant__ CUtensorMap tm_in, const __grid_cons
 #pragma unroll
     for (int s3 = 0; s3 < kWGroup; ++s3) {
       const int first = ((wrow / kPackBN) * kb_total + (fr * 3 + s3) * p.CB + cb) * kPackBN + wrow % kPackBN;
+      // past the packed weights the copy engine reads zeros, without a word: the status word says it
+      if (first + rows > p.w_rows && issue && p.error_flag) atomicCAS(p.error_flag, 0, (int)kErrBounds);
       for (int r = 0; r < rows; r += p.w_box)
         ptx::tma_load_2d_pair(sW + ws * kWStage + s3 * kWTile + (uint32_t)r * 128u, &tm_w, 0, first + r, lead_w_full + 8 * ws, issue);
     }
