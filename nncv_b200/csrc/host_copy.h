@@ -47,8 +47,7 @@ class HostCopier {
     j.base = seq_;
     j.allowed.store(0);
     j.next.store(0);
-    const bool helped = bytes >= kHelpFrom;
-    if (helped) {
+    {
       std::lock_guard<std::mutex> lk(mu_);
       ++generation_;
       open_ = true;
@@ -80,7 +79,7 @@ class HostCopier {
     }
     seq_ = (j.base + j.pieces) % kSlots;
     j.next.store(j.pieces);                        // no helper starts another piece
-    if (helped) {
+    {
       std::unique_lock<std::mutex> lk(mu_);
       open_ = false;                               // a helper that wakes only now finds nothing to do and is not waited for
       idle_.wait(lk, [&] { return busy_ == 0; });
@@ -89,7 +88,7 @@ class HostCopier {
   }
 
  private:
-  static constexpr size_t kPiece = 512 << 10, kHelpFrom = 2 << 20;
+  static constexpr size_t kPiece = 512 << 10;
   static constexpr int kSlots = 16, kHelpers = 3;
   struct Job {
     const char* src = nullptr;

@@ -673,7 +673,7 @@ cudaError_t launch_cfg(const TconvArgs& a, TcParams p, cudaStream_t stream) {
     const long long items = (long long)((p.m_items + 1) / 2) * p.n_tiles;
     static const int fit = max_clusters(kern, 2, kThreads, kSmemLimit, sms);   // the same on every device this library runs on
     const long long pairs = fit;
-    if (BROW && BN == 256 && items > pairs) {
+    if (BROW && items > pairs) {
       const long long tail = items % pairs;   // halves only while both of every item fit in the one round
       if (tail > 0 && 2 * tail <= pairs) p.tail_start = (int)(items - tail);
     }
@@ -816,13 +816,9 @@ cudaError_t launch_tconv(const TconvArgs& args, cudaStream_t stream) {
   p.stages = 0;
   if (p.residual && p.out_f32) return cudaErrorInvalidValue;
   if (brow) {
-    if (a.pair) {   // CTA pairs: 256 x 256 (or 128) tiles
-      if (a.bn == 128) return launch_cfg<128, false, false, true, true>(a, p, stream);
-      return a.bn == 256 ? launch_cfg<256, false, false, true, true>(a, p, stream) : cudaErrorInvalidConfiguration;
-    }
-    if (a.bn == 64) return launch_cfg<64, false, false, false, true>(a, p, stream);
-    if (a.bn == 128) return launch_cfg<128, false, false, false, true>(a, p, stream);
-    if (a.bn == 256) return launch_cfg<256, false, false, false, true>(a, p, stream);
+    if (a.pair && a.bn == 256) return launch_cfg<256, false, false, true, true>(a, p, stream);   // CTA pairs: 256 x 256 tiles
+    if (!a.pair && a.bn == 64) return launch_cfg<64, false, false, false, true>(a, p, stream);
+    if (!a.pair && a.bn == 128) return launch_cfg<128, false, false, false, true>(a, p, stream);
     return cudaErrorInvalidConfiguration;
   }
   if (a.pair) {     // CTA pairs: a.wpack (and a.wpack2) packed for N tile bn / 2, streamed weights, 16-bit output
