@@ -271,22 +271,10 @@ def secondary_configs(torch, rt, flush, sampler, tf_peak):
             call = lambda: check(L.nncv_b200_conv_run(h, P(X), P(Y), n, hw, hw, P(sc), P(sh), None, 1, st))
             call()
             torch.cuda.synchronize()
-            # the entry point converts dense NHWC <-> the kernel's layout around the conv: time the conv
-            # launch itself through the per-launch records
             i0 = sampler.pos() if sampler else 0
-            rt.profile(True)
-            t_end = time.perf_counter() + 0.15
-            k = 0
-            while k < 7 or (time.perf_counter() < t_end and k < 2000):
-                flush.zero_()
-                call()
-                k += 1
-            torch.cuda.synchronize()
-            recs = [r for r in rt.profile_records() if r["kind"] in (2, 5, 7)]
-            rt.profile(False)
-            ms = statistics.median(r["ms"] for r in recs)
-            out["conv3x3_n32"].append(entry(ms, len(recs), recs[0]["flops"], i0, c=c, hw=hw, batch=n, kernel_kind=recs[0]["kind"],
-                                            note="fp16, fused scale/shift + ReLU; the conv launch alone"))
+            ms, reps = _timed_loop(torch, flush, call)
+            out["conv3x3_n32"].append(entry(ms, reps, 2.0 * 9 * c * c * n * hw * hw, i0, c=c, hw=hw, batch=n,
+                                            note="fp16, fused scale/shift + ReLU, dense NHWC in and out: the whole call"))
         finally:
             L.nncv_b200_conv_destroy(h)
     try:
@@ -499,7 +487,7 @@ def run_ours(args):
         c2 = sampler.pos() if sampler else 0
         ms_sus = sum(a.elapsed_time(b) for a, b in evs_s) if args.sustain > 0 else 0.0
         barrier()
-        for _ in range(max(args.warmup, 3)):
+        for _ in range(max(args.warmup, 9)):   # the first eight calls of a batch this large settle in how many parts it runs
             step_host()
         barrier()
         c3 = sampler.pos() if sampler else 0
