@@ -1858,12 +1858,14 @@ struct CopiesInFlight {
   }
 };
 
-// A batch of images in host memory, in n_parts equal parts: every copy, every forward, one wait.
+// A batch of images in host memory, in n_parts parts of equal size: every copy, every forward, one wait.  Where the batch is no
+// multiple, the last part takes images of the one before with it (layers are tuned for one batch size, and a 16-bit image's logits
+// do not depend on its part).
 int forward_host(Model& m, const char* sp, bool pinned, char* dp, bool dst_dev, size_t dst_stride, int N, int H, int W, cudaStream_t st,
                  int n_parts) {
   int rc;
   const size_t ew = m.ele_width, row = (size_t)m.plan.out_features * ew, img_bytes = (size_t)3 * H * W * ew;
-  const int n = N / n_parts;
+  const int n = (N + n_parts - 1) / n_parts;
   if ((rc = ensure_workspace(m, n, H, W))) return rc;
   if (m.in_stage.bytes < (size_t)N * img_bytes) {
     cudaDeviceSynchronize();
@@ -1889,10 +1891,10 @@ int forward_host(Model& m, const char* sp, bool pinned, char* dp, bool dst_dev, 
     CU(cudaStreamWaitEvent(cst, g_dev.copy_done[kMaxParts], 0));
   }
   CopiesInFlight flight{m, cst, st};
-  const size_t in_bytes = (size_t)n * img_bytes;
   auto copy_in = [&](int c) -> int {
-    char* to = (char*)m.in_stage.p + c * in_bytes;
-    const char* from = sp + c * in_bytes;
+    char* to = (char*)m.in_stage.p + (size_t)c * n * img_bytes;
+    const char* from = sp + (size_t)c * n * img_bytes;
+    const size_t in_bytes = (size_t)std::min(n, N - c * n) * img_bytes;
     if (pinned || in_bytes < HostCopier::kWorthIt) CU(cudaMemcpyAsync(to, from, in_bytes, cudaMemcpyHostToDevice, cst));
     else CU(m.copier.copy(to, from, in_bytes, cst));
     if (n_parts > 1) CU(cudaEventRecord(g_dev.copy_done[c], cst));
@@ -1903,11 +1905,11 @@ int forward_host(Model& m, const char* sp, bool pinned, char* dp, bool dst_dev, 
       if ((rc = copy_in(c))) return rc;
   const char* logits = (const char*)(m.io_dt == kF32 ? m.logits32.p : m.logits_io.p);
   for (int c = 0; c < n_parts; ++c) {
-    const size_t first = (size_t)c * n;
+    const size_t first = (size_t)std::min(c * n, N - n);
     if (!pinned && (rc = copy_in(c))) return rc;
     if (n_parts > 1) CU(cudaStreamWaitEvent(st, g_dev.copy_done[c], 0));
     m.logits_off = c * part_bytes;
-    if ((rc = model_forward_device(m, (char*)m.in_stage.p + c * in_bytes, n, H, W, st))) return rc;
+    if ((rc = model_forward_device(m, (char*)m.in_stage.p + first * img_bytes, n, H, W, st))) return rc;
     if (stage_out) CU(cudaMemcpyAsync((char*)m.result.p + 256 + row * first, logits + m.logits_off, row * n, cudaMemcpyDeviceToHost, st));
     else CU(cudaMemcpy2DAsync(dp + first * dst_stride * ew, dst_stride * ew, logits + m.logits_off, row, row, (size_t)n,
                               dst_dev ? cudaMemcpyDeviceToDevice : cudaMemcpyDeviceToHost, st));
@@ -1950,9 +1952,9 @@ Model::HostParts& host_parts(Model& m, int N, int H, int W, bool pinned) {
     h.key = text;
     const std::string* v = g_tune_cache.find(h.key);
     const int said = v ? atoi(v->c_str()) : 0;
-    if ((said == 1 || said == 2 || said == 4) && N % said == 0) h.chosen = said;
-    else if (N % 2 || bytes < kHalves) h.chosen = 1;
-    else if (N % 4 || bytes < kQuarters || !g_autotune) h.chosen = 2;
+    if ((said == 1 || said == 2 || said == 4) && N >= 4 * said) h.chosen = said;
+    else if (N < 16 || bytes < kHalves) h.chosen = 1;
+    else if (N < 32 || bytes < kQuarters || !g_autotune) h.chosen = 2;
   }
   return m.host_parts.emplace(key, std::move(h)).first->second;
 }

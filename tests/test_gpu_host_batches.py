@@ -37,7 +37,7 @@ def test_parts_change_nothing(n, h, w, pinned):
         rt.unload()
 
 
-@pytest.mark.parametrize("n,pinned", [(96, True), (256, True), (256, False)])   # 29 MB: halves; 77 MB: halves and quarters in turn
+@pytest.mark.parametrize("n,pinned", [(96, True), (97, True), (256, True), (257, False)])   # 29 MB: halves; 77 MB: halves and quarters in turn
 def test_the_calls_that_settle_the_way(n, pinned):
     x = torch.from_numpy(random_input(n, 224, 224, 3, "normal").astype(np.float16))
     x = x.pin_memory() if pinned else x
@@ -54,7 +54,7 @@ def test_the_calls_that_settle_the_way(n, pinned):
 
 
 ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
-FORCED = [(16, 64, 64), (20, 64, 40), (68, 32, 64), (100, 224, 220)]   # the last: 59 MB of fp32 images, quarters of 15 MB
+FORCED = [(16, 64, 64), (17, 64, 40), (67, 32, 64), (101, 224, 220)]   # the last: 60 MB of fp32 images, quarters of 15 MB
 
 
 def each_in_the_forced_way():
