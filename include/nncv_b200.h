@@ -74,7 +74,8 @@ enum {
 enum { NNCV_B200_F32 = 0, NNCV_B200_F16 = 1, NNCV_B200_BF16 = 2 };
 
 typedef struct {
-  int compute_dtype; /* NNCV_B200_F32 (fp32 accuracy: three bf16 planes per operand, tcgen05), _F16 or _BF16 (tcgen05 path);
+  int compute_dtype; /* NNCV_B200_F32 (fp32 accuracy: three bf16 planes per operand, tcgen05; activations take 6 bytes an
+                        element), _F16 or _BF16 (tcgen05 path);
                         -1 = follow the params file: eleWidth 4 -> F32, 2 -> F16 */
   unsigned device_mask; /* 0: the model lives on the current CUDA device only.  Otherwise bit d set =
                         a replica of the weights on device d (the current device must be among them):
@@ -242,7 +243,8 @@ int nncv_b200_matmul_noalloc(const void* A, const void* B, void* C, int M, int N
  * epilogue, on NHWC activations.  Weights are prepared once into a plan. */
 typedef struct nncv_b200_conv nncv_b200_conv;
 /* weights: host or device [Kout,C,R,S] of w_dtype.  dtype: activation type (F16/BF16 -> tcgen05
- * implicit GEMM, F32 -> CUDA-core).  algo: 0 = implicit GEMM, A operand fetched by strided TMA
+ * implicit GEMM; F32 -> the same on three bf16 planes per operand, with fp32 accuracy, or the CUDA cores where the channel counts
+ * or a short reduction do not suit it.  F32 values below 2^-110 are kept to an absolute 2^-134).  algo: 0 = implicit GEMM, A operand fetched by strided TMA
  * copies when C % 64 == 0 and by a cp.async gather otherwise (any shape), 3 = always the gather
  * kernel, 1 = Winograd F(2x2,3x3) in three stages (input transform, 16 tcgen05 GEMMs, output
  * transform; same shape limits as algo 2; the counterpart of nncv's disabled F(6x6,3x3) rewrite,
@@ -251,7 +253,11 @@ typedef struct nncv_b200_conv nncv_b200_conv;
 nncv_b200_conv* nncv_b200_conv_create(const void* weights, int w_dtype, int Kout, int C, int R,
                                       int S, int stride, int pad, int dtype, int algo);
 void nncv_b200_conv_destroy(nncv_b200_conv* c);
-/* in [N,H,W,Cpad], out/residual [N,OH,OW,Kout]; scale/shift fp32 [Kout] or NULL. */
+/* in [N,H,W,Cpad], out/residual [N,OH,OW,Kout], on 16-byte boundaries; scale/shift fp32 [Kout] or NULL.
+ * F32 on the tensor cores: a workspace of 6 bytes an input element for the length of the call, in the order of its stream (a
+ * captured call keeps its own until the plan is destroyed); such calls of one plan may run on several streams.  algo 1 and 2 keep
+ * copies of the tensors in the plan, F32 on the CUDA cores partial sums: order the calls of one plan there. The first call of a shape in 16 bits times kernels and tiles (NNCV_B200_AUTOTUNE=0: it does not) --
+ * with algo 2 also whether to convert the tensors' layout -- and cannot be captured. */
 int nncv_b200_conv_run(nncv_b200_conv* c, const void* in, void* out, int N, int H, int W,
                        const float* scale, const float* shift, const void* residual, int relu,
                        void* stream);

@@ -173,7 +173,8 @@ tconv_kernel(const __grid_constant__ CUtensorMap tm_in, const __grid_constant__ 
   const int per_worker = PAIR ? 2 : S;
   const int worker = (int)blockIdx.x / per_worker, workers = (int)gridDim.x / per_worker;
   // The last round of a matmul on pairs, when at most half of the pairs would have an item: every item is cut in two by
-  // columns and the halves run side by side (4096^3, 256 items on 74 pairs: 138 -> 128 us).
+  // columns and the halves run side by side (4096^3, 256 items on 74 pairs: 138 -> 128 us of kernel time when it
+  // was made; with whole-warp copies the kernel takes 102).
   const int full_rounds = PAIR && BROW && p.tail_start >= 0 ? p.tail_start / workers : 0x7fffffff;
   auto item_of = [&](int i, int& n0, int& oy0, int& ox0, int& n_tile) {
     int w = worker + i * workers;
@@ -884,8 +885,8 @@ bool matmul_direct(const void* A, const void* B, void* C, int M, int N, int K, D
   a.N = 1; a.H = 1; a.W = M; a.OH = 1; a.OW = M; a.C = K; a.Kout = N;
   a.in_l = Layout{1, M, 0}; a.out_l = Layout{1, M, 0};
   a.bn = matmul_pick(M, N, K, sms); a.resident = 0; a.ab = ab; a.out_dtype = c; a.relu = relu;
-  // 256 x 256 tiles on CTA pairs read each column of B from L2 half as often: 4096^3 fp16 148 -> 138 us, 8192x4096x512
-  // 38.8 -> 38.1, and 2048^3, with less than a round of pairs, no slower than 128 x 256 on single CTAs
+  // 256 x 256 tiles on CTA pairs read each column of B from L2 half as often: 4096^3 fp16 148 -> 138 us of kernel time when
+  // they were made, 8192x4096x512 38.8 -> 38.1, and 2048^3, with less than a round of pairs, no slower than 128 x 256 on single CTAs
   a.pair = a.bn == 256;
   a.sm_count = sms; a.error_flag = error_flag;
   return true;

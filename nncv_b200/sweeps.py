@@ -1,12 +1,13 @@
 """Kernel and network sweeps over the benchmark configs other than the headline one.
 
-    python -m nncv_b200.sweeps [gemm [SIZE]] [conv] [nets] [hbm] [mobilenet [BATCH]]
+    python -m nncv_b200.sweeps [gemm [SIZE]] [conv] [nets] [nets_f32 [BATCH]] [hbm] [mobilenet [BATCH]]
 
   gemm : M=N=K in {512,1024,2048,4096}, fp16 in / fp32 accumulate (fp16 and fp32 C), optional fused
-         bias + ReLU, and the fp32 CUDA-core path (config 1).
+         bias + ReLU, and fp32 (config 1).
   conv : 3x3 stride-1 pad-1, batch 32 (and 256 with "conv256"), (C=K, H=W) in {(64,64),(128,32),(256,16),(512,8)}, fp16, fused
          scale/shift + ReLU (config 2), for the shifted-view kernel and the TMA-fed per-tap kernel.
   nets : ResNet-18 fp32 N=1 @256 (config 0), ResNet-50 fp16 N=512 @224 (config 4), device-resident.
+  nets_f32 : ResNet-18 fp32 @224, batch 8 unless given, device-resident.
   hbm  : the memory-bound operators (depthwise conv + BN + hard-swish, activations, SE scaling, concat,
          2x upsampling, max-pool, global average pool) on MobileNetV3 / YOLOv5-sized maps: GB/s of
          algorithmic bytes (elements read + written) against the measured HBM copy bandwidth.
@@ -123,6 +124,17 @@ def nets():
         rt.unload()
 
 
+def nets_f32(batch=8):
+    """ResNet-18 in fp32 on a small batch, as nncv's example program runs it."""
+    from .split_params import random_state_dict, to_flat_array
+    s = torch.cuda.current_stream().cuda_stream
+    rt.load_blob("resnet18", to_flat_array(18, random_state_dict(18, 0), np.float32).blob(), F32)
+    x, o = torch.rand((batch, 3, 224, 224), device="cuda"), torch.empty((batch, 1000), device="cuda")
+    ms = _time(lambda: rt.forward_device(o, x, s))
+    print(json.dumps({"sweep": "nets_f32", "config": "R18 fp32 @224", "batch": batch, "ms": round(ms, 4)}), flush=True)
+    rt.unload()
+
+
 PEAK_GBS = 6540.5
 
 
@@ -204,6 +216,10 @@ if __name__ == "__main__":
         which = [a for a in which if a != "mobilenet" and not a.isdigit()]
         if not which:
             sys.exit(0)
+    if "nets_f32" in which:
+        nums = [int(a) for a in which if a.isdigit()]
+        nets_f32(nums[0] if nums else 8)
+        sys.exit(0)
     sizes = tuple(int(a) for a in which if a.isdigit())
     if "gemm" in which:
         gemm(sizes or (512, 1024, 2048, 4096))
