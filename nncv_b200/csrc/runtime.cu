@@ -1184,7 +1184,8 @@ struct Model {
   PinnedBuf result;           // status word, then logits on their way to pageable memory
   size_t logits_off = 0;      // bytes: where the current part's logits go in logits_io / logits32
   struct HostParts {           // parts a batch in host memory is cut into
-    int chosen = 0, calls = 0;   // 0: halves and quarters still in turn
+    int chosen = 0, calls = 0;   // 0: `first` and twice as many still in turn
+    int first = 2;
     double us[2] = {1e30, 1e30};
     std::string key;             // in the tuning cache
   };
@@ -1930,13 +1931,15 @@ int forward_host(Model& m, const char* sp, bool pinned, char* dp, bool dst_dev, 
 // How many parts a batch in host memory runs in, so that the copies of later parts overlap the forward of earlier ones (copies on
 // their own stream, ordered by events).  More parts leave less of the last one exposed but make smaller, less efficient
 // forwards.  fp32 convolutions split their sums by the batch, so there a batch keeps one way: halves from 128 images on.  In 16
-// bits a part's logits are the whole's, and the bytes that are copied decide.  From kHalves on halves are the better way (fp16, 224 x 224,
-// pinned, whole and halves in us: ResNet-18 64 images, 19 MB, 749 707, 128 1320 1121; ResNet-50 64 1495 1598, 128 2603 2593;
-// MobileNetV3 64 862 974, 128 1413 1357), and the activations take half the room.  From kQuarters on quarters may be better still: 256
-// images, 77 MB, in halves and quarters: ResNet-18 2017 1910, ResNet-50 4473 4809, MobileNetV3 2092 2362; fp32 images 3424 3207 and,
-// MobileNetV3, 3495 3320.  There the first eight calls of a shape go either way in turn, and the faster one stays (it is kept in the
-// tuning cache).  A call never runs its batch twice.
-constexpr size_t kHalves = 24u << 20, kQuarters = 64u << 20;
+// bits a part's logits are the whole's, and the bytes that are copied decide, as far as they can.  224 x 224, pinned, us:
+//   whole, halves   ResNet-18 fp16 48 images (14 MB) 628 631, 64 (19) 749 707, 128 (39) 1320 1121; fp32 images 32 (19) 749 654
+//                   ResNet-50 64 1495 1598, 96 (29) 2119 2143, 128 2603 2593; MobileNetV3 64 862 974, 96 1190 1157, 128 1413 1357
+//   halves, quarters of 256 images (77 MB)   ResNet-18 2017 1910, ResNet-50 4473 4809, MobileNetV3 2092 2362; fp32 images 3424 3207 and,
+//                   MobileNetV3, 3495 3320
+// So batches of less than kHalves run whole, from kSurely on in halves; between, and from kQuarters on, the next way may be the better one:
+// there the first eight calls of a shape go either way in turn, and the faster one stays (it is kept in the tuning cache).  A call never
+// runs its batch twice.
+constexpr size_t kHalves = 16u << 20, kSurely = 40u << 20, kQuarters = 64u << 20;
 Model::HostParts& host_parts(Model& m, int N, int H, int W, bool pinned) {
   const std::array<int, 4> key{N, H, W, (int)pinned};
   auto it = m.host_parts.find(key);
@@ -1954,7 +1957,9 @@ Model::HostParts& host_parts(Model& m, int N, int H, int W, bool pinned) {
     const int said = v ? atoi(v->c_str()) : 0;
     if ((said == 1 || said == 2 || said == 4) && N >= 4 * said) h.chosen = said;
     else if (N < 16 || bytes < kHalves) h.chosen = 1;
-    else if (N < 32 || bytes < kQuarters || !g_autotune) h.chosen = 2;
+    else if (bytes < kSurely) h.first = 1;
+    else if (N < 32 || bytes < kQuarters) h.chosen = 2;
+    if (!h.chosen && !g_autotune) h.chosen = bytes < (kHalves + kSurely) / 2 ? 1 : 2;
   }
   return m.host_parts.emplace(key, std::move(h)).first->second;
 }
@@ -1981,15 +1986,15 @@ int forward_slice(Model& m, const char* sp, bool src_dev, char* dp, bool dst_dev
   const bool pinned = is_pinned_ptr(sp);
   Model::HostParts& h = host_parts(m, N, H, W, pinned);
   // a call in the way that is settled, or in the next of the two that are still compared
-  const int way = h.calls & 1, n_parts = h.chosen ? h.chosen : 2 << way;
+  const int way = h.calls & 1, n_parts = h.chosen ? h.chosen : h.first << way;
   const auto t0 = std::chrono::steady_clock::now();
   if ((rc = forward_host(m, sp, pinned, dp, dst_dev, dst_stride, N, H, W, st, n_parts)) || h.chosen) return rc;
   if (h.calls++ >= 2)   // the first call of either way tuned its layers
     h.us[way] = std::min(h.us[way], std::chrono::duration<double, std::micro>(std::chrono::steady_clock::now() - t0).count());
   if (h.calls == 8) {
-    h.chosen = h.us[1] < 0.98 * h.us[0] ? 4 : 2;
-    g_tune_cache.put(h.key, h.chosen == 4 ? "4" : "2");
-    log_line(1, "%s: %d (%.0f us in halves, %.0f in quarters)", h.key.c_str(), h.chosen, h.us[0], h.us[1]);
+    h.chosen = h.us[1] < 0.98 * h.us[0] ? 2 * h.first : h.first;
+    g_tune_cache.put(h.key, std::to_string(h.chosen));
+    log_line(1, "%s: %d (%.0f us in %d parts, %.0f in %d)", h.key.c_str(), h.chosen, h.us[0], h.first, h.us[1], 2 * h.first);
   }
   return rc;
 }
