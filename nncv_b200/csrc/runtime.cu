@@ -1934,12 +1934,11 @@ int forward_host(Model& m, const char* sp, bool pinned, char* dp, bool dst_dev, 
 // bits a part's logits are the whole's, and the bytes that are copied decide, as far as they can.  224 x 224, pinned, us:
 //   whole, halves   ResNet-18 fp16 48 images (14 MB) 628 631, 64 (19) 749 707, 128 (39) 1320 1121; fp32 images 32 (19) 749 654
 //                   ResNet-50 64 1495 1598, 96 (29) 2119 2143, 128 2603 2593; MobileNetV3 64 862 974, 96 1190 1157, 128 1413 1357
-//   halves, quarters of 256 images (77 MB)   ResNet-18 2017 1910, ResNet-50 4473 4809, MobileNetV3 2092 2362; fp32 images 3424 3207 and,
+//   halves, quarters   ResNet-18 fp32 images 96 (58) 1420 1327; 256 images (77 MB) ResNet-18 2017 1910, ResNet-50 4473 4809, MobileNetV3 2092 2362; fp32 images 3424 3207 and,
 //                   MobileNetV3, 3495 3320
-// So batches of less than kHalves run whole, from kSurely on in halves; between, and from kQuarters on, the next way may be the better one:
-// there the first eight calls of a shape go either way in turn, and the faster one stays (it is kept in the tuning cache).  A call never
-// runs its batch twice.
-constexpr size_t kHalves = 16u << 20, kSurely = 40u << 20, kQuarters = 64u << 20;
+// So batches of less than kHalves run whole.  The first eight calls of a larger shape go whole and in halves, from kQuarters on in halves
+// and in quarters, in turn, and the faster way stays (it is kept in the tuning cache).  A call never runs its batch twice.
+constexpr size_t kHalves = 16u << 20, kQuarters = 40u << 20;
 Model::HostParts& host_parts(Model& m, int N, int H, int W, bool pinned) {
   const std::array<int, 4> key{N, H, W, (int)pinned};
   auto it = m.host_parts.find(key);
@@ -1957,9 +1956,8 @@ Model::HostParts& host_parts(Model& m, int N, int H, int W, bool pinned) {
     const int said = v ? atoi(v->c_str()) : 0;
     if ((said == 1 || said == 2 || said == 4) && N >= 4 * said) h.chosen = said;
     else if (N < 16 || bytes < kHalves) h.chosen = 1;
-    else if (bytes < kSurely) h.first = 1;
-    else if (N < 32 || bytes < kQuarters) h.chosen = 2;
-    if (!h.chosen && !g_autotune) h.chosen = bytes < (kHalves + kSurely) / 2 ? 1 : 2;
+    else if (!g_autotune) h.chosen = bytes < (kHalves + kQuarters) / 2 ? 1 : 2;
+    else h.first = N < 32 || bytes < kQuarters ? 1 : 2;
   }
   return m.host_parts.emplace(key, std::move(h)).first->second;
 }

@@ -37,7 +37,7 @@ def test_parts_change_nothing(n, h, w, pinned):
         rt.unload()
 
 
-@pytest.mark.parametrize("n,pinned", [(97, True), (97, False), (141, True), (256, True), (257, False)])   # 29 MB: whole and halves in turn; 42: halves; 77: and quarters
+@pytest.mark.parametrize("n,pinned", [(97, True), (97, False), (141, True), (257, False)])   # 29 MB: whole and halves in turn; 42 and 77: halves and quarters
 def test_the_calls_that_settle_the_way(n, pinned):
     x = torch.from_numpy(random_input(n, 224, 224, 3, "normal").astype(np.float16))
     x = x.pin_memory() if pinned else x
