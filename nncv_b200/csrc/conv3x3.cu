@@ -277,7 +277,6 @@ conv3x3_kernel(const __grid_constant__ CUtensorMap tm_in, const __grid_constant_
     // ------------------------------------------------------------------ epilogue --------
     // Eight independent warps (epilogue.cuh); slabs of an item: sub-tile major, then 64 columns.
     const int ew = warp - 2, quad = warp & 3, half = ew >> 2;
-    const uint32_t sw = (uint32_t)(lane & 7);
     const int nb = p.epi_bufs;
     const uint32_t my_stage = sStage + (uint32_t)(ew * nb) * epi::kBufBytes;
     const uint32_t my_res = res_full + (uint32_t)(ew * epi::kMaxBufs) * 8u;
@@ -335,7 +334,7 @@ conv3x3_kernel(const __grid_constant__ CUtensorMap tm_in, const __grid_constant_
         const bool live = q0 < p.T;
         const uint32_t taddr = tmem_base + ((uint32_t)(quad * 32) << 16) + ab * (MT * BN) + (uint32_t)(t * BN + sl * 64);
         uint32_t acc[64];
-        ptx::tmem_ld_32x64(taddr, acc);
+        epi::load_slab(taddr, acc);
         epi::put_cols(tab, cols, lane);
         if (p.has_res) {
           if (lane == 0) ptx::bulk_wait_read<0>();   // the buffer the next residual goes to was stored from one slab ago
@@ -356,7 +355,7 @@ conv3x3_kernel(const __grid_constant__ CUtensorMap tm_in, const __grid_constant_
         have = slab_of(j + 2, q0n, ncoln);
         cols = epi::fetch_cols(p.scale, p.shift, have ? ncoln : 0, p.Kout, lane);
         if (live) {
-          const uint32_t srow = my_stage + (uint32_t)b * epi::kBufBytes + (uint32_t)lane * 128u;
+          const uint32_t buf = my_stage + (uint32_t)b * epi::kBufBytes;
           if (p.has_res) {
             okw = ptx::mbar_wait_abortable(my_res + 8 * b, (phase >> b) & 1u, abort_flag);
             okw = __all_sync(0xffffffffu, okw);
@@ -364,12 +363,12 @@ conv3x3_kernel(const __grid_constant__ CUtensorMap tm_in, const __grid_constant_
             phase ^= 1u << b;
             inflight &= ~(1u << b);
           }
-          epi::row64_by_mode<1>(mode, acc, tab, srow, sw);
-          if (!keep) epi::zero_row(srow);
+          epi::slab64_by_mode<1>(mode, acc, tab, buf, lane);
+          epi::zero_pads(buf, lane, keep);
           ptx::fence_proxy_async_smem();
           __syncwarp();
           if (lane == 0) {
-            ptx::tma_store_2d(&tm_out, ncol, q0, my_stage + (uint32_t)b * epi::kBufBytes);
+            ptx::tma_store_2d(&tm_out, ncol, q0, buf);
             ptx::bulk_commit();
           }
         }

@@ -58,6 +58,11 @@ __device__ __forceinline__ uint4 lds128(uint32_t addr) {
   asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(addr));
   return v;
 }
+__device__ __forceinline__ float lds32(uint32_t addr) {
+  float v;
+  asm volatile("ld.shared.f32 %0, [%1];" : "=f"(v) : "r"(addr));
+  return v;
+}
 __device__ __forceinline__ void sts128(uint32_t addr, uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
   asm volatile("st.shared.v4.u32 [%0], {%1,%2,%3,%4};" ::"r"(addr), "r"(a), "r"(b), "r"(c), "r"(d) : "memory");
 }
@@ -97,18 +102,31 @@ __device__ __forceinline__ unsigned long long add2(unsigned long long a, unsigne
   return d;
 }
 
-// One row's 64 accumulator columns -> scale / shift (+ residual, read from the staging row) (+ activation) -> the 128-byte
-// staging row, 16-byte chunks XOR-swizzled by the row.  Sixteen columns at a time, the next sixteen's scale, shift and
-// residual on their way from shared memory meanwhile.
+// A warp's 32 x 64 accumulator slab -> scale / shift (+ residual, read from the staging buffer) (+ activation) -> the staging
+// buffer's rows of 128 bytes, 16-byte chunks XOR-swizzled by the row.
+//
+// The slab is held as matrix fragments (ptx::tmem_ld_16x64, rows 0-15 in acc[0..31], rows 16-31 after), so a thread owns the
+// same sixteen columns in all of its four rows and reads 8 x 16 bytes of scale and shift a slab; residual and result pass
+// through ldmatrix / stmatrix.  With a row a thread (32 lanes x 64 columns) every thread read all 32 x 16 bytes: at four clocks
+// a 16-byte read 2048 clocks of the shared-memory port for a 128 x 256 tile, beside which TMA and the tensor core, which use the
+// same port, waited.  ResNet-50 at batch 512, before and now, us: 64 -> 256 pointwise 219 185, with residual 301 285, 128 -> 512
+// 180 163, 256 -> 1024 116 103, 512 -> 2048 70 64, 64 -> 64 3x3 107 105.
+__device__ __forceinline__ void load_slab(uint32_t taddr, uint32_t (&acc)[64]) {
+  ptx::tmem_ld_16x64<0>(taddr, acc);
+  ptx::tmem_ld_16x64<32>(taddr + (16u << 16), acc);
+}
 template <bool BF16, bool RES, int ACT>
-__device__ __forceinline__ void row64(const uint32_t (&acc)[64], uint32_t tab, uint32_t srow, uint32_t sw) {
-  uint4 t[2][8], r[2][2];
-  auto load = [&](int c, int s) {
-#pragma unroll
-    for (int h = 0; h < 8; ++h) t[s][h] = lds128(tab + (uint32_t)(c * 8 + h) * 16u);
+__device__ __forceinline__ void slab64(const uint32_t (&acc)[64], uint32_t tab, uint32_t buf, int lane) {
+  const uint32_t row = buf + (uint32_t)(lane & 15) * 128u, hi = (uint32_t)(lane >> 4), sw = (uint32_t)(lane & 7);
+  const uint32_t t0 = tab + (uint32_t)(lane & 3) * 16u;
+  uint4 t[2][2];
+  uint32_t r[2][2][4];
+  auto load = [&](int c, int s) {   // column groups 2c and 2c + 1
+    t[s][0] = lds128(t0 + (uint32_t)(2 * c) * 64u);
+    t[s][1] = lds128(t0 + (uint32_t)(2 * c + 1) * 64u);
     if (RES) {
-      r[s][0] = lds128(srow + (((uint32_t)(2 * c) ^ sw) << 4));
-      r[s][1] = lds128(srow + (((uint32_t)(2 * c + 1) ^ sw) << 4));
+      ptx::ldmatrix4(row + ((((uint32_t)(2 * c)) | hi) ^ sw) * 16u, r[s][0]);
+      ptx::ldmatrix4(row + 16u * 128u + ((((uint32_t)(2 * c)) | hi) ^ sw) * 16u, r[s][1]);
     }
   };
   load(0, 0);
@@ -116,89 +134,98 @@ __device__ __forceinline__ void row64(const uint32_t (&acc)[64], uint32_t tab, u
   for (int c = 0; c < 4; ++c) {
     const int s = c & 1;
     if (c < 3) load(c + 1, s ^ 1);
-    uint32_t o[8];
 #pragma unroll
-    for (int h = 0; h < 8; ++h) {
-      const uint4 q = t[s][h];
-      unsigned long long v = fma2(pk(__uint_as_float(acc[c * 16 + 2 * h]), __uint_as_float(acc[c * 16 + 2 * h + 1])),
-                                  pk(__uint_as_float(q.x), __uint_as_float(q.y)), pk(__uint_as_float(q.z), __uint_as_float(q.w)));
-      if (RES) {
-        const uint4 w4 = r[s][h >> 2];
-        const uint32_t w = (h & 3) == 0 ? w4.x : ((h & 3) == 1 ? w4.y : ((h & 3) == 2 ? w4.z : w4.w));
-        const float2 f = unpack16(w, BF16);
-        v = add2(v, pk(f.x, f.y));
+    for (int h = 0; h < 2; ++h) {
+      uint32_t o[4];
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {   // group 2c: rows 0-7, rows 8-15; group 2c + 1 likewise
+        const uint4 q = t[s][e >> 1];
+        const int at = h * 32 + (2 * c + (e >> 1)) * 4 + (e & 1) * 2;
+        unsigned long long v = fma2(pk(__uint_as_float(acc[at]), __uint_as_float(acc[at + 1])), pk(__uint_as_float(q.x), __uint_as_float(q.y)),
+                                    pk(__uint_as_float(q.z), __uint_as_float(q.w)));
+        if (RES) {
+          const float2 f = unpack16(r[s][h][e], BF16);
+          v = add2(v, pk(f.x, f.y));
+        }
+        float a, b;
+        unpk(v, a, b);
+        // hard-swish x * min(max(x + 3, 0), 6) / 6 or SiLU x / (1 + exp(-x)); a NaN stays NaN through the product with x
+        if (ACT == 2) {
+          a *= __saturatef(fmaf(a, 0.16666667f, 0.5f));
+          b *= __saturatef(fmaf(b, 0.16666667f, 0.5f));
+        } else if (ACT == 3) {
+          a *= __fdividef(1.0f, __expf(-a) + 1.0f);
+          b *= __fdividef(1.0f, __expf(-b) + 1.0f);
+        }
+        o[e] = pack16(a, b, BF16, ACT == 1);
       }
-      float a, b;
-      unpk(v, a, b);
-      // hard-swish x * min(max(x + 3, 0), 6) / 6 or SiLU x / (1 + exp(-x)); a NaN stays NaN through the product with x
-      if (ACT == 2) {
-        a *= __saturatef(fmaf(a, 0.16666667f, 0.5f));
-        b *= __saturatef(fmaf(b, 0.16666667f, 0.5f));
-      } else if (ACT == 3) {
-        a *= __fdividef(1.0f, __expf(-a) + 1.0f);
-        b *= __fdividef(1.0f, __expf(-b) + 1.0f);
-      }
-      o[h] = pack16(a, b, BF16, ACT == 1);
+      ptx::stmatrix4(row + (uint32_t)h * 16u * 128u + ((((uint32_t)(2 * c)) | hi) ^ sw) * 16u, o[0], o[1], o[2], o[3]);
     }
-    sts128(srow + (((uint32_t)(2 * c) ^ sw) << 4), o[0], o[1], o[2], o[3]);
-    sts128(srow + (((uint32_t)(2 * c + 1) ^ sw) << 4), o[4], o[5], o[6], o[7]);
   }
 }
 
 // ACTS: the highest activation a kernel needs (1: none or ReLU, 3: all).
 template <int ACTS>
-__device__ __forceinline__ void row64_by_mode(int mode, const uint32_t (&acc)[64], uint32_t tab, uint32_t srow, uint32_t sw) {
-#define NNCV_ROW(B_, R_, A_) \
-  case (B_ ? kModeBf16 : 0) | (R_ ? kModeRes : 0) | (A_ << kModeActShift): row64<B_, R_, A_>(acc, tab, srow, sw); break;
+__device__ __forceinline__ void slab64_by_mode(int mode, const uint32_t (&acc)[64], uint32_t tab, uint32_t buf, int lane) {
+#define NNCV_SLAB(B_, R_, A_) \
+  case (B_ ? kModeBf16 : 0) | (R_ ? kModeRes : 0) | (A_ << kModeActShift): slab64<B_, R_, A_>(acc, tab, buf, lane); break;
   switch (mode) {
-    NNCV_ROW(false, false, 0) NNCV_ROW(false, false, 1) NNCV_ROW(false, true, 0) NNCV_ROW(false, true, 1)
-    NNCV_ROW(true, false, 0) NNCV_ROW(true, false, 1) NNCV_ROW(true, true, 0) NNCV_ROW(true, true, 1)
+    NNCV_SLAB(false, false, 0) NNCV_SLAB(false, false, 1) NNCV_SLAB(false, true, 0) NNCV_SLAB(false, true, 1)
+    NNCV_SLAB(true, false, 0) NNCV_SLAB(true, false, 1) NNCV_SLAB(true, true, 0) NNCV_SLAB(true, true, 1)
     default:
       if constexpr (ACTS > 1) {
         switch (mode) {
-          NNCV_ROW(false, false, 2) NNCV_ROW(false, true, 2) NNCV_ROW(true, false, 2) NNCV_ROW(true, true, 2)
-          NNCV_ROW(false, false, 3) NNCV_ROW(false, true, 3) NNCV_ROW(true, false, 3) NNCV_ROW(true, true, 3)
+          NNCV_SLAB(false, false, 2) NNCV_SLAB(false, true, 2) NNCV_SLAB(true, false, 2) NNCV_SLAB(true, true, 2)
+          NNCV_SLAB(false, false, 3) NNCV_SLAB(false, true, 3) NNCV_SLAB(true, false, 3) NNCV_SLAB(true, true, 3)
           default: break;
         }
       }
       break;
   }
-#undef NNCV_ROW
+#undef NNCV_SLAB
 }
 
-// fp32 results: 32 columns fill the 128-byte row.
+// fp32 results: 32 columns fill the 128-byte row.  Rows 0-15 of the slab in acc[0..15], rows 16-31 in acc[16..31].
+__device__ __forceinline__ void load_slab_f32(uint32_t taddr, uint32_t (&acc)[64]) {
+  ptx::tmem_ld_16x32<0>(taddr, acc);
+  ptx::tmem_ld_16x32<16>(taddr + (16u << 16), acc);
+}
 template <bool RELU>
-__device__ __forceinline__ void row32_f32(const uint32_t (&acc)[32], uint32_t tab, uint32_t srow, uint32_t sw) {
+__device__ __forceinline__ void slab32_f32(const uint32_t (&acc)[64], uint32_t tab, uint32_t buf, int lane) {
+  const uint32_t row = buf + (uint32_t)(lane & 15) * 128u, hi = (uint32_t)(lane >> 4), sw = (uint32_t)(lane & 7);
+  const uint32_t t0 = tab + (uint32_t)((lane >> 1) & 1) * 16u + (uint32_t)(lane & 1) * 4u;
+  float s[8], h[8];
 #pragma unroll
-  for (int c = 0; c < 2; ++c) {
-    uint4 t[8];
+  for (int g = 0; g < 8; ++g) {
+    s[g] = lds32(t0 + (uint32_t)g * 32u);
+    h[g] = lds32(t0 + (uint32_t)g * 32u + 8u);
+  }
 #pragma unroll
-    for (int h = 0; h < 8; ++h) t[h] = lds128(tab + (uint32_t)(c * 8 + h) * 16u);
+  for (int half = 0; half < 2; ++half)
 #pragma unroll
-    for (int g = 0; g < 4; ++g) {
+    for (int c = 0; c < 4; ++c) {   // column groups 2c and 2c + 1 of four
       float v[4];
 #pragma unroll
-      for (int h = 0; h < 2; ++h) {
-        const uint4 q = t[2 * g + h];
-        const int e = c * 16 + g * 4 + 2 * h;
-        unpk(fma2(pk(__uint_as_float(acc[e]), __uint_as_float(acc[e + 1])), pk(__uint_as_float(q.x), __uint_as_float(q.y)),
-                  pk(__uint_as_float(q.z), __uint_as_float(q.w))),
-             v[2 * h], v[2 * h + 1]);
+      for (int e = 0; e < 2; ++e) {
+        const int g = 2 * c + e, at = half * 16 + 2 * g;
+        unpk(fma2(pk(__uint_as_float(acc[at]), __uint_as_float(acc[at + 1])), pk(s[g], s[g]), pk(h[g], h[g])), v[2 * e], v[2 * e + 1]);
       }
       if (RELU) {
 #pragma unroll
-        for (int h = 0; h < 4; ++h) v[h] = !(v[h] <= 0.0f) ? v[h] : 0.0f;
+        for (int e = 0; e < 4; ++e) v[e] = !(v[e] <= 0.0f) ? v[e] : 0.0f;
       }
-      sts128(srow + (((uint32_t)(c * 4 + g) ^ sw) << 4), __float_as_uint(v[0]), __float_as_uint(v[1]), __float_as_uint(v[2]),
-             __float_as_uint(v[3]));
+      ptx::stmatrix4(row + (uint32_t)half * 16u * 128u + ((((uint32_t)(2 * c)) | hi) ^ sw) * 16u, __float_as_uint(v[0]), __float_as_uint(v[1]),
+                     __float_as_uint(v[2]), __float_as_uint(v[3]));
     }
-  }
 }
 
-// A row that is a pad slot leaves as zeros.
-__device__ __forceinline__ void zero_row(uint32_t srow) {
+// Rows that are pad slots (keep: lane l's row l is none) leave as zeros.
+__device__ __forceinline__ void zero_pads(uint32_t buf, int lane, bool keep) {
+  if (__all_sync(0xffffffffu, keep)) return;
+  __syncwarp();   // other lanes wrote the row
+  if (keep) return;
 #pragma unroll
-  for (uint32_t c = 0; c < 8; ++c) sts128(srow + (c << 4), 0u, 0u, 0u, 0u);
+  for (uint32_t c = 0; c < 8; ++c) sts128(buf + (uint32_t)lane * 128u + (c << 4), 0u, 0u, 0u, 0u);
 }
 
 // n / d for 0 <= n < 2^31 without a division.

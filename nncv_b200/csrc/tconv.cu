@@ -470,8 +470,8 @@ tconv_kernel(const __grid_constant__ CUtensorMap tm_in, const __grid_constant__ 
         const bool live = live_at(cur, ncol) && !(halved(i) && sl * slab_cols >= BN / 2);
         const uint32_t taddr = tmem_base + ((uint32_t)(quad * 32) << 16) + ab * ACC_W + (uint32_t)(oi * BN + sl * slab_cols);
         uint32_t acc[64];
-        if (p.out_f32) ptx::tmem_ld_32x32(taddr, reinterpret_cast<uint32_t (&)[32]>(acc));
-        else ptx::tmem_ld_32x64(taddr, acc);
+        if (p.out_f32) epi::load_slab_f32(taddr, acc);
+        else epi::load_slab(taddr, acc);
         epi::put_cols(tab, cols, lane);
         if (has_res) {
           // the buffer the next residual goes to was stored from one slab ago
@@ -489,7 +489,7 @@ tconv_kernel(const __grid_constant__ CUtensorMap tm_in, const __grid_constant__ 
         if (j + 2 >= end_j) hand_back();
         cols = cols_of((j + 2) >> spi_log, (j + 2) & (spi - 1), colpos);
         if (live) {
-          const uint32_t srow = my_stage + (uint32_t)b * epi::kBufBytes + (uint32_t)lane * 128u;
+          const uint32_t buf = my_stage + (uint32_t)b * epi::kBufBytes;
           if (has_res) {
             okw = ptx::mbar_wait_abortable(my_res + 8 * b, (phase >> b) & 1u, abort_flag);
             okw = __all_sync(0xffffffffu, okw);
@@ -498,16 +498,15 @@ tconv_kernel(const __grid_constant__ CUtensorMap tm_in, const __grid_constant__ 
             inflight &= ~(1u << b);
           }
           if (p.out_f32) {
-            if (p.relu) epi::row32_f32<true>(reinterpret_cast<const uint32_t (&)[32]>(acc), tab, srow, sw);
-            else epi::row32_f32<false>(reinterpret_cast<const uint32_t (&)[32]>(acc), tab, srow, sw);
+            if (p.relu) epi::slab32_f32<true>(acc, tab, buf, lane);
+            else epi::slab32_f32<false>(acc, tab, buf, lane);
           } else {
-            epi::row64_by_mode<DUAL ? 1 : 3>(oi ? mode2 : mode, acc, tab, srow, sw);
+            epi::slab64_by_mode<DUAL ? 1 : 3>(oi ? mode2 : mode, acc, tab, buf, lane);
           }
           ptx::fence_proxy_async_smem();
           __syncwarp();
           if (lane == 0) {
-            ptx::tma_store_4d((DUAL && oi) ? &tm_out2 : &tm_out, ncol, cur.ox0 + qx + p.out_off, cur.oy0 + qy + p.out_off, cur.n0 + qn,
-                              my_stage + (uint32_t)b * epi::kBufBytes);
+            ptx::tma_store_4d((DUAL && oi) ? &tm_out2 : &tm_out, ncol, cur.ox0 + qx + p.out_off, cur.oy0 + qy + p.out_off, cur.n0 + qn, buf);
             ptx::bulk_commit();
           }
         }
