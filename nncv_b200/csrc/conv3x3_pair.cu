@@ -191,7 +191,7 @@ conv3x3_pair_kernel(const __grid_constant__ CUtensorMap tm_in, const __grid_cons
         // [t * 128, +128) of both CTAs' tiles
         const int row0 = (m_item * 2 + (int)rank) * 128 * MT - p.P - 1;
         for (int cb = 0; cb < p.CB && okw; ++cb) {
-          if (!ptx::warp_wait_cluster(in_empty + 8 * st, ring, abort_flag)) { okw = false; break; }
+          if (!ptx::warp_wait(in_empty + 8 * st, ring, abort_flag)) { okw = false; break; }
           if (rank == 0) ptx::mbar_arrive_expect_tx(in_full + 8 * st, 2u * (uint32_t)in_stage_bytes, issue);
           for (int bx = 0; bx < p.n_boxes; ++bx)
             ptx::tma_load_2d_pair(sIn + st * in_stage_bytes + (uint32_t)(bx * p.box_rows) * 128u, &tm_in, cb * 64,
@@ -200,11 +200,11 @@ conv3x3_pair_kernel(const __grid_constant__ CUtensorMap tm_in, const __grid_cons
           if (p.w_resident && i > 0) continue;       // resident weights were loaded with the first item
           for (int fr = 0; fr < 3; ++fr, ++w_cnt) {   // one filter row (three taps) per weight stage
             if (w_cnt >= early) {
-              if (!ptx::warp_all(w_seen) && !ptx::warp_wait_cluster(w_empty + 8 * ws, w_ring, abort_flag)) { okw = false; break; }
+              if (!ptx::warp_all(w_seen) && !ptx::warp_wait(w_empty + 8 * ws, w_ring, abort_flag)) { okw = false; break; }
               load_weights(n_tile, sub, parts, cb, fr, ws, issue);
             }
             if (++ws == (uint32_t)p.w_stages) { ws = 0; w_ring ^= 1u; }
-            w_seen = ptx::mbar_peek_cluster(w_empty + 8 * ws, w_ring);
+            w_seen = ptx::mbar_peek(w_empty + 8 * ws, w_ring);
           }
         }
       }
@@ -218,30 +218,30 @@ conv3x3_pair_kernel(const __grid_constant__ CUtensorMap tm_in, const __grid_cons
       uint32_t in_st = 0, in_ring = 0, acc_cnt = 0;
       uint32_t w_st = 0, w_ring = 0;   // weight stage, parity of the ring's round (resident: each stage's first filling)
       bool okw = true;
-      uint32_t in_seen = ptx::mbar_peek_cluster(in_full, 0), w_seen = ptx::mbar_peek_cluster(w_full, 0);
+      uint32_t in_seen = ptx::mbar_peek(in_full, 0), w_seen = ptx::mbar_peek(w_full, 0);
       for (int i = 0; okw; ++i) {
         int m_item, n_tile, sub, parts;
         if (!item_of(i, m_item, n_tile, sub, parts)) break;
         const uint32_t idesc = parts == 1 ? idesc_full : ptx::umma_idesc(256, kBNPair / parts, p.bf16 ? 1 : 0);
         const uint32_t ab = acc_cnt % kAB;
-        if (!ptx::warp_wait_cluster(acc_empty + 8 * ab, ((acc_cnt / kAB) & 1u) ^ 1u, abort_flag)) { okw = false; break; }
+        if (!ptx::warp_wait(acc_empty + 8 * ab, ((acc_cnt / kAB) & 1u) ^ 1u, abort_flag)) { okw = false; break; }
         ptx::tc_fence_after();
         const uint32_t d = tmem_base + ab * (uint32_t)(kBNPair * MT);
         for (int cb = 0; cb < p.CB && okw; ++cb) {
           const uint32_t st = in_st;
-          if (!ptx::warp_all(in_seen) && !ptx::warp_wait_cluster(in_full + 8 * st, in_ring, abort_flag)) { okw = false; break; }
+          if (!ptx::warp_all(in_seen) && !ptx::warp_wait(in_full + 8 * st, in_ring, abort_flag)) { okw = false; break; }
           if (++in_st == (uint32_t)p.in_stages) { in_st = 0; in_ring ^= 1u; }
           ptx::tc_fence_after();
           const uint32_t a_stage = sIn + st * in_stage_bytes;
           for (int fr = 0; fr < 3; ++fr) {
             const uint32_t ws = w_st;   // resident: stage cb * 3 + fr, filled once
             if (!p.w_resident || i == 0) {
-              if (!ptx::warp_all(w_seen) && !ptx::warp_wait_cluster(w_full + 8 * ws, w_ring, abort_flag)) { okw = false; break; }
+              if (!ptx::warp_all(w_seen) && !ptx::warp_wait(w_full + 8 * ws, w_ring, abort_flag)) { okw = false; break; }
               ptx::tc_fence_after();
             }
             if (++w_st == (uint32_t)p.w_stages) { w_st = 0; w_ring ^= 1u; }
-            if (!p.w_resident || i == 0) w_seen = ptx::mbar_peek_cluster(w_full + 8 * w_st, w_ring);
-            if (fr == 2) in_seen = ptx::mbar_peek_cluster(in_full + 8 * in_st, in_ring);
+            if (!p.w_resident || i == 0) w_seen = ptx::mbar_peek(w_full + 8 * w_st, w_ring);
+            if (fr == 2) in_seen = ptx::mbar_peek(in_full + 8 * in_st, in_ring);
 #pragma unroll
             for (int t = 0; t < MT; ++t) {   // the stage's three weight tiles serve every sub-tile
 #pragma unroll

@@ -263,7 +263,6 @@ tconv_kernel(const __grid_constant__ CUtensorMap tm_in, const __grid_constant__ 
       __syncwarp();
       const uint32_t issue = ptx::elect_one();
       uint32_t cnt = 0, st = 0, ring = 1;   // stages begun; the next one and the parity of its round
-      auto peek = [&](uint32_t bar, uint32_t parity) { return PAIR ? ptx::mbar_peek_cluster(bar, parity) : ptx::mbar_peek(bar, parity); };
       uint32_t seen = 1;                    // nothing has used the ring yet
       bool okw = true;
       for (int i = 0; okw; ++i) {
@@ -279,8 +278,7 @@ tconv_kernel(const __grid_constant__ CUtensorMap tm_in, const __grid_constant__ 
             if (DUAL && tap == p.taps) { r = centre_r; s = centre_s; }   // the extra tap re-reads the centre tap's pixels
             const bool begun = cnt < early;   // this stage's first use: weights already issued
             if (!ptx::warp_all(seen)) {
-              const bool freed = PAIR ? ptx::warp_wait_cluster(empty + 8 * st, ring, abort_flag) : ptx::warp_wait(empty + 8 * st, ring, abort_flag);
-              if (!freed) { okw = false; break; }
+              if (!ptx::warp_wait(empty + 8 * st, ring, abort_flag)) { okw = false; break; }
             }
             if (!begun) expect_stage(st, issue, halved(i));
             const uint32_t dst = sRing + st * stage_bytes;
@@ -305,7 +303,7 @@ tconv_kernel(const __grid_constant__ CUtensorMap tm_in, const __grid_constant__ 
             const bool wrap = st + 1 == (uint32_t)p.stages;
             st = wrap ? 0u : st + 1;
             ring ^= wrap ? 1u : 0u;
-            seen = peek(empty + 8 * st, ring);
+            seen = ptx::mbar_peek(empty + 8 * st, ring);
           }
         }
       }
@@ -317,30 +315,26 @@ tconv_kernel(const __grid_constant__ CUtensorMap tm_in, const __grid_constant__ 
     {
       const uint32_t issue = ptx::elect_one();
       const uint32_t idesc = ptx::umma_idesc(PAIR ? 256 : 128, BN, p.bf16 ? 1 : 0) | (BROW ? (1u << 16) : 0u);   // bit 16: B is MN-major
-      auto wait = [&](uint32_t bar, uint32_t parity) {
-        return PAIR ? ptx::warp_wait_cluster(bar, parity, abort_flag) : ptx::warp_wait(bar, parity, abort_flag);
-      };
       bool okw = true;
       if (RESIDENT) okw = ptx::warp_wait(w_full, 0, abort_flag);
-      auto peek = [&](uint32_t bar, uint32_t parity) { return PAIR ? ptx::mbar_peek_cluster(bar, parity) : ptx::mbar_peek(bar, parity); };
       uint32_t st = 0, ring = 0, acc_cnt = 0;   // stage, parity of the ring's round
-      uint32_t seen = okw ? peek(full, 0) : 0u;
+      uint32_t seen = okw ? ptx::mbar_peek(full, 0) : 0u;
       for (int i = 0; okw; ++i) {
         int n0, oy0, ox0, n_tile;
         if (!item_of(i, n0, oy0, ox0, n_tile)) break;
         const uint32_t ab = acc_cnt & 1u;
-        if (!wait(acc_empty + 8 * ab, ((acc_cnt >> 1) & 1u) ^ 1u)) { okw = false; break; }
+        if (!ptx::warp_wait(acc_empty + 8 * ab, ((acc_cnt >> 1) & 1u) ^ 1u, abort_flag)) { okw = false; break; }
         ptx::tc_fence_after();
         const uint32_t d = tmem_base + ab * ACC_W;
         const uint32_t id = halved(i) ? idesc - ((uint32_t)(BN / 2 / 8) << 17) : idesc;   // N field
         for (int cb = cb_lo; cb < cb_hi && okw; ++cb)
           for (int tap = 0; tap < taps_x; ++tap) {   // producer order: cb outer, tap inner
             const bool second = DUAL && tap == p.taps;
-            if (!ptx::warp_all(seen) && !wait(full + 8 * st, ring)) { okw = false; break; }
+            if (!ptx::warp_all(seen) && !ptx::warp_wait(full + 8 * st, ring, abort_flag)) { okw = false; break; }
             ptx::tc_fence_after();
             const bool wrap = st + 1 == (uint32_t)p.stages;
             const uint32_t st_next = wrap ? 0u : st + 1, ring_next = ring ^ (wrap ? 1u : 0u);
-            seen = peek(full + 8 * st_next, ring_next);
+            seen = ptx::mbar_peek(full + 8 * st_next, ring_next);
             const uint32_t a_addr = sRing + st * stage_bytes;
             const uint32_t a_lo = ptx::smem_desc_k128_lo(a_addr);
             // MN-major B: leading-dimension offset 8192 bytes (next 64 columns), one k step of 16 = two 8-row groups
@@ -434,8 +428,7 @@ tconv_kernel(const __grid_constant__ CUtensorMap tm_in, const __grid_constant__ 
     for (int i = 0; okw; ++i) {
       if (!seek(cur, i)) break;
       const uint32_t ab = (uint32_t)i & 1u;
-      okw = PAIR ? ptx::mbar_wait_cluster_abortable(acc_full + 8 * ab, ((uint32_t)i >> 1) & 1u, abort_flag)
-                 : ptx::mbar_wait_abortable(acc_full + 8 * ab, ((uint32_t)i >> 1) & 1u, abort_flag);
+      okw = ptx::mbar_wait_abortable(acc_full + 8 * ab, ((uint32_t)i >> 1) & 1u, abort_flag);
       okw = __all_sync(0xffffffffu, okw);
       if (!okw) break;
       ptx::tc_fence_after();
@@ -458,7 +451,7 @@ tconv_kernel(const __grid_constant__ CUtensorMap tm_in, const __grid_constant__ 
         __syncwarp();
         if (lane == 0) {
           if (!PAIR || rank == 0) ptx::mbar_arrive(acc_empty + 8 * ab);
-          else ptx::mbar_arrive_remote(ptx::map_to_cta(acc_empty, 0) + 8 * ab);
+          else ptx::mbar_arrive_remote_relaxed(ptx::map_to_cta(acc_empty, 0) + 8 * ab);
         }
       };
       const int end_j = (i + 1) << spi_log;
