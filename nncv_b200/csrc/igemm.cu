@@ -400,7 +400,7 @@ int igemm_pick_bn(long long M, int Kout) {
 cudaError_t launch_pack_weights(const void* src, DType src_dt, long long sn, long long sc,
                                 long long stap, int Kout, int C, int Cpad, int taps, int bn,
                                 DType dst_dt, void* dst, cudaStream_t stream) {
-  if (Cpad % 8 != 0 || (bn != 64 && bn != 128 && bn != 256) || dst_dt == kF32)
+  if (Cpad % 8 != 0 || (bn != 32 && bn != 64 && bn != 128 && bn != 256) || dst_dt == kF32)
     return cudaErrorInvalidValue;
   switch (src_dt) {
     case kF32: return pack_dispatch<float>(src, sn, sc, stap, Kout, C, Cpad, taps, bn, dst_dt, dst, stream);

@@ -128,6 +128,14 @@ bool matmul_direct(const void* A, const void* B, void* C, int M, int N, int K, D
                    int* error_flag, TconvArgs* out);
 void tconv_pick(long long m_items, int C, int Kout, int taps, int* bn, int* resident);
 cudaError_t launch_tconv(const TconvArgs& a, cudaStream_t stream);
+void pointwise_as_matrix(TconvArgs* a);
+
+// The same convolutions on 64 x 32 tiles, for small batches (conv_small.cu): wpack (and wpack2) packed for N tile 32; bn, resident and
+// pair are not used.  Bit-identical to launch_tconv.
+constexpr int kSmallBN = 32;
+void conv_small_tile(int N, int OH, int OW, int* tw, int* th, int* tn);
+long long conv_small_tiles(int N, int OH, int OW, int Kout);
+cudaError_t launch_conv_small(const TconvArgs& a, cudaStream_t stream);
 
 // ---- Winograd F(2x2,3x3), three stages (filter transform once; input transform, 16 GEMMs, output
 // transform per call); dense NHWC, 16-bit types ----------------------------------------------------

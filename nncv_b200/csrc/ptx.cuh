@@ -298,6 +298,22 @@ __device__ __forceinline__ bool warp_wait(uint32_t bar, uint32_t parity, volatil
 }
 
 // Arrives on the mbarrier once every tcgen05.mma issued so far by this thread has finished.
+// The same by testing without a pause, for a warp on whose next step a whole chain waits and whose SM has little else to issue.
+__device__ __forceinline__ bool warp_spin(uint32_t bar, uint32_t parity, volatile int* abort_flag) {
+  long long t0 = 0;
+  for (uint32_t i = 0;; ++i) {
+    if (warp_all(mbar_peek(bar, parity) != 0)) return true;
+    if ((i & 255u) == 255u) {
+      const long long now = clock64();
+      if (t0 == 0) t0 = now;
+      if (warp_all(*abort_flag != 0)) return false;
+      if (warp_all(now - t0 > (1LL << 31))) {
+        *abort_flag = 1;
+        return false;
+      }
+    }
+  }
+}
 __device__ __forceinline__ void tc_commit(uint32_t bar, uint32_t issue) {
   asm volatile(
       "{\n"
@@ -380,6 +396,15 @@ __device__ __forceinline__ void tmem_ld_16x32(uint32_t taddr, uint32_t (&r)[64])
       "tcgen05.ld.sync.aligned.16x128b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
       : "=r"(r[OFF + 0]), "=r"(r[OFF + 1]), "=r"(r[OFF + 2]), "=r"(r[OFF + 3]), "=r"(r[OFF + 4]), "=r"(r[OFF + 5]), "=r"(r[OFF + 6]), "=r"(r[OFF + 7]),
         "=r"(r[OFF + 8]), "=r"(r[OFF + 9]), "=r"(r[OFF + 10]), "=r"(r[OFF + 11]), "=r"(r[OFF + 12]), "=r"(r[OFF + 13]), "=r"(r[OFF + 14]), "=r"(r[OFF + 15])
+      : "r"(taddr)
+      : "memory");
+}
+// 16 lanes x 32 columns as fragments like those of tmem_ld_16x64.
+__device__ __forceinline__ void tmem_ld_16x32_f(uint32_t taddr, uint32_t (&r)[16]) {
+  asm volatile(
+      "tcgen05.ld.sync.aligned.16x256b.x4.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
+      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]), "=r"(r[9]),
+        "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
       : "r"(taddr)
       : "memory");
 }

@@ -429,7 +429,7 @@ struct TuneCache {
 TuneCache g_tune_cache;
 
 struct ConvChoice {
-  int kernel = 5;  // 2 shifted-view conv3x3, 5 per-tap TMA kernel
+  int kernel = 5;  // 2 shifted-view conv3x3, 5 per-tap TMA kernel, 7 and 8 the same on CTA pairs, 9 per-tap on 64 x 32 tiles
   int bn = 64, mt = 1, resident = 0;
 };
 
@@ -670,7 +670,7 @@ int conv_run(nncv_b200_conv* c, const void* in, Layout in_l, void* out, Layout o
       a.pair = ch.kernel == 8;
       a.weights_ready = 1;
       if (fb) {
-        rc = conv_prepare(fb->conv, a.pair ? 64 : 128, st, &a.wpack2, true);
+        rc = conv_prepare(fb->conv, ch.kernel == 9 ? kSmallBN : a.pair ? 64 : 128, st, &a.wpack2, true);
         if (rc) return rc;
         a.scale2 = fb->scale; a.shift2 = fb->shift; a.out2 = fb->out;
       }
@@ -681,7 +681,7 @@ int conv_run(nncv_b200_conv* c, const void* in, Layout in_l, void* out, Layout o
       a.sm_count = g_dev.sm_count; a.error_flag = g_dev.error_flag;
       if (profile) prof_begin(5, flops, bytes, (int)M, c->Kout, c->C * c->R * c->S, ch.bn * 10 + ch.resident + (a.pair ? 2 : 0), st);
       ++g_launches;
-      const cudaError_t e = launch_tconv(a, st);
+      const cudaError_t e = ch.kernel == 9 ? launch_conv_small(a, st) : launch_tconv(a, st);
       if (profile) prof_end(st);
       return e == cudaSuccess ? 0 : -1;
     };
@@ -704,7 +704,9 @@ int conv_run(nncv_b200_conv* c, const void* in, Layout in_l, void* out, Layout o
       ch = ConvChoice{5, 128, 1, 0};
     }
     if (c->cfg3.bn) {
-      if (fb) {
+      if (c->cfg3.bn == kSmallBN && tc_ok) {
+        ch = ConvChoice{9, kSmallBN, 1, 0};
+      } else if (fb) {
         if (c->cfg3.resident >= 2) ch.kernel = 8;   // forced: the fused launch on CTA pairs
       } else {
         ch.bn = c->cfg3.bn; ch.mt = c->cfg3.mt > 0 ? c->cfg3.mt : 1; ch.resident = c->cfg3.resident;
@@ -721,8 +723,8 @@ int conv_run(nncv_b200_conv* c, const void* in, Layout in_l, void* out, Layout o
         if (const std::string* v = g_tune_cache.find(ckey)) {
           ConvChoice m;
           if (sscanf(v->c_str(), "%d %d %d %d", &m.kernel, &m.bn, &m.mt, &m.resident) == 4 &&
-              (((m.kernel == 5 || m.kernel == 8) && tc_ok) || ((m.kernel == 2 || m.kernel == 7) && sv_ok)) &&
-              (!fb || ((m.kernel == 5 || m.kernel == 8) && m.bn == 128 && !m.resident)))
+              (((m.kernel == 5 || m.kernel == 8 || (m.kernel == 9 && m.bn == kSmallBN)) && tc_ok) || ((m.kernel == 2 || m.kernel == 7) && sv_ok)) &&
+              (!fb || ((m.kernel == 5 || m.kernel == 8) && m.bn == 128 && !m.resident) || m.kernel == 9))
             it = c->tuned.emplace(key, m).first;
         }
       }
@@ -755,6 +757,8 @@ int conv_run(nncv_b200_conv* c, const void* in, Layout in_l, void* out, Layout o
             for (int bn : {128, 256})
               if (c->Kout % bn == 0) cand.push_back(ConvChoice{8, bn, 1, 0});   // CTA pairs
         }
+        // (with more than two tiles an SM the 128-row kernels were faster throughout)
+        if (tc_ok && conv_small_tiles(N, OH, OW, c->Kout) <= 2LL * g_dev.sm_count) cand.push_back(ConvChoice{9, kSmallBN, 1, 0});
         cudaEvent_t e0, e1;
         CU(cudaEventCreate(&e0));
         CU(cudaEventCreate(&e1));
@@ -781,6 +785,7 @@ int conv_run(nncv_b200_conv* c, const void* in, Layout in_l, void* out, Layout o
           // and would look fastest: read the status word and never choose, keep or persist such a one.
           int flag = 0;
           if (read_kernel_status(&flag) != NNCV_B200_OK || flag != 0) continue;
+          log_line(2, "  %s: kernel %d tile %d x%d mode %d %.1f us", ckey, k.kernel, k.bn, k.mt, k.resident, ms * 250.0f);
           if (ms < best) { best = ms; best_ch = k; }
         }
         cudaEventDestroy(e0);

@@ -753,10 +753,10 @@ void tconv_tile(int N, int OH, int OW, int* tw, int* th, int* tn) {
   (void)N;
 }
 
-cudaError_t launch_tconv(const TconvArgs& args, cudaStream_t stream) {
-  TconvArgs a = args;
-  // a pointwise convolution between dense tensors is a matrix of N * H * W rows (a fully connected layer's tile would hold
-  // sixteen of its one-pixel images)
+// A pointwise convolution between dense tensors is a matrix of N * H * W rows (a fully connected layer's tile would hold
+// sixteen of its one-pixel images).
+void pointwise_as_matrix(TconvArgs* t) {
+  TconvArgs& a = *t;
   if (a.R == 1 && a.S == 1 && a.stride == 1 && a.pad == 0 && !a.wpack2 && a.in_l.off == 0 && a.in_l.pitch == a.W && a.in_l.img_rows == a.H &&
       a.out_l.off == 0 && a.out_l.pitch == a.W && a.out_l.img_rows == a.H && (long long)a.N * a.H * a.W < (1LL << 30)) {
     const int rows = a.N * a.H * a.W;
@@ -765,6 +765,11 @@ cudaError_t launch_tconv(const TconvArgs& args, cudaStream_t stream) {
     a.W = a.OW = rows;
     a.in_l = a.out_l = Layout{1, rows, 0};
   }
+}
+
+cudaError_t launch_tconv(const TconvArgs& args, cudaStream_t stream) {
+  TconvArgs a = args;
+  pointwise_as_matrix(&a);
   const bool brow = a.b_rowmajor != nullptr;
   if (brow) {   // plain GEMM with a row-major B: K and N multiples of 8 (16-byte row pitches), nothing else
     if (a.ab == kF32 || a.C % 8 != 0 || a.Kout % 8 != 0 || a.R != 1 || a.S != 1 || a.stride != 1 || a.pad != 0 || a.wpack2 ||

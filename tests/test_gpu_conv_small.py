@@ -1,0 +1,66 @@
+"""The convolutions on 64 x 32 tiles (small batches) against the 128-row kernels, bit for bit, and against the oracle."""
+import numpy as np
+import pytest
+import torch
+
+from nncv_b200._lib import BF16, F16, check, lib
+from oracle import binding as ob
+from tests import gpu_util as G
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("case", [
+    # n, c, h, w, k, r, stride: one block, more blocks than stages, ragged channels and columns, tiles of several images, odd maps
+    (1, 8, 5, 7, 8, 1, 1), (1, 64, 8, 8, 32, 1, 1), (1, 512, 7, 7, 512, 3, 1), (3, 72, 7, 9, 40, 3, 1), (2, 24, 17, 19, 88, 3, 2),
+    (5, 128, 28, 28, 24, 1, 1), (1, 64, 56, 56, 64, 3, 1), (9, 64, 4, 4, 72, 1, 2), (1, 16, 3, 130, 48, 3, 1), (2, 256, 14, 14, 1000, 1, 1),
+])
+@pytest.mark.parametrize("dtype,res,relu", [(F16, False, False), (F16, True, True), (BF16, True, False), (BF16, False, True)])
+def test_small_tiles(case, dtype, res, relu):
+    n, c, h, w, k, r, stride = case
+    g = np.random.default_rng(n + c + h + w + k + r)
+    x = g.standard_normal((n, c, h, w)).astype(np.float32)
+    wt = (g.standard_normal((k, c, r, r)) * np.sqrt(2.0 / (r * r * c))).astype(np.float32)
+    scale, shift = g.uniform(0.5, 1.5, k).astype(np.float32), (g.standard_normal(k) * 0.1).astype(np.float32)
+    pad = r // 2
+    oh, ow = (h + 2 * pad - r) // stride + 1, (w + 2 * pad - r) // stride + 1
+    rs = g.standard_normal((n, k, oh, ow)).astype(np.float32) if res else None
+    conv = G.Conv(wt, stride, pad, dtype)
+    try:
+        check(lib().nncv_b200_conv_set_tile(conv.h, 32, 1, 0))
+        small, xq = conv.run(x, scale, shift, rs, relu)
+        check(lib().nncv_b200_conv_set_tile(conv.h, 64, 1, 0))
+        want, _ = conv.run(x, scale, shift, rs, relu)
+    finally:
+        conv.close()
+    assert np.array_equal(small, want)
+    q = lambda a: torch.from_numpy(a).to(G.TORCH_DT[dtype]).float().numpy()
+    ref = ob.conv2d(xq, q(wt), stride, pad, acc64=True) * scale[None, :, None, None] + shift[None, :, None, None]
+    ref = ref + q(rs) if res else ref
+    ref = np.where(ref > 0, ref, 0) if relu else ref
+    assert G.rel_l2(small, ref) <= (2e-3 if dtype == F16 else 8e-3)
+    assert lib().nncv_b200_device_status() == 0
+
+
+@pytest.mark.parametrize("n,c,h,w,k", [(1, 64, 56, 56, 128), (3, 256, 14, 14, 512), (1, 64, 9, 13, 128)])
+def test_small_tiles_with_branch(n, c, h, w, k):
+    g = np.random.default_rng(n + c + h)
+    x = g.standard_normal((n, c, h, w)).astype(np.float32)
+    w3 = (g.standard_normal((k, c, 3, 3)) * np.sqrt(2.0 / (9 * c))).astype(np.float32)
+    w1 = (g.standard_normal((k, c, 1, 1)) * np.sqrt(2.0 / c)).astype(np.float32)
+    cols = [G.dev(a.astype(np.float32)) for a in (g.uniform(0.5, 1.5, k), g.standard_normal(k), g.uniform(0.5, 1.5, k), g.standard_normal(k))]
+    X = G.dev(np.ascontiguousarray(x.transpose(0, 2, 3, 1)), F16)
+    oh, ow = (h - 1) // 2 + 1, (w - 1) // 2 + 1
+    main, branch = G.Conv(w3, 2, 1, F16), G.Conv(w1, 2, 0, F16)
+    got = []
+    try:
+        for bn in (32, 128):
+            check(lib().nncv_b200_conv_set_tile(main.h, bn, 1, 0))
+            Y = [torch.full((n, oh, ow, k), float("nan"), device="cuda", dtype=torch.float16) for _ in range(2)]
+            check(lib().nncv_b200_conv_run_fused(main.h, branch.h, G.p(X), G.p(Y[0]), G.p(Y[1]), n, h, w, *map(G.p, cols), 1, G.stream_ptr()))
+            G.sync_check()
+            got.append(Y)
+    finally:
+        main.close()
+        branch.close()
+    assert torch.equal(got[0][0], got[1][0]) and torch.equal(got[0][1], got[1][1]) and not got[0][0].isnan().any()
