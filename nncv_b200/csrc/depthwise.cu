@@ -8,9 +8,11 @@
 // tiles of 8 output rows x TW output columns x CB channels and one thread issues, two tiles ahead,
 // ONE tensor copy per tile: the input patch with its halo, out-of-range pixels filled with zeros by
 // the copy engine (no bounds checks on the input side at all).  The 256 threads then read the
-// patch from shared memory: thread = (four channels, output column), computing a column strip of eight output rows in fp32
-// pairs (fma.rn.f32x2), so that each input value is loaded once per filter column and reused down the strip, and each
-// filter value serves eight outputs.  With eight channels a thread and strips of four rows the 5x5 layers were bound by
+// patch from shared memory: thread = (four channels, one or two output columns), computing a column strip of output rows in fp32
+// pairs (fma.rn.f32x2), so that each input value is loaded once per input column and reused down the strip, and each
+// filter value serves the strip.  What bounds the 16-bit kernels is the pipe of the packed multiply-adds, on which the conversions
+// to fp32 run too (64x112x112x96 hard-swish: 64 % of its rate with one column a thread, 15 conversions beside 18 multiply-adds
+// for an output of four channels; two columns share four of six input columns: 10).  With eight channels a thread and strips of four rows the 5x5 layers were bound by
 // shared memory: a filter vector of eight fp32 is two loads at a stride of 32 bytes, two-way bank conflicts, and those loads
 // were two thirds of the traffic (14x14x240 at batch 256: 9.8 M wavefronts, 48 us); now a lane's four filter values are 16
 // contiguous bytes and are read half as often.  Filter, scale and shift sit in shared memory: for the 16-bit types as the
@@ -24,6 +26,8 @@
 #include <cuda_runtime.h>
 #include <cudaTypedefs.h>
 
+#include <algorithm>
+#include <cmath>
 #include <mutex>
 
 #include "epilogue.cuh"
@@ -34,11 +38,11 @@ namespace nncv_b200 {
 
 namespace {
 
-constexpr int kThreads = 256;
-constexpr int kTH = 8;           // output rows per tile
-// output rows per thread: the tile's eight, or four in fp32, whose rows are twice as long (with strips of eight a tile
-// needs 38 KB a stage and only two CTAs fit an SM)
-template <typename T> constexpr int kRows = sizeof(T) == 4 ? 4 : 8;
+// What a thread computes: KP output rows x PX adjacent output columns of four channels.
+// Threads at most, and CTAs of that size an SM (by registers)
+template <typename T> constexpr int kMaxThreads = sizeof(T) == 4 ? 256 : 128;
+template <typename T, int KS, int PX> constexpr int kCtas = sizeof(T) == 4 ? (KS == 3 ? 3 : 2) : PX == 2 ? (KS == 3 ? 4 : 3) : (KS == 3 ? 6 : 4);
+template <typename T, int KP> constexpr int kTH = sizeof(T) == 4 ? 8 : KP;   // output rows of a tile
 template <typename T> constexpr bool kFold = sizeof(T) == 2;   // the scale multiplied into the filter
 constexpr int kMaxStages = 3;
 
@@ -50,7 +54,7 @@ struct DwParams {
   void* y;             // [N,OH,OW,C]
   int N, H, W, C, OH, OW, pad, act;
   Layout in_l, out_l;  // input coordinates and output pixels are shifted by the layouts' pad offsets
-  int tw, cbv;         // output columns per tile, 16-byte channel vectors per chunk (tw * cbv <= 128)
+  int tw, cbv;         // output columns per tile, 16-byte channel vectors per chunk
   int tiles_x, tiles_y, n_tiles;   // spatial tiles (n_tiles = N * tiles_y * tiles_x)
   epi::FastDiv div_tx, div_ty;
   int stages;
@@ -114,15 +118,15 @@ __device__ __forceinline__ float act1(float x, int act) {
   }
 }
 
-template <typename T, int KS, int STRIDE>
-__global__ void __launch_bounds__(kThreads, KS == 3 ? 3 : 2) depthwise_tma_kernel(const __grid_constant__ CUtensorMap tm_in, const DwParams p) {
+template <typename T, int KS, int STRIDE, int PX, int kP>
+__global__ void __launch_bounds__(kMaxThreads<T>, kCtas<T, KS, PX>) depthwise_tma_kernel(const __grid_constant__ CUtensorMap tm_in, const DwParams p) {
   ptx::grid_dependency_wait();
   ptx::grid_launch_dependents();
   constexpr int V = 4;                                  // channels of a thread
-  constexpr int kP = kRows<T>;                          // output rows of a thread
+  constexpr int TH = kTH<T, kP>;
   constexpr int kPer = 16 / (V * sizeof(T));            // threads of a 16-byte vector
   using Raw = typename Vec<T>::type;
-  constexpr int NR = (kP - 1) * STRIDE + KS;            // input rows under one strip of kP outputs
+  constexpr int NR = (kP - 1) * STRIDE + KS, NC = (PX - 1) * STRIDE + KS;   // input rows and columns under a thread's outputs
   extern __shared__ __align__(128) unsigned char smem[];
   __shared__ __align__(8) unsigned long long full_bar[kMaxStages];
   __shared__ int abort_flag;
@@ -143,22 +147,6 @@ __global__ void __launch_bounds__(kThreads, KS == 3 ? 3 : 2) depthwise_tma_kerne
     ptx::mbar_fence_init();
     ptx::prefetch_tensormap(&tm_in);
   }
-  for (int i = tid; i < KS * KS * CB; i += kThreads) {
-    const int tap = i / CB, c = i - tap * CB;
-    float v = 0.0f;
-    if (c0 + c < p.C) {
-      const size_t idx = (size_t)(c0 + c) * (KS * KS) + tap;
-      v = p.w_half ? __half2float(reinterpret_cast<const __half*>(p.w)[idx]) : reinterpret_cast<const float*>(p.w)[idx];
-      if (kFold<T> && p.scale) v *= p.scale[c0 + c];
-    }
-    sw[i] = v;
-  }
-  for (int c = tid; c < CB; c += kThreads) {
-    ssh[c] = (c0 + c < p.C && p.shift) ? p.shift[c0 + c] : 0.0f;
-    if (!kFold<T>) ssc[c] = (c0 + c < p.C && p.scale) ? p.scale[c0 + c] : 1.0f;
-  }
-  __syncthreads();
-
   const int my_tiles = ((int)blockIdx.x < p.n_tiles) ? (p.n_tiles - 1 - (int)blockIdx.x) / (int)gridDim.x + 1 : 0;
   auto issue = [&](int k) {      // thread 0: the copy of this CTA's k-th tile into stage k % stages
     const int sp = blockIdx.x + k * gridDim.x;
@@ -166,17 +154,34 @@ __global__ void __launch_bounds__(kThreads, KS == 3 ? 3 : 2) depthwise_tma_kerne
     const int n = (int)epi::div_by((uint32_t)t2, p.div_ty), ty = t2 - n * p.tiles_y;
     const int s = k % p.stages;
     const uint32_t bar = ptx::smem_u32(&full_bar[s]);
-    tile_info[s] = make_int4(n, ty * kTH, tx * tw, 0);   // read by the others after they have seen the barrier complete
+    tile_info[s] = make_int4(n, ty * TH, tx * tw, 0);   // read by the others after they have seen the barrier complete
     ptx::mbar_arrive_expect_tx(bar, p.stage_bytes);
     ptx::tma_load_4d(ptx::smem_u32(smem + (size_t)s * p.stage_stride), &tm_in, c0, tx * tw * STRIDE - p.pad + p.in_l.off,
-                     ty * kTH * STRIDE - p.pad + p.in_l.off, n, bar);
+                     ty * TH * STRIDE - p.pad + p.in_l.off, n, bar);
   };
   int issued = 0;
   if (tid == 0)
     for (; issued < p.stages - 1 && issued < my_tiles; ++issued) issue(issued);
 
-  const int xs = tid / (kPer * cbv), cvec = tid - xs * (kPer * cbv);
-  const int ys = kP == kTH ? 0 : xs / tw, x = xs - ys * tw;   // strip of rows, column
+  // filter, scale and shift: all loads of a channel in flight together, behind the first copies
+  for (int c = tid; c < CB; c += (int)blockDim.x) {
+    const bool in = c0 + c < p.C;
+    float v[KS * KS];
+#pragma unroll
+    for (int tap = 0; tap < KS * KS; ++tap) {
+      const size_t idx = (size_t)(c0 + c) * (KS * KS) + tap;
+      v[tap] = !in ? 0.0f : p.w_half ? __half2float(reinterpret_cast<const __half*>(p.w)[idx]) : reinterpret_cast<const float*>(p.w)[idx];
+    }
+    const float scale = in && p.scale ? p.scale[c0 + c] : 1.0f;
+    ssh[c] = in && p.shift ? p.shift[c0 + c] : 0.0f;
+    if (!kFold<T>) ssc[c] = scale;
+#pragma unroll
+    for (int tap = 0; tap < KS * KS; ++tap) sw[tap * CB + c] = kFold<T> ? v[tap] * scale : v[tap];
+  }
+  __syncthreads();
+
+  const int xs = tid / (kPer * cbv), cvec = tid - xs * (kPer * cbv), pairs = tw / PX;
+  const int ys = TH == kP ? 0 : xs / pairs, x = (xs - ys * pairs) * PX;   // strip of rows, first column
   int k = 0;
   for (; k < my_tiles; ++k) {
     const int s = k % p.stages;
@@ -185,57 +190,69 @@ __global__ void __launch_bounds__(kThreads, KS == 3 ? 3 : 2) depthwise_tma_kerne
     if (__syncthreads_or(!ok)) break;
     if (tid == 0 && issued < my_tiles) { issue(issued); ++issued; }
 
-    if (kP == kTH ? x >= tw : ys >= kTH / kP) continue;  // no strip of the tile is this thread's
+    if (xs >= pairs * (TH / kP)) continue;   // no strip of the tile is this thread's
     const unsigned char* st = smem + (size_t)s * p.stage_stride;
     // folded: the sums start at the shift, the filter carries the scale
-    u64 acc[kP][2];
+    u64 acc[PX][kP][2];
     {
       const ulonglong2 sh = kFold<T> ? *reinterpret_cast<const ulonglong2*>(ssh + cvec * V) : make_ulonglong2(0, 0);
 #pragma unroll
-      for (int o = 0; o < kP; ++o) { acc[o][0] = sh.x; acc[o][1] = sh.y; }
+      for (int px = 0; px < PX; ++px)
+#pragma unroll
+        for (int o = 0; o < kP; ++o) { acc[px][o][0] = sh.x; acc[px][o][1] = sh.y; }
     }
+    ulonglong2 wr[KS][KS];   // filter column kx in wr[kx], live while an output column needs it
 #pragma unroll
-    for (int kx = 0; kx < KS; ++kx) {
-      ulonglong2 wr[KS];
+    for (int ix = 0; ix < NC; ++ix) {
+      if (ix < KS) {
 #pragma unroll
-      for (int q = 0; q < KS; ++q) wr[q] = *reinterpret_cast<const ulonglong2*>(sw + (q * KS + kx) * CB + cvec * V);
-      const unsigned char* col = st + (size_t)(ys * kP * STRIDE * IW + x * STRIDE + kx) * cbv * 16 + cvec * sizeof(Raw);
+        for (int q = 0; q < KS; ++q) wr[ix][q] = *reinterpret_cast<const ulonglong2*>(sw + (q * KS + ix) * CB + cvec * V);
+      }
+      const unsigned char* col = st + (size_t)(ys * kP * STRIDE * IW + x * STRIDE + ix) * cbv * 16 + cvec * sizeof(Raw);
 #pragma unroll
       for (int ry = 0; ry < NR; ++ry) {
         u64 f[2];
         unpack(*reinterpret_cast<const Raw*>(col + (size_t)ry * IW * cbv * 16), f, T{});
 #pragma unroll
-        for (int o = 0; o < kP; ++o) {
-          const int q = ry - o * STRIDE;               // compile-time after unrolling
-          if (q >= 0 && q < KS) {
-            acc[o][0] = epi::fma2(f[0], wr[q].x, acc[o][0]);
-            acc[o][1] = epi::fma2(f[1], wr[q].y, acc[o][1]);
+        for (int px = 0; px < PX; ++px) {
+          const int kx = ix - px * STRIDE;
+          if (kx < 0 || kx >= KS) continue;
+#pragma unroll
+          for (int o = 0; o < kP; ++o) {
+            const int q = ry - o * STRIDE;               // compile-time after unrolling
+            if (q >= 0 && q < KS) {
+              acc[px][o][0] = epi::fma2(f[0], wr[kx][q].x, acc[px][o][0]);
+              acc[px][o][1] = epi::fma2(f[1], wr[kx][q].y, acc[px][o][1]);
+            }
           }
         }
       }
     }
     // epilogue: activation, store
     const int4 ti = tile_info[s];
-    const int ox = ti.z + x, c = c0 + cvec * V;
-    if (ox < p.OW && c < p.C) {
+    const int c = c0 + cvec * V, rows = min(kP, p.OH - ti.y - ys * kP);
+    if (c >= p.C) continue;
+#pragma unroll
+    for (int px = 0; px < PX; ++px) {
+      const int ox = ti.z + x + px;
+      if (ox >= p.OW) break;
       if (!kFold<T>) {
         const ulonglong2 sc = *reinterpret_cast<const ulonglong2*>(ssc + cvec * V), sh = *reinterpret_cast<const ulonglong2*>(ssh + cvec * V);
 #pragma unroll
         for (int o = 0; o < kP; ++o) {
-          acc[o][0] = epi::fma2(acc[o][0], sc.x, sh.x);
-          acc[o][1] = epi::fma2(acc[o][1], sc.y, sh.y);
+          acc[px][o][0] = epi::fma2(acc[px][o][0], sc.x, sh.x);
+          acc[px][o][1] = epi::fma2(acc[px][o][1], sc.y, sh.y);
         }
       }
       T* yp = reinterpret_cast<T*>(p.y) + (((size_t)ti.x * p.out_l.img_rows + ti.y + ys * kP + p.out_l.off) * p.out_l.pitch + ox + p.out_l.off) * p.C + c;
       const size_t row_step = (size_t)p.out_l.pitch * p.C;
-      const int rows = min(kP, p.OH - ti.y - ys * kP);
       auto finish = [&](auto f4) {
 #pragma unroll
         for (int o = 0; o < kP; ++o) {
           if (o >= rows) break;
           float v[4];
-          f4(acc[o][0], v[0], v[1]);
-          f4(acc[o][1], v[2], v[3]);
+          f4(acc[px][o][0], v[0], v[1]);
+          f4(acc[px][o][1], v[2], v[3]);
           *reinterpret_cast<Raw*>(yp + o * row_step) = pack(v, T{});
         }
       };
@@ -278,23 +295,111 @@ PFN_cuTensorMapEncodeTiled_v12000 dw_get_encode() {
   return fn;
 }
 
-template <typename T, int KS, int STRIDE>
-cudaError_t launch_one(const CUtensorMap& tm, const DwParams& p, dim3 grid, size_t smem, cudaStream_t st) {
-  auto kern = depthwise_tma_kernel<T, KS, STRIDE>;
+template <typename T, int KS, int STRIDE, int PX, int KP>
+cudaError_t launch_one(const CUtensorMap& tm, const DwParams& p, dim3 grid, int threads, size_t smem, cudaStream_t st) {
+  auto kern = depthwise_tma_kernel<T, KS, STRIDE, PX, KP>;
   if (smem > 48 * 1024) {
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
   }
-  launch_pdl(kern, grid, dim3(kThreads), smem, st, tm, p);
+  launch_pdl(kern, grid, dim3((unsigned)threads), smem, st, tm, p);
   return cudaGetLastError();
 }
 
+template <typename T, int PX, int KP>
+cudaError_t launch_typed(const CUtensorMap& tm, const DwParams& p, int ks, int stride, dim3 grid, int threads, size_t smem, cudaStream_t st) {
+  if (ks == 3 && stride == 1) return launch_one<T, 3, 1, PX, KP>(tm, p, grid, threads, smem, st);
+  if (ks == 3 && stride == 2) return launch_one<T, 3, 2, PX, KP>(tm, p, grid, threads, smem, st);
+  if (ks == 5 && stride == 1) return launch_one<T, 5, 1, PX, KP>(tm, p, grid, threads, smem, st);
+  return launch_one<T, 5, 2, PX, KP>(tm, p, grid, threads, smem, st);
+}
 template <typename T>
-cudaError_t launch_typed(const CUtensorMap& tm, const DwParams& p, int ks, int stride, dim3 grid, size_t smem, cudaStream_t st) {
-  if (ks == 3 && stride == 1) return launch_one<T, 3, 1>(tm, p, grid, smem, st);
-  if (ks == 3 && stride == 2) return launch_one<T, 3, 2>(tm, p, grid, smem, st);
-  if (ks == 5 && stride == 1) return launch_one<T, 5, 1>(tm, p, grid, smem, st);
-  return launch_one<T, 5, 2>(tm, p, grid, smem, st);
+cudaError_t launch_shape(int px, const CUtensorMap& tm, const DwParams& p, int ks, int stride, dim3 grid, int threads, size_t smem, cudaStream_t st) {
+  if (px == 1) return launch_typed<T, 1, 8>(tm, p, ks, stride, grid, threads, smem, st);
+  if (ks == 3) return stride == 1 ? launch_one<T, 3, 1, 2, 8>(tm, p, grid, threads, smem, st) : launch_one<T, 3, 2, 2, 4>(tm, p, grid, threads, smem, st);
+  return stride == 1 ? launch_one<T, 5, 1, 2, 8>(tm, p, grid, threads, smem, st) : launch_one<T, 5, 2, 2, 4>(tm, p, grid, threads, smem, st);
+}
+
+// Tile, outputs of a thread and block of a layer: what dw_shape chooses.
+struct DwShape { int cbv, tw, px, kp, threads, stages, per_sm; size_t smem; };
+
+// 16-bit types: two columns x eight rows a thread at stride 1 (two x four at stride 2, where a patch has twice the rows) read and
+// convert each input value for two columns at once; one column x eight rows leaves none of an odd, narrow map's threads idle, needs
+// fewer registers and, with few channels, meets fewer bank conflicts.  fp32, whose rows are twice as long and need no conversion:
+// four rows of one column.  A tile is any split of columns and whole 16-byte channel vectors that a block's threads cover, and the
+// block has as many threads as it needs.  For 16 bits the least modelled cost counts, in instructions of a thread per output:
+// multiply-adds, conversions and (twice, with their bank conflicts) shared-memory reads, times the outputs, idle ones included, that
+// the busiest SM computes; halo columns, rows of a patch shorter than 256 (and more so 128) bytes, few warps and few blocks an SM,
+// which leave the wait for a tile bare, count against it.
+// Batch 256 fp16, us, one column x eight rows, two x eight (stride 2: two x four): 240 channels 5x5 on 14x14 37.6 34.3, 576 on 7x7
+// 24.3 28.7, 88 3x3 on 28x28 27.2 25.3, 16 3x3 stride 2 112 -> 56 32.6 43.6, 72 3x3 stride 2 56 -> 28 41.9 29.9; 64x112x112x96 89.1
+// 74.4.  (Since then the filter is fetched behind the first copies, all of a channel's values in flight, 2 to 3 us less each: the last
+// one takes 71.2, where 256 threads of one column x eight rows took 84.3.)
+DwShape dw_choose(int N, int C, int OH, int OW, int R, int stride, int es, int sms) {
+  const int V = 16 / es, cv = C / V;
+  const size_t wvec = (size_t)(R * R + (es == 2 ? 1 : 2)) * V * sizeof(float);   // filter and shift (scale) of a channel vector
+  DwShape best{};
+  double least = 1e30;
+  for (int px = es == 2 ? 2 : 1; px >= 1; --px) {
+    const int kp = es == 4 || (px == 2 && stride == 2) ? 4 : 8, th = es == 4 ? 8 : kp, ih = (th - 1) * stride + R;
+    const int most = es == 4 ? kMaxThreads<float> : kMaxThreads<__half>, slots = most * px / 2;   // 16-byte vectors of a tile
+    const int by_regs = es == 4 ? most * (R == 3 ? 3 : 2) : px == 2 ? most * (R == 3 ? 4 : 3) : most * (R == 3 ? 6 : 4);
+    const double loads = (double)((kp - 1) * stride + R) * ((px - 1) * stride + R) / (kp * px);
+    for (int v = std::min(32, cv); v >= 2; --v) {        // ties go to the wider chunk (longer contiguous runs in memory)
+      const int widest = slots / v / px * px, fewest = (OW + widest - 1) / widest, chunks = (cv + v - 1) / v, bytes = v * 16;
+      // the 128 bytes that half a warp reads are `groups` pixels, px * stride pixels apart
+      const int groups = bytes >= 128 ? 1 : 128 / bytes, step = px * stride * bytes % 128;
+      const int apart = step == 0 ? 1 : 128 / (step & -step), ways = groups > apart ? groups / apart : 1;
+      const double per_output = 2.0 * R * R + (es == 2 ? 4.0 : 0.0) * loads + 2.0 * ways * loads + 8.0;
+      for (int tiles = fewest; tiles <= fewest + (es == 2 ? 2 : 0); ++tiles) {
+        const int t = ((OW + tiles - 1) / tiles + px - 1) / px * px, iw = (t - 1) * stride + R;
+        if (iw > 256) continue;
+        const size_t stage = ((size_t)iw * ih * bytes + 127) & ~(size_t)127;
+        if (2 * stage + v * wvec > 200 * 1024) continue;
+        const int threads = (t * v * 2 / px + 31) & ~31, regs_fit = std::min(by_regs / threads, 16);
+        const auto fit = [&](int stages) { return std::min(regs_fit, (int)((220 * 1024) / (stages * stage + v * wvec + 1024))); };
+        const int per_sm = fit(2);
+        if (per_sm < 1) continue;
+        double cost;
+        if (es == 4) {
+          // the share of idle threads and outputs; stages so large that fewer than three blocks fit an SM
+          double use = (double)cv / (chunks * v) * OW / (((OW + t - 1) / t) * t) * (t * v) / slots;
+          use *= 0.5 + 0.5 * (t * stride) / iw;
+          if (v < 8) use *= 0.5 + 0.5 * v / 8.0;
+          const size_t need = 2 * stage + v * wvec;
+          if (need > 72 * 1024) use *= need > 110 * 1024 ? 0.6 : 0.9;
+          cost = 1.0 / use;
+        } else {
+          // blocks' worth of work that the busiest SM does one after another
+          const double turns = std::ceil((double)N * ((OH + th - 1) / th) * ((OW + t - 1) / t) * chunks / sms);
+          const double beside = std::min((double)per_sm, turns);
+          cost = per_output * kp * px * threads * turns * (1.0 + 3.3 * 32.0 / (beside * threads)) * (1.0 + 0.15 / beside);
+          cost /= 0.5 + 0.5 * (t * stride) / iw;
+          if (v < 16) cost /= 0.94 + 0.06 * v / 16.0;
+          if (v < 8) cost /= 0.5 + 0.5 * v / 8.0;
+        }
+        if (cost < least * (1.0 - 1e-9)) {
+          least = cost;
+          // a third stage where it costs no block of an SM (fp32, of a large patch, 56x56x72 at stride 2: 83 us with it, 79 without)
+          const int stages = fit(3) == per_sm && (es == 2 || per_sm > 1) ? 3 : 2;
+          best = DwShape{v, t, px, kp, threads, stages, per_sm, stages * stage + v * wvec};
+        }
+      }
+    }
+  }
+  return best;
+}
+// The same, kept for the layers a thread asks for in turn: choosing takes longer than a launch.
+const DwShape& dw_shape(int N, int C, int OH, int OW, int R, int stride, int es, int sms) {
+  struct Kept { int key[8]; DwShape shape; };
+  static thread_local Kept kept[64] = {};
+  Kept& k = kept[((unsigned)C * 31u + (unsigned)OW * 7u + (unsigned)(R * 2 + stride) * 5u + (unsigned)es + (unsigned)N * 3u) % 64u];
+  const int key[8] = {N, C, OH, OW, R, stride, es, sms};
+  if (!std::equal(key, key + 8, k.key)) {
+    k.shape = dw_choose(N, C, OH, OW, R, stride, es, sms);
+    std::copy(key, key + 8, k.key);
+  }
+  return k.shape;
 }
 
 }  // namespace
@@ -305,7 +410,7 @@ bool depthwise_tma_supported(DType dt, int N, int H, int W, int C, int R, int S,
   if (C % V != 0 || C / V < 2) return false;
   const int OH = (H + 2 * pad - R) / stride + 1, OW = (W + 2 * pad - S) / stride + 1;
   if (OH <= 0 || OW <= 0) return false;
-  return (long long)N * ((OH + kTH - 1) / kTH) * ((OW + 7) / 8) < (1LL << 30);
+  return (long long)N * ((OH + 3) / 4) * ((OW + 1) / 2) < (1LL << 30);
 }
 
 cudaError_t launch_depthwise_tma(const void* x, const void* w, DType w_dt, const float* scale, const float* shift, void* y, DType dt,
@@ -314,39 +419,18 @@ cudaError_t launch_depthwise_tma(const void* x, const void* w, DType w_dt, const
   if (!depthwise_tma_supported(dt, N, H, W, C, R, S, stride, pad) || (reinterpret_cast<uintptr_t>(x) & 15) ||
       (reinterpret_cast<uintptr_t>(y) & 15))
     return cudaErrorInvalidValue;
-  const int es = (int)dtype_size(dt), V = 16 / es, cv = C / V;
+  const int es = (int)dtype_size(dt), V = 16 / es, cv = C / V;   // cv: 16-byte channel vectors
   const int OH = (H + 2 * pad - R) / stride + 1, OW = (W + 2 * pad - S) / stride + 1;
   DwParams p{};
-  // 256 threads: (column, four-channel vector) pairs of a tile in any split of whole 16-byte vectors: the one that leaves the
-  // fewest threads idle or outside the map and the channels.  Halo columns, rows of a patch shorter than 128 bytes and
-  // stages so large that fewer than three CTAs fit an SM count against it.
-  const int slots = kThreads / 2;                      // 16-byte vectors of a tile
-  int cbv = 0, tw = 0;
-  double best = 0.0;
-  for (int cand = 32; cand >= 2; --cand) {             // ties go to the wider chunk (longer contiguous runs in memory)
-    if (cand > cv) continue;
-    const int tiles = (OW + slots / cand - 1) / (slots / cand), t = (OW + tiles - 1) / tiles;
-    const int chunks = (cv + cand - 1) / cand, iw = (t - 1) * stride + R, ih = (kTH - 1) * stride + R;
-    const size_t need = 2 * (((size_t)iw * ih * cand * 16 + 127) & ~(size_t)127) + (size_t)(R * S + (es == 2 ? 1 : 2)) * cand * V * sizeof(float);
-    if (need > 200 * 1024 || iw > 256) continue;
-    double use = (double)cv / (chunks * cand) * OW / (tiles * t) * (t * cand) / slots;
-    use *= 0.5 + 0.5 * (t * stride) / iw;
-    if (cand < 8) use *= 0.5 + 0.5 * cand / 8.0;
-    if (need > 72 * 1024) use *= need > 110 * 1024 ? 0.6 : 0.9;
-    if (use > best + 1e-9) { best = use; cbv = cand; tw = t; }
-  }
-  if (cbv == 0) return cudaErrorInvalidValue;
+  const int sms = sm_count > 0 ? sm_count : 148;
+  const DwShape d = dw_shape(N, C, OH, OW, R, stride, es, sms);
+  if (d.cbv == 0) return cudaErrorInvalidValue;
+  const int tw = d.tw, cbv = d.cbv, px = d.px, kp = d.kp, th = es == 2 ? kp : 8, IH = (th - 1) * stride + R, IW = (tw - 1) * stride + R;
   p.tw = tw; p.cbv = cbv;
-  const int IW = (tw - 1) * stride + R, IH = (kTH - 1) * stride + R;
-  if (IW > 256 || IH > 256) return cudaErrorInvalidValue;
   p.stage_bytes = (uint32_t)IW * IH * cbv * 16;
   p.stage_stride = (p.stage_bytes + 127u) & ~127u;
-  const size_t wbytes = (size_t)(R * S + (es == 2 ? 1 : 2)) * cbv * V * sizeof(float);
-  int stages = kMaxStages;
-  while (stages > 2 && (size_t)stages * p.stage_stride + wbytes > 72 * 1024) --stages;   // three CTAs per SM when it fits
-  const size_t smem = (size_t)stages * p.stage_stride + wbytes;
-  if (smem > 200 * 1024) return cudaErrorInvalidValue;
-  p.stages = stages;
+  p.stages = d.stages;
+  const size_t smem = d.smem;
   p.w = w; p.w_half = w_dt == kF16; p.scale = scale; p.shift = shift; p.y = y;
   p.N = N; p.H = H; p.W = W; p.C = C; p.OH = OH; p.OW = OW; p.pad = pad; p.act = act;
   if (in_l.pitch == 0) in_l = dense_layout(H, W);
@@ -355,7 +439,7 @@ cudaError_t launch_depthwise_tma(const void* x, const void* w, DType w_dt, const
   // (zero-filled), so the halo reads the same values as over a dense map
   if (in_l.off != 0 && (in_l.off != 1 || in_l.pitch != W + 1 || in_l.img_rows != H + 1)) return cudaErrorInvalidValue;
   p.in_l = in_l; p.out_l = out_l;
-  p.tiles_x = (OW + tw - 1) / tw; p.tiles_y = (OH + kTH - 1) / kTH;
+  p.tiles_x = (OW + tw - 1) / tw; p.tiles_y = (OH + th - 1) / th;
   p.n_tiles = N * p.tiles_y * p.tiles_x;
   p.div_tx = epi::fast_div((uint32_t)p.tiles_x); p.div_ty = epi::fast_div((uint32_t)p.tiles_y);
   p.error_flag = error_flag;
@@ -374,15 +458,14 @@ cudaError_t launch_depthwise_tma(const void* x, const void* w, DType w_dt, const
     return cudaErrorInvalidValue;
 
   const int chunks = (cv + cbv - 1) / cbv;
-  const int per_sm = smem <= 72 * 1024 ? 3 : smem <= 110 * 1024 ? 2 : 1;
-  int gx = (sm_count > 0 ? sm_count : 148) * per_sm / chunks;
+  int gx = sms * d.per_sm / chunks;
   if (gx < 1) gx = 1;
   if (gx > p.n_tiles) gx = p.n_tiles;
   const dim3 grid((unsigned)gx, (unsigned)chunks);
   if (chunks > 65535) return cudaErrorInvalidValue;
-  if (dt == kF32) return launch_typed<float>(tm, p, R, stride, grid, smem, st);
-  if (dt == kF16) return launch_typed<__half>(tm, p, R, stride, grid, smem, st);
-  return launch_typed<__nv_bfloat16>(tm, p, R, stride, grid, smem, st);
+  if (dt == kF32) return launch_typed<float, 1, 4>(tm, p, R, stride, grid, d.threads, smem, st);
+  if (dt == kF16) return launch_shape<__half>(px, tm, p, R, stride, grid, d.threads, smem, st);
+  return launch_shape<__nv_bfloat16>(px, tm, p, R, stride, grid, d.threads, smem, st);
 }
 
 }  // namespace nncv_b200
