@@ -7,7 +7,8 @@
 // block outermost, tap, 16 channels a step), so the results are the same bits and the tile may be chosen by timing.
 // One image, us a layer in a row of launches, 128-row tiles before and this: 512 -> 512 3x3 on 7x7 12.4 9.7, 256 -> 256 on 14x14 8.1
 // 7.0, with the 1x1 branch 256 -> 512 11.8 8.1, 2048 -> 512 pointwise 9.3 7.2, 1024 -> 256 7.1 5.5; a layer of one block takes 4.1
-// either way.  Forwards of one image: ResNet-18 145 -> 114, ResNet-50 317 -> 267, MobileNetV3 273 -> 251.
+// either way.  Forwards of one image: ResNet-18 145 -> 114, ResNet-50 317 -> 267, MobileNetV3 273 -> 251; with the epilogue's
+// combinations as functions of their own 99, 227 and (with other kernels' gains) 201.
 //
 // One tile a CTA.  Warp 0 issues the MMAs.  Warps 1-4 copy, step j by warp j mod 4 (TMA; weights before the previous kernel
 // ends): one warp needs some 300 clocks a block (115 to see a free stage, 45 to announce the bytes, the rest for two copies), three
@@ -51,8 +52,73 @@ struct SmallParams {
   int tw_log, th_log;
   int tiles_x, tiles_y, n_tiles;
   epi::FastDiv div_taps, div_s;        // by the taps of a channel block, the branch's included, and by the filter's width
-  int stages_log, relu, act, bf16, out_f32, w_ready;
+  int stages_log, relu, bf16, out_f32, w_ready;
+  int mode;                            // of the epilogue (epi::mode_of)
 };
+
+// A load that stays where it stands: the compiler moves plain ones down to their use, behind the wait for the accumulator, where
+// their latency is bare (0.5 us a layer).
+__device__ __forceinline__ float2 load_now(const float* v) {
+  float2 r;
+  asm volatile("ld.global.nc.v2.f32 {%0, %1}, [%2];" : "=f"(r.x), "=f"(r.y) : "l"(v));
+  return r;
+}
+__device__ __forceinline__ uint32_t load_now(const unsigned short* v) {
+  uint32_t r;
+  asm volatile("ld.global.u32 %0, [%1];" : "=r"(r) : "l"(v));
+  return r;
+}
+
+// A thread's 2 x 8 values -> memory.  Each combination is a function of its own, as in epilogue.cuh: with the choices tested for
+// every pair a warp, alone on its scheduler, took 1300 to 2000 clocks for them, a quarter of a layer's time.
+template <bool BF16, bool RES, int ACT>
+__device__ __forceinline__ void finish(const uint32_t (&acc)[16], const float2 (&sc)[4], const float2 (&sh)[4], const uint32_t (&res)[2][4],
+                                       unsigned short* out, const long long (&at)[2], int cols0, int Kout) {
+  uint32_t o[2][4];
+#pragma unroll
+  for (int g = 0; g < 4; ++g)
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      unsigned long long v = epi::fma2(epi::pk(__uint_as_float(acc[4 * g + 2 * h]), __uint_as_float(acc[4 * g + 2 * h + 1])),
+                                       epi::pk(sc[g].x, sc[g].y), epi::pk(sh[g].x, sh[g].y));
+      if (RES) {
+        const float2 f = epi::unpack16(res[h][g], BF16);
+        v = epi::add2(v, epi::pk(f.x, f.y));
+      }
+      float a, b;
+      epi::unpk(v, a, b);
+      if (ACT == 2) {
+        a *= __saturatef(fmaf(a, 0.16666667f, 0.5f));
+        b *= __saturatef(fmaf(b, 0.16666667f, 0.5f));
+      } else if (ACT == 3) {
+        a *= __fdividef(1.0f, __expf(-a) + 1.0f);
+        b *= __fdividef(1.0f, __expf(-b) + 1.0f);
+      }
+      o[h][g] = epi::pack16(a, b, BF16, ACT == 1);
+    }
+#pragma unroll
+  for (int h = 0; h < 2; ++h)
+#pragma unroll
+    for (int g = 0; g < 4; ++g)
+      if (at[h] >= 0 && cols0 + 8 * g < Kout) *reinterpret_cast<uint32_t*>(out + at[h] + cols0 + 8 * g) = o[h][g];
+}
+__device__ __forceinline__ void finish_f32(const uint32_t (&acc)[16], const float2 (&sc)[4], const float2 (&sh)[4], bool relu, float* out,
+                                           const long long (&at)[2], int cols0, int Kout) {
+#pragma unroll
+  for (int h = 0; h < 2; ++h)
+#pragma unroll
+    for (int g = 0; g < 4; ++g) {
+      float a, b;
+      epi::unpk(epi::fma2(epi::pk(__uint_as_float(acc[4 * g + 2 * h]), __uint_as_float(acc[4 * g + 2 * h + 1])), epi::pk(sc[g].x, sc[g].y),
+                          epi::pk(sh[g].x, sh[g].y)),
+                a, b);
+      if (relu) {
+        a = !(a <= 0.0f) ? a : 0.0f;
+        b = !(b <= 0.0f) ? b : 0.0f;
+      }
+      if (at[h] >= 0 && cols0 + 8 * g < Kout) *reinterpret_cast<float2*>(out + at[h] + cols0 + 8 * g) = make_float2(a, b);
+    }
+}
 
 template <bool DUAL>
 __global__ void __launch_bounds__(kThreads)
@@ -168,7 +234,7 @@ conv_small_kernel(const __grid_constant__ CUtensorMap tm_in, const SmallParams p
     auto columns = [&](const float* v, float one, float2 (&c)[4]) {
 #pragma unroll
       for (int g = 0; g < 4; ++g)
-        c[g] = v && cols0 + 8 * g < p.Kout ? __ldg(reinterpret_cast<const float2*>(v + cols0 + 8 * g)) : make_float2(one, one);
+        c[g] = v && cols0 + 8 * g < p.Kout ? load_now(v + cols0 + 8 * g) : make_float2(one, one);
     };
     float2 sc[4], sh[4];
     uint32_t res[2][4];
@@ -182,7 +248,7 @@ conv_small_kernel(const __grid_constant__ CUtensorMap tm_in, const SmallParams p
 #pragma unroll
       for (int g = 0; g < 4; ++g)
         res[h][g] = p.residual && at[h] >= 0 && cols0 + 8 * g < p.Kout
-                        ? *reinterpret_cast<const uint32_t*>(static_cast<const unsigned short*>(p.residual) + at[h] + cols0 + 8 * g) : 0u;
+                        ? load_now(static_cast<const unsigned short*>(p.residual) + at[h] + cols0 + 8 * g) : 0u;
     const bool okw = ptx::warp_spin(acc_full, 0, abort_flag);
     if (okw) {
       ptx::tc_fence_after();
@@ -192,42 +258,26 @@ conv_small_kernel(const __grid_constant__ CUtensorMap tm_in, const SmallParams p
         uint32_t acc[16];
         ptx::tmem_ld_16x32_f(tmem + ((uint32_t)(quad * 32) << 16) + (uint32_t)(o * kBN), acc);
         ptx::tmem_ld_wait();
-        void* out = o ? p.out2 : p.out;
-        const bool with_res = o == 0 && p.residual != nullptr, relu = o == 0 && p.relu != 0;
-        const int act = o == 0 ? p.act : 0;
-#pragma unroll
-        for (int g = 0; g < 4; ++g) {
-          if (cols0 + 8 * g >= p.Kout) continue;
-#pragma unroll
-          for (int h = 0; h < 2; ++h) {
-            if (at[h] < 0) continue;
-            unsigned long long v = epi::fma2(epi::pk(__uint_as_float(acc[4 * g + 2 * h]), __uint_as_float(acc[4 * g + 2 * h + 1])),
-                                             epi::pk(sc[g].x, sc[g].y), epi::pk(sh[g].x, sh[g].y));
-            if (with_res) {
-              const float2 f = epi::unpack16(res[h][g], p.bf16 != 0);
-              v = epi::add2(v, epi::pk(f.x, f.y));
-            }
-            float a, b;
-            epi::unpk(v, a, b);
-            if (act == kActHardSwish) {
-              a *= __saturatef(fmaf(a, 0.16666667f, 0.5f));
-              b *= __saturatef(fmaf(b, 0.16666667f, 0.5f));
-            } else if (act == kActSilu) {
-              a *= __fdividef(1.0f, __expf(-a) + 1.0f);
-              b *= __fdividef(1.0f, __expf(-b) + 1.0f);
-            }
-            if (p.out_f32) {
-              if (relu) {
-                a = !(a <= 0.0f) ? a : 0.0f;
-                b = !(b <= 0.0f) ? b : 0.0f;
-              }
-              *reinterpret_cast<float2*>(static_cast<float*>(out) + at[h] + cols0 + 8 * g) = make_float2(a, b);
-            } else {
-              *reinterpret_cast<uint32_t*>(static_cast<unsigned short*>(out) + at[h] + cols0 + 8 * g) =
-                  epi::pack16(a, b, p.bf16 != 0, relu && act == 0);
-            }
-          }
+        if (p.out_f32) {
+          finish_f32(acc, sc, sh, p.relu != 0, static_cast<float*>(p.out), at, cols0, p.Kout);
+          continue;
         }
+        unsigned short* out = static_cast<unsigned short*>(o ? p.out2 : p.out);
+#define NNCV_FINISH(B_, R_, A_) \
+  case (B_ ? epi::kModeBf16 : 0) | (R_ ? epi::kModeRes : 0) | (A_ << epi::kModeActShift): finish<B_, R_, A_>(acc, sc, sh, res, out, at, cols0, p.Kout); break;
+        switch (o ? (p.mode & epi::kModeBf16) : p.mode) {
+          NNCV_FINISH(false, false, 0) NNCV_FINISH(false, false, 1) NNCV_FINISH(false, true, 0) NNCV_FINISH(false, true, 1)
+          NNCV_FINISH(true, false, 0) NNCV_FINISH(true, false, 1) NNCV_FINISH(true, true, 0) NNCV_FINISH(true, true, 1)
+          default:
+            if constexpr (!DUAL) {
+              switch (p.mode) {
+                NNCV_FINISH(false, false, 2) NNCV_FINISH(false, true, 2) NNCV_FINISH(true, false, 2) NNCV_FINISH(true, true, 2)
+                NNCV_FINISH(false, false, 3) NNCV_FINISH(false, true, 3) NNCV_FINISH(true, false, 3) NNCV_FINISH(true, true, 3)
+                default: break;
+              }
+            }
+        }
+#undef NNCV_FINISH
       }
     } else if (lane == 0 && p.error_flag) {
       atomicCAS(p.error_flag, 0, (int)kErrWaitEpilogue);
@@ -305,7 +355,7 @@ cudaError_t launch_conv_small(const TconvArgs& args, cudaStream_t stream) {
   p.n_tiles = (a.Kout + kBN - 1) / kBN;
   const long long tiles = conv_small_tiles(a.N, a.OH, a.OW, a.Kout);
   if (tiles <= 0 || tiles > 0x7fffffffLL) return cudaErrorInvalidValue;
-  p.relu = a.relu; p.act = a.act; p.bf16 = a.ab == kBF16; p.out_f32 = a.out_dtype == kF32; p.w_ready = a.weights_ready;
+  p.relu = a.relu; p.bf16 = a.ab == kBF16; p.mode = epi::mode_of(a.ab == kBF16, a.residual != nullptr, a.relu != 0, a.act); p.out_f32 = a.out_dtype == kF32; p.w_ready = a.weights_ready;
   const int taps_x = p.taps + (a.wpack2 ? 1 : 0);
   p.div_taps = epi::fast_div((uint32_t)taps_x); p.div_s = epi::fast_div((uint32_t)a.S);
   p.stages_log = 1;
