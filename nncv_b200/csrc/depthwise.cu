@@ -392,7 +392,7 @@ DwShape dw_choose(int N, int C, int OH, int OW, int R, int stride, int es, int s
 // The same, kept for the layers a thread asks for in turn: choosing takes longer than a launch.
 const DwShape& dw_shape(int N, int C, int OH, int OW, int R, int stride, int es, int sms) {
   struct Kept { int key[8]; DwShape shape; };
-  static thread_local Kept kept[64] = {};
+  thread_local Kept kept[64] = {};
   Kept& k = kept[((unsigned)C * 31u + (unsigned)OW * 7u + (unsigned)(R * 2 + stride) * 5u + (unsigned)es + (unsigned)N * 3u) % 64u];
   const int key[8] = {N, C, OH, OW, R, stride, es, sms};
   if (!std::equal(key, key + 8, k.key)) {
