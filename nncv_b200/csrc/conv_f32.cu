@@ -478,6 +478,334 @@ conv_f32_kernel(const __grid_constant__ CUtensorMap tm_in, const F32Params p) {
   }
 }
 
+// ------------------------------------------------------------------ small batches ----------
+// The same convolution on 64 x 32 tiles, one a CTA, for few pixels.  At one image what bounds a layer is its chain, and most of
+// that of the kernel above is not tensor work: after 2 to 9 blocks of 1550 clocks (its MMAs read 6 KB each, 48 clocks) a CTA of a
+// cluster waits 1000 to 2600 clocks for its peers' word, 2400 for 32 KB of their partial sums and 1600 until all may leave.  Here
+// a block takes 16 MMAs, two products side by side where they share an operand, of 24 to 32 clocks each; four warps copy, whole blocks are handed over, and the partial sums, a quarter
+// as many, are SENT: every CTA stores the rows that a peer finishes into that peer's shared memory and arrives on its barrier, so
+// that nobody reads from a CTA that could leave, and nobody waits for more than its own rows.
+// The sums are formed as above: each step of 16 channels of the large products rounded to registers, small products in groups; but
+// with fewer CTAs to a tile a sum has more terms one after another, so a block's four steps are added first, and even and odd
+// blocks apart (one chain: 9.5e-8 instead of 7.1e-8 off the result in 64 bits for 64 channels 3x3, where the kernel above split).
+constexpr int kSM = 64, kSN = 32;                       // tile
+constexpr int kSABytes = kSM * 128, kSBBytes = kSN * 128;
+constexpr int kSB = 3 * kSABytes, kSStage = kSB + 3 * kSBBytes;   // the pixels' planes, then the filter's, one below the other
+constexpr int kSStages = 6;                             // 216 KB: six blocks of 64 channels
+constexpr size_t kSSmem = 1024 + (size_t)kSStages * kSStage;
+constexpr int kSCopyWarps = 4, kSThreads = (1 + kSCopyWarps + 4) * 32;
+
+// Loads that stay where they stand (the compiler moves plain ones down to their use, behind the waits they should overlap).
+__device__ __forceinline__ uint2 load_now(const __nv_bfloat16* q) {
+  uint2 r;
+  asm volatile("ld.global.v2.u32 {%0, %1}, [%2];" : "=r"(r.x), "=r"(r.y) : "l"(q));
+  return r;
+}
+__device__ __forceinline__ float4 load_now(const float* q) {
+  float4 r;
+  asm volatile("ld.global.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(r.x), "=f"(r.y), "=f"(r.z), "=f"(r.w) : "l"(q));
+  return r;
+}
+__device__ __forceinline__ float4 load_single(const float* q) {   // four values that need not lie on a 16-byte boundary
+  float4 r;
+  asm volatile("ld.global.f32 %0, [%4];\n ld.global.f32 %1, [%4 + 4];\n ld.global.f32 %2, [%4 + 8];\n ld.global.f32 %3, [%4 + 12];"
+               : "=f"(r.x), "=f"(r.y), "=f"(r.z), "=f"(r.w) : "l"(q));
+  return r;
+}
+
+__global__ void __launch_bounds__(kSThreads, 1) conv_f32_small_kernel(const __grid_constant__ CUtensorMap tm_in, const F32Params p) {
+  constexpr uint32_t kQuad = 4 * kSN, kSmallCols = 2 * kQuad;   // two sets of the four large steps' accumulators, two pairs of small ones
+  extern __shared__ uint8_t smem_raw[];
+  __shared__ __align__(16) float s_recv[kSM * kSN];             // [part][row of this CTA's][column]
+  __shared__ int s_abort;
+  __shared__ uint32_t s_tmem;
+  __shared__ __align__(8) unsigned long long s_bars[2 * kSStages + 9];
+  const uint32_t ring = (ptx::smem_u32(smem_raw) + 1023u) & ~1023u;
+  const uint32_t full = ptx::smem_u32(s_bars), empty = full + 8 * kSStages, d_full = empty + 8 * kSStages, d_empty = d_full + 16;
+  const uint32_t s_full = d_empty + 16, s_empty = s_full + 16, recv = s_empty + 16;
+  const int warp = ptx::warp_uniform((int)threadIdx.x >> 5), lane = threadIdx.x & 31;
+  const int S = p.splits;
+  const uint32_t rank = S > 1 ? ptx::cluster_ctarank() : 0u;
+  if (threadIdx.x == 0) {
+    s_abort = 0;
+    for (int i = 0; i < 2 * kSStages; ++i) ptx::mbar_init(full + 8 * i, 1);
+    for (int i = 0; i < 2; ++i) {
+      ptx::mbar_init(d_full + 8 * i, 1);
+      ptx::mbar_init(d_empty + 8 * i, 4);
+      ptx::mbar_init(s_full + 8 * i, 1);
+      ptx::mbar_init(s_empty + 8 * i, 4);
+    }
+    ptx::mbar_init(recv, S > 4 ? S : 4);   // one arrival of each warp that sends rows here
+    ptx::mbar_fence_init();
+    ptx::prefetch_tensormap(&tm_in);
+  }
+  if (warp == 0) {
+    ptx::tmem_alloc(ptx::smem_u32(&s_tmem), 512);
+    ptx::tmem_relinquish();
+  }
+  ptx::tc_fence_before();
+  __syncthreads();
+  if (S > 1) ptx::cluster_sync_all();   // every CTA's barriers exist before anyone sends
+  ptx::tc_fence_after();
+  const uint32_t tmem = (uint32_t)ptx::warp_uniform((int)*reinterpret_cast<volatile uint32_t*>(&s_tmem));
+  volatile int* abort_flag = &s_abort;
+
+  const int w = (int)blockIdx.x / S;
+  const int m_item = (int)epi::div_by((uint32_t)w, p.div_nt), n_tile = w - m_item * p.n_tiles;
+  const int t2 = (int)epi::div_by((uint32_t)m_item, p.div_tx), t3 = (int)epi::div_by((uint32_t)t2, p.div_ty);
+  const int ox0 = (m_item - t2 * p.tiles_x) * p.tw, oy0 = (t2 - t3 * p.tiles_y) * p.th, n0 = t3 * p.tn;
+  const int kb_all = p.taps * p.CB, kb0 = kb_all * (int)rank / S, blocks = kb_all * ((int)rank + 1) / S - kb0;   // this CTA's part
+
+  if (warp == 0) {
+    // ------------------------------------------------------------------ MMAs ------------
+    const uint32_t issue = ptx::elect_one();
+    const uint32_t idesc = ptx::umma_idesc(kSM, kSN, 1), idesc2 = ptx::umma_idesc(kSM, 2 * kSN, 1);
+    const uint32_t ring_lo = ptx::smem_desc_k128_lo(ring);
+    // pixels' plane pa times the filter's plane pb (and the next one, idesc2)
+    auto mma = [&](uint32_t d, uint32_t at, uint32_t pa, uint32_t pb, uint32_t k4, uint32_t id, uint32_t accumulate) {
+      ptx::umma_f16(d, ptx::desc_from_halves(at + ((pa * kSABytes) >> 4) + k4 * 2, ptx::kSmemDescK128Hi),
+                    ptx::desc_from_halves(at + ((kSB + pb * kSBBytes) >> 4) + k4 * 2, ptx::kSmemDescK128Hi), id, accumulate, issue);
+    };
+    uint32_t st = 0, par = 0;
+    bool okw = true;
+    for (int i = 0; i < blocks; ++i) {
+      const uint32_t q = (uint32_t)i & 1u, group = (uint32_t)i / kSmallBlocks, sb = group & 1u;
+      const bool first = i % kSmallBlocks == 0, last = i % kSmallBlocks == kSmallBlocks - 1 || i + 1 == blocks;
+      if (!ptx::warp_spin(full + 8 * st, par, abort_flag) || (i >= 2 && !ptx::warp_spin(d_empty + 8 * q, (((uint32_t)i >> 1) & 1u) ^ 1u, abort_flag)) ||
+          (first && group >= 2 && !ptx::warp_spin(s_empty + 8 * sb, ((group >> 1) & 1u) ^ 1u, abort_flag))) {
+        okw = false;
+        break;
+      }
+      ptx::tc_fence_after();
+      const uint32_t at = ring_lo + st * (uint32_t)(kSStage >> 4), ds = tmem + kSmallCols + sb * 2 * kSN;
+#pragma unroll
+      for (uint32_t k4 = 0; k4 < 4; ++k4) mma(tmem + q * kQuad + k4 * kSN, at, 0, 0, k4, idesc, 0u);
+      ptx::tc_commit(d_full + 8 * q, issue);
+      // the small products in two accumulators side by side: a1 b2 | a1 b3, a2 b1 | a2 b2, a3 b1
+#pragma unroll
+      for (uint32_t k4 = 0; k4 < 4; ++k4) mma(ds, at, 0, 1, k4, idesc2, first && k4 == 0 ? 0u : 1u);
+#pragma unroll
+      for (uint32_t k4 = 0; k4 < 4; ++k4) mma(ds, at, 1, 0, k4, idesc2, 1u);
+#pragma unroll
+      for (uint32_t k4 = 0; k4 < 4; ++k4) mma(ds, at, 2, 0, k4, idesc, 1u);
+      ptx::tc_commit(empty + 8 * st, issue);
+      if (last) ptx::tc_commit(s_full + 8 * sb, issue);
+      if (++st == kSStages) { st = 0; par ^= 1u; }
+    }
+    if (!okw && lane == 0 && p.error_flag) atomicCAS(p.error_flag, 0, (int)kErrWaitMma);
+    ptx::grid_dependency_wait();
+  } else if (warp <= kSCopyWarps) {
+    // ------------------------------------------------------------------ copies: block i by warp 1 + i % 4 ----
+    const uint32_t issue = ptx::elect_one();
+    const int me = warp - 1;
+    auto where = [&](int i, int& cb, int& tap) {
+      cb = (kb0 + i) / p.taps;
+      tap = kb0 + i - cb * p.taps;
+    };
+    auto load_weights = [&](int cb, int tap, uint32_t st) {
+#pragma unroll
+      for (int pl = 0; pl < 3; ++pl)   // packed as tiles of 64 output channels: half of one
+        ptx::bulk_g2s(ring + st * kSStage + kSB + pl * kSBBytes,
+                      p.wpack + (((size_t)(n_tile >> 1) * 3 + pl) * kb_all + (size_t)tap * p.CB + cb) * kBBytes + (n_tile & 1) * kSBBytes, kSBBytes, full + 8 * st, issue);
+    };
+    // the packed weights never change: their first copies do not wait for the previous kernel
+    for (int i = me; i < kSStages && i < blocks; i += kSCopyWarps) {
+      int cb, tap;
+      where(i, cb, tap);
+      ptx::mbar_arrive_expect_tx(full + 8 * i, kSStage, issue);
+      load_weights(cb, tap, (uint32_t)i);
+    }
+    const int xb = p.stride * ox0 - p.pad_x, yb = p.stride * oy0 - p.pad_y;
+    int cb, tap;
+    where(me, cb, tap);
+    int r = tap / p.S, s = tap - r * p.S;
+    ptx::grid_dependency_wait();
+    ptx::grid_launch_dependents();
+    bool okw = true;
+    for (int i = me; i < blocks; i += kSCopyWarps) {
+      const uint32_t turn = (uint32_t)i / kSStages, st = (uint32_t)i - turn * kSStages;
+      if (turn > 0) {
+        if (!ptx::warp_spin(empty + 8 * st, (turn & 1u) ^ 1u, abort_flag)) { okw = false; break; }
+        ptx::mbar_arrive_expect_tx(full + 8 * st, kSStage, issue);
+      }
+#pragma unroll
+      for (int pl = 0; pl < 3; ++pl)
+        ptx::tma_load_5d(ring + st * kSStage + pl * kSABytes, &tm_in, cb * 64, xb + s, yb + r, n0, pl, full + 8 * st, issue);
+      if (turn > 0) load_weights(cb, tap, st);
+      where(i + kSCopyWarps, cb, tap);
+      r = tap / p.S;
+      s = tap - r * p.S;
+    }
+    if (!okw && lane == 0 && p.error_flag) atomicCAS(p.error_flag, 0, (int)kErrWaitProducer);
+  } else {
+    // ------------------------------------------------------------------ epilogue --------
+    ptx::grid_dependency_wait();
+    // rows 16 quad .. 16 quad + 15 of the tile lie in the first sixteen lanes of the warp's quadrant
+    const int quad = warp & 3, et = (int)threadIdx.x - (1 + kSCopyWarps) * 32;
+    const int rows_each = kSM / S, n = n_tile * kSN + 4 * (et & 7);
+    const bool live = n < p.Kout;
+    // the rows this thread finishes, four columns each: (et >> 3) + 16 k of this CTA's
+    long long pix[4];
+    uint2 res[4][3];
+    float4 res32[4];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      const int rr = (et >> 3) + 16 * k, r = (int)rank * rows_each + rr;
+      const int t1 = (int)epi::div_by((uint32_t)r, p.div_tw), tj = r - t1 * p.tw;
+      const int tt = (int)epi::div_by((uint32_t)t1, p.div_th), ti = t1 - tt * p.th;
+      const int img = n0 + tt, oy = oy0 + ti, ox = ox0 + tj;
+      pix[k] = live && rr < rows_each && img < p.NB && oy < p.OH && ox < p.OW ? ((long long)img * p.OH + oy) * p.OW + ox : -1;
+      if (p.residual && pix[k] >= 0) {
+        if (p.res_f32) {
+          res32[k] = load_now(static_cast<const float*>(p.residual) + pix[k] * p.ldo + n);
+        } else {
+#pragma unroll
+          for (int q = 0; q < 3; ++q) res[k][q] = load_now(static_cast<const __nv_bfloat16*>(p.residual) + q * p.res_plane + pix[k] * p.Kout + n);
+        }
+      }
+    }
+    const float4 sc = p.scale && live ? load_single(p.scale + n) : make_float4(1.f, 1.f, 1.f, 1.f);
+    const float4 sh = p.shift && live ? load_single(p.shift + n) : make_float4(0.f, 0.f, 0.f, 0.f);
+    // large products of even and of odd blocks, small products: three sums, added at the end
+    float sum[16], odd[16], rest[16];
+#pragma unroll
+    for (int e = 0; e < 16; ++e) sum[e] = odd[e] = rest[e] = 0.0f;
+    const uint32_t lane_base = tmem + ((uint32_t)(quad * 32) << 16);
+    auto hand_back = [&](uint32_t bar) {
+      ptx::tc_fence_before();
+      __syncwarp();
+      if (lane == 0) ptx::mbar_arrive(bar);
+    };
+    bool okw = true;
+    for (int i = 0; i < blocks; ++i) {
+      const uint32_t q = (uint32_t)i & 1u;
+      if (!ptx::warp_spin(d_full + 8 * q, ((uint32_t)i >> 1) & 1u, abort_flag)) { okw = false; break; }
+      ptx::tc_fence_after();
+      uint32_t v[4][16];
+#pragma unroll
+      for (uint32_t k4 = 0; k4 < 4; ++k4) ptx::tmem_ld_16x32_f(lane_base + q * kQuad + k4 * kSN, v[k4]);
+      ptx::tmem_ld_wait();
+      hand_back(d_empty + 8 * q);
+      float t[16];
+#pragma unroll
+      for (int e = 0; e < 16; ++e)
+        t[e] = (__uint_as_float(v[0][e]) + __uint_as_float(v[1][e])) + (__uint_as_float(v[2][e]) + __uint_as_float(v[3][e]));
+      if (q) {
+#pragma unroll
+        for (int e = 0; e < 16; ++e) odd[e] += t[e];
+      } else {
+#pragma unroll
+        for (int e = 0; e < 16; ++e) sum[e] += t[e];
+      }
+      if (i % kSmallBlocks == kSmallBlocks - 1 || i + 1 == blocks) {
+        const uint32_t group = (uint32_t)i / kSmallBlocks, sb = group & 1u;
+        if (!ptx::warp_spin(s_full + 8 * sb, (group >> 1) & 1u, abort_flag)) { okw = false; break; }
+        ptx::tc_fence_after();
+        ptx::tmem_ld_16x32_f(lane_base + kSmallCols + sb * 2 * kSN, v[0]);
+        ptx::tmem_ld_16x32_f(lane_base + kSmallCols + sb * 2 * kSN + kSN, v[1]);
+        ptx::tmem_ld_wait();
+        hand_back(s_empty + 8 * sb);
+#pragma unroll
+        for (int e = 0; e < 16; ++e) rest[e] += __uint_as_float(v[0][e]) + __uint_as_float(v[1][e]);
+      }
+    }
+    if (okw) {
+      // what the steps lost on average is given back with the small products; an infinite or NaN sum stays as it is (see take_small)
+#pragma unroll
+      for (int e = 0; e < 16; ++e) {
+        const float s = sum[e] + odd[e], t = s + fmaf(s, kCut, rest[e]);
+        sum[e] = fabsf(s) <= FLT_MAX ? t : s;
+      }
+      // rows to the CTA that finishes them (a lone CTA is no cluster: it keeps them by plain stores)
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        const int r = quad * 16 + h * 8 + (lane >> 2), to = r / rows_each, rr = r - to * rows_each;
+        float* const own = s_recv + ((int)rank * rows_each + rr) * kSN + 2 * (lane & 3);
+        const uint32_t dst = S > 1 ? ptx::map_to_cta(ptx::smem_u32(own), (uint32_t)to) : 0u;
+#pragma unroll
+        for (int g = 0; g < 4; ++g) {
+          if (S > 1) ptx::st_cluster_f2(dst + (uint32_t)g * 32u, sum[4 * g + 2 * h], sum[4 * g + 2 * h + 1]);
+          else *reinterpret_cast<float2*>(own + 8 * g) = make_float2(sum[4 * g + 2 * h], sum[4 * g + 2 * h + 1]);
+        }
+      }
+      __syncwarp();
+      if (S == 1) {
+        if (lane == 0) ptx::mbar_arrive(recv);
+      } else if (lane < (S == 8 ? 2 : 1)) {   // a warp's sixteen rows are one CTA's, of eight CTAs two's
+        ptx::mbar_arrive_remote(ptx::map_to_cta(recv, (uint32_t)(quad * 16 / rows_each + lane)));
+      }
+      okw = S > 1 ? ptx::warp_spin_cluster(recv, 0, abort_flag) : ptx::warp_spin(recv, 0, abort_flag);
+    }
+    if (okw) {
+      float4 v[4];
+      const float* mine = s_recv + (et >> 3) * kSN + 4 * (et & 7);
+      auto add = [&](float4& a, const float4& b) { a.x += b.x; a.y += b.y; a.z += b.z; a.w += b.w; };
+      if (S == 1) {
+#pragma unroll
+        for (int k = 0; k < 4; ++k) v[k] = *reinterpret_cast<const float4*>(mine + 16 * k * kSN);
+      } else {   // parts in rank order
+#pragma unroll
+        for (int k = 0; k < 2; ++k) {
+          const int rr = (et >> 3) + 16 * k;
+          v[k] = make_float4(0.f, 0.f, 0.f, 0.f);
+          if (rr >= rows_each) continue;
+          v[k] = *reinterpret_cast<const float4*>(mine + 16 * k * kSN);
+          for (int q = 1; q < S; ++q) add(v[k], *reinterpret_cast<const float4*>(mine + (16 * k + q * rows_each) * kSN));
+        }
+        v[2] = v[3] = make_float4(0.f, 0.f, 0.f, 0.f);
+      }
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        v[k].x = fmaf(v[k].x, sc.x, sh.x); v[k].y = fmaf(v[k].y, sc.y, sh.y);
+        v[k].z = fmaf(v[k].z, sc.z, sh.z); v[k].w = fmaf(v[k].w, sc.w, sh.w);
+      }
+      if (p.residual) {
+        if (p.res_f32) {
+#pragma unroll
+          for (int k = 0; k < 4; ++k)
+            if (pix[k] >= 0) add(v[k], res32[k]);
+        } else {
+#pragma unroll
+          for (int k = 0; k < 4; ++k)
+            if (pix[k] >= 0) add(v[k], join4(res[k]));
+        }
+      }
+      if (p.relu) {
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+          v[k].x = !(v[k].x <= 0.0f) ? v[k].x : 0.0f; v[k].y = !(v[k].y <= 0.0f) ? v[k].y : 0.0f;
+          v[k].z = !(v[k].z <= 0.0f) ? v[k].z : 0.0f; v[k].w = !(v[k].w <= 0.0f) ? v[k].w : 0.0f;
+        }
+      }
+      if (p.out_f32) {
+#pragma unroll
+        for (int k = 0; k < 4; ++k)
+          if (pix[k] >= 0) *reinterpret_cast<float4*>(static_cast<float*>(p.out) + pix[k] * p.ldo + n) = v[k];
+      } else {
+#pragma unroll
+        for (int k = 0; k < 4; ++k)
+          if (pix[k] >= 0) {
+            uint2 o[3];
+            split4(v[k], o);
+#pragma unroll
+            for (int q = 0; q < 3; ++q)
+              *reinterpret_cast<uint2*>(static_cast<__nv_bfloat16*>(p.out) + q * p.out_plane + pix[k] * p.Kout + n) = o[q];
+          }
+      }
+    } else if (lane == 0 && p.error_flag) {
+      atomicCAS(p.error_flag, 0, (int)kErrWaitEpilogue);
+    }
+  }
+  ptx::tc_fence_before();
+  __syncthreads();
+  // Everything that was sent to this CTA has arrived, unless a wait gave up: then it stays until the others have left or given up too.
+  if (S > 1 && s_abort) ptx::cluster_sync_all();
+  if (warp == 0) {
+    __syncwarp();
+    ptx::tmem_dealloc(tmem, 512);
+  }
+}
+
 // ------------------------------------------------------------------ weights and layouts ----
 // Filter value w(n, t, c), t = tap, c = channel of a block, as three planes of swizzled 64 x 64 tiles.  STEM: the four
 // "taps" are pairs of input rows, the 64 "channels" the 2 rows x 8 pixels x 4 channels of a window (see nchw_to_planes).
@@ -707,7 +1035,7 @@ static int clusters_that_fit(int s, int sms) {
   return fit.of[s];
 }
 
-static void pick_tile(long long m_tiles, int Kout, int kb_all, int sms, int* bn, int* splits) {
+static double pick_tile(long long m_tiles, int Kout, int kb_all, int sms, int* bn, int* splits) {
   double best = 1e30;
   for (int b = 64; b <= (Kout > 64 ? 128 : 64); b *= 2)
     for (int s = 1; s <= 8 && s <= kb_all; s *= 2) {
@@ -717,6 +1045,19 @@ static void pick_tile(long long m_tiles, int Kout, int kb_all, int sms, int* bn,
       const double t = rounds * (((kb_all + s - 1) / s) * (b == 64 ? 1560.0 : 2000.0) + (b == 64 ? 4700.0 : 12000.0)) + 5000.0 + (s > 1 ? 1500.0 : 0.0);
       if (t < best) { best = t; *bn = b; *splits = s; }
     }
+  return best;
+}
+
+// Small tiles where the modelled time of all rounds is less: about 620 clocks a block, 4500 besides, 1000 for sending.
+static bool pick_small(long long tiles, int kb_all, int sms, double other, int* splits) {
+  static const ClusterFit fit = cluster_fit(conv_f32_small_kernel, kSThreads, kSSmem, sms);
+  bool found = false;
+  for (int s = 1; s <= 8 && s <= kb_all; s *= 2) {
+    const double rounds = (double)((tiles + fit.of[s] - 1) / fit.of[s]);
+    const double t = rounds * ((kb_all + s - 1) / s * 620.0 + 4500.0 + (s > 1 ? 1000.0 : 0.0));
+    if (t < other) { other = t; *splits = s; found = true; }
+  }
+  return found;
 }
 
 template <int BN>
@@ -740,6 +1081,26 @@ static cudaError_t launch_f32_cfg(const CUtensorMap& tm, const F32Params& p, int
   cfg.attrs = attr;
   cfg.numAttrs = p.splits > 1 ? 2 : 1;
   return cudaLaunchKernelEx(&cfg, conv_f32_kernel<BN>, tm, p);
+}
+
+static cudaError_t launch_f32_small(const CUtensorMap& tm, const F32Params& p, cudaStream_t stream) {
+  cudaError_t e = cudaFuncSetAttribute(conv_f32_small_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSSmem);
+  if (e != cudaSuccess) return e;
+  if ((long long)p.items * p.splits > 0x7fffffffLL) return cudaErrorInvalidValue;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)(p.items * p.splits));
+  cfg.blockDim = dim3(kSThreads);
+  cfg.dynamicSmemBytes = kSSmem;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  attr[1].id = cudaLaunchAttributeClusterDimension;
+  attr[1].val.clusterDim.x = (unsigned)p.splits;
+  attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = p.splits > 1 ? 2 : 1;
+  return cudaLaunchKernelEx(&cfg, conv_f32_small_kernel, tm, p);
 }
 
 cudaError_t launch_conv_f32(const ConvF32Args& args, cudaStream_t stream) {
@@ -780,10 +1141,17 @@ cudaError_t launch_conv_f32(const ConvF32Args& args, cudaStream_t stream) {
   const long long tiles_n = (a.N + tn - 1) / tn;
   const int sms = a.sm_count > 0 ? a.sm_count : 148;
   const long long m_tiles = (long long)p.tiles_x * p.tiles_y * tiles_n;
-  int bn = 64;
-  pick_tile(m_tiles, a.Kout, p.taps * p.CB, sms, &bn, &p.splits);
+  int bn = 64, sw, sh, sn;
+  conv_small_tile(a.N, a.OH, a.OW, &sw, &sh, &sn);
+  const long long small_m = (long long)((a.OW + sw - 1) / sw) * ((a.OH + sh - 1) / sh) * ((a.N + sn - 1) / sn);
+  const double wide = pick_tile(m_tiles, a.Kout, p.taps * p.CB, sms, &bn, &p.splits);
+  if ((sw > sh ? sw : sh) * p.stride <= 256 && pick_small(small_m * ((a.Kout + kSN - 1) / kSN), p.taps * p.CB, sms, wide, &p.splits)) {
+    bn = kSN;
+    p.tw = tw = sw; p.th = th = sh; p.tn = tn = sn;
+    p.tiles_x = (a.OW + tw - 1) / tw; p.tiles_y = (a.OH + th - 1) / th;
+  }
   p.n_tiles = (a.Kout + bn - 1) / bn;
-  const long long items = m_tiles * p.n_tiles;
+  const long long items = (bn == kSN ? small_m : m_tiles) * p.n_tiles;
   if (items <= 0 || items > 0x7fffffffLL) return cudaErrorInvalidValue;
   p.items = (int)items;
   p.div_tx = epi::fast_div((uint32_t)p.tiles_x); p.div_ty = epi::fast_div((uint32_t)p.tiles_y); p.div_nt = epi::fast_div((uint32_t)p.n_tiles);
@@ -808,6 +1176,7 @@ cudaError_t launch_conv_f32(const ConvF32Args& args, cudaStream_t stream) {
   if (enc(&tm, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 5, const_cast<void*>(a.in), gdim, gstr, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
           CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
     return cudaErrorInvalidValue;
+  if (bn == kSN) return launch_f32_small(tm, p, stream);
   return bn == 64 ? launch_f32_cfg<64>(tm, p, sms, stream) : launch_f32_cfg<128>(tm, p, sms, stream);
 }
 

@@ -530,6 +530,24 @@ __device__ __forceinline__ void tmem_relinquish_pair() {
 __device__ __forceinline__ void tmem_dealloc_pair(uint32_t taddr, uint32_t ncols) {
   asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(ncols) : "memory");
 }
+__device__ __forceinline__ bool warp_spin_cluster(uint32_t bar, uint32_t parity, volatile int* abort_flag) {
+  long long t0 = 0;
+  for (uint32_t i = 0;; ++i) {
+    if (warp_all(mbar_try_wait_cluster(bar, parity))) return true;
+    if ((i & 63u) == 63u) {
+      const long long now = clock64();
+      if (t0 == 0) t0 = now;
+      if (warp_all(*abort_flag != 0)) return false;
+      if (warp_all(now - t0 > (1LL << 31))) {
+        *abort_flag = 1;
+        return false;
+      }
+    }
+  }
+}
+__device__ __forceinline__ void st_cluster_f2(uint32_t cluster_addr, float a, float b) {
+  asm volatile("st.shared::cluster.v2.f32 [%0], {%1, %2};" ::"r"(cluster_addr), "f"(a), "f"(b) : "memory");
+}
 __device__ __forceinline__ bool warp_wait_cluster(uint32_t bar, uint32_t parity, volatile int* abort_flag) {
   return warp_all(mbar_wait_cluster_abortable(bar, parity, abort_flag));
 }
