@@ -111,9 +111,9 @@ __device__ __forceinline__ void matvec(const float* m, int rows, int k, const fl
       for (int im = 0; im < G; ++im)
 #pragma unroll
         for (int d = L / 2; d > 0; d >>= 1) s[r][im] += __shfl_xor_sync(0xffffffffu, s[r][im], d);
-      if (j < rows && lane == 0) {
+      if (j < rows && lane < kCluster) {   // every lane has the sums: each sees to one CTA of the cluster
 #pragma unroll
-        for (int im = 0; im < G; ++im) out(j, im, s[r][im]);
+        for (int im = 0; im < G; ++im) out(j, im, s[r][im], lane);
       }
     }
   }
@@ -121,12 +121,6 @@ __device__ __forceinline__ void matvec(const float* m, int rows, int k, const fl
 
 // first of the n rows that CTA `rank` of the cluster owns
 __device__ __forceinline__ int row_of(int n, int rank) { return n * rank / kCluster; }
-__device__ __forceinline__ int owner_of(int n, int row) {   // the CTA whose rows [row_of(r), row_of(r + 1)) hold it
-  int r = row * kCluster / n;
-  if (row_of(n, r + 1) <= row) ++r;
-  return r;
-}
-
 template <typename T, int G, bool STAGED>   // G images a cluster (1, 2 or 4); the matrices staged in shared memory
 __global__ void __cluster_dims__(kCluster, 1, 1) __launch_bounds__(kThreads, 4) se_kernel(T* __restrict__ x, const SeParams p) {
   using VT = Vec8<T>;
@@ -135,10 +129,9 @@ __global__ void __cluster_dims__(kCluster, 1, 1) __launch_bounds__(kThreads, 4) 
   __shared__ __align__(8) unsigned long long w_bar;
   const int C = p.C, Cr = p.Cr, HW = p.H * p.W;
   float* part = smem;                          // [G][kThreads][V]: sums of the pixel slots of this CTA's slices
-  float* slice_sum = part + G * kThreads * V;         // [G][C]: this CTA's slices (G of the G * 8 of the cluster); later its gates
-  float* pooled = slice_sum + C + 8 * G;       // [G][C]; later the gates of its image
-  float* hid = pooled + G * C;                 // [G][Cr]: the hidden values this CTA computed
-  float* hidden = hid + G * Cr;                // [G][Cr]: all of them
+  float* slice_sum = part + G * kThreads * V;  // [C]: the sum of this CTA's slices (G of the G * 8 of the cluster)
+  float* pooled = slice_sum + C;               // [G][C]; later the gates of its image
+  float* hidden = pooled + G * C;              // [G][Cr]
   float* m1 = hidden + G * Cr;                 // its rows of W1 and W2
   cg::cluster_group cluster = cg::this_cluster();
   const int rank = (int)cluster.block_rank();
@@ -235,32 +228,24 @@ __global__ void __cluster_dims__(kCluster, 1, 1) __launch_bounds__(kThreads, 4) 
   // bounded; every thread of the cluster takes the same way out of a copy that does not arrive: none, the sums are then
   // wrong and the status word says so
   if (STAGED && !ptx::mbar_wait(bar, 0) && p.error_flag && threadIdx.x == 0) atomicCAS(p.error_flag, 0, (int)kErrWaitLoader);
-  auto to_hidden = [&](int j, int im, float v) {
+  // Hidden values and gates are stored into the CTAs that use them: nobody reads another's shared memory after the first exchange,
+  // so that a CTA may leave when it is done.  (Collected by their readers, with a last barrier before anyone left, the exchanges took
+  // 2500 clocks more, at two images a fifth of the kernel.)
+  auto to_hidden = [&](int j, int im, float v, int q) {
     v += __ldg(p.b1 + r1 + j);
-    hid[im * Cr + j] = !(v <= 0.0f) ? v : 0.0f;
+    *cluster.map_shared_rank(&hidden[im * Cr + r1 + j], q) = !(v <= 0.0f) ? v : 0.0f;
   };
   const float* w1 = STAGED ? m1 : p.w1 + (size_t)r1 * C;
   if (n1 <= 3 * kWarps) matvec<G, 32, STAGED>(w1, n1, C, pooled, to_hidden);
   else matvec<G, 8, STAGED>(w1, n1, C, pooled, to_hidden);
-  cluster.sync();                              // also: nobody reads slice_sum any more
-  for (int i = threadIdx.x; i < G * Cr; i += kThreads) {
-    const int im = i / Cr, j = i - im * Cr, q = owner_of(Cr, j);
-    hidden[i] = *cluster.map_shared_rank(&hid[im * Cr + j - row_of(Cr, q)], q);
-  }
-  __syncthreads();
-  auto to_gate = [&](int j, int im, float v) { slice_sum[im * n2 + j] = hard_sigmoid<T>(v + __ldg(p.b2 + r2 + j)); };
+  cluster.sync();                              // also: nobody reads slice_sum or pooled any more
+  auto to_gate = [&](int j, int im, float v, int q) {   // to the CTAs of image im
+    if (q < per) *cluster.map_shared_rank(&pooled[r2 + j], im * per + q) = hard_sigmoid<T>(v + __ldg(p.b2 + r2 + j));
+  };
   const float* w2 = STAGED ? m2 : p.w2 + (size_t)r2 * Cr;
   if (n2 <= 3 * kWarps) matvec<G, 32, STAGED>(w2, n2, Cr, hidden, to_gate);
   else matvec<G, 8, STAGED>(w2, n2, Cr, hidden, to_gate);
   cluster.sync();
-  {                                            // the gates of this CTA's image
-    const int im = rank / per;
-    for (int c = threadIdx.x; c < C; c += kThreads) {
-      const int q = owner_of(C, c), lo = row_of(C, q);
-      pooled[c] = *cluster.map_shared_rank(&slice_sum[im * (row_of(C, q + 1) - lo) + c - lo], q);
-    }
-  }
-  cluster.sync();                              // the other CTAs' reads of this CTA's shared memory are over
   if (!live) return;
   float g[V];
 #pragma unroll
@@ -279,7 +264,7 @@ __global__ void __cluster_dims__(kCluster, 1, 1) __launch_bounds__(kThreads, 4) 
 
 size_t se_smem(bool staged, int V, int G, int C, int Cr) {
   const size_t m = staged ? (size_t)((Cr + kCluster - 1) / kCluster) * C + (size_t)((C + kCluster - 1) / kCluster) * Cr : 0;
-  return ((size_t)G * kThreads * V + (size_t)(C + 8 * G + G * C) + 2 * (size_t)G * Cr + m) * sizeof(float);
+  return ((size_t)G * kThreads * V + (size_t)(C + G * C) + (size_t)G * Cr + m) * sizeof(float);
 }
 
 template <typename T, int G, bool STAGED>
