@@ -909,6 +909,9 @@ cudaError_t launch_stem_pool(const StemArgs& a, cudaStream_t stream) {
   // bands: enough items to fill the SMs several times over, at least 4 pooled rows each
   int band_rows = p.PH;
   while (band_rows > 4 && (long long)a.N * ((p.PH + band_rows - 1) / band_rows) < 6LL * sms) band_rows = (band_rows + 1) / 2;
+  // fewer where all bands still run at once: then the longest band is the kernel's time (a band of four rows works on eleven row
+  // pairs, of one on five)
+  while (band_rows > 1 && (long long)a.N * ((p.PH + (band_rows + 1) / 2 - 1) / ((band_rows + 1) / 2)) <= sms) band_rows = (band_rows + 1) / 2;
   p.band_rows = band_rows;
   p.bands = (p.PH + band_rows - 1) / band_rows;
   const size_t smem = 1024 + p.w_bytes + (size_t)kRingSlots * p.slot_bytes + 256 +
