@@ -58,9 +58,9 @@ struct SmallParams {
 
 // A load that stays where it stands: the compiler moves plain ones down to their use, behind the wait for the accumulator, where
 // their latency is bare (0.5 us a layer).
-__device__ __forceinline__ float2 load_now(const float* v) {
+__device__ __forceinline__ float2 load_now(const float* v) {   // one by one: scale and shift may lie on any float's boundary
   float2 r;
-  asm volatile("ld.global.nc.v2.f32 {%0, %1}, [%2];" : "=f"(r.x), "=f"(r.y) : "l"(v));
+  asm volatile("ld.global.nc.f32 %0, [%2];\n ld.global.nc.f32 %1, [%2 + 4];" : "=&f"(r.x), "=f"(r.y) : "l"(v));
   return r;
 }
 __device__ __forceinline__ uint32_t load_now(const unsigned short* v) {
@@ -336,9 +336,7 @@ cudaError_t launch_conv_small(const TconvArgs& args, cudaStream_t stream) {
   if (a.wpack2 && (!a.out2 || a.out_dtype == kF32 || a.R != a.S || a.R % 2 == 0 || a.pad != a.R / 2)) return cudaErrorInvalidValue;
   const uintptr_t al = reinterpret_cast<uintptr_t>(a.in) | reinterpret_cast<uintptr_t>(a.out) | reinterpret_cast<uintptr_t>(a.wpack) |
                        reinterpret_cast<uintptr_t>(a.wpack2) | reinterpret_cast<uintptr_t>(a.out2);
-  const uintptr_t cols = reinterpret_cast<uintptr_t>(a.scale) | reinterpret_cast<uintptr_t>(a.shift) | reinterpret_cast<uintptr_t>(a.scale2) |
-                         reinterpret_cast<uintptr_t>(a.shift2);
-  if ((al & 15) || (cols & 7) || (reinterpret_cast<uintptr_t>(a.residual) & 31)) return cudaErrorMisalignedAddress;
+  if ((al & 15) || (reinterpret_cast<uintptr_t>(a.residual) & 31)) return cudaErrorMisalignedAddress;
   SmallParams p;
   p.wpack = static_cast<const uint8_t*>(a.wpack); p.wpack2 = static_cast<const uint8_t*>(a.wpack2);
   p.scale = a.scale; p.shift = a.shift; p.scale2 = a.scale2; p.shift2 = a.shift2;

@@ -64,3 +64,57 @@ def test_small_tiles_with_branch(n, c, h, w, k):
         main.close()
         branch.close()
     assert torch.equal(got[0][0], got[1][0]) and torch.equal(got[0][1], got[1][1]) and not got[0][0].isnan().any()
+
+
+def _off(a, floats):
+    """A device copy of the vector that starts `floats` floats past a 256-byte boundary."""
+    t = torch.zeros(a.size + 8, device="cuda")
+    t[floats:floats + a.size] = torch.from_numpy(a).cuda()
+    return t[floats:floats + a.size]
+
+
+@pytest.mark.parametrize("bn", [0, 32, 64])
+@pytest.mark.parametrize("algo", [0, 2])
+def test_scale_and_shift_on_any_float_boundary(algo, bn):
+    """A shape's kernel is settled (bn 0: by timing) with aligned vectors; the same call then takes vectors one to three floats on."""
+    n, c, h, w, k = 1, 128, 7, 9, 64
+    g = np.random.default_rng(3)
+    wt = (g.standard_normal((k, c, 3, 3)) * np.sqrt(2.0 / (9 * c))).astype(np.float32)
+    scale, shift = g.uniform(0.5, 1.5, k).astype(np.float32), g.standard_normal(k).astype(np.float32)
+    X = G.dev(g.standard_normal((n, h, w, c)).astype(np.float32), F16)
+    conv, got = G.Conv(wt, 1, 1, F16, algo), []
+    try:
+        check(lib().nncv_b200_conv_set_tile(conv.h, bn, 1, 0))
+        for off in (0, 1, 2, 3):
+            S, H = _off(scale, off), _off(shift, (off + 1) % 4 if off else 0)
+            Y = torch.full((n, h, w, k), float("nan"), device="cuda", dtype=torch.float16)
+            check(lib().nncv_b200_conv_run(conv.h, G.p(X), G.p(Y), n, h, w, G.p(S), G.p(H), None, 1, G.stream_ptr()))
+            G.sync_check()
+            got.append(Y)
+    finally:
+        conv.close()
+    assert not got[0].isnan().any() and all(torch.equal(y, got[0]) for y in got[1:])
+
+
+@pytest.mark.parametrize("bn", [0, 32, 128])
+def test_branch_scale_and_shift_on_any_float_boundary(bn):
+    n, c, h, w, k = 1, 64, 9, 13, 128
+    g = np.random.default_rng(4)
+    w3 = (g.standard_normal((k, c, 3, 3)) * np.sqrt(2.0 / (9 * c))).astype(np.float32)
+    w1 = (g.standard_normal((k, c, 1, 1)) * np.sqrt(2.0 / c)).astype(np.float32)
+    cols = [a.astype(np.float32) for a in (g.uniform(0.5, 1.5, k), g.standard_normal(k), g.uniform(0.5, 1.5, k), g.standard_normal(k))]
+    X = G.dev(g.standard_normal((n, h, w, c)).astype(np.float32), F16)
+    oh, ow = (h - 1) // 2 + 1, (w - 1) // 2 + 1
+    main, branch, got = G.Conv(w3, 2, 1, F16), G.Conv(w1, 2, 0, F16), []
+    try:
+        check(lib().nncv_b200_conv_set_tile(main.h, bn, 1, 0))
+        for off in (0, 1):
+            v = [_off(a, off) for a in cols]
+            Y = [torch.full((n, oh, ow, k), float("nan"), device="cuda", dtype=torch.float16) for _ in range(2)]
+            check(lib().nncv_b200_conv_run_fused(main.h, branch.h, G.p(X), G.p(Y[0]), G.p(Y[1]), n, h, w, *map(G.p, v), 1, G.stream_ptr()))
+            G.sync_check()
+            got.append(Y)
+    finally:
+        main.close()
+        branch.close()
+    assert not got[0][0].isnan().any() and torch.equal(got[0][0], got[1][0]) and torch.equal(got[0][1], got[1][1])
