@@ -5,14 +5,16 @@
 // The operator is bound by HBM: 2 bytes in and 2 bytes out per element, 9 or 25 multiply-adds.  A
 // kernel that fetches its taps with per-thread global loads spends its time waiting for them (a
 // few loads in flight per thread, bounds checks between them), so here a persistent CTA walks
-// tiles of 8 output rows x TW output columns x CB channels and one thread issues, two tiles ahead,
-// ONE tensor copy per tile: the input patch with its halo, out-of-range pixels filled with zeros by
-// the copy engine (no bounds checks on the input side at all).  The 256 threads then read the
-// patch from shared memory: thread = (four channels, one or two output columns), computing a column strip of output rows in fp32
-// pairs (fma.rn.f32x2), so that each input value is loaded once per input column and reused down the strip, and each
-// filter value serves the strip.  What bounds the 16-bit kernels is the pipe of the packed multiply-adds, on which the conversions
-// to fp32 run too (64x112x112x96 hard-swish: 64 % of its rate with one column a thread, 15 conversions beside 18 multiply-adds
-// for an output of four channels; two columns share four of six input columns: 10).  With eight channels a thread and strips of four rows the 5x5 layers were bound by
+// tiles of 4 or 8 output rows x TW output columns x CB channels and one thread issues, one or two tiles
+// ahead, ONE tensor copy per tile: the input patch with its halo, out-of-range pixels filled with zeros by
+// the copy engine (no bounds checks on the input side at all).  The block's threads (up to 128, in fp32
+// 256) then read the patch from shared memory: thread = (four channels, one or two output columns),
+// computing a column strip of output rows in fp32 pairs (fma.rn.f32x2), so that each input value is
+// loaded once per input column and reused down the strip, and each filter value serves the strip.
+// What bounds the 16-bit kernels is the pipe of the packed multiply-adds, on which the conversions to
+// fp32 run too (64x112x112x96 hard-swish: 64 % of its rate with one column a thread, 15 conversions
+// beside 18 multiply-adds for an output of four channels; two columns share four of six input columns:
+// 10).  With eight channels a thread and strips of four rows the 5x5 layers were bound by
 // shared memory: a filter vector of eight fp32 is two loads at a stride of 32 bytes, two-way bank conflicts, and those loads
 // were two thirds of the traffic (14x14x240 at batch 256: 9.8 M wavefronts, 48 us); now a lane's four filter values are 16
 // contiguous bytes and are read half as often.  Filter, scale and shift sit in shared memory: for the 16-bit types as the
@@ -26,10 +28,9 @@
 #include <cuda_runtime.h>
 #include <cudaTypedefs.h>
 
-#include <algorithm>
-#include <cmath>
 #include <mutex>
 
+#include "depthwise_shape.h"
 #include "epilogue.cuh"
 #include "kernels.h"
 #include "ptx.cuh"
@@ -38,13 +39,10 @@ namespace nncv_b200 {
 
 namespace {
 
-// What a thread computes: KP output rows x PX adjacent output columns of four channels.
-// Threads at most, and CTAs of that size an SM (by registers)
-template <typename T> constexpr int kMaxThreads = sizeof(T) == 4 ? 256 : 128;
-template <typename T, int KS, int PX> constexpr int kCtas = sizeof(T) == 4 ? (KS == 3 ? 3 : 2) : PX == 2 ? (KS == 3 ? 4 : 3) : (KS == 3 ? 6 : 4);
+// What a thread computes: KP output rows x PX adjacent output columns of four channels (depthwise_shape.h).
 template <typename T, int KP> constexpr int kTH = sizeof(T) == 4 ? 8 : KP;   // output rows of a tile
 template <typename T> constexpr bool kFold = sizeof(T) == 2;   // the scale multiplied into the filter
-constexpr int kMaxStages = 3;
+using dw::kMaxStages;
 
 struct DwParams {
   const void* w;       // [C][KS*KS], fp32 or fp16
@@ -119,7 +117,7 @@ __device__ __forceinline__ float act1(float x, int act) {
 }
 
 template <typename T, int KS, int STRIDE, int PX, int kP>
-__global__ void __launch_bounds__(kMaxThreads<T>, kCtas<T, KS, PX>) depthwise_tma_kernel(const __grid_constant__ CUtensorMap tm_in, const DwParams p) {
+__global__ void __launch_bounds__(dw::max_threads(sizeof(T)), dw::ctas(sizeof(T), KS, PX)) depthwise_tma_kernel(const __grid_constant__ CUtensorMap tm_in, const DwParams p) {
   ptx::grid_dependency_wait();
   ptx::grid_launch_dependents();
   constexpr int V = 4;                                  // channels of a thread
@@ -320,88 +318,6 @@ cudaError_t launch_shape(int px, const CUtensorMap& tm, const DwParams& p, int k
   return stride == 1 ? launch_one<T, 5, 1, 2, 8>(tm, p, grid, threads, smem, st) : launch_one<T, 5, 2, 2, 4>(tm, p, grid, threads, smem, st);
 }
 
-// Tile, outputs of a thread and block of a layer: what dw_shape chooses.
-struct DwShape { int cbv, tw, px, kp, threads, stages, per_sm; size_t smem; };
-
-// 16-bit types: two columns x eight rows a thread at stride 1 (two x four at stride 2, where a patch has twice the rows) read and
-// convert each input value for two columns at once; one column x eight rows leaves none of an odd, narrow map's threads idle, needs
-// fewer registers and, with few channels, meets fewer bank conflicts.  fp32, whose rows are twice as long and need no conversion:
-// four rows of one column.  A tile is any split of columns and whole 16-byte channel vectors that a block's threads cover, and the
-// block has as many threads as it needs.  For 16 bits the least modelled cost counts, in instructions of a thread per output:
-// multiply-adds, conversions and (twice, with their bank conflicts) shared-memory reads, times the outputs, idle ones included, that
-// the busiest SM computes; halo columns, rows of a patch shorter than 256 (and more so 128) bytes, few warps and few blocks an SM,
-// which leave the wait for a tile bare, count against it.
-// Batch 256 fp16, us, one column x eight rows, two x eight (stride 2: two x four): 240 channels 5x5 on 14x14 37.6 34.3, 576 on 7x7
-// 24.3 28.7, 88 3x3 on 28x28 27.2 25.3, 16 3x3 stride 2 112 -> 56 32.6 43.6, 72 3x3 stride 2 56 -> 28 41.9 29.9; 64x112x112x96 89.1
-// 74.4.  (Since then the filter is fetched behind the first copies, all of a channel's values in flight, 2 to 3 us less each: the last
-// one takes 71.2, where 256 threads of one column x eight rows took 84.3.)
-DwShape dw_choose(int N, int C, int OH, int OW, int R, int stride, int es, int sms) {
-  const int V = 16 / es, cv = C / V;
-  const size_t wvec = (size_t)(R * R + (es == 2 ? 1 : 2)) * V * sizeof(float);   // filter and shift (scale) of a channel vector
-  DwShape best{};
-  double least = 1e30;
-  for (int px = es == 2 ? 2 : 1; px >= 1; --px) {
-    const int kp = es == 4 || (px == 2 && stride == 2) ? 4 : 8, th = es == 4 ? 8 : kp, ih = (th - 1) * stride + R;
-    const int most = es == 4 ? kMaxThreads<float> : kMaxThreads<__half>, slots = most * px / 2;   // 16-byte vectors of a tile
-    const int by_regs = es == 4 ? most * (R == 3 ? 3 : 2) : px == 2 ? most * (R == 3 ? 4 : 3) : most * (R == 3 ? 6 : 4);
-    const double loads = (double)((kp - 1) * stride + R) * ((px - 1) * stride + R) / (kp * px);
-    for (int v = std::min(32, cv); v >= 2; --v) {        // ties go to the wider chunk (longer contiguous runs in memory)
-      const int widest = slots / v / px * px, fewest = (OW + widest - 1) / widest, chunks = (cv + v - 1) / v, bytes = v * 16;
-      // the 128 bytes that half a warp reads are `groups` pixels, px * stride pixels apart
-      const int groups = bytes >= 128 ? 1 : 128 / bytes, step = px * stride * bytes % 128;
-      const int apart = step == 0 ? 1 : 128 / (step & -step), ways = groups > apart ? groups / apart : 1;
-      const double per_output = 2.0 * R * R + (es == 2 ? 4.0 : 0.0) * loads + 2.0 * ways * loads + 8.0;
-      for (int tiles = fewest; tiles <= fewest + (es == 2 ? 2 : 0); ++tiles) {
-        const int t = ((OW + tiles - 1) / tiles + px - 1) / px * px, iw = (t - 1) * stride + R;
-        if (iw > 256) continue;
-        const size_t stage = ((size_t)iw * ih * bytes + 127) & ~(size_t)127;
-        if (2 * stage + v * wvec > 200 * 1024) continue;
-        const int threads = (t * v * 2 / px + 31) & ~31, regs_fit = std::min(by_regs / threads, 16);
-        const auto fit = [&](int stages) { return std::min(regs_fit, (int)((220 * 1024) / (stages * stage + v * wvec + 1024))); };
-        const int per_sm = fit(2);
-        if (per_sm < 1) continue;
-        double cost;
-        if (es == 4) {
-          // the share of idle threads and outputs; stages so large that fewer than three blocks fit an SM
-          double use = (double)cv / (chunks * v) * OW / (((OW + t - 1) / t) * t) * (t * v) / slots;
-          use *= 0.5 + 0.5 * (t * stride) / iw;
-          if (v < 8) use *= 0.5 + 0.5 * v / 8.0;
-          const size_t need = 2 * stage + v * wvec;
-          if (need > 72 * 1024) use *= need > 110 * 1024 ? 0.6 : 0.9;
-          cost = 1.0 / use;
-        } else {
-          // blocks' worth of work that the busiest SM does one after another
-          const double turns = std::ceil((double)N * ((OH + th - 1) / th) * ((OW + t - 1) / t) * chunks / sms);
-          const double beside = std::min((double)per_sm, turns);
-          cost = per_output * kp * px * threads * turns * (1.0 + 3.3 * 32.0 / (beside * threads)) * (1.0 + 0.15 / beside);
-          cost /= 0.5 + 0.5 * (t * stride) / iw;
-          if (v < 16) cost /= 0.94 + 0.06 * v / 16.0;
-          if (v < 8) cost /= 0.5 + 0.5 * v / 8.0;
-        }
-        if (cost < least * (1.0 - 1e-9)) {
-          least = cost;
-          // a third stage where it costs no block of an SM (fp32, of a large patch, 56x56x72 at stride 2: 83 us with it, 79 without)
-          const int stages = fit(3) == per_sm && (es == 2 || per_sm > 1) ? 3 : 2;
-          best = DwShape{v, t, px, kp, threads, stages, per_sm, stages * stage + v * wvec};
-        }
-      }
-    }
-  }
-  return best;
-}
-// The same, kept for the layers a thread asks for in turn: choosing takes longer than a launch.
-const DwShape& dw_shape(int N, int C, int OH, int OW, int R, int stride, int es, int sms) {
-  struct Kept { int key[8]; DwShape shape; };
-  thread_local Kept kept[64] = {};
-  Kept& k = kept[((unsigned)C * 31u + (unsigned)OW * 7u + (unsigned)(R * 2 + stride) * 5u + (unsigned)es + (unsigned)N * 3u) % 64u];
-  const int key[8] = {N, C, OH, OW, R, stride, es, sms};
-  if (!std::equal(key, key + 8, k.key)) {
-    k.shape = dw_choose(N, C, OH, OW, R, stride, es, sms);
-    std::copy(key, key + 8, k.key);
-  }
-  return k.shape;
-}
-
 }  // namespace
 
 bool depthwise_tma_supported(DType dt, int N, int H, int W, int C, int R, int S, int stride, int pad) {
@@ -423,7 +339,7 @@ cudaError_t launch_depthwise_tma(const void* x, const void* w, DType w_dt, const
   const int OH = (H + 2 * pad - R) / stride + 1, OW = (W + 2 * pad - S) / stride + 1;
   DwParams p{};
   const int sms = sm_count > 0 ? sm_count : 148;
-  const DwShape d = dw_shape(N, C, OH, OW, R, stride, es, sms);
+  const dw::Shape d = dw::shape_of(N, C, OH, OW, R, stride, es, sms);
   if (d.cbv == 0) return cudaErrorInvalidValue;
   const int tw = d.tw, cbv = d.cbv, px = d.px, kp = d.kp, th = es == 2 ? kp : 8, IH = (th - 1) * stride + R, IW = (tw - 1) * stride + R;
   p.tw = tw; p.cbv = cbv;
