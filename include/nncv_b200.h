@@ -184,11 +184,13 @@ int nncv_b200_activation_bytes(size_t* arena_bytes, size_t* unshared_bytes);
 /* Per-launch timing with CUDA events on the launching stream (off by default).  The reference
  * only has wall-clock timers around the whole forward (examples/Res18/main.cpp:95-99). */
 typedef struct {
-  int kind;      /* 0 tcgen05 implicit GEMM (gathered A), 1 fp32 CUDA-core conv, 2 tcgen05 3x3 shifted-view
+  int kind;      /* 0 tcgen05 implicit GEMM (gathered A), 1 fp32 convolution, 2 tcgen05 3x3 shifted-view
                     conv, 3 memory-bound helper, 4 fused stem conv + max-pool, 5 tcgen05 implicit GEMM
                     (TMA-fed A), 6 Winograd F(2x2,3x3) (all three stages), 7 shifted-view conv on CTA pairs */
   int M, N, K;   /* GEMM view of the launch (helpers: elements, channels, 0) */
-  int bn;        /* N tile (kind 0); helper id (kind 3) */
+  int bn;        /* N tile (kind 0; kind 1 on the CUDA cores); N tile * 10 + CTAs of a tile (kind 1 on the
+                    tensor cores); N tile * 10 + 1 with resident weights, + 2 on CTA pairs (kind 5); helper
+                    id (kind 3) */
   double flops;  /* algorithmic: 2*M*N*K with K = C*R*S (direct-convolution count) */
   double bytes;  /* algorithmic: each operand and result once */
   float ms;      /* device time of the launch */
@@ -274,12 +276,14 @@ int nncv_b200_conv_run_fused(nncv_b200_conv* c, nncv_b200_conv* branch, const vo
                              const float* shift, const float* scale_branch,
                              const float* shift_branch, int relu, void* stream);
 
-/* Force the tile configuration (N tile 64/128/256; algo 2: sub-tiles per CTA 1/2/4; resident: 1 =
+/* Force the tile configuration (N tile 32/64/128/256; algo 2: sub-tiles per CTA 1/2/4; resident: 1 =
  * weights resident in shared memory, 0 = streamed; algo 2 with Kout a multiple of bn: 2 = the
  * CTA-pair kernel on tcgen05.mma.cta_group::2 (bn columns per pair), 3 = the same with the items of
  * a mostly empty last round sliced by columns; algo 0 with Kout a multiple of bn = 128 or 256:
- * 2 = the per-tap kernel on CTA pairs); bn = 0 restores the built-in choice.  A tuning
- * and test hook with no counterpart in the reference. */
+ * 2 = the per-tap kernel on CTA pairs); bn = 32: the kernel of 64 x 32 tiles for small batches,
+ * whatever mt and resident say; bn = 0 restores the built-in choice.  F32 on the tensor cores: bn = 32,
+ * 64 or 128, mt = CTAs that share a tile's reduction (1, 2, 4 or 8); what does not fit the layer is
+ * chosen as without it.  A tuning and test hook with no counterpart in the reference. */
 int nncv_b200_conv_set_tile(nncv_b200_conv* c, int bn, int mt, int resident);
 
 /* The ResNet stem in one kernel (tests/Nets/Res18.mlir:118-151): tensor.pad 3 + 7x7 stride-2

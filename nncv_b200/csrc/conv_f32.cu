@@ -1023,48 +1023,66 @@ cudaError_t launch_avgpool_planes(const void* src, void* dst, int N, int HW, int
 
 bool conv_f32_supported(int C, int Kout, int tw_stride) { return C % 8 == 0 && Kout % 4 == 0 && tw_stride <= 256; }
 
+// A pointwise convolution is a matrix of N * H * W rows: no tile straddles an image's border (a 7 x 7 map fills 49 of the 64 slots of
+// its half tile).
+static bool as_matrix(ConvF32Args* a) {
+  if (a->stem || a->R != 1 || a->S != 1 || a->stride != 1 || a->pad != 0 || (long long)a->N * a->H * a->W >= (1LL << 30)) return false;
+  a->W = a->OW = a->N * a->H * a->W;
+  a->N = a->H = a->OH = 1;
+  return true;
+}
+static void f32_tile(const ConvF32Args& a, bool matrix, int bn, int* tw, int* th, int* tn) {
+  if (bn == kSN) {
+    conv_small_tile(a.N, a.OH, a.OW, tw, th, tn);
+  } else if (matrix) {
+    *tw = 128; *th = *tn = 1;
+  } else {
+    tconv_tile(a.N, a.OH, a.OW, tw, th, tn);
+  }
+}
+// Clusters of s CTAs with tiles of bn columns that run at once.  Fewer fit the GPU than its SMs would hold (they do not cross GPC
+// borders), so the runtime is asked.
+static int clusters_that_fit(int bn, int s, int sms) {
+  static const ClusterFit small = cluster_fit(conv_f32_small_kernel, kSThreads, kSSmem, sms);
+  static const ClusterFit wide = cluster_fit(conv_f32_kernel<64>, kThreads, Ring<64>::kSmem, sms);
+  static const ClusterFit wider = cluster_fit(conv_f32_kernel<128>, kThreads, Ring<128>::kSmem, sms);
+  return bn == kSN ? small.of[s] : bn == 64 ? wide.of[s] : wider.of[s];
+}
+
 // Tile width and the CTAs of a cluster that share a tile's reduction: the pair with the least rounds x time.  A block of 64
 // channels takes about 1560 clocks with 64 columns and 2000 with 128 when every SM works (both bound by L2 -> shared
 // memory, 46 to 48 bytes a clock and SM: 72 and 96 KB; 3x3 filters of 256 and 512 channels at batch 64); everything else about
-// 4700 and 12000 a tile (the wide tile is finished in two passes), a split 1500 more.  Clusters of sixteen were slower at batch 1 than clusters of eight (21 us
-// against 15 for a layer of 256 channels on 16 x 16 pixels).  Fewer clusters fit the GPU than its SMs would hold (they do not
-// cross GPC borders), so the runtime is asked.
-template <int BN>
-static int clusters_that_fit(int s, int sms) {
-  static const ClusterFit fit = cluster_fit(conv_f32_kernel<BN>, kThreads, Ring<BN>::kSmem, sms);
-  return fit.of[s];
-}
-
-static double pick_tile(long long m_tiles, int Kout, int kb_all, int sms, int* bn, int* splits) {
+// 4700 and 12000 a tile (the wide tile is finished in two passes), a split 1500 more.  Clusters of sixteen were slower at batch 1
+// than clusters of eight (21 us against 15 for a layer of 256 channels on 16 x 16 pixels).
+void conv_f32_choose(ConvF32Args* args) {
+  ConvF32Args a = *args;
+  const bool matrix = as_matrix(&a);
+  const int kb_all = (a.stem ? 4 : a.R * a.S) * (a.stem ? 1 : (a.C + 63) / 64), stride = a.stem ? 1 : a.stride, sms = a.sm_count > 0 ? a.sm_count : 148;
   double best = 1e30;
-  for (int b = 64; b <= (Kout > 64 ? 128 : 64); b *= 2)
-    for (int s = 1; s <= 8 && s <= kb_all; s *= 2) {
-      const int slots = b == 64 ? clusters_that_fit<64>(s, sms) : clusters_that_fit<128>(s, sms);
-      const long long tiles = m_tiles * ((Kout + b - 1) / b);
-      const double rounds = (double)((tiles + slots - 1) / slots);
-      const double t = rounds * (((kb_all + s - 1) / s) * (b == 64 ? 1560.0 : 2000.0) + (b == 64 ? 4700.0 : 12000.0)) + 5000.0 + (s > 1 ? 1500.0 : 0.0);
-      if (t < best) { best = t; *bn = b; *splits = s; }
+  for (int forced = 2; forced >= 0 && best == 1e30; --forced)   // what was asked for, the tile alone, neither
+    for (int b : {64, 128, kSN}) {
+      if ((b == 128 && a.Kout <= 64) || (forced >= 1 && a.bn != 0 && b != a.bn)) continue;
+      int tw, th, tn;
+      f32_tile(a, matrix, b, &tw, &th, &tn);
+      if (b == kSN && (tw > th ? tw : th) * stride > 256) continue;
+      const long long tiles = (long long)((a.OW + tw - 1) / tw) * ((a.OH + th - 1) / th) * ((a.N + tn - 1) / tn) * ((a.Kout + b - 1) / b);
+      for (int s = 1; s <= 8 && s <= kb_all; s *= 2) {
+        if (forced == 2 && a.splits != 0 && s != a.splits) continue;
+        const int slots = clusters_that_fit(b, s, sms), blocks = (kb_all + s - 1) / s;
+        const double rounds = (double)((tiles + slots - 1) / slots);
+        // 64 x 32 tiles: about 620 clocks a block, 4500 besides, 1000 for sending
+        const double t = b == kSN ? rounds * (blocks * 620.0 + 4500.0 + (s > 1 ? 1000.0 : 0.0))
+                                  : rounds * (blocks * (b == 64 ? 1560.0 : 2000.0) + (b == 64 ? 4700.0 : 12000.0)) + 5000.0 + (s > 1 ? 1500.0 : 0.0);
+        if (t < best) { best = t; args->bn = b; args->splits = s; }
+      }
     }
-  return best;
-}
-
-// Small tiles where the modelled time of all rounds is less: about 620 clocks a block, 4500 besides, 1000 for sending.
-static bool pick_small(long long tiles, int kb_all, int sms, double other, int* splits) {
-  static const ClusterFit fit = cluster_fit(conv_f32_small_kernel, kSThreads, kSSmem, sms);
-  bool found = false;
-  for (int s = 1; s <= 8 && s <= kb_all; s *= 2) {
-    const double rounds = (double)((tiles + fit.of[s] - 1) / fit.of[s]);
-    const double t = rounds * ((kb_all + s - 1) / s * 620.0 + 4500.0 + (s > 1 ? 1000.0 : 0.0));
-    if (t < other) { other = t; *splits = s; found = true; }
-  }
-  return found;
 }
 
 template <int BN>
 static cudaError_t launch_f32_cfg(const CUtensorMap& tm, const F32Params& p, int sms, cudaStream_t stream) {
   cudaError_t e = cudaFuncSetAttribute(conv_f32_kernel<BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Ring<BN>::kSmem);
   if (e != cudaSuccess) return e;
-  const int slots = clusters_that_fit<BN>(p.splits, sms);
+  const int slots = clusters_that_fit(BN, p.splits, sms);
   const int clusters = p.items < slots ? p.items : slots;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)(clusters * p.splits));
@@ -1106,13 +1124,7 @@ static cudaError_t launch_f32_small(const CUtensorMap& tm, const F32Params& p, c
 cudaError_t launch_conv_f32(const ConvF32Args& args, cudaStream_t stream) {
   ConvF32Args a = args;
   const bool stem = a.stem != 0;
-  // a pointwise convolution is a matrix of N * H * W rows: no tile straddles an image's border (a 7 x 7 map fills 49 of the 64
-  // slots of its half tile)
-  const bool matrix = !stem && a.R == 1 && a.S == 1 && a.stride == 1 && a.pad == 0 && (long long)a.N * a.H * a.W < (1LL << 30);
-  if (matrix) {
-    a.W = a.OW = a.N * a.H * a.W;
-    a.N = a.H = a.OH = 1;
-  }
+  const bool matrix = as_matrix(&a);
   F32Params p{};
   p.wpack = static_cast<const uint8_t*>(a.wpack);
   p.scale = a.scale; p.shift = a.shift;
@@ -1130,28 +1142,19 @@ cudaError_t launch_conv_f32(const ConvF32Args& args, cudaStream_t stream) {
   if (pixels > 0x7fffffffLL) return cudaErrorInvalidValue;
   p.res_plane = p.out_plane = pixels * a.Kout;
   int tw, th, tn;
-  tconv_tile(a.N, a.OH, a.OW, &tw, &th, &tn);
-  if (matrix) { tw = 128; th = tn = 1; }
+  f32_tile(a, matrix, 64, &tw, &th, &tn);
   if (!conv_f32_supported(stem ? 64 : a.C, a.Kout, (tw > th ? tw : th) * p.stride)) return cudaErrorInvalidValue;
   if ((reinterpret_cast<uintptr_t>(a.in) & 15) || (reinterpret_cast<uintptr_t>(a.out) & 15) || (reinterpret_cast<uintptr_t>(a.residual) & (a.res_f32 ? 15 : 7)) ||
       ((a.out_f32 || a.res_f32) && a.ldo % 4 != 0))
     return cudaErrorMisalignedAddress;
+  conv_f32_choose(&a);
+  const int bn = a.bn, sms = a.sm_count > 0 ? a.sm_count : 148;
+  f32_tile(a, matrix, bn, &tw, &th, &tn);
+  p.splits = a.splits;
   p.tw = tw; p.th = th; p.tn = tn;
   p.tiles_x = (a.OW + tw - 1) / tw; p.tiles_y = (a.OH + th - 1) / th;
-  const long long tiles_n = (a.N + tn - 1) / tn;
-  const int sms = a.sm_count > 0 ? a.sm_count : 148;
-  const long long m_tiles = (long long)p.tiles_x * p.tiles_y * tiles_n;
-  int bn = 64, sw, sh, sn;
-  conv_small_tile(a.N, a.OH, a.OW, &sw, &sh, &sn);
-  const long long small_m = (long long)((a.OW + sw - 1) / sw) * ((a.OH + sh - 1) / sh) * ((a.N + sn - 1) / sn);
-  const double wide = pick_tile(m_tiles, a.Kout, p.taps * p.CB, sms, &bn, &p.splits);
-  if ((sw > sh ? sw : sh) * p.stride <= 256 && pick_small(small_m * ((a.Kout + kSN - 1) / kSN), p.taps * p.CB, sms, wide, &p.splits)) {
-    bn = kSN;
-    p.tw = tw = sw; p.th = th = sh; p.tn = tn = sn;
-    p.tiles_x = (a.OW + tw - 1) / tw; p.tiles_y = (a.OH + th - 1) / th;
-  }
   p.n_tiles = (a.Kout + bn - 1) / bn;
-  const long long items = (bn == kSN ? small_m : m_tiles) * p.n_tiles;
+  const long long items = (long long)p.tiles_x * p.tiles_y * ((a.N + tn - 1) / tn) * p.n_tiles;
   if (items <= 0 || items > 0x7fffffffLL) return cudaErrorInvalidValue;
   p.items = (int)items;
   p.div_tx = epi::fast_div((uint32_t)p.tiles_x); p.div_ty = epi::fast_div((uint32_t)p.tiles_y); p.div_nt = epi::fast_div((uint32_t)p.n_tiles);

@@ -206,9 +206,12 @@ struct ConvF32Args {
   int stem = 0;                     // 7x7 stride-2 pad-3 convolution of the 3-channel input (H, W: the image)
   int N = 0, H = 0, W = 0, C = 0, OH = 0, OW = 0, Kout = 0, R = 1, S = 1, stride = 1, pad = 0;
   int relu = 0;
+  int bn = 0, splits = 0;           // output channels of a tile (32: the 64 x 32 tiles, 64, 128) and CTAs that share its reduction; 0: as modelled
   int sm_count = 0;
   int* error_flag = nullptr;
 };
+// Fills in bn and splits where they are 0 or what the layer cannot take; launch_conv_f32 calls it too.
+void conv_f32_choose(ConvF32Args* a);
 bool conv_f32_supported(int C, int Kout, int tw_stride);
 cudaError_t launch_conv_f32(const ConvF32Args& a, cudaStream_t stream);
 size_t packed_planes_bytes(int Kout, int C, int taps);   // stem: C = 64, taps = 4

@@ -3,21 +3,39 @@ import numpy as np
 import pytest
 import torch
 
+from nncv_b200 import runtime as rt
 from nncv_b200._lib import F32, check, lib
+from nncv_b200.split_params import random_input, random_state_dict, to_flat_array
 from oracle import binding as ob
 from tests import gpu_util as G
 
 pytestmark = pytest.mark.gpu
 
 
+def _tile_of(run):
+    """What `run` returns, and tile * 10 + CTAs of a tile of the tensor-core launch that it made."""
+    check(lib().nncv_b200_profile(1))
+    try:
+        y = run()
+        made = [r["bn"] for r in rt.profile_records() if r["kind"] == 1]
+    finally:
+        check(lib().nncv_b200_profile(0))
+    assert len(made) == 1
+    return y, made[0]
+
+
+@pytest.mark.parametrize("splits", [1, 2, 4, 8])
 @pytest.mark.parametrize("case", [
-    # n, c, h, w, k, r, stride: one block; two of a CTA; more blocks than stages; split over 2, 4 and 8; ragged channels, columns, maps
-    (1, 64, 8, 8, 32, 1, 1), (1, 72, 3, 5, 36, 1, 1), (1, 64, 56, 56, 64, 3, 1), (2, 128, 28, 28, 128, 3, 1), (1, 256, 14, 14, 256, 3, 1),
-    (1, 512, 8, 8, 512, 3, 1), (3, 512, 7, 7, 100, 3, 2), (1, 8, 9, 9, 4, 3, 1), (1, 2048, 7, 7, 512, 1, 1), (5, 40, 6, 10, 240, 1, 1), (1, 1024, 1, 1, 1000, 1, 1),
+    # n, c, h, w, k, r, stride: one block (one CTA), two; more blocks than stages; ragged channels, columns, maps
+    (1, 64, 8, 8, 128, 1, 1), (1, 72, 3, 5, 36, 1, 1), (1, 64, 56, 56, 64, 3, 1), (2, 128, 28, 28, 128, 3, 1), (1, 256, 14, 14, 256, 3, 1),
+    (1, 512, 8, 8, 512, 3, 1), (3, 512, 7, 7, 100, 3, 2), (1, 8, 9, 9, 4, 3, 1), (1, 2048, 7, 7, 512, 1, 1), (5, 40, 6, 10, 240, 3, 1), (1, 1024, 1, 1, 1000, 1, 1),
 ])
 @pytest.mark.parametrize("res,relu", [(True, True), (False, False)])
-def test_small_tiles(case, res, relu):
+def test_small_tiles(case, splits, res, relu):
     n, c, h, w, k, r, stride = case
+    blocks = r * r * -(-c // 64)
+    if splits > blocks:
+        pytest.skip("more CTAs than blocks of 64 channels")
     g = np.random.default_rng(sum(case))
     x = g.standard_normal((n, c, h, w)).astype(np.float32)
     wt = (g.standard_normal((k, c, r, r)) * np.sqrt(2.0 / (c * r * r))).astype(np.float32)
@@ -26,7 +44,9 @@ def test_small_tiles(case, res, relu):
     rs = g.standard_normal((n, k, oh, ow)).astype(np.float32) if res else None
     conv = G.Conv(wt, stride, r // 2, F32)
     try:
-        y, _ = conv.run(x, scale, shift, rs, relu)
+        check(lib().nncv_b200_conv_set_tile(conv.h, 32, splits, 0))
+        (y, _), made = _tile_of(lambda: conv.run(x, scale, shift, rs, relu))
+        assert made == 320 + splits
         again, _ = conv.run(x, scale, shift, rs, relu)
     finally:
         conv.close()
@@ -38,6 +58,42 @@ def test_small_tiles(case, res, relu):
     bound = 2.0 ** -23 + 2.0 ** -24 * (np.sqrt(4 * r * r * np.ceil(c / 64)) + 8 + 3)
     assert np.isfinite(y).all() and G.rel_l2(y, ref) <= bound
     assert lib().nncv_b200_device_status() == 0
+
+
+@pytest.mark.parametrize("bn,splits", [(64, 1), (64, 8), (128, 2), (32, 4), (32, 8), (32, 16), (256, 1)])
+def test_a_forced_tile_that_does_not_fit_is_the_modelled_one(bn, splits):
+    """Tiles of 64 and 128 columns are forced the same way; more CTAs than there are blocks, or a tile there is none of: as modelled."""
+    g = np.random.default_rng(1)
+    x, wt = g.standard_normal((1, 128, 9, 7)).astype(np.float32), g.standard_normal((160, 128, 1, 1)).astype(np.float32)
+    conv = G.Conv(wt, 1, 0, F32)
+    try:
+        (want, _), modelled = _tile_of(lambda: conv.run(x))
+        check(lib().nncv_b200_conv_set_tile(conv.h, bn, splits, 0))
+        (y, _), made = _tile_of(lambda: conv.run(x))
+    finally:
+        conv.close()
+    if bn == 256:
+        assert made == modelled
+    else:
+        assert made // 10 == bn and (made % 10 == splits if splits <= 2 else made % 10 in (1, 2))
+    assert G.rel_l2(y, want) <= 1e-6
+
+
+@pytest.mark.parametrize("h,w", [(64, 64), (97, 75)])
+def test_a_network_of_one_image_on_small_tiles(h, w):
+    """Residuals and results as planes: most layers of ResNet-18 take the small tiles at one image, blocks with residual among them."""
+    blob = to_flat_array(18, random_state_dict(18, 0)).blob()
+    rt.load_blob("resnet18", blob, F32)
+    x, y = random_input(1, h, w, 3, "normal"), np.zeros((1, 1000), np.float32)
+    rt.forward(y, x)
+    rt.profile(True)
+    rt.forward(y, x)
+    layers = [r for r in rt.profile_records() if r["kind"] == 1]
+    rt.profile(False)
+    rt.unload()
+    small = [r for r in layers if r["bn"] // 10 == 32]
+    assert len(small) >= len(layers) // 2 and any(r["bn"] % 10 > 1 for r in small)
+    assert G.rel_l2(y, ob.resnet_forward(18, x, blob)) <= 1e-5
 
 
 def test_small_tiles_have_no_bias():

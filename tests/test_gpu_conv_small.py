@@ -1,4 +1,8 @@
 """The convolutions on 64 x 32 tiles (small batches) against the 128-row kernels, bit for bit, and against the oracle."""
+import os
+import subprocess
+import sys
+
 import numpy as np
 import pytest
 import torch
@@ -118,3 +122,54 @@ def test_branch_scale_and_shift_on_any_float_boundary(bn):
         main.close()
         branch.close()
     assert not got[0][0].isnan().any() and torch.equal(got[0][0], got[1][0]) and torch.equal(got[0][1], got[1][1])
+
+
+FORWARD = """
+import sys
+sys.path.insert(0, {root!r})
+import numpy as np
+from nncv_b200 import runtime as rt
+from nncv_b200.split_params import random_input, random_state_dict, to_flat_array
+from tests import plan_util as P
+name, compute, silu, out = sys.argv[1], int(sys.argv[2]), sys.argv[3] == "1", sys.argv[4]
+if name == "mobilenetv3":
+    text = open({root!r} + "/tests/golden/mobilenetv3_from_mlir.plan").read()
+    if silu:
+        text = "\\n".join(l.replace("act=3", "act=5") if l.startswith("conv") else l for l in text.splitlines())
+    total, classes, nodes = P.parse_plan_text(text)
+    rt.load_blob("plan:" + text, P.random_blob(total, nodes, seed=4), compute)
+else:
+    rt.load_blob(name, to_flat_array(18, random_state_dict(18, 0)).blob(), compute)
+x = random_input(2, 97, 75, 5, "normal")
+y = np.zeros((2, 1000), np.float32)
+rt.forward(y, x)
+rt.profile(True)
+rt.forward(y, x)
+tiles = [r["bn"] for r in rt.profile_records() if r["kind"] == 5]
+rt.profile(False)
+np.savez(out, y=y, small=sum(t == 320 for t in tiles), launches=len(tiles))
+"""
+
+
+@pytest.mark.parametrize("name,compute,silu", [("resnet18", F16, False), ("resnet18", BF16, False), ("mobilenetv3", F16, False), ("mobilenetv3", F16, True)])
+def test_networks_on_small_tiles_throughout(tmp_path, name, compute, silu):
+    """Every convolution of a network on 64 x 32 tiles, by a cache of decisions that says so, against 64-column tiles: bit for bit.
+    ResNet-18 has maps with pad slots, residuals, branches and fp32 logits; the mobile network fused hard-swish (or SiLU) and odd
+    channel counts."""
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    cache, got = tmp_path / "tune.txt", {}
+    for kind in ("timed", "9 32 1 0", "5 64 1 0"):
+        if kind != "timed":
+            # (a launch fused with a branch exists for 128 columns)
+            cache.write_text("".join(f"{k} = {kind if not (k.split()[-2] in ('res2', 'res3') and kind[0] == '5') else '5 128 1 0'}\n" if k.startswith("conv c") else f"{k} = {v}\n"
+                                     for k, v in (line.split(" = ") for line in decisions)))
+        out = str(tmp_path / "out.npz")
+        r = subprocess.run([sys.executable, "-c", FORWARD.format(root=root), name, str(compute), str(int(silu)), out], capture_output=True, text=True,
+                           timeout=600, env=dict(os.environ, NNCV_B200_TUNE_CACHE=str(cache)))
+        assert r.returncode == 0, r.stderr[-2000:]
+        if kind == "timed":
+            decisions = cache.read_text().splitlines()
+        got[kind] = dict(np.load(out))
+    small, wide = got["9 32 1 0"], got["5 64 1 0"]
+    assert small["launches"] > 15 and small["small"] == small["launches"] and wide["small"] == 0
+    assert np.isfinite(small["y"]).all() and np.array_equal(small["y"], wide["y"])
