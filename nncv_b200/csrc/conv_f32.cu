@@ -1049,11 +1049,17 @@ static int clusters_that_fit(int bn, int s, int sms) {
   return bn == kSN ? small.of[s] : bn == 64 ? wide.of[s] : wider.of[s];
 }
 
-// Tile width and the CTAs of a cluster that share a tile's reduction: the pair with the least rounds x time.  A block of 64
-// channels takes about 1560 clocks with 64 columns and 2000 with 128 when every SM works (both bound by L2 -> shared
-// memory, 46 to 48 bytes a clock and SM: 72 and 96 KB; 3x3 filters of 256 and 512 channels at batch 64); everything else about
-// 4700 and 12000 a tile (the wide tile is finished in two passes), a split 1500 more.  Clusters of sixteen were slower at batch 1
-// than clusters of eight (21 us against 15 for a layer of 256 channels on 16 x 16 pixels).
+// Tile width and the CTAs of a cluster that share a tile's reduction: the pair with the least rounds x time, in clocks.  Wide tiles: a
+// block of 64 channels takes about 1560 with 64 columns and 2000 with 128 when every SM works (both bound by L2 -> shared memory, 46 to
+// 48 bytes a clock and SM: 72 and 96 KB; 3x3 filters of 256 and 512 channels at batch 64); everything else about 4700 and 12000 a tile
+// (the widest is finished in two passes), a split 1500 more.  Clusters of sixteen were slower at batch 1 than clusters of eight (21 us
+// against 15 for a layer of 256 channels on 16 x 16 pixels).
+// 64 x 32 tiles: 820 a block, 6000 besides, 2600 for sending, beside a launch of wide ones that starts 7000 later.  Fitted to 376 layers
+// of 1 to 64 images (ResNet-18's and ResNet-50's, and random ones), each at every tile and split: the choice takes 0.7 % more than the
+// fastest, and 6 layers take 3 % more than on wide tiles.  (With 620, 4500, 1000 and 5000, which leave the small tiles' launch out, it
+// was 43 layers: 11x12x8x168 -> 192 3x3 22.4 us for 15.8.)  On either side of the line, us (64 x 32, wide): 14x14x256 -> 256 3x3 of one
+// image 11.0 13.4, of two 14.9 16.7, of three 21.2 17.1; 28x28x128 -> 256 3x3 stride 2 of two 11.4 13.4, of four 14.2 14.5;
+// 7x7x512 -> 2048 of two 9.1 10.9, of three 15.5 12.6.
 void conv_f32_choose(ConvF32Args* args) {
   ConvF32Args a = *args;
   const bool matrix = as_matrix(&a);
@@ -1070,9 +1076,8 @@ void conv_f32_choose(ConvF32Args* args) {
         if (forced == 2 && a.splits != 0 && s != a.splits) continue;
         const int slots = clusters_that_fit(b, s, sms), blocks = (kb_all + s - 1) / s;
         const double rounds = (double)((tiles + slots - 1) / slots);
-        // 64 x 32 tiles: about 620 clocks a block, 4500 besides, 1000 for sending
-        const double t = b == kSN ? rounds * (blocks * 620.0 + 4500.0 + (s > 1 ? 1000.0 : 0.0))
-                                  : rounds * (blocks * (b == 64 ? 1560.0 : 2000.0) + (b == 64 ? 4700.0 : 12000.0)) + 5000.0 + (s > 1 ? 1500.0 : 0.0);
+        const double t = b == kSN ? rounds * (blocks * 820.0 + 6000.0 + (s > 1 ? 2600.0 : 0.0))
+                                  : rounds * (blocks * (b == 64 ? 1560.0 : 2000.0) + (b == 64 ? 4700.0 : 12000.0)) + 7000.0 + (s > 1 ? 1500.0 : 0.0);
         if (t < best) { best = t; args->bn = b; args->splits = s; }
       }
     }

@@ -60,6 +60,24 @@ def test_small_tiles(case, splits, res, relu):
     assert lib().nncv_b200_device_status() == 0
 
 
+@pytest.mark.parametrize("case,small", [
+    # two rounds of 64 x 32 tiles, or one that is slower than wide tiles that share their reduction: 3 to 41 % slower
+    ((11, 168, 12, 8, 192, 3, 1), False), ((2, 112, 22, 67, 416, 3, 1), False), ((50, 32, 10, 59, 24, 3, 1), False),
+    ((4, 64, 56, 56, 128, 1, 2), False), ((12, 1024, 14, 14, 256, 1, 1), False),
+    # 12 to 30 % faster on 64 x 32 tiles
+    ((1, 256, 14, 14, 256, 3, 1), True), ((2, 512, 7, 7, 2048, 1, 1), True), ((1, 512, 28, 28, 128, 1, 1), True), ((1, 256, 56, 56, 64, 1, 1), True),
+])
+def test_small_tiles_are_taken_where_they_are_faster(case, small):
+    """The lines between tile widths, at layers a good way from them (a GPU of 148 SMs)."""
+    n, c, h, w, k, r, stride = case
+    conv = G.Conv(np.ones((k, c, r, r), np.float32), stride, r // 2, F32)
+    try:
+        _, made = _tile_of(lambda: conv.run(np.zeros((n, c, h, w), np.float32)))
+    finally:
+        conv.close()
+    assert (made // 10 == 32) == small
+
+
 @pytest.mark.parametrize("bn,splits", [(64, 1), (64, 8), (128, 2), (32, 4), (32, 8), (32, 16), (256, 1)])
 def test_a_forced_tile_that_does_not_fit_is_the_modelled_one(bn, splits):
     """Tiles of 64 and 128 columns are forced the same way; more CTAs than there are blocks, or a tile there is none of: as modelled."""
