@@ -759,8 +759,13 @@ int conv_run(nncv_b200_conv* c, const void* in, Layout in_l, void* out, Layout o
             for (int bn : {128, 256})
               if (c->Kout % bn == 0) cand.push_back(ConvChoice{8, bn, 1, 0});   // CTA pairs
         }
-        // (with more than two tiles an SM the 128-row kernels were faster throughout)
-        if (tc_ok && conv_small_tiles(N, OH, OW, c->Kout) <= 2LL * g_dev.sm_count) cand.push_back(ConvChoice{9, kSmallBN, 1, 0});
+        // 64 x 32 tiles: with more than two an SM the 128-row kernels were faster throughout.  The tiles of the shape that is launched: a
+        // fully connected layer is one matrix (as images of one pixel 128 x 1000 would count 512 tiles, of 64)
+        TconvArgs shape;
+        shape.N = N; shape.H = H; shape.W = W; shape.OH = OH; shape.OW = OW; shape.R = c->R; shape.S = c->S; shape.stride = c->stride; shape.pad = c->pad;
+        shape.in_l = in_l; shape.out_l = out_l;
+        if (!fb) pointwise_as_matrix(&shape);
+        if (tc_ok && conv_small_tiles(shape.N, shape.OH, shape.OW, c->Kout) <= 2LL * g_dev.sm_count) cand.push_back(ConvChoice{9, kSmallBN, 1, 0});
         cudaEvent_t e0, e1;
         CU(cudaEventCreate(&e0));
         CU(cudaEventCreate(&e1));

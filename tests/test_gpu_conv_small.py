@@ -173,3 +173,30 @@ def test_networks_on_small_tiles_throughout(tmp_path, name, compute, silu):
     small, wide = got["9 32 1 0"], got["5 64 1 0"]
     assert small["launches"] > 15 and small["small"] == small["launches"] and wide["small"] == 0
     assert np.isfinite(small["y"]).all() and np.array_equal(small["y"], wide["y"])
+
+
+CANDIDATES = """
+import sys
+sys.path.insert(0, {root!r})
+import numpy as np
+from nncv_b200._lib import F16
+from tests import gpu_util as G
+n, c, h, w, k = map(int, sys.argv[1:])
+conv = G.Conv(np.ones((k, c, 1, 1), np.float32), 1, 0, F16)
+conv.run(np.ones((n, c, h, w), np.float32))
+conv.close()
+"""
+
+
+@pytest.mark.parametrize("n,c,h,w,k,timed", [
+    (128, 64, 1, 1, 1000, True), (5, 64, 7, 7, 512, True),     # one matrix of 64 tiles (as images of one pixel 512); the same of 7 x 7
+    (64, 64, 7, 7, 512, False), (2048, 64, 1, 1, 1000, False),
+])
+def test_the_launched_shape_decides_whether_small_tiles_are_timed(n, c, h, w, k, timed):
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    env = dict(os.environ, NNCV_B200_LOG="2")
+    env.pop("NNCV_B200_TUNE_CACHE", None)
+    r = subprocess.run([sys.executable, "-c", CANDIDATES.format(root=root), *map(str, (n, c, h, w, k))], env=env, capture_output=True, text=True, timeout=600)
+    assert r.returncode == 0, r.stderr[-2000:]
+    log = r.stdout + r.stderr
+    assert "kernel 5 tile 64" in log and ("kernel 9 tile 32" in log) == timed
