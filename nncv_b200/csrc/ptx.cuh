@@ -297,7 +297,6 @@ __device__ __forceinline__ bool warp_wait(uint32_t bar, uint32_t parity, volatil
   return warp_all(mbar_wait_abortable(bar, parity, abort_flag));
 }
 
-// Arrives on the mbarrier once every tcgen05.mma issued so far by this thread has finished.
 // The same by testing without a pause, for a warp on whose next step a whole chain waits and whose SM has little else to issue.
 __device__ __forceinline__ bool warp_spin(uint32_t bar, uint32_t parity, volatile int* abort_flag) {
   long long t0 = 0;
@@ -314,6 +313,7 @@ __device__ __forceinline__ bool warp_spin(uint32_t bar, uint32_t parity, volatil
     }
   }
 }
+// Arrives on the mbarrier once every tcgen05.mma issued so far by this thread has finished.
 __device__ __forceinline__ void tc_commit(uint32_t bar, uint32_t issue) {
   asm volatile(
       "{\n"
@@ -447,12 +447,13 @@ __device__ __forceinline__ float4 ld_cluster_f4(uint32_t cluster_addr) {
 __device__ __forceinline__ void mbar_arrive_remote(uint32_t cluster_addr) {
   asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
 }
-// The same where nothing but the arrival itself passes between the CTAs (tensor memory that was read and may be written
-// again; the reads are complete, tcgen05.wait::ld).  A release at cluster scope is a memory barrier that waits for all earlier
-// copies and stores of the thread: in the epilogue warps of the CTA pairs 12 % of their time (ResNet-50 at batch 512: 256 -> 1024
-// pointwise with residual on pairs 131 us, now 95, where single CTAs take 103).
-__device__ __forceinline__ void mbar_arrive_remote_relaxed(uint32_t cluster_addr) {
-  asm volatile("mbarrier.arrive.relaxed.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
+// The same where nothing but the arrival itself passes between the CTAs: tensor memory that was read (tcgen05.wait::ld, then
+// tcgen05.fence::before_thread_sync) and may be written again by the MMAs that the arrival's waiter issues after
+// tcgen05.fence::after_thread_sync.  A release at cluster scope is a memory barrier that waits for all earlier copies and stores of the
+// thread: in the epilogue warps of the CTA pairs 12 % of their time (ResNet-50 at batch 512: 256 -> 1024 pointwise with residual on
+// pairs 131 us, now 95, where single CTAs take 103).  The default release, at CTA scope, is none.
+__device__ __forceinline__ void mbar_arrive_remote_cta(uint32_t cluster_addr) {
+  asm volatile("mbarrier.arrive.release.cta.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
 }
 __device__ __forceinline__ bool mbar_try_wait_cluster(uint32_t bar, uint32_t parity) {
   uint32_t ok;

@@ -451,7 +451,7 @@ tconv_kernel(const __grid_constant__ CUtensorMap tm_in, const __grid_constant__ 
         __syncwarp();
         if (lane == 0) {
           if (!PAIR || rank == 0) ptx::mbar_arrive(acc_empty + 8 * ab);
-          else ptx::mbar_arrive_remote_relaxed(ptx::map_to_cta(acc_empty, 0) + 8 * ab);
+          else ptx::mbar_arrive_remote_cta(ptx::map_to_cta(acc_empty, 0) + 8 * ab);
         }
       };
       const int end_j = (i + 1) << spi_log;
