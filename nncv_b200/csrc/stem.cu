@@ -446,7 +446,9 @@ __global__ void __launch_bounds__(kThreads, 1) stem_pool_kernel(const __grid_con
       return all;
     };
     // accumulator c -> scale/shift -> 16 packed pairs; the buffer goes back to the issuers.  (The type is a parameter of the kernel:
-    // tested for each pair, both conversions stood in the loop, ResNet-18's stem at batch 256 114 -> 109 us.)
+    // tested for each pair, both conversions stood in the loop, ResNet-18's stem at batch 256 114 -> 109 us.)  Packed multiply-adds with
+    // the swizzled operand, single ones with plain rows: there packed ones took more registers (a spill with two x tiles) and
+    // longer: 37x225x301 72.0 us, single ones 66.1; 11x512x480 60.9, 55.6.
     auto drain = [&](uint32_t c, uint32_t (&cur)[16]) {
       uint32_t acc[32];
       __syncwarp();
@@ -459,9 +461,14 @@ __global__ void __launch_bounds__(kThreads, 1) stem_pool_kernel(const __grid_con
       for (int h = 0; h < 16; ++h) {
         const float4 s4 = sc[h >> 1], b4 = sh[h >> 1];
         float a, b;
-        epi::unpk(epi::fma2(epi::pk(__uint_as_float(acc[2 * h]), __uint_as_float(acc[2 * h + 1])),
-                            (h & 1) ? epi::pk(s4.z, s4.w) : epi::pk(s4.x, s4.y), (h & 1) ? epi::pk(b4.z, b4.w) : epi::pk(b4.x, b4.y)),
-                  a, b);
+        if constexpr (SW) {
+          epi::unpk(epi::fma2(epi::pk(__uint_as_float(acc[2 * h]), __uint_as_float(acc[2 * h + 1])),
+                              (h & 1) ? epi::pk(s4.z, s4.w) : epi::pk(s4.x, s4.y), (h & 1) ? epi::pk(b4.z, b4.w) : epi::pk(b4.x, b4.y)),
+                    a, b);
+        } else {
+          a = fmaf(__uint_as_float(acc[2 * h]), (h & 1) ? s4.z : s4.x, (h & 1) ? b4.z : b4.x);
+          b = fmaf(__uint_as_float(acc[2 * h + 1]), (h & 1) ? s4.w : s4.y, (h & 1) ? b4.w : b4.y);
+        }
         cur[h] = epi::pack16(a, b, BF16, false);
       }
     };
