@@ -255,7 +255,8 @@ typedef struct nncv_b200_conv nncv_b200_conv;
 nncv_b200_conv* nncv_b200_conv_create(const void* weights, int w_dtype, int Kout, int C, int R,
                                       int S, int stride, int pad, int dtype, int algo);
 void nncv_b200_conv_destroy(nncv_b200_conv* c);
-/* in [N,H,W,Cpad], out/residual [N,OH,OW,Kout], on 16-byte boundaries; scale/shift fp32 [Kout] or NULL.
+/* in [N,H,W,Cpad], out/residual [N,OH,OW,Kout], on 16-byte boundaries (a 16-bit residual with algo 0: 32); scale/shift fp32 [Kout]
+ * on any float's boundary, or NULL.
  * F32 on the tensor cores: a workspace of 6 bytes an input element for the length of the call, in the order of its stream (a
  * captured call keeps its own until the plan is destroyed); such calls of one plan may run on several streams.  algo 1 and 2 keep
  * copies of the tensors in the plan, F32 on the CUDA cores partial sums: order the calls of one plan there. The first call of a shape in 16 bits times kernels and tiles (NNCV_B200_AUTOTUNE=0: it does not) --

@@ -22,14 +22,15 @@
 // The 7x7 stride-2 stem reads row pairs through a tensor map with overlapping strides, as stem.cu does: it becomes a
 // convolution with four taps of 64 "channels".
 //
-// One CTA computes 128 pixels x 64 or 128 output channels.  What bounds it: 72 or 96 KB of planes from L2 per block of 64
-// channels (1560 or 2000 clocks with every SM at work), then the 24 MMAs (1150 or 1540 clocks).  With few pixels (batch 1) a
+// Two kernels.  conv_f32_kernel: one CTA computes 128 pixels x 64 or 128 output channels.  What bounds it: 72 or 96 KB of planes from
+// L2 per block of 64 channels (1560 or 2000 clocks with every SM at work), then the 24 MMAs (1150 or 1540 clocks).  With few pixels a
 // cluster of up to eight CTAs splits the reduction of a tile; each leaves its partial sums in shared memory and finishes
 // its share of the rows from all of them, in rank order, so that the result does not depend on timing.  (The CUDA-core
 // kernel needed a second pass over partial sums in global memory for that, and ran at a fifth of the fp32 rate.)
-//
-// ResNet-18 fp32 against the CUDA-core kernel, from device memory: 1x256 470 -> 233 us, 8x224 1626 -> 452 us.
 // Roles: warp 0 TMA producer, one plane of both operands per ring slot; warp 1 MMA issuer; warps 2-9 epilogue.
+// conv_f32_small_kernel, for one to four images: 64 pixels x 32 output channels, below.  conv_f32_choose takes one by a model of both.
+//
+// ResNet-18 fp32 against the CUDA-core kernel, from device memory: 1x256 470 -> 192 us, 8x224 1626 -> 449 us.
 // Every wait is bounded and abortable; a timed-out wait sets the device status word.
 #include <cuda.h>
 #include <cudaTypedefs.h>
@@ -480,11 +481,13 @@ conv_f32_kernel(const __grid_constant__ CUtensorMap tm_in, const F32Params p) {
 
 // ------------------------------------------------------------------ small batches ----------
 // The same convolution on 64 x 32 tiles, one a CTA, for few pixels.  At one image what bounds a layer is its chain, and most of
-// that of the kernel above is not tensor work: after 2 to 9 blocks of 1550 clocks (its MMAs read 6 KB each, 48 clocks) a CTA of a
-// cluster waits 1000 to 2600 clocks for its peers' word, 2400 for 32 KB of their partial sums and 1600 until all may leave.  Here
-// a block takes 16 MMAs, two products side by side where they share an operand, of 24 to 32 clocks each; four warps copy, whole blocks are handed over, and the partial sums, a quarter
-// as many, are SENT: every CTA stores the rows that a peer finishes into that peer's shared memory and arrives on its barrier, so
-// that nobody reads from a CTA that could leave, and nobody waits for more than its own rows.
+// that of the kernel above is not tensor work: after 2 to 9 blocks, whose MMAs read 6 KB each (48 clocks), a CTA of a cluster waits
+// for its peers' word, for 32 KB of their partial sums and until all may leave.  Here a block takes 16 MMAs, two products side by
+// side where they share an operand, of 24 to 32 clocks each; four warps copy, whole blocks are handed over, and the partial sums,
+// a quarter as many, are SENT: every CTA stores the rows that a peer finishes into that peer's shared memory and arrives on its
+// barrier, so that nobody reads from a CTA that could leave, and nobody waits for more than its own rows.  One image, us, wide tiles
+// and these: 14x14x256 -> 256 3x3 13.4 11.0 (128 CTAs; the tensor pipe 12 % busy), 7x7x512 -> 512 16.1 14.1, 56x56x256 -> 64 pointwise
+// 11.0 8.0; ResNet-18 224 -> 187.
 // The sums are formed as above: each step of 16 channels of the large products rounded to registers, small products in groups; but
 // with fewer CTAs to a tile a sum has more terms one after another, so a block's four steps are added first, and even and odd
 // blocks apart (one chain: 9.5e-8 instead of 7.1e-8 off the result in 64 bits for 64 channels 3x3, where the kernel above split).

@@ -1,20 +1,21 @@
 // Convolutions and fully connected layers of small batches: the implicit GEMM of tconv.cu on 64 x 32 tiles.
 //
 // What bounds a layer of one or a few images is one chain: launch, first copies, R*S*C/64 blocks one after another on a few
-// SMs, epilogue, stores.  A block of a 128 x 64 tile takes 190 clocks, because its MMAs read 6 KB of operands each through the
-// shared-memory port (48 clocks); those of a 64 x 32 tile read 3 KB.  Four times the tiles also spread the weights, of which every
-// CTA brings its own rows from L2, over four times the SMs.  Sums are formed in the order of the other 16-bit kernels (channel
-// block outermost, tap, 16 channels a step), so the results are the same bits and the tile may be chosen by timing.
-// One image, us a layer in a row of launches, 128-row tiles before and this: 512 -> 512 3x3 on 7x7 12.4 9.7, 256 -> 256 on 14x14 8.1
-// 7.0, with the 1x1 branch 256 -> 512 11.8 8.1, 2048 -> 512 pointwise 9.3 7.2, 1024 -> 256 7.1 5.5; a layer of one block takes 4.1
-// either way.  Forwards of one image: ResNet-18 145 -> 114, ResNet-50 317 -> 267, MobileNetV3 273 -> 251; with the epilogue's
-// combinations as functions of their own 99, 227 and (with other kernels' gains) 201.
+// SMs, epilogue, stores (counters of 14x14x256 -> 256 3x3: 32 CTAs, the tensor pipe 13 % busy on the busiest SM, an instruction
+// issued every sixth clock).  The MMAs of a block of a 128 x 64 tile read 6 KB of operands each through the shared-memory port,
+// 48 clocks; those of a 64 x 32 tile read 3 KB.  Four times the tiles also spread the weights, of which every CTA brings its own
+// rows from L2, over four times the SMs.  Sums are formed in the order of the other 16-bit kernels (channel block outermost, tap,
+// 16 channels a step), so the results are the same bits and the tile may be chosen by timing.
+// One image, us a layer in a row of launches, 128-row tiles before and this: 512 -> 512 3x3 on 7x7 12.4 9.7, 256 -> 256 on 14x14
+// 8.1 7.0, with the 1x1 branch 256 -> 512 11.8 8.1, 2048 -> 512 pointwise 9.3 7.2, 1024 -> 256 7.1 5.5; a layer of one block takes
+// 4.1 either way.  Forwards of one image: ResNet-18 141 -> 96, ResNet-50 326 -> 222, MobileNetV3 275 -> 200.
 //
 // One tile a CTA.  Warp 0 issues the MMAs.  Warps 1-4 copy, step j by warp j mod 4 (TMA; weights before the previous kernel
-// ends): one warp needs some 300 clocks a block (115 to see a free stage, 45 to announce the bytes, the rest for two copies), three
-// times what its MMAs take.  A step is two blocks, so that the issuing warp waits and commits once for eight MMAs (one block: 178
-// clocks, two: 139 a block; four: no better).  Both test their barriers without a pause.  Then they drain 16 rows x 32 columns each, from registers straight to global memory: a staging tile and a
-// TMA store would make the chain longer, and few bytes leave.  For M = 64 the accumulator's rows 16w .. 16w + 15 lie in the first sixteen lanes of warp w's quadrant.
+// ends): to see a free stage, announce the bytes and issue two copies takes a warp longer than a block's MMAs take (512 -> 512
+// on 7x7: one copying warp 18.1 us, four 11.3).  A step is two blocks, so that the issuing warp waits and commits once for
+// eight MMAs (9.7 us; four blocks: no better).  Both test their barriers without a pause.  Then they drain 16 rows x 32 columns
+// each, from registers straight to global memory: a staging tile and a TMA store would make the chain longer, and few bytes
+// leave.  For M = 64 the accumulator's rows 16w .. 16w + 15 lie in the first sixteen lanes of warp w's quadrant.
 // DUAL: the 1x1 branch on the centre tap of tconv.cu, a second accumulator.
 #include <cuda.h>
 #include <cudaTypedefs.h>
@@ -70,7 +71,7 @@ __device__ __forceinline__ uint32_t load_now(const unsigned short* v) {
 }
 
 // A thread's 2 x 8 values -> memory.  Each combination is a function of its own, as in epilogue.cuh: with the choices tested for
-// every pair a warp, alone on its scheduler, took 1300 to 2000 clocks for them, a quarter of a layer's time.
+// every pair by a warp alone on its scheduler, ResNet-18 took 114 us for one image, now 99.
 template <bool BF16, bool RES, int ACT>
 __device__ __forceinline__ void finish(const uint32_t (&acc)[16], const float2 (&sc)[4], const float2 (&sh)[4], const uint32_t (&res)[2][4],
                                        unsigned short* out, const long long (&at)[2], int cols0, int Kout) {
@@ -353,7 +354,8 @@ cudaError_t launch_conv_small(const TconvArgs& args, cudaStream_t stream) {
   p.n_tiles = (a.Kout + kBN - 1) / kBN;
   const long long tiles = conv_small_tiles(a.N, a.OH, a.OW, a.Kout);
   if (tiles <= 0 || tiles > 0x7fffffffLL) return cudaErrorInvalidValue;
-  p.relu = a.relu; p.bf16 = a.ab == kBF16; p.mode = epi::mode_of(a.ab == kBF16, a.residual != nullptr, a.relu != 0, a.act); p.out_f32 = a.out_dtype == kF32; p.w_ready = a.weights_ready;
+  p.relu = a.relu; p.bf16 = a.ab == kBF16; p.out_f32 = a.out_dtype == kF32; p.w_ready = a.weights_ready;
+  p.mode = epi::mode_of(a.ab == kBF16, a.residual != nullptr, a.relu != 0, a.act);
   const int taps_x = p.taps + (a.wpack2 ? 1 : 0);
   p.div_taps = epi::fast_div((uint32_t)taps_x); p.div_s = epi::fast_div((uint32_t)a.S);
   p.stages_log = 1;

@@ -450,8 +450,8 @@ __device__ __forceinline__ void mbar_arrive_remote(uint32_t cluster_addr) {
 // The same where nothing but the arrival itself passes between the CTAs: tensor memory that was read (tcgen05.wait::ld, then
 // tcgen05.fence::before_thread_sync) and may be written again by the MMAs that the arrival's waiter issues after
 // tcgen05.fence::after_thread_sync.  A release at cluster scope is a memory barrier that waits for all earlier copies and stores of the
-// thread: in the epilogue warps of the CTA pairs 12 % of their time (ResNet-50 at batch 512: 256 -> 1024 pointwise with residual on
-// pairs 131 us, now 95, where single CTAs take 103).  The default release, at CTA scope, is none.
+// thread (ResNet-50 at batch 512: 256 -> 1024 pointwise with residual on pairs 131 us, now 95, where single CTAs take 103).  The
+// default release, at CTA scope, is none.
 __device__ __forceinline__ void mbar_arrive_remote_cta(uint32_t cluster_addr) {
   asm volatile("mbarrier.arrive.release.cta.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
 }

@@ -2,12 +2,12 @@
 //   pooled = mean over pixels;  gate = hard_sigmoid(W2 relu(W1 pooled + b1) + b2);  x *= gate.
 //
 // As three kernels (pool, gate, scaling) the nine blocks of MobileNetV3 took 361 of 1115 us at batch 256 and, at small
-// batches, 27 launches of a few microseconds each.  Here a cluster of eight CTAs owns one, two or four images from beginning to
-// end: the map is read from L2 twice and written once, and what the CTAs exchange (pixel sums, hidden values, gates) goes
-// through distributed shared memory.  With few images each CTA keeps its eighth of both matrices in shared memory, copied
-// before the previous kernel of the stream has ended (read from L2 as they were needed, 576 -> 144 -> 576 took 30 us at batch
-// 4, most of it latency; now 13); with many they are read from L2, once for the images of the cluster (50 us at batch 256 with
-// one row a warp at a time, now 33).  MobileNetV3 fp16 256x224: 1115 -> 1016 us.
+// batches, 27 launches of a few microseconds each; now 213 of 913.  Here a cluster of eight CTAs owns one, two or four images
+// from beginning to end: the map is read from L2 twice and written once, and what the CTAs exchange (pixel sums, hidden values,
+// gates) goes through distributed shared memory.  With few images each CTA keeps its eighth of both matrices in shared memory,
+// copied before the previous kernel of the stream has ended (read from L2 as they were needed, 576 -> 144 -> 576 took 30 us at
+// batch 4, most of it latency); with many they are read from L2, once for the images of the cluster (50 us at batch 256 with one
+// row a warp at a time, now 29).
 //
 // An image's pixels are always cut into the same eight slices, the slices added pairwise, whatever the number of images a
 // cluster owns: an image's result does not depend on the batch it came in.
