@@ -220,7 +220,8 @@ cudaError_t launch_pack_planes(const void* src, DType src_dt, long long sn, long
 cudaError_t launch_split_planes(const float* src, void* dst, long long n, cudaStream_t stream);
 long long stem_planes_elems(int N, int H, int W);        // elements of one plane
 cudaError_t launch_nchw_to_planes(const void* src, DType src_dt, void* dst, int N, int H, int W, cudaStream_t stream);
-cudaError_t launch_maxpool_planes(const void* src, void* dst, int N, int H, int W, int C, int k, int stride, int pad, cudaStream_t stream);
+cudaError_t launch_maxpool_planes(const void* src, int src_f32, void* dst, int N, int H, int W, int C, int k, int stride, int pad,
+                                  cudaStream_t stream);
 cudaError_t launch_avgpool_planes(const void* src, void* dst, int N, int HW, int C, cudaStream_t stream);
 
 // ---- memory-bound helpers (NHWC, 128-bit accesses) ---------------------------------------

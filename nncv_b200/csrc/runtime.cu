@@ -857,6 +857,7 @@ struct PlanNode {
   int fused_into = -1;    // the reverse link
   int stem_pool = -1;     // conv: the max-pool node the fused stem kernel absorbs
   int absorbed = 0;       // max-pool node computed by the stem kernel
+  int pool_only = 0;      // conv: nothing but one max-pool reads its tensor
 };
 struct Plan {
   std::string name;
@@ -1114,6 +1115,8 @@ int finalize_plan(Plan& p, bool act16) {
   for (const PlanNode& n : p.nodes)
     if (n.kind == PlanNode::kSe && readers[n.in] != 1)
       return fail(NNCV_B200_EINVAL, "plan: tensor %d is scaled in place by squeeze-and-excitation node %d but has other readers", n.in, n.id);
+  for (const PlanNode& n : p.nodes)
+    if (n.kind == PlanNode::kMaxPool && readers[n.in] == 1 && p.nodes[producer[n.in]].kind == PlanNode::kConv) p.nodes[producer[n.in]].pool_only = 1;
   if (!act16) return NNCV_B200_OK;
   for (size_t i = 0; i < p.nodes.size(); ++i) {
     PlanNode& a = p.nodes[i];
@@ -1478,7 +1481,7 @@ int model_forward_device(Model& m, const void* src_dev, int N, int H, int W, cud
   const bool sp = adt != kF32;  // tensor-core path keeps block activations in shared-pad NHWC
   auto lay = [&](int h, int w) { return sp ? sp_layout(h, w) : dense_layout(h, w); };
   const double aes = (double)dtype_size(adt);
-  struct Ten { void* p = nullptr; Layout l{0, 0, 0}; int h = 0, w = 0, c = 0; };
+  struct Ten { void* p = nullptr; Layout l{0, 0, 0}; int h = 0, w = 0, c = 0, plain = 0; };   // plain: fp32 where a network keeps planes
   std::map<int, Ten> tens;   // tensor id -> where it lives in this forward
   auto conv_of = [&](const PlanNode& n) -> nncv_b200_conv& { return *m.convs[n.conv_idx]; };
   // the workspace conv_run may take for this convolution: noted in the planning pass
@@ -1605,8 +1608,9 @@ int model_forward_device(Model& m, const void* src_dev, int N, int H, int W, cud
         res = it->second.p;
       }
       if (m.planes) {
-        if (begin_op({in.p, res}) &&
-            (rc = conv_run_planes(&c, in.p, n.in == 0, N, in.h, in.w, m.scale[n.conv_idx], m.shift[n.conv_idx], res, 0, n.relu, o.p, 0, 0, st)))
+        o.plain = n.pool_only;
+        if (begin_op({in.p, res}) && (rc = conv_run_planes(&c, in.p, n.in == 0, N, in.h, in.w, m.scale[n.conv_idx], m.shift[n.conv_idx], res, 0,
+                                                           n.relu, o.p, o.plain, o.plain ? c.Kout : 0, st)))
           return rc;
         tens[n.id] = o;
         continue;
@@ -1753,7 +1757,7 @@ int model_forward_device(Model& m, const void* src_dev, int N, int H, int W, cud
       if ((rc = next_act(m, N, oh, ow, in.c, o.l, st, &o.p))) return rc;
       if (begin_op({in.p})) {
         prof_begin(3, 0, aes * in.c * N * ((double)in.h * in.w + (double)oh * ow), N * in.h * in.w, in.c, 0, 1, st);
-        if (m.planes) LAUNCH(launch_maxpool_planes(in.p, o.p, N, in.h, in.w, in.c, n.k, n.stride, n.pad, st));
+        if (m.planes) LAUNCH(launch_maxpool_planes(in.p, in.plain, o.p, N, in.h, in.w, in.c, n.k, n.stride, n.pad, st));
         else LAUNCH(launch_maxpool_nhwc(in.p, o.p, adt, N, in.h, in.w, in.c, n.k, n.stride, n.pad, in.l, o.l, st));
         prof_end(st);
       }
