@@ -238,6 +238,8 @@ cudaError_t launch_relayout(const void* src, Layout src_l, void* dst, Layout dst
 // scale = gamma * rsqrt(var + 1e-5f); shift = beta - mean * scale  (inputs of type dt)
 cudaError_t launch_bn_fold(const void* gamma, const void* beta, const void* mean, const void* var, DType dt, int C, float eps,
                            float* scale, float* shift, cudaStream_t stream);
+// Results to page-locked host memory (dst, flag_out as the device addresses them), with the status word.
+cudaError_t launch_deliver(const void* src, void* dst, size_t bytes, const int* flag, int* flag_out, cudaStream_t stream);
 cudaError_t launch_convert(const void* src, DType src_dt, void* dst, DType dst_dt, size_t n,
                            cudaStream_t stream);
 

@@ -277,6 +277,16 @@ bool is_device_ptr(const void* p) {
   return attr.type == cudaMemoryTypeDevice || attr.type == cudaMemoryTypeManaged;
 }
 
+// Device memory of the current device, which its kernels may write.
+bool is_own_device_ptr(const void* p) {
+  cudaPointerAttributes attr;
+  if (cudaPointerGetAttributes(&attr, p) != cudaSuccess) {
+    cudaGetLastError();
+    return false;
+  }
+  return attr.type == cudaMemoryTypeDevice && attr.device == g_dev.id;
+}
+
 // Page-locked host memory the copy engine reads directly?
 bool is_pinned_ptr(const void* p) {
   cudaPointerAttributes attr;
@@ -1454,8 +1464,8 @@ int finish_act_plan(Model& m) {
 }
 
 // Runs the network on a dense NCHW device tensor; logits (io type) land in m.logits_io
-// (or m.logits32 when io is fp32).  Asynchronous on `st`.
-int model_forward_device(Model& m, const void* src_dev, int N, int H, int W, cudaStream_t st) {
+// (or m.logits32 when io is fp32) at m.logits_off, or in `logits`, device memory on a 32-byte boundary.  Asynchronous on `st`.
+int model_forward_device(Model& m, const void* src_dev, int N, int H, int W, cudaStream_t st, void* logits = nullptr) {
   int rc = ensure_workspace(m, N, H, W);
   if (rc) return rc;
   if (!m.planned && !m.planning) {
@@ -1464,7 +1474,7 @@ int model_forward_device(Model& m, const void* src_dev, int N, int H, int W, cud
     m.act_plan.clear();
     m.split_bytes = 0;
     m.op_idx = 0;
-    rc = model_forward_device(m, src_dev, m.wsN, H, W, st);
+    rc = model_forward_device(m, src_dev, m.wsN, H, W, st, logits);
     m.planning = false;
     if (rc) return rc;
     if ((rc = finish_act_plan(m))) return rc;
@@ -1798,19 +1808,18 @@ int model_forward_device(Model& m, const void* src_dev, int N, int H, int W, cud
         continue;
       }
       const int of = m.plan.out_features;
-      note_planes(*fc, in.p, m.logits32.p, nullptr, 1, 1);
+      // 16-bit logits wanted and computed in the same type: the FC epilogue rounds once, exactly as the fp32 -> io conversion
+      // kernel would, and that kernel is not launched
+      const bool in_place = m.io_dt == adt || m.io_dt == kF32;
+      void* const io = logits ? logits : (char*)(m.io_dt == kF32 ? m.logits32.p : m.logits_io.p) + m.logits_off;
+      void* const to = in_place ? io : (char*)m.logits32.p + m.logits_off;
+      const DType to_dt = in_place ? m.io_dt : kF32;
+      note_planes(*fc, in.p, to, nullptr, 1, 1);
       if (!begin_op({in.p})) return NNCV_B200_OK;   // the planning pass ends with the last reader of an activation tensor
-      if (m.io_dt == adt && adt != kF32) {
-        // 16-bit logits wanted and computed in the same type: the FC epilogue rounds once, exactly as
-        // the fp32 -> io conversion kernel would, and that kernel is not launched
-        return conv_run(fc, in.p, dense_layout(1, 1), (char*)m.logits_io.p + m.logits_off, dense_layout(1, 1), N, 1, 1, nullptr, bias, nullptr, 0, adt, of,
-                        st);
-      }
-      rc = m.planes ? conv_run_planes(fc, in.p, false, N, 1, 1, nullptr, bias, nullptr, 0, 0, (char*)m.logits32.p + m.logits_off, 1, of, st)
-                    : conv_run(fc, in.p, dense_layout(1, 1), (char*)m.logits32.p + m.logits_off, dense_layout(1, 1), N, 1, 1, nullptr, bias, nullptr, 0, kF32, of, st, nullptr, &m.split_planes);
+      rc = m.planes ? conv_run_planes(fc, in.p, false, N, 1, 1, nullptr, bias, nullptr, 0, 0, to, 1, of, st)
+                    : conv_run(fc, in.p, dense_layout(1, 1), to, dense_layout(1, 1), N, 1, 1, nullptr, bias, nullptr, 0, to_dt, of, st, nullptr, &m.split_planes);
       if (rc) return rc;
-      if (m.io_dt != kF32)
-        LAUNCH(launch_convert((char*)m.logits32.p + m.logits_off, kF32, (char*)m.logits_io.p + m.logits_off, m.io_dt, (size_t)N * of, st));
+      if (!in_place) LAUNCH(launch_convert(to, kF32, io, m.io_dt, (size_t)N * of, st));
       return NNCV_B200_OK;
     }
   }
@@ -1878,6 +1887,7 @@ struct CopiesInFlight {
 // A batch of images in host memory, in n_parts parts of equal size: every copy, every forward, one wait.  Where the batch is no
 // multiple, the last part takes images of the one before with it (layers are tuned for one batch size, and a 16-bit image's logits
 // do not depend on its part).
+constexpr size_t kDeliver = 64 << 10;   // results that go into pinned memory of the caller's by way of the library's: as far as the host's copy takes less
 int forward_host(Model& m, const char* sp, bool pinned, char* dp, bool dst_dev, size_t dst_stride, int N, int H, int W, cudaStream_t st,
                  int n_parts) {
   int rc;
@@ -1894,7 +1904,9 @@ int forward_host(Model& m, const char* sp, bool pinned, char* dp, bool dst_dev, 
     cudaDeviceSynchronize();
     if ((rc = reserve_logits(m, logits_bytes))) return rc;
   }
-  const bool stage_out = !dst_dev && !is_pinned_ptr(dp) && row * N <= (4u << 20);   // small results leave through pinned memory
+  // Small results and the status word leave through the library's pinned memory, which one kernel writes: the step from one copy of the
+  // copy engine to the next takes 3 us.
+  const bool stage_out = !dst_dev && row * N <= (is_pinned_ptr(dp) ? kDeliver : 4u << 20);
   if ((rc = m.result.reserve(256 + (stage_out ? row * N : 0)))) return rc;
   cudaStream_t cst = st;
   if (n_parts > 1) {
@@ -1927,12 +1939,12 @@ int forward_host(Model& m, const char* sp, bool pinned, char* dp, bool dst_dev, 
     if (n_parts > 1) CU(cudaStreamWaitEvent(st, g_dev.copy_done[c], 0));
     m.logits_off = c * part_bytes;
     if ((rc = model_forward_device(m, (char*)m.in_stage.p + first * img_bytes, n, H, W, st))) return rc;
-    if (stage_out) CU(cudaMemcpyAsync((char*)m.result.p + 256 + row * first, logits + m.logits_off, row * n, cudaMemcpyDeviceToHost, st));
+    if (stage_out) LAUNCH(launch_deliver(logits + m.logits_off, (char*)m.result.p + 256 + row * first, row * n, g_dev.error_flag, (int*)m.result.p, st));
     else CU(cudaMemcpy2DAsync(dp + first * dst_stride * ew, dst_stride * ew, logits + m.logits_off, row, row, (size_t)n,
                               dst_dev ? cudaMemcpyDeviceToDevice : cudaMemcpyDeviceToHost, st));
   }
   int* status = (int*)m.result.p;
-  CU(cudaMemcpyAsync(status, g_dev.error_flag, sizeof(int), cudaMemcpyDeviceToHost, st));
+  if (!stage_out) CU(cudaMemcpyAsync(status, g_dev.error_flag, sizeof(int), cudaMemcpyDeviceToHost, st));
   CU(cudaStreamSynchronize(st));
   flight.waited = true;   // the copies in come before the forwards that read them
   if (*status != 0) {
@@ -1988,7 +2000,15 @@ int forward_slice(Model& m, const char* sp, bool src_dev, char* dp, bool dst_dev
   if (src_dev) {
     if ((rc = ensure_workspace(m, N, H, W))) return rc;
     m.logits_off = 0;
-    if ((rc = model_forward_device(m, sp, N, H, W, st))) return rc;
+    // rows without gaps in this GPU's memory, on the boundary of the widest store: the last layer writes them itself
+    const bool in_place = dst_dev && dst_stride * ew == row && !(reinterpret_cast<uintptr_t>(dp) & 31) && is_own_device_ptr(dp);
+    if ((rc = model_forward_device(m, sp, N, H, W, st, in_place ? dp : nullptr))) return rc;
+    if (in_place) {
+      if (device_only) return ok();
+      CU(cudaStreamSynchronize(st));
+      if ((rc = check_kernel_status())) return rc;
+      return ok();
+    }
     const void* logits = m.io_dt == kF32 ? m.logits32.p : m.logits_io.p;
     if (device_only && dst_stride * ew == row) CU(cudaMemcpyAsync(dp, logits, row * N, cudaMemcpyDeviceToDevice, st));
     else CU(cudaMemcpy2DAsync(dp, dst_stride * ew, logits, row, row, (size_t)N, dst_dev ? cudaMemcpyDeviceToDevice : cudaMemcpyDeviceToHost, st));
