@@ -283,8 +283,9 @@ int nncv_b200_conv_run_fused(nncv_b200_conv* c, nncv_b200_conv* branch, const vo
  * a mostly empty last round sliced by columns; algo 0 with Kout a multiple of bn = 128 or 256:
  * 2 = the per-tap kernel on CTA pairs); bn = 32: the kernel of 64 x 32 tiles for small batches,
  * whatever mt and resident say; bn = 0 restores the built-in choice.  F32 on the tensor cores: bn = 32,
- * 64 or 128, mt = CTAs that share a tile's reduction (1, 2, 4 or 8); what does not fit the layer is
- * chosen as without it.  A tuning and test hook with no counterpart in the reference. */
+ * 64 or 128, mt = CTAs that share a tile's reduction (1, 2, 4 or 8), resident = 1 with bn = 64: the
+ * pixels of every filter tap copied by themselves, 2: those of a column of the filter at once; what
+ * does not fit the layer is chosen as without it.  A tuning and test hook with no counterpart in the reference. */
 int nncv_b200_conv_set_tile(nncv_b200_conv* c, int bn, int mt, int resident);
 
 /* The ResNet stem in one kernel (tests/Nets/Res18.mlir:118-151): tensor.pad 3 + 7x7 stride-2

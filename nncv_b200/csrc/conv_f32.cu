@@ -22,21 +22,29 @@
 // The 7x7 stride-2 stem reads row pairs through a tensor map with overlapping strides, as stem.cu does: it becomes a
 // convolution with four taps of 64 "channels".
 //
-// Two kernels.  conv_f32_kernel: one CTA computes 128 pixels x 64 or 128 output channels.  What bounds it: 72 or 96 KB of planes from
-// L2 per block of 64 channels (1560 or 2000 clocks with every SM at work), then the 24 MMAs (1150 or 1540 clocks).  With few pixels a
+// Two kernels.  conv_f32_kernel: one CTA computes 128 pixels x 64 or 128 output channels.  What bounds it: the port of shared memory, 128
+// bytes a clock for what the MMAs of a block of 64 channels read (1152 or 1536 clocks) and about twice that for what is copied in (72 or
+// 96 KB); 1430 and 1900 clocks a block are measured.  HALO, for filters of stride 1: one box of pixels serves a whole column of the filter
+// (42 KB a block), and the filter's planes lie together, so that a1 multiplies b2 and b3 in one MMA of 128 columns (896 clocks): 1220.
+// Two warps issue the MMAs, one the large products: an MMA takes its warp about 29 clocks, a wait or a commit about 80.  us before and
+// now: 56x56x64 of eight images 24.5 23.0, of 32 77 70, 28x28x128 of eight 24 21; 64 x 32 tiles 512 -> 512 on 7x7 by one CTA a tile 38.9
+// 28.6.  With few pixels a
 // cluster of up to eight CTAs splits the reduction of a tile; each leaves its partial sums in shared memory and finishes
 // its share of the rows from all of them, in rank order, so that the result does not depend on timing.  (The CUDA-core
 // kernel needed a second pass over partial sums in global memory for that, and ran at a fifth of the fp32 rate.)
-// Roles: warp 0 TMA producer, one plane of both operands per ring slot; warp 1 MMA issuer; warps 2-9 epilogue.
+// Roles: warp 0 TMA producer, one plane of both operands per ring slot (HALO: boxes, and blocks of the filter); warps 1 and 18 MMA
+// issuers; warps 2-17 epilogue (with eight of them, twice the columns each, ResNet-18 8x224 took 421 us and ResNet-50 4x224 802, where
+// these took 395 and 704; sixteen in two sets, a pair of accumulators each, saved nothing in the blocks and cost 1 us a tile).
 // conv_f32_small_kernel, for one to four images: 64 pixels x 32 output channels, below.  conv_f32_choose takes one by a model of both.
 //
-// ResNet-18 fp32 against the CUDA-core kernel, from device memory: 1x256 470 -> 192 us, 8x224 1626 -> 449 us.
+// ResNet-18 fp32 against the CUDA-core kernel, from device memory: 1x256 470 -> 177 us, 8x224 1626 -> 403 us.
 // Every wait is bounded and abortable; a timed-out wait sets the device status word.
 #include <cuda.h>
 #include <cudaTypedefs.h>
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cfloat>
 #include <mutex>
 
@@ -48,12 +56,13 @@ namespace nncv_b200 {
 
 namespace {
 
-constexpr int kEpiThreads = epi::kThreads;
-constexpr int kThreads = 64 + kEpiThreads;
+constexpr int kEpiWarps = 16, kEpiThreads = 32 * kEpiWarps;
+constexpr int kLargeWarp = 2 + kEpiWarps, kThreads = 32 * (kLargeWarp + 1);
 constexpr int kABytes = 128 * 128;
 constexpr int kBBytes = 64 * 128;           // packed weights: tiles of 64 output channels x 64 input channels
 constexpr int kTileBytes = 128 * 64 * 4;    // partial sums of 64 of the tile's columns, fp32
 constexpr int kSmallBlocks = 4;             // blocks of 64 channels whose small products share an accumulator
+constexpr int kHaloB = 8, kBoxes = 2;       // halo tiles: blocks of weights (three planes) and boxes that rings can hold
 constexpr float kCut = 3.0f / (1 << 28);    // what a step of the tensor core cuts off its sum, on average (0.19 * 2^-24)
 template <int BN>
 struct Ring {   // a slot holds one plane of a block: 128 pixels and BN output channels x 64 channels
@@ -74,9 +83,12 @@ struct F32Params {
   int out_f32, res_f32, relu;
   int Kout, CB, taps, S, stride, pad_x, pad_y;
   int OH, OW, NB;
-  int tw, th;
-  int tn, tiles_x, tiles_y, n_tiles, items;
-  epi::FastDiv div_tx, div_ty, div_nt, div_tw, div_th;
+  // row r of a tile is pixel (r / mp / rows_img, r / mp % rows_img, r % mp) of its tn x th x tw, or none
+  int tw, th, tn, mp, rows_img;
+  int tiles_x, tiles_y, n_tiles, items;
+  epi::FastDiv div_tx, div_ty, div_nt, div_mp, div_ri;
+  // halo tiles: rows of the filter, bytes of a plane's box, blocks of weights that fit
+  int R, a_plane, b_stages;
   int splits;                 // CTAs of a cluster that share a tile's reduction (a power of two up to 8)
 };
 
@@ -135,24 +147,29 @@ __device__ __forceinline__ float4 join4(const uint2 (&w)[3]) {
   return v;
 }
 
-template <int kBN>   // output channels of a tile: 64 or 128
+template <int kBN, bool HALO>   // output channels of a tile: 64 or 128
 __global__ void __launch_bounds__(kThreads, 1)
 conv_f32_kernel(const __grid_constant__ CUtensorMap tm_in, const F32Params p) {
-  constexpr int kSlots = Ring<kBN>::kSlots, kSlot = Ring<kBN>::kSlot, kNT = kBN / 64;
+  static_assert(!HALO || kBN == 64, "halo tiles are 64 channels wide");
+  constexpr int kSlots = HALO ? kHaloB : Ring<kBN>::kSlots, kSlot = HALO ? 3 * kBBytes : Ring<kBN>::kSlot, kNT = kBN / 64;
   // Accumulators: pairs for two steps of the large products, and two for the small ones.  A pair is handed over as one: the
   // epilogue's time is the latency of a hand-over, about 400 clocks, and four a block of 64 channels took longer than the copies.
   constexpr uint32_t kPairs = kBN == 64 ? 2 : 1, kAcc = kPairs + 2;
   constexpr uint32_t kTmemCols = 512, kSmallCols = kPairs * 2 * kBN;
-  constexpr int kCols = kBN / 2;            // columns of a thread's row
+  constexpr int kCols = kBN / 4;            // columns of a thread's row
   extern __shared__ uint8_t smem_raw[];
   __shared__ int s_abort;
-  __shared__ __align__(8) unsigned long long s_bars[2 * kSlots + 2 * kAcc + 2];
+  __shared__ __align__(8) unsigned long long s_bars[2 * kSlots + 2 * kAcc + 2 + 2 * kBoxes];
   const uint32_t raw = ptx::smem_u32(smem_raw);
-  const uint32_t sRing = (raw + 1023u) & ~1023u;
-  const uint32_t sTile = sRing + kSlots * kSlot;
+  // the ring; with halo tiles the boxes of pixels, then a ring of weights alone
+  const uint32_t sBox = (raw + 1023u) & ~1023u;
+  const int slots = HALO ? p.b_stages : kSlots;
+  const uint32_t sRing = sBox + (HALO ? (uint32_t)(kBoxes * 3 * p.a_plane) : 0u);
+  const uint32_t sTile = sRing + slots * kSlot;
   const uint32_t full = ptx::smem_u32(s_bars), empty = full + 8 * kSlots;
   const uint32_t d_full = empty + 8 * kSlots, d_empty = d_full + 8 * kAcc;   // pairs first
   const uint32_t part_ready = d_empty + 8 * kAcc, part_done = part_ready + 8;
+  const uint32_t a_full = part_done + 8, a_empty = a_full + 8 * kBoxes;
   __shared__ uint32_t s_tmem;
   const int warp = ptx::warp_uniform((int)threadIdx.x >> 5), lane = threadIdx.x & 31;
   const int S = p.splits;
@@ -162,14 +179,18 @@ conv_f32_kernel(const __grid_constant__ CUtensorMap tm_in, const F32Params p) {
     s_abort = 0;
     for (int i = 0; i < kSlots; ++i) {
       ptx::mbar_init(full + 8 * i, 1);
-      ptx::mbar_init(empty + 8 * i, 1);
+      ptx::mbar_init(empty + 8 * i, 2);   // both issuing warps
     }
     for (uint32_t i = 0; i < kAcc; ++i) {
       ptx::mbar_init(d_full + 8 * i, 1);
-      ptx::mbar_init(d_empty + 8 * i, epi::kWarps);
+      ptx::mbar_init(d_empty + 8 * i, kEpiWarps);
     }
     ptx::mbar_init(part_ready, S);
     ptx::mbar_init(part_done, S);
+    for (int i = 0; i < kBoxes; ++i) {
+      ptx::mbar_init(a_full + 8 * i, 1);
+      ptx::mbar_init(a_empty + 8 * i, 2);
+    }
     ptx::mbar_fence_init();
     ptx::prefetch_tensormap(&tm_in);
   }
@@ -210,12 +231,38 @@ conv_f32_kernel(const __grid_constant__ CUtensorMap tm_in, const F32Params p) {
                     p.wpack + (((size_t)t * 3 + plane) * kb_all + (size_t)tap * p.CB + cb) * kBBytes, kBBytes, full + 8 * slot, issue);
     }
   };
+  // halo tiles: blocks go channel block outermost, then filter column c, then filter row r
+  auto block_of = [&](int kb, int& cb, int& c, int& r) {
+    cb = kb / p.taps;
+    c = (kb - cb * p.taps) / p.R;
+    r = kb - cb * p.taps - c * p.R;
+  };
+  auto next_block = [&](int& cb, int& c, int& r) {
+    if (++r == p.R) {
+      r = 0;
+      if (++c == p.S) { c = 0; ++cb; }
+    }
+  };
+  auto load_block = [&](int n_tile, int cb, int tap, uint32_t slot, uint32_t issue) {
+#pragma unroll
+    for (int pl = 0; pl < 3; ++pl)
+      ptx::bulk_g2s(sRing + slot * kSlot + pl * kBBytes, p.wpack + (((size_t)n_tile * 3 + pl) * kb_all + (size_t)tap * p.CB + cb) * kBBytes, kBBytes,
+                    full + 8 * slot, issue);
+  };
   // the packed weights never change: their first copies do not wait for the previous kernel
   uint32_t early = 0;
   if (warp == 0) {
     const uint32_t issue = ptx::elect_one();
     int n0, oy0, ox0, n_tile;
-    if (item_of(0, n0, oy0, ox0, n_tile)) {
+    if (HALO && item_of(0, n0, oy0, ox0, n_tile)) {
+      int cb, c, r;
+      block_of(kb0, cb, c, r);
+      for (int kb = kb0; kb < kb1 && early < (uint32_t)slots; ++kb, ++early) {
+        ptx::mbar_arrive_expect_tx(full + 8 * early, kSlot, issue);
+        load_block(n_tile, cb, r * p.S + c, early, issue);
+        next_block(cb, c, r);
+      }
+    } else if (!HALO && item_of(0, n0, oy0, ox0, n_tile)) {
       int cb = kb0 / p.taps, tap = kb0 - cb * p.taps;
       for (int kb = kb0; kb < kb1 && early < (uint32_t)kSlots; ++kb) {
         for (int pl = 0; pl < 3 && early < (uint32_t)kSlots; ++pl, ++early) {
@@ -231,7 +278,35 @@ conv_f32_kernel(const __grid_constant__ CUtensorMap tm_in, const F32Params p) {
 
   if (warp == 0) {
     // ------------------------------------------------------------------ TMA producer ----
-    {
+    if constexpr (HALO) {
+      const uint32_t issue = ptx::elect_one();
+      uint32_t slot = 0, ring = 0, cnt = 0, seen = 1, as = 0, a_ring = 0;
+      bool okw = true;
+      for (int i = 0; okw; ++i) {
+        int n0, oy0, ox0, n_tile;
+        if (!item_of(i, n0, oy0, ox0, n_tile)) break;
+        int cb, c, r;
+        block_of(kb0, cb, c, r);
+        for (int kb = kb0; kb < kb1 && okw; ++kb, ++cnt) {
+          if (kb == kb0 || r == 0) {   // the pixels under a column of the filter
+            if (!ptx::warp_wait(a_empty + 8 * as, a_ring ^ 1u, abort_flag)) { okw = false; break; }
+            ptx::mbar_arrive_expect_tx(a_full + 8 * as, 3u * (uint32_t)p.a_plane, issue);
+            for (int pl = 0; pl < 3; ++pl)
+              ptx::tma_load_5d(sBox + (as * 3 + pl) * (uint32_t)p.a_plane, &tm_in, cb * 64, ox0 - p.pad_x + c, oy0 - p.pad_y, n0, pl, a_full + 8 * as, issue);
+            if (++as == (uint32_t)kBoxes) { as = 0; a_ring ^= 1u; }
+          }
+          if (cnt >= early) {
+            if (!ptx::warp_all(seen) && !ptx::warp_wait(empty + 8 * slot, ring ^ 1u, abort_flag)) { okw = false; break; }
+            ptx::mbar_arrive_expect_tx(full + 8 * slot, kSlot, issue);
+            load_block(n_tile, cb, r * p.S + c, slot, issue);
+          }
+          if (++slot == (uint32_t)slots) { slot = 0; ring ^= 1u; }
+          seen = ptx::mbar_peek(empty + 8 * slot, ring ^ 1u);
+          next_block(cb, c, r);
+        }
+      }
+      if (!okw && lane == 0 && p.error_flag) atomicCAS(p.error_flag, 0, (int)kErrWaitProducer);
+    } else {
       const uint32_t issue = ptx::elect_one();
       uint32_t slot = 0, ring = 0, cnt = 0, seen = 1;
       bool okw = true;
@@ -258,173 +333,227 @@ conv_f32_kernel(const __grid_constant__ CUtensorMap tm_in, const F32Params p) {
       }
       if (!okw && lane == 0 && p.error_flag) atomicCAS(p.error_flag, 0, (int)kErrWaitProducer);
     }
-  } else if (warp == 1) {
-    // ------------------------------------------------------------------ MMA issuer ------
+  } else if (warp == 1 || warp == kLargeWarp) {
+    // ------------------------------------------------------------------ MMA issuers -----
+    // One warp for the large products, one for the small ones: an MMA takes its warp about 29 clocks and a wait or a commit about 80,
+    // so a lone warp needed longer for the 20 or 24 MMAs of a block, with their hand-overs, than the tensor core.
+    const bool large_warp = warp == kLargeWarp;
     const uint32_t issue = ptx::elect_one();
-    const uint32_t idesc = ptx::umma_idesc(128, kBN, 1);
-    uint32_t slot = 0, ring = 0;
-    uint32_t large = 0, small = 0;   // running counts of uses of pairs and of small accumulators
+    const uint32_t idesc = ptx::umma_idesc(128, kBN, 1), idesc2 = HALO ? ptx::umma_idesc(128, 128, 1) : idesc;
+    uint32_t slot = 0, ring = 0, as = 0, a_ring = 0;   // halo tiles: the box in use
+    uint32_t uses = 0;               // of pairs, or of small accumulators
     bool okw = true;
     uint32_t seen = ptx::mbar_peek(full, 0);
-    auto step = [&]() {
-      if (++slot == kSlots) { slot = 0; ring ^= 1u; }
+    // the next slot is full
+    auto arrive = [&](uint32_t& now) {
+      if (!ptx::warp_all(seen) && !ptx::warp_wait(full + 8 * slot, ring, abort_flag)) return false;
+      ptx::tc_fence_after();
+      now = slot;
+      if (++slot == (uint32_t)slots) { slot = 0; ring ^= 1u; }
       seen = ptx::mbar_peek(full + 8 * slot, ring);
+      return true;
     };
-    auto mma = [&](uint32_t d, uint32_t a, uint32_t b, uint32_t k4, uint32_t accumulate) {
-      ptx::umma_f16(d, ptx::desc_from_halves(ptx::smem_desc_k128_lo(a) + k4 * 2, ptx::kSmemDescK128Hi),
-                    ptx::desc_from_halves(ptx::smem_desc_k128_lo(b) + k4 * 2, ptx::kSmemDescK128Hi), idesc, accumulate, issue);
+    // step k4 (16 channels) of operands whose descriptors start at a and b
+    auto mma = [&](uint32_t d, uint32_t a, uint32_t b, uint32_t k4, uint32_t id, uint32_t accumulate) {
+      ptx::umma_f16(d, ptx::desc_from_halves(a + k4 * 2, ptx::kSmemDescK128Hi), ptx::desc_from_halves(b + k4 * 2, ptx::kSmemDescK128Hi), id, accumulate, issue);
     };
     // a product of two planes of the block: four steps of 16 channels
-    auto product = [&](uint32_t d, uint32_t a, uint32_t b, uint32_t fresh) {
+    auto product = [&](uint32_t d, uint32_t a, uint32_t b, uint32_t id, uint32_t fresh) {
 #pragma unroll
-      for (uint32_t k4 = 0; k4 < 4; ++k4) mma(d, a, b, k4, k4 == 0 ? (fresh ^ 1u) : 1u);
+      for (uint32_t k4 = 0; k4 < 4; ++k4) mma(d, a, b, k4, id, k4 == 0 ? (fresh ^ 1u) : 1u);
     };
-    // waits until the epilogue has emptied accumulator acc, filled `turn` times before
-    auto wait_empty = [&](uint32_t acc, uint32_t turn) { return ptx::warp_wait(d_empty + 8 * acc, (turn & 1u) ^ 1u, abort_flag); };
+    // the four steps of the large products, each into an accumulator of its own, handed over in pairs
+    auto four_large = [&](uint32_t a, uint32_t b) {
+#pragma unroll
+      for (uint32_t k4 = 0; k4 < 4; k4 += 2, ++uses) {
+        const uint32_t pair = uses % kPairs;
+        if (!ptx::warp_wait(d_empty + 8 * pair, ((uses / kPairs) & 1u) ^ 1u, abort_flag)) return false;
+        ptx::tc_fence_after();
+#pragma unroll
+        for (uint32_t j = 0; j < 2; ++j) mma(tmem_base + (2 * pair + j) * kBN, a, b, k4 + j, idesc, 0u);
+        ptx::tc_commit(d_full + 8 * pair, issue);
+      }
+      return true;
+    };
     for (int i = 0; okw; ++i) {
       int n0, oy0, ox0, n_tile;
       if (!item_of(i, n0, oy0, ox0, n_tile)) break;
+      int r = HALO ? kb0 % p.R : 0;   // rows of the filter divide the taps
       for (int kb = kb0; kb < kb1; ++kb) {
         const bool group_first = (kb - kb0) % kSmallBlocks == 0, group_last = (kb - kb0) % kSmallBlocks == kSmallBlocks - 1 || kb + 1 == kb1;
-        const uint32_t small_acc = kPairs + (small & 1u), ds = tmem_base + kSmallCols + (small & 1u) * kBN;
-        uint32_t at[3], sl[3];
-        // the next plane of the block
-        auto arrive = [&](int pl) {
-          if (!ptx::warp_all(seen) && !ptx::warp_wait(full + 8 * slot, ring, abort_flag)) return false;
+        const uint32_t acc = kPairs + (uses & 1u), ds = tmem_base + kSmallCols + (uses & 1u) * (HALO ? 2 : 1) * kBN;
+        auto small_ready = [&]() {
+          if (!group_first) return true;
+          if (!ptx::warp_wait(d_empty + 8 * acc, ((uses >> 1) & 1u) ^ 1u, abort_flag)) return false;
           ptx::tc_fence_after();
-          sl[pl] = slot;
-          at[pl] = sRing + slot * kSlot;
-          step();
           return true;
         };
-        // two steps of the large products, each into an accumulator of its own
-        auto two_large = [&](uint32_t k4) {
-          const uint32_t pair = large % kPairs;
-          if (!wait_empty(pair, large / kPairs)) return false;
-          ptx::tc_fence_after();
+        const uint32_t fresh = group_first ? 1u : 0u;
+        uint32_t now[3];
+        if constexpr (HALO) {
+          if ((kb == kb0 || r == 0) && !ptx::warp_wait(a_full + 8 * as, a_ring, abort_flag)) { okw = false; break; }
+          if (!arrive(now[0])) { okw = false; break; }
+          // filter row r reads the box from its row r on: mp pixels, a multiple of eight rows of 128 bytes
+          const uint32_t b = ptx::smem_desc_k128_lo(sRing + now[0] * kSlot), bp = kBBytes >> 4, ap = (uint32_t)p.a_plane >> 4;
+          const uint32_t a = ptx::smem_desc_k128_lo(sBox + as * 3 * (uint32_t)p.a_plane + (uint32_t)(r * p.mp) * 128u);
+          if (large_warp) {
+            if (!four_large(a, b)) { okw = false; break; }
+          } else {
+            if (!small_ready()) { okw = false; break; }
+            // two accumulators side by side: a1 b2 | a1 b3, a2 b1 | a2 b2, a3 b1
+            product(ds, a, b + bp, idesc2, fresh);
+            product(ds, a + ap, b, idesc2, 0u);
+            product(ds, a + 2 * ap, b, idesc, 0u);
+          }
+          ptx::tc_commit(empty + 8 * now[0], issue);
+          if (++r == p.R) r = 0;
+          if (r == 0 || kb + 1 == kb1) {
+            ptx::tc_commit(a_empty + 8 * as, issue);
+            if (++as == (uint32_t)kBoxes) { as = 0; a_ring ^= 1u; }
+          }
+        } else {
+          auto at = [&](uint32_t sl) { return ptx::smem_desc_k128_lo(sRing + sl * kSlot); };
+          constexpr uint32_t kB = kABytes >> 4;
+          if (!arrive(now[0])) { okw = false; break; }
+          if (large_warp) {
+            if (!four_large(at(now[0]), at(now[0]) + kB)) { okw = false; break; }
+            ptx::tc_commit(empty + 8 * now[0], issue);
+            // nothing to do with the other planes: they have come when the barrier counts this use of their slots
+            if (!arrive(now[1])) { okw = false; break; }
+            if (lane == 0) ptx::mbar_arrive(empty + 8 * now[1]);
+            if (!arrive(now[2])) { okw = false; break; }
+            if (lane == 0) ptx::mbar_arrive(empty + 8 * now[2]);
+          } else {
+            if (!arrive(now[1]) || !small_ready()) { okw = false; break; }
+            product(ds, at(now[0]), at(now[1]) + kB, idesc, fresh);
+            product(ds, at(now[1]), at(now[0]) + kB, idesc, 0u);
+            product(ds, at(now[1]), at(now[1]) + kB, idesc, 0u);
+            if (!arrive(now[2])) { okw = false; break; }
+            product(ds, at(now[0]), at(now[2]) + kB, idesc, 0u);
+            product(ds, at(now[2]), at(now[0]) + kB, idesc, 0u);
 #pragma unroll
-          for (uint32_t j = 0; j < 2; ++j) mma(tmem_base + (2 * pair + j) * kBN, at[0], at[0] + kABytes, k4 + j, 0u);
-          ptx::tc_commit(d_full + 8 * pair, issue);
-          ++large;
-          return true;
-        };
-        if (!arrive(0) || !two_large(0)) { okw = false; break; }
-        if (!arrive(1) || (group_first && !wait_empty(small_acc, small >> 1))) { okw = false; break; }
-        ptx::tc_fence_after();
-        product(ds, at[0], at[1] + kABytes, group_first ? 1u : 0u);
-        product(ds, at[1], at[0] + kABytes, 0u);
-        product(ds, at[1], at[1] + kABytes, 0u);
-        // the other two steps, when the epilogue has had the time to empty the accumulators
-        if (!two_large(2) || !arrive(2)) { okw = false; break; }
-        product(ds, at[0], at[2] + kABytes, 0u);
-        product(ds, at[2], at[0] + kABytes, 0u);
-#pragma unroll
-        for (int pl = 0; pl < 3; ++pl) ptx::tc_commit(empty + 8 * sl[pl], issue);
-        if (group_last) {
-          ptx::tc_commit(d_full + 8 * small_acc, issue);
-          ++small;
+            for (int pl = 0; pl < 3; ++pl) ptx::tc_commit(empty + 8 * now[pl], issue);
+          }
+        }
+        if (!large_warp && group_last) {
+          ptx::tc_commit(d_full + 8 * acc, issue);
+          ++uses;
         }
       }
     }
     if (!okw && lane == 0 && p.error_flag) atomicCAS(p.error_flag, 0, (int)kErrWaitMma);
   } else {
     // ------------------------------------------------------------------ epilogue --------
-    const int ew = warp - 2, quad = warp & 3, half = ew >> 2;
+    const int quad = warp & 3, part = (warp - 2) >> 2;   // rows, and a quarter of the tile's columns
     const int row = quad * 32 + lane;
     const int et = (int)threadIdx.x - 64;
     const int rows_each = 128 / S, row_lo = (int)rank * rows_each;
     const int g = et & 15;             // four columns of the tile
+    constexpr int kRows = 128 * 16 / kEpiThreads;   // rows a thread finishes
     uint32_t large = 0, small = 0;     // running counts of uses of the accumulators
     bool okw = true;
     for (int i = 0; okw; ++i) {
       int n0, oy0, ox0, n_tile;
       if (!item_of(i, n0, oy0, ox0, n_tile)) break;
-      const uint32_t lane_base = tmem_base + ((uint32_t)(quad * 32) << 16) + (uint32_t)(half * kCols);
-      // the pixels this thread finishes: row r of the tile -> its index in the output, -1 outside
-      int pix[8];
+      const uint32_t lane_base = tmem_base + ((uint32_t)(quad * 32) << 16) + (uint32_t)(part * kCols);
+      // 64 columns: the large products in two sums, of steps 0 and 1 and of steps 2 and 3 of the blocks, half as many roundings one after
+      // another: clusters of fewer CTAs have longer sums, and with one sum the logits of ResNet-18 were 1.0 % further off on average than
+      // before these tiles, with two 0.1 % (ResNet-50 0.2 % and 1.4 % nearer).  396 -> 403 us and 706 -> 729 us for it.
+      constexpr bool kTwo = kBN == 64;
+      float sum[kCols], other[kTwo ? kCols : 1];
 #pragma unroll
-      for (int k = 0; k < 8; ++k) {
-        const int rr = (et >> 4) + k * (kEpiThreads / 16), r = row_lo + rr;
-        const int t1 = (int)epi::div_by((uint32_t)r, p.div_tw), tj = r - t1 * p.tw;
-        const int t2 = (int)epi::div_by((uint32_t)t1, p.div_th), ti = t1 - t2 * p.th;
-        const int img = n0 + t2, oy = oy0 + ti, ox = ox0 + tj;
-        pix[k] = rr < rows_each && img < p.NB && oy < p.OH && ox < p.OW ? (img * p.OH + oy) * p.OW + ox : -1;
-      }
-      auto load_res = [&](int k, int n, uint2 (&w)[3]) {
-#pragma unroll
-        for (int q = 0; q < 3; ++q)
-          w[q] = __ldg(reinterpret_cast<const uint2*>(static_cast<const __nv_bfloat16*>(p.residual) + q * p.res_plane + (long long)pix[k] * p.Kout + n));
-      };
-      const int n_first = n_tile * kBN + (g >> 3) * kCols + 4 * (g & 7);
-      // residual planes, requested before the sums are there (the wide tile needs its registers for the sums)
-      constexpr bool kEarlyRes = kNT == 1;
-      uint2 res[kEarlyRes ? 8 : 1][3];
-      if (kEarlyRes && p.residual && !p.res_f32 && n_first < p.Kout) {
-#pragma unroll
-        for (int k = 0; k < 8; ++k)
-          if (pix[k] >= 0) load_res(k, n_first, res[kEarlyRes ? k : 0]);
-      }
-      float sum[kCols];
-#pragma unroll
-      for (int e = 0; e < kCols; ++e) sum[e] = 0.0f;
+      for (int e = 0; e < kCols; ++e) sum[e] = other[kTwo ? e : 0] = 0.0f;
       auto hand_back = [&](uint32_t acc) {
         ptx::tc_fence_before();
         __syncwarp();
         if (lane == 0) ptx::mbar_arrive(d_empty + 8 * acc);
       };
-      // adds a pair's columns (this thread's row) to the sums
-      auto take_pair = [&](uint32_t pair, uint32_t turn) {
+      // adds a pair's columns (this thread's row) to the sums `into`
+      auto take_pair = [&](uint32_t pair, uint32_t turn, float* into) {
         if (!ptx::warp_wait(d_full + 8 * pair, turn & 1u, abort_flag)) return false;
         ptx::tc_fence_after();
 #pragma unroll
-        for (int h = 0; h < kCols / 32; ++h) {
-          uint32_t v[2][32];
+        for (int h = 0; h < kCols / 16; ++h) {
+          uint32_t v[2][16];
 #pragma unroll
-          for (uint32_t j = 0; j < 2; ++j) ptx::tmem_ld_32x32(lane_base + (2 * pair + j) * kBN + h * 32, v[j]);
+          for (uint32_t j = 0; j < 2; ++j) ptx::tmem_ld_32x16(lane_base + (2 * pair + j) * kBN + h * 16, v[j]);
           ptx::tmem_ld_wait();
-          if (h == kCols / 32 - 1) hand_back(pair);
+          if (h == kCols / 16 - 1) hand_back(pair);
 #pragma unroll
-          for (int e = 0; e < 32; ++e) sum[h * 32 + e] += __uint_as_float(v[0][e]) + __uint_as_float(v[1][e]);
+          for (int e = 0; e < 16; ++e) into[h * 16 + e] += __uint_as_float(v[0][e]) + __uint_as_float(v[1][e]);
         }
         return true;
       };
-      // adds small products; `cut` of the sum is given back with the last of them, whose low bits decide how it rounds.  An
-      // infinite or NaN operand has made the sum what it has to be; its small products (inf * 0, inf - inf) say nothing.
-      auto take_small = [&](float cut) {
+      // adds small products; kCut of the sum is given back with the last of them, whose low bits decide how it rounds.  An
+      // infinite or NaN operand makes the large products what they have to be; its small products (inf * 0, inf - inf) say nothing.
+      auto take_small = [&](bool last) {
         const uint32_t acc = kPairs + (small & 1u);
         if (!ptx::warp_wait(d_full + 8 * acc, (small >> 1) & 1u, abort_flag)) return false;
         ptx::tc_fence_after();
 #pragma unroll
-        for (int h = 0; h < kCols / 32; ++h) {
-          uint32_t v[32];
-          ptx::tmem_ld_32x32(lane_base + kSmallCols + (small & 1u) * kBN + h * 32, v);
+        for (int h = 0; h < kCols / 16; ++h) {
+          uint32_t v[16], w[HALO ? 16 : 1];
+          ptx::tmem_ld_32x16(lane_base + kSmallCols + (small & 1u) * (HALO ? 2 * kBN : kBN) + h * 16, v);
+          if constexpr (HALO) ptx::tmem_ld_32x16(lane_base + kSmallCols + (small & 1u) * 2 * kBN + kBN + h * 16, w);
           ptx::tmem_ld_wait();
-          if (h == kCols / 32 - 1) hand_back(acc);
+          if (h == kCols / 16 - 1) hand_back(acc);
 #pragma unroll
-          for (int e = 0; e < 32; ++e) {
-            const float s = sum[h * 32 + e], t = s + fmaf(s, cut, __uint_as_float(v[e]));
-            sum[h * 32 + e] = fabsf(s) <= FLT_MAX ? t : s;
+          for (int e = 0; e < 16; ++e) {
+            float rest = HALO ? __uint_as_float(v[e]) + __uint_as_float(w[HALO ? e : 0]) : __uint_as_float(v[e]);
+            rest = fabsf(rest) <= FLT_MAX ? rest : 0.0f;
+            float& s = sum[h * 16 + e];
+            if (!last) { s += rest; continue; }
+            if (kTwo) s += other[kTwo ? h * 16 + e : 0];
+            s = fabsf(s) <= FLT_MAX ? s + fmaf(s, kCut, rest) : s;
           }
         }
         ++small;
         return true;
       };
       for (int kb = kb0; kb < kb1 && okw; ++kb) {
-        for (int k4 = 0; k4 < 4 && okw; k4 += 2, ++large) okw = take_pair(large % kPairs, large / kPairs);
-        if (okw && ((kb - kb0) % kSmallBlocks == kSmallBlocks - 1 || kb + 1 == kb1)) okw = take_small(kb + 1 == kb1 ? kCut : 0.0f);
+        okw = take_pair(large % kPairs, large / kPairs, sum);
+        ++large;
+        okw = okw && take_pair(large % kPairs, large / kPairs, kTwo ? other : sum);
+        ++large;
+        if (okw && ((kb - kb0) % kSmallBlocks == kSmallBlocks - 1 || kb + 1 == kb1)) okw = take_small(kb + 1 == kb1);
       }
-      // 64 columns at a time: 32 of either half of the tile
+      // the pixels this thread finishes: row r of the tile -> its index in the output, -1 outside
+      int pix[kRows];
+#pragma unroll
+      for (int k = 0; k < kRows; ++k) {
+        const int rr = (et >> 4) + k * (kEpiThreads / 16), r = row_lo + rr;
+        const int t1 = (int)epi::div_by((uint32_t)r, p.div_mp), tj = r - t1 * p.mp;
+        const int t2 = (int)epi::div_by((uint32_t)t1, p.div_ri), ti = t1 - t2 * p.rows_img;
+        const int img = n0 + t2, oy = oy0 + ti, ox = ox0 + tj;
+        const bool in_tile = !HALO || (tj < p.tw && ti < p.th && t2 < p.tn);
+        pix[k] = in_tile && rr < rows_each && img < p.NB && oy < p.OH && ox < p.OW ? (img * p.OH + oy) * p.OW + ox : -1;
+      }
+      // 64 columns at a time
 #pragma unroll
       for (int pass = 0; pass < kNT; ++pass) {
       const uint32_t turn = (uint32_t)(i * kNT + pass);   // uses of the shared tile
-      const int n = n_first + pass * 32;
+      const int n = n_tile * kBN + pass * 64 + 4 * g;
+      // residual planes, requested before the sums are in the shared tile
+      uint2 res[kRows][3];
+      if (p.residual && !p.res_f32 && n < p.Kout) {
+#pragma unroll
+        for (int k = 0; k < kRows; ++k)
+          if (pix[k] >= 0) {
+#pragma unroll
+            for (int q = 0; q < 3; ++q)
+              res[k][q] = __ldg(reinterpret_cast<const uint2*>(static_cast<const __nv_bfloat16*>(p.residual) + q * p.res_plane + (long long)pix[k] * p.Kout + n));
+          }
+      }
       // the previous item's partial sums have been read by everybody
       if (okw && turn > 0 && S > 1) okw = ptx::warp_wait_cluster(part_done, (turn - 1) & 1u, abort_flag);
       if (!ptx::named_bar_and(1, kEpiThreads, okw)) { okw = false; break; }
+      if (kNT == 1 || part >> 1 == pass) {
+        constexpr int kChunks = kCols / 4;   // 16 bytes each; sixteen chunks a row, those of a row's parts one after another
 #pragma unroll
-      for (int c = 0; c < 8; ++c)
-        epi::sts128(sTile + (uint32_t)row * 256u + (((uint32_t)(half * 8 + c) ^ (uint32_t)(row & 7)) << 4), __float_as_uint(sum[pass * 32 + 4 * c]),
-                    __float_as_uint(sum[pass * 32 + 4 * c + 1]), __float_as_uint(sum[pass * 32 + 4 * c + 2]), __float_as_uint(sum[pass * 32 + 4 * c + 3]));
+        for (int c = 0; c < kChunks; ++c)
+          epi::sts128(sTile + (uint32_t)row * 256u + (((uint32_t)((kNT == 1 ? part : part & 1) * kChunks + c) ^ (uint32_t)(row & 7)) << 4),
+                      __float_as_uint(sum[4 * c]), __float_as_uint(sum[4 * c + 1]), __float_as_uint(sum[4 * c + 2]), __float_as_uint(sum[4 * c + 3]));
+      }
       ptx::named_bar_sync(2, kEpiThreads);
       if (S > 1) {
         if (et < S) ptx::mbar_arrive_remote(ptx::map_to_cta(part_ready, (uint32_t)et));
@@ -441,7 +570,7 @@ conv_f32_kernel(const __grid_constant__ CUtensorMap tm_in, const F32Params p) {
           if (p.shift) shp[e] = __ldg(p.shift + n + e);
         }
 #pragma unroll
-        for (int k = 0; k < 8; ++k) {
+        for (int k = 0; k < kRows; ++k) {
           if (pix[k] < 0) continue;
           const int r = row_lo + (et >> 4) + k * (kEpiThreads / 16);
           const uint32_t at = sTile + (uint32_t)r * 256u + (((uint32_t)g ^ (uint32_t)(r & 7)) << 4);
@@ -462,8 +591,7 @@ conv_f32_kernel(const __grid_constant__ CUtensorMap tm_in, const F32Params p) {
             if (p.res_f32) {
               f = __ldg(reinterpret_cast<const float4*>(static_cast<const float*>(p.residual) + (long long)pix[k] * p.ldo + n));
             } else {
-              if (!kEarlyRes) load_res(k, n, res[0]);
-              f = join4(res[kEarlyRes ? k : 0]);
+              f = join4(res[k]);
             }
             v.x += f.x; v.y += f.y; v.z += f.z; v.w += f.w;
           }
@@ -517,7 +645,7 @@ constexpr int kSABytes = kSM * 128, kSBBytes = kSN * 128;
 constexpr int kSB = 3 * kSABytes, kSStage = kSB + 3 * kSBBytes;   // the pixels' planes, then the filter's, one below the other
 constexpr int kSStages = 6;                             // 216 KB: six blocks of 64 channels
 constexpr size_t kSSmem = 1024 + (size_t)kSStages * kSStage;
-constexpr int kSCopyWarps = 4, kSThreads = (1 + kSCopyWarps + 4) * 32;
+constexpr int kSCopyWarps = 4, kSLargeWarp = 1 + kSCopyWarps + 4, kSThreads = (kSLargeWarp + 1) * 32;
 
 // Loads that stay where they stand (the compiler moves plain ones down to their use, behind the waits they should overlap).
 __device__ __forceinline__ uint2 load_now(const __nv_bfloat16* q) {
@@ -552,7 +680,10 @@ __global__ void __launch_bounds__(kSThreads, 1) conv_f32_small_kernel(const __gr
   const uint32_t rank = S > 1 ? ptx::cluster_ctarank() : 0u;
   if (threadIdx.x == 0) {
     s_abort = 0;
-    for (int i = 0; i < 2 * kSStages; ++i) ptx::mbar_init(full + 8 * i, 1);
+    for (int i = 0; i < kSStages; ++i) {
+      ptx::mbar_init(full + 8 * i, 1);
+      ptx::mbar_init(empty + 8 * i, 2);   // both issuing warps
+    }
     for (int i = 0; i < 2; ++i) {
       ptx::mbar_init(d_full + 8 * i, 1);
       ptx::mbar_init(d_empty + 8 * i, 4);
@@ -580,8 +711,9 @@ __global__ void __launch_bounds__(kSThreads, 1) conv_f32_small_kernel(const __gr
   const int ox0 = (m_item - t2 * p.tiles_x) * p.tw, oy0 = (t2 - t3 * p.tiles_y) * p.th, n0 = t3 * p.tn;
   const int kb_all = p.taps * p.CB, kb0 = kb_all * (int)rank / S, blocks = kb_all * ((int)rank + 1) / S - kb0;   // this CTA's part
 
-  if (warp == 0) {
-    // ------------------------------------------------------------------ MMAs ------------
+  if (warp == 0 || warp == kSLargeWarp) {
+    // ------------------------------------------------------------------ MMAs: large products, small ones ----
+    const bool large_warp = warp == kSLargeWarp;
     const uint32_t issue = ptx::elect_one();
     const uint32_t idesc = ptx::umma_idesc(kSM, kSN, 1), idesc2 = ptx::umma_idesc(kSM, 2 * kSN, 1);
     const uint32_t ring_lo = ptx::smem_desc_k128_lo(ring);
@@ -595,25 +727,27 @@ __global__ void __launch_bounds__(kSThreads, 1) conv_f32_small_kernel(const __gr
     for (int i = 0; i < blocks; ++i) {
       const uint32_t q = (uint32_t)i & 1u, group = (uint32_t)i / kSmallBlocks, sb = group & 1u;
       const bool first = i % kSmallBlocks == 0, last = i % kSmallBlocks == kSmallBlocks - 1 || i + 1 == blocks;
-      if (!ptx::warp_spin(full + 8 * st, par, abort_flag) || (i >= 2 && !ptx::warp_spin(d_empty + 8 * q, (((uint32_t)i >> 1) & 1u) ^ 1u, abort_flag)) ||
-          (first && group >= 2 && !ptx::warp_spin(s_empty + 8 * sb, ((group >> 1) & 1u) ^ 1u, abort_flag))) {
-        okw = false;
-        break;
-      }
-      ptx::tc_fence_after();
+      if (!ptx::warp_spin(full + 8 * st, par, abort_flag)) { okw = false; break; }
       const uint32_t at = ring_lo + st * (uint32_t)(kSStage >> 4), ds = tmem + kSmallCols + sb * 2 * kSN;
+      if (large_warp) {
+        if (i >= 2 && !ptx::warp_spin(d_empty + 8 * q, (((uint32_t)i >> 1) & 1u) ^ 1u, abort_flag)) { okw = false; break; }
+        ptx::tc_fence_after();
 #pragma unroll
-      for (uint32_t k4 = 0; k4 < 4; ++k4) mma(tmem + q * kQuad + k4 * kSN, at, 0, 0, k4, idesc, 0u);
-      ptx::tc_commit(d_full + 8 * q, issue);
-      // the small products in two accumulators side by side: a1 b2 | a1 b3, a2 b1 | a2 b2, a3 b1
+        for (uint32_t k4 = 0; k4 < 4; ++k4) mma(tmem + q * kQuad + k4 * kSN, at, 0, 0, k4, idesc, 0u);
+        ptx::tc_commit(d_full + 8 * q, issue);
+      } else {
+        if (first && group >= 2 && !ptx::warp_spin(s_empty + 8 * sb, ((group >> 1) & 1u) ^ 1u, abort_flag)) { okw = false; break; }
+        ptx::tc_fence_after();
+        // the small products in two accumulators side by side: a1 b2 | a1 b3, a2 b1 | a2 b2, a3 b1
 #pragma unroll
-      for (uint32_t k4 = 0; k4 < 4; ++k4) mma(ds, at, 0, 1, k4, idesc2, first && k4 == 0 ? 0u : 1u);
+        for (uint32_t k4 = 0; k4 < 4; ++k4) mma(ds, at, 0, 1, k4, idesc2, first && k4 == 0 ? 0u : 1u);
 #pragma unroll
-      for (uint32_t k4 = 0; k4 < 4; ++k4) mma(ds, at, 1, 0, k4, idesc2, 1u);
+        for (uint32_t k4 = 0; k4 < 4; ++k4) mma(ds, at, 1, 0, k4, idesc2, 1u);
 #pragma unroll
-      for (uint32_t k4 = 0; k4 < 4; ++k4) mma(ds, at, 2, 0, k4, idesc, 1u);
+        for (uint32_t k4 = 0; k4 < 4; ++k4) mma(ds, at, 2, 0, k4, idesc, 1u);
+        if (last) ptx::tc_commit(s_full + 8 * sb, issue);
+      }
       ptx::tc_commit(empty + 8 * st, issue);
-      if (last) ptx::tc_commit(s_full + 8 * sb, issue);
       if (++st == kSStages) { st = 0; par ^= 1u; }
     }
     if (!okw && lane == 0 && p.error_flag) atomicCAS(p.error_flag, 0, (int)kErrWaitMma);
@@ -675,8 +809,8 @@ __global__ void __launch_bounds__(kSThreads, 1) conv_f32_small_kernel(const __gr
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
       const int rr = (et >> 3) + 16 * k, r = (int)rank * rows_each + rr;
-      const int t1 = (int)epi::div_by((uint32_t)r, p.div_tw), tj = r - t1 * p.tw;
-      const int tt = (int)epi::div_by((uint32_t)t1, p.div_th), ti = t1 - tt * p.th;
+      const int t1 = (int)epi::div_by((uint32_t)r, p.div_mp), tj = r - t1 * p.mp;
+      const int tt = (int)epi::div_by((uint32_t)t1, p.div_ri), ti = t1 - tt * p.rows_img;
       const int img = n0 + tt, oy = oy0 + ti, ox = ox0 + tj;
       pix[k] = live && rr < rows_each && img < p.NB && oy < p.OH && ox < p.OW ? ((long long)img * p.OH + oy) * p.OW + ox : -1;
       if (p.residual && pix[k] >= 0) {
@@ -1084,89 +1218,126 @@ static bool as_matrix(ConvF32Args* a) {
   a->N = a->H = a->OH = 1;
   return true;
 }
-static void f32_tile(const ConvF32Args& a, bool matrix, int bn, int* tw, int* th, int* tn) {
-  if (bn == kSN) {
-    conv_small_tile(a.N, a.OH, a.OW, tw, th, tn);
-  } else if (matrix) {
-    *tw = 128; *th = *tn = 1;
-  } else {
-    tconv_tile(a.N, a.OH, a.OW, tw, th, tn);
+// The pixels of a tile: tn images x th rows x tw columns.  Row r of the tile is column r % mp of row r / mp, rows_img rows an image.
+// Halo tiles (filters of stride 1 and more than one row): one box brings the pixels of a block of 64 channels under a whole column of the
+// filter, and filter row r reads it from its row r on.  mp is a multiple of 8, so that every view is whole groups of eight rows of 128
+// bytes, as the operand's layout has them.  (One box for all taps, 180 pixels for 128 with eight rows 1280 bytes apart, was no faster:
+// 57.2 us and 57.3 for 512 -> 512 on 7x7 by one CTA a tile.)  The tile of the fewest, then of the least to copy.
+struct F32Tile {
+  int tw = 0, th = 0, tn = 1, mp = 0, rows_img = 0;
+  int box_h = 0, box_n = 1;
+  long long tiles = 0;
+  int plane() const { return mp * box_h * box_n * 128; }
+};
+static long long tiles_of(const F32Tile& t, const ConvF32Args& a) {
+  return (long long)((a.OW + t.tw - 1) / t.tw) * ((a.OH + t.th - 1) / t.th) * ((a.N + t.tn - 1) / t.tn);
+}
+constexpr size_t kHaloSmem = 226 * 1024, kHaloFixed = 1024 + kTileBytes, kHaloBlock = 3 * kBBytes;   // all; neither boxes nor weights; a block of weights
+static bool halo_fits(const F32Tile& t) {   // two boxes and three blocks of weights
+  return t.box_h <= 256 && kHaloFixed + 2 * 3 * (size_t)t.plane() + 3 * kHaloBlock <= kHaloSmem;
+}
+static bool halo_tile(const ConvF32Args& a, F32Tile* best) {
+  constexpr int rows = 128;
+  const int R = a.stem ? 4 : a.R;
+  if (!a.stem && (a.stride != 1 || R == 1)) return false;
+  bool found = false;
+  auto offer = [&](F32Tile t) {
+    t.tiles = tiles_of(t, a);
+    if (!halo_fits(t) || (found && (t.tiles > best->tiles || (t.tiles == best->tiles && t.plane() >= best->plane())))) return;
+    *best = t;
+    found = true;
+  };
+  for (int mp : {8, 16, 32, 64, 128, (a.OW + 7) & ~7}) {
+    if (mp > rows || mp >= a.OW + 8) continue;
+    F32Tile t;
+    t.mp = mp;
+    t.tw = mp < a.OW ? mp : a.OW;
+    t.th = a.OH < rows / mp ? a.OH : rows / mp;
+    t.rows_img = 256;
+    t.box_h = t.th + R - 1;
+    offer(t);
+    // whole images one below the other: the row above an image is zero and serves the one before as the row below
+    const int images = (rows / mp + 1) / (a.OH + 1);
+    if (!a.stem && R == 3 && a.pad == 1 && images > 1) {
+      t.th = a.OH;
+      t.rows_img = t.box_h = a.OH + 1;
+      t.tn = images;
+      t.box_n = images + 1;
+      offer(t);
+    }
   }
+  return found;
+}
+static F32Tile f32_tile(const ConvF32Args& a, bool matrix, int bn) {
+  F32Tile t;
+  if (bn == kSN) {
+    conv_small_tile(a.N, a.OH, a.OW, &t.tw, &t.th, &t.tn);
+  } else if (matrix) {
+    t.tw = 128;
+    t.th = 1;
+  } else {
+    tconv_tile(a.N, a.OH, a.OW, &t.tw, &t.th, &t.tn);
+  }
+  t.mp = t.tw;
+  t.rows_img = t.th;
+  t.tiles = tiles_of(t, a);
+  return t;
 }
 // Clusters of s CTAs with tiles of bn columns that run at once.  Fewer fit the GPU than its SMs would hold (they do not cross GPC
 // borders), so the runtime is asked.
 static int clusters_that_fit(int bn, int s, int sms) {
   static const ClusterFit small = cluster_fit(conv_f32_small_kernel, kSThreads, kSSmem, sms);
-  static const ClusterFit wide = cluster_fit(conv_f32_kernel<64>, kThreads, Ring<64>::kSmem, sms);
-  static const ClusterFit wider = cluster_fit(conv_f32_kernel<128>, kThreads, Ring<128>::kSmem, sms);
+  static const ClusterFit wide = cluster_fit(conv_f32_kernel<64, false>, kThreads, Ring<64>::kSmem, sms);
+  static const ClusterFit wider = cluster_fit(conv_f32_kernel<128, false>, kThreads, Ring<128>::kSmem, sms);
   return bn == kSN ? small.of[s] : bn == 64 ? wide.of[s] : wider.of[s];
 }
 
-// Tile width and the CTAs of a cluster that share a tile's reduction: the pair with the least rounds x time, in clocks.  Wide tiles: a
-// block of 64 channels takes about 1560 with 64 columns and 2000 with 128 when every SM works (both bound by L2 -> shared memory, 46 to
-// 48 bytes a clock and SM: 72 and 96 KB; 3x3 filters of 256 and 512 channels at batch 64); everything else about 4700 and 12000 a tile
-// (the widest is finished in two passes), a split 1500 more.  Clusters of sixteen were slower at batch 1 than clusters of eight (21 us
-// against 15 for a layer of 256 channels on 16 x 16 pixels).
-// 64 x 32 tiles: 820 a block, 6000 besides, 2600 for sending, beside a launch of wide ones that starts 7000 later.  Fitted to 376 layers
-// of 1 to 64 images (ResNet-18's and ResNet-50's, and random ones), each at every tile and split: the choice takes 0.7 % more than the
-// fastest, and 6 layers take 3 % more than on wide tiles.  (With 620, 4500, 1000 and 5000, which leave the small tiles' launch out, it
-// was 43 layers: 11x12x8x168 -> 192 3x3 22.4 us for 15.8.)  On either side of the line, us (64 x 32, wide): 14x14x256 -> 256 3x3 of one
-// image 11.0 13.4, of two 14.9 16.7, of three 21.2 17.1; 28x28x128 -> 256 3x3 stride 2 of two 11.4 13.4, of four 14.2 14.5;
-// 7x7x512 -> 2048 of two 9.1 10.9, of three 15.5 12.6.
+// Tile width and the CTAs of a cluster that share a tile's reduction: the pair with the least rounds x time, in clocks.  A block of 64
+// channels, as measured by one CTA a tile: 560 on 64 x 32 tiles, on 128 x 64 tiles 1220 with halo tiles and 1450 without (which fill
+// better on narrow maps), on 128 x 128 tiles 1920; without boxes the copies of all SMs together allow 1565 and 2087.  A tile's beginning
+// and end 9000, 5560 and 11100 (the widest is finished in two passes), a launch of wide tiles 6700 more, a split 2700 or 2000: fitted to
+// 190 layers of 1 to 32 images (ResNet-18's and ResNet-50's, and random ones), each at every tile and split, of which the choice takes
+// 0.3 % more than the fastest.  On either side of the lines, us: 14x14x256 -> 256 3x3 of one image 64 x 32 10.4, wide 11.4; 7x7x512 -> 512
+// of one 12.6 and 15.1; 28x28x128 of eight 128 x 64 22.0, 128 x 128 23.9, 64 x 32 39.8.  Clusters of sixteen were slower at batch 1 than
+// clusters of eight (21 us against 15 for 256 channels on 16 x 16 pixels).
 void conv_f32_choose(ConvF32Args* args) {
+  if (args->chosen) return;
+  args->chosen = 1;
   ConvF32Args a = *args;
   const bool matrix = as_matrix(&a);
   const int kb_all = (a.stem ? 4 : a.R * a.S) * (a.stem ? 1 : (a.C + 63) / 64), stride = a.stem ? 1 : a.stride, sms = a.sm_count > 0 ? a.sm_count : 148;
   double best = 1e30;
+  F32Tile box;
+  const bool boxes = args->halo >= 0 && halo_tile(a, &box);
   for (int forced = 2; forced >= 0 && best == 1e30; --forced)   // what was asked for, the tile alone, neither
     for (int b : {64, 128, kSN}) {
       if ((b == 128 && a.Kout <= 64) || (forced >= 1 && a.bn != 0 && b != a.bn)) continue;
-      int tw, th, tn;
-      f32_tile(a, matrix, b, &tw, &th, &tn);
-      if (b == kSN && (tw > th ? tw : th) * stride > 256) continue;
-      const long long tiles = (long long)((a.OW + tw - 1) / tw) * ((a.OH + th - 1) / th) * ((a.N + tn - 1) / tn) * ((a.Kout + b - 1) / b);
-      for (int s = 1; s <= 8 && s <= kb_all; s *= 2) {
-        if (forced == 2 && a.splits != 0 && s != a.splits) continue;
-        const int slots = clusters_that_fit(b, s, sms), blocks = (kb_all + s - 1) / s;
-        const double rounds = (double)((tiles + slots - 1) / slots);
-        const double t = b == kSN ? rounds * (blocks * 820.0 + 6000.0 + (s > 1 ? 2600.0 : 0.0))
-                                  : rounds * (blocks * (b == 64 ? 1560.0 : 2000.0) + (b == 64 ? 4700.0 : 12000.0)) + 7000.0 + (s > 1 ? 1500.0 : 0.0);
-        if (t < best) { best = t; args->bn = b; args->splits = s; }
+      for (int halo = 0; halo < (b == 64 && boxes ? 2 : 1); ++halo) {
+        if (!halo && b == 64 && boxes && a.halo > 0) continue;
+        const F32Tile t = halo ? box : f32_tile(a, matrix, b);
+        if (b == kSN && (t.tw > t.th ? t.tw : t.th) * stride > 256) continue;
+        const long long tiles = t.tiles * ((a.Kout + b - 1) / b);
+        for (int s = 1; s <= 8 && s <= kb_all; s *= 2) {
+          if (forced == 2 && a.splits != 0 && s != a.splits) continue;
+          const int slots = clusters_that_fit(b, s, sms), blocks = (kb_all + s - 1) / s;
+          const double rounds = (double)((tiles + slots - 1) / slots), load = (double)(std::min<long long>(tiles, slots) * s) / sms;
+          const double block = b == kSN ? 560.0 : halo ? 1220.0 : b == 64 ? std::max(1450.0, 1565.0 * load) : std::max(1920.0, 2087.0 * load);
+          const double cost = b == kSN ? rounds * (blocks * block + 9000.0 + (s > 1 ? 2700.0 : 0.0))
+                                       : rounds * (blocks * block + (b == 64 ? 5560.0 : 11100.0)) + 6700.0 + (s > 1 ? 2000.0 : 0.0);
+          if (cost < best) { best = cost; args->bn = b; args->splits = s; args->halo = halo ? 1 : -1; }
+        }
       }
     }
 }
 
-template <int BN>
-static cudaError_t launch_f32_cfg(const CUtensorMap& tm, const F32Params& p, int sms, cudaStream_t stream) {
-  cudaError_t e = cudaFuncSetAttribute(conv_f32_kernel<BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Ring<BN>::kSmem);
+template <typename Kern>
+static cudaError_t launch_f32(Kern kern, int threads, size_t smem, int ctas, const CUtensorMap& tm, const F32Params& p, cudaStream_t stream) {
+  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;
-  const int slots = clusters_that_fit(BN, p.splits, sms);
-  const int clusters = p.items < slots ? p.items : slots;
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3((unsigned)(clusters * p.splits));
-  cfg.blockDim = dim3(kThreads);
-  cfg.dynamicSmemBytes = Ring<BN>::kSmem;
-  cfg.stream = stream;
-  cudaLaunchAttribute attr[2];
-  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[0].val.programmaticStreamSerializationAllowed = 1;
-  attr[1].id = cudaLaunchAttributeClusterDimension;
-  attr[1].val.clusterDim.x = (unsigned)p.splits;
-  attr[1].val.clusterDim.y = 1;
-  attr[1].val.clusterDim.z = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = p.splits > 1 ? 2 : 1;
-  return cudaLaunchKernelEx(&cfg, conv_f32_kernel<BN>, tm, p);
-}
-
-static cudaError_t launch_f32_small(const CUtensorMap& tm, const F32Params& p, cudaStream_t stream) {
-  cudaError_t e = cudaFuncSetAttribute(conv_f32_small_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSSmem);
-  if (e != cudaSuccess) return e;
-  if ((long long)p.items * p.splits > 0x7fffffffLL) return cudaErrorInvalidValue;
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3((unsigned)(p.items * p.splits));
-  cfg.blockDim = dim3(kSThreads);
-  cfg.dynamicSmemBytes = kSSmem;
+  cfg.gridDim = dim3((unsigned)ctas);
+  cfg.blockDim = dim3((unsigned)threads);
+  cfg.dynamicSmemBytes = smem;
   cfg.stream = stream;
   cudaLaunchAttribute attr[2];
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
@@ -1176,7 +1347,7 @@ static cudaError_t launch_f32_small(const CUtensorMap& tm, const F32Params& p, c
   attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
   cfg.attrs = attr;
   cfg.numAttrs = p.splits > 1 ? 2 : 1;
-  return cudaLaunchKernelEx(&cfg, conv_f32_small_kernel, tm, p);
+  return cudaLaunchKernelEx(&cfg, kern, tm, p);
 }
 
 cudaError_t launch_conv_f32(const ConvF32Args& args, cudaStream_t stream) {
@@ -1199,24 +1370,32 @@ cudaError_t launch_conv_f32(const ConvF32Args& args, cudaStream_t stream) {
   const long long pixels = (long long)a.N * a.OH * a.OW;
   if (pixels > 0x7fffffffLL) return cudaErrorInvalidValue;
   p.res_plane = p.out_plane = pixels * a.Kout;
-  int tw, th, tn;
-  f32_tile(a, matrix, 64, &tw, &th, &tn);
-  if (!conv_f32_supported(stem ? 64 : a.C, a.Kout, (tw > th ? tw : th) * p.stride)) return cudaErrorInvalidValue;
+  const F32Tile wide = f32_tile(a, matrix, 64);
+  if (!conv_f32_supported(stem ? 64 : a.C, a.Kout, (wide.tw > wide.th ? wide.tw : wide.th) * p.stride)) return cudaErrorInvalidValue;
   if ((reinterpret_cast<uintptr_t>(a.in) & 15) || (reinterpret_cast<uintptr_t>(a.out) & 15) || (reinterpret_cast<uintptr_t>(a.residual) & (a.res_f32 ? 15 : 7)) ||
       ((a.out_f32 || a.res_f32) && a.ldo % 4 != 0))
     return cudaErrorMisalignedAddress;
   conv_f32_choose(&a);
   const int bn = a.bn, sms = a.sm_count > 0 ? a.sm_count : 148;
-  f32_tile(a, matrix, bn, &tw, &th, &tn);
+  F32Tile t = f32_tile(a, matrix, bn);
+  if (a.halo > 0 && !halo_tile(a, &t)) return cudaErrorInvalidValue;
   p.splits = a.splits;
-  p.tw = tw; p.th = th; p.tn = tn;
-  p.tiles_x = (a.OW + tw - 1) / tw; p.tiles_y = (a.OH + th - 1) / th;
+  p.tw = t.tw; p.th = t.th; p.tn = t.tn; p.mp = t.mp; p.rows_img = t.rows_img;
+  p.tiles_x = (a.OW + t.tw - 1) / t.tw; p.tiles_y = (a.OH + t.th - 1) / t.th;
   p.n_tiles = (a.Kout + bn - 1) / bn;
-  const long long items = (long long)p.tiles_x * p.tiles_y * ((a.N + tn - 1) / tn) * p.n_tiles;
-  if (items <= 0 || items > 0x7fffffffLL) return cudaErrorInvalidValue;
+  const long long items = t.tiles * p.n_tiles;
+  if (items <= 0 || items * a.splits > 0x7fffffffLL) return cudaErrorInvalidValue;
   p.items = (int)items;
   p.div_tx = epi::fast_div((uint32_t)p.tiles_x); p.div_ty = epi::fast_div((uint32_t)p.tiles_y); p.div_nt = epi::fast_div((uint32_t)p.n_tiles);
-  p.div_tw = epi::fast_div((uint32_t)tw); p.div_th = epi::fast_div((uint32_t)th);
+  p.div_mp = epi::fast_div((uint32_t)t.mp); p.div_ri = epi::fast_div((uint32_t)t.rows_img);
+  size_t smem = bn == kSN ? kSSmem : bn == 64 ? Ring<64>::kSmem : Ring<128>::kSmem;
+  if (a.halo > 0) {
+    // two boxes, weights in the rest
+    p.R = stem ? 4 : a.R;
+    p.a_plane = t.plane();
+        p.b_stages = (int)std::min((kHaloSmem - kHaloFixed - 3 * (size_t)p.a_plane * kBoxes) / kHaloBlock, (size_t)kHaloB);
+    smem = kHaloFixed + 3 * (size_t)p.a_plane * kBoxes + kHaloBlock * p.b_stages;
+  }
 
   auto enc = f32_get_encode();
   if (!enc) return cudaErrorNotSupported;
@@ -1231,14 +1410,20 @@ cudaError_t launch_conv_f32(const ConvF32Args& args, cudaStream_t stream) {
     gdim[0] = (cuuint64_t)a.C; gdim[1] = (cuuint64_t)a.W; gdim[2] = (cuuint64_t)a.H; gdim[3] = (cuuint64_t)a.N; gdim[4] = 3;
     gstr[0] = px; gstr[1] = px * a.W; gstr[2] = px * a.W * a.H; gstr[3] = px * a.W * a.H * a.N;
   }
-  cuuint32_t box[5] = {64, (cuuint32_t)(tw * p.stride), (cuuint32_t)(th * p.stride), (cuuint32_t)tn, 1};
+  cuuint32_t box[5] = {64, (cuuint32_t)(t.tw * p.stride), (cuuint32_t)(t.th * p.stride), (cuuint32_t)t.tn, 1};
+  if (a.halo > 0) { box[1] = (cuuint32_t)t.mp; box[2] = (cuuint32_t)t.box_h; box[3] = (cuuint32_t)t.box_n; }
   cuuint32_t estr[5] = {1, (cuuint32_t)p.stride, (cuuint32_t)p.stride, 1, 1};
   CUtensorMap tm;
   if (enc(&tm, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 5, const_cast<void*>(a.in), gdim, gstr, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
           CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
     return cudaErrorInvalidValue;
-  if (bn == kSN) return launch_f32_small(tm, p, stream);
-  return bn == 64 ? launch_f32_cfg<64>(tm, p, sms, stream) : launch_f32_cfg<128>(tm, p, sms, stream);
+  if (bn == kSN) {
+    return launch_f32(conv_f32_small_kernel, kSThreads, smem, p.items * p.splits, tm, p, stream);
+  }
+  const int slots = clusters_that_fit(bn, p.splits, sms), ctas = (p.items < slots ? p.items : slots) * p.splits;
+  if (a.halo > 0) return launch_f32(conv_f32_kernel<64, true>, kThreads, smem, ctas, tm, p, stream);
+  return bn == 64 ? launch_f32(conv_f32_kernel<64, false>, kThreads, smem, ctas, tm, p, stream)
+                  : launch_f32(conv_f32_kernel<128, false>, kThreads, smem, ctas, tm, p, stream);
 }
 
 }  // namespace nncv_b200

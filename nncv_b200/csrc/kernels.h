@@ -207,6 +207,8 @@ struct ConvF32Args {
   int N = 0, H = 0, W = 0, C = 0, OH = 0, OW = 0, Kout = 0, R = 1, S = 1, stride = 1, pad = 0;
   int relu = 0;
   int bn = 0, splits = 0;           // output channels of a tile (32: the 64 x 32 tiles, 64, 128) and CTAs that share its reduction; 0: as modelled
+  int chosen = 0;                   // bn, splits and halo are what conv_f32_choose made of them
+  int halo = 0;                     // 64 columns: one box of pixels for a column of the filter (1; where that fits), a copy for every tap (-1); 0: as modelled
   int sm_count = 0;
   int* error_flag = nullptr;
 };

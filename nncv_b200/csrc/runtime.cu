@@ -531,7 +531,7 @@ int conv_run_planes(nncv_b200_conv* c, const void* in, bool stem, int N, int H, 
   a.OH = (H + 2 * c->pad - c->R) / c->stride + 1;
   a.OW = (W + 2 * c->pad - c->S) / c->stride + 1;
   a.relu = relu; a.sm_count = g_dev.sm_count; a.error_flag = g_dev.error_flag;
-  if (c->cfg3.bn == kSmallBN || c->cfg3.bn == 64 || c->cfg3.bn == 128) { a.bn = c->cfg3.bn; a.splits = c->cfg3.mt; }
+  if (c->cfg3.bn == kSmallBN || c->cfg3.bn == 64 || c->cfg3.bn == 128) { a.bn = c->cfg3.bn; a.splits = c->cfg3.mt; a.halo = c->cfg3.resident == 1 ? -1 : c->cfg3.resident == 2 ? 1 : 0; }
   conv_f32_choose(&a);
   const double Ms = (double)N * a.OH * a.OW;
   prof_begin(1, 2.0 * Ms * c->Kout * c->C * c->R * c->S,
