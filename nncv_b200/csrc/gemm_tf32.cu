@@ -45,6 +45,7 @@ constexpr int kBN = 128;                   // N tile
 constexpr int kConvWarps = 4, kConvGroups = 3, kEpiWarps = 4;
 constexpr int kConvThreads = kConvWarps * 32, kEpiThreads = kEpiWarps * 32;
 constexpr int kThreads = 64 + kConvGroups * kConvThreads + kEpiThreads;
+static_assert(64 <= 4 * (kThreads / 32), "four rows a warp finish half of a tile");
 constexpr int kTile = 128 * 128;           // bytes of one operand tile: 128 rows (pixels of A / columns of B) x 32 fp32
 constexpr int kStageBytes = 3 * kTile;     // A as it came, B hi, B lo
 constexpr int kStages = 4;
@@ -56,6 +57,22 @@ constexpr int kSlabBytes = 128 * 128;      // 128 rows x 32 fp32
 // leaves no error of one sign to pile up over a long k loop (cutting gave rel-L2 1.5e-5 at K = 2048).
 __device__ __forceinline__ float tf32_round(float x) {
   return __uint_as_float((__float_as_uint(x) + 0x1000u) & 0xFFFFE000u);
+}
+
+// A load that is under way until its value is used.  (As `inside ? load : 0` the value was waited for where it was chosen: a converter
+// group stood 2200 clocks of the 4300 of a block before it asked for its next stage.)
+__device__ __forceinline__ float load_or_zero(const float* q, bool inside) {
+  float v;
+  asm volatile(
+      "{\n"
+      ".reg .pred p;\n"
+      "setp.ne.u32 p, %2, 0;\n"
+      "mov.f32 %0, 0f00000000;\n"
+      "@p ld.global.nc.f32 %0, [%1];\n"
+      "}\n"
+      : "=&f"(v)
+      : "l"(q), "r"((uint32_t)inside));
+  return v;
 }
 
 struct GtParams {
@@ -201,7 +218,7 @@ gemm_tf32x3_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_consta
       const int n = n0 + t, k0 = (kb_lo + (int)(cnt - i * len)) * 32;
       const float* bp = p.B + (size_t)k0 * p.N + n;
 #pragma unroll
-      for (int k = 0; k < 32; ++k) bv[k] = (n < p.N && k0 + k < p.K) ? __ldg(bp + (size_t)k * p.N) : 0.0f;
+      for (int k = 0; k < 32; ++k) bv[k] = load_or_zero(bp + (size_t)k * p.N, n < p.N && k0 + k < p.K);
       return true;
     };
     {
@@ -343,17 +360,23 @@ gemm_tf32x3_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_consta
     const int n = n0 + lane * 4, rows = 128 / S;
     float4 bias = make_float4(0.f, 0.f, 0.f, 0.f);
     if (p.bias && n < p.N) bias = make_float4(__ldg(p.bias + n), __ldg(p.bias + n + 1), __ldg(p.bias + n + 2), __ldg(p.bias + n + 3));
-    for (int r = rank * rows + warp; r < (rank + 1) * rows; r += kThreads / 32) {
-      if (n >= p.N || m0 + r >= p.M || s_abort) continue;
-      const uint32_t at = sRing + (uint32_t)r * (kBN * 4) + (((uint32_t)lane ^ (uint32_t)(r & 7)) << 4);
-      float4 part[8];
+    // a warp's rows, at most 8 / S of them: the parts of all are asked for before the first is added (row by row 4200 clocks)
+    float4 part[8];
+    auto row_of = [&](int e) { return rank * rows + warp + e / S * (kThreads / 32); };
+    auto mine = [&](int r) { return r < (rank + 1) * rows && n < p.N && m0 + r < p.M && !s_abort; };
 #pragma unroll
-      for (int q = 0; q < 8; ++q)
-        if (q < S) part[q] = ptx::ld_cluster_f4(ptx::map_to_cta(at, (uint32_t)q));
-      float4 v = part[0];
+    for (int e = 0; e < 8; ++e) {
+      const int r = row_of(e);
+      if (mine(r)) part[e] = ptx::ld_cluster_f4(ptx::map_to_cta(sRing + (uint32_t)r * (kBN * 4) + (((uint32_t)lane ^ (uint32_t)(r & 7)) << 4), (uint32_t)(e % S)));
+    }
+    float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
-      for (int q = 1; q < 8; ++q)
-        if (q < S) { v.x += part[q].x; v.y += part[q].y; v.z += part[q].z; v.w += part[q].w; }
+    for (int e = 0; e < 8; ++e) {
+      const int r = row_of(e);
+      if (!mine(r)) continue;
+      if (e % S == 0) v = part[e];
+      else { v.x += part[e].x; v.y += part[e].y; v.z += part[e].z; v.w += part[e].w; }
+      if (e % S != S - 1) continue;
       v.x += bias.x; v.y += bias.y; v.z += bias.z; v.w += bias.w;
       if (p.relu) {
         v.x = !(v.x <= 0.0f) ? v.x : 0.0f; v.y = !(v.y <= 0.0f) ? v.y : 0.0f;
