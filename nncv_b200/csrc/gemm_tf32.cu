@@ -12,21 +12,22 @@
 // Alo*Blo term being about 2^-24 of the product.
 // Data path: kind::tf32 takes K-major operands only (an MN-major B, which the 16-bit kinds accept,
 // gives wrong products -- measured), so the row-major B[K,N] is transposed on the way in.  TMA lands
-// 128 x 32 fp32 tiles of A with the 128-byte swizzle; three groups of four converter warps take the
-// stages in turn.  A thread owns one column n of the 32 x 128 B tile: its 32 k values come with coalesced
-// global loads (a warp reads 128 contiguous bytes of a row of B per load) that are under way while the
-// group waits for its stage, and it writes them as row n of the K-major hi and lo tiles in the swizzled
-// layout.  It also owns one row of A, which it splits into TENSOR MEMORY: the MMAs then read only B from
-// shared memory, 4 KB instead of 8 in the 64 clocks that 128 bytes a clock allow for.  One warp issues
+// 128 x 32 fp32 tiles of A with the 128-byte swizzle and 32 x 128 tiles of B as they lie; three groups of four
+// converter warps take the stages in turn.  A thread owns one row of A, which it splits into TENSOR MEMORY: the MMAs then
+// read only B from shared memory, 4 KB instead of 8 in the 64 clocks that 128 bytes a clock allow for.  It also owns one column
+// n of B; when the whole group has its values in registers, the hi and lo parts go, K-major and swizzled, where B and A
+// came, so that a stage is 32 KB and six fit.  (With global loads of B by its thread the group stood 2000 clocks of 3450
+// issuing them, 32 a block; with a place of its own for the lo part four stages fit, as long as the way from one use of a
+// stage to the next.)  One warp issues
 // 3 x 4 MMAs per stage; four epilogue warps drain the accumulator through a swizzled staging slab and TMA
-// stores.  TMEM holds one pair of accumulators and the A parts of four stages: a second pair would hide
+// stores.  TMEM holds one pair of accumulators and the A parts of four blocks: a second pair would hide
 // the 2 us of an epilogue, but leaves no room for A (2048 x 2048 x 256 takes as long either way).
-// With fewer tiles than SMs, clusters share a tile's k blocks (see the launch).  What bounds it now: the
-// converters' chain, 1700 clocks a block of 32 in three groups, and for small matrices 13 us of launch, cold
-// reads and epilogue.  Out-of-range rows/columns read as zero and are clipped on store, so N and K need
-// only be multiples of 4 (16-byte row pitches of A and C).
-// Cold L2, us, before the clusters and A in tensor memory and with them: 1024^3 41.0, 25.6; 2048^3 137, 122;
-// 100x1000x2048 69.6, 19.5; 1900x1500x520 44.0, 39.9.
+// With fewer tiles than SMs, clusters share a tile's k blocks (see the launch).  What bounds it now: 880 clocks a block of 32, where its
+// MMAs take 780; for small matrices the 3500 clocks to the first MMA and, with clusters, the 5000 after the last one: 32 KB of partial
+// sums come from the other CTA at about 16 bytes a clock.  Out-of-range rows/columns read as zero and are clipped on store, so N and K
+// need only be multiples of 4 (16-byte row pitches of A, B and C).
+// us, inputs in L2, with B by global loads and now: 1024^3 20.2 15.5; 2048^3 112 77; 100x1000x2048 14.0 12.5; 1900x1500x520 37.7 29.0;
+// 4096x4096x512 112 91; 128x128x4096 19.9 16.0.
 // Every wait is bounded and abortable; a timed-out wait sets the device status word.
 #include <cuda.h>
 #include <cudaTypedefs.h>
@@ -47,9 +48,9 @@ constexpr int kConvThreads = kConvWarps * 32, kEpiThreads = kEpiWarps * 32;
 constexpr int kThreads = 64 + kConvGroups * kConvThreads + kEpiThreads;
 static_assert(64 <= 4 * (kThreads / 32), "four rows a warp finish half of a tile");
 constexpr int kTile = 128 * 128;           // bytes of one operand tile: 128 rows (pixels of A / columns of B) x 32 fp32
-constexpr int kStageBytes = 3 * kTile;     // A as it came, B hi, B lo
-constexpr int kStages = 4;
-// TMEM: the accumulators of the hi*hi products and of the cross terms, then A hi and A lo of every stage
+constexpr int kStageBytes = 2 * kTile;     // A and B as they came, then B lo and B hi in their places
+constexpr int kStages = 6, kAStages = 4;   // and parts of A in tensor memory
+// TMEM: the accumulators of the hi*hi products and of the cross terms, then A hi and A lo of kAStages blocks
 constexpr uint32_t kTmemA = 2 * kBN, kTmemStage = 64;
 constexpr int kSlabBytes = 128 * 128;      // 128 rows x 32 fp32
 
@@ -59,8 +60,7 @@ __device__ __forceinline__ float tf32_round(float x) {
   return __uint_as_float((__float_as_uint(x) + 0x1000u) & 0xFFFFE000u);
 }
 
-// A load that is under way until its value is used.  (As `inside ? load : 0` the value was waited for where it was chosen: a converter
-// group stood 2200 clocks of the 4300 of a block before it asked for its next stage.)
+// A load that is under way until its value is used (as `inside ? load : 0` the value is waited for where it is chosen).
 __device__ __forceinline__ float load_or_zero(const float* q, bool inside) {
   float v;
   asm volatile(
@@ -77,17 +77,17 @@ __device__ __forceinline__ float load_or_zero(const float* q, bool inside) {
 
 struct GtParams {
   const float* bias;
-  const float* B;
   float* C;
   int* error_flag;
   int M, N, K;
   int m_tiles, n_tiles, k_blocks;
   int relu;
-  int splits;   // CTAs of a cluster that share a tile's k blocks (then every cluster has one tile); 1: no clusters
+  int splits_log;   // (as a power of two) CTAs of a cluster that share a tile's k blocks (then every cluster has one tile); 1: no clusters
 };
 
 __global__ void __launch_bounds__(kThreads, 1)
-gemm_tf32x3_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ CUtensorMap tm_c, const GtParams p) {
+gemm_tf32x3_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ CUtensorMap tm_b, const __grid_constant__ CUtensorMap tm_c,
+                   const GtParams p) {
   extern __shared__ uint8_t smem_raw[];
   __shared__ int s_abort;
   const uint32_t raw = ptx::smem_u32(smem_raw);
@@ -96,7 +96,7 @@ gemm_tf32x3_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_consta
   const uint32_t sStage = sRing + kStages * kStageBytes;
   const uint32_t bars = sStage + 2 * kSlabBytes;
   const uint32_t full = bars, conv = bars + 8 * kStages, empty = conv + 8 * kStages;
-  const uint32_t acc_full = empty + 8 * kStages, acc_empty = acc_full + 8;
+  const uint32_t a_empty = empty + 8 * kStages, acc_full = a_empty + 8 * kAStages, acc_empty = acc_full + 8;
   const uint32_t tmem_slot = acc_empty + 8;
   {
     uint32_t dyn_bytes;
@@ -114,36 +114,40 @@ gemm_tf32x3_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_consta
       ptx::mbar_init(conv + 8 * i, kConvThreads);
       ptx::mbar_init(empty + 8 * i, 1);
     }
+    for (int i = 0; i < kAStages; ++i) ptx::mbar_init(a_empty + 8 * i, 1);
     ptx::mbar_init(acc_full, 1);
     ptx::mbar_init(acc_empty, kEpiThreads);
     ptx::mbar_fence_init();
     ptx::prefetch_tensormap(&tm_a);
-    ptx::prefetch_tensormap(&tm_c);
+    ptx::prefetch_tensormap(&tm_b);
+    if (p.splits_log == 0) ptx::prefetch_tensormap(&tm_c);
   }
   if (warp == 1) {
-    ptx::tmem_alloc(tmem_slot, kTmemA + kStages * kTmemStage);
+    ptx::tmem_alloc(tmem_slot, kTmemA + kAStages * kTmemStage);
     ptx::tmem_relinquish();
   }
   ptx::tc_fence_before();
   __syncthreads();
   ptx::tc_fence_after();
   const uint32_t tmem_base = (uint32_t)ptx::warp_uniform(*reinterpret_cast<volatile int*>(smem_raw + (tmem_slot - raw)));
-  ptx::grid_dependency_wait();
-  ptx::grid_launch_dependents();
   volatile int* abort_flag = &s_abort;
 
+  // all of this before the wait for the previous kernel: with 64-bit divisions behind it the first copy left 1700 clocks later
   const int total = p.m_tiles * p.n_tiles;
-  const int S = p.splits;
+  const int S = 1 << p.splits_log, first = (int)blockIdx.x >> p.splits_log, step = (int)gridDim.x >> p.splits_log;
   const int rank = S > 1 ? (int)ptx::cluster_ctarank() : 0;
-  const int kb_lo = (int)((long long)p.k_blocks * rank / S), kb_hi = (int)((long long)p.k_blocks * (rank + 1) / S);
+  const int kb_lo = (p.k_blocks * rank) >> p.splits_log, kb_hi = (p.k_blocks * (rank + 1)) >> p.splits_log;
+  const int first_mt = first / p.n_tiles;
   auto item_of = [&](int i, int& m0, int& n0) {
-    const int w = (int)blockIdx.x / S + i * ((int)gridDim.x / S);
+    const int w = first + i * step;
     if (w >= total) return false;
-    const int mt = w / p.n_tiles;
+    const int mt = i == 0 ? first_mt : w / p.n_tiles;
     m0 = mt * 128;
     n0 = (w - mt * p.n_tiles) * kBN;
     return true;
   };
+  ptx::grid_dependency_wait();
+  ptx::grid_launch_dependents();
 
   if (warp == 0) {
     // ------------------------------------------------------------------ TMA producer ----
@@ -156,8 +160,9 @@ gemm_tf32x3_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_consta
         for (int kb = kb_lo; kb < kb_hi; ++kb, ++cnt) {
           const uint32_t st = cnt % kStages;
           if (!ptx::mbar_wait_abortable(empty + 8 * st, ((cnt / kStages) & 1u) ^ 1u, abort_flag)) { okw = false; break; }
-          ptx::mbar_arrive_expect_tx(full + 8 * st, kTile);
+          ptx::mbar_arrive_expect_tx(full + 8 * st, 2 * kTile);
           ptx::tma_load_2d(sRing + st * kStageBytes, &tm_a, kb * 32, m0, full + 8 * st);
+          ptx::tma_load_2d(sRing + st * kStageBytes + kTile, &tm_b, n0, kb * 32, full + 8 * st);
         }
       }
       if (!okw && p.error_flag) atomicCAS(p.error_flag, 0, (int)kErrWaitProducer);
@@ -179,12 +184,12 @@ gemm_tf32x3_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_consta
         // large sum to one step per k block of 8 instead of three makes it three times smaller
         const uint32_t d = tmem_base, dl = d + kBN;
         for (int kb = kb_lo; kb < kb_hi; ++kb, ++cnt) {
-          const uint32_t st = cnt % kStages;
+          const uint32_t st = cnt % kStages, ta = cnt % kAStages;
           if (!ptx::warp_wait(conv + 8 * st, (cnt / kStages) & 1u, abort_flag)) { okw = false; break; }
           ptx::tc_fence_after();
           const uint32_t s0 = sRing + st * kStageBytes;
-          const uint32_t a_hi = tmem_base + kTmemA + st * kTmemStage, a_lo = a_hi + 32;
-          const uint32_t b_hi = ptx::smem_desc_k128_lo(s0 + kTile), b_lo = ptx::smem_desc_k128_lo(s0 + 2 * kTile);
+          const uint32_t a_hi = tmem_base + kTmemA + ta * kTmemStage, a_lo = a_hi + 32;
+          const uint32_t b_hi = ptx::smem_desc_k128_lo(s0 + kTile), b_lo = ptx::smem_desc_k128_lo(s0);
 #pragma unroll
           for (uint32_t k4 = 0; k4 < 4; ++k4) {   // k step of 8 fp32: 8 columns of A, 32 bytes along the rows of B
             const uint64_t bh = ptx::desc_from_halves(b_hi + k4 * 2, ptx::kSmemDescK128Hi);
@@ -194,6 +199,7 @@ gemm_tf32x3_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_consta
             ptx::umma_tf32_ts(d, a_hi + k4 * 8, bh, idesc, kb != kb_lo || k4 != 0 ? 1u : 0u, issue);
           }
           ptx::tc_commit(empty + 8 * st, issue);
+          ptx::tc_commit(a_empty + 8 * ta, issue);
         }
         if (!okw) break;
         ptx::tc_commit(acc_full, issue);
@@ -208,32 +214,25 @@ gemm_tf32x3_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_consta
     const uint32_t swz = (uint32_t)(t & 7);
     const int quad = warp & 3;                         // tensor-memory lanes this warp may write
     bool okw = true;
-    const uint32_t len = (uint32_t)(kb_hi - kb_lo);
-    float bv[32];
-    // this thread's column of the block with this number; false past the last one
-    auto load_b = [&](uint32_t cnt) {
-      const uint32_t i = cnt / len;
-      int m0, n0;
-      if (!item_of((int)i, m0, n0)) return false;
-      const int n = n0 + t, k0 = (kb_lo + (int)(cnt - i * len)) * 32;
-      const float* bp = p.B + (size_t)k0 * p.N + n;
-#pragma unroll
-      for (int k = 0; k < 32; ++k) bv[k] = load_or_zero(bp + (size_t)k * p.N, n < p.N && k0 + k < p.K);
-      return true;
-    };
+    // blocks of all tiles of this CTA
+    const uint32_t tiles = (uint32_t)(first < total ? (total - first - 1) / step + 1 : 0);
+    const uint32_t blocks = tiles * (uint32_t)(kb_hi - kb_lo);
     {
-      bool more = load_b((uint32_t)grp);
-      for (uint32_t cnt = (uint32_t)grp; more; cnt += kConvGroups) {
-        const uint32_t st = cnt % kStages;
-        // the MMAs that read this stage last have finished: its B and lo tiles may be rewritten
-        bool got = ptx::mbar_wait_abortable(empty + 8 * st, ((cnt / kStages) & 1u) ^ 1u, abort_flag);
-        got = got && ptx::mbar_wait_abortable(full + 8 * st, (cnt / kStages) & 1u, abort_flag);
+      for (uint32_t cnt = (uint32_t)grp; cnt < blocks; cnt += kConvGroups) {
+        const uint32_t st = cnt % kStages, ta = cnt % kAStages;
+        // the stage has come, and the MMAs that read these columns of A last have finished
+        bool got = ptx::mbar_wait_abortable(full + 8 * st, (cnt / kStages) & 1u, abort_flag);
+        got = got && ptx::mbar_wait_abortable(a_empty + 8 * ta, ((cnt / kAStages) & 1u) ^ 1u, abort_flag);
         if (!ptx::named_bar_and(4 + grp, kConvThreads, got)) { okw = false; break; }
         const uint32_t s0 = sRing + st * kStageBytes;
-        ptx::tc_fence_after();   // the MMAs that read the stage's columns of A are over
+        ptx::tc_fence_after();
+        float bv[32];   // column t of B: 32 rows of 128 columns, a warp's loads of one row meet no bank twice
+#pragma unroll
+        for (int k = 0; k < 32; ++k)
+          asm volatile("ld.shared.f32 %0, [%1];" : "=f"(bv[k]) : "r"(s0 + kTile + (uint32_t)k * (kBN * 4) + (uint32_t)t * 4u));
         // row (quad, lane) of A: out of shared memory, in two parts into tensor memory
         const uint32_t arow = s0 + (uint32_t)(quad * 32 + lane) * 128u;
-        const uint32_t acol = tmem_base + ((uint32_t)(quad * 32) << 16) + kTmemA + st * kTmemStage;
+        const uint32_t acol = tmem_base + ((uint32_t)(quad * 32) << 16) + kTmemA + ta * kTmemStage;
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
           float hi[16], lo[16];
@@ -252,8 +251,10 @@ gemm_tf32x3_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_consta
           ptx::tmem_st_32x16(acol + h * 16, hi);
           ptx::tmem_st_32x16(acol + 32 + h * 16, lo);
         }
+        // every thread of the group has its values in registers: the parts of B go where A and B were
+        ptx::named_bar_sync(4 + grp, kConvThreads);
         // column n of B becomes row t of the K-major tiles: 8 chunks of 4 k values, chunk index XOR (row % 8)
-        const uint32_t brow = s0 + kTile + (uint32_t)t * 128u;
+        const uint32_t brow = s0 + (uint32_t)t * 128u;
 #pragma unroll
         for (int j = 0; j < 8; ++j) {
           float hi[4], lo[4];
@@ -263,14 +264,13 @@ gemm_tf32x3_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_consta
             lo[e] = tf32_round(bv[4 * j + e] - hi[e]);
           }
           const uint32_t dst = brow + (((uint32_t)j ^ swz) << 4);
-          asm volatile("st.shared.v4.f32 [%0], {%1,%2,%3,%4};" ::"r"(dst), "f"(hi[0]), "f"(hi[1]), "f"(hi[2]), "f"(hi[3]) : "memory");
-          asm volatile("st.shared.v4.f32 [%0], {%1,%2,%3,%4};" ::"r"(dst + kTile), "f"(lo[0]), "f"(lo[1]), "f"(lo[2]), "f"(lo[3]) : "memory");
+          asm volatile("st.shared.v4.f32 [%0], {%1,%2,%3,%4};" ::"r"(dst + kTile), "f"(hi[0]), "f"(hi[1]), "f"(hi[2]), "f"(hi[3]) : "memory");
+          asm volatile("st.shared.v4.f32 [%0], {%1,%2,%3,%4};" ::"r"(dst), "f"(lo[0]), "f"(lo[1]), "f"(lo[2]), "f"(lo[3]) : "memory");
         }
         ptx::fence_proxy_async_smem();
         ptx::tmem_st_wait();
         ptx::tc_fence_before();
         ptx::mbar_arrive(conv + 8 * st);
-        more = load_b(cnt + kConvGroups);   // on its way while the group waits for the stage
       }
     }
     if (!okw && p.error_flag && t == 0) atomicCAS(p.error_flag, 0, (int)kErrWaitLoader);
@@ -354,42 +354,46 @@ gemm_tf32x3_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_consta
   __syncthreads();
   if (S > 1) {
     // every CTA finishes its share of the rows from all partial sums, in rank order: the result does not depend on timing
-    ptx::cluster_sync_all();
     int m0, n0;
     item_of(0, m0, n0);
     const int n = n0 + lane * 4, rows = 128 / S;
-    float4 bias = make_float4(0.f, 0.f, 0.f, 0.f);
-    if (p.bias && n < p.N) bias = make_float4(__ldg(p.bias + n), __ldg(p.bias + n + 1), __ldg(p.bias + n + 2), __ldg(p.bias + n + 3));
-    // a warp's rows, at most 8 / S of them: the parts of all are asked for before the first is added (row by row 4200 clocks)
+    float bias[4];
+#pragma unroll
+    for (int e = 0; e < 4; ++e) bias[e] = load_or_zero(p.bias + n + e, p.bias != nullptr && n < p.N);
+    ptx::cluster_sync_all();
+    // a warp's rows, at most 8 / S of them: the parts of all are asked for before the first is added
     float4 part[8];
-    auto row_of = [&](int e) { return rank * rows + warp + e / S * (kThreads / 32); };
-    auto mine = [&](int r) { return r < (rank + 1) * rows && n < p.N && m0 + r < p.M && !s_abort; };
+    auto row_of = [&](int e) { return rank * rows + warp + (e >> p.splits_log) * (kThreads / 32); };
+    auto mine = [&](int r) { return r < (rank + 1) * rows && m0 + r < p.M && !s_abort; };   // the same for the whole warp
 #pragma unroll
     for (int e = 0; e < 8; ++e) {
-      const int r = row_of(e);
-      if (mine(r)) part[e] = ptx::ld_cluster_f4(ptx::map_to_cta(sRing + (uint32_t)r * (kBN * 4) + (((uint32_t)lane ^ (uint32_t)(r & 7)) << 4), (uint32_t)(e % S)));
+      const int r = row_of(e), q = e & (S - 1);
+      if (!mine(r)) continue;
+      const uint32_t at = sRing + (uint32_t)r * (kBN * 4) + (((uint32_t)lane ^ (uint32_t)(r & 7)) << 4);
+      if (q == rank) asm volatile("ld.shared.v4.f32 {%0,%1,%2,%3}, [%4];" : "=f"(part[e].x), "=f"(part[e].y), "=f"(part[e].z), "=f"(part[e].w) : "r"(at));
+      else part[e] = ptx::ld_cluster_f4(ptx::map_to_cta(at, (uint32_t)q));
     }
     float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
     for (int e = 0; e < 8; ++e) {
       const int r = row_of(e);
       if (!mine(r)) continue;
-      if (e % S == 0) v = part[e];
+      if ((e & (S - 1)) == 0) v = part[e];
       else { v.x += part[e].x; v.y += part[e].y; v.z += part[e].z; v.w += part[e].w; }
-      if (e % S != S - 1) continue;
-      v.x += bias.x; v.y += bias.y; v.z += bias.z; v.w += bias.w;
+      if ((e & (S - 1)) != S - 1) continue;
+      v.x += bias[0]; v.y += bias[1]; v.z += bias[2]; v.w += bias[3];
       if (p.relu) {
         v.x = !(v.x <= 0.0f) ? v.x : 0.0f; v.y = !(v.y <= 0.0f) ? v.y : 0.0f;
         v.z = !(v.z <= 0.0f) ? v.z : 0.0f; v.w = !(v.w <= 0.0f) ? v.w : 0.0f;
       }
-      *reinterpret_cast<float4*>(p.C + (size_t)(m0 + r) * p.N + n) = v;
+      if (n < p.N) *reinterpret_cast<float4*>(p.C + (size_t)(m0 + r) * p.N + n) = v;
     }
     __syncwarp();
     ptx::cluster_sync_all();   // the peers' reads of this CTA's partial sums are over
   }
   if (warp == 1) {
     __syncwarp();
-    ptx::tmem_dealloc(tmem_base, kTmemA + kStages * kTmemStage);
+    ptx::tmem_dealloc(tmem_base, kTmemA + kAStages * kTmemStage);
   }
 }
 
@@ -406,16 +410,16 @@ PFN_cuTensorMapEncodeTiled_v12000 gt_get_encode() {
   return fn;
 }
 
-// 2-D map over a row-major fp32 [rows, cols] matrix, box 32 columns (128 bytes) x box_rows, 128-byte swizzle.
-bool gt_map(CUtensorMap* m, const void* ptr, long long rows, long long cols, int box_rows) {
+// 2-D map over a row-major fp32 [rows, cols] matrix; swizzle: rows of 128 bytes (32 columns) with the 128-byte swizzle.
+bool gt_map(CUtensorMap* m, const void* ptr, long long rows, long long cols, int box_cols, int box_rows, bool swizzle) {
   auto enc = gt_get_encode();
   if (!enc) return false;
   cuuint64_t gdim[2] = {(cuuint64_t)cols, (cuuint64_t)rows};
   cuuint64_t gstr[1] = {(cuuint64_t)cols * 4};
-  cuuint32_t box[2] = {32, (cuuint32_t)box_rows};
+  cuuint32_t box[2] = {(cuuint32_t)box_cols, (cuuint32_t)box_rows};
   cuuint32_t estr[2] = {1, 1};
   return enc(m, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, const_cast<void*>(ptr), gdim, gstr, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-             CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+             swizzle ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
 }  // namespace
@@ -425,30 +429,32 @@ bool gemm_tf32x3_supported(int M, int N, int K) { return M > 0 && N >= 32 && K >
 cudaError_t launch_gemm_tf32x3(const float* A, const float* B, float* C, int M, int N, int K, const float* bias, int relu,
                                int sm_count, int* error_flag, cudaStream_t stream) {
   if (!gemm_tf32x3_supported(M, N, K)) return cudaErrorInvalidValue;
-  if ((reinterpret_cast<uintptr_t>(A) & 15) || (reinterpret_cast<uintptr_t>(B) & 3) || (reinterpret_cast<uintptr_t>(C) & 15))
+  if ((reinterpret_cast<uintptr_t>(A) & 15) || (reinterpret_cast<uintptr_t>(B) & 15) || (reinterpret_cast<uintptr_t>(C) & 15))
     return cudaErrorMisalignedAddress;
-  GtParams p;
-  p.bias = bias; p.B = B; p.C = C; p.error_flag = error_flag; p.M = M; p.N = N; p.K = K; p.relu = relu;
+  GtParams p{};
+  p.bias = bias; p.C = C; p.error_flag = error_flag; p.M = M; p.N = N; p.K = K; p.relu = relu;
   p.m_tiles = (M + 127) / 128; p.n_tiles = (N + kBN - 1) / kBN; p.k_blocks = (K + 31) / 32;
   if ((long long)p.m_tiles * p.n_tiles > 0x7fffffffLL) return cudaErrorInvalidValue;
-  CUtensorMap tm_a, tm_c;
-  if (!gt_map(&tm_a, A, M, K, 128) || !gt_map(&tm_c, C, M, N, 128)) return cudaErrorInvalidValue;
+  CUtensorMap tm_a, tm_b, tm_c = {};   // shared tiles are written without a map
+  if (!gt_map(&tm_a, A, M, K, 32, 128, true) || !gt_map(&tm_b, B, K, N, kBN, 32, false)) return cudaErrorInvalidValue;
   const size_t smem = 1024 + (size_t)kStages * kStageBytes + 2 * kSlabBytes + 256;
   cudaError_t e = cudaFuncSetAttribute(gemm_tf32x3_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;
   const int sms = sm_count > 0 ? sm_count : 148;
   const int items = p.m_tiles * p.n_tiles;
   // Fewer tiles than SMs: clusters split the k blocks of a tile, as far as all of them run at once and each CTA keeps four
-  // blocks (a block takes about 0.9 us, the exchange of partial sums 2).
+  // blocks (a block takes about 0.5 us, the exchange of partial sums 2.5).
   static const ClusterFit fit = cluster_fit(gemm_tf32x3_kernel, kThreads, smem, sms);
-  p.splits = 1;
+  int splits = 1;
   for (int s = 2; s <= 8; s *= 2) {
     if (items > fit.of[s] || p.k_blocks < 4 * s) break;
-    p.splits = s;
+    splits = s;
+    ++p.splits_log;
   }
-  if (p.splits == 1) return launch_pdl(gemm_tf32x3_kernel, dim3(items < sms ? items : sms), dim3(kThreads), smem, stream, tm_a, tm_c, p);
+  if (splits == 1 && !gt_map(&tm_c, C, M, N, 32, 128, true)) return cudaErrorInvalidValue;
+  if (splits == 1) return launch_pdl(gemm_tf32x3_kernel, dim3(items < sms ? items : sms), dim3(kThreads), smem, stream, tm_a, tm_b, tm_c, p);
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3((unsigned)(items * p.splits));
+  cfg.gridDim = dim3((unsigned)(items * splits));
   cfg.blockDim = dim3(kThreads);
   cfg.dynamicSmemBytes = smem;
   cfg.stream = stream;
@@ -456,11 +462,11 @@ cudaError_t launch_gemm_tf32x3(const float* A, const float* B, float* C, int M, 
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   attr[1].id = cudaLaunchAttributeClusterDimension;
-  attr[1].val.clusterDim.x = (unsigned)p.splits;
+  attr[1].val.clusterDim.x = (unsigned)splits;
   attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 2;
-  return cudaLaunchKernelEx(&cfg, gemm_tf32x3_kernel, tm_a, tm_c, p);
+  return cudaLaunchKernelEx(&cfg, gemm_tf32x3_kernel, tm_a, tm_b, tm_c, p);
 }
 
 }  // namespace nncv_b200
