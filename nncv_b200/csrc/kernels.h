@@ -260,10 +260,10 @@ cudaError_t launch_depthwise(const void* x, const void* w, DType w_dt, int w_f16
                              int N, int H, int W, int C, int R, int S, int stride, int pad, int act, Layout in_l, Layout out_l,
                              int sm_count, int* error_flag, cudaStream_t st);
 // 3x3 convolution on the 3-channel NCHW network input, 16 .. 64 output channels, scale / shift / activation, NHWC
-// output in `out_l` (16-bit activations); w: fp32 [Cout][3][3][3], w_f16: values that fp16 holds
+// output in `out_l` (16-bit activations); w: fp32 [Cout][3][3][3]
 bool stem3x3_supported(int Cin, int Cout, int R, int S, DType act_dt, int act);
 cudaError_t launch_stem3x3(const void* src, DType src_dt, const float* w, const float* scale, const float* shift, void* dst, DType dt,
-                           Layout out_l, int N, int H, int W, int Cout, int stride, int pad, int act, int w_f16, int* error_flag, cudaStream_t st);
+                           Layout out_l, int N, int H, int W, int Cout, int stride, int pad, int act, cudaStream_t st);
 // 1x1 stride-1 convolution with at most 128 channels on either side, on CUDA cores (16-bit NHWC, any layout)
 struct PointwiseArgs {
   const void* in = nullptr;

@@ -1559,7 +1559,7 @@ int model_forward_device(Model& m, const void* src_dev, int N, int H, int W, cud
         prof_begin(3, 2.0 * N * oh * ow * n.cout * 27.0, (double)N * (3.0 * H * W * m.ele_width + aes * oh * ow * n.cout), N * oh * ow,
                    n.cout, 27, 8, st);
         LAUNCH(launch_stem3x3(src_dev, m.io_dt, m.stem3_w, m.scale[n.conv_idx], m.shift[n.conv_idx], o.p, adt, o.l, N, H, W, n.cout,
-                              n.stride, n.pad, n.act, m.ele_width == 2, g_dev.error_flag, st));
+                              n.stride, n.pad, n.act, st));
         ++g_launches;
         prof_end(st);
       }

@@ -7,14 +7,15 @@
 // of the NCHW input, one write of the output), and it does not fit the tensor-core kernels: as an
 // implicit GEMM its K of 27 would be padded to 9 x 64 and its N of 16 to 64 (measured on the TMA-fed
 // kernel: 821 us at batch 256, plus 109 us for the NCHW -> NHWC conversion in front of it).  Here one
-// thread computes 16 output channels of one pixel straight from the NCHW input (a warp reads
+// thread computes 16 output channels of one pixel, or of four (stride 1 and 2), straight from the NCHW input (a warp reads
 // consecutive columns of a row), filter / scale / shift in shared memory read as broadcast vectors,
-// fp32 accumulation on register pairs, and the conversion pass disappears.
+// fp32 accumulation on register pairs, and the conversion pass disappears.  fp16 images with an fp16 filter fit mma.sync's windows
+// (46 us for 80), but the tensor core's sums are not those of rounded multiply-adds, and what an fp16 file gave was not what the same
+// values in an fp32 file gave (logits of MobileNetV3 6e-4 apart, either 5.3e-4 from 64 bits).
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>
 
-#include "epilogue.cuh"
 #include "kernels.h"
 #include "ptx.cuh"
 
@@ -273,163 +274,6 @@ __global__ void __launch_bounds__(256, 2) stem3x3_row_kernel(const TI* __restric
   }
 }
 
-// fp16 images and an fp16 filter, stride 2, pad 1, W a multiple of 8: the tensor cores' (mma.sync) work.  On the fma pipe the 27 x 16
-// multiply-adds of a pixel bound the layer: 80 us at batch 256 (224 x 224 -> 16 channels, 180 MB, 28 us of HBM), 46 us here.  tcgen05
-// would need the windows laid out in shared memory; an A fragment of mma.sync takes them as they lie in the rows of the image.
-// K: the nine (channel, filter row) pairs, four columns of the input each -- two aligned words, of which the first value is no tap and
-// is cleared, so that an infinity or NaN there does not reach the sum.  A warp computes 16 adjacent pixels x 16 channels: the columns of
-// the two 8-channel halves are dealt so that a thread ends up with four adjacent channels, 8 bytes to store.  Products are exact, sums
-// fp32, as before.  The rows come to shared memory as bulk copies, three (one a channel) for kRowsOut rows of output, the next ones while
-// these are computed: read straight from global memory, in words, too few bytes were on their way (77 us).
-__device__ __forceinline__ void mma16(float (&d)[4], const uint32_t (&a)[4], const uint32_t (&b)[2]) {
-  asm("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
-      : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3]) : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b[0]), "r"(b[1]));
-}
-__device__ __forceinline__ void mma8(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t b) {
-  asm("mma.sync.aligned.m16n8k8.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5}, {%6}, {%0,%1,%2,%3};"
-      : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3]) : "r"(a0), "r"(a1), "r"(b));
-}
-
-constexpr int kRowsOut = 4, kRowsIn = 2 * kRowsOut + 1;   // rows of output and input a block works on at a time
-constexpr int kMmaThreads = 256;
-
-__device__ __forceinline__ uint32_t lds(uint32_t addr) {
-  uint32_t v;
-  asm volatile("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"(addr));
-  return v;
-}
-
-template <bool BF16, bool HSWISH>
-__global__ void __launch_bounds__(kMmaThreads, 4) stem3x3_mma_kernel(const __half* __restrict__ src, const float* __restrict__ w, const float* __restrict__ scale,
-                                                          const float* __restrict__ shift, void* __restrict__ dst, Layout ol, int H, int W,
-                                                          int OH, int OW, int Cout, int act, epi::FastDiv div_groups, epi::FastDiv div_x, int units,
-                                                          int* error_flag) {
-  extern __shared__ __align__(128) uint8_t rows_raw[];   // 16 bytes, two stages of [channel][kRowsIn][W] halves, 128 bytes
-  __shared__ __align__(8) unsigned long long s_full[2];
-  const uint32_t rows0 = ptx::smem_u32(rows_raw) + 16u, full = ptx::smem_u32(s_full);
-  const int row_bytes = 2 * W, stage_bytes = 3 * kRowsIn * row_bytes;
-  if (threadIdx.x == 0) {
-    ptx::mbar_init(full, 1);
-    ptx::mbar_init(full + 8, 1);
-    ptx::mbar_fence_init();
-  }
-  __syncthreads();
-  ptx::grid_dependency_wait();
-  ptx::grid_launch_dependents();
-  const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3, c0 = (int)blockIdx.y * kCG;
-  // step s (16 k values), half h (8 of them): k = 2t, 2t + 1 of the half are columns 2 (t & 1), + 1 of input row j = 4s + 2h + t / 2
-  uint32_t b[5][2];       // [2s + h][half of the channels]
-  int row[5];             // where row j lies in a stage, bytes from the output row's first input row
-  unsigned top = 0, bottom = 0;   // bit 2s + h: row j is the one above, the one below
-#pragma unroll
-  for (int sh = 0; sh < 5; ++sh) {
-    const int j = 2 * sh + (t >> 1), ci = j / 3, ky = j - 3 * ci;
-    row[sh] = j < 9 ? (ci * kRowsIn + ky) * row_bytes : 0;   // there is no tenth: what is read there is cleared
-    if (ky == 0) top |= 1u << sh;
-    if (ky == 2) bottom |= 1u << sh;
-#pragma unroll
-    for (int q = 0; q < 2; ++q) {
-      const int ch = c0 + 4 * (g >> 1) + 2 * q + (g & 1);   // column g of half q
-      __half2 v = __floats2half2_rn(0.0f, 0.0f);
-      if (j < 9) {
-        const float* wp = w + ch * 27 + j * 3;
-        v = (t & 1) ? __floats2half2_rn(wp[1], wp[2]) : __floats2half2_rn(0.0f, wp[0]);
-      }
-      b[sh][q] = *reinterpret_cast<const uint32_t*>(&v);
-    }
-  }
-  const bool ninth = t < 2;   // the last step holds one row: the other threads' is none
-  const uint32_t taps = (t & 1) ? 0xffffffffu : 0xffff0000u;
-  float sc[4], sf[4];
-#pragma unroll
-  for (int e = 0; e < 4; ++e) {
-    sc[e] = scale ? scale[c0 + 4 * t + e] : 1.0f;
-    sf[e] = shift ? shift[c0 + 4 * t + e] : 0.0f;
-  }
-  unsigned short* const out_first = reinterpret_cast<unsigned short*>(dst) + ((long long)ol.off * ol.pitch + ol.off) * Cout + c0 + 4 * t;
-  const int warp = threadIdx.x >> 5;
-  auto fetch = [&](int u, int st) {   // one thread: the rows under output rows oy0 ..
-    const int n = (int)epi::div_by((uint32_t)u, div_groups), iy = 2 * kRowsOut * (u - n * (int)div_groups.d) - 1;
-    const int lo = max(iy, 0), hi = min(iy + kRowsIn, H);
-    const uint32_t bytes = (uint32_t)((hi - lo) * row_bytes);
-    ptx::mbar_arrive_expect_tx(full + 8 * st, 3 * bytes);
-    for (int ci = 0; ci < 3; ++ci)
-      ptx::bulk_g2s(rows0 + (uint32_t)(st * stage_bytes + (ci * kRowsIn + lo - iy) * row_bytes), src + ((size_t)(n * 3 + ci) * H + lo) * W, bytes, full + 8 * st);
-  };
-  if (threadIdx.x == 0 && (int)blockIdx.x < units) fetch((int)blockIdx.x, 0);
-  uint32_t turn = 0;   // stages waited for
-  for (int u = (int)blockIdx.x; u < units; u += (int)gridDim.x, ++turn) {
-    const uint32_t st = turn & 1u;
-    if (threadIdx.x == 0 && u + (int)gridDim.x < units) fetch(u + (int)gridDim.x, (int)(st ^ 1u));
-    if (__syncthreads_or(!ptx::mbar_wait(full + 8 * st, (turn >> 1) & 1u))) {
-      if (threadIdx.x == 0) {
-        if (error_flag) atomicCAS(error_flag, 0, (int)kErrWaitProducer);
-        ptx::mbar_wait(full + 8 * st, (turn >> 1) & 1u);   // once more: no copy may outlive its shared memory
-        if (u + (int)gridDim.x < units) ptx::mbar_wait(full + 8 * (st ^ 1u), ((turn + 1) >> 1) & 1u);
-      }
-      break;
-    }
-    const int n = (int)epi::div_by((uint32_t)u, div_groups), oy0 = kRowsOut * (u - n * (int)div_groups.d), rows = min(kRowsOut, OH - oy0);
-    const int tiles = rows * (int)div_x.d;
-    const uint32_t stage = rows0 + st * (uint32_t)stage_bytes + 4u * (uint32_t)(g + (t & 1)) - 4u;
-    // the warps take turns with the first tile, so that a remainder does not always fall to the same ones
-    for (int k = (warp + (int)turn * 4) & 7; k < tiles; k += kMmaThreads / 32) {
-      const int ry = (int)epi::div_by((uint32_t)k, div_x), oy = oy0 + ry, x0 = (k - ry * (int)div_x.d) * 16, px = x0 + g;
-      // words px - 1 (t even) and px (t odd) of a row; pixel px + 8 eight words on.  Past the right edge lies other data, which only
-      // reaches pixels that are not stored; on the left edge and in rows outside the image zeros take its place.
-      const uint32_t at = stage + (uint32_t)(2 * ry * row_bytes + 4 * x0);
-      uint32_t v[5][2];
-#pragma unroll
-      for (int sh = 0; sh < 5; ++sh) {
-        v[sh][0] = lds(at + (uint32_t)row[sh]);
-        v[sh][1] = lds(at + (uint32_t)row[sh] + 32u);
-      }
-      const uint32_t left = px == 0 && !(t & 1) ? 0u : taps;
-#pragma unroll
-      for (int sh = 0; sh < 4; ++sh) {
-        v[sh][0] &= left;
-        v[sh][1] &= taps;
-      }
-      v[4][0] &= ninth ? left : 0u;
-      v[4][1] &= ninth ? taps : 0u;
-      if (oy == 0 || 2 * oy + 1 >= H) {
-        const unsigned out = (oy == 0 ? top : 0u) | (2 * oy + 1 >= H ? bottom : 0u);
-#pragma unroll
-        for (int sh = 0; sh < 5; ++sh)
-          if (out >> sh & 1u) v[sh][0] = v[sh][1] = 0u;
-      }
-      float d[2][4];
-#pragma unroll
-      for (int q = 0; q < 2; ++q) {
-        d[q][0] = d[q][1] = d[q][2] = d[q][3] = 0.0f;
-#pragma unroll
-        for (int s = 0; s < 2; ++s)
-          mma16(d[q], {v[2 * s][0], v[2 * s][1], v[2 * s + 1][0], v[2 * s + 1][1]}, {b[2 * s][q], b[2 * s + 1][q]});
-        mma8(d[q], v[4][0], v[4][1], b[4][q]);
-      }
-      unsigned short* to = out_first + (((long long)n * ol.img_rows + oy) * ol.pitch + px) * Cout;
-#pragma unroll
-      for (int h = 0; h < 2; ++h) {
-        float y[4];
-#pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          const float a = fmaf(d[e >> 1][2 * h + (e & 1)], sc[e], sf[e]);
-          y[e] = HSWISH ? a * __saturatef(fmaf(a, 0.16666667f, 0.5f)) : act16(a, act);
-        }
-        uint2 o;
-        if (BF16) {
-          const __nv_bfloat162 lo = __floats2bfloat162_rn(y[0], y[1]), hi = __floats2bfloat162_rn(y[2], y[3]);
-          o = make_uint2(*reinterpret_cast<const uint32_t*>(&lo), *reinterpret_cast<const uint32_t*>(&hi));
-        } else {
-          o = make_uint2(ptx::pack_half2_sat(y[0], y[1]), ptx::pack_half2_sat(y[2], y[3]));
-        }
-        if (px + 8 * h < OW) *reinterpret_cast<uint2*>(to + 8 * h * Cout) = o;
-      }
-    }
-    __syncthreads();   // the stage may be filled again
-  }
-}
-
 template <typename TI, bool BF16>
 cudaError_t launch_row(const TI* src, const float* w, const float* scale, const float* shift, void* dst, Layout ol, int N, int H, int W, int OH,
                        int OW, int Cout, int stride, int pad, int act, cudaStream_t st) {
@@ -454,25 +298,13 @@ bool stem3x3_supported(int Cin, int Cout, int R, int S, DType act_dt, int act) {
 }
 
 cudaError_t launch_stem3x3(const void* src, DType src_dt, const float* w, const float* scale, const float* shift, void* dst, DType dt,
-                           Layout out_l, int N, int H, int W, int Cout, int stride, int pad, int act, int w_f16, int* error_flag, cudaStream_t st) {
+                           Layout out_l, int N, int H, int W, int Cout, int stride, int pad, int act, cudaStream_t st) {
   if (!stem3x3_supported(3, Cout, 3, 3, dt, act) || src_dt == kBF16 || stride < 1 || pad < 0) return cudaErrorInvalidValue;
   const int OH = (H + 2 * pad - 3) / stride + 1, OW = (W + 2 * pad - 3) / stride + 1;
   if (OH <= 0 || OW <= 0) return cudaErrorInvalidValue;
   if (out_l.pitch == 0) out_l = dense_layout(OH, OW);
   const long long total = (long long)N * OH * OW * (Cout / kCG);
   if (total >= (1LL << 31) - (1LL << 21)) return cudaErrorInvalidValue;
-  // operands that fp16 holds exactly, rows that bulk copies can take (then OW == W / 2), two stages of them in a quarter of an SM's memory
-  const size_t rows_smem = (size_t)2 * 3 * kRowsIn * 2 * W + 144;
-  if (src_dt == kF16 && w_f16 && stride == 2 && pad == 1 && W % 8 == 0 && rows_smem <= 48 * 1024 && !(reinterpret_cast<uintptr_t>(src) & 15)) {
-    const int groups = (OH + kRowsOut - 1) / kRowsOut, units = N * groups;
-    const dim3 grid((unsigned)(units < 148 * 4 ? units : 148 * 4), (unsigned)(Cout / kCG));
-    auto go = [&](auto kern) {
-      return launch_pdl(kern, grid, dim3(kMmaThreads), rows_smem, st, (const __half*)src, w, scale, shift, dst, out_l, H, W, OH, OW, Cout, act,
-                        epi::fast_div((uint32_t)groups), epi::fast_div((uint32_t)((OW + 15) / 16)), units, error_flag);
-    };
-    if (act == kActHardSwish) return dt == kBF16 ? go(stem3x3_mma_kernel<true, true>) : go(stem3x3_mma_kernel<false, true>);
-    return dt == kBF16 ? go(stem3x3_mma_kernel<true, false>) : go(stem3x3_mma_kernel<false, false>);
-  }
   if (stride <= 2) {   // wider strides share no input between neighbours
     if (src_dt == kF32)
       return dt == kBF16 ? launch_row<float, true>((const float*)src, w, scale, shift, dst, out_l, N, H, W, OH, OW, Cout, stride, pad, act, st)
