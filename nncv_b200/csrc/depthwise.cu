@@ -11,14 +11,14 @@
 // 256) then read the patch from shared memory: thread = (four channels, one or two output columns),
 // computing a column strip of output rows in fp32 pairs (fma.rn.f32x2), so that each input value is
 // loaded once per input column and reused down the strip, and each filter value serves the strip.
-// What bounds the 16-bit kernels with an fp32 filter is the pipe of the packed multiply-adds, on which the conversions to
+// What bounds the 16-bit kernels is the pipe of the packed multiply-adds, on which the conversions to
 // fp32 run too (64x112x112x96 hard-swish: 64 % of its rate with one column a thread, 15 conversions
 // beside 18 multiply-adds for an output of four channels; two columns share four of six input columns:
-// 10).  An fp16 map is converted by multiply-adds with 1, which run at twice the rate of conversions (that layer 69.2 -> 65.4 us).
-// Where fp16 holds the filter too, fma.rn.f32.f16 takes map and filter as they are, 121 a clock and SM where packed pairs reach 109:
-// no conversions, half the registers and reads for the filter, and with nothing to share one column a thread is enough (5x5 at
-// batch 256, us: 14x14x240 32.1 29.4, 14x14x120 20.2 17.7, 7x7x576 22.5 18.7, 28x28x96 stride 2 22.2 20.5; 3x3 28x28x88 22.3 19.5,
-// 56x56x72 stride 2 29.9 26.7; MobileNetV3, 256 images, 868 817).  With eight channels a thread and strips of four rows the 5x5 layers were bound by
+// 10).  An fp16 map is converted by multiply-adds with 1, which run at twice the rate of conversions and give the same values (that layer
+// 69.2 -> 65.4 us; MobileNetV3, 256 images, 906 -> 876).  A filter that fp16 holds could be multiplied as it is, too (fma.rn.f32.f16 takes
+// map and filter; 845), but then without the scale in it, which gives other sums, and it pays only with more than one tile an SM: an
+// image's result came to depend on its batch.
+// With eight channels a thread and strips of four rows the 5x5 layers were bound by
 // shared memory: a filter vector of eight fp32 is two loads at a stride of 32 bytes, two-way bank conflicts, and those loads
 // were two thirds of the traffic (14x14x240 at batch 256: 9.8 M wavefronts, 48 us); now a lane's four filter values are 16
 // contiguous bytes and are read half as often.  Filter, scale and shift sit in shared memory: for the 16-bit types as the
@@ -33,7 +33,6 @@
 #include <cudaTypedefs.h>
 
 #include <mutex>
-#include <type_traits>
 
 #include "depthwise_shape.h"
 #include "epilogue.cuh"
@@ -46,7 +45,7 @@ namespace {
 
 // What a thread computes: KP output rows x PX adjacent output columns of four channels (depthwise_shape.h).
 template <typename T, int KP> constexpr int kTH = sizeof(T) == 4 ? 8 : KP;   // output rows of a tile
-template <typename T, bool HW> constexpr bool kFold = sizeof(T) == 2 && !HW;   // the scale multiplied into the filter
+template <typename T> constexpr bool kFold = sizeof(T) == 2;   // the scale multiplied into the filter
 using dw::kMaxStages;
 
 struct DwParams {
@@ -72,7 +71,7 @@ __device__ __forceinline__ u64 mul2(u64 a, u64 b) {
   return d;
 }
 
-// a * b + c of two fp16 values and an fp32 one, the product exact, rounded once: as many a clock as with fp32 operands, and no conversions
+// a * b + c of two fp16 values and an fp32 one, the product exact, rounded once
 __device__ __forceinline__ void fma_halves(float& d0, float& d1, uint32_t a, uint32_t b) {
   asm("{\n.reg .b16 al, ah, bl, bh;\nmov.b32 {al, ah}, %2;\nmov.b32 {bl, bh}, %3;\nfma.rn.f32.f16 %0, al, bl, %0;\nfma.rn.f32.f16 %1, ah, bh, %1;\n}\n"
       : "+f"(d0), "+f"(d1) : "r"(a), "r"(b));
@@ -130,9 +129,8 @@ __device__ __forceinline__ float act1(float x, int act) {
   }
 }
 
-// HW: fp16 holds the filter's values.  Map and filter are multiplied as they are (fma_halves).
-template <typename T, int KS, int STRIDE, int PX, int kP, bool HW>
-__global__ void __launch_bounds__(dw::max_threads(sizeof(T)), dw::ctas(sizeof(T), KS, PX, HW)) depthwise_tma_kernel(const __grid_constant__ CUtensorMap tm_in, const DwParams p) {
+template <typename T, int KS, int STRIDE, int PX, int kP>
+__global__ void __launch_bounds__(dw::max_threads(sizeof(T)), dw::ctas(sizeof(T), KS, PX)) depthwise_tma_kernel(const __grid_constant__ CUtensorMap tm_in, const DwParams p) {
   ptx::grid_dependency_wait();
   ptx::grid_launch_dependents();
   constexpr int V = 4;                                  // channels of a thread
@@ -150,9 +148,8 @@ __global__ void __launch_bounds__(dw::max_threads(sizeof(T)), dw::ctas(sizeof(T)
   const int CB = cbv * kPer * V;                         // channels per chunk
   const int IW = (tw - 1) * STRIDE + KS;
   const int c0 = blockIdx.y * CB;
-  using Wt = std::conditional_t<HW, __half, float>;
-  Wt* sw = reinterpret_cast<Wt*>(smem + (size_t)p.stages * p.stage_stride);   // [KS*KS][CB] filter, shift[CB], scale[CB] unless folded
-  float* ssh = reinterpret_cast<float*>(sw + KS * KS * CB);
+  float* sw = reinterpret_cast<float*>(smem + (size_t)p.stages * p.stage_stride);   // [KS*KS][CB] filter, shift[CB], scale[CB] unless folded
+  float* ssh = sw + KS * KS * CB;
   float* ssc = ssh + CB;
 
   if (tid == 0) {
@@ -188,9 +185,9 @@ __global__ void __launch_bounds__(dw::max_threads(sizeof(T)), dw::ctas(sizeof(T)
     }
     const float scale = in && p.scale ? p.scale[c0 + c] : 1.0f;
     ssh[c] = in && p.shift ? p.shift[c0 + c] : 0.0f;
-    if (!kFold<T, HW>) ssc[c] = scale;
+    if (!kFold<T>) ssc[c] = scale;
 #pragma unroll
-    for (int tap = 0; tap < KS * KS; ++tap) sw[tap * CB + c] = static_cast<Wt>(kFold<T, HW> ? v[tap] * scale : v[tap]);
+    for (int tap = 0; tap < KS * KS; ++tap) sw[tap * CB + c] = kFold<T> ? v[tap] * scale : v[tap];
   }
   __syncthreads();
 
@@ -209,54 +206,12 @@ __global__ void __launch_bounds__(dw::max_threads(sizeof(T)), dw::ctas(sizeof(T)
     // folded: the sums start at the shift, the filter carries the scale
     u64 acc[PX][kP][2];
     {
-      const ulonglong2 sh = kFold<T, HW> ? *reinterpret_cast<const ulonglong2*>(ssh + cvec * V) : make_ulonglong2(0, 0);
+      const ulonglong2 sh = kFold<T> ? *reinterpret_cast<const ulonglong2*>(ssh + cvec * V) : make_ulonglong2(0, 0);
 #pragma unroll
       for (int px = 0; px < PX; ++px)
 #pragma unroll
         for (int o = 0; o < kP; ++o) { acc[px][o][0] = sh.x; acc[px][o][1] = sh.y; }
     }
-    if constexpr (HW) {
-      float sum[PX][kP][4];
-#pragma unroll
-      for (int px = 0; px < PX; ++px)
-#pragma unroll
-        for (int o = 0; o < kP; ++o)
-#pragma unroll
-          for (int e = 0; e < 4; ++e) sum[px][o][e] = 0.0f;
-      uint2 wr[KS][KS];
-#pragma unroll
-      for (int ix = 0; ix < NC; ++ix) {
-        if (ix < KS) {
-#pragma unroll
-          for (int q = 0; q < KS; ++q) wr[ix][q] = *reinterpret_cast<const uint2*>(sw + (q * KS + ix) * CB + cvec * V);
-        }
-        const unsigned char* col = st + (size_t)(ys * kP * STRIDE * IW + x * STRIDE + ix) * cbv * 16 + cvec * sizeof(Raw);
-#pragma unroll
-        for (int ry = 0; ry < NR; ++ry) {
-          const uint2 f = *reinterpret_cast<const uint2*>(col + (size_t)ry * IW * cbv * 16);
-#pragma unroll
-          for (int px = 0; px < PX; ++px) {
-            const int kx = ix - px * STRIDE;
-            if (kx < 0 || kx >= KS) continue;
-#pragma unroll
-            for (int o = 0; o < kP; ++o) {
-              const int q = ry - o * STRIDE;               // compile-time after unrolling
-              if (q >= 0 && q < KS) {
-                fma_halves(sum[px][o][0], sum[px][o][1], f.x, wr[kx][q].x);
-                fma_halves(sum[px][o][2], sum[px][o][3], f.y, wr[kx][q].y);
-              }
-            }
-          }
-        }
-      }
-#pragma unroll
-      for (int px = 0; px < PX; ++px)
-#pragma unroll
-        for (int o = 0; o < kP; ++o) {
-          acc[px][o][0] = epi::pk(sum[px][o][0], sum[px][o][1]);
-          acc[px][o][1] = epi::pk(sum[px][o][2], sum[px][o][3]);
-        }
-    } else {
     ulonglong2 wr[KS][KS];   // filter column kx in wr[kx], live while an output column needs it
 #pragma unroll
     for (int ix = 0; ix < NC; ++ix) {
@@ -284,7 +239,6 @@ __global__ void __launch_bounds__(dw::max_threads(sizeof(T)), dw::ctas(sizeof(T)
         }
       }
     }
-    }
     // epilogue: activation, store
     const int4 ti = tile_info[s];
     const int c = c0 + cvec * V, rows = min(kP, p.OH - ti.y - ys * kP);
@@ -293,7 +247,7 @@ __global__ void __launch_bounds__(dw::max_threads(sizeof(T)), dw::ctas(sizeof(T)
     for (int px = 0; px < PX; ++px) {
       const int ox = ti.z + x + px;
       if (ox >= p.OW) break;
-      if (!kFold<T, HW>) {
+      if (!kFold<T>) {
         const ulonglong2 sc = *reinterpret_cast<const ulonglong2*>(ssc + cvec * V), sh = *reinterpret_cast<const ulonglong2*>(ssh + cvec * V);
 #pragma unroll
         for (int o = 0; o < kP; ++o) {
@@ -352,9 +306,9 @@ PFN_cuTensorMapEncodeTiled_v12000 dw_get_encode() {
   return fn;
 }
 
-template <typename T, int KS, int STRIDE, int PX, int KP, bool HW>
+template <typename T, int KS, int STRIDE, int PX, int KP>
 cudaError_t launch_one(const CUtensorMap& tm, const DwParams& p, dim3 grid, int threads, size_t smem, cudaStream_t st) {
-  auto kern = depthwise_tma_kernel<T, KS, STRIDE, PX, KP, HW>;
+  auto kern = depthwise_tma_kernel<T, KS, STRIDE, PX, KP>;
   if (smem > 48 * 1024) {
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
@@ -363,19 +317,18 @@ cudaError_t launch_one(const CUtensorMap& tm, const DwParams& p, dim3 grid, int 
   return cudaGetLastError();
 }
 
-template <typename T, int PX, int KP, bool HW>
+template <typename T, int PX, int KP>
 cudaError_t launch_typed(const CUtensorMap& tm, const DwParams& p, int ks, int stride, dim3 grid, int threads, size_t smem, cudaStream_t st) {
-  if (ks == 3 && stride == 1) return launch_one<T, 3, 1, PX, KP, HW>(tm, p, grid, threads, smem, st);
-  if (ks == 3 && stride == 2) return launch_one<T, 3, 2, PX, KP, HW>(tm, p, grid, threads, smem, st);
-  if (ks == 5 && stride == 1) return launch_one<T, 5, 1, PX, KP, HW>(tm, p, grid, threads, smem, st);
-  return launch_one<T, 5, 2, PX, KP, HW>(tm, p, grid, threads, smem, st);
+  if (ks == 3 && stride == 1) return launch_one<T, 3, 1, PX, KP>(tm, p, grid, threads, smem, st);
+  if (ks == 3 && stride == 2) return launch_one<T, 3, 2, PX, KP>(tm, p, grid, threads, smem, st);
+  if (ks == 5 && stride == 1) return launch_one<T, 5, 1, PX, KP>(tm, p, grid, threads, smem, st);
+  return launch_one<T, 5, 2, PX, KP>(tm, p, grid, threads, smem, st);
 }
-template <typename T, bool HW>
+template <typename T>
 cudaError_t launch_shape(int px, const CUtensorMap& tm, const DwParams& p, int ks, int stride, dim3 grid, int threads, size_t smem, cudaStream_t st) {
-  if (px == 1) return launch_typed<T, 1, 8, HW>(tm, p, ks, stride, grid, threads, smem, st);
-  if (stride == 2) return ks == 3 ? launch_one<T, 3, 2, 2, 4, HW>(tm, p, grid, threads, smem, st) : launch_one<T, 5, 2, 2, 4, HW>(tm, p, grid, threads, smem, st);
-  if constexpr (!HW) return ks == 3 ? launch_one<T, 3, 1, 2, 8, HW>(tm, p, grid, threads, smem, st) : launch_one<T, 5, 1, 2, 8, HW>(tm, p, grid, threads, smem, st);
-  return cudaErrorInvalidValue;   // no such choice
+  if (px == 1) return launch_typed<T, 1, 8>(tm, p, ks, stride, grid, threads, smem, st);
+  if (ks == 3) return stride == 1 ? launch_one<T, 3, 1, 2, 8>(tm, p, grid, threads, smem, st) : launch_one<T, 3, 2, 2, 4>(tm, p, grid, threads, smem, st);
+  return stride == 1 ? launch_one<T, 5, 1, 2, 8>(tm, p, grid, threads, smem, st) : launch_one<T, 5, 2, 2, 4>(tm, p, grid, threads, smem, st);
 }
 
 }  // namespace
@@ -389,7 +342,7 @@ bool depthwise_tma_supported(DType dt, int N, int H, int W, int C, int R, int S,
   return (long long)N * ((OH + 3) / 4) * ((OW + 1) / 2) < (1LL << 30);
 }
 
-cudaError_t launch_depthwise_tma(const void* x, const void* w, DType w_dt, int w_f16, const float* scale, const float* shift, void* y, DType dt,
+cudaError_t launch_depthwise_tma(const void* x, const void* w, DType w_dt, const float* scale, const float* shift, void* y, DType dt,
                                  int N, int H, int W, int C, int R, int S, int stride, int pad, int act, Layout in_l, Layout out_l,
                                  int sm_count, int* error_flag, cudaStream_t st) {
   if (!depthwise_tma_supported(dt, N, H, W, C, R, S, stride, pad) || (reinterpret_cast<uintptr_t>(x) & 15) ||
@@ -399,12 +352,7 @@ cudaError_t launch_depthwise_tma(const void* x, const void* w, DType w_dt, int w
   const int OH = (H + 2 * pad - R) / stride + 1, OW = (W + 2 * pad - S) / stride + 1;
   DwParams p{};
   const int sms = sm_count > 0 ? sm_count : 148;
-  dw::Shape d = dw::shape_of(N, C, OH, OW, R, stride, es, sms);
-  // a filter that fp16 holds is multiplied as it is where an SM has more than one tile.  With one a warp's instructions count, not the
-  // pipes, and packed pairs are fewer: MobileNetV3, one image, 185.4 us with pairs and 187.4, 8 images 218.7 and 216, 256 images 871 and 817.
-  const bool halves = dt == kF16 && w_f16 && d.cbv != 0 &&
-                      (long long)N * ((OH + d.kp - 1) / d.kp) * ((OW + d.tw - 1) / d.tw) * ((cv + d.cbv - 1) / d.cbv) > sms;
-  if (halves) d = dw::shape_of(N, C, OH, OW, R, stride, es, sms, true);
+  const dw::Shape d = dw::shape_of(N, C, OH, OW, R, stride, es, sms);
   if (d.cbv == 0) return cudaErrorInvalidValue;
   const int tw = d.tw, cbv = d.cbv, px = d.px, kp = d.kp, th = es == 2 ? kp : 8, IH = (th - 1) * stride + R, IW = (tw - 1) * stride + R;
   p.tw = tw; p.cbv = cbv;
@@ -444,10 +392,9 @@ cudaError_t launch_depthwise_tma(const void* x, const void* w, DType w_dt, int w
   if (gx > p.n_tiles) gx = p.n_tiles;
   const dim3 grid((unsigned)gx, (unsigned)chunks);
   if (chunks > 65535) return cudaErrorInvalidValue;
-  if (dt == kF32) return launch_typed<float, 1, 4, false>(tm, p, R, stride, grid, d.threads, smem, st);
-  if (halves) return launch_shape<__half, true>(px, tm, p, R, stride, grid, d.threads, smem, st);
-  if (dt == kF16) return launch_shape<__half, false>(px, tm, p, R, stride, grid, d.threads, smem, st);
-  return launch_shape<__nv_bfloat16, false>(px, tm, p, R, stride, grid, d.threads, smem, st);
+  if (dt == kF32) return launch_typed<float, 1, 4>(tm, p, R, stride, grid, d.threads, smem, st);
+  if (dt == kF16) return launch_shape<__half>(px, tm, p, R, stride, grid, d.threads, smem, st);
+  return launch_shape<__nv_bfloat16>(px, tm, p, R, stride, grid, d.threads, smem, st);
 }
 
 }  // namespace nncv_b200

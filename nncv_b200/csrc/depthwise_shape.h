@@ -10,8 +10,7 @@ namespace dw {
 // Threads of a block at most, and blocks of that size an SM (by registers; the kernel's launch bounds).  es: bytes of an element,
 // px: output columns of a thread.
 constexpr int max_threads(int es) { return es == 4 ? 256 : 128; }
-// w_f16: the filter in fp16.
-constexpr int ctas(int es, int ks, int px, bool w_f16 = false) { return es == 4 ? (ks == 3 ? 3 : 2) : px == 2 ? (ks == 3 ? 4 : 3) : (ks == 3 ? 6 : w_f16 ? 5 : 4); }
+constexpr int ctas(int es, int ks, int px) { return es == 4 ? (ks == 3 ? 3 : 2) : px == 2 ? (ks == 3 ? 4 : 3) : (ks == 3 ? 6 : 4); }
 constexpr int kMaxStages = 3;
 // Shared memory of an SM, and what a block takes of it besides its own: 1 KB of the system's and the kernel's static variables.
 constexpr size_t kSmSmem = 228 * 1024, kBlockSmem = 1024 + 128;
@@ -37,15 +36,15 @@ struct Shape { int cbv, tw, px, kp, threads, stages, per_sm; size_t smem; };
 // threads of one column x eight rows throughout.
 // Batch 256 fp16, us, one column, two columns: 240 channels 5x5 on 14x14 37.6 34.3, 576 on 7x7 24.3 28.7, 88 3x3 on 28x28 27.2 25.3, 16
 // 3x3 stride 2 112 -> 56 32.6 43.6, 72 3x3 stride 2 56 -> 28 41.9 29.9.
-inline Shape choose(int N, int C, int OH, int OW, int R, int stride, int es, int sms, bool w_f16 = false) {
+inline Shape choose(int N, int C, int OH, int OW, int R, int stride, int es, int sms) {
   const int V = 16 / es, cv = C / V;
   const size_t wvec = (size_t)(R * R + (es == 2 ? 1 : 2)) * V * sizeof(float);   // filter and shift (scale) of a channel vector
   Shape best{};
   double least = 1e30;
-  for (int px = es == 2 && !(w_f16 && stride == 1) ? 2 : 1; px >= 1; --px) {
+  for (int px = es == 2 ? 2 : 1; px >= 1; --px) {
     const int kp = es == 4 || (px == 2 && stride == 2) ? 4 : 8, th = es == 4 ? 8 : kp, ih = (th - 1) * stride + R;
     const int most = max_threads(es), slots = most * px / 2;   // 16-byte vectors of a tile
-    const int by_regs = most * ctas(es, R, px, w_f16), tiles_y = (OH + th - 1) / th;
+    const int by_regs = most * ctas(es, R, px), tiles_y = (OH + th - 1) / th;
     const double loads = (double)((kp - 1) * stride + R) * ((px - 1) * stride + R);
     const double work = ((2.0 * R * R + 1.0) * kp * px + 2.0 * loads) * (px == 2 ? 1.1 : 1.0);
     for (int v = std::min(32, cv); v >= 2; --v) {        // ties go to the wider chunk (longer contiguous runs in memory)
@@ -87,19 +86,19 @@ inline Shape choose(int N, int C, int OH, int OW, int R, int stride, int es, int
 
 // The same, kept for the layers that a thread asks for in turn: choosing takes longer than a launch.  Four places for the layers of
 // one hash value, so that a network's few dozen do not push one another out.
-inline Shape shape_of(int N, int C, int OH, int OW, int R, int stride, int es, int sms, bool w_f16 = false) {
-  struct Kept { int key[9]; Shape shape; };
+inline Shape shape_of(int N, int C, int OH, int OW, int R, int stride, int es, int sms) {
+  struct Kept { int key[8]; Shape shape; };
   struct Row { Kept way[4]; unsigned next; };
   thread_local Row table[32] = {};
-  const int key[9] = {N, C, OH, OW, R, stride, es, sms, w_f16};
+  const int key[8] = {N, C, OH, OW, R, stride, es, sms};
   unsigned h = 2166136261u;
   for (int k : key) h = (h ^ (unsigned)k) * 16777619u;
   Row& row = table[(h >> 16) % 32u];
   for (const Kept& k : row.way)
-    if (std::equal(key, key + 9, k.key)) return k.shape;
+    if (std::equal(key, key + 8, k.key)) return k.shape;
   Kept& k = row.way[row.next++ % 4u];
-  k.shape = choose(N, C, OH, OW, R, stride, es, sms, w_f16);
-  std::copy(key, key + 9, k.key);
+  k.shape = choose(N, C, OH, OW, R, stride, es, sms);
+  std::copy(key, key + 8, k.key);
   return k.shape;
 }
 

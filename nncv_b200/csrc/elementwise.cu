@@ -286,7 +286,7 @@ int grid_for(long long work, int threads) {
 
 }  // namespace
 
-cudaError_t launch_depthwise(const void* x, const void* w, DType w_dt, int w_f16, const float* scale, const float* shift, void* y, DType dt,
+cudaError_t launch_depthwise(const void* x, const void* w, DType w_dt, const float* scale, const float* shift, void* y, DType dt,
                              int N, int H, int W, int C, int R, int S, int stride, int pad, int act, Layout in_l, Layout out_l,
                              int sm_count, int* error_flag, cudaStream_t st) {
   const int V = 16 / (int)dtype_size(dt);
@@ -294,7 +294,7 @@ cudaError_t launch_depthwise(const void* x, const void* w, DType w_dt, int w_f16
   if (dt != kF16 && w_dt != kF32) return cudaErrorInvalidValue;
   if (depthwise_tma_supported(dt, N, H, W, C, R, S, stride, pad) && (reinterpret_cast<uintptr_t>(x) & 15) == 0 &&
       (reinterpret_cast<uintptr_t>(y) & 15) == 0) {
-    const cudaError_t e = launch_depthwise_tma(x, w, w_dt, w_f16, scale, shift, y, dt, N, H, W, C, R, S, stride, pad, act, in_l, out_l, sm_count,
+    const cudaError_t e = launch_depthwise_tma(x, w, w_dt, scale, shift, y, dt, N, H, W, C, R, S, stride, pad, act, in_l, out_l, sm_count,
                                                error_flag, st);
     if (e == cudaSuccess) return e;
     cudaGetLastError();

@@ -254,9 +254,9 @@ cudaError_t launch_gemm_tf32x3(const float* A, const float* B, float* C, int M, 
 enum Activation : int { kActNone = 0, kActRelu = 1, kActHardSigmoid = 2, kActHardSwish = 3, kActSigmoid = 4, kActSilu = 5 };
 // depthwise conv, weights [C][R*S] (fp32, or fp16 with fp16 activations), folded batch-norm, activation
 // 3x3 / 5x5, stride 1 / 2 with at least two 16-byte channel vectors take the TMA-staged kernel (depthwise.cu), the rest a
-// one-thread-per-output kernel; w_f16: fp16 holds the filter's values, whatever w_dt they come in; error_flag is the device status word for the staged kernel's bounded waits
+// one-thread-per-output kernel; error_flag is the device status word for the staged kernel's bounded waits
 // in_l / out_l: where the pixels live (pitch 0 = dense NHWC)
-cudaError_t launch_depthwise(const void* x, const void* w, DType w_dt, int w_f16, const float* scale, const float* shift, void* y, DType dt,
+cudaError_t launch_depthwise(const void* x, const void* w, DType w_dt, const float* scale, const float* shift, void* y, DType dt,
                              int N, int H, int W, int C, int R, int S, int stride, int pad, int act, Layout in_l, Layout out_l,
                              int sm_count, int* error_flag, cudaStream_t st);
 // 3x3 convolution on the 3-channel NCHW network input, 16 .. 64 output channels, scale / shift / activation, NHWC
@@ -281,7 +281,7 @@ struct PointwiseArgs {
 bool pointwise_supported(int C, int Kout, int R, int S, int stride, int pad, DType dt);
 cudaError_t launch_pointwise(const PointwiseArgs& a, cudaStream_t st);
 bool depthwise_tma_supported(DType dt, int N, int H, int W, int C, int R, int S, int stride, int pad);
-cudaError_t launch_depthwise_tma(const void* x, const void* w, DType w_dt, int w_f16, const float* scale, const float* shift, void* y, DType dt,
+cudaError_t launch_depthwise_tma(const void* x, const void* w, DType w_dt, const float* scale, const float* shift, void* y, DType dt,
                                  int N, int H, int W, int C, int R, int S, int stride, int pad, int act, Layout in_l, Layout out_l,
                                  int sm_count, int* error_flag, cudaStream_t st);
 cudaError_t launch_activation(const void* x, void* y, DType dt, size_t n, int act, cudaStream_t st);

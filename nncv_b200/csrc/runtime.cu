@@ -1714,7 +1714,7 @@ int model_forward_device(Model& m, const void* src_dev, int N, int H, int W, cud
         const Model::DwW& w = m.dws[n.aux_idx];
         prof_begin(3, 2.0 * N * oh * ow * in.c * n.k * n.k, aes * in.c * N * ((double)in.h * in.w + (double)oh * ow), N * oh * ow, in.c,
                    n.k * n.k, 5, st);
-        if (launch_depthwise(in.p, w.w, kF32, m.ele_width == 2, w.scale, w.shift, o.p, adt, N, in.h, in.w, in.c, n.k, n.k, n.stride, n.pad, n.act, in.l,
+        if (launch_depthwise(in.p, w.w, kF32, w.scale, w.shift, o.p, adt, N, in.h, in.w, in.c, n.k, n.k, n.stride, n.pad, n.act, in.l,
                              o.l, g_dev.sm_count, g_dev.error_flag, st) != cudaSuccess) {
           cudaGetLastError();
           return fail(NNCV_B200_EINVAL, "depthwise node %d: %d channels are not a multiple of the 16-byte vector", n.id, in.c);
@@ -2987,7 +2987,7 @@ int nncv_b200_depthwise_conv_nhwc(const void* in, const void* weights, int w_dty
   if (!in || !weights || !out || N <= 0 || H <= 0 || W <= 0 || C <= 0 || R <= 0 || S <= 0 || stride <= 0 || pad < 0 || dtype < 0 ||
       dtype > 2 || act < 0 || act > 5)
     return fail(NNCV_B200_EINVAL, "depthwise_conv: bad argument");
-  if (launch_depthwise(in, weights, (DType)w_dtype, w_dtype == NNCV_B200_F16, scale, shift, out, (DType)dtype, N, H, W, C, R, S, stride, pad, act,
+  if (launch_depthwise(in, weights, (DType)w_dtype, scale, shift, out, (DType)dtype, N, H, W, C, R, S, stride, pad, act,
                        Layout{0, 0, 0}, Layout{0, 0, 0}, g_dev.sm_count, g_dev.error_flag, (cudaStream_t)stream) != cudaSuccess) {
     cudaGetLastError();
     return fail(NNCV_B200_EINVAL, "depthwise_conv: C must be a multiple of %d, weights fp32 (or fp16 with fp16 activations), output not empty",

@@ -1,6 +1,5 @@
-"""Depthwise convolution of fp16 maps with a filter in fp16, multiplied as it is, and with one in fp32 (the map converted by
-multiply-adds): against torch in 64 bits, at edges of tiles on both sides of the line between the two, with subnormals, infinities
-and NaN."""
+"""Depthwise convolution of fp16 maps (converted by multiply-adds with 1) with a filter in fp16 and in fp32: against torch in 64 bits,
+at edges of tiles, in one tile an SM and in several, with subnormals, infinities and NaN; the same bits in every batch."""
 import pytest
 
 torch = pytest.importorskip("torch")
@@ -64,3 +63,14 @@ def test_depthwise_halves_special(n, k, stride, half):
     fine = ~nan & ~big
     assert ((got.double() - ref).abs()[fine] <= (ref.abs() * 2.0 ** -11 + 2.0 ** -25 + 25 * 2.0 ** -24 * 65504)[fine]).all()
     assert (got.double()[big & ~nan] == ref[big & ~nan].sign() * 65504).all()
+
+
+@pytest.mark.parametrize("c,o,k,stride", [(288, 7, 5, 2), (120, 14, 5, 1), (144, 14, 5, 1), (576, 7, 5, 1), (88, 28, 3, 1)])
+@pytest.mark.parametrize("half", [True, False])
+def test_an_image_does_not_depend_on_its_batch(c, o, k, stride, half):
+    x, wt, scale, shift = _inputs(64, c, o * stride, o * stride, k, half)
+    whole, _ = _run(x, wt, scale, shift, stride, 1)
+    for n in (1, 16, 32, 48):
+        assert torch.equal(_run(x[:n], wt, scale, shift, stride, 1)[0], whole[:n])
+    # nor on what holds the filter
+    assert torch.equal(_run(x, wt.float(), scale, shift, stride, 1)[0], whole)
