@@ -26,14 +26,20 @@
 // bytes a clock for what the MMAs of a block of 64 channels read (1152 or 1536 clocks) and about twice that for what is copied in (72 or
 // 96 KB); 1430 and 1900 clocks a block are measured.  HALO, for filters of stride 1: one box of pixels serves a whole column of the filter
 // (42 KB a block), and the filter's planes lie together, so that a1 multiplies b2 and b3 in one MMA of 128 columns (896 clocks): 1220.
-// Two warps issue the MMAs, one the large products: an MMA takes its warp about 29 clocks, a wait or a commit about 80.  us before and
-// now: 56x56x64 of eight images 24.5 23.0, of 32 77 70, 28x28x128 of eight 24 21; 64 x 32 tiles 512 -> 512 on 7x7 by one CTA a tile 38.9
-// 28.6.  With few pixels a
+// Two warps issue the MMAs of 64-column tiles, one the large products: an MMA takes its warp about 29 clocks, a wait or a commit about 80.
+// us before and now: 56x56x64 of eight images 24.5 23.0, of 32 77 70, 28x28x128 of eight 24 21; 64 x 32 tiles 512 -> 512 on 7x7 by one CTA a
+// tile 38.9 28.6.  128 columns leave room for one pair of accumulators, and what the tensor core does while that pair is handed over decides:
+// one warp issues, ten of the twenty small steps between the two halves of the large products (512 -> 512 on 7x7 of 64 images by two
+// warps 99 us, by one with twelve steps and eight 92, with ten and ten 90).
+// Without HALO the first planes, which both issuing warps read, have a ring of their own: in one ring the warp of the large products has to
+// wait for the other planes too, or a slot's barrier could be two uses ahead of it.  Slots for first and other planes, us: 64 columns,
+// 64 -> 128 on 56x56 at stride 2 of eight images, one ring 16.7, 2 + 5 17.1, 3 + 4 16.35, 4 + 3 16.8; 128 columns, 128 -> 128 on 28x28 of
+// 32, one ring 57.5, 1 + 4 72.6, 2 + 3 56.8, 3 + 2 65.8.  With few pixels a
 // cluster of up to eight CTAs splits the reduction of a tile; each leaves its partial sums in shared memory and finishes
 // its share of the rows from all of them, in rank order, so that the result does not depend on timing.  (The CUDA-core
 // kernel needed a second pass over partial sums in global memory for that, and ran at a fifth of the fp32 rate.)
 // Roles: warp 0 TMA producer, one plane of both operands per ring slot (HALO: boxes, and blocks of the filter); warps 1 and 18 MMA
-// issuers; warps 2-17 epilogue (with eight of them, twice the columns each, ResNet-18 8x224 took 421 us and ResNet-50 4x224 802, where
+// issuers (128 columns: warp 1); warps 2-17 epilogue (with eight of them, twice the columns each, ResNet-18 8x224 took 421 us and ResNet-50 4x224 802, where
 // these took 395 and 704; sixteen in two sets, a pair of accumulators each, saved nothing in the blocks and cost 1 us a tile).
 // conv_f32_small_kernel, for one to four images: 64 pixels x 32 output channels, below.  conv_f32_choose takes one by a model of both.
 //
@@ -67,6 +73,7 @@ constexpr float kCut = 3.0f / (1 << 28);    // what a step of the tensor core cu
 template <int BN>
 struct Ring {   // a slot holds one plane of a block: 128 pixels and BN output channels x 64 channels
   static constexpr int kSlots = BN == 64 ? 7 : 5;
+  static constexpr int kFirst = BN == 64 ? 3 : 2;   // of them for first planes
   static constexpr int kSlot = kABytes + BN / 64 * kBBytes;
   static constexpr size_t kSmem = 1024 + (size_t)kSlots * kSlot + kTileBytes + 256;
 };
@@ -170,6 +177,9 @@ conv_f32_kernel(const __grid_constant__ CUtensorMap tm_in, const F32Params p) {
   const uint32_t d_full = empty + 8 * kSlots, d_empty = d_full + 8 * kAcc;   // pairs first
   const uint32_t part_ready = d_empty + 8 * kAcc, part_done = part_ready + 8;
   const uint32_t a_full = part_done + 8, a_empty = a_full + 8 * kBoxes;
+  // the slots for first planes, and for the others (halo tiles: one ring of blocks of weights)
+  constexpr uint32_t kFirst = HALO ? 0u : (uint32_t)Ring<kBN>::kFirst;
+  constexpr bool kOneIssuer = !HALO && kBN == 128;
   __shared__ uint32_t s_tmem;
   const int warp = ptx::warp_uniform((int)threadIdx.x >> 5), lane = threadIdx.x & 31;
   const int S = p.splits;
@@ -179,7 +189,7 @@ conv_f32_kernel(const __grid_constant__ CUtensorMap tm_in, const F32Params p) {
     s_abort = 0;
     for (int i = 0; i < kSlots; ++i) {
       ptx::mbar_init(full + 8 * i, 1);
-      ptx::mbar_init(empty + 8 * i, 2);   // both issuing warps
+      ptx::mbar_init(empty + 8 * i, !kOneIssuer && (HALO || i < (int)kFirst) ? 2 : 1);   // the issuing warps that read it
     }
     for (uint32_t i = 0; i < kAcc; ++i) {
       ptx::mbar_init(d_full + 8 * i, 1);
@@ -249,6 +259,14 @@ conv_f32_kernel(const __grid_constant__ CUtensorMap tm_in, const F32Params p) {
       ptx::bulk_g2s(sRing + slot * kSlot + pl * kBBytes, p.wpack + (((size_t)n_tile * 3 + pl) * kb_all + (size_t)tap * p.CB + cb) * kBBytes, kBBytes,
                     full + 8 * slot, issue);
   };
+  // the slots of a ring in turn
+  struct Turn {
+    uint32_t slot, first, end, ring = 0;
+    __device__ __forceinline__ void next() {
+      if (++slot == end) { slot = first; ring ^= 1u; }
+    }
+  };
+  const Turn firsts{0, 0, HALO ? (uint32_t)slots : kFirst}, others{kFirst, kFirst, (uint32_t)kSlots};
   // the packed weights never change: their first copies do not wait for the previous kernel
   uint32_t early = 0;
   if (warp == 0) {
@@ -264,11 +282,17 @@ conv_f32_kernel(const __grid_constant__ CUtensorMap tm_in, const F32Params p) {
       }
     } else if (!HALO && item_of(0, n0, oy0, ox0, n_tile)) {
       int cb = kb0 / p.taps, tap = kb0 - cb * p.taps;
-      for (int kb = kb0; kb < kb1 && early < (uint32_t)kSlots; ++kb) {
-        for (int pl = 0; pl < 3 && early < (uint32_t)kSlots; ++pl, ++early) {
-          ptx::mbar_arrive_expect_tx(full + 8 * early, kSlot, issue);
-          load_weights(n_tile, pl, cb, tap, early, issue);
+      Turn t1 = firsts, t2 = others;
+      for (int kb = kb0; kb < kb1; ++kb) {
+        int pl = 0;
+        for (; pl < 3; ++pl, ++early) {
+          Turn& t = pl == 0 ? t1 : t2;
+          if (t.ring != 0) break;   // round once
+          ptx::mbar_arrive_expect_tx(full + 8 * t.slot, kSlot, issue);
+          load_weights(n_tile, pl, cb, tap, t.slot, issue);
+          t.next();
         }
+        if (pl < 3) break;
         if (++tap == p.taps) { tap = 0; ++cb; }
       }
     }
@@ -308,7 +332,8 @@ conv_f32_kernel(const __grid_constant__ CUtensorMap tm_in, const F32Params p) {
       if (!okw && lane == 0 && p.error_flag) atomicCAS(p.error_flag, 0, (int)kErrWaitProducer);
     } else {
       const uint32_t issue = ptx::elect_one();
-      uint32_t slot = 0, ring = 0, cnt = 0, seen = 1;
+      Turn t1 = firsts, t2 = others;
+      uint32_t cnt = 0, seen = 1;
       bool okw = true;
       for (int i = 0; okw; ++i) {
         int n0, oy0, ox0, n_tile;
@@ -317,15 +342,18 @@ conv_f32_kernel(const __grid_constant__ CUtensorMap tm_in, const F32Params p) {
         int cb = kb0 / p.taps, tap = kb0 - cb * p.taps;
         int r = tap / p.S, s = tap - r * p.S;
         for (int kb = kb0; kb < kb1 && okw; ++kb) {
+#pragma unroll
           for (int pl = 0; pl < 3; ++pl, ++cnt) {
             const bool begun = cnt < early;
-            if (!ptx::warp_all(seen) && !ptx::warp_wait(empty + 8 * slot, ring ^ 1u, abort_flag)) { okw = false; break; }
-            if (!begun) ptx::mbar_arrive_expect_tx(full + 8 * slot, kSlot, issue);
-            const uint32_t dst = sRing + slot * kSlot;
-            ptx::tma_load_5d(dst, &tm_in, cb * 64, xb + s, yb + r, n0, pl, full + 8 * slot, issue);
-            if (!begun) load_weights(n_tile, pl, cb, tap, slot, issue);
-            if (++slot == kSlots) { slot = 0; ring ^= 1u; }
-            seen = ptx::mbar_peek(empty + 8 * slot, ring ^ 1u);
+            Turn& t = pl == 0 ? t1 : t2;
+            if (!ptx::warp_all(seen) && !ptx::warp_wait(empty + 8 * t.slot, t.ring ^ 1u, abort_flag)) { okw = false; break; }
+            if (!begun) ptx::mbar_arrive_expect_tx(full + 8 * t.slot, kSlot, issue);
+            const uint32_t dst = sRing + t.slot * kSlot;
+            ptx::tma_load_5d(dst, &tm_in, cb * 64, xb + s, yb + r, n0, pl, full + 8 * t.slot, issue);
+            if (!begun) load_weights(n_tile, pl, cb, tap, t.slot, issue);
+            t.next();
+            const Turn& n = pl == 2 ? t1 : t2;
+            seen = ptx::mbar_peek(empty + 8 * n.slot, n.ring ^ 1u);
           }
           if (++s == p.S) { s = 0; ++r; }
           if (++tap == p.taps) { tap = r = s = 0; ++cb; }
@@ -336,21 +364,23 @@ conv_f32_kernel(const __grid_constant__ CUtensorMap tm_in, const F32Params p) {
   } else if (warp == 1 || warp == kLargeWarp) {
     // ------------------------------------------------------------------ MMA issuers -----
     // One warp for the large products, one for the small ones: an MMA takes its warp about 29 clocks and a wait or a commit about 80,
-    // so a lone warp needed longer for the 20 or 24 MMAs of a block, with their hand-overs, than the tensor core.
+    // so a lone warp needed longer for the 20 or 24 MMAs of a block, with their hand-overs, than the tensor core.  MMAs of 128 columns
+    // take twice as long, and a lone warp orders them.
     const bool large_warp = warp == kLargeWarp;
     const uint32_t issue = ptx::elect_one();
     const uint32_t idesc = ptx::umma_idesc(128, kBN, 1), idesc2 = HALO ? ptx::umma_idesc(128, 128, 1) : idesc;
-    uint32_t slot = 0, ring = 0, as = 0, a_ring = 0;   // halo tiles: the box in use
-    uint32_t uses = 0;               // of pairs, or of small accumulators
+    Turn t1 = firsts, t2 = others;   // halo tiles: blocks of weights, none
+    uint32_t as = 0, a_ring = 0;     // halo tiles: the box in use
+    uint32_t uses = 0, pair_uses = 0;   // of small accumulators and of pairs, as far as this warp fills them
     bool okw = true;
     uint32_t seen = ptx::mbar_peek(full, 0);
-    // the next slot is full
-    auto arrive = [&](uint32_t& now) {
-      if (!ptx::warp_all(seen) && !ptx::warp_wait(full + 8 * slot, ring, abort_flag)) return false;
+    // the slot t is full; `then` is the one that this warp needs after it
+    auto arrive = [&](Turn& t, const Turn& then, uint32_t& now) {
+      if (!ptx::warp_all(seen) && !ptx::warp_wait(full + 8 * t.slot, t.ring, abort_flag)) return false;
       ptx::tc_fence_after();
-      now = slot;
-      if (++slot == (uint32_t)slots) { slot = 0; ring ^= 1u; }
-      seen = ptx::mbar_peek(full + 8 * slot, ring);
+      now = t.slot;
+      t.next();
+      seen = ptx::mbar_peek(full + 8 * then.slot, then.ring);
       return true;
     };
     // step k4 (16 channels) of operands whose descriptors start at a and b
@@ -362,20 +392,18 @@ conv_f32_kernel(const __grid_constant__ CUtensorMap tm_in, const F32Params p) {
 #pragma unroll
       for (uint32_t k4 = 0; k4 < 4; ++k4) mma(d, a, b, k4, id, k4 == 0 ? (fresh ^ 1u) : 1u);
     };
-    // the four steps of the large products, each into an accumulator of its own, handed over in pairs
-    auto four_large = [&](uint32_t a, uint32_t b) {
+    // two steps of the large products, each into an accumulator of its own, handed over as a pair
+    auto two_large = [&](uint32_t a, uint32_t b, uint32_t k4) {
+      const uint32_t pair = pair_uses % kPairs;
+      if (!ptx::warp_wait(d_empty + 8 * pair, ((pair_uses / kPairs) & 1u) ^ 1u, abort_flag)) return false;
+      ptx::tc_fence_after();
 #pragma unroll
-      for (uint32_t k4 = 0; k4 < 4; k4 += 2, ++uses) {
-        const uint32_t pair = uses % kPairs;
-        if (!ptx::warp_wait(d_empty + 8 * pair, ((uses / kPairs) & 1u) ^ 1u, abort_flag)) return false;
-        ptx::tc_fence_after();
-#pragma unroll
-        for (uint32_t j = 0; j < 2; ++j) mma(tmem_base + (2 * pair + j) * kBN, a, b, k4 + j, idesc, 0u);
-        ptx::tc_commit(d_full + 8 * pair, issue);
-      }
+      for (uint32_t j = 0; j < 2; ++j) mma(tmem_base + (2 * pair + j) * kBN, a, b, k4 + j, idesc, 0u);
+      ptx::tc_commit(d_full + 8 * pair, issue);
+      ++pair_uses;
       return true;
     };
-    for (int i = 0; okw; ++i) {
+    for (int i = 0; okw && !(kOneIssuer && large_warp); ++i) {
       int n0, oy0, ox0, n_tile;
       if (!item_of(i, n0, oy0, ox0, n_tile)) break;
       int r = HALO ? kb0 % p.R : 0;   // rows of the filter divide the taps
@@ -392,12 +420,12 @@ conv_f32_kernel(const __grid_constant__ CUtensorMap tm_in, const F32Params p) {
         uint32_t now[3];
         if constexpr (HALO) {
           if ((kb == kb0 || r == 0) && !ptx::warp_wait(a_full + 8 * as, a_ring, abort_flag)) { okw = false; break; }
-          if (!arrive(now[0])) { okw = false; break; }
+          if (!arrive(t1, t1, now[0])) { okw = false; break; }
           // filter row r reads the box from its row r on: mp pixels, a multiple of eight rows of 128 bytes
           const uint32_t b = ptx::smem_desc_k128_lo(sRing + now[0] * kSlot), bp = kBBytes >> 4, ap = (uint32_t)p.a_plane >> 4;
           const uint32_t a = ptx::smem_desc_k128_lo(sBox + as * 3 * (uint32_t)p.a_plane + (uint32_t)(r * p.mp) * 128u);
           if (large_warp) {
-            if (!four_large(a, b)) { okw = false; break; }
+            if (!two_large(a, b, 0) || !two_large(a, b, 2)) { okw = false; break; }
           } else {
             if (!small_ready()) { okw = false; break; }
             // two accumulators side by side: a1 b2 | a1 b3, a2 b1 | a2 b2, a3 b1
@@ -414,23 +442,27 @@ conv_f32_kernel(const __grid_constant__ CUtensorMap tm_in, const F32Params p) {
         } else {
           auto at = [&](uint32_t sl) { return ptx::smem_desc_k128_lo(sRing + sl * kSlot); };
           constexpr uint32_t kB = kABytes >> 4;
-          if (!arrive(now[0])) { okw = false; break; }
+          if (!arrive(t1, large_warp ? t1 : t2, now[0])) { okw = false; break; }
+          const uint32_t first = at(now[0]);
           if (large_warp) {
-            if (!four_large(at(now[0]), at(now[0]) + kB)) { okw = false; break; }
+            if (!two_large(first, first + kB, 0) || !two_large(first, first + kB, 2)) { okw = false; break; }
             ptx::tc_commit(empty + 8 * now[0], issue);
-            // nothing to do with the other planes: they have come when the barrier counts this use of their slots
-            if (!arrive(now[1])) { okw = false; break; }
-            if (lane == 0) ptx::mbar_arrive(empty + 8 * now[1]);
-            if (!arrive(now[2])) { okw = false; break; }
-            if (lane == 0) ptx::mbar_arrive(empty + 8 * now[2]);
           } else {
-            if (!arrive(now[1]) || !small_ready()) { okw = false; break; }
-            product(ds, at(now[0]), at(now[1]) + kB, idesc, fresh);
-            product(ds, at(now[1]), at(now[0]) + kB, idesc, 0u);
-            product(ds, at(now[1]), at(now[1]) + kB, idesc, 0u);
-            if (!arrive(now[2])) { okw = false; break; }
-            product(ds, at(now[0]), at(now[2]) + kB, idesc, 0u);
-            product(ds, at(now[2]), at(now[0]) + kB, idesc, 0u);
+            if (kOneIssuer && !two_large(first, first + kB, 0)) { okw = false; break; }
+            if (!arrive(t2, t2, now[1]) || !small_ready()) { okw = false; break; }
+            product(ds, first, at(now[1]) + kB, idesc, fresh);
+            product(ds, at(now[1]), first + kB, idesc, 0u);
+            const uint32_t second = at(now[1]);
+#pragma unroll
+            for (uint32_t k4 = 0; k4 < 4; ++k4) {
+              // half of the twenty small steps later, when the epilogue has had the time to empty the accumulators
+              if (kOneIssuer && k4 == 2 && !two_large(first, first + kB, 2)) { okw = false; break; }
+              mma(ds, second, second + kB, k4, idesc, 1u);
+            }
+            if (!okw) break;
+            if (!arrive(t2, t1, now[2])) { okw = false; break; }
+            product(ds, first, at(now[2]) + kB, idesc, 0u);
+            product(ds, at(now[2]), first + kB, idesc, 0u);
 #pragma unroll
             for (int pl = 0; pl < 3; ++pl) ptx::tc_commit(empty + 8 * now[pl], issue);
           }
@@ -1393,7 +1425,7 @@ cudaError_t launch_conv_f32(const ConvF32Args& args, cudaStream_t stream) {
     // two boxes, weights in the rest
     p.R = stem ? 4 : a.R;
     p.a_plane = t.plane();
-        p.b_stages = (int)std::min((kHaloSmem - kHaloFixed - 3 * (size_t)p.a_plane * kBoxes) / kHaloBlock, (size_t)kHaloB);
+    p.b_stages = (int)std::min((kHaloSmem - kHaloFixed - 3 * (size_t)p.a_plane * kBoxes) / kHaloBlock, (size_t)kHaloB);
     smem = kHaloFixed + 3 * (size_t)p.a_plane * kBoxes + kHaloBlock * p.b_stages;
   }
 

@@ -61,3 +61,33 @@ def test_a_box_keeps_infinities_where_they_belong():
     want = np.zeros((4, 64, 7, 7), bool)
     want[1, :, 5:7, 2:5] = True
     assert np.array_equal(np.isinf(y), want) and not np.isnan(y).any()
+
+
+@pytest.mark.parametrize("bn,splits", [(64, 1), (64, 4), (128, 1), (128, 2), (128, 8)])
+@pytest.mark.parametrize("case", [
+    # n, c, h, w, k, r, stride: one block of 64 channels, two, four, as many as the rings hold and more, a multiple of neither ring
+    (2, 64, 9, 9, 128, 1, 1), (2, 128, 9, 9, 132, 1, 1), (1, 232, 5, 7, 260, 1, 1), (2, 64, 20, 21, 128, 3, 2), (3, 136, 13, 11, 192, 3, 2), (2, 512, 7, 7, 256, 3, 1),
+    # more tiles than SMs: the rings go on from tile to tile
+    (40, 72, 28, 28, 256, 1, 1), (24, 64, 57, 55, 128, 3, 2), (70, 48, 15, 15, 320, 1, 2),
+])
+def test_a_copy_for_every_tap(case, bn, splits):
+    n, c, h, w, k, r, stride = case
+    if splits > r * r * -(-c // 64):
+        pytest.skip("more CTAs than blocks of 64 channels")
+    g = np.random.default_rng(sum(case))
+    x = g.standard_normal((n, c, h, w)).astype(np.float32)
+    wt = (g.standard_normal((k, c, r, r)) * np.sqrt(2.0 / (c * r * r))).astype(np.float32)
+    conv = G.Conv(wt, stride, r // 2, F32)
+    try:
+        check(lib().nncv_b200_conv_set_tile(conv.h, bn, splits, 1))
+        check(lib().nncv_b200_profile(1))
+        y, _ = conv.run(x)
+        made = [q["bn"] for q in rt.profile_records() if q["kind"] == 1]
+        check(lib().nncv_b200_profile(0))
+        again, _ = conv.run(x)
+    finally:
+        conv.close()
+    assert made == [10 * bn + splits] and np.array_equal(y, again)
+    ref = torch.nn.functional.conv2d(torch.from_numpy(x).double(), torch.from_numpy(wt).double(), stride=stride, padding=r // 2).numpy()
+    assert np.isfinite(y).all() and G.rel_l2(y, ref) <= 4 * 2.0 ** -23 + 2.0 ** -24 * np.sqrt(4 * r * r * np.ceil(c / 64))
+    assert lib().nncv_b200_device_status() == 0
