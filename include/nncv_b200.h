@@ -188,8 +188,8 @@ typedef struct {
                     conv, 3 memory-bound helper, 4 fused stem conv + max-pool, 5 tcgen05 implicit GEMM
                     (TMA-fed A), 6 Winograd F(2x2,3x3) (all three stages), 7 shifted-view conv on CTA pairs */
   int M, N, K;   /* GEMM view of the launch (helpers: elements, channels, 0) */
-  int bn;        /* N tile (kind 0; kind 1 on the CUDA cores); N tile * 10 + CTAs of a tile (kind 1 on the
-                    tensor cores); N tile * 10 + 1 with resident weights, + 2 on CTA pairs (kind 5); helper
+  int bn;        /* N tile (kind 0; kind 1 on the CUDA cores); N tile * 10 + CTAs of a tile, + 1000 where the
+                    pixels of a filter column are copied at once (kind 1 on the tensor cores); N tile * 10 + 1 with resident weights, + 2 on CTA pairs (kind 5); helper
                     id (kind 3) */
   double flops;  /* algorithmic: 2*M*N*K with K = C*R*S (direct-convolution count) */
   double bytes;  /* algorithmic: each operand and result once */

@@ -536,7 +536,7 @@ int conv_run_planes(nncv_b200_conv* c, const void* in, bool stem, int N, int H, 
   const double Ms = (double)N * a.OH * a.OW;
   prof_begin(1, 2.0 * Ms * c->Kout * c->C * c->R * c->S,
              6.0 * ((double)N * H * W * c->C + (double)c->Kout * c->C * c->R * c->S + Ms * c->Kout * (residual ? 2 : 1)), (int)Ms, c->Kout,
-             c->C * c->R * c->S, a.bn * 10 + a.splits, st);
+             c->C * c->R * c->S, a.bn * 10 + a.splits + (a.halo > 0 ? 1000 : 0), st);
   LAUNCH(launch_conv_f32(a, st));
   prof_end(st);
   return NNCV_B200_OK;

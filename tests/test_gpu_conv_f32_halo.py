@@ -35,7 +35,7 @@ def test_one_box_for_a_column_of_the_filter(case, splits):
             y, _ = conv.run(x)
             made = [q["bn"] for q in rt.profile_records() if q["kind"] == 1]
             check(lib().nncv_b200_profile(0))
-            assert made == [640 + splits]
+            assert made == [640 + splits + (1000 if way == 2 else 0)]   # what ran: boxes for columns, copies for taps
             got.append(y)
     finally:
         conv.close()
@@ -55,12 +55,36 @@ def test_a_box_keeps_infinities_where_they_belong():
     conv = G.Conv(np.full((64, 64, 3, 3), 0.125, np.float32), 1, 1, F32)
     try:
         check(lib().nncv_b200_conv_set_tile(conv.h, 64, 1, 2))
+        check(lib().nncv_b200_profile(1))
         y, _ = conv.run(x)
+        made = [q["bn"] for q in rt.profile_records() if q["kind"] == 1]
+        check(lib().nncv_b200_profile(0))
     finally:
         conv.close()
+    assert made == [1641]
     want = np.zeros((4, 64, 7, 7), bool)
     want[1, :, 5:7, 2:5] = True
     assert np.array_equal(np.isinf(y), want) and not np.isnan(y).any()
+
+
+@pytest.mark.parametrize("case", [(2, 128, 9, 9, 64, 1, 1), (2, 64, 9, 9, 64, 3, 2), (1, 64, 40, 24, 64, 19, 1)])
+def test_what_boxes_do_not_fit_is_copied_by_taps(case):
+    """1x1 filters, strides, and columns too long for two boxes in shared memory."""
+    n, c, h, w, k, r, stride = case
+    g = np.random.default_rng(sum(case))
+    x, wt = g.standard_normal((n, c, h, w)).astype(np.float32), (g.standard_normal((k, c, r, r)) / r).astype(np.float32)
+    conv = G.Conv(wt, stride, r // 2, F32)
+    try:
+        check(lib().nncv_b200_conv_set_tile(conv.h, 64, 1, 2))
+        check(lib().nncv_b200_profile(1))
+        y, _ = conv.run(x)
+        made = [q["bn"] for q in rt.profile_records() if q["kind"] == 1]
+        check(lib().nncv_b200_profile(0))
+    finally:
+        conv.close()
+    assert made == [641]
+    ref = torch.nn.functional.conv2d(torch.from_numpy(x).double(), torch.from_numpy(wt).double(), stride=stride, padding=r // 2).numpy()
+    assert G.rel_l2(y, ref) <= 4 * 2.0 ** -23 + 2.0 ** -24 * np.sqrt(4 * r * r)
 
 
 @pytest.mark.parametrize("bn,splits", [(64, 1), (64, 4), (128, 1), (128, 2), (128, 8)])
