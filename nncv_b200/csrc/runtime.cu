@@ -1884,10 +1884,20 @@ struct CopiesInFlight {
   }
 };
 
+// Results that leave through the library's pinned memory, which a kernel writes together with the status word, and from there to the
+// caller's by the host: up to these bytes, by what memory of the caller's they go to.  A small network's calls, us, by two copies of the
+// copy engine and by the kernel: to pinned memory 31 KB 37.6 27.1, 62 KB 32.4 30.3, 125 KB 38.7 37.0, 250 KB 41.5 46.1, 1 MB 56 98 (the host's
+// copy is what grows); to pageable memory, which the copies reached by way of pinned memory too, 62 KB 36.2 30.8, 500 KB 66.7 60.7, 4 MB
+// 385 378, and with rows of 1001 fp16 values, written in twos of bytes, 29 KB 40.2 36.0, 2 MB 222 218.
+constexpr size_t kDeliverPinned = 64 << 10, kDeliverPageable = 4 << 20;
+// Rows in this device's memory that the last layer writes itself instead of leaving them to a copy.  Forwards of 224 x 224 images, us, by
+// copy and in place: ResNet-18 fp16 one image 99.2 94.7, 8 (16 KB) 139.7 134.5, 16 187.3 179.3, 32 (64 KB) 236.3 233.2; from there on nothing:
+// 48 313.3 313.4, 64 343.7 341.6, 128 585 611, 256 1122 1131 (runs differ by 4 %); MobileNetV3 8 221.8 215.4, 32 318.1 316.5, 256 870 867.
+constexpr size_t kInPlace = 64 << 10;
+
 // A batch of images in host memory, in n_parts parts of equal size: every copy, every forward, one wait.  Where the batch is no
 // multiple, the last part takes images of the one before with it (layers are tuned for one batch size, and a 16-bit image's logits
 // do not depend on its part).
-constexpr size_t kDeliver = 64 << 10;   // results that go into pinned memory of the caller's by way of the library's: as far as the host's copy takes less
 int forward_host(Model& m, const char* sp, bool pinned, char* dp, bool dst_dev, size_t dst_stride, int N, int H, int W, cudaStream_t st,
                  int n_parts) {
   int rc;
@@ -1904,9 +1914,7 @@ int forward_host(Model& m, const char* sp, bool pinned, char* dp, bool dst_dev, 
     cudaDeviceSynchronize();
     if ((rc = reserve_logits(m, logits_bytes))) return rc;
   }
-  // Small results and the status word leave through the library's pinned memory, which one kernel writes: the step from one copy of the
-  // copy engine to the next takes 3 us.
-  const bool stage_out = !dst_dev && row * N <= (is_pinned_ptr(dp) ? kDeliver : 4u << 20);
+  const bool stage_out = !dst_dev && row * N <= (is_pinned_ptr(dp) ? kDeliverPinned : kDeliverPageable);
   if ((rc = m.result.reserve(256 + (stage_out ? row * N : 0)))) return rc;
   cudaStream_t cst = st;
   if (n_parts > 1) {
@@ -2000,10 +2008,8 @@ int forward_slice(Model& m, const char* sp, bool src_dev, char* dp, bool dst_dev
   if (src_dev) {
     if ((rc = ensure_workspace(m, N, H, W))) return rc;
     m.logits_off = 0;
-    // Rows without gaps in this GPU's memory, on the boundary of the widest store: the last layer writes them itself, one image in 93.7 us
-    // instead of 95.3.  Results of long passes are copied as before: without the pause that the copy makes between passes, 256 images
-    // took 1156 us, with it 1149 (ResNet-18, many passes, the GPU at its power limit).
-    const bool in_place = row * N <= kDeliver && dst_dev && dst_stride * ew == row && !(reinterpret_cast<uintptr_t>(dp) & 31) && is_own_device_ptr(dp);
+    // rows without gaps in this GPU's memory, on the boundary of the widest store
+    const bool in_place = row * N <= kInPlace && dst_dev && dst_stride * ew == row && !(reinterpret_cast<uintptr_t>(dp) & 31) && is_own_device_ptr(dp);
     if ((rc = model_forward_device(m, sp, N, H, W, st, in_place ? dp : nullptr))) return rc;
     if (in_place) {
       if (device_only) return ok();
