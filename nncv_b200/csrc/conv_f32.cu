@@ -24,7 +24,7 @@
 //
 // Two kernels.  conv_f32_kernel: one CTA computes 128 pixels x 64 or 128 output channels.  What bounds it: the port of shared memory, 128
 // bytes a clock for what the MMAs of a block of 64 channels read (1152 or 1536 clocks) and about twice that for what is copied in (72 or
-// 96 KB); 1430 and 1900 clocks a block are measured.  HALO, for filters of stride 1: one box of pixels serves a whole column of the filter
+// 96 KB); 1430 and 1900 clocks a block were measured.  HALO, for filters of stride 1: one box of pixels serves a whole column of the filter
 // (42 KB a block), and the filter's planes lie together, so that a1 multiplies b2 and b3 in one MMA of 128 columns (896 clocks): 1220.
 // Two warps issue the MMAs of 64-column tiles, one the large products: an MMA takes its warp about 29 clocks, a wait or a commit about 80.
 // us before and now: 56x56x64 of eight images 24.5 23.0, of 32 77 70, 28x28x128 of eight 24 21; 64 x 32 tiles 512 -> 512 on 7x7 by one CTA a
@@ -40,10 +40,10 @@
 // kernel needed a second pass over partial sums in global memory for that, and ran at a fifth of the fp32 rate.)
 // Roles: warp 0 TMA producer, one plane of both operands per ring slot (HALO: boxes, and blocks of the filter); warps 1 and 18 MMA
 // issuers (128 columns: warp 1); warps 2-17 epilogue (with eight of them, twice the columns each, ResNet-18 8x224 took 421 us and ResNet-50 4x224 802, where
-// these took 395 and 704; sixteen in two sets, a pair of accumulators each, saved nothing in the blocks and cost 1 us a tile).
+// these took 395 and 704 with one sum a column; sixteen in two sets, a pair of accumulators each, saved nothing in the blocks and cost 1 us a tile).
 // conv_f32_small_kernel, for one to four images: 64 pixels x 32 output channels, below.  conv_f32_choose takes one by a model of both.
 //
-// ResNet-18 fp32 against the CUDA-core kernel, from device memory: 1x256 470 -> 177 us, 8x224 1626 -> 403 us.
+// ResNet-18 fp32 against the CUDA-core kernel, from device memory: 1x256 470 -> 177 us, 8x224 1626 -> 401 us.
 // Every wait is bounded and abortable; a timed-out wait sets the device status word.
 #include <cuda.h>
 #include <cudaTypedefs.h>
@@ -490,7 +490,7 @@ conv_f32_kernel(const __grid_constant__ CUtensorMap tm_in, const F32Params p) {
       const uint32_t lane_base = tmem_base + ((uint32_t)(quad * 32) << 16) + (uint32_t)(part * kCols);
       // 64 columns: the large products in two sums, of steps 0 and 1 and of steps 2 and 3 of the blocks, half as many roundings one after
       // another: clusters of fewer CTAs have longer sums, and with one sum the logits of ResNet-18 were 1.0 % further off on average than
-      // before these tiles, with two 0.1 % (ResNet-50 0.2 % and 1.4 % nearer).  396 -> 403 us and 706 -> 729 us for it.
+      // before these tiles, with two 0.1 % (ResNet-50 0.2 % and 1.4 % nearer), for 0.3 % of the time (ResNet-18 8x224 399 -> 401 us).
       constexpr bool kTwo = kBN == 64;
       float sum[kCols], other[kTwo ? kCols : 1];
 #pragma unroll
@@ -563,89 +563,89 @@ conv_f32_kernel(const __grid_constant__ CUtensorMap tm_in, const F32Params p) {
       // 64 columns at a time
 #pragma unroll
       for (int pass = 0; pass < kNT; ++pass) {
-      const uint32_t turn = (uint32_t)(i * kNT + pass);   // uses of the shared tile
-      const int n = n_tile * kBN + pass * 64 + 4 * g;
-      // residual planes, requested before the sums are in the shared tile
-      uint2 res[kRows][3];
-      if (p.residual && !p.res_f32 && n < p.Kout) {
+        const uint32_t turn = (uint32_t)(i * kNT + pass);   // uses of the shared tile
+        const int n = n_tile * kBN + pass * 64 + 4 * g;
+        // residual planes, requested before the sums are in the shared tile
+        uint2 res[kRows][3];
+        if (p.residual && !p.res_f32 && n < p.Kout) {
 #pragma unroll
-        for (int k = 0; k < kRows; ++k)
-          if (pix[k] >= 0) {
+          for (int k = 0; k < kRows; ++k)
+            if (pix[k] >= 0) {
 #pragma unroll
-            for (int q = 0; q < 3; ++q)
-              res[k][q] = __ldg(reinterpret_cast<const uint2*>(static_cast<const __nv_bfloat16*>(p.residual) + q * p.res_plane + (long long)pix[k] * p.Kout + n));
-          }
-      }
-      // the previous item's partial sums have been read by everybody
-      if (okw && turn > 0 && S > 1) okw = ptx::warp_wait_cluster(part_done, (turn - 1) & 1u, abort_flag);
-      if (!ptx::named_bar_and(1, kEpiThreads, okw)) { okw = false; break; }
-      if (kNT == 1 || part >> 1 == pass) {
-        constexpr int kChunks = kCols / 4;   // 16 bytes each; sixteen chunks a row, those of a row's parts one after another
-#pragma unroll
-        for (int c = 0; c < kChunks; ++c)
-          epi::sts128(sTile + (uint32_t)row * 256u + (((uint32_t)((kNT == 1 ? part : part & 1) * kChunks + c) ^ (uint32_t)(row & 7)) << 4),
-                      __float_as_uint(sum[4 * c]), __float_as_uint(sum[4 * c + 1]), __float_as_uint(sum[4 * c + 2]), __float_as_uint(sum[4 * c + 3]));
-      }
-      ptx::named_bar_sync(2, kEpiThreads);
-      if (S > 1) {
-        if (et < S) ptx::mbar_arrive_remote(ptx::map_to_cta(part_ready, (uint32_t)et));
-        okw = ptx::warp_wait_cluster(part_ready, turn & 1u, abort_flag);
+              for (int q = 0; q < 3; ++q)
+                res[k][q] = __ldg(reinterpret_cast<const uint2*>(static_cast<const __nv_bfloat16*>(p.residual) + q * p.res_plane + (long long)pix[k] * p.Kout + n));
+            }
+        }
+        // the previous item's partial sums have been read by everybody
+        if (okw && turn > 0 && S > 1) okw = ptx::warp_wait_cluster(part_done, (turn - 1) & 1u, abort_flag);
         if (!ptx::named_bar_and(1, kEpiThreads, okw)) { okw = false; break; }
-      }
-      if (n < p.Kout) {
-        float4 sc = make_float4(1.f, 1.f, 1.f, 1.f), sh = make_float4(0.f, 0.f, 0.f, 0.f);
-        float* scp = reinterpret_cast<float*>(&sc);
-        float* shp = reinterpret_cast<float*>(&sh);
+        if (kNT == 1 || part >> 1 == pass) {
+          constexpr int kChunks = kCols / 4;   // 16 bytes each; sixteen chunks a row, those of a row's parts one after another
 #pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          if (p.scale) scp[e] = __ldg(p.scale + n + e);
-          if (p.shift) shp[e] = __ldg(p.shift + n + e);
+          for (int c = 0; c < kChunks; ++c)
+            epi::sts128(sTile + (uint32_t)row * 256u + (((uint32_t)((kNT == 1 ? part : part & 1) * kChunks + c) ^ (uint32_t)(row & 7)) << 4),
+                        __float_as_uint(sum[4 * c]), __float_as_uint(sum[4 * c + 1]), __float_as_uint(sum[4 * c + 2]), __float_as_uint(sum[4 * c + 3]));
         }
-#pragma unroll
-        for (int k = 0; k < kRows; ++k) {
-          if (pix[k] < 0) continue;
-          const int r = row_lo + (et >> 4) + k * (kEpiThreads / 16);
-          const uint32_t at = sTile + (uint32_t)r * 256u + (((uint32_t)g ^ (uint32_t)(r & 7)) << 4);
-          float4 v;
-          if (S == 1) {
-            const uint4 w = epi::lds128(at);
-            v = make_float4(__uint_as_float(w.x), __uint_as_float(w.y), __uint_as_float(w.z), __uint_as_float(w.w));
-          } else {
-            v = ptx::ld_cluster_f4(ptx::map_to_cta(at, 0));
-            for (int q = 1; q < S; ++q) {
-              const float4 w = ptx::ld_cluster_f4(ptx::map_to_cta(at, (uint32_t)q));
-              v.x += w.x; v.y += w.y; v.z += w.z; v.w += w.w;
-            }
-          }
-          v.x = fmaf(v.x, sc.x, sh.x); v.y = fmaf(v.y, sc.y, sh.y); v.z = fmaf(v.z, sc.z, sh.z); v.w = fmaf(v.w, sc.w, sh.w);
-          if (p.residual) {
-            float4 f;
-            if (p.res_f32) {
-              f = __ldg(reinterpret_cast<const float4*>(static_cast<const float*>(p.residual) + (long long)pix[k] * p.ldo + n));
-            } else {
-              f = join4(res[k]);
-            }
-            v.x += f.x; v.y += f.y; v.z += f.z; v.w += f.w;
-          }
-          if (p.relu) {
-            v.x = !(v.x <= 0.0f) ? v.x : 0.0f; v.y = !(v.y <= 0.0f) ? v.y : 0.0f;
-            v.z = !(v.z <= 0.0f) ? v.z : 0.0f; v.w = !(v.w <= 0.0f) ? v.w : 0.0f;
-          }
-          if (p.out_f32) {
-            *reinterpret_cast<float4*>(reinterpret_cast<float*>(p.out) + (long long)pix[k] * p.ldo + n) = v;
-          } else {
-            uint2 o[3];
-            split4(v, o);
-#pragma unroll
-            for (int q = 0; q < 3; ++q)
-              *reinterpret_cast<uint2*>(reinterpret_cast<__nv_bfloat16*>(p.out) + q * p.out_plane + (long long)pix[k] * p.Kout + n) = o[q];
-          }
-        }
-      }
-      if (S > 1) {
         ptx::named_bar_sync(2, kEpiThreads);
-        if (et < S) ptx::mbar_arrive_remote(ptx::map_to_cta(part_done, (uint32_t)et));
-      }
+        if (S > 1) {
+          if (et < S) ptx::mbar_arrive_remote(ptx::map_to_cta(part_ready, (uint32_t)et));
+          okw = ptx::warp_wait_cluster(part_ready, turn & 1u, abort_flag);
+          if (!ptx::named_bar_and(1, kEpiThreads, okw)) { okw = false; break; }
+        }
+        if (n < p.Kout) {
+          float4 sc = make_float4(1.f, 1.f, 1.f, 1.f), sh = make_float4(0.f, 0.f, 0.f, 0.f);
+          float* scp = reinterpret_cast<float*>(&sc);
+          float* shp = reinterpret_cast<float*>(&sh);
+#pragma unroll
+          for (int e = 0; e < 4; ++e) {
+            if (p.scale) scp[e] = __ldg(p.scale + n + e);
+            if (p.shift) shp[e] = __ldg(p.shift + n + e);
+          }
+#pragma unroll
+          for (int k = 0; k < kRows; ++k) {
+            if (pix[k] < 0) continue;
+            const int r = row_lo + (et >> 4) + k * (kEpiThreads / 16);
+            const uint32_t at = sTile + (uint32_t)r * 256u + (((uint32_t)g ^ (uint32_t)(r & 7)) << 4);
+            float4 v;
+            if (S == 1) {
+              const uint4 w = epi::lds128(at);
+              v = make_float4(__uint_as_float(w.x), __uint_as_float(w.y), __uint_as_float(w.z), __uint_as_float(w.w));
+            } else {
+              v = ptx::ld_cluster_f4(ptx::map_to_cta(at, 0));
+              for (int q = 1; q < S; ++q) {
+                const float4 w = ptx::ld_cluster_f4(ptx::map_to_cta(at, (uint32_t)q));
+                v.x += w.x; v.y += w.y; v.z += w.z; v.w += w.w;
+              }
+            }
+            v.x = fmaf(v.x, sc.x, sh.x); v.y = fmaf(v.y, sc.y, sh.y); v.z = fmaf(v.z, sc.z, sh.z); v.w = fmaf(v.w, sc.w, sh.w);
+            if (p.residual) {
+              float4 f;
+              if (p.res_f32) {
+                f = __ldg(reinterpret_cast<const float4*>(static_cast<const float*>(p.residual) + (long long)pix[k] * p.ldo + n));
+              } else {
+                f = join4(res[k]);
+              }
+              v.x += f.x; v.y += f.y; v.z += f.z; v.w += f.w;
+            }
+            if (p.relu) {
+              v.x = !(v.x <= 0.0f) ? v.x : 0.0f; v.y = !(v.y <= 0.0f) ? v.y : 0.0f;
+              v.z = !(v.z <= 0.0f) ? v.z : 0.0f; v.w = !(v.w <= 0.0f) ? v.w : 0.0f;
+            }
+            if (p.out_f32) {
+              *reinterpret_cast<float4*>(reinterpret_cast<float*>(p.out) + (long long)pix[k] * p.ldo + n) = v;
+            } else {
+              uint2 o[3];
+              split4(v, o);
+#pragma unroll
+              for (int q = 0; q < 3; ++q)
+                *reinterpret_cast<uint2*>(reinterpret_cast<__nv_bfloat16*>(p.out) + q * p.out_plane + (long long)pix[k] * p.Kout + n) = o[q];
+            }
+          }
+        }
+        if (S > 1) {
+          ptx::named_bar_sync(2, kEpiThreads);
+          if (et < S) ptx::mbar_arrive_remote(ptx::map_to_cta(part_done, (uint32_t)et));
+        }
       }
     }
     if (!okw && et == 0 && p.error_flag) atomicCAS(p.error_flag, 0, (int)kErrWaitEpilogue);
@@ -1328,10 +1328,11 @@ static int clusters_that_fit(int bn, int s, int sms) {
 // channels, as measured by one CTA a tile: 560 on 64 x 32 tiles, on 128 x 64 tiles 1220 with halo tiles and 1450 without (which fill
 // better on narrow maps), on 128 x 128 tiles 1920; without boxes the copies of all SMs together allow 1565 and 2087.  A tile's beginning
 // and end 9000, 5560 and 11100 (the widest is finished in two passes), a launch of wide tiles 6700 more, a split 2700 or 2000: fitted to
-// 190 layers of 1 to 32 images (ResNet-18's and ResNet-50's, and random ones), each at every tile and split, of which the choice takes
-// 0.3 % more than the fastest.  On either side of the lines, us: 14x14x256 -> 256 3x3 of one image 64 x 32 10.4, wide 11.4; 7x7x512 -> 512
-// of one 12.6 and 15.1; 28x28x128 of eight 128 x 64 22.0, 128 x 128 23.9, 64 x 32 39.8.  Clusters of sixteen were slower at batch 1 than
-// clusters of eight (21 us against 15 for 256 channels on 16 x 16 pixels).
+// 190 layers of 1 to 32 images (ResNet-18's and ResNet-50's, and random ones), each at every tile and split, before the first planes had a
+// ring and 128 columns one issuing warp; of 250 such layers of 1 to 64 images since, the choice takes 0.2 % more than the fastest.  On
+// either side of the lines, us: 14x14x256 -> 256 3x3 of one image 64 x 32 10.4, wide 11.4; 7x7x512 -> 512 of one 12.6 and 15.1; 28x28x128
+// of eight 128 x 64 22.0, 128 x 128 23.9, 64 x 32 39.8.  Clusters of sixteen were slower at batch 1 than clusters of eight (21 us against
+// 15 for 256 channels on 16 x 16 pixels).
 void conv_f32_choose(ConvF32Args* args) {
   if (args->chosen) return;
   args->chosen = 1;

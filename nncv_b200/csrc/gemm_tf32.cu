@@ -26,8 +26,8 @@
 // MMAs take 780; for small matrices the 3500 clocks to the first MMA and, with clusters, the 5000 after the last one: 32 KB of partial
 // sums come from the other CTA at about 16 bytes a clock.  Out-of-range rows/columns read as zero and are clipped on store, so N and K
 // need only be multiples of 4 (16-byte row pitches of A, B and C).
-// us, inputs in L2, with B by global loads and now: 1024^3 20.2 15.5; 2048^3 112 77; 100x1000x2048 14.0 12.5; 1900x1500x520 37.7 29.0;
-// 4096x4096x512 112 91; 128x128x4096 19.9 16.0.
+// us, with B by global loads and now, inputs in L2 and (from memory): 1024^3 20.6 16.0 (26.6 22.5); 2048^3 113 76 (125 88); 100x1000x2048
+// 14.0 12.4 (20.5 18.4); 1900x1500x520 37.8 29.1 (43.0 34.8); 4096x4096x512 112 89 (123 100); 128x128x4096 20.0 15.7 (24.6 22.5).
 // Every wait is bounded and abortable; a timed-out wait sets the device status word.
 #include <cuda.h>
 #include <cudaTypedefs.h>
